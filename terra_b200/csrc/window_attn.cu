@@ -4,25 +4,31 @@
 //
 //   * activations are stored unshifted, window-major: rank p of the window dimension holds
 //     [B, nW_p, shardN, *] rows for its flat window range [win_start[p], win_start[p+1]);
-//   * a CTA owns one window of the *shifted* frame and a group of heads; every token of that window is
+//   * a CTA walks over windows of the *shifted* frame for a fixed group of heads; every token of a window is
 //     located (owner rank, row) in closed form and its Q/K/V row is read from the owner's buffer
 //     (a peer pointer over NVLink when the owner is another GPU); outputs are stored to the token's
 //     home row, again possibly on a peer;
 //   * relative-position bias comes from a shared-memory copy of the table, the shifted-window mask
 //     from the token's region id in the rolled frame; nothing of size [nW, N, N] is materialised.
 //
-// Windows here are small (N = wh*ww <= 128 keys), far below the tile sizes at which tcgen05 pays off,
-// and the op is bound by the Q/K/V/O traffic, so the products run on warp-level mma.sync with operands
-// staged in shared memory by 16-byte gathers.
+// Windows here are small (N = wh*ww <= 128 keys), far below the tile sizes at which tcgen05 pays off, so the products
+// run on warp-level mma.sync. The kernels are bound by instruction issue: every score element costs a scale + bias, a
+// max, an exponential and a sum besides its share of the products, so what the design buys is few other instructions
+// per element and enough independent warps:
+//   * one warp owns one 16-row block of the window for the whole kernel (block = NPAD / 16 warps), so everything that
+//     depends on (row, column) only is computed once: bias addresses become a register plus an immediate for windows 8
+//     or 12 wide, and the bias gradient of a thread's score elements is summed over all windows in registers (windows
+//     of 64 tokens) or in a private shared-memory slot (larger ones) and folded into the table once at the end;
+//   * the rows of the next window are fetched by cp.async while the current one is computed (two stages where the
+//     shared memory allows it); the token tables are computed two windows ahead;
+//   * a window's results are staged over its own dead operand rows and leave as 16-byte vectors, warp by warp.
+#include <atomic>
 #include "common.cuh"
 #include "host_api.h"
 #include "window_geo.cuh"
 
 namespace tb {
 namespace {
-
-constexpr int WA_THREADS = 128;
-constexpr int WA_WARPS = 4;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile(
@@ -41,502 +47,583 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
                : "r"(smem_u32(p)));
 }
 
-// 16-byte asynchronous copy global -> shared; `valid == false` writes zeros without reading the source.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
-  const int bytes = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+// 16-byte asynchronous copy global -> shared
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// 32-bit shared-memory load by address (keeps the table lookups of the softmax on LDS with one integer add each).
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));   // the table is read-only inside the item loop
-  return v;
-}
-
 constexpr float WA_LOG2E = 1.4426950408889634f;
 
-// Kernel layout.
-//   A CTA (4 warps) loops over (batch, window) items for one group of heads (G = heads_per_cta * HD channels).
-//   Per item: locate the window's tokens, gather Q/K/V [dO] rows into shared memory, then per head
-//     phase 1 (a warp per 16 query rows): S = Q K^T, P = softmax(scale S + bias [+ mask]) with the scores kept in the
-//       mma accumulator registers; forward: O = P V; backward: dP = dO V^T, dS = P (dP - rowsum(P dP)), dQ = dS K,
-//       P and dS stashed as bf16 for phase 2, bias gradient by shared-memory reductions;
-//     phase 2 (backward, a warp per 16 keys): dV = P^T dO, dK = dS^T Q;
-//   finally the results are scattered to the tokens' home rows.
-//   Softmax runs in the base-2 domain: the table is stored pre-multiplied by log2(e) and the scale carries the same
-//   factor, so an element costs one fused multiply-add, one table read, one max, one subtract and one ex2.
-//   Windows whose tokens share one mask region (all windows of unshifted layers, the interior windows of shifted
-//   ones) with N == NPAD take a branch-free path; the others a general one with the mask and padding tests.
-template <int HD, int NPAD, bool BWD>
-__global__ void __launch_bounds__(WA_THREADS, NPAD > 64 ? 1 : (BWD ? 3 : 5)) window_attn_kernel(const __grid_constant__ WindowAttnArgs a) {
+// Shared-memory layout of one instantiation. G = channels of a row handled by the CTA (HPC heads), rows padded by 16
+// bytes so that the eight rows of an ldmatrix fall into different banks for every G (16, 32, 64, 128).
+template <int HD, int NPAD, int HPC, bool BWD>
+struct WaCfg {
+  static constexpr int G = HD * HPC;
+  static constexpr int PITCH = G + 8;
+  static constexpr int PP = NPAD + 8;                            // pitch of the P / dS stash (backward)
+  static constexpr int THREADS = NPAD * 2;                       // a warp per 16 rows
+  static constexpr int MATS = BWD ? 4 : 3;                       // q, k, v [, dO]
+  static constexpr int MAT = NPAD * PITCH;                       // elements
+  static constexpr int STAGE = MATS * MAT;
+  static constexpr int STASH = BWD ? 2 * NPAD * PP : 0;          // P and dS, bf16
+  // dQ is staged in the warp's own stash rows before P and dS go there; a 128-channel head does not fit into them
+  static constexpr bool DQ_IN_STASH = HD <= NPAD;
+  static constexpr int DQ = (BWD && !DQ_IN_STASH) ? MAT : 0;
+  static constexpr bool ACC_REGS = NPAD == 64;                   // bias-gradient sums: registers or shared memory
+  static constexpr int ACC = (BWD && !ACC_REGS) ? NPAD * NPAD : 0;   // floats
+  static constexpr int FIXED = (STASH + DQ) * 2 + ACC * 4 + 3 * NPAD * 8 + NPAD * 4;
+  // Two stages unless the second one would cost resident CTAs: 56 KB lets four CTAs of four warps share an SM, the
+  // backward kernel is held to three (NPAD = 64) or fewer by its registers anyway.
+  static constexpr int TWO = FIXED + 2 * STAGE * 2;
+  static constexpr int STAGES = TWO <= (BWD ? (NPAD == 64 ? 74 : 110) : (NPAD == 64 ? 57 : 100)) * 1024 ? 2 : 1;
+  static constexpr size_t bytes(int nrel) { return static_cast<size_t>(FIXED) + STAGES * STAGE * 2 + HPC * nrel * 4; }
+  // resident CTAs per SM asked of the compiler: bounds the registers per thread
+  static constexpr int MIN_CTAS = NPAD > 96 ? 1 : (BWD ? (NPAD > 64 ? (HD > 64 ? 1 : 2) : (HD > 64 ? 2 : 3))
+                                                       : (NPAD > 64 ? 2 : (HD > 64 ? 4 : 5)));
+};
+
+struct WaItem {
+  int b, ii, jj;
+};
+
+__device__ __forceinline__ WaItem wa_item(const WindowAttnArgs& a, int item, int my_nw) {
+  WaItem w;
+  w.b = 0;
+  if (a.B > 1) {
+    w.b = item / my_nw;
+    item -= w.b * my_nw;
+  }
+  const int flat = a.win_start[a.my_wg] + item;
+  w.ii = flat / a.nWw;
+  w.jj = flat - w.ii * a.nWw;
+  return w;
+}
+
+// Row tables of one window: {row in the owner's buffer (-1: no such token), peer slot | region << 8} per token. Thread
+// `tid` < NPAD writes its token's entry.
+__device__ __forceinline__ void wa_table(const WindowAttnArgs& a, const Geo& geo, const WaItem& w, int ti, int tj, int2* entry) {
+  if (a.n_wg * a.sp * a.tp == 1 && !TB_DEBUG_BOUNDS) {
+    // one rank owns every token: a shifted token lies in its own window or the next one per axis
+    int ri = ti + a.sh, wi = w.ii, rj = tj + a.sw, wj = w.jj;
+    if (ri >= a.wh) {
+      ri -= a.wh;
+      wi = wi + 1 == a.nWh ? 0 : wi + 1;
+    }
+    if (rj >= a.ww) {
+      rj -= a.ww;
+      wj = wj + 1 == a.nWw ? 0 : wj + 1;
+    }
+    const int rh = (a.sh > 0 && w.ii == a.nWh - 1) ? (ti < a.wh - a.sh ? 1 : 2) : 0;
+    const int rw = (a.sw > 0 && w.jj == a.nWw - 1) ? (tj < a.ww - a.sw ? 1 : 2) : 0;
+    *entry = make_int2(((w.b * a.nWh + wi) * a.nWw + wj) * geo.N + ri * a.ww + rj, (rh * 3 + rw) << 8);
+  } else {
+    const Home h = locate_ij(a, geo, w.b, w.ii, w.jj, ti, tj);
+    *entry = make_int2(static_cast<int>(h.row), h.slot | (h.region << 8));
+  }
+}
+
+// Row-wise copies of one window into a stage: VPR lanes per row move its 16-byte vectors of q, k, v [and dO].
+template <class Cfg, bool BWD>
+__device__ __forceinline__ void wa_gather(const WindowAttnArgs& a, const int2* tab, uint32_t stage, int ch0, int tid, int q0, int q1) {
+  constexpr int VPR = Cfg::G / 8, RPP = Cfg::THREADS / VPR, NPAD = Cfg::MAT / Cfg::PITCH;
+  static_assert(Cfg::THREADS % VPR == 0, "lanes per row");
+  const int v = tid % VPR;
+#pragma unroll
+  for (int i = 0; i < (NPAD + RPP - 1) / RPP; ++i) {
+    const int r = tid / VPR + i * RPP;
+    if (NPAD % RPP != 0 && r >= NPAD) break;
+    const int2 e = tab[r];
+    if (e.x < 0) continue;                   // a padding row: zero since the start
+    const int slot = e.y & 255;
+    const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.qkv[slot]) + static_cast<long long>(e.x) * (3 * a.C) + ch0 + v * 8;
+    const uint32_t dst = stage + (r * Cfg::PITCH + v * 8) * 2;
+    if (BWD || (r >= q0 && r < q1)) cp_async16(dst, src);
+    cp_async16(dst + Cfg::MAT * 2, src + a.C);
+    cp_async16(dst + Cfg::MAT * 4, src + 2 * a.C);
+    if (BWD)
+      cp_async16(dst + Cfg::MAT * 6,
+                 static_cast<const __nv_bfloat16*>(a.dout[slot]) + static_cast<long long>(e.x) * a.C + ch0 + v * 8);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// 16 rows x CH channels staged in shared memory (pitch in elements) to the rows' home buffers.
+template <int CH>
+__device__ __forceinline__ void wa_store(void* const* bases, long long ld, int col, const __nv_bfloat16* src, int pitch,
+                                         const int2* tab, int row0, int lane, int q0, int q1) {
+  constexpr int VPR = CH / 8;
+#pragma unroll
+  for (int i = 0; i < (16 * VPR + 31) / 32; ++i) {
+    const int idx = lane + 32 * i;
+    const int r = idx / VPR, v = idx % VPR;
+    if (row0 + r >= q0 && row0 + r < q1) {
+      const int2 e = tab[row0 + r];
+      __nv_bfloat16* o = static_cast<__nv_bfloat16*>(bases[e.y & 255]) + static_cast<long long>(e.x) * ld + col + v * 8;
+      *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(src + r * pitch + v * 8);
+    }
+  }
+}
+
+// Scores of a 16-row block: s <- s * scale + bias (+ mask), base-2 domain, and the row maxima of this thread's columns.
+// `tb` is the head's table in shared memory, pre-multiplied by log2(e). The table index of (query r, key c) is
+// cofs(r) - cofs(c) + rel0 with cofs(t) = (t / ww) (2 ww - 1) + t % ww. For windows 8 (12) wide the columns of a thread
+// repeat every 1 (3) blocks of 8, so an index is one of 1 (3) per-thread bases plus a compile-time constant; other
+// widths read cofs from shared memory.
+template <int NPAD, int WW>
+__device__ __forceinline__ void wa_scores(float (&s)[NPAD / 8][4], float scale2, const float* tb, int rel0, const int* cofs,
+                                          const int2* tab, int r0, int tq, int N, bool general, bool use_mask, float& mx0,
+                                          float& mx1) {
+  const int r1 = r0 + 8;
+  if (!general) {
+    if constexpr (WW == 8) {
+      // row r1 = r0 + 8 is the next window row, same column: its bias at key block nb is row r0's at block nb - 1
+      const float* p = tb + ((r0 >> 3) * 15 + (r0 & 7) - 2 * tq + rel0);
+      float b0 = p[15], b1 = p[14];
+#pragma unroll
+      for (int nb = 0; nb < NPAD / 8; ++nb) {
+        s[nb][2] = fmaf(s[nb][2], scale2, b0);
+        s[nb][3] = fmaf(s[nb][3], scale2, b1);
+        b0 = p[-15 * nb];
+        b1 = p[-15 * nb - 1];
+        s[nb][0] = fmaf(s[nb][0], scale2, b0);
+        s[nb][1] = fmaf(s[nb][1], scale2, b1);
+        mx0 = fmaxf(mx0, fmaxf(s[nb][0], s[nb][1]));
+        mx1 = fmaxf(mx1, fmaxf(s[nb][2], s[nb][3]));
+      }
+    } else if constexpr (WW == 12) {
+      const int ro0 = cofs[r0] + rel0, dr = cofs[r1] - cofs[r0];
+      // columns 8 m + 2 tq of the first three blocks, m = 0, 1, 2; later blocks are whole window rows (2 per 3 blocks) on
+      const float* p[3];
+      p[0] = tb + ro0 - 2 * tq;
+      p[1] = tb + ro0 - (tq < 2 ? 8 + 2 * tq : 23 + 2 * tq - 4);
+      p[2] = tb + ro0 - (23 + 4 + 2 * tq);
+#pragma unroll
+      for (int nb = 0; nb < NPAD / 8; ++nb) {
+        const float* c = p[nb % 3] - (nb / 3) * 46;
+        s[nb][0] = fmaf(s[nb][0], scale2, c[0]);
+        s[nb][1] = fmaf(s[nb][1], scale2, c[-1]);
+        s[nb][2] = fmaf(s[nb][2], scale2, c[dr]);
+        s[nb][3] = fmaf(s[nb][3], scale2, c[dr - 1]);
+        mx0 = fmaxf(mx0, fmaxf(s[nb][0], s[nb][1]));
+        mx1 = fmaxf(mx1, fmaxf(s[nb][2], s[nb][3]));
+      }
+    } else {
+      const float *t0 = tb + cofs[r0] + rel0, *t1 = tb + cofs[r1] + rel0;
+#pragma unroll
+      for (int nb = 0; nb < NPAD / 8; ++nb) {
+        const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
+        s[nb][0] = fmaf(s[nb][0], scale2, t0[-co.x]);
+        s[nb][1] = fmaf(s[nb][1], scale2, t0[-co.y]);
+        s[nb][2] = fmaf(s[nb][2], scale2, t1[-co.x]);
+        s[nb][3] = fmaf(s[nb][3], scale2, t1[-co.y]);
+        mx0 = fmaxf(mx0, fmaxf(s[nb][0], s[nb][1]));
+        mx1 = fmaxf(mx1, fmaxf(s[nb][2], s[nb][3]));
+      }
+    }
+  } else {
+    // windows that the mask cuts, and windows with padding columns (their scores are lowest, their probabilities zero)
+    const int reg0 = tab[r0].y >> 8, reg1 = tab[r1].y >> 8;
+    const bool row0 = r0 < N, row1 = r1 < N;
+    const float *t0 = tb + (row0 ? cofs[r0] + rel0 : 0), *t1 = tb + (row1 ? cofs[r1] + rel0 : 0);
+#pragma unroll
+    for (int nb = 0; nb < NPAD / 8; ++nb) {
+      const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int col = nb * 8 + tq * 2 + (k & 1);
+        const bool lo = k < 2;
+        float v = s[nb][k] * scale2;
+        if (col < N) {
+          if (lo ? row0 : row1) v += (lo ? t0 : t1)[-((k & 1) ? co.y : co.x)];
+          if (use_mask && (tab[col].y >> 8) != (lo ? reg0 : reg1)) v += -100.f * WA_LOG2E;
+        } else {
+          v = -1e30f;
+        }
+        s[nb][k] = v;
+        if (lo) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
+      }
+    }
+  }
+}
+
+// d[nb] += A(16 rows at `arow`, HD channels) * B(NPAD rows at `bmat`)^T, both row-major bf16 in shared memory
+template <int HD, int NPAD, int PITCH>
+__device__ __forceinline__ void wa_mma_nt(float (&d)[NPAD / 8][4], const __nv_bfloat16* arow, const __nv_bfloat16* bmat, int lane) {
+#pragma unroll
+  for (int nb = 0; nb < NPAD / 8; ++nb)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d[nb][k] = 0.f;
+#pragma unroll
+  for (int kk = 0; kk < HD / 16; ++kk) {
+    uint32_t af[4];
+    ldsm_x4(af, arow + (lane & 15) * PITCH + kk * 16 + (lane >> 4) * 8);
+#pragma unroll
+    for (int nb = 0; nb < NPAD / 8; nb += 2) {
+      uint32_t bf[4];
+      ldsm_x4(bf, bmat + (nb * 8 + (lane & 7) + (lane >> 4) * 8) * PITCH + kk * 16 + ((lane >> 3) & 1) * 8);
+      const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
+      mma_bf16_16816(d[nb], af, b0);
+      mma_bf16_16816(d[nb + 1], af, b1);
+    }
+  }
+}
+
+// o = P (16 x NPAD, fp32 accumulator layout, rounded to bf16) * B (NPAD rows, HD channels, row-major in shared memory)
+template <int HD, int NPAD, int PITCH>
+__device__ __forceinline__ void wa_mma_pn(float (&o)[HD / 8][4], const float (&p)[NPAD / 8][4], const __nv_bfloat16* bmat, int lane) {
+#pragma unroll
+  for (int nb = 0; nb < HD / 8; ++nb)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[nb][k] = 0.f;
+#pragma unroll
+  for (int j = 0; j < NPAD / 16; ++j) {
+    const uint32_t pf[4] = {pack_bf16x2(p[2 * j][0], p[2 * j][1]), pack_bf16x2(p[2 * j][2], p[2 * j][3]),
+                            pack_bf16x2(p[2 * j + 1][0], p[2 * j + 1][1]), pack_bf16x2(p[2 * j + 1][2], p[2 * j + 1][3])};
+#pragma unroll
+    for (int nb = 0; nb < HD / 8; nb += 2) {
+      uint32_t bf[4];
+      ldsm_x4_t(bf, bmat + (j * 16 + (lane & 15)) * PITCH + nb * 8 + (lane >> 4) * 8);
+      const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
+      mma_bf16_16816(o[nb], pf, b0);
+      mma_bf16_16816(o[nb + 1], pf, b1);
+    }
+  }
+}
+
+// Softmax numerators of the block (in place) and the reciprocal row sums.
+template <int NPAD>
+__device__ __forceinline__ void wa_softmax(float (&s)[NPAD / 8][4], float mx0, float mx1, float& inv0, float& inv1) {
+  mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+  mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+  mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+  mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+  float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+  for (int nb = 0; nb < NPAD / 8; ++nb) {
+    s[nb][0] = exp2f(s[nb][0] - mx0);
+    s[nb][1] = exp2f(s[nb][1] - mx0);
+    s[nb][2] = exp2f(s[nb][2] - mx1);
+    s[nb][3] = exp2f(s[nb][3] - mx1);
+    sum0 += s[nb][0] + s[nb][1];
+    sum1 += s[nb][2] + s[nb][3];
+  }
+  sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
+  sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
+  sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
+  sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
+  inv0 = 1.f / sum0;
+  inv1 = 1.f / sum1;
+}
+
+// A warp's 16 x HD accumulator tile, scaled per row, to bf16 rows in shared memory (rows r0 = gq and r0 + 8 of the tile).
+template <int HD>
+__device__ __forceinline__ void wa_stage(__nv_bfloat16* dst, int pitch, const float (&o)[HD / 8][4], float f0, float f1, int gq,
+                                         int tq, bool ok0, bool ok1) {
+#pragma unroll
+  for (int nb = 0; nb < HD / 8; ++nb) {
+    if (ok0) *reinterpret_cast<uint32_t*>(dst + gq * pitch + nb * 8 + tq * 2) = pack_bf16x2(o[nb][0] * f0, o[nb][1] * f0);
+    if (ok1) *reinterpret_cast<uint32_t*>(dst + (gq + 8) * pitch + nb * 8 + tq * 2) = pack_bf16x2(o[nb][2] * f1, o[nb][3] * f1);
+  }
+}
+
+template <int HD, int NPAD, int HPC, int WW, bool BWD>
+__global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD, NPAD, HPC, BWD>::MIN_CTAS))
+    window_attn_kernel(const __grid_constant__ WindowAttnArgs a) {
+  using Cfg = WaCfg<HD, NPAD, HPC, BWD>;
+  static_assert(!BWD || HPC == 1, "the backward kernel keeps one head's bias-gradient sums");
+  constexpr int G = Cfg::G, PITCH = Cfg::PITCH, PP = Cfg::PP, STAGES = Cfg::STAGES, NB = NPAD / 8;
   extern __shared__ __align__(16) uint8_t smem[];
-  const int hpc = a.heads_per_cta;
-  const int G = hpc * HD;
-  const int stride = G + 8;
-  constexpr int pstride = NPAD + 8;
+  __nv_bfloat16* stages = reinterpret_cast<__nv_bfloat16*>(smem);
+  __nv_bfloat16* Ps = stages + STAGES * Cfg::STAGE;             // backward: [NPAD][PP] each
+  __nv_bfloat16* dSs = Ps + Cfg::STASH / 2;
+  __nv_bfloat16* dQs = dSs + Cfg::STASH / 2;                     // backward, 128-channel heads
+  float* acc_s = reinterpret_cast<float*>(dQs + Cfg::DQ);        // backward: [NB / 1][THREADS][4] bias-gradient sums
+  int2* tabs = reinterpret_cast<int2*>(acc_s + Cfg::ACC);        // [3][NPAD]
+  int* cofs = reinterpret_cast<int*>(tabs + 3 * NPAD);           // [NPAD]
+  float* bias_s = reinterpret_cast<float*>(cofs + NPAD);         // [HPC][nrel], times log2(e)
+
   Geo geo;
   geo.N = a.wh * a.ww;
   geo.nrel = (2 * a.wh - 1) * (2 * a.ww - 1);
   geo.Hg = a.nWh * a.wh;
   geo.Wg = a.nWw * a.ww;
   const int N = geo.N;
-
-  __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem);
-  __nv_bfloat16* Ks = Qs + NPAD * stride;
-  __nv_bfloat16* Vs = Ks + NPAD * stride;
-  __nv_bfloat16* dOs = Vs + NPAD * stride;                              // BWD only
-  __nv_bfloat16* dQs = dOs + (BWD ? NPAD * stride : 0);                 // BWD only
-  __nv_bfloat16* Ps = dQs + (BWD ? NPAD * stride : 0);                  // BWD only [NPAD][pstride]
-  __nv_bfloat16* dSs = Ps + (BWD ? NPAD * pstride : 0);                 // BWD only
-  float* bias_s = reinterpret_cast<float*>(dSs + (BWD ? NPAD * pstride : 0));   // [hpc][nrel], times log2(e)
-  float* dbias_s = bias_s + hpc * geo.nrel;                                      // BWD only [hpc][nrel]
-  // the float tables have an arbitrary length: round up so that the 8-byte row offsets are aligned
-  // (offset arithmetic on the shared array itself, so the compiler keeps these accesses in the shared state space)
-  const size_t tables_off =
-      (static_cast<size_t>(reinterpret_cast<uint8_t*>(dbias_s + (BWD ? hpc * geo.nrel : 0)) - smem) + 15) & ~size_t(15);
-  long long* rowofs = reinterpret_cast<long long*>(smem + tables_off);                       // [NPAD]
-  int* rowslot = reinterpret_cast<int*>(rowofs + NPAD);                                      // [NPAD]
-  int* rowreg = rowslot + NPAD;                                                              // [NPAD]
-  // cofs[t] = 4 * ((t / ww) * (2 ww - 1) + (t % ww)): the byte offset into a head's table of the relative position
-  // of (query r, key c) is cofs[r] - cofs[c] + 4 * rel0, so the inner loops need no division.
-  int* cofs = rowreg + NPAD;                                                                 // [NPAD]
-  // bias gradient (BWD): posofs[tj * ww + cj] = tj * pstride + cj (low 16 bits) | tj << 16; one ww*ww fp32 scratch per warp
-  int* posofs = cofs + NPAD;                                                                 // [ww*ww]
-  float* mbuf = reinterpret_cast<float*>(posofs + (BWD ? a.ww * a.ww : 0));                  // [WA_WARPS][ww*ww]
   const int rel0 = (a.wh - 1) * (2 * a.ww - 1) + (a.ww - 1);
-
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gq = lane >> 2, tq = lane & 3;
-  const int cg = blockIdx.y;            // head group
-  const int head0 = cg * hpc;
+  const int head0 = blockIdx.y * HPC, ch0 = blockIdx.y * G;
   const bool use_bias = a.bias_table != nullptr;
   const bool bias_grad = BWD && use_bias && a.dbias_table != nullptr;
   const int my_nw = a.win_start[a.my_wg + 1] - a.win_start[a.my_wg];
+  const int items = a.B * my_nw;
   const int q0 = a.my_sp * a.shardN;
   const int q1 = min(N, q0 + a.shardN);
   const float scale2 = a.scale * WA_LOG2E;
+  const int ti = tid / a.ww, tj = tid % a.ww;                    // token `tid` of a window
 
-  for (int i = tid; i < hpc * geo.nrel; i += WA_THREADS) {
+  for (int i = tid; i < HPC * geo.nrel; i += Cfg::THREADS) {
     const int h = i / geo.nrel, r = i % geo.nrel;
     bias_s[i] = use_bias ? a.bias_table[r * a.num_heads + head0 + h] * WA_LOG2E : 0.f;
-    if (BWD) dbias_s[i] = 0.f;
   }
-  for (int t = tid; t < NPAD; t += WA_THREADS) cofs[t] = 4 * ((t / a.ww) * (2 * a.ww - 1) + (t % a.ww));
-  if (BWD)
-    for (int t = tid; t < a.ww * a.ww; t += WA_THREADS) posofs[t] = ((t / a.ww) * pstride + (t % a.ww)) | ((t / a.ww) << 16);
-  // Row-wise copies between global and shared memory: a warp takes whole rows, lane l moves the 16-byte vectors
-  // l and l + 32 of the row's (matrix, vector) list. The (matrix, vector) split is computed once here, so the
-  // copy loops contain no division.
-  const int vpr = G / 8;                       // 16-byte vectors per row and matrix
-  const int gather_mats = BWD ? 4 : 3;         // q, k, v [, dO]
-  int gm[2], gv[2];
-  bool gok[2];
+  if (tid < NPAD) {
+    cofs[tid] = ti * (2 * a.ww - 1) + tj;
+    if (tid >= N)
+      for (int k = 0; k < 3; ++k) tabs[k * NPAD + tid] = make_int2(-1, 15 << 8);
+  }
+  if (N < NPAD)   // padding rows are never written again
+    for (int i = tid; i < STAGES * Cfg::MATS * (NPAD - N) * (PITCH / 2); i += Cfg::THREADS) {
+      const int m = i / ((NPAD - N) * (PITCH / 2)), o = i % ((NPAD - N) * (PITCH / 2));
+      reinterpret_cast<uint32_t*>(stages + m * Cfg::MAT + N * PITCH)[o] = 0u;
+    }
+  for (int i = tid; i < Cfg::ACC; i += Cfg::THREADS) acc_s[i] = 0.f;
+
+  float acc[(BWD && Cfg::ACC_REGS) ? NB : 1][4];
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int idx = lane + 32 * k;
-    gok[k] = idx < gather_mats * vpr;
-    gm[k] = gok[k] ? idx / vpr : 0;
-    gv[k] = gok[k] ? idx % vpr : 0;
+  for (int nb = 0; nb < (BWD && Cfg::ACC_REGS ? NB : 1); ++nb)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[nb][k] = 0.f;
+
+  const int step = gridDim.x;
+  const int row0 = warp * 16, r0 = row0 + gq, r1 = r0 + 8;
+  const bool in0 = r0 < N, in1 = r1 < N;
+  const float own0 = (r0 >= q0 && r0 < q1) ? 1.f : 0.f, own1 = (r1 >= q0 && r1 < q1) ? 1.f : 0.f;   // this rank's query rows
+
+  WaItem next = wa_item(a, blockIdx.x, my_nw);      // the item whose table was written last
+  WaItem cur = next;
+  if (tid < N) wa_table(a, geo, next, ti, tj, tabs + tid);
+  __syncthreads();
+  if (STAGES == 2) wa_gather<Cfg, BWD>(a, tabs, smem_u32(stages), ch0, tid, q0, q1);
+  if (static_cast<int>(blockIdx.x) + step < items) {
+    next = wa_item(a, blockIdx.x + step, my_nw);
+    if (tid < N) wa_table(a, geo, next, ti, tj, tabs + NPAD + tid);
   }
 
-  const int items = a.B * my_nw;
-  for (int item = blockIdx.x; item < items; item += gridDim.x) {
-    const int b = item / my_nw, lw = item % my_nw;
-    const int flat = a.win_start[a.my_wg] + lw;
-    const int ii = flat / a.nWw, jj = flat % a.nWw;
-    __syncthreads();   // previous item fully consumed
-    int differs = 0;
-    if (tid < NPAD) {
-      if (tid < N) {
-        const Home h = locate(a, geo, b, ii, jj, tid);
-        rowofs[tid] = h.row;
-        rowslot[tid] = h.slot;
-        rowreg[tid] = h.region;
-        differs = h.region != region_of(a, geo, ii * a.wh, jj * a.ww);
-      } else {
-        rowofs[tid] = -1;
-        rowslot[tid] = 0;
-        rowreg[tid] = 15;
-      }
-    }
-    // (also the barrier that publishes the row tables)
-    const bool general = (__syncthreads_or(differs) != 0 && a.use_mask) || N != NPAD;
-    // ---- gather Q (query rows), K, V (all rows) [and dO] for this head group with 16-byte asynchronous copies
-    //      (global or peer memory -> shared memory, zero fill for rows outside the window / shard): all of a lane's
-    //      copies are in flight at once, one memory round trip per item
-    for (int r = warp; r < NPAD; r += WA_WARPS) {
-      const long long ro = rowofs[r];
-      const int sl = rowslot[r];
-      const bool in_win = r < N;
-      const __nv_bfloat16* qb = static_cast<const __nv_bfloat16*>(a.qkv[sl]) + (in_win ? ro * (3LL * a.C) + cg * G : 0);
-      const __nv_bfloat16* db =
-          BWD ? static_cast<const __nv_bfloat16*>(a.dout[sl]) + (in_win ? ro * a.C + cg * G : 0) : nullptr;
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        if (gok[k]) {
-          const int m = gm[k];
-          const bool q_like = (m == 0 || m == 3);
-          const bool valid = in_win && (!q_like || BWD || (r >= q0 && r < q1));
-          const __nv_bfloat16* src = (m < 3) ? qb + (valid ? m * a.C + gv[k] * 8 : 0) : db + (valid ? gv[k] * 8 : 0);
-          __nv_bfloat16* dst = (m == 0 ? Qs : (m == 1 ? Ks : (m == 2 ? Vs : dOs))) + r * stride + gv[k] * 8;
-          cp_async16(dst, src, valid);
-        }
-      }
+  int slot = 0, buf = 0;
+  for (int item = blockIdx.x; item < items; item += step) {
+    const int2* tab = tabs + slot * NPAD;
+    const int slot1 = slot == 2 ? 0 : slot + 1, slot2 = slot1 == 2 ? 0 : slot1 + 1;
+    __nv_bfloat16* Qs = stages + buf * Cfg::STAGE;
+    __nv_bfloat16 *Ks = Qs + Cfg::MAT, *Vs = Ks + Cfg::MAT, *dOs = Vs + Cfg::MAT;
+    if (STAGES == 1) {
+      __syncthreads();          // the previous window has been consumed, this window's table is visible
+      wa_gather<Cfg, BWD>(a, tab, smem_u32(Qs), ch0, tid, q0, q1);
     }
     cp_async_wait_all();
-    __syncthreads();
-
-    constexpr int rblocks = NPAD / 16;
-    for (int hh = 0; hh < hpc; ++hh) {
-      const uint32_t btb = smem_u32(bias_s + hh * geo.nrel);
-      // =============================== phase 1: per 16-query-row block
-      for (int rb = warp; rb < rblocks; rb += WA_WARPS) {
-        if (rb * 16 >= N) continue;
-        if (!BWD && (rb * 16 >= q1 || rb * 16 + 16 <= q0)) continue;
-        float s[NPAD / 8][4];
-#pragma unroll
-        for (int nb = 0; nb < NPAD / 8; ++nb)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) s[nb][k] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          uint32_t af[4];
-          ldsm_x4(af, Qs + (rb * 16 + (lane & 15)) * stride + hh * HD + kk * 16 + (lane >> 4) * 8);
-#pragma unroll
-          for (int nb = 0; nb < NPAD / 8; nb += 2) {
-            uint32_t bf[4];
-            ldsm_x4(bf, Ks + (nb * 8 + (lane & 7) + (lane >> 4) * 8) * stride + hh * HD + kk * 16 + ((lane >> 3) & 1) * 8);
-            const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
-            mma_bf16_16816(s[nb], af, b0);
-            mma_bf16_16816(s[nb + 1], af, b1);
-          }
-        }
-        // scale, bias, mask, softmax numerators (rows gq and gq+8 of the block), base-2 domain
-        const int r0 = rb * 16 + gq, r1 = r0 + 8;
-        const int ro0 = cofs[r0] + 4 * rel0, ro1 = cofs[r1] + 4 * rel0;   // r1 < NPAD always
-        float mx0 = -1e30f, mx1 = -1e30f;
-        if (!general) {
-#pragma unroll
-          for (int nb = 0; nb < NPAD / 8; ++nb) {
-            const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
-            s[nb][0] = fmaf(s[nb][0], scale2, lds_f32(btb + (ro0 - co.x)));
-            s[nb][1] = fmaf(s[nb][1], scale2, lds_f32(btb + (ro0 - co.y)));
-            s[nb][2] = fmaf(s[nb][2], scale2, lds_f32(btb + (ro1 - co.x)));
-            s[nb][3] = fmaf(s[nb][3], scale2, lds_f32(btb + (ro1 - co.y)));
-            mx0 = fmaxf(mx0, fmaxf(s[nb][0], s[nb][1]));
-            mx1 = fmaxf(mx1, fmaxf(s[nb][2], s[nb][3]));
-          }
-        } else {
-          const int reg0 = rowreg[r0], reg1 = rowreg[r1];
-          const bool row0 = r0 < N, row1 = r1 < N;
-#pragma unroll
-          for (int nb = 0; nb < NPAD / 8; ++nb) {
-            const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
-            const int2 cr = *reinterpret_cast<const int2*>(rowreg + nb * 8 + tq * 2);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int col = nb * 8 + tq * 2 + (k & 1);
-              const bool lo = k < 2;
-              float v = s[nb][k] * scale2;
-              if (col < N) {
-                if (lo ? row0 : row1) v += lds_f32(btb + ((lo ? ro0 : ro1) - ((k & 1) ? co.y : co.x)));
-                if (a.use_mask && ((k & 1) ? cr.y : cr.x) != (lo ? reg0 : reg1)) v += -100.f * WA_LOG2E;
-              } else {
-                v = -1e30f;
-              }
-              s[nb][k] = v;
-              if (lo) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
-            }
-          }
-        }
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-        for (int nb = 0; nb < NPAD / 8; ++nb) {
-          s[nb][0] = exp2f(s[nb][0] - mx0);
-          s[nb][1] = exp2f(s[nb][1] - mx0);
-          s[nb][2] = exp2f(s[nb][2] - mx1);
-          s[nb][3] = exp2f(s[nb][3] - mx1);
-          sum0 += s[nb][0] + s[nb][1];
-          sum1 += s[nb][2] + s[nb][3];
-        }
-        sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
-        sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
-        sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
-        sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
-        const float inv0 = 1.f / sum0, inv1 = 1.f / sum1;
-        if (!BWD) {
-          // O = P V with the numerators as P; the row normalisation is applied to the (much smaller) output.
-          // Staged over this warp's own Q rows (no other warp reads them).
-          float o[HD / 8][4];
-#pragma unroll
-          for (int nb = 0; nb < HD / 8; ++nb)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) o[nb][k] = 0.f;
-#pragma unroll
-          for (int j = 0; j < NPAD / 16; ++j) {
-            const uint32_t pf[4] = {pack_bf16x2(s[2 * j][0], s[2 * j][1]), pack_bf16x2(s[2 * j][2], s[2 * j][3]),
-                                    pack_bf16x2(s[2 * j + 1][0], s[2 * j + 1][1]),
-                                    pack_bf16x2(s[2 * j + 1][2], s[2 * j + 1][3])};
-#pragma unroll
-            for (int nb = 0; nb < HD / 8; nb += 2) {
-              uint32_t bf[4];
-              ldsm_x4_t(bf, Vs + (j * 16 + (lane & 15)) * stride + hh * HD + nb * 8 + (lane >> 4) * 8);
-              const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
-              mma_bf16_16816(o[nb], pf, b0);
-              mma_bf16_16816(o[nb + 1], pf, b1);
-            }
-          }
-          __syncwarp();
-#pragma unroll
-          for (int nb = 0; nb < HD / 8; ++nb) {
-            *reinterpret_cast<uint32_t*>(Qs + r0 * stride + hh * HD + nb * 8 + tq * 2) =
-                pack_bf16x2(o[nb][0] * inv0, o[nb][1] * inv0);
-            *reinterpret_cast<uint32_t*>(Qs + r1 * stride + hh * HD + nb * 8 + tq * 2) =
-                pack_bf16x2(o[nb][2] * inv1, o[nb][3] * inv1);
-          }
-        } else {
-#pragma unroll
-          for (int nb = 0; nb < NPAD / 8; ++nb) {
-            s[nb][0] *= inv0;
-            s[nb][1] *= inv0;
-            s[nb][2] *= inv1;
-            s[nb][3] *= inv1;
-          }
-          // dP = dO V^T
-          float dp[NPAD / 8][4];
-#pragma unroll
-          for (int nb = 0; nb < NPAD / 8; ++nb)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dp[nb][k] = 0.f;
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) {
-            uint32_t af[4];
-            ldsm_x4(af, dOs + (rb * 16 + (lane & 15)) * stride + hh * HD + kk * 16 + (lane >> 4) * 8);
-#pragma unroll
-            for (int nb = 0; nb < NPAD / 8; nb += 2) {
-              uint32_t bf[4];
-              ldsm_x4(bf, Vs + (nb * 8 + (lane & 7) + (lane >> 4) * 8) * stride + hh * HD + kk * 16 + ((lane >> 3) & 1) * 8);
-              const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
-              mma_bf16_16816(dp[nb], af, b0);
-              mma_bf16_16816(dp[nb + 1], af, b1);
-            }
-          }
-          float d0 = 0.f, d1 = 0.f;
-#pragma unroll
-          for (int nb = 0; nb < NPAD / 8; ++nb) {
-            d0 += s[nb][0] * dp[nb][0] + s[nb][1] * dp[nb][1];
-            d1 += s[nb][2] * dp[nb][2] + s[nb][3] * dp[nb][3];
-          }
-          d0 += __shfl_xor_sync(0xffffffffu, d0, 1);
-          d0 += __shfl_xor_sync(0xffffffffu, d0, 2);
-          d1 += __shfl_xor_sync(0xffffffffu, d1, 1);
-          d1 += __shfl_xor_sync(0xffffffffu, d1, 2);
-          // dS = P * (dP - D); stash P and dS (bf16) for phase 2 and the bias gradient
-#pragma unroll
-          for (int nb = 0; nb < NPAD / 8; ++nb) {
-            float ds[4];
-            ds[0] = s[nb][0] * (dp[nb][0] - d0);
-            ds[1] = s[nb][1] * (dp[nb][1] - d0);
-            ds[2] = s[nb][2] * (dp[nb][2] - d1);
-            ds[3] = s[nb][3] * (dp[nb][3] - d1);
-            const int col = nb * 8 + tq * 2;
-            *reinterpret_cast<uint32_t*>(Ps + r0 * pstride + col) = pack_bf16x2(s[nb][0], s[nb][1]);
-            *reinterpret_cast<uint32_t*>(Ps + r1 * pstride + col) = pack_bf16x2(s[nb][2], s[nb][3]);
-            *reinterpret_cast<uint32_t*>(dSs + r0 * pstride + col) = pack_bf16x2(ds[0], ds[1]);
-            *reinterpret_cast<uint32_t*>(dSs + r1 * pstride + col) = pack_bf16x2(ds[2], ds[3]);
-            dp[nb][0] = ds[0]; dp[nb][1] = ds[1]; dp[nb][2] = ds[2]; dp[nb][3] = ds[3];
-          }
-          // dQ = scale * dS K
-          float dq[HD / 8][4];
-#pragma unroll
-          for (int nb = 0; nb < HD / 8; ++nb)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dq[nb][k] = 0.f;
-#pragma unroll
-          for (int j = 0; j < NPAD / 16; ++j) {
-            const uint32_t pf[4] = {pack_bf16x2(dp[2 * j][0], dp[2 * j][1]), pack_bf16x2(dp[2 * j][2], dp[2 * j][3]),
-                                    pack_bf16x2(dp[2 * j + 1][0], dp[2 * j + 1][1]),
-                                    pack_bf16x2(dp[2 * j + 1][2], dp[2 * j + 1][3])};
-#pragma unroll
-            for (int nb = 0; nb < HD / 8; nb += 2) {
-              uint32_t bf[4];
-              ldsm_x4_t(bf, Ks + (j * 16 + (lane & 15)) * stride + hh * HD + nb * 8 + (lane >> 4) * 8);
-              const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
-              mma_bf16_16816(dq[nb], pf, b0);
-              mma_bf16_16816(dq[nb + 1], pf, b1);
-            }
-          }
-#pragma unroll
-          for (int nb = 0; nb < HD / 8; ++nb) {
-            *reinterpret_cast<uint32_t*>(dQs + r0 * stride + hh * HD + nb * 8 + tq * 2) =
-                pack_bf16x2(dq[nb][0] * a.scale, dq[nb][1] * a.scale);
-            *reinterpret_cast<uint32_t*>(dQs + r1 * stride + hh * HD + nb * 8 + tq * 2) =
-                pack_bf16x2(dq[nb][2] * a.scale, dq[nb][3] * a.scale);
-          }
-        }
-      }
-      if (BWD) {
-        __syncthreads();
-        // Bias gradient: entry (di, dj) of the table collects dS[r][c] over the pairs with r - c = (di, dj), for
-        // this rank's query rows. A warp takes the row displacements di, di + 4, ...: its lanes first add up, for
-        // each in-row position pair (tj, cj), the ww x ww blocks (ti, ci = ti - di) of dS (conflict-free reads,
-        // balanced over the warps), then lanes sum the diagonals tj - cj = dj of that small matrix. Every entry
-        // has one owner, so no atomics are needed inside the CTA.
-        if (bias_grad) {
-          const int ww2 = a.ww * a.ww, ndi = 2 * a.wh - 1, ndj = 2 * a.ww - 1;
-          const bool partial = q0 > 0 || q1 < N;
-          float* Mw = mbuf + warp * ww2;
-          for (int di_idx = warp; di_idx < ndi; di_idx += WA_WARPS) {
-            const int di = di_idx - (a.wh - 1);
-            const int ti_lo = max(0, di), ti_hi = min(a.wh, a.wh + di);
-            for (int pos = lane; pos < ww2; pos += 32) {
-              const int po = posofs[pos] & 0xffff, tj = posofs[pos] >> 16;
-              float acc = 0.f;
-              for (int ti = ti_lo; ti < ti_hi; ++ti) {
-                const int r = ti * a.ww + tj;
-                if (!partial || (r >= q0 && r < q1))
-                  acc += __bfloat162float(dSs[ti * a.ww * pstride + (ti - di) * a.ww + po]);
-              }
-              Mw[pos] = acc;
-            }
-            __syncwarp();
-            for (int dj_idx = lane; dj_idx < ndj; dj_idx += 32) {
-              const int dj = dj_idx - (a.ww - 1);
-              float acc = 0.f;
-              for (int tj = max(0, dj); tj < min(a.ww, a.ww + dj); ++tj) acc += Mw[tj * (a.ww + 1) - dj];
-              dbias_s[hh * geo.nrel + di_idx * ndj + dj_idx] += acc;
-            }
-            __syncwarp();
-          }
-        }
-        // =============================== phase 2: per 16-key block: dV = P^T dO, dK = scale * dS^T Q
-        for (int kb = warp; kb < rblocks; kb += WA_WARPS) {
-          if (kb * 16 >= N) continue;
-          float dv[HD / 8][4], dk[HD / 8][4];
-#pragma unroll
-          for (int nb = 0; nb < HD / 8; ++nb)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dv[nb][k] = dk[nb][k] = 0.f;
-#pragma unroll
-          for (int j = 0; j < NPAD / 16; ++j) {   // query blocks (contraction)
-            uint32_t pa[4], sa[4];
-            const int prow = j * 16 + (lane & 7) + (lane >> 4) * 8;
-            const int pcol = kb * 16 + ((lane >> 3) & 1) * 8;
-            ldsm_x4_t(pa, Ps + prow * pstride + pcol);
-            ldsm_x4_t(sa, dSs + prow * pstride + pcol);
-#pragma unroll
-            for (int nb = 0; nb < HD / 8; nb += 2) {
-              uint32_t bf[4];
-              ldsm_x4_t(bf, dOs + (j * 16 + (lane & 15)) * stride + hh * HD + nb * 8 + (lane >> 4) * 8);
-              const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
-              mma_bf16_16816(dv[nb], pa, b0);
-              mma_bf16_16816(dv[nb + 1], pa, b1);
-              ldsm_x4_t(bf, Qs + (j * 16 + (lane & 15)) * stride + hh * HD + nb * 8 + (lane >> 4) * 8);
-              const uint32_t c0[2] = {bf[0], bf[1]}, c1[2] = {bf[2], bf[3]};
-              mma_bf16_16816(dk[nb], sa, c0);
-              mma_bf16_16816(dk[nb + 1], sa, c1);
-            }
-          }
-          // K and V columns of this head are dead after phase 1: reuse them as the staging of dK, dV
-          const int r0 = kb * 16 + gq, r1 = r0 + 8;
-          __syncwarp();
-#pragma unroll
-          for (int nb = 0; nb < HD / 8; ++nb) {
-            const int c = hh * HD + nb * 8 + tq * 2;
-            *reinterpret_cast<uint32_t*>(Ks + r0 * stride + c) = pack_bf16x2(dk[nb][0] * a.scale, dk[nb][1] * a.scale);
-            *reinterpret_cast<uint32_t*>(Ks + r1 * stride + c) = pack_bf16x2(dk[nb][2] * a.scale, dk[nb][3] * a.scale);
-            *reinterpret_cast<uint32_t*>(Vs + r0 * stride + c) = pack_bf16x2(dv[nb][0], dv[nb][1]);
-            *reinterpret_cast<uint32_t*>(Vs + r1 * stride + c) = pack_bf16x2(dv[nb][2], dv[nb][3]);
-          }
-        }
-        // the next head's phase 1 writes Ps/dSs again: wait for every reader
-        __syncthreads();
-      }
+    __syncthreads();            // this window's rows are visible; with two stages the previous one has been consumed
+    const WaItem mine = cur;
+    cur = next;
+    if (STAGES == 2 && item + step < items)
+      wa_gather<Cfg, BWD>(a, tabs + slot1 * NPAD, smem_u32(stages + (buf ^ 1) * Cfg::STAGE), ch0, tid, q0, q1);
+    if (item + 2 * step < items) {
+      next = wa_item(a, item + 2 * step, my_nw);
+      if (tid < N) wa_table(a, geo, next, ti, tj, tabs + slot2 * NPAD + tid);
     }
-    __syncthreads();
-    // ---- scatter results to the home rows (a warp per row; lanes over the row's vectors)
-    if (!BWD) {
-      for (int r = q0 + warp; r < q1; r += WA_WARPS) {
-        __nv_bfloat16* base = static_cast<__nv_bfloat16*>(a.out[rowslot[r]]) + rowofs[r] * a.C + cg * G;
-        if (lane < vpr) *reinterpret_cast<uint4*>(base + lane * 8) = *reinterpret_cast<const uint4*>(Qs + r * stride + lane * 8);
+    const bool general = N != NPAD || (a.use_mask && ((a.sh > 0 && mine.ii == a.nWh - 1) || (a.sw > 0 && mine.jj == a.nWw - 1)));
+
+    if constexpr (!BWD) {
+      if (row0 < q1 && row0 + 16 > q0) {
+#pragma unroll 1
+        for (int hh = 0; hh < HPC; ++hh) {
+          float s[NB][4];
+          wa_mma_nt<HD, NPAD, PITCH>(s, Qs + row0 * PITCH + hh * HD, Ks + hh * HD, lane);
+          float mx0 = -1e30f, mx1 = -1e30f, inv0, inv1;
+          wa_scores<NPAD, WW>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx0, mx1);
+          wa_softmax<NPAD>(s, mx0, mx1, inv0, inv1);
+          // O = P V with the numerators as P, the row normalisation applied to the (smaller) output; staged over this
+          // warp's own Q rows, which no other warp reads
+          float o[HD / 8][4];
+          wa_mma_pn<HD, NPAD, PITCH>(o, s, Vs + hh * HD, lane);
+          __syncwarp();
+          wa_stage<HD>(Qs + row0 * PITCH + hh * HD, PITCH, o, inv0, inv1, gq, tq, in0, in1);
+        }
+        __syncwarp();
+        wa_store<G>(a.out, a.C, ch0, Qs + row0 * PITCH, PITCH, tab, row0, lane, q0, q1);
       }
     } else {
-      // With sequence parallelism every rank of the window recomputes the whole window (cheap) and keeps only the
-      // gradients of its own token shard, so no cross-rank reduction of dK/dV is needed.
-      for (int r = q0 + warp; r < q1; r += WA_WARPS) {
-        __nv_bfloat16* base = static_cast<__nv_bfloat16*>(a.dqkv[rowslot[r]]) + rowofs[r] * (3LL * a.C) + cg * G;
+      // ---- phase 1, a warp per 16 query rows: P, dS, dQ
+      if (row0 < N) {
+        float s[NB][4], dp[NB][4];
+        wa_mma_nt<HD, NPAD, PITCH>(s, Qs + row0 * PITCH, Ks, lane);
+        float mx0 = -1e30f, mx1 = -1e30f, inv0, inv1;
+        wa_scores<NPAD, WW>(s, scale2, bias_s, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx0, mx1);
+        wa_softmax<NPAD>(s, mx0, mx1, inv0, inv1);
+        wa_mma_nt<HD, NPAD, PITCH>(dp, dOs + row0 * PITCH, Vs, lane);        // dP = dO V^T
+        float d0 = 0.f, d1 = 0.f;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const int m = gm[k];
-          if (gok[k] && m < 3)
-            *reinterpret_cast<uint4*>(base + m * a.C + gv[k] * 8) =
-                *reinterpret_cast<const uint4*>((m == 0 ? dQs : (m == 1 ? Ks : Vs)) + r * stride + gv[k] * 8);
+        for (int nb = 0; nb < NB; ++nb) {
+          s[nb][0] *= inv0;
+          s[nb][1] *= inv0;
+          s[nb][2] *= inv1;
+          s[nb][3] *= inv1;
+          d0 += s[nb][0] * dp[nb][0] + s[nb][1] * dp[nb][1];
+          d1 += s[nb][2] * dp[nb][2] + s[nb][3] * dp[nb][3];
+        }
+        d0 += __shfl_xor_sync(0xffffffffu, d0, 1);
+        d0 += __shfl_xor_sync(0xffffffffu, d0, 2);
+        d1 += __shfl_xor_sync(0xffffffffu, d1, 1);
+        d1 += __shfl_xor_sync(0xffffffffu, d1, 2);
+        // dS = P (dP - rowsum(P dP)); its sum over the windows is the gradient of the bias
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          dp[nb][0] = s[nb][0] * (dp[nb][0] - d0);
+          dp[nb][1] = s[nb][1] * (dp[nb][1] - d0);
+          dp[nb][2] = s[nb][2] * (dp[nb][2] - d1);
+          dp[nb][3] = s[nb][3] * (dp[nb][3] - d1);
+          if constexpr (Cfg::ACC_REGS) {
+            acc[nb][0] = fmaf(dp[nb][0], own0, acc[nb][0]);
+            acc[nb][1] = fmaf(dp[nb][1], own0, acc[nb][1]);
+            acc[nb][2] = fmaf(dp[nb][2], own1, acc[nb][2]);
+            acc[nb][3] = fmaf(dp[nb][3], own1, acc[nb][3]);
+          } else if (bias_grad) {
+            float4* t = reinterpret_cast<float4*>(acc_s) + nb * Cfg::THREADS + tid;
+            float4 v = *t;
+            v.x = fmaf(dp[nb][0], own0, v.x);
+            v.y = fmaf(dp[nb][1], own0, v.y);
+            v.z = fmaf(dp[nb][2], own1, v.z);
+            v.w = fmaf(dp[nb][3], own1, v.w);
+            *t = v;
+          }
+        }
+        {
+          float dq[HD / 8][4];
+          wa_mma_pn<HD, NPAD, PITCH>(dq, dp, Ks, lane);
+          // the stash rows of this block were last read before the barrier that opened this window
+          __nv_bfloat16* st = Cfg::DQ_IN_STASH ? Ps + row0 * PP : dQs + row0 * PITCH;
+          constexpr int stp = Cfg::DQ_IN_STASH ? PP : PITCH;
+          wa_stage<HD>(st, stp, dq, a.scale, a.scale, gq, tq, true, true);
+          __syncwarp();
+          wa_store<HD>(a.dqkv, 3LL * a.C, ch0, st, stp, tab, row0, lane, q0, q1);
+          __syncwarp();
+        }
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          const int col = nb * 8 + tq * 2;
+          *reinterpret_cast<uint32_t*>(Ps + r0 * PP + col) = pack_bf16x2(s[nb][0], s[nb][1]);
+          *reinterpret_cast<uint32_t*>(Ps + r1 * PP + col) = pack_bf16x2(s[nb][2], s[nb][3]);
+          *reinterpret_cast<uint32_t*>(dSs + r0 * PP + col) = pack_bf16x2(dp[nb][0], dp[nb][1]);
+          *reinterpret_cast<uint32_t*>(dSs + r1 * PP + col) = pack_bf16x2(dp[nb][2], dp[nb][3]);
         }
       }
+      __syncthreads();
+      // ---- phase 2, a warp per 16 keys: dV = P^T dO, dK = scale dS^T Q. K and V are dead: their rows stage the results.
+      // With sequence parallelism every rank of the window recomputes the whole window (cheap) and keeps only the
+      // gradients of its own token shard, so no cross-rank reduction of dK / dV is needed.
+      if (row0 < N) {
+        float dv[HD / 8][4], dk[HD / 8][4];
+#pragma unroll
+        for (int nb = 0; nb < HD / 8; ++nb)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) dv[nb][k] = dk[nb][k] = 0.f;
+        const int qblocks = (N + 15) >> 4;
+#pragma unroll
+        for (int j = 0; j < NPAD / 16; ++j) {   // query blocks (contraction); blocks without a token were not stashed
+          if (j >= qblocks) break;
+          uint32_t pa[4], sa[4];
+          const int prow = j * 16 + (lane & 7) + (lane >> 4) * 8;
+          const int pcol = row0 + ((lane >> 3) & 1) * 8;
+          ldsm_x4_t(pa, Ps + prow * PP + pcol);
+          ldsm_x4_t(sa, dSs + prow * PP + pcol);
+#pragma unroll
+          for (int nb = 0; nb < HD / 8; nb += 2) {
+            uint32_t bf[4];
+            ldsm_x4_t(bf, dOs + (j * 16 + (lane & 15)) * PITCH + nb * 8 + (lane >> 4) * 8);
+            const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
+            mma_bf16_16816(dv[nb], pa, b0);
+            mma_bf16_16816(dv[nb + 1], pa, b1);
+            ldsm_x4_t(bf, Qs + (j * 16 + (lane & 15)) * PITCH + nb * 8 + (lane >> 4) * 8);
+            const uint32_t c0[2] = {bf[0], bf[1]}, c1[2] = {bf[2], bf[3]};
+            mma_bf16_16816(dk[nb], sa, c0);
+            mma_bf16_16816(dk[nb + 1], sa, c1);
+          }
+        }
+        wa_stage<HD>(Ks + row0 * PITCH, PITCH, dk, a.scale, a.scale, gq, tq, in0, in1);
+        wa_stage<HD>(Vs + row0 * PITCH, PITCH, dv, 1.f, 1.f, gq, tq, in0, in1);
+        __syncwarp();
+        wa_store<HD>(a.dqkv, 3LL * a.C, a.C + ch0, Ks + row0 * PITCH, PITCH, tab, row0, lane, q0, q1);
+        wa_store<HD>(a.dqkv, 3LL * a.C, 2 * a.C + ch0, Vs + row0 * PITCH, PITCH, tab, row0, lane, q0, q1);
+      }
     }
+    slot = slot1;
+    if (STAGES == 2) buf ^= 1;
   }
+
   if (bias_grad) {
+    // Spread the sums out as an [N][NPAD + 1] matrix over the operand stages, then fold its diagonals into the table: entry
+    // (di, dj) collects the pairs with query - key = (di, dj).
+    float* D = reinterpret_cast<float*>(smem);
+    static_assert(!BWD || static_cast<size_t>(NPAD) * (NPAD + 1) * 4 <= static_cast<size_t>(STAGES * Cfg::STAGE + Cfg::STASH) * 2,
+                  "scratch of the bias-gradient fold");
     __syncthreads();
-    for (int i = tid; i < hpc * geo.nrel; i += WA_THREADS) {
-      const int h = i / geo.nrel, r = i % geo.nrel;
-      atomicAdd(&a.dbias_table[r * a.num_heads + head0 + h], dbias_s[i]);
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      float4 v;
+      if constexpr (BWD && Cfg::ACC_REGS) v = make_float4(acc[nb][0], acc[nb][1], acc[nb][2], acc[nb][3]);
+      else v = reinterpret_cast<const float4*>(acc_s)[nb * Cfg::THREADS + tid];
+      const int col = nb * 8 + tq * 2;
+      D[r0 * (NPAD + 1) + col] = v.x;
+      D[r0 * (NPAD + 1) + col + 1] = v.y;
+      D[r1 * (NPAD + 1) + col] = v.z;
+      D[r1 * (NPAD + 1) + col + 1] = v.w;
+    }
+    __syncthreads();
+    const int ndj = 2 * a.ww - 1;
+    for (int i = tid; i < geo.nrel; i += Cfg::THREADS) {
+      const int di = i / ndj - (a.wh - 1), dj = i % ndj - (a.ww - 1);
+      float t = 0.f;
+      for (int y = max(0, di); y < min(a.wh, a.wh + di); ++y)
+        for (int x = max(0, dj); x < min(a.ww, a.ww + dj); ++x)
+          t += D[(y * a.ww + x) * (NPAD + 1) + (y - di) * a.ww + x - dj];
+      atomicAdd(&a.dbias_table[i * a.num_heads + head0], t);
     }
   }
 }
 
-template <int HD, int NPAD, bool BWD>
-size_t smem_bytes(int hpc, int nrel, int ww) {
-  const int G = hpc * HD, stride = G + 8, pstride = NPAD + 8;
-  size_t b = static_cast<size_t>(NPAD) * stride * 2 * (BWD ? 5 : 3);
-  if (BWD) b += static_cast<size_t>(NPAD) * pstride * 2 * 2;
-  b += static_cast<size_t>(hpc) * nrel * 4 * (BWD ? 2 : 1);
-  b += 16;   // alignment slack before the row tables
-  b += NPAD * (8 + 4 + 4 + 4);
-  if (BWD) b += static_cast<size_t>(ww) * ww * 4 * (1 + WA_WARPS);
-  return b;
-}
-
-template <int HD, int NPAD, bool BWD>
+template <int HD, int NPAD, int HPC, int WW, bool BWD>
 int launch(WindowAttnArgs a, cudaStream_t stream) {
+  using Cfg = WaCfg<HD, NPAD, HPC, BWD>;
   const int nrel = (2 * a.wh - 1) * (2 * a.ww - 1);
-  // heads per CTA: 64 channels (128-byte row segments) keep the CTA small enough for several per SM
-  int hpc = 64 / HD;
-  if (hpc < 1) hpc = 1;
-  while (hpc > 1 && (a.num_heads % hpc != 0 || smem_bytes<HD, NPAD, BWD>(hpc, nrel, a.ww) > 200 * 1024)) --hpc;
-  const size_t sb = smem_bytes<HD, NPAD, BWD>(hpc, nrel, a.ww);
+  const size_t sb = Cfg::bytes(nrel);
   if (sb > 227 * 1024) return -20;
-  a.heads_per_cta = hpc;
-  static size_t configured = 0;
-  static int occupancy = 0;
-  if (sb > configured) {
-    if (cudaFuncSetAttribute(window_attn_kernel<HD, NPAD, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(sb)) != cudaSuccess)
-      return -21;
-    configured = sb;
-    occupancy = 0;
+  auto kernel = window_attn_kernel<HD, NPAD, HPC, WW, BWD>;
+  // resident CTAs per SM for the last shared-memory size seen (one word, so that threads read a matching pair)
+  static std::atomic<unsigned long long> known{0};
+  unsigned long long k = known.load(std::memory_order_relaxed);
+  if ((k >> 8) != sb) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return -21;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, Cfg::THREADS, sb) != cudaSuccess || occ < 1) occ = 1;
+    k = (static_cast<unsigned long long>(sb) << 8) | static_cast<unsigned long long>(occ);
+    known.store(k, std::memory_order_relaxed);
   }
-  if (occupancy == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy, window_attn_kernel<HD, NPAD, BWD>, WA_THREADS, sb) !=
-            cudaSuccess || occupancy < 1)
-      occupancy = 1;
-  }
+  const int occupancy = static_cast<int>(k & 255);
   const int my_nw = a.win_start[a.my_wg + 1] - a.win_start[a.my_wg];
   const int items = a.B * my_nw;
   if (items <= 0) return 0;
-  const int groups = a.num_heads / hpc;
+  a.heads_per_cta = HPC;
+  const int groups = a.num_heads / HPC;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int gx = (sms * occupancy + groups - 1) / groups;
+  int gx = sms * occupancy / groups;             // one resident wave: a CTA of a second wave would repeat the set-up
+  if (gx < 1) gx = 1;
   if (gx > items) gx = items;
-  dim3 grid(gx, groups);
-  window_attn_kernel<HD, NPAD, BWD><<<grid, WA_THREADS, sb, stream>>>(a);
+  kernel<<<dim3(gx, groups), Cfg::THREADS, sb, stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -22;
+}
+
+template <int HD, int NPAD, bool BWD>
+int launch_hd(const WindowAttnArgs& a, cudaStream_t stream) {
+  // Forward: 64 channels per CTA (128-byte row segments) where the head count allows it, so that a window's set-up is
+  // shared by several heads. Backward: one head, whose bias-gradient sums stay in registers.
+  constexpr int HPC = (BWD || HD >= 64) ? 1 : 2;
+  const bool grouped = HPC > 1 && a.num_heads % HPC == 0;
+#define TB_WA_WIDTH(WW_)                                                                       \
+  return grouped ? launch<HD, NPAD, HPC, WW_, BWD>(a, stream) : launch<HD, NPAD, 1, WW_, BWD>(a, stream)
+  // (the specialised widths serve windows without padding tokens; 96 = 8 x 12 or 12 x 8)
+  if constexpr (NPAD != 96) { if (a.ww == 8) { TB_WA_WIDTH(8); } }
+  if constexpr (NPAD == 96) { if (a.ww == 12) { TB_WA_WIDTH(12); } }
+  TB_WA_WIDTH(0);
+#undef TB_WA_WIDTH
 }
 
 template <bool BWD>
@@ -548,7 +635,7 @@ int dispatch(const WindowAttnArgs& a, cudaStream_t stream) {
   if (a.sp < 1 || a.shardN < 1 || a.n_wg < 1 || a.n_wg > 8 || a.n_wg * a.sp > WA_MAX_PEERS) return -12;
   const int npad = N <= 64 ? 64 : (N <= 96 ? 96 : 128);
 #define TB_WA_CASE(HD_, NP_) \
-  if (hd == HD_ && npad == NP_) return launch<HD_, NP_, BWD>(a, stream);
+  if (hd == HD_ && npad == NP_) return launch_hd<HD_, NP_, BWD>(a, stream);
   TB_WA_CASE(16, 64) TB_WA_CASE(32, 64) TB_WA_CASE(64, 64) TB_WA_CASE(128, 64)
   TB_WA_CASE(16, 96) TB_WA_CASE(32, 96) TB_WA_CASE(64, 96) TB_WA_CASE(128, 96)
   TB_WA_CASE(16, 128) TB_WA_CASE(32, 128) TB_WA_CASE(64, 128) TB_WA_CASE(128, 128)

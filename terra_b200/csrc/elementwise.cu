@@ -260,8 +260,15 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 }
 
 // ------------------------------------------------------------------------------------------ GroupNorm
-// x: [B, HW, C] bf16. Block = (C/8 column vectors) x (rows in flight); per-channel partials in shared memory,
-// folded to groups, two atomics per (block, group).
+// x: [B, HW, C] bf16. Every kernel is one pass over the image, bound by HBM: a block is (column vectors) x (pixels in
+// flight), so a thread's column constants (statistics, affine parameters) are loaded once for all of its pixels, and it
+// keeps several independent 16-byte loads in flight. blockIdx.y is the sample; the pixel range of a sample is split over
+// blockIdx.x so that the grid is about one resident wave. (Before, the apply kernels divided to find every vector's channel
+// and loaded its constants again, and one load per thread was in flight. 557056 pixels x 384, before -> now: statistics
+// 98 -> 96 us, apply with shortcut 355 -> 225, backward sums 366 -> 258, backward apply 406 -> 264; one copy of the image
+// each way at 6.65 TB/s is 129 us.)
+//
+// Statistics: per-channel partials in shared memory, folded to groups, two atomics per (block, group).
 __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat16* __restrict__ x,
                                                               float* __restrict__ sums, long long HW, int C, int groups,
                                                               int pix_per_block) {
@@ -274,13 +281,23 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
   const long long p1 = min(HW, p0 + pix_per_block);
   for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (long long p = p0 + threadIdx.y; p < p1; p += blockDim.y) {
-      float f[8];
-      unpack8(*reinterpret_cast<const uint4*>(x + (static_cast<long long>(b) * HW + p) * C + vi * 8), f);
+    const uint4* src = reinterpret_cast<const uint4*>(x) + static_cast<long long>(b) * HW * nvec + vi;
+    for (long long p = p0 + threadIdx.y; p < p1; p += 4 * blockDim.y) {
+      uint4 t[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        s[j] += f[j];
-        q[j] += f[j] * f[j];
+      for (int u = 0; u < 4; ++u) {
+        t[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (p + u * blockDim.y < p1) t[u] = src[(p + u * blockDim.y) * nvec];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float f[8];
+        unpack8(t[u], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s[j] += f[j];
+          q[j] += f[j] * f[j];
+        }
       }
     }
 #pragma unroll
@@ -304,78 +321,127 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + __expf(-z)); }
 
-__global__ void __launch_bounds__(256) groupnorm_silu_apply_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                   const float* __restrict__ stats,
-                                                                   const __nv_bfloat16* __restrict__ gamma,
-                                                                   const __nv_bfloat16* __restrict__ beta,
-                                                                   const __nv_bfloat16* __restrict__ res,
-                                                                   __nv_bfloat16* __restrict__ y, long long HW, int C,
-                                                                   int groups, long long total_vec) {
+// A thread's eight channels: statistics of their groups and affine parameters.
+struct GnChannels {
+  float mu[8], rs[8], g[8], bt[8];
+};
+__device__ __forceinline__ void gn_channels(GnChannels& c, const float* __restrict__ stats, const __nv_bfloat16* __restrict__ gamma,
+                                            const __nv_bfloat16* __restrict__ beta, int b, int vi, int cpg, int groups) {
+  unpack8(reinterpret_cast<const uint4*>(gamma)[vi], c.g);
+  unpack8(reinterpret_cast<const uint4*>(beta)[vi], c.bt);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int grp = (vi * 8 + j) / cpg;
+    c.mu[j] = stats[(b * groups + grp) * 2];
+    c.rs[j] = stats[(b * groups + grp) * 2 + 1];
+  }
+}
+
+__global__ void __launch_bounds__(256, 3) groupnorm_silu_apply_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                      const float* __restrict__ stats,
+                                                                      const __nv_bfloat16* __restrict__ gamma,
+                                                                      const __nv_bfloat16* __restrict__ beta,
+                                                                      const __nv_bfloat16* __restrict__ res,
+                                                                      __nv_bfloat16* __restrict__ y, long long HW, int C,
+                                                                      int groups, int pix_per_block) {
   const int nvec = C >> 3;
-  const int cpg = C / groups;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total_vec;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int vi = static_cast<int>(i % nvec);
-    const long long pix = i / nvec;
-    const int b = static_cast<int>(pix / HW);
-    float f[8], g[8], bt[8], o[8];
-    unpack8(reinterpret_cast<const uint4*>(x)[i], f);
-    unpack8(reinterpret_cast<const uint4*>(gamma)[vi], g);
-    unpack8(reinterpret_cast<const uint4*>(beta)[vi], bt);
+  const int b = blockIdx.y;
+  const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
+  const long long p1 = min(HW, p0 + pix_per_block);
+  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
+    GnChannels c;
+    gn_channels(c, stats, gamma, beta, b, vi, C / groups, groups);
+    const long long first = static_cast<long long>(b) * HW * nvec + vi;
+    const uint4* src = reinterpret_cast<const uint4*>(x) + first;
+    const uint4* add = reinterpret_cast<const uint4*>(res) + first;
+    uint4* dst = reinterpret_cast<uint4*>(y) + first;
+    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
+      uint4 t[2], r[2];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int grp = (vi * 8 + j) / cpg;
-      const float mu = stats[(b * groups + grp) * 2], rs = stats[(b * groups + grp) * 2 + 1];
-      const float z = (f[j] - mu) * rs * g[j] + bt[j];
-      o[j] = z * sigmoidf_(z);
-    }
-    if (res != nullptr) {
-      float rr[8];
-      unpack8(reinterpret_cast<const uint4*>(res)[i], rr);
+      for (int u = 0; u < 2; ++u) {
+        if (p + u * blockDim.y < p1) {
+          t[u] = src[(p + u * blockDim.y) * nvec];
+          if (res != nullptr) r[u] = add[(p + u * blockDim.y) * nvec];
+        }
+      }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] += rr[j];
+      for (int u = 0; u < 2; ++u) {
+        if (p + u * blockDim.y >= p1) break;
+        float f[8], o[8];
+        unpack8(t[u], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float z = (f[j] - c.mu[j]) * c.rs[j] * c.g[j] + c.bt[j];
+          o[j] = z * sigmoidf_(z);
+        }
+        if (res != nullptr) {
+          float rr[8];
+          unpack8(r[u], rr);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += rr[j];
+        }
+        dst[(p + u * blockDim.y) * nvec] = pack8(o);
+      }
     }
-    reinterpret_cast<uint4*>(y)[i] = pack8(o);
   }
 }
 
 // pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}
-__global__ void __launch_bounds__(512) groupnorm_silu_bwd_reduce_kernel(
+__global__ void __launch_bounds__(256, 3) groupnorm_silu_bwd_reduce_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta, float* __restrict__ red,
     long long HW, int C, int groups, int pix_per_block, float* __restrict__ dgamma, float* __restrict__ dbeta) {
   extern __shared__ float sh[];  // [2][C]
   const int nvec = C >> 3;
-  const int cpg = C / groups;
   const int b = blockIdx.y;
   for (int c = threadIdx.y * blockDim.x + threadIdx.x; c < 2 * C; c += blockDim.x * blockDim.y) sh[c] = 0.f;
   __syncthreads();
   const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
   const long long p1 = min(HW, p0 + pix_per_block);
   for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
-    float g[8], bt[8], mu[8], rs[8];
-    unpack8(reinterpret_cast<const uint4*>(gamma)[vi], g);
-    unpack8(reinterpret_cast<const uint4*>(beta)[vi], bt);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int grp = (vi * 8 + j) / cpg;
-      mu[j] = stats[(b * groups + grp) * 2];
-      rs[j] = stats[(b * groups + grp) * 2 + 1];
-    }
-    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (long long p = p0 + threadIdx.y; p < p1; p += blockDim.y) {
-      const long long off = (static_cast<long long>(b) * HW + p) * C + vi * 8;
-      float f[8], d[8];
-      unpack8(*reinterpret_cast<const uint4*>(x + off), f);
-      unpack8(*reinterpret_cast<const uint4*>(dy + off), d);
+    // (the affine parameters stay packed: 16 registers less)
+    float rs[8], mu[8];
+    const uint4 gq = reinterpret_cast<const uint4*>(gamma)[vi], bq = reinterpret_cast<const uint4*>(beta)[vi];
+    {
+      GnChannels c;
+      gn_channels(c, stats, gamma, beta, b, vi, C / groups, groups);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float xh = (f[j] - mu[j]) * rs[j];
-        const float z = xh * g[j] + bt[j];
-        const float sg = sigmoidf_(z);
-        const float dz = d[j] * sg * (1.f + z * (1.f - sg));
-        s[j] += dz;
-        q[j] += dz * xh;
+        rs[j] = c.rs[j];
+        mu[j] = c.mu[j];
+      }
+    }
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const long long first = static_cast<long long>(b) * HW * nvec + vi;
+    const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
+    const uint4* ds = reinterpret_cast<const uint4*>(dy) + first;
+    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
+      uint4 t[2], d2[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        t[u] = d2[u] = make_uint4(0u, 0u, 0u, 0u);     // dz = 0 behind the range
+        if (p + u * blockDim.y < p1) {
+          t[u] = xs[(p + u * blockDim.y) * nvec];
+          d2[u] = ds[(p + u * blockDim.y) * nvec];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float f[8], d[8], g[8], bt[8];
+        unpack8(t[u], f);
+        unpack8(d2[u], d);
+        unpack8(gq, g);
+        unpack8(bq, bt);
+        if (p + u * blockDim.y >= p1) break;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = (f[j] - mu[j]) * rs[j];
+          const float z = xh * g[j] + bt[j];
+          const float sg = sigmoidf_(z);
+          const float dz = d[j] * sg * (1.f + z * (1.f - sg));
+          s[j] += dz;
+          q[j] += dz * xh;
+        }
       }
     }
 #pragma unroll
@@ -428,46 +494,66 @@ __global__ void __launch_bounds__(256) strided_add_kernel(float* __restrict__ sr
 }
 
 // pass 2: dx = rstd * (dz*gamma - s1/n - xhat * s2/n), s1 = sum_c gamma_c red[b][c][0], s2 likewise with [1]
-__global__ void __launch_bounds__(256) groupnorm_silu_bwd_apply_kernel(
+__global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const float* __restrict__ red, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
-    __nv_bfloat16* __restrict__ dx, int B, long long HW, int C, int groups, float inv_count, long long total_vec) {
-  extern __shared__ float gs[];  // [B][groups][2]
-  const int cpg = C / groups;
-  for (int i = threadIdx.x; i < B * groups; i += blockDim.x) {
-    const int b = i / groups, g = i % groups;
+    __nv_bfloat16* __restrict__ dx, long long HW, int C, int groups, float inv_count, int pix_per_block) {
+  extern __shared__ float gs[];  // [groups][2] of this block's sample
+  const int cpg = C / groups, nvec = C >> 3;
+  const int b = blockIdx.y;
+  for (int g = threadIdx.y * blockDim.x + threadIdx.x; g < groups; g += blockDim.x * blockDim.y) {
     float s1 = 0.f, s2 = 0.f;
     for (int c = g * cpg; c < (g + 1) * cpg; ++c) {
       const float gm = __bfloat162float(gamma[c]);
-      s1 += gm * red[(static_cast<long long>(b) * C + c) * 2];
-      s2 += gm * red[(static_cast<long long>(b) * C + c) * 2 + 1];
+      const float2 r = reinterpret_cast<const float2*>(red)[static_cast<long long>(b) * C + c];
+      s1 += gm * r.x;
+      s2 += gm * r.y;
     }
-    gs[i * 2] = s1 * inv_count;
-    gs[i * 2 + 1] = s2 * inv_count;
+    gs[g * 2] = s1 * inv_count;
+    gs[g * 2 + 1] = s2 * inv_count;
   }
   __syncthreads();
-  const int nvec = C >> 3;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total_vec;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int vi = static_cast<int>(i % nvec);
-    const long long pix = i / nvec;
-    const int b = static_cast<int>(pix / HW);
-    float f[8], d[8], g[8], bt[8], o[8];
-    unpack8(reinterpret_cast<const uint4*>(x)[i], f);
-    unpack8(reinterpret_cast<const uint4*>(dy)[i], d);
-    unpack8(reinterpret_cast<const uint4*>(gamma)[vi], g);
-    unpack8(reinterpret_cast<const uint4*>(beta)[vi], bt);
+  const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
+  const long long p1 = min(HW, p0 + pix_per_block);
+  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
+    GnChannels c;
+    gn_channels(c, stats, gamma, beta, b, vi, cpg, groups);
+    float m1[8], m2[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int grp = (vi * 8 + j) / cpg;
-      const float mu = stats[(b * groups + grp) * 2], rs = stats[(b * groups + grp) * 2 + 1];
-      const float xh = (f[j] - mu) * rs;
-      const float z = xh * g[j] + bt[j];
-      const float sg = sigmoidf_(z);
-      const float dz = d[j] * sg * (1.f + z * (1.f - sg));
-      o[j] = rs * (dz * g[j] - gs[(b * groups + grp) * 2] - xh * gs[(b * groups + grp) * 2 + 1]);
+      m1[j] = gs[(vi * 8 + j) / cpg * 2];
+      m2[j] = gs[(vi * 8 + j) / cpg * 2 + 1];
     }
-    reinterpret_cast<uint4*>(dx)[i] = pack8(o);
+    const long long first = static_cast<long long>(b) * HW * nvec + vi;
+    const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
+    const uint4* ds = reinterpret_cast<const uint4*>(dy) + first;
+    uint4* dst = reinterpret_cast<uint4*>(dx) + first;
+    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
+      uint4 t[2], d2[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (p + u * blockDim.y < p1) {
+          t[u] = xs[(p + u * blockDim.y) * nvec];
+          d2[u] = ds[(p + u * blockDim.y) * nvec];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (p + u * blockDim.y >= p1) break;
+        float f[8], d[8], o[8];
+        unpack8(t[u], f);
+        unpack8(d2[u], d);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = (f[j] - c.mu[j]) * c.rs[j];
+          const float z = xh * c.g[j] + c.bt[j];
+          const float sg = sigmoidf_(z);
+          const float dz = d[j] * sg * (1.f + z * (1.f - sg));
+          o[j] = c.rs[j] * (dz * c.g[j] - m1[j] - xh * m2[j]);
+        }
+        dst[(p + u * blockDim.y) * nvec] = pack8(o);
+      }
+    }
   }
 }
 
@@ -758,26 +844,42 @@ int colsum_bf16(const void* x, float* out, float* partials, long long rows, int 
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+// Launch shape of the GroupNorm kernels: `threads` per block as (column vectors) x (pixels), pixels split over about
+// `waves` blocks per SM in all (at least two loop rounds of `unroll` pixels per thread, so that tiny images do not pay for
+// more blocks than they fill).
+struct GnShape {
+  dim3 block, grid;
+  int pix;
+  GnShape(int B, long long HW, int C, int threads, int waves, int unroll) {
+    const int nvec = C / 8;
+    const int bx = nvec < 64 ? nvec : 64;
+    const int by = threads / bx > 0 ? threads / bx : 1;
+    block = dim3(bx, by);
+    const long long blocks = (148LL * waves + B - 1) / B;
+    const long long least = static_cast<long long>(by) * unroll;
+    long long p = (HW + blocks - 1) / blocks;
+    p = (p + least - 1) / least * least;
+    pix = static_cast<int>(p);
+    grid = dim3(static_cast<unsigned>((HW + p - 1) / p), B);
+  }
+};
+
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {
   if (C % 8 != 0 || C % groups != 0) return -1;
-  const int nvec = C / 8;
-  const int bx = nvec < 64 ? nvec : 64;
-  dim3 block(bx, 512 / bx > 0 ? 512 / bx : 1);
-  const int pix_per_block = 1024;
-  dim3 grid(static_cast<unsigned>((HW + pix_per_block - 1) / pix_per_block), B);
-  groupnorm_stats_kernel<<<grid, block, 2 * C * sizeof(float), stream>>>(static_cast<const __nv_bfloat16*>(x), sums, HW,
-                                                                         C, groups, pix_per_block);
+  const GnShape s(B, HW, C, 512, 3, 4);
+  groupnorm_stats_kernel<<<s.grid, s.block, 2 * C * sizeof(float), stream>>>(static_cast<const __nv_bfloat16*>(x), sums, HW,
+                                                                             C, groups, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, const void* beta, const void* res, void* y,
                          int B, long long HW, int C, int groups, cudaStream_t stream) {
   if (C % 8 != 0 || C % groups != 0) return -1;
-  const long long total_vec = static_cast<long long>(B) * HW * (C / 8);
-  groupnorm_silu_apply_kernel<<<grid_for(total_vec, 256), 256, 0, stream>>>(
+  const GnShape s(B, HW, C, 256, 6, 2);
+  groupnorm_silu_apply_kernel<<<s.grid, s.block, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
       static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(y), HW,
-      C, groups, total_vec);
+      C, groups, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -785,15 +887,11 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
                               float* red, float* dgamma, float* dbeta, int B, long long HW, int C, int groups,
                               cudaStream_t stream) {
   if (C % 8 != 0 || C % groups != 0) return -1;
-  const int nvec = C / 8;
-  const int bx = nvec < 64 ? nvec : 64;
-  dim3 block(bx, 512 / bx > 0 ? 512 / bx : 1);
-  const int pix_per_block = 1024;
-  dim3 grid(static_cast<unsigned>((HW + pix_per_block - 1) / pix_per_block), B);
-  groupnorm_silu_bwd_reduce_kernel<<<grid, block, 2 * C * sizeof(float), stream>>>(
+  const GnShape s(B, HW, C, 256, 3, 2);
+  groupnorm_silu_bwd_reduce_kernel<<<s.grid, s.block, 2 * C * sizeof(float), stream>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
       static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups,
-      pix_per_block, dgamma, dbeta);
+      s.pix, dgamma, dbeta);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -815,11 +913,11 @@ int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, 
                              const void* beta, void* dx, int B, long long HW, int C, int groups, float inv_count,
                              cudaStream_t stream) {
   if (C % 8 != 0 || C % groups != 0) return -1;
-  const long long total_vec = static_cast<long long>(B) * HW * (C / 8);
-  groupnorm_silu_bwd_apply_kernel<<<grid_for(total_vec, 256), 256, B * groups * 2 * sizeof(float), stream>>>(
+  const GnShape s(B, HW, C, 256, 4, 2);
+  groupnorm_silu_bwd_apply_kernel<<<s.grid, s.block, groups * 2 * sizeof(float), stream>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red,
       static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
-      static_cast<__nv_bfloat16*>(dx), B, HW, C, groups, inv_count, total_vec);
+      static_cast<__nv_bfloat16*>(dx), HW, C, groups, inv_count, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -169,6 +169,36 @@ void attn_rowdot(const torch::Tensor& o, const torch::Tensor& dout, torch::Tenso
            "attn_rowdot");
 }
 
+void check_patches(const torch::Tensor& image, const torch::Tensor& patches, int64_t p) {
+  need(image.is_cuda() && image.is_contiguous() && image.dim() == 4 && image.scalar_type() == torch::kBFloat16, "image: [B,H,W,C] bf16");
+  need(patches.is_contiguous() && patches.dim() == 4 && patches.scalar_type() == torch::kBFloat16 && p >= 1 &&
+           patches.size(0) == image.size(0) && patches.size(3) == p * p * image.size(3),
+       "patches: [B,h,w,p*p*C] bf16");
+}
+
+// patches <- the padded image (zeros outside)
+void pad_patchify(const torch::Tensor& image, torch::Tensor& patches, int64_t p, int64_t top, int64_t left) {
+  check_patches(image, patches, p);
+  const c10::cuda::CUDAGuard guard(image.device());
+  tb::note_launch();
+  rc_check(tb::patch_relayout(image.data_ptr(), nullptr, patches.data_ptr(), nullptr, 1, image.size(0), image.size(1), image.size(2),
+                              image.size(3), p, patches.size(1) * p, patches.size(2) * p, top, left, cur_stream()),
+           "pad_patchify");
+}
+
+// out <- the image inside the patches (+ add)
+void unpatchify_crop(const torch::Tensor& patches, const c10::optional<torch::Tensor>& add, torch::Tensor& out, int64_t p,
+                     int64_t top, int64_t left) {
+  check_patches(out, patches, p);
+  need(!add.has_value() || (add->is_contiguous() && add->scalar_type() == torch::kBFloat16 && add->sizes() == out.sizes()),
+       "unpatchify_crop: add must look like out");
+  const c10::cuda::CUDAGuard guard(out.device());
+  tb::note_launch();
+  rc_check(tb::patch_relayout(nullptr, opt_ptr(add), const_cast<void*>(patches.data_ptr()), out.data_ptr(), 0, out.size(0), out.size(1),
+                              out.size(2), out.size(3), p, patches.size(1) * p, patches.size(2) * p, top, left, cur_stream()),
+           "unpatchify_crop");
+}
+
 void grad_inspect(const torch::Tensor& grad, torch::Tensor& out2) {
   need(grad.is_cuda() && grad.is_contiguous() && grad.scalar_type() == torch::kFloat32, "grad_inspect: fp32 contiguous");
   need(out2.scalar_type() == torch::kFloat32 && out2.numel() >= 2, "grad_inspect: out2 fp32 [2]");
@@ -349,6 +379,8 @@ void bind_elementwise(pybind11::module_& m) {
   m.def("groupnorm_silu_bwd_apply", &groupnorm_silu_bwd_apply);
   m.def("masked_loss", &masked_loss);
   m.def("adamw_step", &adamw_step);
+  m.def("pad_patchify", &pad_patchify);
+  m.def("unpatchify_crop", &unpatchify_crop);
   m.def("grad_inspect", &grad_inspect);
   m.def("attn_rowdot", &attn_rowdot);
   m.def("sum_slots", &sum_slots, pybind11::arg("slots"), pybind11::arg("out"), pybind11::arg("bias") = pybind11::none(),

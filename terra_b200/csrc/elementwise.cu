@@ -789,6 +789,72 @@ __global__ void conv_s2_col2im_kernel(const uint4* __restrict__ dcol, void* __re
   }
 }
 
+// Image [B, H, W, C] <-> patches [B, Hp / p, Wp / p, (p1, p2, c)] of the image padded to Hp x Wp (`top` rows above, `left`
+// columns left). A patch row (p2, c) is p * C contiguous elements on both sides, so the rearrangement is one pass of
+// contiguous copies, bound by HBM; V (16, 8, 4 or 2 bytes) divides the byte length of a patch row, of an image row and of
+// the left padding, so that no vector crosses the edge of the image. `row_units` = vectors of a padded row,
+// `seg_units` = vectors of a patch row. Thread block: one padded row (blockIdx.y) and PATCH_UNROLL vectors per thread.
+constexpr int PATCH_UNROLL = 4;
+template <class V>
+__global__ void __launch_bounds__(256) pad_patchify_kernel(const V* __restrict__ x, V* __restrict__ patches, int H, int p, int hn,
+                                                           int top, int left_units, int img_units, int row_units, int seg_units) {
+  const int yy = blockIdx.y % (hn * p), b = blockIdx.y / (hn * p);
+  const int y = yy - top;
+  const V* src = x + (static_cast<long long>(b) * H + y) * img_units - left_units;
+  V* dst = patches + (static_cast<long long>(b) * hn + yy / p) * p * row_units + static_cast<long long>(yy % p) * seg_units;
+  V t[PATCH_UNROLL];
+#pragma unroll
+  for (int u = 0; u < PATCH_UNROLL; ++u) {
+    const int e = (blockIdx.x * PATCH_UNROLL + u) * blockDim.x + threadIdx.x;
+    t[u] = V{};
+    if (e < row_units && y >= 0 && y < H && e >= left_units && e < left_units + img_units) t[u] = src[e];
+  }
+#pragma unroll
+  for (int u = 0; u < PATCH_UNROLL; ++u) {
+    const int e = (blockIdx.x * PATCH_UNROLL + u) * blockDim.x + threadIdx.x;
+    if (e < row_units) dst[static_cast<long long>(e / seg_units) * p * seg_units + e % seg_units] = t[u];
+  }
+}
+
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+  const float2 x = unpack_bf16x2(a), y = unpack_bf16x2(b);
+  return pack_bf16x2(x.x + y.x, x.y + y.y);
+}
+__device__ __forceinline__ uint4 add_bf16v(uint4 a, uint4 b) {
+  return make_uint4(add_bf16x2(a.x, b.x), add_bf16x2(a.y, b.y), add_bf16x2(a.z, b.z), add_bf16x2(a.w, b.w));
+}
+__device__ __forceinline__ uint2 add_bf16v(uint2 a, uint2 b) { return make_uint2(add_bf16x2(a.x, b.x), add_bf16x2(a.y, b.y)); }
+__device__ __forceinline__ uint32_t add_bf16v(uint32_t a, uint32_t b) { return add_bf16x2(a, b); }
+__device__ __forceinline__ unsigned short add_bf16v(unsigned short a, unsigned short b) {
+  return static_cast<unsigned short>(add_bf16x2(a, b) & 0xffffu);
+}
+
+// The inverse, cropped to the image, with `add` (an image, or null) added in fp32 before the rounding.
+template <class V>
+__global__ void __launch_bounds__(256) unpatchify_crop_kernel(const V* __restrict__ patches, const V* __restrict__ add,
+                                                              V* __restrict__ out, int H, int p, int hn, int top, int left_units,
+                                                              int img_units, int row_units, int seg_units) {
+  const int y = blockIdx.y % H, b = blockIdx.y / H;
+  const int yy = y + top;
+  const V* src = patches + (static_cast<long long>(b) * hn + yy / p) * p * row_units + static_cast<long long>(yy % p) * seg_units;
+  const long long row = (static_cast<long long>(b) * H + y) * img_units;
+  V t[PATCH_UNROLL], r[PATCH_UNROLL];
+#pragma unroll
+  for (int u = 0; u < PATCH_UNROLL; ++u) {
+    const int e = (blockIdx.x * PATCH_UNROLL + u) * blockDim.x + threadIdx.x;
+    if (e < img_units) {
+      const int k = e + left_units;
+      t[u] = src[static_cast<long long>(k / seg_units) * p * seg_units + k % seg_units];
+      if (add != nullptr) r[u] = add[row + e];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < PATCH_UNROLL; ++u) {
+    const int e = (blockIdx.x * PATCH_UNROLL + u) * blockDim.x + threadIdx.x;
+    if (e < img_units) out[row + e] = add != nullptr ? add_bf16v(t[u], r[u]) : t[u];
+  }
+}
+
 // out = sum over `slots` consecutive bf16 buffers of `nvec` 16-byte vectors each (fp32 accumulation), optionally
 // + bias[col] (bf16, `cvec` vectors per row) + residual (bf16, same shape as out): the owner's side of the slot-staged
 // reduce-scatter with the row-parallel layer's bias and the block's shortcut folded in.
@@ -1017,6 +1083,36 @@ int conv_s2_col2im(const void* dcol, void* out, int B, int Ho, int Wo, int W, in
   else
     conv_s2_col2im_kernel<false><<<grid_for(total, 256), 256, 0, stream>>>(static_cast<const uint4*>(dcol), out, B, Ho, Wo, W,
                                                                            C / 8, r0, rows);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+int patch_relayout(const void* image, const void* add, void* patches, void* image_out, int to_patches, int B, int H, int W, int C,
+                   int p, int Hp, int Wp, int top, int left, cudaStream_t stream) {
+  if (p < 1 || Hp % p != 0 || Wp % p != 0 || top < 0 || left < 0 || top + H > Hp || left + W > Wp || B < 1 || H < 1 || W < 1) return -1;
+  const int hn = Hp / p;
+  const long long rows = static_cast<long long>(B) * (to_patches ? Hp : H);
+  if (rows > 65535 || static_cast<long long>(Wp) * C > (1LL << 30)) return -1;
+  unsigned long long bytes = (static_cast<unsigned long long>(p) * C * 2) | (static_cast<unsigned long long>(W) * C * 2) |
+                             (static_cast<unsigned long long>(left) * C * 2) | 16ull;
+  for (const void* q : {image, add, static_cast<const void*>(patches), static_cast<const void*>(image_out)})
+    bytes |= reinterpret_cast<unsigned long long>(q);
+  const auto launch = [&](auto unit) {
+    using V = decltype(unit);
+    const int per = static_cast<int>(sizeof(V) / 2);
+    const int row_units = Wp * C / per, img_units = W * C / per, seg = p * C / per, lu = left * C / per;
+    const int span = to_patches ? row_units : img_units;
+    const dim3 grid((span + 256 * PATCH_UNROLL - 1) / (256 * PATCH_UNROLL), static_cast<unsigned>(rows));
+    if (to_patches)
+      pad_patchify_kernel<V><<<grid, 256, 0, stream>>>(static_cast<const V*>(image), static_cast<V*>(patches), H, p, hn, top, lu,
+                                                       img_units, row_units, seg);
+    else
+      unpatchify_crop_kernel<V><<<grid, 256, 0, stream>>>(static_cast<const V*>(patches), static_cast<const V*>(add),
+                                                          static_cast<V*>(image_out), H, p, hn, top, lu, img_units, row_units, seg);
+  };
+  if (bytes % 16 == 0) launch(uint4{});
+  else if (bytes % 8 == 0) launch(uint2{});
+  else if (bytes % 4 == 0) launch(uint32_t{});
+  else launch(static_cast<unsigned short>(0));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

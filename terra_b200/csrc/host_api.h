@@ -157,6 +157,10 @@ int window_attn_tc_stalls(unsigned long long* out16, int reset);   // [8..13]: s
 // Backward on tcgen05, head dims 16 / 32 / 64: one pass for windows of at most 64 tokens, two passes (dQ; dK, dV) with
 // `lse` and `drow` for larger ones.
 int window_attn_tc_bwd(const WindowAttnArgs& a, void* status, cudaStream_t stream);
+// Image [B, H, W, C] (bf16) to the patches [B, Hp / p, Wp / p, p * p * C] of the padded image (to_patches), or back, cropped,
+// with `add` (an image, or null) added.
+int patch_relayout(const void* image, const void* add, void* patches, void* image_out, int to_patches, int B, int H, int W, int C,
+                   int p, int Hp, int Wp, int top, int left, cudaStream_t stream);
 // drow[row, head] = sum over the head's channels of dO * O (bf16 [rows, C] inputs, fp32 [rows, heads] output).
 int attn_rowdot(const void* o, const void* dout, float* drow, long long rows, int C, int heads, cudaStream_t stream);
 

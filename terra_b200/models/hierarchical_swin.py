@@ -21,6 +21,7 @@ from ..global_env_config import ON_H200
 from ..memory.activation import activation_checkpoint, activation_config_for_sampling
 from ..ops import blocks as B
 from ..ops.conv import conv3x3, conv_transpose2x2, groupnorm_silu
+from ..ops.patch import pad_patchify, patch_kernels_apply, unpatchify_add
 from ..parallel.context import ParallelContext
 from ..profiler.memory_timeline import mark_memory_timeline
 from ..utils.padding import get_padded_shape
@@ -248,13 +249,17 @@ class SequentialHierarchicalSwin(_SwinBase):
         x = input.permute(0, 2, 3, 1) if self.input_nchw else input
         raw_h, raw_w = x.shape[1], x.shape[2]
         xin = x.to(self._compute_dtype(x))
+        left, right, top, bottom = self.initial_padding
+        fits = (raw_h + top + bottom, raw_w + left + right) == tuple(self.padded_shape)
+        if fits and patch_kernels_apply(xin, self.padded_shape):
+            p = self.patch_size
+            y = unpatchify_add(self._core(pad_patchify(xin, p, self.padded_shape, top, left), None), xin, p, top, left)
+            return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y
         if self.need_padding:
-            left, right, top, bottom = self.initial_padding
             xin = torch.nn.functional.pad(xin, (0, 0, left, right, top, bottom))
         patches = patchify(xin, self.patch_size).contiguous()
         y = unpatchify(self._core(patches, None), self.patch_size)
         if self.need_padding:
-            left, right, top, bottom = self.initial_padding
             y = y[:, top:top + raw_h, left:left + raw_w, :]
         y = y + x.to(y.dtype)
         return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y

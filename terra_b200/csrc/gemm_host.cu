@@ -120,6 +120,37 @@ static int pick_bn(long long N, int requested) {
   return 128;
 }
 
+// CTA pairs (256-row tiles, one MMA over two SMs). What bounds the main loop is the shared-memory port (128 B per clock
+// and SM): a k-block of a 128 x BN tile costs (16 + BN / 8) KB of operand fill and as much again for the tensor core's
+// reads. In a pair each CTA stages 128 rows of A and only half of B's BN rows, (16 + BN / 16) KB. Pairs are taken by
+// plain products (no peers, no split, no column sums) as soon as their tiles make eight rounds over the
+// pairs of SMs; with fewer rounds the larger tiles leave more of the last one empty (17280 rows, 576 x 192: 12 us with
+// single CTAs, 18 us with pairs; 139264 rows, 1152 x 384: 130 and 120 us). Returns the pair tile width, 0: single CTAs.
+static bool pairs_enabled() {
+  static const bool on = [] {
+    const char* e = std::getenv("TERRA_GEMM_2CTA");
+    return e == nullptr || std::atoi(e) != 0;
+  }();
+  return on;
+}
+
+static int pick_pair_bn(long long m_blocks, long long N, bool b_mn, int num_sms) {
+  if (!pairs_enabled()) return 0;
+  int best = 0;
+  long long best_cost = 0;
+  for (int bn : {256, 192, 128}) {
+    if (b_mn && bn == 192) continue;               // half of an MN-major B must be whole 64-row boxes
+    const long long n_tiles = (N + bn - 1) / bn;
+    if (((m_blocks + 1) / 2) * n_tiles < 8LL * (num_sms / 2)) continue;
+    const long long cost = n_tiles * (16 + bn / 16);   // KB through the port per 128 rows and k-block
+    if (best == 0 || cost < best_cost) {
+      best = bn;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 static void fill_epilogue(GemmParams& p, const GemmEpilogue& e) {
   p.epi = e.flags;
   p.C = e.C;
@@ -155,22 +186,18 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   // scattered output is either the fp32 atomic form or the plain bf16 form (one staging slot per source GPU)
   if (scatter_c && (epi.flags & EPI_OUT_F32) && !(epi.flags & EPI_ATOMIC)) return -13;
   if ((gather_a || scatter_c) && bn_request >= 1000) return -14;   // single-CTA tiles only
-  // CTA pairs (256-row tiles, one MMA over two SMs): explicit request 1000 + BN, or by policy for the shapes where
-  // the main loop dominates (long contraction or wide output) when TERRA_GEMM_2CTA=1.
+  // CTA pairs: explicit request 1000 + BN, or the rule of pick_pair_bn where no tile width is asked for.
   int ctas = 1;
   if (bn_request >= 1000) {
     ctas = 2;
     bn_request -= 1000;
-    if (bn_request != 128 && bn_request != 256) return -11;
-  } else {
-    static const int policy = [] {
-      const char* e = std::getenv("TERRA_GEMM_2CTA");
-      return (e != nullptr) ? std::atoi(e) : 0;
-    }();
-    if (policy == 1 && !gather_a && !scatter_c && M >= 512 && N >= 128 &&
-        (bn_request == 0 || bn_request == 128 || bn_request == 256)) {
+    if (bn_request != 128 && bn_request != 256 && !(bn_request == 192 && !B.mn_major)) return -11;
+  } else if (bn_request == 0 && !A.mn_major && !gather_a && !scatter_c && split_k <= 1 && epi.colsum == nullptr &&
+             !(epi.flags & EPI_ROW_SHUFFLE)) {
+    const int bn2 = pick_pair_bn((M + GEMM_BM - 1) / GEMM_BM, N, B.mn_major, num_sms);
+    if (bn2 != 0) {
       ctas = 2;
-      if (bn_request == 0) bn_request = (N % 256 == 0 || N >= 1024) ? 256 : 128;
+      bn_request = bn2;
     }
   }
   if (epi.colsum != nullptr) {
@@ -182,7 +209,8 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   p.M = static_cast<int>(M);
   p.N = static_cast<int>(N);
   p.K = static_cast<int>(K);
-  p.num_m_tiles = static_cast<int>((M + GEMM_BM * ctas - 1) / (GEMM_BM * ctas));
+  p.m_blocks = static_cast<int>((M + GEMM_BM - 1) / GEMM_BM);
+  p.num_m_tiles = (p.m_blocks + ctas - 1) / ctas;
   if (gather_a || scatter_c) ctas = 1;
   if (gather_a) {
     p.a_peers = peers.a_peers;
@@ -233,7 +261,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   p.out_w = epi.out_w;
   p.out_h = epi.out_h;
   p.shuffle_cout = epi.shuffle_cout > 0 ? epi.shuffle_cout : 1;
-  if (ctas == 1) try_tma_epilogue(p, M, N);
+  try_tma_epilogue(p, M, N);
   cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
@@ -283,13 +311,17 @@ int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin,
   const int cchunks = (Cin + 63) / 64;
   const int cin_pad = cchunks * 64;
   if (9 * cchunks > GEMM_MAX_KTABLE) return -14;
-  const int bn = pick_bn(Cout, 0);
+  const long long m_blocks = static_cast<long long>((Wo + GEMM_BM - 1) / GEMM_BM) * Ho * B;
+  const int bn2 = pick_pair_bn(m_blocks, Cout, false, num_sms);
+  const int ctas = bn2 != 0 ? 2 : 1;
+  const int bn = bn2 != 0 ? bn2 : pick_bn(Cout, 0);
   p.M = B * Ho * Wo;
   p.N = Cout;
   p.K = 9 * cin_pad;
   p.tile_n0 = (Wo + GEMM_BM - 1) / GEMM_BM;
   p.tile_n1 = Ho;
-  p.num_m_tiles = p.tile_n0 * Ho * B;
+  p.m_blocks = static_cast<int>(m_blocks);
+  p.num_m_tiles = (p.m_blocks + ctas - 1) / ctas;
   p.num_n_tiles = (Cout + bn - 1) / bn;
   p.k_blocks = 9 * cchunks;
   p.split_k = 1;
@@ -308,7 +340,7 @@ int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin,
   unsigned int box[5] = {64, 1, GEMM_BM, 1, 1};
   int rc = make_tensor_map_bf16(&p.map_a, x, 5, dims, str, box);
   if (rc != 0) return rc;
-  rc = map_2d(&p.map_b, w, p.K, Cout, p.K, GEMM_BK, bn);
+  rc = map_2d(&p.map_b, w, p.K, Cout, p.K, GEMM_BK, bn / ctas);
   if (rc != 0) return rc - 1000;
   rc = attach_halos(p, halo_lo, halo_hi, Cin, par, W, H, B, GEMM_BM);
   if (rc != 0) return rc;
@@ -337,7 +369,7 @@ int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin,
   p.out_w = Wo;
   p.out_h = Ho;
   p.shuffle_cout = 1;
-  cudaError_t e = launch_gemm(p, bn, 1, num_sms, stream);
+  cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
 
@@ -361,7 +393,8 @@ int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, i
   p.pix_hmul = stride;
   p.k_blocks = p.pix_n0 * Ho * B;
   p.K = p.k_blocks * GEMM_BK;
-  p.num_m_tiles = (Cout + GEMM_BM - 1) / GEMM_BM;
+  p.m_blocks = (Cout + GEMM_BM - 1) / GEMM_BM;
+  p.num_m_tiles = p.m_blocks;
   p.num_n_tiles = (Cin + bn - 1) / bn;
   p.groups = 9;
   if (split_k < 1) split_k = 1;

@@ -46,8 +46,9 @@ struct GemmCfg {
   static constexpr int B_BYTES = B_ROWS * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   // After the operand ring: 512 bytes of barriers, the per-warp bias slots (together 2 KB), then `bufs` buffers of
-  // 2 KB per epilogue warp (1: the exchange / output staging buffer; 3: two more for the operand the epilogue reads,
-  // loaded ahead by TMA). The ring takes what is left: the launcher passes the stage count to the kernel.
+  // 2 KB per epilogue warp: one or two output staging buffers (one: also the exchange buffer of the per-lane epilogue),
+  // and two more for the operand the epilogue reads, loaded ahead by TMA. The ring takes what is left: the launcher
+  // passes the stage count to the kernel.
   static constexpr int BAR_BYTES = 512;
   static constexpr int FIXED_BASE = 2048;
   static constexpr int EPI_BUF = 2048;
@@ -66,7 +67,15 @@ struct GemmCfg {
   static constexpr bool CAN_COLSUM = CTAS == 1 && 2 * BN + 64 <= 512;
   static_assert(stages_for(3) >= 3 && smem_bytes(1) <= MAX_SMEM && smem_bytes(3) <= MAX_SMEM, "shared memory budget");
   static_assert(GEMM_EPI_WARPS * 32 * 4 + BAR_BYTES <= FIXED_BASE, "bias slots");
-  static_assert(CTAS == 1 || (B_ROWS % 64 == 0), "a CTA's half of B must be whole 64-row boxes");
+  // a CTA's half of an MN-major B must be whole 64-row boxes; K-major rows only need whole 8-row swizzle atoms
+  static constexpr bool CAN_B_MN = B_ROWS % 64 == 0;
+  static_assert(B_ROWS % 8 == 0 && B_BYTES % 1024 == 0, "B tile: whole swizzle atoms");
+  // Output staging buffers per epilogue warp. Two let a chunk be written while the store of the chunk before is still
+  // reading its buffer (that read takes several hundred cycles); not where they would cost an operand stage out of four.
+  static constexpr int out_bufs(bool has_in) {
+    const int in = has_in ? 2 : 0;
+    return (stages_for(2 + in) >= 4 || stages_for(2 + in) == stages_for(1 + in)) ? 2 : 1;
+  }
 };
 
 // Cycle counters of the three roles, summed over CTAs and launches since the last reset (read by gemm_read_stalls):
@@ -271,7 +280,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             tma_load_2d(sB, &p.map_b, &full[s], kb * GEMM_BK, n0);
           } else if (p.b_mode == OP_MNMAJOR_2D) {
 #pragma unroll
-            for (int j = 0; j < Cfg::B_ROWS / 64; ++j)
+            for (int j = 0; Cfg::CAN_B_MN && j < Cfg::B_ROWS / 64; ++j)
               tma_load_2d(sB + j * (GEMM_BK * 128), &p.map_b, &full[s], n0 + j * 64, kb * GEMM_BK);
           } else {  // OP_PIXELS_5D with per-group (tap) displacement
             const short* g = p.grp_off[tc.grp];
@@ -385,23 +394,25 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       return reinterpret_cast<uint4*>(my_x + rr * 64 + (((vec ^ (rr >> 1)) & 3) << 4));
     };
     constexpr int CPW = (CHUNKS + GEMM_EPI_WARPS / 4 - 1) / (GEMM_EPI_WARPS / 4);   // chunks per warp
-    if (!PAIR && !PEERS && p.epi_tma) {
+    if (!PEERS && p.epi_tma) {
       // ---- plain row-major bf16 outputs: chunks leave (and the operand the epilogue reads arrives) through TMA.
       // A chunk is 32 rows of 64 bytes in the 64-byte-swizzled layout, which is also conflict-free for the
-      // row-per-lane 16-byte accesses of the warp. Buffer 0 of the warp stages outputs: one lane issues the store and,
-      // before the next chunk is written, waits until the store has read the buffer. Buffers 1 and 2 receive the
-      // input operand two chunks ahead (across tiles), so its latency hides behind the chunks in between.
-      uint8_t* my_bufs = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
-      uint64_t* my_in = in_bar + (warp - 2) * 2;
+      // row-per-lane 16-byte accesses of the warp. The warp's first one or two buffers stage outputs in turn: one lane
+      // issues the store and, before a buffer is written again, waits until its store has read it. The last two receive
+      // the input operand two chunks ahead (across tiles), so its latency hides behind the chunks in between.
       const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
+      const bool two_out = p.epi_bufs == (has_in ? 4 : 2);
+      uint8_t* my_bufs = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
+      uint8_t* in_bufs = my_bufs + (two_out ? 2 : 1) * Cfg::EPI_BUF;
+      uint64_t* my_in = in_bar + (warp - 2) * 2;
       const uint32_t row_off = static_cast<uint32_t>(lane) * 64u;
       const uint32_t swz = (static_cast<uint32_t>(lane) >> 1) & 3u;
       const uint32_t out_addr = smem_u32(my_bufs);
-      uint32_t issued = 0, consumed = 0;
+      uint32_t issued = 0, consumed = 0, stored = 0;
       int pf_tile = unit, pf_ci = 0;
       auto prefetch_next = [&]() {   // issue the load of this warp's next input chunk, if there is one
         while (pf_tile < total_tiles) {
-          const TileCoord t = decode_tile(p, pf_tile, 1, 0);
+          const TileCoord t = decode_tile(p, pf_tile, CTAS, rank);
           const int c = part + pf_ci * (GEMM_EPI_WARPS / 4);
           const int col = t.n_blk * BN + c * 32;
           const int row = t.m_blk * GEMM_BM + q * 32;
@@ -414,7 +425,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             if (lane == 0) {
               uint64_t* b = my_in + (issued & 1u);
               mbar_expect_tx(b, Cfg::EPI_BUF);
-              tma_load_2d(my_bufs + Cfg::EPI_BUF * (1 + (issued & 1u)), &p.map_in, b, col, row);
+              tma_load_2d(in_bufs + Cfg::EPI_BUF * (issued & 1u), &p.map_in, b, col, row);
             }
             ++issued;
             return;
@@ -422,11 +433,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         }
       };
       auto stage_store = [&](const CUtensorMap* map, const float (&f)[32], int col, int row) {
-        if (lane == 0) bulk_wait_group_read<0>();
+        if (lane == 0) {
+          if (two_out) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
+        }
         __syncwarp();
+        const uint32_t dst = out_addr + (two_out ? (stored & 1u) * Cfg::EPI_BUF : 0u);
+        ++stored;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const uint32_t a = out_addr + row_off + (((static_cast<uint32_t>(j) ^ swz) & 3u) << 4);
+          const uint32_t a = dst + row_off + (((static_cast<uint32_t>(j) ^ swz) & 3u) << 4);
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(pack_bf16x2(f[8 * j], f[8 * j + 1])),
                        "r"(pack_bf16x2(f[8 * j + 2], f[8 * j + 3])), "r"(pack_bf16x2(f[8 * j + 4], f[8 * j + 5])),
                        "r"(pack_bf16x2(f[8 * j + 6], f[8 * j + 7]))
@@ -434,8 +449,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && row < p.M) {
-          tma_store_2d(map, out_addr, col, row);
+        if (lane == 0) {   // a group per chunk, also where the rows lie outside the output: the waits count groups
+          if (row < p.M) tma_store_2d(map, dst, col, row);
           bulk_commit_group();
         }
       };
@@ -445,7 +460,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       }
       bool failed = false;
       for (int tile = unit; tile < total_tiles && !failed; tile += units, ++tcount) {
-        const TileCoord tc = decode_tile(p, tile, 1, 0);
+        const TileCoord tc = decode_tile(p, tile, CTAS, rank);
         const int acc = tcount & 1;
         const uint32_t aph = (tcount >> 1) & 1u;
         const int n0 = tc.n_blk * BN;
@@ -456,7 +471,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         e_wait += clock64() - ew0;
         tc_fence_after();
         bool released = false;
-#pragma unroll
+        auto release = [&]() {   // the accumulator has been read: the MMA thread may start the tile after next
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (PAIR && rank == 1) mbar_arrive_remote(map_to_cta(&tempty[acc], 0));   // the leader's MMA thread waits
+            else mbar_arrive(&tempty[acc]);
+          }
+        };
+        // (not unrolled: one copy of the chunk's code stays in the instruction cache of the twelve warps)
+#pragma unroll 1
         for (int ci = 0; ci < CPW; ++ci) {
           const int c = part + ci * (GEMM_EPI_WARPS / 4);
           if (c >= CHUNKS || n0 + c * 32 >= p.N) break;   // warp-uniform
@@ -483,7 +507,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               failed = true;
               break;
             }
-            const uint32_t src = smem_u32(my_bufs + Cfg::EPI_BUF * (1 + b)) + row_off;
+            const uint32_t src = smem_u32(in_bufs + Cfg::EPI_BUF * b) + row_off;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const uint32_t a = src + (((static_cast<uint32_t>(j) ^ swz) & 3u) << 4);
@@ -495,30 +519,28 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             ++consumed;
           }
           tmem_ld_wait();
-          if (last) {   // the accumulator has been read: the MMA thread may start the tile after next
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[acc]);
+          if (last) {
+            release();
             released = true;
           }
           float f[32];
+          const f32x2 alpha2 = f2_pack(p.alpha, p.alpha);
           if (has_bias) {
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
               const float4 b4 = *reinterpret_cast<const float4*>(my_bias + j);
-              f[j] = fmaf(__uint_as_float(v[j]), p.alpha, b4.x);
-              f[j + 1] = fmaf(__uint_as_float(v[j + 1]), p.alpha, b4.y);
-              f[j + 2] = fmaf(__uint_as_float(v[j + 2]), p.alpha, b4.z);
-              f[j + 3] = fmaf(__uint_as_float(v[j + 3]), p.alpha, b4.w);
+              f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2, f2_pack(b4.x, b4.y)), f[j], f[j + 1]);
+              f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), alpha2, f2_pack(b4.z, b4.w)), f[j + 2], f[j + 3]);
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * p.alpha;
+            for (int j = 0; j < 32; j += 2)
+              f2_unpack(f2_mul(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2), f[j], f[j + 1]);
           }
           if (p.epi & EPI_SAVE_PRE) stage_store(&p.map_c2, f, nb, row0);
           if (p.epi & EPI_GELU) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) f[j] = gelu_erf(f[j]);
+            for (int j = 0; j < 32; j += 2) f2_unpack(gelu_erf2(f2_pack(f[j], f[j + 1])), f[j], f[j + 1]);
           }
           if (has_in) {
             const bool dgelu = (p.epi & EPI_MUL_DGELU) != 0;
@@ -528,13 +550,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
                 const float2 x = unpack_bf16x2(w4[k]);
-                if (dgelu) {
-                  f[8 * j + 2 * k] *= gelu_erf_grad(x.x);
-                  f[8 * j + 2 * k + 1] *= gelu_erf_grad(x.y);
-                } else {
-                  f[8 * j + 2 * k] += x.x;
-                  f[8 * j + 2 * k + 1] += x.y;
-                }
+                const f32x2 f2 = f2_pack(f[8 * j + 2 * k], f[8 * j + 2 * k + 1]), x2 = f2_pack(x.x, x.y);
+                f2_unpack(dgelu ? f2_mul(f2, gelu_erf_grad2(x2)) : f2_add(f2, x2), f[8 * j + 2 * k], f[8 * j + 2 * k + 1]);
               }
             }
             __syncwarp();        // every lane holds its part of the input chunk: its buffer may be refilled
@@ -542,11 +559,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           }
           stage_store(&p.map_c, f, nb, row0);
         }
-        if (!released && !failed) {   // a warp without a chunk in this tile (narrow last column tile)
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[acc]);
-        }
+        if (!released && !failed) release();   // a warp without a chunk in this tile (narrow last column tile)
       }
       if (lane == 0) bulk_wait_group_read<0>();
     } else
@@ -564,7 +577,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           const int t1 = (tc.m_blk / p.tile_n0) % p.tile_n1;
           const int t2 = tc.m_blk / (p.tile_n0 * p.tile_n1);
           const int w = t0 * GEMM_BM + r;
-          return (w < p.out_w) ? (static_cast<long long>(t2) * p.tile_n1 + t1) * p.out_w + w : -1;
+          return (w < p.out_w && tc.m_blk < p.m_blocks) ? (static_cast<long long>(t2) * p.tile_n1 + t1) * p.out_w + w : -1;
         } else if (p.epi & EPI_ROW_SHUFFLE) {
           const long long g = static_cast<long long>(tc.m_blk) * GEMM_BM + r;
           if (g >= p.M) return -1;
@@ -828,10 +841,11 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
     configured = true;
   }
   GemmParams p = p_in;
-  if (CTAS != 1 || PEERS) p.epi_tma = 0;
-  p.epi_bufs = (p.epi_tma && (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU))) ? 3 : 1;
-  p.stages = p.epi_bufs == 3 ? Cfg::stages_for(3) : Cfg::stages_for(1);
-  p.smem_bytes = p.epi_bufs == 3 ? Cfg::smem_bytes(3) : Cfg::smem_bytes(1);
+  if (PEERS) p.epi_tma = 0;
+  const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
+  p.epi_bufs = p.epi_tma ? Cfg::out_bufs(has_in) + (has_in ? 2 : 0) : 1;
+  p.stages = Cfg::stages_for(p.epi_bufs);
+  p.smem_bytes = Cfg::smem_bytes(p.epi_bufs);
   const int total = p.groups * p.num_m_tiles * p.num_n_tiles * p.split_k;
   const int max_units = num_sms / CTAS;
   const int units = total < max_units ? total : max_units;
@@ -869,6 +883,7 @@ cudaError_t launch_gemm(const GemmParams& p, int bn, int ctas, int num_sms, cuda
   if (ctas == 2) {
     switch (bn) {
       case 128: return launch_bn<128, 2>(p, num_sms, stream);
+      case 192: return p.b_mode == OP_KMAJOR_2D ? launch_bn<192, 2>(p, num_sms, stream) : cudaErrorInvalidValue;
       case 256: return launch_bn<256, 2>(p, num_sms, stream);
       default: return cudaErrorInvalidValue;
     }

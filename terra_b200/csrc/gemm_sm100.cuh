@@ -43,6 +43,7 @@ struct GemmParams {
   int img_h;                   // rows of the local image
   int M, N, K;                 // logical output rows, cols, contraction length (elements)
   int num_m_tiles, num_n_tiles;
+  int m_blocks;                // 128-row blocks of the output (a CTA pair's last tile may reach beyond them)
   int k_blocks;                // total 64-wide k-blocks
   int split_k;                 // >1: tiles are (m, n, split); needs EPI_ATOMIC
   int groups;                  // extra outermost tile dimension (conv taps for the weight gradient); >=1
@@ -69,10 +70,10 @@ struct GemmParams {
   int shuffle_cout;
   float alpha;
   KernelStatus* status;
-  // Epilogue through TMA (plain row-major bf16 outputs, single-CTA tiles): every epilogue warp stages its 32 x 32
-  // chunk in shared memory in the 64-byte-swizzled layout and one lane stores it through map_c / map_c2; the operand
-  // the epilogue reads (residual, or the GELU input of the backward pass) arrives through map_in, loaded two chunks
-  // ahead into per-warp buffers. epi_bufs = buffers of 2 KB per epilogue warp (1: output staging; 3: + two inputs).
+  // Epilogue through TMA (plain row-major bf16 outputs): every epilogue warp stages its 32 x 32 chunk in shared memory in
+  // the 64-byte-swizzled layout and one lane stores it through map_c / map_c2; the operand the epilogue reads (residual,
+  // or the GELU input of the backward pass) arrives through map_in, loaded two chunks ahead into per-warp buffers.
+  // epi_bufs = buffers of 2 KB per epilogue warp (1 or 2: output staging; + two where there is an input).
   // stages / smem_bytes: the launcher sizes the operand ring with what the epilogue buffers leave.
   float* colsum;               // weight-gradient form: += column sums of operand A over the contraction (see GemmEpilogue)
   CUtensorMap map_c, map_c2, map_in;

@@ -150,7 +150,7 @@ class _MlpHalfFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, anchor, pk: ParamPack):
         xn, mean, rstd = layernorm_cuda(x, pk.ln_w, pk.ln_b)
-        act, pre = gemm(xn, pk.fc1_w, bias=pk.fc1_b, gelu=True, save_pre=True, bn=256 if pk.fc1_w.shape[0] % 256 == 0 else 0)
+        act, pre = gemm(xn, pk.fc1_w, bias=pk.fc1_b, gelu=True, save_pre=True)
         y = gemm(act, pk.fc2_w, bias=pk.fc2_b, residual=x)
         ctx.save_for_backward(x, mean, rstd, xn, pre, act)
         ctx.pk = pk
@@ -162,7 +162,7 @@ class _MlpHalfFn(torch.autograd.Function):
         pk = ctx.pk
         dy = dy.contiguous()
         wgrad_accumulate(dy, act, pk.fc2_wg, pk.fc2_bg)
-        dpre = gemm(dy, pk.fc2_w, b_mn=True, dgelu_aux=pre, bn=256 if pk.fc2_w.shape[1] % 256 == 0 else 0)
+        dpre = gemm(dy, pk.fc2_w, b_mn=True, dgelu_aux=pre)
         wgrad_accumulate(dpre, xn, pk.fc1_wg, pk.fc1_bg)
         dxn = gemm(dpre, pk.fc1_w, b_mn=True)
         dx = layernorm_bwd_cuda(dxn, x, pk.ln_w, mean, rstd, pk.ln_wg, pk.ln_bg, dres=dy)

@@ -34,8 +34,8 @@ void check_bf16_2d(const torch::Tensor& t, const char* name) {
 void gemm(const torch::Tensor& a, bool a_mn, const torch::Tensor& b, bool b_mn, torch::Tensor& c, int64_t flags,
           const c10::optional<torch::Tensor>& bias, const c10::optional<torch::Tensor>& residual,
           const c10::optional<torch::Tensor>& aux, const c10::optional<torch::Tensor>& c2, double alpha,
-          int64_t split_k, int64_t bn, const c10::optional<torch::Tensor>& status, int64_t shuffle_cout,
-          int64_t out_w, int64_t out_h, int64_t sms, const std::vector<int64_t>& a_peer_ptrs, int64_t rank,
+          int64_t split_k, int64_t bn, const c10::optional<torch::Tensor>& status, int64_t sms,
+          const std::vector<int64_t>& a_peer_ptrs, int64_t rank,
           const std::vector<int64_t>& c_peer_ptrs, int64_t a_flags_ptr, int64_t a_epoch, int64_t a_budget_ns,
           int64_t a_interleave, int64_t a_chunks, const c10::optional<torch::Tensor>& colsum) {
   check_bf16_2d(a, "a");
@@ -57,7 +57,6 @@ void gemm(const torch::Tensor& a, bool a_mn, const torch::Tensor& b, bool b_mn, 
   e.flags = static_cast<int>(flags);
   e.C = c.data_ptr();
   e.ldc = c.dim() >= 2 ? c.stride(c.dim() - 2) : c.size(-1);
-  if (shuffle_cout > 0) e.ldc = shuffle_cout;
   e.C2 = c2.has_value() ? c2->data_ptr() : nullptr;
   e.ldc2 = c2.has_value() ? c2->stride(0) : 0;
   e.bias = opt_ptr(bias);
@@ -67,9 +66,6 @@ void gemm(const torch::Tensor& a, bool a_mn, const torch::Tensor& b, bool b_mn, 
   e.ldaux = aux.has_value() ? aux->stride(0) : 0;
   e.alpha = static_cast<float>(alpha);
   e.status = status.has_value() ? status->data_ptr() : nullptr;
-  e.shuffle_cout = static_cast<int>(shuffle_cout);
-  e.out_w = static_cast<int>(out_w);
-  e.out_h = static_cast<int>(out_h);
   if (colsum.has_value()) {
     TORCH_CHECK(colsum->scalar_type() == torch::kFloat32 && colsum->is_contiguous() && colsum->numel() == M,
                 "gemm: colsum must be contiguous fp32 with one entry per output row");
@@ -150,6 +146,69 @@ void conv3x3_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tenso
   TORCH_CHECK(rc == 0, "terra_b200 conv3x3_wgrad launch failed, code ", rc);
 }
 
+void check_image(const torch::Tensor& t, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.is_contiguous() && t.dim() == 4, name, ": NHWC bf16 contiguous");
+}
+void check_packed(const torch::Tensor& w, int64_t rows, int64_t taps, int64_t channels) {
+  TORCH_CHECK(w.scalar_type() == torch::kBFloat16 && w.is_contiguous() && w.dim() == 2 && w.size(0) == rows &&
+                  w.size(1) == taps * ((channels + 63) / 64 * 64),
+              "packed weights: bf16 [", rows, ", ", taps, " * channels padded to 64]");
+}
+void* status_ptr(const c10::optional<torch::Tensor>& s) { return s.has_value() ? s->data_ptr() : nullptr; }
+
+// dy: [B, Ho, Wo, Cout], dx: [B, H, W, Cin] with Ho = (H + 1) / 2, Wo = W / 2; w: [Cin, 9 * Cout_pad]
+void conv3x3_s2_dgrad(const torch::Tensor& dy, const torch::Tensor& w, torch::Tensor& dx,
+                      const c10::optional<torch::Tensor>& status) {
+  check_image(dy, "dy");
+  check_image(dx, "dx");
+  TORCH_CHECK(dy.size(0) == dx.size(0) && dy.size(1) == (dx.size(1) + 1) / 2 && 2 * dy.size(2) == dx.size(2),
+              "conv3x3_s2_dgrad: dy must be the stride-2 output grid of dx");
+  check_packed(w, dx.size(3), 9, dy.size(3));
+  const c10::cuda::CUDAGuard guard(dy.device());
+  tb::note_launch();
+  const int rc = tb::conv3x3_s2_dgrad_bf16(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), dx.size(0), dx.size(1), dx.size(2), dx.size(3),
+                                           dy.size(3), status_ptr(status), sm_count(), cur_stream());
+  TORCH_CHECK(rc == 0, "terra_b200 conv3x3_s2_dgrad launch failed, code ", rc);
+}
+
+// The three products of the 2x2 / stride-2 transposed convolution, x [B, H, W, Cin] and y / dy [B, 2H, 2W, Cout]:
+// op 0: y from x (w: [4 * Cout, Cin_pad], bias [4 * Cout]); op 1: dx from dy (w: [Cin, 4 * Cout_pad])
+void convt2x2(int64_t op, const torch::Tensor& in, const torch::Tensor& w, const c10::optional<torch::Tensor>& bias4,
+              torch::Tensor& out, const c10::optional<torch::Tensor>& status) {
+  check_image(in, "in");
+  check_image(out, "out");
+  const torch::Tensor &x = op == 0 ? in : out, &y = op == 0 ? out : in;
+  TORCH_CHECK(x.size(0) == y.size(0) && 2 * x.size(1) == y.size(1) && 2 * x.size(2) == y.size(2), "convt2x2: grids");
+  const int64_t Cin = x.size(3), Cout = y.size(3);
+  check_packed(w, op == 0 ? 4 * Cout : Cin, op == 0 ? 1 : 4, op == 0 ? Cin : Cout);
+  TORCH_CHECK(op != 0 || (bias4.has_value() && bias4->scalar_type() == torch::kBFloat16 && bias4->is_contiguous() &&
+                          bias4->numel() == 4 * Cout),
+              "convt2x2: bias bf16 [4 * Cout]");
+  const c10::cuda::CUDAGuard guard(x.device());
+  tb::note_launch();
+  const int rc = op == 0 ? tb::convt2x2_fwd_bf16(x.data_ptr(), w.data_ptr(), opt_ptr(bias4), out.data_ptr(), x.size(0), x.size(1),
+                                                 x.size(2), Cin, Cout, status_ptr(status), sm_count(), cur_stream())
+                         : tb::convt2x2_dgrad_bf16(y.data_ptr(), w.data_ptr(), out.data_ptr(), x.size(0), x.size(1), x.size(2), Cin,
+                                                   Cout, status_ptr(status), sm_count(), cur_stream());
+  TORCH_CHECK(rc == 0, "terra_b200 convt2x2 launch failed, code ", rc);
+}
+
+// dw: [4, Cin, Cout] fp32, accumulated
+void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tensor& dw, int64_t split_k,
+                    const c10::optional<torch::Tensor>& status) {
+  check_image(x, "x");
+  check_image(dy, "dy");
+  TORCH_CHECK(x.size(0) == dy.size(0) && 2 * x.size(1) == dy.size(1) && 2 * x.size(2) == dy.size(2), "convt2x2_wgrad: grids");
+  TORCH_CHECK(dw.scalar_type() == torch::kFloat32 && dw.is_contiguous() && dw.numel() == 4 * x.size(3) * dy.size(3),
+              "dw: fp32 [4, Cin, Cout]");
+  const c10::cuda::CUDAGuard guard(x.device());
+  tb::note_launch();
+  const int rc = tb::convt2x2_wgrad_bf16(x.data_ptr(), dy.data_ptr(), dw.data_ptr<float>(), x.size(0), x.size(1), x.size(2),
+                                         x.size(3), dy.size(3), static_cast<int>(split_k), status_ptr(status), sm_count(),
+                                         cur_stream());
+  TORCH_CHECK(rc == 0, "terra_b200 convt2x2_wgrad launch failed, code ", rc);
+}
+
 }  // namespace
 
 void bind_elementwise(pybind11::module_& m);
@@ -168,14 +227,18 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   namespace py = pybind11;
   m.def("gemm", &gemm, "tcgen05 bf16 GEMM with fused epilogues", py::arg("a"), py::arg("a_mn"), py::arg("b"),
         py::arg("b_mn"), py::arg("c"), py::arg("flags"), py::arg("bias"), py::arg("residual"), py::arg("aux"),
-        py::arg("c2"), py::arg("alpha"), py::arg("split_k"), py::arg("bn"), py::arg("status"), py::arg("shuffle_cout"),
-        py::arg("out_w"), py::arg("out_h"), py::arg("sms"), py::arg("a_peer_ptrs"), py::arg("rank"),
+        py::arg("c2"), py::arg("alpha"), py::arg("split_k"), py::arg("bn"), py::arg("status"), py::arg("sms"),
+        py::arg("a_peer_ptrs"), py::arg("rank"),
         py::arg("c_peer_ptrs"), py::arg("a_flags_ptr"), py::arg("a_epoch"), py::arg("a_budget_ns"),
         py::arg("a_interleave"), py::arg("a_chunks"), py::arg("colsum") = py::none());
   m.def("conv3x3_fwd", &conv3x3_fwd, "implicit-GEMM 3x3 convolution (NHWC bf16)");
   m.def("conv3x3_wgrad", &conv3x3_wgrad, "3x3 convolution weight gradient (fp32 atomics)", py::arg("x"), py::arg("dy"),
         py::arg("dw"), py::arg("stride"), py::arg("split_k"), py::arg("status"), py::arg("halo_lo"), py::arg("halo_hi"),
         py::arg("bias_grad") = py::none());
+  m.def("conv3x3_s2_dgrad", &conv3x3_s2_dgrad, "input gradient of the stride-2 3x3 convolution (NHWC bf16)");
+  m.def("convt2x2", &convt2x2, "2x2 / stride-2 transposed convolution: forward (op 0), input gradient (op 1)", py::arg("op"),
+        py::arg("input"), py::arg("w"), py::arg("bias4"), py::arg("out"), py::arg("status"));
+  m.def("convt2x2_wgrad", &convt2x2_wgrad, "2x2 / stride-2 transposed convolution: weight gradient (fp32 atomics)");
   bind_elementwise(m);
   bind_attention(m);
   bind_copy_engine(m);

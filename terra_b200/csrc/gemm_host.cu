@@ -99,7 +99,7 @@ static void try_tma_epilogue(GemmParams& p, long long M, long long N) {
   }();
   p.epi_tma = 0;
   const int f = p.epi;
-  if (!enabled || (f & (EPI_OUT_F32 | EPI_ATOMIC | EPI_ROW_CONV | EPI_ROW_SHUFFLE))) return;
+  if (!enabled || (f & (EPI_OUT_F32 | EPI_ATOMIC | EPI_ROW_CONV))) return;
   if ((f & EPI_RESIDUAL) && (f & EPI_MUL_DGELU)) return;
   // The input buffers cost the operand ring one or two stages. A long contraction hides the epilogue behind its main
   // loop anyway and wants the deeper ring instead (K = 1536 with a residual measured 15 % slower on three stages).
@@ -125,7 +125,7 @@ static int pick_bn(long long N, int requested) {
 // reads. In a pair each CTA stages 128 rows of A and only half of B's BN rows, (16 + BN / 16) KB. Pairs are taken by
 // plain products (no peers, no split, no column sums) as soon as their tiles make eight rounds over the
 // pairs of SMs; with fewer rounds the larger tiles leave more of the last one empty (17280 rows, 576 x 192: 12 us with
-// single CTAs, 18 us with pairs; 139264 rows, 1152 x 384: 130 and 120 us). Returns the pair tile width, 0: single CTAs.
+// single CTAs, 18 us with pairs; 139264 rows, 1152 x 384: 130 and 117 us). Returns the pair tile width, 0: single CTAs.
 static bool pairs_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("TERRA_GEMM_2CTA");
@@ -192,8 +192,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
     ctas = 2;
     bn_request -= 1000;
     if (bn_request != 128 && bn_request != 256 && !(bn_request == 192 && !B.mn_major)) return -11;
-  } else if (bn_request == 0 && !A.mn_major && !gather_a && !scatter_c && split_k <= 1 && epi.colsum == nullptr &&
-             !(epi.flags & EPI_ROW_SHUFFLE)) {
+  } else if (bn_request == 0 && !A.mn_major && !gather_a && !scatter_c && split_k <= 1 && epi.colsum == nullptr) {
     const int bn2 = pick_pair_bn((M + GEMM_BM - 1) / GEMM_BM, N, B.mn_major, num_sms);
     if (bn2 != 0) {
       ctas = 2;
@@ -258,9 +257,6 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   fill_epilogue(p, epi);
   p.tile_n0 = 1;
   p.tile_n1 = 1;
-  p.out_w = epi.out_w;
-  p.out_h = epi.out_h;
-  p.shuffle_cout = epi.shuffle_cout > 0 ? epi.shuffle_cout : 1;
   try_tma_epilogue(p, M, N);
   cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
@@ -298,105 +294,187 @@ static int attach_halos(GemmParams& p, const void* halo_lo, const void* halo_hi,
   return 0;
 }
 
+//
+// The general form, shared by the transposed convolutions and the strided input gradients: output pixel (i, j) of the tile
+// grid [tiles_h, tiles_w] sums, over the taps of its phase, input pixel (i * hmul + dh, columns split by parity `par`:
+// j + dw of parity `parity`) times the tap's [N, Cin] weights; it is stored at (i * out_mul + oy, parity ox of column j).
+// Measured (us, before -> now): transposed convolution 139264 x 384 -> 557056 x 384, forward 423 (per-lane pixel-shuffle
+// stores) -> 259, input gradient with the un-shuffling copy 147 + 562 -> 182, weight gradient 145 -> 192; input gradient of
+// the stride-2 convolution at 557056 pixels 397 (GEMM to per-tap columns) + 334 (gather) -> 394.
+struct Tap {
+  short parity, dw, dh;
+};
+struct GatherConv {
+  const void* x;
+  int B, H, W, Cin, par;            // input image
+  int tiles_h, tiles_w, hmul;
+  const Tap* taps;
+  int ntaps;
+  int groups;                       // phases with taps of their own (grp_taps[0 .. groups] = their ranges), or 1
+  int grp_taps[5];
+  const void* w;                    // [N, ntaps * Cin_pad], Cin padded to a multiple of 64 with zeros
+  int N;
+  void* y;
+  int out_h, out_w, out_c, out_mul; // output image; out_w = columns of one parity
+  int phase_cols;                   // > 0: phases side by side in N
+  short out_off[4][2];
+};
+
+static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms, cudaStream_t stream, const void* halo_lo,
+                       const void* halo_hi) {
+  if (c.Cin % 8 != 0 || c.out_c % 8 != 0 || c.W % c.par != 0) return -13;
+  const int cchunks = (c.Cin + 63) / 64;
+  if (c.ntaps * cchunks > GEMM_MAX_KTABLE) return -14;
+  GemmParams p;
+  std::memset(&p, 0, sizeof(p));
+  const long long m_blocks = static_cast<long long>((c.tiles_w + GEMM_BM - 1) / GEMM_BM) * c.tiles_h * c.B;
+  const int bn2 = pick_pair_bn(m_blocks * c.groups, c.N, false, num_sms);
+  const int ctas = bn2 != 0 ? 2 : 1;
+  const int bn = bn2 != 0 ? bn2 : pick_bn(c.N, 0);
+  p.M = c.B * c.tiles_h * c.tiles_w;
+  p.N = c.N;
+  p.K = c.ntaps * cchunks * 64;
+  p.tile_n0 = (c.tiles_w + GEMM_BM - 1) / GEMM_BM;
+  p.tile_n1 = c.tiles_h;
+  p.m_blocks = static_cast<int>(m_blocks);
+  p.num_m_tiles = (p.m_blocks + ctas - 1) / ctas;
+  p.num_n_tiles = (c.N + bn - 1) / bn;
+  p.k_blocks = c.ntaps * cchunks;
+  p.split_k = 1;
+  p.groups = c.groups;
+  if (c.groups > 1) {
+    p.grp_ranges = 1;
+    for (int g = 0; g <= c.groups; ++g) p.grp_kb[g] = c.grp_taps[g] * cchunks;
+  }
+  p.a_mode = OP_TABLE_5D;
+  p.b_mode = OP_KMAJOR_2D;
+  int rc = image_map(&p.map_a, c.x, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
+  if (rc != 0) return rc;
+  rc = map_2d(&p.map_b, c.w, p.K, c.N, p.K, GEMM_BK, bn / ctas);
+  if (rc != 0) return rc - 1000;
+  rc = attach_halos(p, halo_lo, halo_hi, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
+  if (rc != 0) return rc;
+  // tile (t0, t1, t2) = (w chunk, row, b): base coordinates
+  p.a_mul0[2] = GEMM_BM;
+  p.a_mul1[3] = c.hmul;
+  p.a_mul2[4] = 1;
+  for (int t = 0; t < c.ntaps; ++t)
+    for (int k = 0; k < cchunks; ++k) {
+      short* e = p.ktable[t * cchunks + k];
+      e[0] = static_cast<short>(k * 64);
+      e[1] = c.taps[t].parity;
+      e[2] = c.taps[t].dw;
+      e[3] = c.taps[t].dh;
+    }
+  fill_epilogue(p, epi);
+  p.C = c.y;
+  p.epi |= EPI_ROW_CONV;
+  p.out_w = c.out_w;
+  p.out_h = c.out_h;
+  p.out_mul = c.out_mul;
+  p.phase_cols = c.phase_cols;
+  std::memcpy(p.out_off, c.out_off, sizeof(p.out_off));
+  if (!(p.epi & ~(EPI_ROW_CONV | EPI_BIAS | EPI_BIAS_F32))) {
+    // 32 pixels x 32 channels per store; rows and channels outside the image are clipped
+    const unsigned long long C = static_cast<unsigned long long>(c.out_c), mul = static_cast<unsigned long long>(c.out_mul);
+    const unsigned long long row = C * 2ull * mul * c.out_w;
+    unsigned long long dims[5] = {C, mul, static_cast<unsigned long long>(c.out_w), static_cast<unsigned long long>(c.out_h),
+                                  static_cast<unsigned long long>(c.B)};
+    unsigned long long str[4] = {C * 2ull, C * 2ull * mul, row, row * c.out_h};
+    unsigned int box[5] = {32, 1, 32, 1, 1};
+    rc = make_tensor_map_bf16_swizzled(&p.map_c, c.y, 5, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc != 0) return rc - 5000;
+    p.epi_tma = 2;
+  } else if (c.out_mul != 1 || c.phase_cols != 0) {
+    return -16;
+  }
+  const cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);
+  return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+}
+
 int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin, int Cout, int stride,
                      const GemmEpilogue& epi, int num_sms, cudaStream_t stream, const void* halo_lo,
                      const void* halo_hi) {
   if (stride != 1 && stride != 2) return -11;
   if (stride == 2 && (W % 2 != 0)) return -12;
-  if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
-  GemmParams p;
-  std::memset(&p, 0, sizeof(p));
-  const int Ho = (stride == 1) ? H : (H + 1) / 2;
-  const int Wo = (stride == 1) ? W : W / 2;
-  const int cchunks = (Cin + 63) / 64;
-  const int cin_pad = cchunks * 64;
-  if (9 * cchunks > GEMM_MAX_KTABLE) return -14;
-  const long long m_blocks = static_cast<long long>((Wo + GEMM_BM - 1) / GEMM_BM) * Ho * B;
-  const int bn2 = pick_pair_bn(m_blocks, Cout, false, num_sms);
-  const int ctas = bn2 != 0 ? 2 : 1;
-  const int bn = bn2 != 0 ? bn2 : pick_bn(Cout, 0);
-  p.M = B * Ho * Wo;
-  p.N = Cout;
-  p.K = 9 * cin_pad;
-  p.tile_n0 = (Wo + GEMM_BM - 1) / GEMM_BM;
-  p.tile_n1 = Ho;
-  p.m_blocks = static_cast<int>(m_blocks);
-  p.num_m_tiles = (p.m_blocks + ctas - 1) / ctas;
-  p.num_n_tiles = (Cout + bn - 1) / bn;
-  p.k_blocks = 9 * cchunks;
-  p.split_k = 1;
-  p.groups = 1;
-  p.a_mode = OP_TABLE_5D;
-  p.b_mode = OP_KMAJOR_2D;
-  // 5-D view of x: {Cin, parity, W / par, H, B}; par = stride.
-  const int par = stride;
-  unsigned long long dims[5] = {static_cast<unsigned long long>(Cin), static_cast<unsigned long long>(par),
-                                static_cast<unsigned long long>(W / par), static_cast<unsigned long long>(H),
-                                static_cast<unsigned long long>(B)};
-  unsigned long long str[4] = {static_cast<unsigned long long>(Cin) * 2ull,
-                               static_cast<unsigned long long>(Cin) * 2ull * par,
-                               static_cast<unsigned long long>(Cin) * 2ull * W,
-                               static_cast<unsigned long long>(Cin) * 2ull * W * H};
-  unsigned int box[5] = {64, 1, GEMM_BM, 1, 1};
-  int rc = make_tensor_map_bf16(&p.map_a, x, 5, dims, str, box);
-  if (rc != 0) return rc;
-  rc = map_2d(&p.map_b, w, p.K, Cout, p.K, GEMM_BK, bn / ctas);
-  if (rc != 0) return rc - 1000;
-  rc = attach_halos(p, halo_lo, halo_hi, Cin, par, W, H, B, GEMM_BM);
-  if (rc != 0) return rc;
-  // tile (t0, t1, t2) = (w chunk, ho, b): base coordinates
-  p.a_mul0[2] = GEMM_BM;          // w (in units of the strided grid)
-  p.a_mul1[3] = stride;           // h_in = ho * stride + dh
-  p.a_mul2[4] = 1;                // b
+  Tap taps[9];
   for (int tap = 0; tap < 9; ++tap) {
     const int dy = tap / 3, dx = tap % 3;
-    for (int c = 0; c < cchunks; ++c) {
-      short* e = p.ktable[tap * cchunks + c];
-      e[0] = static_cast<short>(c * 64);
-      if (stride == 1) {
-        e[1] = 0;
-        e[2] = static_cast<short>(dx - 1);
-      } else {
-        // w_in = 2*wo + dx - 1: dx=0 -> parity 1 of column wo-1; dx=1 -> parity 0 of wo; dx=2 -> parity 1 of wo
-        e[1] = static_cast<short>(dx == 1 ? 0 : 1);
-        e[2] = static_cast<short>(dx == 0 ? -1 : 0);
-      }
-      e[3] = static_cast<short>(dy - 1);
-    }
+    // stride 2: w_in = 2 wo + dx - 1, so dx = 0 -> parity 1 of column wo - 1; 1 -> parity 0 of wo; 2 -> parity 1 of wo
+    taps[tap].parity = static_cast<short>(stride == 1 || dx == 1 ? 0 : 1);
+    taps[tap].dw = static_cast<short>(stride == 1 ? dx - 1 : (dx == 0 ? -1 : 0));
+    taps[tap].dh = static_cast<short>(dy - 1);
   }
-  fill_epilogue(p, epi);
-  p.epi |= EPI_ROW_CONV;
-  p.out_w = Wo;
-  p.out_h = Ho;
-  p.shuffle_cout = 1;
-  cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);
-  return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+  const int Ho = (stride == 1) ? H : (H + 1) / 2, Wo = (stride == 1) ? W : W / 2;
+  GatherConv c = {x, B, H, W, Cin, stride, Ho, Wo, stride, taps, 9, 1, {0, 9}, w, Cout, epi.C, Ho, Wo, Cout, 1, 0, {}};
+  return gather_conv(c, epi, num_sms, stream, halo_lo, halo_hi);
 }
 
-// Weight gradient of the 3x3 convolution: dw[tap][Cout][Cin] (fp32, pre-zeroed, atomically accumulated)
-//   = sum over output pixels of dy[pix][Cout]^T * x[pix shifted by tap][Cin].
-int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
-                       int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo,
-                       const void* halo_hi, float* bias_grad) {
-  if (stride != 1 && stride != 2) return -11;
-  if (stride == 2 && (W % 2 != 0)) return -12;
-  if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
+// Input gradient of the stride-2 convolution: dy [B, Ho, Wo, Cout] -> dx [B, H, W, Cin] (W even). A row of dx of even index
+// takes part in one tap row (ky = 1), one of odd index in two (ky = 0 of the next dy row, ky = 2), columns alike: four
+// phases of 1, 2, 2 and 4 taps. w: [Cin, 9 * Cout_pad], taps in the order of `order` below.
+int conv3x3_s2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, int W, int Cin, int Cout, void* status,
+                          int num_sms, cudaStream_t stream) {
+  if (W % 2 != 0) return -12;
+  // {ky, kx} per tap, the phase with most taps first: its tiles are the longest
+  static const short order[9][2] = {{0, 0}, {0, 2}, {2, 0}, {2, 2}, {1, 0}, {1, 2}, {0, 1}, {2, 1}, {1, 1}};
+  Tap taps[9];
+  for (int t = 0; t < 9; ++t) taps[t] = {0, static_cast<short>(order[t][1] == 0 ? 1 : 0), static_cast<short>(order[t][0] == 0 ? 1 : 0)};
+  const int Ho = (H + 1) / 2, Wo = W / 2;
+  GatherConv c = {dy, B, Ho, Wo, Cout, 1, Ho, Wo, 1, taps, 9, 4, {0, 4, 6, 8, 9}, w, Cin, dx, H, Wo, Cin, 2, 0,
+                  {{1, 1}, {0, 1}, {1, 0}, {0, 0}}};
+  GemmEpilogue epi = {};
+  epi.alpha = 1.0f;
+  epi.status = status;
+  return gather_conv(c, epi, num_sms, stream, nullptr, nullptr);
+}
+
+// 2x2 / stride-2 transposed convolution: x [B, H, W, Cin] -> y [B, 2H, 2W, Cout]; w: [4 * Cout, Cin_pad], rows (dy, dx, co);
+// bias: [4 * Cout]. One tap, the four output phases side by side in N.
+int convt2x2_fwd_bf16(const void* x, const void* w, const void* bias4, void* y, int B, int H, int W, int Cin, int Cout,
+                      void* status, int num_sms, cudaStream_t stream) {
+  if (Cout % 32 != 0) return -13;             // a 32-column chunk of the epilogue lies inside one phase
+  const Tap tap = {0, 0, 0};
+  GatherConv c = {x, B, H, W, Cin, 1, H, W, 1, &tap, 1, 1, {0, 1}, w, 4 * Cout, y, 2 * H, W, Cout, 2, Cout,
+                  {{0, 0}, {0, 1}, {1, 0}, {1, 1}}};
+  GemmEpilogue epi = {};
+  epi.flags = EPI_BIAS;
+  epi.bias = bias4;
+  epi.alpha = 1.0f;
+  epi.status = status;
+  return gather_conv(c, epi, num_sms, stream, nullptr, nullptr);
+}
+
+// Its input gradient: a 2x2 convolution of stride 2 over dy [B, 2H, 2W, Cout]; w: [Cin, 4 * Cout_pad], taps (dy, dx).
+int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, int W, int Cin, int Cout, void* status,
+                        int num_sms, cudaStream_t stream) {
+  const Tap taps[4] = {{0, 0, 0}, {1, 0, 0}, {0, 0, 1}, {1, 0, 1}};
+  GatherConv c = {dy, B, 2 * H, 2 * W, Cout, 2, H, W, 2, taps, 4, 1, {0, 4}, w, Cin, dx, H, W, Cin, 1, 0, {}};
+  GemmEpilogue epi = {};
+  epi.alpha = 1.0f;
+  epi.status = status;
+  return gather_conv(c, epi, num_sms, stream, nullptr, nullptr);
+}
+
+// Weight gradients: dw[tap][M][N] (fp32, atomically accumulated) = sum over the pixels of `a` [B, Ho, Wo, M] of a[pix]^T
+// times `b` [B, H, W, N] at the pixel's tap (hmul = par = stride of the grid of `a` in `b`).
+static int gather_wgrad(const void* a, const void* b, float* dw, int B, int Ho, int Wo, int M, int H, int W, int N, int stride,
+                        const Tap* taps, int ntaps, int split_k, void* status, int num_sms, cudaStream_t stream,
+                        const void* halo_lo, const void* halo_hi, float* colsum) {
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
-  const int Ho = (stride == 1) ? H : (H + 1) / 2;
-  const int Wo = (stride == 1) ? W : W / 2;
-  const int bn = pick_bn(Cin, Cin % 192 == 0 ? 192 : 128);   // 384 input channels: two tiles of 192, a fifth less operand traffic per flop
-  p.M = Cout;
-  p.N = Cin;
+  const int bn = pick_bn(N, N % 192 == 0 ? 192 : 128);   // 384 columns: two tiles of 192, a fifth less operand traffic per flop
+  p.M = M;
+  p.N = N;
   p.pix_n0 = (Wo + GEMM_BK - 1) / GEMM_BK;
   p.pix_n1 = Ho;
   p.pix_hmul = stride;
   p.k_blocks = p.pix_n0 * Ho * B;
   p.K = p.k_blocks * GEMM_BK;
-  p.m_blocks = (Cout + GEMM_BM - 1) / GEMM_BM;
+  p.m_blocks = (M + GEMM_BM - 1) / GEMM_BM;
   p.num_m_tiles = p.m_blocks;
-  p.num_n_tiles = (Cin + bn - 1) / bn;
-  p.groups = 9;
+  p.num_n_tiles = (N + bn - 1) / bn;
+  p.groups = ntaps;
   if (split_k < 1) split_k = 1;
   if (split_k > p.k_blocks) split_k = p.k_blocks;
   {
@@ -406,57 +484,56 @@ int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, i
   p.split_k = split_k;
   p.a_mode = OP_PIXELS_5D;
   p.b_mode = OP_PIXELS_5D;
-  {
-    unsigned long long dims[5] = {static_cast<unsigned long long>(Cout), 1ull, static_cast<unsigned long long>(Wo),
-                                  static_cast<unsigned long long>(Ho), static_cast<unsigned long long>(B)};
-    unsigned long long str[4] = {static_cast<unsigned long long>(Cout) * 2ull, static_cast<unsigned long long>(Cout) * 2ull,
-                                 static_cast<unsigned long long>(Cout) * 2ull * Wo,
-                                 static_cast<unsigned long long>(Cout) * 2ull * Wo * Ho};
-    unsigned int box[5] = {64, 1, GEMM_BK, 1, 1};
-    int rc = make_tensor_map_bf16(&p.map_a, dy, 5, dims, str, box);
-    if (rc != 0) return rc;
+  int rc = image_map(&p.map_a, a, M, 1, Wo, Ho, B, GEMM_BK);
+  if (rc != 0) return rc;
+  rc = image_map(&p.map_b, b, N, stride, W, H, B, GEMM_BK);
+  if (rc != 0) return rc - 1000;
+  rc = attach_halos(p, halo_lo, halo_hi, N, stride, W, H, B, GEMM_BK);
+  if (rc != 0) return rc;
+  for (int t = 0; t < ntaps; ++t) {
+    p.grp_off[t][0] = taps[t].parity;
+    p.grp_off[t][1] = taps[t].dw;
+    p.grp_off[t][2] = taps[t].dh;
   }
-  {
-    const int par = stride;
-    unsigned long long dims[5] = {static_cast<unsigned long long>(Cin), static_cast<unsigned long long>(par),
-                                  static_cast<unsigned long long>(W / par), static_cast<unsigned long long>(H),
-                                  static_cast<unsigned long long>(B)};
-    unsigned long long str[4] = {static_cast<unsigned long long>(Cin) * 2ull,
-                                 static_cast<unsigned long long>(Cin) * 2ull * par,
-                                 static_cast<unsigned long long>(Cin) * 2ull * W,
-                                 static_cast<unsigned long long>(Cin) * 2ull * W * H};
-    unsigned int box[5] = {64, 1, GEMM_BK, 1, 1};
-    int rc = make_tensor_map_bf16(&p.map_b, x, 5, dims, str, box);
-    if (rc != 0) return rc - 1000;
-  }
-  {
-    const int rc = attach_halos(p, halo_lo, halo_hi, Cin, stride, W, H, B, GEMM_BK);
-    if (rc != 0) return rc;
-  }
-  for (int tap = 0; tap < 9; ++tap) {
-    const int dyy = tap / 3, dxx = tap % 3;
-    short* g = p.grp_off[tap];
-    if (stride == 1) {
-      g[0] = 0;
-      g[1] = static_cast<short>(dxx - 1);
-    } else {
-      g[0] = static_cast<short>(dxx == 1 ? 0 : 1);
-      g[1] = static_cast<short>(dxx == 0 ? -1 : 0);
-    }
-    g[2] = static_cast<short>(dyy - 1);
-  }
-  p.grp_c_stride = static_cast<long long>(Cout) * Cin;
+  p.grp_c_stride = static_cast<long long>(M) * N;
   p.epi = EPI_OUT_F32 | EPI_ATOMIC;
-  p.colsum = bias_grad;
+  p.colsum = colsum;
   p.C = dw;
-  p.ldc = Cin;
+  p.ldc = N;
   p.alpha = 1.0f;
   p.status = static_cast<KernelStatus*>(status);
   p.tile_n0 = 1;
   p.tile_n1 = 1;
-  p.shuffle_cout = 1;
-  cudaError_t e = launch_gemm(p, bn, 1, num_sms, stream);
+  const cudaError_t e = launch_gemm(p, bn, 1, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+}
+
+// 3x3 convolution: dw[tap][Cout][Cin] (pre-zeroed), bias_grad[Cout] += the sums of dy from the same kernel.
+int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
+                       int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo,
+                       const void* halo_hi, float* bias_grad) {
+  if (stride != 1 && stride != 2) return -11;
+  if (stride == 2 && (W % 2 != 0)) return -12;
+  if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
+  Tap taps[9];
+  for (int tap = 0; tap < 9; ++tap) {
+    const int dyy = tap / 3, dxx = tap % 3;
+    taps[tap].parity = static_cast<short>(stride == 1 || dxx == 1 ? 0 : 1);
+    taps[tap].dw = static_cast<short>(stride == 1 ? dxx - 1 : (dxx == 0 ? -1 : 0));
+    taps[tap].dh = static_cast<short>(dyy - 1);
+  }
+  const int Ho = (stride == 1) ? H : (H + 1) / 2, Wo = (stride == 1) ? W : W / 2;
+  return gather_wgrad(dy, x, dw, B, Ho, Wo, Cout, H, W, Cin, stride, taps, 9, split_k, status, num_sms, stream, halo_lo,
+                      halo_hi, bias_grad);
+}
+
+// 2x2 / stride-2 transposed convolution: dw[tap][Cin][Cout] (pre-zeroed) from x [B, H, W, Cin] and dy [B, 2H, 2W, Cout].
+int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int split_k,
+                        void* status, int num_sms, cudaStream_t stream) {
+  if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
+  const Tap taps[4] = {{0, 0, 0}, {1, 0, 0}, {0, 0, 1}, {1, 0, 1}};
+  return gather_wgrad(x, dy, dw, B, H, W, Cin, 2 * H, 2 * W, Cout, 2, taps, 4, split_k, status, num_sms, stream, nullptr,
+                      nullptr, nullptr);
 }
 
 int gemm_stall_counters(unsigned long long* out8, int reset) {

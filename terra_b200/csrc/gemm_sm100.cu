@@ -18,6 +18,8 @@
 //   * their weight gradients (both operands MN-major, contraction over tokens, split-K atomics),
 //   * 3x3 convolutions (stride 1 and 2) as implicit GEMM: A rows gathered by 5-D TMA boxes with
 //     zero fill outside the image, k-blocks enumerate (tap, channel chunk),
+//   * 2x2 / stride-2 transposed convolutions, their input gradient, and the input gradient of the stride-2 3x3
+//     convolution: the same gather with other tap tables, outputs stored to every second pixel through 5-D TMA boxes,
 //   * convolution weight gradients (contraction over pixels, one tile group per tap).
 // Two further instantiations: CTA pairs (a cluster of two drives one cta_group::2 MMA over a 256-row tile, see GemmCfg)
 // and the tensor-parallel forms (A gathered from the peers' buffers, output scattered to the owners' buffers, see
@@ -97,9 +99,14 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int tile, 
   r /= p.num_n_tiles;
   t.m_blk = (r % p.num_m_tiles) * ctas + rank;
   t.grp = r / p.num_m_tiles;
-  const int per = (p.k_blocks + p.split_k - 1) / p.split_k;
-  t.kb_begin = t.split * per;
-  t.kb_end = min(p.k_blocks, t.kb_begin + per);
+  if (p.grp_ranges) {
+    t.kb_begin = p.grp_kb[t.grp];
+    t.kb_end = p.grp_kb[t.grp + 1];
+  } else {
+    const int per = (p.k_blocks + p.split_k - 1) / p.split_k;
+    t.kb_begin = t.split * per;
+    t.kb_end = min(p.k_blocks, t.kb_begin + per);
+  }
   return t;
 }
 
@@ -432,7 +439,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           }
         }
       };
-      auto stage_store = [&](const CUtensorMap* map, const float (&f)[32], int col, int row) {
+      auto stage_store = [&](const CUtensorMap* map, const float (&f)[32], int col, int row, int at_tile) {
         if (lane == 0) {
           if (two_out) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
         }
@@ -450,7 +457,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {   // a group per chunk, also where the rows lie outside the output: the waits count groups
-          if (row < p.M) tma_store_2d(map, dst, col, row);
+          if (p.epi_tma == 2) {
+            // 32 consecutive pixels of an image row (decoded again by this one lane: nothing of it is kept in registers)
+            const TileCoord t = decode_tile(p, at_tile, CTAS, rank);
+            const int phase = p.phase_cols > 0 ? col / p.phase_cols : t.grp;
+            const int w = (t.m_blk % p.tile_n0) * GEMM_BM + q * 32;
+            const int h = (t.m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0];
+            if (t.m_blk < p.m_blocks && w < p.out_w && h < p.out_h)
+              tma_store_5d(map, dst, p.phase_cols > 0 ? col - phase * p.phase_cols : col, p.out_off[phase][1], w, h,
+                           t.m_blk / (p.tile_n0 * p.tile_n1));
+          } else if (row < p.M) {
+            tma_store_2d(map, dst, col, row);
+          }
           bulk_commit_group();
         }
       };
@@ -537,7 +555,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             for (int j = 0; j < 32; j += 2)
               f2_unpack(f2_mul(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2), f[j], f[j + 1]);
           }
-          if (p.epi & EPI_SAVE_PRE) stage_store(&p.map_c2, f, nb, row0);
+          if (p.epi & EPI_SAVE_PRE) stage_store(&p.map_c2, f, nb, row0, tile);
           if (p.epi & EPI_GELU) {
 #pragma unroll
             for (int j = 0; j < 32; j += 2) f2_unpack(gelu_erf2(f2_pack(f[j], f[j + 1])), f[j], f[j + 1]);
@@ -557,7 +575,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             __syncwarp();        // every lane holds its part of the input chunk: its buffer may be refilled
             prefetch_next();
           }
-          stage_store(&p.map_c, f, nb, row0);
+          stage_store(&p.map_c, f, nb, row0, tile);
         }
         if (!released && !failed) release();   // a warp without a chunk in this tile (narrow last column tile)
       }
@@ -569,8 +587,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       const uint32_t aph = (tcount >> 1) & 1u;
       const int n0 = tc.n_blk * BN;
       // ---- tile row -> output row index (-1: outside the output)
-      int col0 = n0;
-      if (p.epi & EPI_ROW_SHUFFLE) col0 = n0 % p.shuffle_cout;
       auto out_row = [&](int r) -> long long {
         if (p.epi & EPI_ROW_CONV) {
           const int t0 = tc.m_blk % p.tile_n0;
@@ -578,15 +594,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           const int t2 = tc.m_blk / (p.tile_n0 * p.tile_n1);
           const int w = t0 * GEMM_BM + r;
           return (w < p.out_w && tc.m_blk < p.m_blocks) ? (static_cast<long long>(t2) * p.tile_n1 + t1) * p.out_w + w : -1;
-        } else if (p.epi & EPI_ROW_SHUFFLE) {
-          const long long g = static_cast<long long>(tc.m_blk) * GEMM_BM + r;
-          if (g >= p.M) return -1;
-          const int w = static_cast<int>(g % p.out_w);
-          const long long t = g / p.out_w;
-          const int h = static_cast<int>(t % p.out_h);
-          const long long b = t / p.out_h;
-          const int qd = n0 / p.shuffle_cout;
-          return ((b * 2 * p.out_h + 2 * h + (qd >> 1)) * 2 * p.out_w) + 2 * w + (qd & 1);
         } else if (PEERS && p.a_peers > 1) {
           const int slot = p.a_interleave ? tc.m_blk % p.a_peers : tc.m_blk / p.a_tiles;
           const int peer = (slot + p.a_first) % p.a_peers;
@@ -601,7 +608,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 #pragma unroll
       for (int i = 0; i < 4; ++i) grows[i] = static_cast<int>(out_row(q * 32 + grow + 8 * i));
       const long long gofs = static_cast<long long>(tc.grp) * p.grp_c_stride;
-      const int ncols_out = (p.epi & EPI_ROW_SHUFFLE) ? p.shuffle_cout : p.N;
+      const int ncols_out = p.N;
 
       // bf16 chunk from global memory, global-side layout (zeros outside the output)
       auto fetch_chunk = [&](const __nv_bfloat16* base, long long ld, int cb, uint4 (&t)[4]) {
@@ -656,8 +663,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           if (c < CHUNKS && n0 + c * 32 < p.N) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              if (grows[i] >= 0 && col0 + c * 32 + gvec * 8 < ncols_out)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(pre_ptr + static_cast<long long>(grows[i]) * pre_ld + col0 + c * 32 + gvec * 8));
+              if (grows[i] >= 0 && n0 + c * 32 + gvec * 8 < ncols_out)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(pre_ptr + static_cast<long long>(grows[i]) * pre_ld + n0 + c * 32 + gvec * 8));
           }
         }
       }
@@ -673,16 +680,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       for (int ci = 0; ci < CPW; ++ci) {
         const int c = part + ci * (GEMM_EPI_WARPS / 4);
         if (c >= CHUNKS || n0 + c * 32 >= p.N) break;   // warp-uniform
-        const int cb = col0 + c * 32;          // first output column of this chunk
-        const int nb = n0 + c * 32;            // first logical column (bias index)
+        const int cb = n0 + c * 32;          // first output column of this chunk
         uint4 pre[4];
         if (pre_aux || pre_res) fetch_chunk(pre_ptr, pre_ld, cb, pre);
         if (has_bias) {
           // one coalesced load per warp and chunk; the 32 values are then read back as broadcast float4
           float b = 0.f;
-          if (nb + lane < p.N)
-            b = (p.epi & EPI_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + nb + lane)
-                                       : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[nb + lane]);
+          if (cb + lane < p.N)
+            b = (p.epi & EPI_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + cb + lane)
+                                       : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[cb + lane]);
           __syncwarp();
           my_bias[lane] = b;
           __syncwarp();

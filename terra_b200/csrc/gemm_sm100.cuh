@@ -22,7 +22,6 @@ enum : int {
   EPI_OUT_F32 = 1 << 5,    // C is fp32
   EPI_ATOMIC = 1 << 6,     // fp32 atomic accumulate into C (split-K)
   EPI_ROW_CONV = 1 << 7,   // rows are (w-chunk, h, b) tiles of an image of width out_w
-  EPI_ROW_SHUFFLE = 1 << 8,// transposed-conv 2x2/s2 pixel shuffle store
   EPI_BIAS_F32 = 1 << 9,   // bias pointer is fp32
   EPI_SILU_MUL = 1 << 10,  // reserved
 };
@@ -66,8 +65,15 @@ struct GemmParams {
   const __nv_bfloat16* residual;
   const __nv_bfloat16* aux;
   long long ldc, ldc2, ldr, ldaux;
-  int out_w, out_h;            // EPI_ROW_CONV / EPI_ROW_SHUFFLE geometry
-  int shuffle_cout;
+  // EPI_ROW_CONV: a tile's rows are 128 consecutive pixels of row t1 of the tile grid. Its outputs go to row
+  // t1 * out_mul + out_off[phase][0] and column parity out_off[phase][1] of an image of out_h rows whose columns are
+  // split by parity when out_mul = 2 (out_w columns of each parity); phase = the tile's group, or with phase_cols > 0 the
+  // output column divided by it (N = phases * phase_cols).
+  int out_w, out_h, out_mul, phase_cols;
+  short out_off[4][2];
+  // k-block ranges per group (groups that contract over different taps), instead of the whole range split by split_k
+  int grp_ranges;
+  int grp_kb[5];
   float alpha;
   KernelStatus* status;
   // Epilogue through TMA (plain row-major bf16 outputs): every epilogue warp stages its 32 x 32 chunk in shared memory in
@@ -77,7 +83,7 @@ struct GemmParams {
   // stages / smem_bytes: the launcher sizes the operand ring with what the epilogue buffers leave.
   float* colsum;               // weight-gradient form: += column sums of operand A over the contraction (see GemmEpilogue)
   CUtensorMap map_c, map_c2, map_in;
-  int epi_tma;
+  int epi_tma;                 // 0: per-lane global accesses, 1: 2-D boxes of rows, 2: 5-D boxes of pixels (EPI_ROW_CONV)
   int epi_bufs;
   int stages;
   int smem_bytes;

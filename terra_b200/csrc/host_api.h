@@ -21,7 +21,6 @@ struct GemmEpilogue {
   const void* aux;
   long long ldc, ldc2, ldr, ldaux;
   float alpha;
-  int out_w, out_h, shuffle_cout;
   void* status;       // KernelStatus* (device), may be null
   // Weight-gradient form (A read MN-major, fp32 atomic output): also accumulate the sums of A's columns over the
   // contraction (sum over tokens of dy[token][n], the bias gradient) into colsum[n] (fp32), from an extra
@@ -63,6 +62,14 @@ int gemm_stall_counters(unsigned long long* out8, int reset);
 int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin, int Cout, int stride,
                      const GemmEpilogue& epi, int num_sms, cudaStream_t stream, const void* halo_lo = nullptr,
                      const void* halo_hi = nullptr);
+int conv3x3_s2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, int W, int Cin, int Cout, void* status,
+                          int num_sms, cudaStream_t stream);
+int convt2x2_fwd_bf16(const void* x, const void* w, const void* bias4, void* y, int B, int H, int W, int Cin, int Cout,
+                      void* status, int num_sms, cudaStream_t stream);
+int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, int W, int Cin, int Cout, void* status,
+                        int num_sms, cudaStream_t stream);
+int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int split_k,
+                        void* status, int num_sms, cudaStream_t stream);
 int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
                        int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo = nullptr,
                        const void* halo_hi = nullptr, float* bias_grad = nullptr);   // bias_grad[Cout] += sums of dy

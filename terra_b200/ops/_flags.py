@@ -7,5 +7,4 @@ EPI_MUL_DGELU = 1 << 4
 EPI_OUT_F32 = 1 << 5
 EPI_ATOMIC = 1 << 6
 EPI_ROW_CONV = 1 << 7
-EPI_ROW_SHUFFLE = 1 << 8
 EPI_BIAS_F32 = 1 << 9

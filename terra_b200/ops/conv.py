@@ -3,8 +3,8 @@
 CUDA: 3x3 convolutions (stride 1 / 2, padding 1) are implicit GEMMs on the tcgen05 kernel - the A operand is
 gathered by 5-D TMA boxes with zero fill outside the image, k-blocks enumerate (tap, channel chunk); the input
 gradient of the stride-1 convolution is the same kernel with flipped, transposed weights; weight gradients
-contract over pixels with one tile group per tap. The 2x2/stride-2 transposed convolution is a GEMM whose
-epilogue stores pixel-shuffled. GroupNorm+SiLU is a statistics pass plus one fused apply pass (optionally adding
+contract over pixels with one tile group per tap. The 2x2/stride-2 transposed convolution, its input gradient and that of
+the stride-2 convolution are the same kernel with other tap tables and outputs stored to every second pixel. GroupNorm+SiLU is a statistics pass plus one fused apply pass (optionally adding
 the block's shortcut), its backward a reduce pass plus an apply pass.
 
 With row-stripe domain parallelism (``dom`` given) halo rows come from the neighbours and GroupNorm statistics
@@ -29,6 +29,7 @@ from .blocks import FUSE_BIAS_GRAD, wgrad_accumulate, bias_grad_accumulate
 from ..utils.nvtx import nvtx_range
 
 GN_EPS = 1e-5
+_MAX_TAP_CHUNKS = 128       # (tap, 64-channel chunk) entries of the implicit GEMM's table (GEMM_MAX_KTABLE)
 
 
 # ------------------------------------------------------------------------------------------------ weight packing
@@ -39,6 +40,26 @@ def pack_conv3x3_weight(w: torch.Tensor) -> torch.Tensor:
     wp = torch.zeros(cout, 9, cpad, device=w.device, dtype=torch.bfloat16)
     wp[:, :, :cin] = w.permute(0, 2, 3, 1).reshape(cout, 9, cin)
     return wp.view(cout, 9 * cpad)
+
+
+def _pack_taps(taps: torch.Tensor) -> torch.Tensor:
+    """[N, taps, C] -> bf16 [N, taps * C_pad], C padded to a multiple of 64 with zeros."""
+    n, t, c = taps.shape
+    cpad = (c + 63) // 64 * 64
+    if c == cpad:
+        return taps.reshape(n, t * c).contiguous()
+    out = torch.zeros(n, t, cpad, device=taps.device, dtype=torch.bfloat16)
+    out[:, :, :c] = taps
+    return out.view(n, t * cpad)
+
+
+# The stride-2 input gradient: taps (ky, kx) by the parity of the input pixel they reach, odd row and column first
+_S2_TAPS = (0, 2, 6, 8, 3, 5, 1, 7, 4)
+
+
+def pack_conv3x3_weight_s2_dgrad(w: torch.Tensor) -> torch.Tensor:
+    cout, cin = w.shape[:2]
+    return _pack_taps(w.reshape(cout, cin, 9)[:, :, list(_S2_TAPS)].permute(1, 2, 0))
 
 
 def pack_conv3x3_weight_dgrad(w: torch.Tensor) -> torch.Tensor:
@@ -152,10 +173,18 @@ def _wgrad_split(B, H, W, stride, Cout, Cin):
 
 
 def _conv3x3_s2_dgrad(dy, w16, H, W, dom, weight=None):
-    """Input gradient of the stride-2 convolution: dcol = dy @ W (tap-major columns) on the tcgen05 GEMM,
-    then one gather kernel over the (at most four) taps that reach each input pixel."""
+    """Input gradient of the stride-2 convolution. One launch: the four parities of the input pixel are four tile groups
+    of the implicit GEMM, with the 1, 2, 2 or 4 taps that reach them. With halo rows to give back (multi-rank stripes), or
+    more channels than the tap table holds: dcol = dy @ W (tap-major columns) on the GEMM, then one gather kernel over the
+    taps that reach each input pixel."""
     B, Ho, Wo, Cout = dy.shape
     Cin = w16.shape[1]
+    if not (dom is not None and dom.world > 1) and 9 * ((Cout + 63) // 64) <= _MAX_TAP_CHUNKS:
+        wp = _packed(weight, w16, "s2dgrad_taps", pack_conv3x3_weight_s2_dgrad) if weight is not None else \
+            pack_conv3x3_weight_s2_dgrad(w16)
+        out = torch.empty(B, H, W, Cin, device=dy.device, dtype=torch.bfloat16)
+        _ext.load().conv3x3_s2_dgrad(dy, wp, out, status_word(dy.device))
+        return out
     build = lambda w: w.permute(0, 2, 3, 1).reshape(Cout, 9 * Cin).contiguous()          # [Cout, (tap, ci)]
     wk = _packed(weight, w16, "s2dgrad", build) if weight is not None else build(w16)
     dcol = gemm(dy.view(-1, Cout), wk, b_mn=True).view(B, Ho, Wo, 9, Cin)     # dcol[p, tap, ci]
@@ -190,6 +219,12 @@ def conv3x3(x, conv: torch.nn.Conv2d, stride: int = 1, dom=None):
 
 
 # ------------------------------------------------------------------------------------------------ transposed conv 2x2 / s2
+def _convt_tiled(Cin, Cout):
+    """The gathered forms: a 32-column chunk of the forward epilogue must lie in one (dy, dx) phase, and the (tap, channel
+    chunk) tables must hold the layer. Other channel counts go through a plain GEMM and permuted copies."""
+    return Cout % 32 == 0 and Cin % 8 == 0 and max(4 * ((Cout + 63) // 64), (Cin + 63) // 64) <= _MAX_TAP_CHUNKS
+
+
 class _ConvT2x2Fn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
@@ -198,50 +233,69 @@ class _ConvT2x2Fn(torch.autograd.Function):
         Cout = weight.shape[1]
         w16 = weight.bf16 if getattr(weight, "bf16", None) is not None else weight.detach().to(torch.bfloat16)
         b16 = bias.bf16 if getattr(bias, "bf16", None) is not None else bias.detach().to(torch.bfloat16)
-        wt = _packed(weight, w16, "convT", lambda w: w.permute(2, 3, 1, 0).reshape(4 * Cout, Cin).contiguous())   # [(dy, dx, co), ci]
         b4 = _packed(bias, b16, "convT_bias", lambda b: b.repeat(4))
         y = torch.empty(B, 2 * H, 2 * W, Cout, device=x.device, dtype=torch.bfloat16)
-        x2 = x.view(-1, Cin)
-        bn = 128 if Cout % 128 == 0 else (64 if Cout % 64 == 0 else 0)
-        if bn:
-            # every BN-wide column tile lies inside one (dy, dx) phase: the epilogue stores it pixel-shuffled
-            flags = F.EPI_BIAS | F.EPI_ROW_SHUFFLE
-            ext.gemm(x2, False, wt, False, y.view(-1, Cout), flags, b4, None, None, None, 1.0, 1, bn,
-                     status_word(x.device), Cout, W, H, 0, [], 0, [], 0, 0, 0, 1, 1)
+        if _convt_tiled(Cin, Cout):
+            # rows (dy, dx, co); the epilogue stores every phase to its pixels
+            wt = _packed(weight, w16, "convT", lambda w: _pack_taps(w.permute(2, 3, 1, 0).reshape(4 * Cout, 1, Cin)))
+            ext.convt2x2(0, x.contiguous(), wt, b4, y, status_word(x.device))
         else:
-            flat = gemm(x2, wt, bias=b4)
+            flat = gemm(x.view(-1, Cin), _convt_flat_weight(weight, w16), bias=b4)
             y.copy_(flat.view(B, H, W, 2, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B, 2 * H, 2 * W, Cout))
         ctx.save_for_backward(x)
-        ctx.p = (wt, Cout, weight, bias)
+        ctx.p = (w16, Cout, weight, bias)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         ext = _ext.load()
         (x,) = ctx.saved_tensors
-        wt, Cout, weight, bias = ctx.p
+        w16, Cout, weight, bias = ctx.p
         B, H, W, Cin = x.shape
-        # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it
-        dyu = dy.view(B, H, 2, W, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B * H * W, 4 * Cout)
+        tiled = _convt_tiled(Cin, Cout)
+        dy = dy.contiguous()
         gw, gb = _arena_grad(weight), _arena_grad(bias)
+        if tiled:
+            # [tap, ci, co] staging -> (Cin, Cout, 2, 2)
+            shape, layout = (4, Cin, Cout), (1, Cout * 4, 4)
+            tiles = 4 * ((Cin + 127) // 128) * ((Cout + 191) // 192 if Cout % 192 == 0 else (Cout + 127) // 128)
+            split = balanced_split(tiles, B * H * ((W + 63) // 64))
+            wgrad = lambda dwt: ext.convt2x2_wgrad(x.contiguous(), dy, dwt, split, status_word(x.device))
+        else:
+            # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it. [tap, co, ci] staging
+            dyu = dy.view(B, H, 2, W, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B * H * W, 4 * Cout)
+            shape, layout = (4, Cout, Cin), (1, 4, Cout * 4)
+            wgrad = lambda dwt: wgrad_accumulate(dyu, x.view(-1, Cin), dwt.view(4 * Cout, Cin))
         if gw is not None:
-            dwt = _zero_scratch(x.device, (4 * Cout, Cin), "convT")
-            wgrad_accumulate(dyu, x.view(-1, Cin), dwt)
-            # [(tap), co, ci] staging -> (Cin, Cout, 2, 2) arena view
-            ext.strided_add(dwt.view(4, Cout, Cin), gw, 1, 4, Cout * 4, True)
+            dwt = _zero_scratch(x.device, shape, "convT")
+            wgrad(dwt)
+            ext.strided_add(dwt, gw, *layout, True)
             dw = None
         else:
-            dwt = torch.zeros(4 * Cout, Cin, device=x.device, dtype=torch.float32)
-            wgrad_accumulate(dyu, x.view(-1, Cin), dwt)
-            dw = dwt.view(2, 2, Cout, Cin).permute(3, 2, 0, 1)
+            dwt = torch.zeros(*shape, device=x.device, dtype=torch.float32)
+            wgrad(dwt)
+            dw = dwt.view(2, 2, *shape[1:]).permute(*((2, 3, 0, 1) if tiled else (3, 2, 0, 1)))
         if gb is not None:
-            ext.colsum(dy.reshape(-1, Cout), gb)
+            ext.colsum(dy.view(-1, Cout), gb)
             db = None
         else:
             db = torch.zeros(Cout, device=x.device, dtype=torch.float32)
-            ext.colsum(dy.reshape(-1, Cout), db)
-        dx = gemm(dyu, wt, b_mn=True).view(B, H, W, Cin) if ctx.needs_input_grad[0] else None
+            ext.colsum(dy.view(-1, Cout), db)
+        dx = None
+        if ctx.needs_input_grad[0]:
+            if tiled:
+                dx = torch.empty(B, H, W, Cin, device=x.device, dtype=torch.bfloat16)
+                wd = _packed(weight, w16, "convT_dgrad", lambda w: _pack_taps(w.permute(0, 2, 3, 1).reshape(Cin, 4, Cout)))
+                ext.convt2x2(1, dy, wd, None, dx, status_word(x.device))
+            else:
+                dx = gemm(dyu, _convt_flat_weight(weight, w16), b_mn=True).view(B, H, W, Cin)
         return dx, dw, db
+
+
+def _convt_flat_weight(weight, w16):
+    """(Cin, Cout, 2, 2) -> [(dy, dx, co), ci]"""
+    cin, cout = w16.shape[:2]
+    return _packed(weight, w16, "convT_flat", lambda w: w.permute(2, 3, 1, 0).reshape(4 * cout, cin).contiguous())
 
 
 def conv_transpose2x2(x, convt: torch.nn.ConvTranspose2d):

@@ -126,7 +126,7 @@ def gemm(
               f"res={None if residual is None else (tuple(residual.shape), residual.dtype, residual.stride())}",
               file=sys.stderr, flush=True)
     ext.gemm(a, a_mn, b, b_mn, out, flags, bias, residual, dgelu_aux, pre, float(alpha), int(split_k), int(bn),
-             status_word(a.device), 0, 0, 0, int(sms), list(a_peers or []), int(rank), list(out_peers or []),
+             status_word(a.device), int(sms), list(a_peers or []), int(rank), list(out_peers or []),
              int(a_flags), int(a_epoch), int(a_budget_ns), int(bool(a_interleave)), int(a_chunks), colsum)
     if save_pre:
         return out, pre

@@ -1,0 +1,71 @@
+"""The strided forms of the implicit GEMM: input gradient of the stride-2 convolution and the three products of the 2x2
+transposed convolution, against fp32 PyTorch, at ragged widths (tiles are 128 pixels wide), odd heights, channel counts with
+a padded chunk, sizes that take CTA pairs, and the channel counts that keep the general path.
+
+Bound: bf16 operands are exact, sums fp32, one rounding of the result: 2^-9 = 0.2 % of the norm; the tests allow 0.4 %."""
+import pytest
+import torch
+import torch.nn.functional as TF
+
+pytestmark = pytest.mark.gpu
+REL = 4e-3
+
+
+def _rand(*shape, scale=1.0):
+    return (torch.randn(*shape, device="cuda") * scale).to(torch.bfloat16)
+
+
+def _rel(got, ref):
+    return ((got.float() - ref.float()).norm() / ref.float().norm()).item()
+
+
+@pytest.mark.parametrize("B,H,W,Cin,Cout", [
+    (1, 2, 2, 64, 64), (1, 1, 4, 32, 64), (2, 13, 200, 96, 96), (1, 33, 258, 96, 192), (1, 8, 16, 40, 72), (1, 64, 300, 384, 384),
+    (1, 512, 512, 192, 64),                # CTA pairs
+    (1, 6, 20, 64, 1024),                  # more channels than the tap table holds: columns and gather
+])
+def test_stride2_input_gradient(B, H, W, Cin, Cout):
+    from terra_b200.ops.conv import _conv3x3_s2_dgrad
+    from terra_b200.ops.gemm import check_status
+
+    torch.manual_seed(0)
+    w, dy = _rand(Cout, Cin, 3, 3, scale=0.05), _rand(B, (H + 1) // 2, W // 2, Cout)
+    dx = _conv3x3_s2_dgrad(dy, w, H, W, None)
+    check_status("cuda")
+    x = torch.zeros(B, Cin, H, W, device="cuda", requires_grad=True)
+    TF.conv2d(x, w.float(), stride=2, padding=1).backward(dy.float().permute(0, 3, 1, 2))
+    # the general path rounds its columns to bf16 as well
+    assert _rel(dx.permute(0, 3, 1, 2), x.grad) < (REL if Cout < 1000 else 2 * REL)
+
+
+@pytest.mark.parametrize("B,H,W,Cin,Cout", [
+    (1, 1, 1, 64, 64), (1, 16, 24, 96, 96), (2, 7, 130, 64, 64), (1, 5, 3, 128, 32), (1, 9, 33, 40, 96), (1, 20, 257, 192, 384),
+    (1, 256, 256, 64, 192),                # CTA pairs
+    (1, 6, 10, 64, 40),                    # phases that a 32-column chunk would straddle: GEMM and permuted copy
+])
+def test_transposed_convolution(B, H, W, Cin, Cout):
+    from terra_b200.ops.conv import conv_transpose2x2
+    from terra_b200.ops.gemm import check_status
+    from terra_b200.utils.flat_params import ParamArena
+
+    torch.manual_seed(1)
+    conv = torch.nn.ConvTranspose2d(Cin, Cout, 2, stride=2).cuda()
+    with torch.no_grad():
+        for p in conv.parameters():
+            p.copy_(p.to(torch.bfloat16).float())
+    ref = torch.nn.ConvTranspose2d(Cin, Cout, 2, stride=2).cuda()
+    ref.load_state_dict(conv.state_dict())
+    plain = torch.nn.ConvTranspose2d(Cin, Cout, 2, stride=2).cuda()        # parameters outside an arena
+    plain.load_state_dict(conv.state_dict())
+    ParamArena(conv)
+    x, dy = _rand(B, H, W, Cin), _rand(B, 2 * H, 2 * W, Cout)
+    xr = x.float().permute(0, 3, 1, 2).detach().requires_grad_(True)
+    yr = ref(xr)
+    yr.backward(dy.float().permute(0, 3, 1, 2))
+    for m in (conv, plain):
+        xc = x.clone().requires_grad_(True)
+        y = conv_transpose2x2(xc, m)
+        y.backward(dy)
+        check_status("cuda")
+        assert _rel(y.permute(0, 3, 1, 2), yr) < REL and _rel(xc.grad.permute(0, 3, 1, 2), xr.grad) < REL
+        assert _rel(m.weight.grad, ref.weight.grad) < REL and _rel(m.bias.grad, ref.bias.grad) < REL

@@ -199,6 +199,28 @@ void unpatchify_crop(const torch::Tensor& patches, const c10::optional<torch::Te
            "unpatchify_crop");
 }
 
+// w: contiguous bf16 storage that every index of the packing stays inside; out: [N1 * N2, T * Cpad] bf16
+void pack_taps(const torch::Tensor& w, torch::Tensor& out, int64_t n1, int64_t s1, int64_t n2, int64_t s2, int64_t channels,
+               int64_t sc, const std::vector<int64_t>& offsets) {
+  const int64_t T = static_cast<int64_t>(offsets.size());
+  need(w.is_cuda() && w.is_contiguous() && w.scalar_type() == torch::kBFloat16, "pack_taps: w bf16 contiguous");
+  need(T >= 1 && T <= 9 && out.is_contiguous() && out.scalar_type() == torch::kBFloat16 && out.dim() == 2 &&
+           out.size(0) == n1 * n2 && out.size(1) % (2 * T) == 0 && channels >= 1 && channels <= out.size(1) / T,
+       "pack_taps: out bf16 [n1 * n2, T * Cpad]");
+  int off[9], top = 0;
+  for (int64_t t = 0; t < T; ++t) {
+    need(offsets[t] >= 0, "pack_taps: offsets");
+    off[t] = static_cast<int>(offsets[t]);
+    top = off[t] > top ? off[t] : top;
+  }
+  need(s1 >= 0 && s2 >= 0 && sc >= 0 && (n1 - 1) * s1 + (n2 - 1) * s2 + (channels - 1) * sc + top < w.numel(), "pack_taps: range");
+  const c10::cuda::CUDAGuard guard(w.device());
+  tb::note_launch();
+  rc_check(tb::pack_taps_bf16(w.data_ptr(), out.data_ptr(), static_cast<int>(n1), static_cast<int>(n2), static_cast<int>(T),
+                              static_cast<int>(channels), static_cast<int>(out.size(1) / T), s1, s2, sc, off, cur_stream()),
+           "pack_taps");
+}
+
 void grad_inspect(const torch::Tensor& grad, torch::Tensor& out2) {
   need(grad.is_cuda() && grad.is_contiguous() && grad.scalar_type() == torch::kFloat32, "grad_inspect: fp32 contiguous");
   need(out2.scalar_type() == torch::kFloat32 && out2.numel() >= 2, "grad_inspect: out2 fp32 [2]");
@@ -381,6 +403,7 @@ void bind_elementwise(pybind11::module_& m) {
   m.def("adamw_step", &adamw_step);
   m.def("pad_patchify", &pad_patchify);
   m.def("unpatchify_crop", &unpatchify_crop);
+  m.def("pack_taps", &pack_taps);
   m.def("grad_inspect", &grad_inspect);
   m.def("attn_rowdot", &attn_rowdot);
   m.def("sum_slots", &sum_slots, pybind11::arg("slots"), pybind11::arg("out"), pybind11::arg("bias") = pybind11::none(),

@@ -33,24 +33,26 @@ _MAX_TAP_CHUNKS = 128       # (tap, 64-channel chunk) entries of the implicit GE
 
 
 # ------------------------------------------------------------------------------------------------ weight packing
+def _pack_taps(w, n1, s1, n2, s2, channels, sc, offsets):
+    """bf16 ``[n1 * n2, taps * C_pad]`` with ``out[i * n2 + j, t, c] = w.flatten()[i * s1 + j * s2 + c * sc + offsets[t]]``, the
+    channels padded to a multiple of 64 with zeros."""
+    cpad, taps = (channels + 63) // 64 * 64, len(offsets)
+    if w.is_cuda and w.dtype == torch.bfloat16:
+        out = torch.empty(n1 * n2, taps * cpad, device=w.device, dtype=torch.bfloat16)
+        _ext.load().pack_taps(w.contiguous(), out, n1, s1, n2, s2, channels, sc, list(offsets))
+        return out
+    steps = [(n1, s1), (n2, s2), (1, 0), (channels, sc)]
+    at = sum(torch.arange(n, device=w.device).view([-1 if d == e else 1 for e in range(4)]) * s for d, (n, s) in enumerate(steps))
+    at = at + torch.tensor(list(offsets), device=w.device).view(1, 1, -1, 1)
+    out = torch.zeros(n1 * n2, taps, cpad, device=w.device, dtype=torch.bfloat16)
+    out[:, :, :channels] = w.reshape(-1)[at.reshape(-1)].view(n1 * n2, taps, channels)
+    return out.view(n1 * n2, taps * cpad)
+
+
 def pack_conv3x3_weight(w: torch.Tensor) -> torch.Tensor:
     """(Cout, Cin, 3, 3) -> bf16 [Cout, 9 * Cin_pad], tap-major, Cin padded to a multiple of 64 with zeros."""
     cout, cin = w.shape[:2]
-    cpad = (cin + 63) // 64 * 64
-    wp = torch.zeros(cout, 9, cpad, device=w.device, dtype=torch.bfloat16)
-    wp[:, :, :cin] = w.permute(0, 2, 3, 1).reshape(cout, 9, cin)
-    return wp.view(cout, 9 * cpad)
-
-
-def _pack_taps(taps: torch.Tensor) -> torch.Tensor:
-    """[N, taps, C] -> bf16 [N, taps * C_pad], C padded to a multiple of 64 with zeros."""
-    n, t, c = taps.shape
-    cpad = (c + 63) // 64 * 64
-    if c == cpad:
-        return taps.reshape(n, t * c).contiguous()
-    out = torch.zeros(n, t, cpad, device=taps.device, dtype=torch.bfloat16)
-    out[:, :, :c] = taps
-    return out.view(n, t * cpad)
+    return _pack_taps(w, 1, 0, cout, cin * 9, cin, 9, range(9))
 
 
 # The stride-2 input gradient: taps (ky, kx) by the parity of the input pixel they reach, odd row and column first
@@ -59,14 +61,13 @@ _S2_TAPS = (0, 2, 6, 8, 3, 5, 1, 7, 4)
 
 def pack_conv3x3_weight_s2_dgrad(w: torch.Tensor) -> torch.Tensor:
     cout, cin = w.shape[:2]
-    return _pack_taps(w.reshape(cout, cin, 9)[:, :, list(_S2_TAPS)].permute(1, 2, 0))
+    return _pack_taps(w, 1, 0, cin, 9, cout, cin * 9, _S2_TAPS)
 
 
 def pack_conv3x3_weight_dgrad(w: torch.Tensor) -> torch.Tensor:
     """Weights of the stride-1 input-gradient convolution: taps flipped, channels swapped."""
-    return pack_conv3x3_weight(w.flip(2, 3).transpose(0, 1))
-
-
+    cout, cin = w.shape[:2]
+    return _pack_taps(w, 1, 0, cin, 9, cout, cin * 9, range(8, -1, -1))
 
 
 _SCRATCH = {}
@@ -237,7 +238,7 @@ class _ConvT2x2Fn(torch.autograd.Function):
         y = torch.empty(B, 2 * H, 2 * W, Cout, device=x.device, dtype=torch.bfloat16)
         if _convt_tiled(Cin, Cout):
             # rows (dy, dx, co); the epilogue stores every phase to its pixels
-            wt = _packed(weight, w16, "convT", lambda w: _pack_taps(w.permute(2, 3, 1, 0).reshape(4 * Cout, 1, Cin)))
+            wt = _packed(weight, w16, "convT", lambda w: _pack_taps(w, 4, 1, Cout, 4, Cin, 4 * Cout, (0,)))
             ext.convt2x2(0, x.contiguous(), wt, b4, y, status_word(x.device))
         else:
             flat = gemm(x.view(-1, Cin), _convt_flat_weight(weight, w16), bias=b4)
@@ -285,7 +286,7 @@ class _ConvT2x2Fn(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             if tiled:
                 dx = torch.empty(B, H, W, Cin, device=x.device, dtype=torch.bfloat16)
-                wd = _packed(weight, w16, "convT_dgrad", lambda w: _pack_taps(w.permute(0, 2, 3, 1).reshape(Cin, 4, Cout)))
+                wd = _packed(weight, w16, "convT_dgrad", lambda w: _pack_taps(w, 1, 0, Cin, 4 * Cout, Cout, 4, range(4)))
                 ext.convt2x2(1, dy, wd, None, dx, status_word(x.device))
             else:
                 dx = gemm(dyu, _convt_flat_weight(weight, w16), b_mn=True).view(B, H, W, Cin)

@@ -213,6 +213,7 @@ void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tens
 
 void bind_elementwise(pybind11::module_& m);
 void bind_attention(pybind11::module_& m);
+void bind_halves(pybind11::module_& m);
 void bind_copy_engine(pybind11::module_& m);
 void bind_comm(pybind11::module_& m);
 
@@ -241,6 +242,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("convt2x2_wgrad", &convt2x2_wgrad, "2x2 / stride-2 transposed convolution: weight gradient (fp32 atomics)");
   bind_elementwise(m);
   bind_attention(m);
+  bind_halves(m);
   bind_copy_engine(m);
   bind_comm(m);
 }

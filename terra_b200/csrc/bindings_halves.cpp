@@ -1,0 +1,268 @@
+// The transformer block halves as one native call per direction: the same launches in the same order as the Python form
+// (which the multi-rank layouts use), without the interpreter between them. A small layer is bound by its launches: on 512
+// rows of width 96 the Python form spent about 20 us per launch on the host against 1 to 10 us of kernel time.
+#include <algorithm>
+#include <stdexcept>
+#include <string>
+#include <vector>
+#include <torch/extension.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include "host_api.h"
+#include "launch_count.h"
+
+namespace {
+
+using torch::Tensor;
+using OptTensor = c10::optional<torch::Tensor>;
+
+cudaStream_t cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+void need(bool ok, const char* what) {
+  if (!ok) throw std::runtime_error(std::string("terra_b200: ") + what);
+}
+void rc_check(int rc, const char* what) {
+  if (rc != 0) throw std::runtime_error(std::string("terra_b200: ") + what + " failed with code " + std::to_string(rc));
+}
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+bool rows_bf16(const Tensor& t) {
+  return t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 2 && t.is_contiguous();
+}
+// rows of any pitch (a product's operand)
+bool rows_pitched(const Tensor& t) {
+  return t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 2 && t.stride(1) == 1;
+}
+bool vec(const Tensor& t, at::ScalarType ty, int64_t n) { return t.is_cuda() && t.scalar_type() == ty && t.is_contiguous() && t.numel() == n; }
+
+struct Epi {
+  int flags = 0;
+  const Tensor* bias = nullptr;
+  const Tensor* residual = nullptr;
+  const Tensor* aux = nullptr;
+  const Tensor* pre = nullptr;
+};
+
+// out [M, N] = epilogue(a [M, K] * w), w [N, K] or, with b_mn, [K, N]
+void product(const Tensor& a, const Tensor& w, bool b_mn, const Tensor& out, const Epi& e, const Tensor& status) {
+  tb::GemmOperand A{a.data_ptr(), a.stride(0), 0}, B{w.data_ptr(), w.stride(0), b_mn ? 1 : 0};
+  tb::GemmEpilogue g{};
+  g.flags = e.flags;
+  g.C = out.data_ptr();
+  g.ldc = out.stride(0);
+  if (e.bias != nullptr) {
+    g.flags |= tb::EPI_BIAS;
+    g.bias = e.bias->data_ptr();
+  }
+  if (e.residual != nullptr) {
+    g.flags |= tb::EPI_RESIDUAL;
+    g.residual = e.residual->data_ptr();
+    g.ldr = e.residual->stride(0);
+  }
+  if (e.aux != nullptr) {
+    g.flags |= tb::EPI_MUL_DGELU;
+    g.aux = e.aux->data_ptr();
+    g.ldaux = e.aux->stride(0);
+  }
+  if (e.pre != nullptr) {
+    g.flags |= tb::EPI_SAVE_PRE;
+    g.C2 = e.pre->data_ptr();
+    g.ldc2 = e.pre->stride(0);
+  }
+  g.alpha = 1.0f;
+  g.status = status.data_ptr();
+  need(a.size(1) == w.size(b_mn ? 0 : 1) && out.size(0) == a.size(0) && out.size(1) == w.size(b_mn ? 1 : 0), "block half: operand shapes");
+  tb::note_launch();
+  rc_check(tb::gemm_bf16(A, B, a.size(0), out.size(1), a.size(1), g, 1, 0, sm_count(), cur_stream()), "gemm");
+}
+
+void column_sums(const Tensor& dy, const Tensor& out) {
+  const int64_t parts = (dy.size(0) + tb::colsum_rows_per_block() - 1) / tb::colsum_rows_per_block();
+  auto partials = torch::empty({parts, dy.size(1)}, dy.options().dtype(torch::kFloat32));
+  tb::note_launch();
+  rc_check(tb::colsum_bf16(dy.data_ptr(), out.data_ptr<float>(), partials.data_ptr<float>(), dy.size(0), dy.size(1), dy.stride(0),
+                           cur_stream()),
+           "colsum");
+}
+
+// grad_w [N, K] (fp32) += dy [M, N]^T x [M, K]; grad_b [N] += column sums of dy, from the same kernel (`fuse_bias`: a
+// 16-column MMA of the dy tiles against ones) where its accumulators fit beside the tile's (widths up to 192).
+void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTensor& grad_b, bool fuse_bias, const Tensor& status) {
+  need(rows_pitched(dy) && rows_pitched(x) && dy.size(0) == x.size(0) && grad_w.scalar_type() == torch::kFloat32 && grad_w.dim() == 2 &&
+           grad_w.is_contiguous() && grad_w.size(0) == dy.size(1) && grad_w.size(1) == x.size(1),
+       "wgrad: dy [M, N], x [M, K] bf16, grad_w [N, K] fp32");
+  need(!grad_b.has_value() || vec(*grad_b, torch::kFloat32, dy.size(1)), "wgrad: grad_b fp32 [N]");
+  const c10::cuda::CUDAGuard guard(dy.device());
+  const int64_t M = dy.size(0), N = dy.size(1), K = x.size(1);
+  bool sums = grad_b.has_value();
+  const bool wide = K % 256 == 0 && K >= 1024 && (!(sums && fuse_bias) || K % 192 != 0);
+  const int bn = wide ? 256 : (K % 192 == 0 ? 192 : 128);
+  if (sums && (!fuse_bias || bn == 256)) {
+    column_sums(dy, *grad_b);
+    sums = false;
+  }
+  // enough splits of the contraction to fill the GPU once, never more than its 64-wide blocks
+  const int64_t tiles = ((N + 127) / 128) * ((K + bn - 1) / bn), blocks = (M + 63) / 64;
+  const int64_t split = std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>(1, sm_count() / tiles), blocks));
+  tb::GemmOperand A{dy.data_ptr(), dy.stride(0), 1}, B{x.data_ptr(), x.stride(0), 1};
+  tb::GemmEpilogue g{};
+  g.flags = tb::EPI_OUT_F32 | tb::EPI_ATOMIC;
+  g.C = grad_w.data_ptr();
+  g.ldc = grad_w.stride(0);
+  g.alpha = 1.0f;
+  g.status = status.data_ptr();
+  g.colsum = sums ? grad_b->data_ptr<float>() : nullptr;
+  tb::note_launch();
+  rc_check(tb::gemm_bf16(A, B, N, K, M, g, static_cast<int>(split), bn, sm_count(), cur_stream()), "gemm (weight gradient)");
+}
+
+struct Norm {
+  Tensor xn, mean, rstd;
+};
+Norm norm_fwd(const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
+  need(rows_bf16(x) && vec(w, torch::kBFloat16, x.size(1)) && vec(b, torch::kBFloat16, x.size(1)), "block half: x [rows, C], norm weights bf16");
+  Norm n;
+  n.xn = torch::empty_like(x);
+  n.mean = torch::empty({x.size(0)}, x.options().dtype(torch::kFloat32));
+  n.rstd = torch::empty_like(n.mean);
+  tb::note_launch();
+  rc_check(tb::layernorm_fwd(x.data_ptr(), w.data_ptr(), b.data_ptr(), n.xn.data_ptr(), n.mean.data_ptr<float>(),
+                             n.rstd.data_ptr<float>(), x.size(0), static_cast<int>(x.size(1)), static_cast<float>(eps), cur_stream()),
+           "layernorm_fwd");
+  return n;
+}
+Tensor norm_bwd(const Tensor& dxn, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, const Tensor& gw,
+                const Tensor& gb, const Tensor& dres) {
+  need(vec(gw, torch::kFloat32, x.size(1)) && vec(gb, torch::kFloat32, x.size(1)), "block half: norm gradients fp32");
+  Tensor dx = torch::empty_like(x);
+  tb::note_launch();
+  rc_check(tb::layernorm_bwd(dxn.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(),
+                             gw.data_ptr<float>(), gb.data_ptr<float>(), dres.data_ptr(), x.size(0), static_cast<int>(x.size(1)),
+                             cur_stream()),
+           "layernorm_bwd");
+  return dx;
+}
+
+// Window geometry of a rank that owns every window and token: {B, nWh, nWw, wh, ww, heads, sh, sw, use_mask}
+tb::WindowAttnArgs window_args(const std::vector<int64_t>& g, int64_t C, const OptTensor& table, double scale, int64_t rows) {
+  need(g.size() == 9 && g[5] > 0, "block half: window geometry");
+  tb::WindowAttnArgs a{};
+  a.B = static_cast<int>(g[0]);
+  a.nWh = static_cast<int>(g[1]);
+  a.nWw = static_cast<int>(g[2]);
+  a.wh = static_cast<int>(g[3]);
+  a.ww = static_cast<int>(g[4]);
+  a.num_heads = static_cast<int>(g[5]);
+  a.sh = static_cast<int>(g[6]);
+  a.sw = static_cast<int>(g[7]);
+  a.use_mask = g[8] != 0 ? 1 : 0;
+  a.tp = a.n_wg = a.sp = 1;
+  a.win_start[1] = a.nWh * a.nWw;
+  a.shardN = a.wh * a.ww;
+  a.C = static_cast<int>(C);
+  a.scale = static_cast<float>(scale);
+  need(static_cast<int64_t>(a.B) * a.win_start[1] * a.shardN == rows, "block half: rows = B * windows * tokens");
+  if (table.has_value()) {
+    need(vec(*table, torch::kFloat32, static_cast<int64_t>(2 * a.wh - 1) * (2 * a.ww - 1) * a.num_heads), "block half: bias table fp32");
+    a.bias_table = table->data_ptr<float>();
+  }
+  return a;
+}
+
+// -> y, mean, rstd, xn, qkv, o
+std::vector<Tensor> attn_half_fwd(const Tensor& x, const Tensor& ln_w, const Tensor& ln_b, const Tensor& qkv_w, const Tensor& qkv_b,
+                                  const Tensor& proj_w, const Tensor& proj_b, const OptTensor& table,
+                                  const std::vector<int64_t>& geo, double scale, double eps, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  Norm n = norm_fwd(x, ln_w, ln_b, eps);
+  const int64_t rows = x.size(0), C = x.size(1);
+  tb::WindowAttnArgs a = window_args(geo, C, table, scale, rows);
+  Tensor qkv = torch::empty({rows, 3 * C}, x.options()), o = torch::empty_like(x), y = torch::empty_like(x);
+  Epi e;
+  e.bias = &qkv_b;
+  product(n.xn, qkv_w, false, qkv, e, status);
+  a.qkv[0] = qkv.data_ptr();
+  a.out[0] = o.data_ptr();
+  tb::note_launch();
+  rc_check(tb::window_attn_fwd(a, cur_stream()), "window_attn_fwd");
+  e.bias = &proj_b;
+  e.residual = &x;
+  product(o, proj_w, false, y, e, status);
+  return {y, n.mean, n.rstd, n.xn, qkv, o};
+}
+
+// -> dx; the parameter gradients (fp32) are accumulated in place
+Tensor attn_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, const Tensor& rstd, const Tensor& xn, const Tensor& qkv,
+                     const Tensor& o, const Tensor& ln_w, const Tensor& qkv_w, const Tensor& proj_w, const OptTensor& table,
+                     const Tensor& ln_wg, const Tensor& ln_bg, const Tensor& qkv_wg, const Tensor& qkv_bg, const Tensor& proj_wg,
+                     const Tensor& proj_bg, const OptTensor& table_g, const std::vector<int64_t>& geo, double scale, bool fuse_bias,
+                     const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  need(rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: dy like x");
+  tb::WindowAttnArgs a = window_args(geo, x.size(1), table, scale, x.size(0));
+  wgrad(dy, o, proj_wg, proj_bg, fuse_bias, status);
+  Tensor dout = torch::empty_like(x), dqkv = torch::empty_like(qkv), dxn = torch::empty_like(x);
+  product(dy, proj_w, true, dout, Epi(), status);
+  a.qkv[0] = qkv.data_ptr();
+  a.dout[0] = dout.data_ptr();
+  a.dqkv[0] = dqkv.data_ptr();
+  if (table_g.has_value()) {
+    need(table.has_value() && vec(*table_g, torch::kFloat32, table->numel()), "block half: bias table gradient fp32");
+    a.dbias_table = table_g->data_ptr<float>();
+  }
+  tb::note_launch();
+  rc_check(tb::window_attn_bwd(a, cur_stream()), "window_attn_bwd");
+  wgrad(dqkv, xn, qkv_wg, qkv_bg, fuse_bias, status);
+  product(dqkv, qkv_w, true, dxn, Epi(), status);
+  return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy);
+}
+
+// -> y, mean, rstd, xn, pre, act
+std::vector<Tensor> mlp_half_fwd(const Tensor& x, const Tensor& ln_w, const Tensor& ln_b, const Tensor& fc1_w, const Tensor& fc1_b,
+                                 const Tensor& fc2_w, const Tensor& fc2_b, double eps, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  Norm n = norm_fwd(x, ln_w, ln_b, eps);
+  Tensor pre = torch::empty({x.size(0), fc1_w.size(0)}, x.options()), act = torch::empty_like(pre), y = torch::empty_like(x);
+  Epi e;
+  e.flags = tb::EPI_GELU;
+  e.bias = &fc1_b;
+  e.pre = &pre;
+  product(n.xn, fc1_w, false, act, e, status);
+  Epi r;
+  r.bias = &fc2_b;
+  r.residual = &x;
+  product(act, fc2_w, false, y, r, status);
+  return {y, n.mean, n.rstd, n.xn, pre, act};
+}
+
+Tensor mlp_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, const Tensor& rstd, const Tensor& xn, const Tensor& pre,
+                    const Tensor& act, const Tensor& ln_w, const Tensor& fc1_w, const Tensor& fc2_w, const Tensor& ln_wg,
+                    const Tensor& ln_bg, const Tensor& fc1_wg, const Tensor& fc1_bg, const Tensor& fc2_wg, const Tensor& fc2_bg,
+                    bool fuse_bias, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  need(rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: dy like x");
+  wgrad(dy, act, fc2_wg, fc2_bg, fuse_bias, status);
+  Tensor dpre = torch::empty_like(pre), dxn = torch::empty_like(x);
+  Epi e;
+  e.aux = &pre;
+  product(dy, fc2_w, true, dpre, e, status);
+  wgrad(dpre, xn, fc1_wg, fc1_bg, fuse_bias, status);
+  product(dpre, fc1_w, true, dxn, Epi(), status);
+  return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy);
+}
+
+}  // namespace
+
+void bind_halves(pybind11::module_& m) {
+  m.def("wgrad", &wgrad, "weight (and bias) gradient of a linear layer, accumulated in fp32");
+  m.def("attn_half_fwd", &attn_half_fwd);
+  m.def("attn_half_bwd", &attn_half_bwd);
+  m.def("mlp_half_fwd", &mlp_half_fwd);
+  m.def("mlp_half_bwd", &mlp_half_bwd);
+}

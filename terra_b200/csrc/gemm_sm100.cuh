@@ -1,6 +1,7 @@
 // Parameter block shared by the host launcher and the tcgen05 GEMM / implicit-GEMM kernel.
 #pragma once
 #include "common.cuh"
+#include "host_api.h"   // EPI_* flags
 
 namespace tb {
 
@@ -11,19 +12,6 @@ enum : int {
   OP_TABLE_5D = 2,     // K-major rows gathered from a 5-D tensor (implicit-GEMM convolution):
                        //   coords = tile base + per-k-block offset table
   OP_PIXELS_5D = 3,    // MN-major, contraction runs over pixels of a 5-D tensor (conv weight grad)
-};
-
-enum : int {
-  EPI_BIAS = 1 << 0,       // + bias[col]
-  EPI_GELU = 1 << 1,       // exact-erf GELU after bias
-  EPI_SAVE_PRE = 1 << 2,   // also store the pre-activation (bf16) to C2
-  EPI_RESIDUAL = 1 << 3,   // + R[row][col]
-  EPI_MUL_DGELU = 1 << 4,  // acc *= gelu'(aux[row][col])      (backward of fc1's GELU)
-  EPI_OUT_F32 = 1 << 5,    // C is fp32
-  EPI_ATOMIC = 1 << 6,     // fp32 atomic accumulate into C (split-K)
-  EPI_ROW_CONV = 1 << 7,   // rows are (w-chunk, h, b) tiles of an image of width out_w
-  EPI_BIAS_F32 = 1 << 9,   // bias pointer is fp32
-  EPI_SILU_MUL = 1 << 10,  // reserved
 };
 
 constexpr int GEMM_BM = 128;

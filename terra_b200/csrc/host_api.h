@@ -12,8 +12,22 @@ struct GemmOperand {
   int mn_major;      // 0: stored [rows][K] (K contiguous); 1: stored [K][rows] (rows contiguous)
 };
 
+// What the GEMM epilogue does to an accumulator (GemmEpilogue::flags)
+enum : int {
+  EPI_BIAS = 1 << 0,       // + bias[col]
+  EPI_GELU = 1 << 1,       // exact-erf GELU after bias
+  EPI_SAVE_PRE = 1 << 2,   // also store the pre-activation (bf16) to C2
+  EPI_RESIDUAL = 1 << 3,   // + R[row][col]
+  EPI_MUL_DGELU = 1 << 4,  // acc *= gelu'(aux[row][col])      (backward of fc1's GELU)
+  EPI_OUT_F32 = 1 << 5,    // C is fp32
+  EPI_ATOMIC = 1 << 6,     // fp32 atomic accumulate into C (split-K)
+  EPI_ROW_CONV = 1 << 7,   // rows are (w-chunk, h, b) tiles of an image of width out_w
+  EPI_BIAS_F32 = 1 << 9,   // bias pointer is fp32
+  EPI_SILU_MUL = 1 << 10,  // reserved
+};
+
 struct GemmEpilogue {
-  int flags;          // EPI_* bit mask (gemm_sm100.cuh)
+  int flags;          // EPI_* bit mask
   void* C;
   void* C2;
   const void* bias;

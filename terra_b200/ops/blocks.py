@@ -23,8 +23,8 @@ import torch
 import torch.nn.functional as TF
 
 from .. import _ext
-from .attention import (MAX_KERNEL_WINDOW_TOKENS, WindowGeometry, launch_window_attn_bwd, launch_window_attn_fwd,
-                        window_attention)
+from .attention import (MAX_KERNEL_WINDOW_TOKENS, WindowGeometry, attn_backward_impl, attn_forward_impl,
+                        launch_window_attn_bwd, launch_window_attn_fwd, window_attention)
 from .gemm import gemm, status_word
 from .packed import fp32_values
 from ..utils.nvtx import nvtx_range
@@ -37,27 +37,10 @@ LN_EPS = 1e-5
 FUSE_BIAS_GRAD = os.environ.get("TERRA_FUSED_BIAS_GRAD", "1") == "1"
 
 
-def _split_k_for(m_tiles_n_tiles: int, k_blocks: int, sms: int = 148) -> int:
-    """Enough K splits to fill the GPU once, never more than the number of 64-wide k-blocks."""
-    want = max(1, sms // max(1, m_tiles_n_tiles))
-    return max(1, min(want, k_blocks))
-
-
 def wgrad_accumulate(dy: torch.Tensor, x: torch.Tensor, grad_w: torch.Tensor, grad_b: torch.Tensor = None) -> None:
     """grad_w[N, K] (fp32) += dy[M, N]^T @ x[M, K]; with ``grad_b``: grad_b[N] (fp32) += column sums of dy, from the
     same kernel (a 16-column MMA of the dy tiles against ones), which saves the separate pass over dy."""
-    N, K = grad_w.shape
-    if grad_b is not None and not FUSE_BIAS_GRAD:
-        bias_grad_accumulate(dy, grad_b)
-        grad_b = None
-    wide = K % 256 == 0 and K >= 1024 and (grad_b is None or K % 192 != 0)     # the sums need tile widths <= 192
-    bn = 256 if wide else (192 if K % 192 == 0 else 128)
-    tiles = ((N + 127) // 128) * ((K + bn - 1) // bn)
-    split = _split_k_for(tiles, (dy.shape[0] + 63) // 64)
-    if grad_b is not None and bn == 256:
-        bias_grad_accumulate(dy, grad_b)
-        grad_b = None
-    gemm(dy, x, a_mn=True, b_mn=True, out=grad_w, accumulate=True, split_k=split, bn=bn, colsum=grad_b)
+    _ext.load().wgrad(dy, x, grad_w, grad_b, FUSE_BIAS_GRAD, status_word(dy.device))
 
 
 def bias_grad_accumulate(dy: torch.Tensor, grad_b: torch.Tensor) -> None:
@@ -94,11 +77,28 @@ def _views(p: torch.nn.Parameter):
     return p.bf16, p.grad
 
 
+def _native_half(comm, geo: WindowGeometry, impl: str) -> bool:
+    """One native call runs the half when this rank owns every window and token and the small-window kernels are the
+    selected ones (not in the bounds-checked build, whose reports go through the Python launches)."""
+    return comm is None and impl == "mma" and geo.sp == 1 and geo.tp == 1 and geo.n_wg == 1 and not _ext.DEBUG_BOUNDS
+
+
+def _native_geometry(geo: WindowGeometry, num_heads, shifted, use_mask):
+    return [geo.B, geo.nWh, geo.nWw, geo.wh, geo.ww, num_heads, *geo.shift(shifted), int(bool(use_mask and shifted))]
+
+
 class _AttnHalfFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, anchor, pk: ParamPack, geo: WindowGeometry, num_heads, shifted, use_mask, scale, comm):
         ext = _ext.load()
         C = x.shape[1]
+        ctx.pk, ctx.geo, ctx.args, ctx.comm = pk, geo, (num_heads, shifted, use_mask, scale), comm
+        if _native_half(comm, geo, attn_forward_impl(geo.N)):
+            y, mean, rstd, xn, qkv, o = ext.attn_half_fwd(
+                x, pk.ln_w, pk.ln_b, pk.qkv_w, pk.qkv_b, pk.proj_w, pk.proj_b, pk.bias_table,
+                _native_geometry(geo, num_heads, shifted, use_mask), scale, LN_EPS, status_word(x.device))
+            ctx.save_for_backward(x, mean, rstd, xn, qkv, o)
+            return y
         xn, mean, rstd = layernorm_cuda(x, pk.ln_w, pk.ln_b)
         if comm is not None:
             qkv = comm.alloc_qkv(x.shape[0], 3 * C)
@@ -115,7 +115,6 @@ class _AttnHalfFn(torch.autograd.Function):
             o, qkv = comm.attn_forward_done(o, qkv, shifted)
         y = gemm(o, pk.proj_w, bias=pk.proj_b, residual=x)
         ctx.save_for_backward(x, mean, rstd, xn, qkv, o)
-        ctx.pk, ctx.geo, ctx.args, ctx.comm = pk, geo, (num_heads, shifted, use_mask, scale), comm
         return y
 
     @staticmethod
@@ -126,6 +125,12 @@ class _AttnHalfFn(torch.autograd.Function):
         num_heads, shifted, use_mask, scale = ctx.args
         C = x.shape[1]
         dy = dy.contiguous()
+        if _native_half(comm, geo, attn_backward_impl(geo.N, C // num_heads)):
+            dx = ext.attn_half_bwd(dy, x, mean, rstd, xn, qkv, o, pk.ln_w, pk.qkv_w, pk.proj_w, pk.bias_table, pk.ln_wg, pk.ln_bg,
+                                   pk.qkv_wg, pk.qkv_bg, pk.proj_wg, pk.proj_bg, pk.bias_table_g,
+                                   _native_geometry(geo, num_heads, shifted, use_mask), scale, FUSE_BIAS_GRAD,
+                                   status_word(x.device))
+            return dx, None, None, None, None, None, None, None, None
         wgrad_accumulate(dy, o, pk.proj_wg, pk.proj_bg)
         if comm is not None:
             do = comm.alloc_dout(x.shape[0], C)
@@ -149,9 +154,8 @@ class _AttnHalfFn(torch.autograd.Function):
 class _MlpHalfFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, anchor, pk: ParamPack):
-        xn, mean, rstd = layernorm_cuda(x, pk.ln_w, pk.ln_b)
-        act, pre = gemm(xn, pk.fc1_w, bias=pk.fc1_b, gelu=True, save_pre=True)
-        y = gemm(act, pk.fc2_w, bias=pk.fc2_b, residual=x)
+        y, mean, rstd, xn, pre, act = _ext.load().mlp_half_fwd(x, pk.ln_w, pk.ln_b, pk.fc1_w, pk.fc1_b, pk.fc2_w, pk.fc2_b, LN_EPS,
+                                                               status_word(x.device))
         ctx.save_for_backward(x, mean, rstd, xn, pre, act)
         ctx.pk = pk
         return y
@@ -161,11 +165,8 @@ class _MlpHalfFn(torch.autograd.Function):
         x, mean, rstd, xn, pre, act = ctx.saved_tensors
         pk = ctx.pk
         dy = dy.contiguous()
-        wgrad_accumulate(dy, act, pk.fc2_wg, pk.fc2_bg)
-        dpre = gemm(dy, pk.fc2_w, b_mn=True, dgelu_aux=pre)
-        wgrad_accumulate(dpre, xn, pk.fc1_wg, pk.fc1_bg)
-        dxn = gemm(dpre, pk.fc1_w, b_mn=True)
-        dx = layernorm_bwd_cuda(dxn, x, pk.ln_w, mean, rstd, pk.ln_wg, pk.ln_bg, dres=dy)
+        dx = _ext.load().mlp_half_bwd(dy, x, mean, rstd, xn, pre, act, pk.ln_w, pk.fc1_w, pk.fc2_w, pk.ln_wg, pk.ln_bg, pk.fc1_wg,
+                                      pk.fc1_bg, pk.fc2_wg, pk.fc2_bg, FUSE_BIAS_GRAD, status_word(x.device))
         return dx, None, None
 
 
@@ -225,17 +226,17 @@ def attention_half(x, mod, geo: WindowGeometry, shifted: bool, comm=None):
         fused = getattr(mod.attn, "fused", None)
         if fused is None:
             raise RuntimeError("CUDA path needs flattened parameters (ParamArena)")
-        has_bias = mod.attn.use_relative_position_bias
+        attn, ln_w, ln_b = mod.attn, mod.norm1.weight, mod.norm1.bias
+        proj_w, proj_b = attn.proj.weight, attn.proj.bias
+        qkv_w, qkv_b = fused["qkv_weight"], fused["qkv_bias"]
+        table = attn.relative_position_bias_table if attn.use_relative_position_bias else None
         pk = ParamPack(
-            ln_w=mod.norm1.weight.bf16, ln_b=mod.norm1.bias.bf16, ln_wg=mod.norm1.weight.grad, ln_bg=mod.norm1.bias.grad,
-            qkv_w=fused["qkv_weight"].bf16, qkv_b=fused["qkv_bias"].bf16, qkv_wg=fused["qkv_weight"].grad,
-            qkv_bg=fused["qkv_bias"].grad,
-            proj_w=mod.attn.proj.weight.bf16, proj_b=mod.attn.proj.bias.bf16, proj_wg=mod.attn.proj.weight.grad,
-            proj_bg=mod.attn.proj.bias.grad,
-            bias_table=fp32_values(mod.attn.relative_position_bias_table) if has_bias else None,
-            bias_table_g=mod.attn.relative_position_bias_table.grad if has_bias else None)
-        return _AttnHalfFn.apply(x, mod.norm1.weight, pk, geo, mod.attn.num_heads, shifted, mod.use_attn_mask,
-                                 mod.attn.scale, comm)
+            ln_w=ln_w.bf16, ln_b=ln_b.bf16, ln_wg=ln_w.grad, ln_bg=ln_b.grad,
+            qkv_w=qkv_w.bf16, qkv_b=qkv_b.bf16, qkv_wg=qkv_w.grad, qkv_bg=qkv_b.grad,
+            proj_w=proj_w.bf16, proj_b=proj_b.bf16, proj_wg=proj_w.grad, proj_bg=proj_b.grad,
+            bias_table=fp32_values(table) if table is not None else None,
+            bias_table_g=table.grad if table is not None else None)
+        return _AttnHalfFn.apply(x, ln_w, pk, geo, attn.num_heads, shifted, mod.use_attn_mask, attn.scale, comm)
     a = mod.attn
     xn = TF.layer_norm(x, (x.shape[-1],), mod.norm1.weight, mod.norm1.bias, LN_EPS)
     qkv = torch.cat([a.q_linear(xn), a.k_linear(xn), a.v_linear(xn)], dim=-1)
@@ -247,11 +248,13 @@ def attention_half(x, mod, geo: WindowGeometry, shifted: bool, comm=None):
 def mlp_half(x, mod):
     """x + fc2(gelu(fc1(norm2(x))))."""
     if x.is_cuda:
+        ln_w, ln_b, fc1, fc2 = mod.norm2.weight, mod.norm2.bias, mod.fc1, mod.fc2
+        w1, b1, w2, b2 = fc1.weight, fc1.bias, fc2.weight, fc2.bias
         pk = ParamPack(
-            ln_w=mod.norm2.weight.bf16, ln_b=mod.norm2.bias.bf16, ln_wg=mod.norm2.weight.grad, ln_bg=mod.norm2.bias.grad,
-            fc1_w=mod.fc1.weight.bf16, fc1_b=mod.fc1.bias.bf16, fc1_wg=mod.fc1.weight.grad, fc1_bg=mod.fc1.bias.grad,
-            fc2_w=mod.fc2.weight.bf16, fc2_b=mod.fc2.bias.bf16, fc2_wg=mod.fc2.weight.grad, fc2_bg=mod.fc2.bias.grad)
-        return _MlpHalfFn.apply(x, mod.norm2.weight, pk)
+            ln_w=ln_w.bf16, ln_b=ln_b.bf16, ln_wg=ln_w.grad, ln_bg=ln_b.grad,
+            fc1_w=w1.bf16, fc1_b=b1.bf16, fc1_wg=w1.grad, fc1_bg=b1.grad,
+            fc2_w=w2.bf16, fc2_b=b2.bf16, fc2_wg=w2.grad, fc2_bg=b2.grad)
+        return _MlpHalfFn.apply(x, ln_w, pk)
     xn = TF.layer_norm(x, (x.shape[-1],), mod.norm2.weight, mod.norm2.bias, LN_EPS)
     return x + mod.fc2(TF.gelu(mod.fc1(xn)))
 

@@ -129,7 +129,7 @@ void conv3x3_fwd(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor& 
 // dw: [9, Cout, Cin] fp32 (zeroed by the caller)
 void conv3x3_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tensor& dw, int64_t stride, int64_t split_k,
                    const c10::optional<torch::Tensor>& status, const c10::optional<torch::Tensor>& halo_lo,
-                   const c10::optional<torch::Tensor>& halo_hi, const c10::optional<torch::Tensor>& bias_grad) {
+                   const c10::optional<torch::Tensor>& halo_hi, const c10::optional<torch::Tensor>& bias_grad, int64_t stack) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() == 4, "x: NHWC bf16");
   TORCH_CHECK(dy.scalar_type() == torch::kBFloat16 && dy.is_contiguous() && dy.dim() == 4, "dy: NHWC bf16");
   TORCH_CHECK(!bias_grad.has_value() || (bias_grad->scalar_type() == torch::kFloat32 && bias_grad->is_contiguous() &&
@@ -142,7 +142,8 @@ void conv3x3_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tenso
                                         x.size(2), x.size(3), dy.size(3), static_cast<int>(stride),
                                         static_cast<int>(split_k), status.has_value() ? status->data_ptr() : nullptr,
                                         sm_count(), cur_stream(), opt_ptr(halo_lo), opt_ptr(halo_hi),
-                                        bias_grad.has_value() ? bias_grad->data_ptr<float>() : nullptr);
+                                        bias_grad.has_value() ? bias_grad->data_ptr<float>() : nullptr,
+                                        static_cast<int>(stack));
   TORCH_CHECK(rc == 0, "terra_b200 conv3x3_wgrad launch failed, code ", rc);
 }
 
@@ -195,7 +196,7 @@ void convt2x2(int64_t op, const torch::Tensor& in, const torch::Tensor& w, const
 
 // dw: [4, Cin, Cout] fp32, accumulated
 void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tensor& dw, int64_t split_k,
-                    const c10::optional<torch::Tensor>& status) {
+                    const c10::optional<torch::Tensor>& status, int64_t stack) {
   check_image(x, "x");
   check_image(dy, "dy");
   TORCH_CHECK(x.size(0) == dy.size(0) && 2 * x.size(1) == dy.size(1) && 2 * x.size(2) == dy.size(2), "convt2x2_wgrad: grids");
@@ -205,7 +206,7 @@ void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tens
   tb::note_launch();
   const int rc = tb::convt2x2_wgrad_bf16(x.data_ptr(), dy.data_ptr(), dw.data_ptr<float>(), x.size(0), x.size(1), x.size(2),
                                          x.size(3), dy.size(3), static_cast<int>(split_k), status_ptr(status), sm_count(),
-                                         cur_stream());
+                                         cur_stream(), static_cast<int>(stack));
   TORCH_CHECK(rc == 0, "terra_b200 convt2x2_wgrad launch failed, code ", rc);
 }
 
@@ -235,11 +236,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("conv3x3_fwd", &conv3x3_fwd, "implicit-GEMM 3x3 convolution (NHWC bf16)");
   m.def("conv3x3_wgrad", &conv3x3_wgrad, "3x3 convolution weight gradient (fp32 atomics)", py::arg("x"), py::arg("dy"),
         py::arg("dw"), py::arg("stride"), py::arg("split_k"), py::arg("status"), py::arg("halo_lo"), py::arg("halo_hi"),
-        py::arg("bias_grad") = py::none());
+        py::arg("bias_grad") = py::none(), py::arg("stack") = 1);
   m.def("conv3x3_s2_dgrad", &conv3x3_s2_dgrad, "input gradient of the stride-2 3x3 convolution (NHWC bf16)");
   m.def("convt2x2", &convt2x2, "2x2 / stride-2 transposed convolution: forward (op 0), input gradient (op 1)", py::arg("op"),
         py::arg("input"), py::arg("w"), py::arg("bias4"), py::arg("out"), py::arg("status"));
-  m.def("convt2x2_wgrad", &convt2x2_wgrad, "2x2 / stride-2 transposed convolution: weight gradient (fp32 atomics)");
+  m.def("convt2x2_wgrad", &convt2x2_wgrad, "2x2 / stride-2 transposed convolution: weight gradient (fp32 atomics)",
+        py::arg("x"), py::arg("dy"), py::arg("dw"), py::arg("split_k"), py::arg("status"), py::arg("stack") = 1);
   bind_elementwise(m);
   bind_attention(m);
   bind_halves(m);

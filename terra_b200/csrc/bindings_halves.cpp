@@ -91,6 +91,40 @@ void column_sums(const Tensor& dy, const Tensor& out) {
            "colsum");
 }
 
+// Tile width, row blocks per tile and split of the contraction for N x K outputs over M rows. A k-block costs a CTA its
+// operand fill plus the tensor core's reads through the shared-memory port, in KB; the column sums add 40 KB per row block,
+// shared out over the column tiles. Every split pays its start and its pass of atomics (about 1000 KB a row block). Widths
+// of 256 leave no room for the sums' accumulators: dy is then read once more (5 TB/s against 3.7 us per 1000 KB).
+// Measured (139264 rows, us): 1152 x 384 unstacked / stacked 125 / 132, 1536 x 384 163 / 155, 384 x 1536 171 / 212 (three
+// row blocks stack badly).
+struct WgradPlan {
+  int bn, stack, split;
+};
+WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
+  const int64_t m_blocks = (N + 127) / 128, k_blocks = (M + 63) / 64, sms = sm_count();
+  WgradPlan best{128, 1, 1};
+  double least = -1.0;
+  for (int stack : {1, 2}) {
+    if (stack > m_blocks) continue;
+    for (int bn : {192, 128, 256}) {
+      const int64_t n = (K + bn - 1) / bn, tiles = (m_blocks + stack - 1) / stack * n;
+      const double kb = 16.0 * stack + bn / 8 + stack * (16.0 + bn / 8) + (sums && bn < 256 ? 40.0 * stack / n : 0.0);
+      const double extra = sums && bn == 256 ? 2.0 * M * N / 5e6 / 0.0037 : 0.0;
+      // whole rounds of CTAs: the largest split of one round, two rounds, ...
+      for (int64_t rounds = 1; rounds <= 3; ++rounds) {
+        const int64_t split = std::max<int64_t>(1, std::min(rounds * sms / tiles, k_blocks));
+        const int64_t per = (k_blocks + split - 1) / split;
+        const double cost = static_cast<double>((tiles * split + sms - 1) / sms) * (per * kb + 1000.0 * stack) + extra;
+        if (least < 0.0 || cost < least * 0.995) {
+          least = cost;
+          best = {bn, stack, static_cast<int>(split)};
+        }
+      }
+    }
+  }
+  return best;
+}
+
 // grad_w [N, K] (fp32) += dy [M, N]^T x [M, K]; grad_b [N] += column sums of dy, from the same kernel (`fuse_bias`: a
 // 16-column MMA of the dy tiles against ones) where its accumulators fit beside the tile's (widths up to 192).
 void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTensor& grad_b, bool fuse_bias, const Tensor& status) {
@@ -101,15 +135,15 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
   const c10::cuda::CUDAGuard guard(dy.device());
   const int64_t M = dy.size(0), N = dy.size(1), K = x.size(1);
   bool sums = grad_b.has_value();
-  const bool wide = K % 256 == 0 && K >= 1024 && (!(sums && fuse_bias) || K % 192 != 0);
-  const int bn = wide ? 256 : (K % 192 == 0 ? 192 : 128);
-  if (sums && (!fuse_bias || bn == 256)) {
+  if (sums && !fuse_bias) {
     column_sums(dy, *grad_b);
     sums = false;
   }
-  // enough splits of the contraction to fill the GPU once, never more than its 64-wide blocks
-  const int64_t tiles = ((N + 127) / 128) * ((K + bn - 1) / bn), blocks = (M + 63) / 64;
-  const int64_t split = std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>(1, sm_count() / tiles), blocks));
+  const WgradPlan plan = plan_wgrad(N, K, M, sums);
+  if (sums && plan.bn == 256) {
+    column_sums(dy, *grad_b);
+    sums = false;
+  }
   tb::GemmOperand A{dy.data_ptr(), dy.stride(0), 1}, B{x.data_ptr(), x.stride(0), 1};
   tb::GemmEpilogue g{};
   g.flags = tb::EPI_OUT_F32 | tb::EPI_ATOMIC;
@@ -118,8 +152,9 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
   g.alpha = 1.0f;
   g.status = status.data_ptr();
   g.colsum = sums ? grad_b->data_ptr<float>() : nullptr;
+  g.stack = plan.stack;
   tb::note_launch();
-  rc_check(tb::gemm_bf16(A, B, N, K, M, g, static_cast<int>(split), bn, sm_count(), cur_stream()), "gemm (weight gradient)");
+  rc_check(tb::gemm_bf16(A, B, N, K, M, g, plan.split, plan.bn, sm_count(), cur_stream()), "gemm (weight gradient)");
 }
 
 struct Norm {

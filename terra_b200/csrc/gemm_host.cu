@@ -125,7 +125,7 @@ static int pick_bn(long long N, int requested) {
 // reads. In a pair each CTA stages 128 rows of A and only half of B's BN rows, (16 + BN / 16) KB. Pairs are taken by
 // plain products (no peers, no split, no column sums) as soon as their tiles make eight rounds over the
 // pairs of SMs; with fewer rounds the larger tiles leave more of the last one empty (17280 rows, 576 x 192: 12 us with
-// single CTAs, 18 us with pairs; 139264 rows, 1152 x 384: 130 and 117 us). Returns the pair tile width, 0: single CTAs.
+// single CTAs, 18 us with pairs; 139264 rows, 1152 x 384: 130 and 117 us).
 static bool pairs_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("TERRA_GEMM_2CTA");
@@ -134,21 +134,28 @@ static bool pairs_enabled() {
   return on;
 }
 
-static int pick_pair_bn(long long m_blocks, long long N, bool b_mn, int num_sms) {
-  if (!pairs_enabled()) return 0;
-  int best = 0;
-  long long best_cost = 0;
-  for (int bn : {256, 192, 128}) {
-    if (b_mn && bn == 192) continue;               // half of an MN-major B must be whole 64-row boxes
-    const long long n_tiles = (N + bn - 1) / bn;
-    if (((m_blocks + 1) / 2) * n_tiles < 8LL * (num_sms / 2)) continue;
-    const long long cost = n_tiles * (16 + bn / 16);   // KB through the port per 128 rows and k-block
-    if (best == 0 || cost < best_cost) {
-      best = bn;
-      best_cost = cost;
+// Tile of a plain product with many tiles: the width and CTA count with the fewest cycles per 128 rows, a tile taking the
+// longer of its main loop (operand fill and tensor-core reads through the shared-memory port) and its epilogue (rounds of
+// 32-column chunks over three warps per lane quadrant, by what a chunk does). Measured on 139264 rows, pairs of 192 / 256:
+// 1152 x 384 with bias 126 / 130 us, 3072 x 1024 804 / 645 us; times GELU' 1536 x 384, single 192 / pairs 256: 352 / 364 us.
+static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, int num_sms, int* bn_out, int* ctas_out) {
+  *bn_out = pick_bn(N, 0);
+  *ctas_out = 1;
+  if (!pairs_enabled() || N < 128 || ((m_blocks + 1) / 2) * ((N + 255) / 256) < 8LL * (num_sms / 2)) return;
+  const long long chunk = (flags & EPI_MUL_DGELU) ? 4500 : (flags & EPI_SAVE_PRE) ? 3800 : (flags & EPI_RESIDUAL) ? 3500 : 1800;
+  long long best = 0;
+  for (int ctas : {2, 1})
+    for (int bn : {256, 192, 128}) {
+      if (ctas == 2 && b_mn && bn == 192) continue;      // half of an MN-major B must be whole 64-row boxes
+      const long long loop = static_cast<long long>(k_blocks) * 16 * (16 + bn / (8 * ctas));
+      const long long epilogue = chunk * ((bn / 32 + 2) / 3);
+      const long long cost = (N + bn - 1) / bn * (loop > epilogue ? loop : epilogue);
+      if (best == 0 || cost < best) {
+        best = cost;
+        *bn_out = bn;
+        *ctas_out = ctas;
+      }
     }
-  }
-  return best;
 }
 
 static void fill_epilogue(GemmParams& p, const GemmEpilogue& e) {
@@ -186,18 +193,15 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   // scattered output is either the fp32 atomic form or the plain bf16 form (one staging slot per source GPU)
   if (scatter_c && (epi.flags & EPI_OUT_F32) && !(epi.flags & EPI_ATOMIC)) return -13;
   if ((gather_a || scatter_c) && bn_request >= 1000) return -14;   // single-CTA tiles only
-  // CTA pairs: explicit request 1000 + BN, or the rule of pick_pair_bn where no tile width is asked for.
+  // CTA pairs: explicit request 1000 + BN, or the rule of pick_tile where no tile width is asked for.
   int ctas = 1;
   if (bn_request >= 1000) {
     ctas = 2;
     bn_request -= 1000;
     if (bn_request != 128 && bn_request != 256 && !(bn_request == 192 && !B.mn_major)) return -11;
   } else if (bn_request == 0 && !A.mn_major && !gather_a && !scatter_c && split_k <= 1 && epi.colsum == nullptr) {
-    const int bn2 = pick_pair_bn((M + GEMM_BM - 1) / GEMM_BM, N, B.mn_major, num_sms);
-    if (bn2 != 0) {
-      ctas = 2;
-      bn_request = bn2;
-    }
+    pick_tile((M + GEMM_BM - 1) / GEMM_BM, N, static_cast<int>((K + GEMM_BK - 1) / GEMM_BK), B.mn_major, epi.flags, num_sms,
+              &bn_request, &ctas);
   }
   if (epi.colsum != nullptr) {
     // column sums ride on the weight-gradient form only, and need room for their accumulators behind the tile's
@@ -210,6 +214,13 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   p.K = static_cast<int>(K);
   p.m_blocks = static_cast<int>((M + GEMM_BM - 1) / GEMM_BM);
   p.num_m_tiles = (p.m_blocks + ctas - 1) / ctas;
+  if (epi.stack == 2) {
+    if (!A.mn_major || ctas != 1 || gather_a || scatter_c || !(epi.flags & EPI_ATOMIC) || bn < 128 ||
+        (bn == 256 && epi.colsum != nullptr))
+      return -17;
+    p.stack = 2;
+    p.num_m_tiles = (p.m_blocks + 1) / 2;
+  }
   if (gather_a || scatter_c) ctas = 1;
   if (gather_a) {
     p.a_peers = peers.a_peers;
@@ -328,9 +339,8 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
   const long long m_blocks = static_cast<long long>((c.tiles_w + GEMM_BM - 1) / GEMM_BM) * c.tiles_h * c.B;
-  const int bn2 = pick_pair_bn(m_blocks * c.groups, c.N, false, num_sms);
-  const int ctas = bn2 != 0 ? 2 : 1;
-  const int bn = bn2 != 0 ? bn2 : pick_bn(c.N, 0);
+  int bn = 0, ctas = 1;
+  pick_tile(m_blocks * c.groups, c.N, c.ntaps * cchunks / c.groups, false, epi.flags, num_sms, &bn, &ctas);
   p.M = c.B * c.tiles_h * c.tiles_w;
   p.N = c.N;
   p.K = c.ntaps * cchunks * 64;
@@ -460,7 +470,7 @@ int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, i
 // times `b` [B, H, W, N] at the pixel's tap (hmul = par = stride of the grid of `a` in `b`).
 static int gather_wgrad(const void* a, const void* b, float* dw, int B, int Ho, int Wo, int M, int H, int W, int N, int stride,
                         const Tap* taps, int ntaps, int split_k, void* status, int num_sms, cudaStream_t stream,
-                        const void* halo_lo, const void* halo_hi, float* colsum) {
+                        const void* halo_lo, const void* halo_hi, float* colsum, int stack) {
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
   const int bn = pick_bn(N, N % 192 == 0 ? 192 : 128);   // 384 columns: two tiles of 192, a fifth less operand traffic per flop
@@ -472,7 +482,8 @@ static int gather_wgrad(const void* a, const void* b, float* dw, int B, int Ho, 
   p.k_blocks = p.pix_n0 * Ho * B;
   p.K = p.k_blocks * GEMM_BK;
   p.m_blocks = (M + GEMM_BM - 1) / GEMM_BM;
-  p.num_m_tiles = p.m_blocks;
+  p.stack = stack == 2 && bn >= 128 ? 2 : 1;
+  p.num_m_tiles = (p.m_blocks + p.stack - 1) / p.stack;
   p.num_n_tiles = (N + bn - 1) / bn;
   p.groups = ntaps;
   if (split_k < 1) split_k = 1;
@@ -511,7 +522,7 @@ static int gather_wgrad(const void* a, const void* b, float* dw, int B, int Ho, 
 // 3x3 convolution: dw[tap][Cout][Cin] (pre-zeroed), bias_grad[Cout] += the sums of dy from the same kernel.
 int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
                        int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo,
-                       const void* halo_hi, float* bias_grad) {
+                       const void* halo_hi, float* bias_grad, int stack) {
   if (stride != 1 && stride != 2) return -11;
   if (stride == 2 && (W % 2 != 0)) return -12;
   if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
@@ -524,16 +535,16 @@ int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, i
   }
   const int Ho = (stride == 1) ? H : (H + 1) / 2, Wo = (stride == 1) ? W : W / 2;
   return gather_wgrad(dy, x, dw, B, Ho, Wo, Cout, H, W, Cin, stride, taps, 9, split_k, status, num_sms, stream, halo_lo,
-                      halo_hi, bias_grad);
+                      halo_hi, bias_grad, stack);
 }
 
 // 2x2 / stride-2 transposed convolution: dw[tap][Cin][Cout] (pre-zeroed) from x [B, H, W, Cin] and dy [B, 2H, 2W, Cout].
 int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int split_k,
-                        void* status, int num_sms, cudaStream_t stream) {
+                        void* status, int num_sms, cudaStream_t stream, int stack) {
   if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
   const Tap taps[4] = {{0, 0, 0}, {1, 0, 0}, {0, 0, 1}, {1, 0, 1}};
   return gather_wgrad(x, dy, dw, B, H, W, Cin, 2 * H, 2 * W, Cout, 2, taps, 4, split_k, status, num_sms, stream, nullptr,
-                      nullptr, nullptr);
+                      nullptr, nullptr, stack);
 }
 
 int gemm_stall_counters(unsigned long long* out8, int reset) {

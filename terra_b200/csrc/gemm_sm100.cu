@@ -41,9 +41,16 @@ constexpr int GEMM_THREADS = 64 + 32 * GEMM_EPI_WARPS;
 // its own 128 rows of A and its own half of B, so a k-block costs each SM (16 + BN / 8) KB of shared-memory fill instead
 // of (16 + BN / 4) KB: the operand traffic per flop through shared memory, which bounds the single-CTA main loop, drops
 // by a third at BN = 256.
-template <int BN, int CTAS>
+//
+// STACK = 2 (weight gradients, one CTA): two 128-row blocks of A share a tile of B, 256 x BN outputs in both accumulators.
+// The operand stream through L2 bounds those products (12 TB/s measured with 128 x 192 tiles: 40 KB per k-block); stacked, a
+// k-block costs 56 KB for twice the outputs. There is no second accumulator set to overlap the epilogue with the next
+// tile, which a contraction over thousands of k-blocks does not need.
+template <int BN, int CTAS, int STACK = 1>
 struct GemmCfg {
-  static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
+  static constexpr int BLOCK_BYTES = GEMM_BM * GEMM_BK * 2;   // one 128-row block of A
+  static constexpr int A_BYTES = STACK * BLOCK_BYTES;
+  static constexpr int ACCS = STACK == 1 ? 2 : 1;          // accumulator sets
   static constexpr int B_ROWS = BN / CTAS;                 // rows of B staged by one CTA
   static constexpr int B_BYTES = B_ROWS * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -62,12 +69,12 @@ struct GemmCfg {
                                                                             : (MAX_SMEM - 1024 - fixed_bytes(bufs)) / STAGE_BYTES;
   }
   static constexpr int smem_bytes(int bufs) { return stages_for(bufs) * STAGE_BYTES + fixed_bytes(bufs) + 1024; }   // + alignment slack
-  // two accumulators; the allocation must be a power of two
+  // two accumulators (of alternating tiles, or of a tile's two row blocks); the allocation must be a power of two
   // behind them two 32-column accumulators of the column sums (weight-gradient form with a bias gradient, BN <= 192)
   static constexpr int SUM_COL0 = 2 * BN;
   static constexpr int TMEM_COLS = (2 * BN + 64 <= 256) ? 256 : 512;
   static constexpr bool CAN_COLSUM = CTAS == 1 && 2 * BN + 64 <= 512;
-  static_assert(stages_for(3) >= 3 && smem_bytes(1) <= MAX_SMEM && smem_bytes(3) <= MAX_SMEM, "shared memory budget");
+  static_assert((STACK == 2 ? stages_for(1) : stages_for(3)) >= 3 && smem_bytes(1) <= MAX_SMEM && smem_bytes(3) <= MAX_SMEM, "shared memory budget");
   static_assert(GEMM_EPI_WARPS * 32 * 4 + BAR_BYTES <= FIXED_BASE, "bias slots");
   // a CTA's half of an MN-major B must be whole 64-row boxes; K-major rows only need whole 8-row swizzle atoms
   static constexpr bool CAN_B_MN = B_ROWS % 64 == 0;
@@ -90,15 +97,31 @@ struct TileCoord {
   int kb_begin, kb_end;
 };
 
+// Column sums of A (weight-gradient form): every tile of a row block streams the same A tiles, so the sums are shared out by
+// k-block, kb % ways == the tile's place among its row block's `ways` tiles. (A 16-column MMA costs as much of the
+// tensor pipe and of the shared-memory port as 40 KB of operand stream: left to the first column tile it made that tile
+// half as slow again, and the launch waits for the slowest.) Returns this tile's first such k-block.
+__device__ __forceinline__ int first_sum_kb(const GemmParams& p, const TileCoord& t, int ways) {
+  const int place = t.grp * p.num_n_tiles + t.n_blk;
+  return t.kb_begin + (place + ways - t.kb_begin % ways) % ways;
+}
+
 // p.num_m_tiles counts tiles of ctas * 128 rows; m_blk is returned in units of 128 rows for CTA `rank` of the pair.
-__device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int tile, int ctas = 1, int rank = 0) {
+// Stacked tiles (p.stack = 2 blocks of rows): the row tile varies slowest, so that the last one, which may hold a single
+// block, is handed out last.
+__device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int tile, int ctas = 1, int rank = 0, int stack = 1) {
   TileCoord t;
   t.split = tile % p.split_k;
   int r = tile / p.split_k;
   t.n_blk = r % p.num_n_tiles;
   r /= p.num_n_tiles;
-  t.m_blk = (r % p.num_m_tiles) * ctas + rank;
-  t.grp = r / p.num_m_tiles;
+  if (stack > 1) {
+    t.grp = r % p.groups;
+    t.m_blk = r / p.groups * stack;
+  } else {
+    t.m_blk = (r % p.num_m_tiles) * ctas + rank;
+    t.grp = r / p.num_m_tiles;
+  }
   if (p.grp_ranges) {
     t.kb_begin = p.grp_kb[t.grp];
     t.kb_end = p.grp_kb[t.grp + 1];
@@ -112,9 +135,10 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int tile, 
 
 // PEERS: the tensor-parallel variants (A gathered from peer buffers, output scattered to peer buffers). A separate
 // instantiation, so that the plain kernel carries none of their registers and branches.
-template <int BN, int CTAS, bool PEERS>
+template <int BN, int CTAS, bool PEERS, int STACK = 1>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
-  using Cfg = GemmCfg<BN, CTAS>;
+  static_assert(STACK == 1 || (CTAS == 1 && !PEERS), "stacked tiles: one CTA, no peers");
+  using Cfg = GemmCfg<BN, CTAS, STACK>;
   constexpr bool PAIR = CTAS == 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -208,8 +232,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       long long t_wait = 0;
       unsigned int peers_ready = 0u;   // bit per (peer, chunk) whose flag has been seen
       for (int tile = unit; tile < total_tiles && !*abort_flag; tile += units) {
-        const TileCoord tc = decode_tile(p, tile, CTAS, rank);
+        const TileCoord tc = decode_tile(p, tile, CTAS, rank, STACK);
         const int m0 = tc.m_blk * GEMM_BM;
+        const int blocks = STACK > 1 ? min(STACK, p.m_blocks - tc.m_blk) : 1;   // 128-row blocks of this tile
         const int n0 = tc.n_blk * BN + rank * Cfg::B_ROWS;   // this CTA's rows of B
         int abase[5] = {0, 0, 0, 0, 0};
         if (p.a_mode == OP_TABLE_5D) {
@@ -225,7 +250,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           t_wait += clock64() - w0;
           uint8_t* sA = smem + s * Cfg::STAGE_BYTES;
           uint8_t* sB = sA + Cfg::A_BYTES;
-          mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
+          mbar_expect_tx(&full[s], STACK > 1 ? Cfg::B_BYTES + blocks * Cfg::BLOCK_BYTES : Cfg::STAGE_BYTES);
           int pw = 0, ph_ = 0, pb = 0;
           if (p.a_mode == OP_PIXELS_5D || p.b_mode == OP_PIXELS_5D) {
             pw = kb % p.pix_n0;
@@ -263,8 +288,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             }
           } else if (p.a_mode == OP_MNMAJOR_2D) {
 #pragma unroll
-            for (int j = 0; j < GEMM_BM / 64; ++j)
-              tma_load_2d(sA + j * (GEMM_BK * 128), &p.map_a, &full[s], m0 + j * 64, kb * GEMM_BK);
+            for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
+              if (STACK == 1 || j < blocks * (GEMM_BM / 64))
+                tma_load_2d(sA + j * (GEMM_BK * 128), &p.map_a, &full[s], m0 + j * 64, kb * GEMM_BK);
           } else if (p.a_mode == OP_TABLE_5D) {
             const short* e = p.ktable[kb];
             int h = abase[3] + e[3];
@@ -279,8 +305,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             tma_load_5d(sA, m, &full[s], abase[0] + e[0], abase[1] + e[1], abase[2] + e[2], h, abase[4]);
           } else {  // OP_PIXELS_5D: {channels, 1, w, h, b}
 #pragma unroll
-            for (int j = 0; j < GEMM_BM / 64; ++j)
-              tma_load_5d(sA + j * (GEMM_BK * 128), &p.map_a, &full[s], m0 + j * 64, 0, pw * GEMM_BK, ph_, pb);
+            for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
+              if (STACK == 1 || j < blocks * (GEMM_BM / 64))
+                tma_load_5d(sA + j * (GEMM_BK * 128), &p.map_a, &full[s], m0 + j * 64, 0, pw * GEMM_BK, ph_, pb);
           }
           // ---- operand B
           if (p.b_mode == OP_KMAJOR_2D) {
@@ -326,15 +353,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       const long long t_begin = clock64();
       long long t_acc = 0, t_ops = 0;
       for (int tile = unit; tile < total_tiles && !*abort_flag; tile += units, ++tcount) {
-        const TileCoord tc = decode_tile(p, tile, CTAS, rank);
-        const int acc = tcount & 1;
-        const uint32_t aph = (tcount >> 1) & 1u;
+        const TileCoord tc = decode_tile(p, tile, CTAS, rank, STACK);
+        const int acc = tcount % Cfg::ACCS;
+        const uint32_t aph = (tcount / Cfg::ACCS) & 1u;
+        const int blocks = STACK > 1 ? min(STACK, p.m_blocks - tc.m_blk) : 1;
         const long long w0 = clock64();
         if (!mbar_wait<PAIR>(&tempty[acc], aph ^ 1u, abort_flag, p.status, 0x200u + acc, mbar_budget)) break;
         t_acc += clock64() - w0;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        const bool sums = Cfg::CAN_COLSUM && p.colsum != nullptr && tc.n_blk == 0 && tc.grp == 0;
+        const int ways = p.groups * p.num_n_tiles;
+        const int sum_first = Cfg::CAN_COLSUM && p.colsum != nullptr ? first_sum_kb(p, tc, ways) : tc.kb_end;
+        int sum_kb = sum_first;
         const uint32_t d_sums = tmem_base + Cfg::SUM_COL0 + acc * 32;
         bool ok = true;
         for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
@@ -348,14 +378,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           const uint64_t da = make_smem_desc(sA, a_lbo, 1024);
           const uint64_t db = make_smem_desc(sB, b_lbo, 1024);
 #pragma unroll
-          for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
-            umma_bf16<CTAS>(d_tmem, da + kk * a_kstep, db + kk * b_kstep, idesc, (kb > tc.kb_begin || kk > 0) ? 1u : 0u);
-          }
-          if (sums) {   // column sums of A: the same A tiles against 16 columns of ones
+          for (int mb = 0; mb < STACK; ++mb) {
+            if (STACK > 1 && mb >= blocks) break;
+            const uint64_t dm = da + mb * (Cfg::BLOCK_BYTES >> 4);
 #pragma unroll
-            for (int kk = 0; kk < GEMM_BK / 16; ++kk)
-              umma_bf16<CTAS>(d_sums, da + kk * a_kstep, d_ones, idesc_sums, (kb > tc.kb_begin || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
+              umma_bf16<CTAS>(d_tmem + mb * BN, dm + kk * a_kstep, db + kk * b_kstep, idesc, (kb > tc.kb_begin || kk > 0) ? 1u : 0u);
+            }
+            if (Cfg::CAN_COLSUM && kb == sum_kb) {   // column sums of A: the same A tiles against 16 columns of ones
+#pragma unroll
+              for (int kk = 0; kk < GEMM_BK / 16; ++kk)
+                umma_bf16<CTAS>(d_sums + mb * 32, dm + kk * a_kstep, d_ones, idesc_sums, (kb > sum_first || kk > 0) ? 1u : 0u);
+            }
           }
+          if (kb == sum_kb) sum_kb += ways;
           umma_commit<CTAS>(&empty[s]);     // frees stage s (in both CTAs of a pair)
         }
         if (!ok) break;
@@ -401,7 +437,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       return reinterpret_cast<uint4*>(my_x + rr * 64 + (((vec ^ (rr >> 1)) & 3) << 4));
     };
     constexpr int CPW = (CHUNKS + GEMM_EPI_WARPS / 4 - 1) / (GEMM_EPI_WARPS / 4);   // chunks per warp
-    if (!PEERS && p.epi_tma) {
+    if (!PEERS && STACK == 1 && p.epi_tma) {
       // ---- plain row-major bf16 outputs: chunks leave (and the operand the epilogue reads arrives) through TMA.
       // A chunk is 32 rows of 64 bytes in the 64-byte-swizzled layout, which is also conflict-free for the
       // row-per-lane 16-byte accesses of the warp. The warp's first one or two buffers stage outputs in turn: one lane
@@ -416,13 +452,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       const uint32_t swz = (static_cast<uint32_t>(lane) >> 1) & 3u;
       const uint32_t out_addr = smem_u32(my_bufs);
       uint32_t issued = 0, consumed = 0, stored = 0;
-      int pf_tile = unit, pf_ci = 0;
+      int pf_tile = unit, pf_ci = 0, pf_n0 = 0, pf_row = 0;
       auto prefetch_next = [&]() {   // issue the load of this warp's next input chunk, if there is one
         while (pf_tile < total_tiles) {
-          const TileCoord t = decode_tile(p, pf_tile, CTAS, rank);
+          if (pf_ci == 0) {      // the divisions once per tile
+            const TileCoord t = decode_tile(p, pf_tile, CTAS, rank);
+            pf_n0 = t.n_blk * BN;
+            pf_row = t.m_blk * GEMM_BM + q * 32;
+          }
           const int c = part + pf_ci * (GEMM_EPI_WARPS / 4);
-          const int col = t.n_blk * BN + c * 32;
-          const int row = t.m_blk * GEMM_BM + q * 32;
+          const int col = pf_n0 + c * 32, row = pf_row;
           const bool ok = c < CHUNKS && col < p.N;
           if (++pf_ci >= CPW) {
             pf_ci = 0;
@@ -582,232 +621,247 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       if (lane == 0) bulk_wait_group_read<0>();
     } else
     for (int tile = unit; tile < total_tiles; tile += units, ++tcount) {
-      const TileCoord tc = decode_tile(p, tile, CTAS, rank);
-      const int acc = tcount & 1;
-      const uint32_t aph = (tcount >> 1) & 1u;
-      const int n0 = tc.n_blk * BN;
-      // ---- tile row -> output row index (-1: outside the output)
-      auto out_row = [&](int r) -> long long {
-        if (p.epi & EPI_ROW_CONV) {
-          const int t0 = tc.m_blk % p.tile_n0;
-          const int t1 = (tc.m_blk / p.tile_n0) % p.tile_n1;
-          const int t2 = tc.m_blk / (p.tile_n0 * p.tile_n1);
-          const int w = t0 * GEMM_BM + r;
-          return (w < p.out_w && tc.m_blk < p.m_blocks) ? (static_cast<long long>(t2) * p.tile_n1 + t1) * p.out_w + w : -1;
-        } else if (PEERS && p.a_peers > 1) {
-          const int slot = p.a_interleave ? tc.m_blk % p.a_peers : tc.m_blk / p.a_tiles;
-          const int peer = (slot + p.a_first) % p.a_peers;
-          const int lr = (p.a_interleave ? tc.m_blk / p.a_peers : tc.m_blk % p.a_tiles) * GEMM_BM + r;
-          return (lr < p.a_rows) ? static_cast<long long>(peer) * p.a_rows + lr : -1;
-        } else {
-          const long long g = static_cast<long long>(tc.m_blk) * GEMM_BM + r;
-          return (g < p.M) ? g : -1;
-        }
-      };
-      int grows[4];   // row indices fit 32 bits (element offsets may not)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) grows[i] = static_cast<int>(out_row(q * 32 + grow + 8 * i));
-      const long long gofs = static_cast<long long>(tc.grp) * p.grp_c_stride;
-      const int ncols_out = p.N;
+      const TileCoord first = decode_tile(p, tile, CTAS, rank, STACK);
+      const int acc = tcount % Cfg::ACCS;
+      const uint32_t aph = (tcount / Cfg::ACCS) & 1u;
+      const int n0 = first.n_blk * BN;
+      bool failed = false;
+#pragma unroll 1
+      for (int mb = 0; mb < STACK; ++mb) {       // the tile's row blocks
+        TileCoord tc = first;
+        tc.m_blk += mb;
+        if (STACK > 1 && tc.m_blk >= p.m_blocks) break;
+        const int dcol = (STACK > 1 ? mb : acc);    // which of the two accumulators
+        // ---- tile row -> output row index (-1: outside the output)
+        auto out_row = [&](int r) -> long long {
+          if (p.epi & EPI_ROW_CONV) {
+            const int t0 = tc.m_blk % p.tile_n0;
+            const int t1 = (tc.m_blk / p.tile_n0) % p.tile_n1;
+            const int t2 = tc.m_blk / (p.tile_n0 * p.tile_n1);
+            const int w = t0 * GEMM_BM + r;
+            return (w < p.out_w && tc.m_blk < p.m_blocks) ? (static_cast<long long>(t2) * p.tile_n1 + t1) * p.out_w + w : -1;
+          } else if (PEERS && p.a_peers > 1) {
+            const int slot = p.a_interleave ? tc.m_blk % p.a_peers : tc.m_blk / p.a_tiles;
+            const int peer = (slot + p.a_first) % p.a_peers;
+            const int lr = (p.a_interleave ? tc.m_blk / p.a_peers : tc.m_blk % p.a_tiles) * GEMM_BM + r;
+            return (lr < p.a_rows) ? static_cast<long long>(peer) * p.a_rows + lr : -1;
+          } else {
+            const long long g = static_cast<long long>(tc.m_blk) * GEMM_BM + r;
+            return (g < p.M) ? g : -1;
+          }
+        };
+        int grows[4];   // row indices fit 32 bits (element offsets may not)
+  #pragma unroll
+        for (int i = 0; i < 4; ++i) grows[i] = static_cast<int>(out_row(q * 32 + grow + 8 * i));
+        const long long gofs = static_cast<long long>(tc.grp) * p.grp_c_stride;
+        const int ncols_out = p.N;
 
-      // bf16 chunk from global memory, global-side layout (zeros outside the output)
-      auto fetch_chunk = [&](const __nv_bfloat16* base, long long ld, int cb, uint4 (&t)[4]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          t[i] = make_uint4(0, 0, 0, 0);
-          if (grows[i] >= 0 && cb + gvec * 8 < ncols_out)
-            t[i] = *reinterpret_cast<const uint4*>(base + static_cast<long long>(grows[i]) * ld + cb + gvec * 8);
-        }
-      };
-      // global-side registers -> row-per-lane registers
-      auto turn_chunk = [&](const uint4 (&t)[4], uint4 (&u)[4]) {
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) *xaddr(grow + 8 * i, gvec) = t[i];
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 4; ++j) u[j] = *xaddr(lane, j);
-      };
-      // 32 floats of the row-per-lane layout to bf16 global memory
-      auto store_chunk = [&](__nv_bfloat16* base, long long ld, int cb, const float (&f)[32]) {
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          *xaddr(lane, j) = make_uint4(pack_bf16x2(f[8 * j], f[8 * j + 1]), pack_bf16x2(f[8 * j + 2], f[8 * j + 3]),
-                                       pack_bf16x2(f[8 * j + 4], f[8 * j + 5]), pack_bf16x2(f[8 * j + 6], f[8 * j + 7]));
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint4 t = *xaddr(grow + 8 * i, gvec);
-          if (grows[i] >= 0 && cb + gvec * 8 < ncols_out) {
-            __nv_bfloat16* o = base + static_cast<long long>(grows[i]) * ld + cb + gvec * 8;
-            if (PEERS && p.c_peers > 1 && base == static_cast<__nv_bfloat16*>(p.C) + gofs)   // the row's owner stages it
-              o = static_cast<__nv_bfloat16*>(p.c_peer[grows[i] / p.c_rows]) + gofs +
-                  (static_cast<long long>(p.c_slot) * p.c_rows + grows[i] % p.c_rows) * ld + cb + gvec * 8;
-            *reinterpret_cast<uint4*>(o) = t;
+        // bf16 chunk from global memory, global-side layout (zeros outside the output)
+        auto fetch_chunk = [&](const __nv_bfloat16* base, long long ld, int cb, uint4 (&t)[4]) {
+  #pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            t[i] = make_uint4(0, 0, 0, 0);
+            if (grows[i] >= 0 && cb + gvec * 8 < ncols_out)
+              t[i] = *reinterpret_cast<const uint4*>(base + static_cast<long long>(grows[i]) * ld + cb + gvec * 8);
+          }
+        };
+        // global-side registers -> row-per-lane registers
+        auto turn_chunk = [&](const uint4 (&t)[4], uint4 (&u)[4]) {
+          __syncwarp();
+  #pragma unroll
+          for (int i = 0; i < 4; ++i) *xaddr(grow + 8 * i, gvec) = t[i];
+          __syncwarp();
+  #pragma unroll
+          for (int j = 0; j < 4; ++j) u[j] = *xaddr(lane, j);
+        };
+        // 32 floats of the row-per-lane layout to bf16 global memory
+        auto store_chunk = [&](__nv_bfloat16* base, long long ld, int cb, const float (&f)[32]) {
+          __syncwarp();
+  #pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *xaddr(lane, j) = make_uint4(pack_bf16x2(f[8 * j], f[8 * j + 1]), pack_bf16x2(f[8 * j + 2], f[8 * j + 3]),
+                                         pack_bf16x2(f[8 * j + 4], f[8 * j + 5]), pack_bf16x2(f[8 * j + 6], f[8 * j + 7]));
+          __syncwarp();
+  #pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint4 t = *xaddr(grow + 8 * i, gvec);
+            if (grows[i] >= 0 && cb + gvec * 8 < ncols_out) {
+              __nv_bfloat16* o = base + static_cast<long long>(grows[i]) * ld + cb + gvec * 8;
+              if (PEERS && p.c_peers > 1 && base == static_cast<__nv_bfloat16*>(p.C) + gofs)   // the row's owner stages it
+                o = static_cast<__nv_bfloat16*>(p.c_peer[grows[i] / p.c_rows]) + gofs +
+                    (static_cast<long long>(p.c_slot) * p.c_rows + grows[i] % p.c_rows) * ld + cb + gvec * 8;
+              *reinterpret_cast<uint4*>(o) = t;
+            }
+          }
+        };
+
+        // The operand the epilogue reads (GELU input of the backward pass, or the residual) does not depend on the
+        // accumulator: pull it into L2 before waiting for the tile, so the DRAM latency hides behind the main loop;
+        // the chunk loop then fetches it (an L2 hit) under the latency of its tcgen05.ld.
+        const bool pre_aux = (p.epi & EPI_MUL_DGELU) != 0;
+        const bool pre_res = !pre_aux && (p.epi & EPI_RESIDUAL) != 0;
+        const __nv_bfloat16* pre_ptr = pre_aux ? p.aux : p.residual;
+        const long long pre_ld = pre_aux ? p.ldaux : p.ldr;
+        if (pre_aux || pre_res) {
+  #pragma unroll
+          for (int ci = 0; ci < CPW; ++ci) {
+            const int c = part + ci * (GEMM_EPI_WARPS / 4);
+            if (c < CHUNKS && n0 + c * 32 < p.N) {
+  #pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (grows[i] >= 0 && n0 + c * 32 + gvec * 8 < ncols_out)
+                  asm volatile("prefetch.global.L2 [%0];" ::"l"(pre_ptr + static_cast<long long>(grows[i]) * pre_ld + n0 + c * 32 + gvec * 8));
+            }
           }
         }
-      };
+        if (mb == 0) {
+          const long long ew0 = clock64();
+          // Every lane polls for itself and may leave the wait in a different iteration; the vote reconverges the warp
+          // before the warp-collective tcgen05.ld below (and makes a failed wait leave the loop as one warp).
+          const bool tile_ready = mbar_wait<PAIR>(&tfull[acc], aph, abort_flag, p.status, 0x400u + acc, mbar_budget);
+          if (!__all_sync(0xffffffffu, tile_ready)) {
+            failed = true;
+            break;
+          }
+          e_wait += clock64() - ew0;
+          tc_fence_after();
+        }
 
-      // The operand the epilogue reads (GELU input of the backward pass, or the residual) does not depend on the
-      // accumulator: pull it into L2 before waiting for the tile, so the DRAM latency hides behind the main loop;
-      // the chunk loop then fetches it (an L2 hit) under the latency of its tcgen05.ld.
-      const bool pre_aux = (p.epi & EPI_MUL_DGELU) != 0;
-      const bool pre_res = !pre_aux && (p.epi & EPI_RESIDUAL) != 0;
-      const __nv_bfloat16* pre_ptr = pre_aux ? p.aux : p.residual;
-      const long long pre_ld = pre_aux ? p.ldaux : p.ldr;
-      if (pre_aux || pre_res) {
-#pragma unroll
+  #pragma unroll
         for (int ci = 0; ci < CPW; ++ci) {
           const int c = part + ci * (GEMM_EPI_WARPS / 4);
-          if (c < CHUNKS && n0 + c * 32 < p.N) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (grows[i] >= 0 && n0 + c * 32 + gvec * 8 < ncols_out)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(pre_ptr + static_cast<long long>(grows[i]) * pre_ld + n0 + c * 32 + gvec * 8));
+          if (c >= CHUNKS || n0 + c * 32 >= p.N) break;   // warp-uniform
+          const int cb = n0 + c * 32;          // first output column of this chunk
+          uint4 pre[4];
+          if (pre_aux || pre_res) fetch_chunk(pre_ptr, pre_ld, cb, pre);
+          if (has_bias) {
+            // one coalesced load per warp and chunk; the 32 values are then read back as broadcast float4
+            float b = 0.f;
+            if (cb + lane < p.N)
+              b = (p.epi & EPI_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + cb + lane)
+                                         : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[cb + lane]);
+            __syncwarp();
+            my_bias[lane] = b;
+            __syncwarp();
           }
-        }
-      }
-      const long long ew0 = clock64();
-      // Every lane polls for itself and may leave the wait in a different iteration; the vote reconverges the warp
-      // before the warp-collective tcgen05.ld below (and makes a failed wait leave the loop as one warp).
-      const bool tile_ready = mbar_wait<PAIR>(&tfull[acc], aph, abort_flag, p.status, 0x400u + acc, mbar_budget);
-      if (!__all_sync(0xffffffffu, tile_ready)) break;
-      e_wait += clock64() - ew0;
-      tc_fence_after();
-
-#pragma unroll
-      for (int ci = 0; ci < CPW; ++ci) {
-        const int c = part + ci * (GEMM_EPI_WARPS / 4);
-        if (c >= CHUNKS || n0 + c * 32 >= p.N) break;   // warp-uniform
-        const int cb = n0 + c * 32;          // first output column of this chunk
-        uint4 pre[4];
-        if (pre_aux || pre_res) fetch_chunk(pre_ptr, pre_ld, cb, pre);
-        if (has_bias) {
-          // one coalesced load per warp and chunk; the 32 values are then read back as broadcast float4
-          float b = 0.f;
-          if (cb + lane < p.N)
-            b = (p.epi & EPI_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + cb + lane)
-                                       : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[cb + lane]);
-          __syncwarp();
-          my_bias[lane] = b;
-          __syncwarp();
-        }
-        uint32_t v[32];
-        tmem_ld_32x32(tmem_base + acc * BN + c * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
-        tmem_ld_wait();
-        float f[32];
-        if (has_bias) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 b4 = *reinterpret_cast<const float4*>(my_bias + j);
-            f[j] = fmaf(__uint_as_float(v[j]), p.alpha, b4.x);
-            f[j + 1] = fmaf(__uint_as_float(v[j + 1]), p.alpha, b4.y);
-            f[j + 2] = fmaf(__uint_as_float(v[j + 2]), p.alpha, b4.z);
-            f[j + 3] = fmaf(__uint_as_float(v[j + 3]), p.alpha, b4.w);
-          }
-        } else if (p.alpha != 1.0f) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * p.alpha;
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-        }
-        if (p.epi & EPI_SAVE_PRE) store_chunk(static_cast<__nv_bfloat16*>(p.C2), p.ldc2, cb, f);
-        if (p.epi & EPI_GELU) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = gelu_erf(f[j]);
-        }
-        if (p.epi & EPI_MUL_DGELU) {
-          uint4 u[4];
-          turn_chunk(pre, u);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t w4[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float2 x = unpack_bf16x2(w4[k]);
-              f[8 * j + 2 * k] *= gelu_erf_grad(x.x);
-              f[8 * j + 2 * k + 1] *= gelu_erf_grad(x.y);
+          uint32_t v[32];
+          tmem_ld_32x32(tmem_base + dcol * BN + c * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
+          tmem_ld_wait();
+          float f[32];
+          if (has_bias) {
+  #pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const float4 b4 = *reinterpret_cast<const float4*>(my_bias + j);
+              f[j] = fmaf(__uint_as_float(v[j]), p.alpha, b4.x);
+              f[j + 1] = fmaf(__uint_as_float(v[j + 1]), p.alpha, b4.y);
+              f[j + 2] = fmaf(__uint_as_float(v[j + 2]), p.alpha, b4.z);
+              f[j + 3] = fmaf(__uint_as_float(v[j + 3]), p.alpha, b4.w);
             }
-          }
-        }
-        if (p.epi & EPI_RESIDUAL) {
-          uint4 u[4];
-          if (pre_res) {
-            turn_chunk(pre, u);
+          } else if (p.alpha != 1.0f) {
+  #pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * p.alpha;
           } else {
-            uint4 t[4];
-            fetch_chunk(p.residual, p.ldr, cb, t);
-            turn_chunk(t, u);
+  #pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
           }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t w4[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float2 x = unpack_bf16x2(w4[k]);
-              f[8 * j + 2 * k] += x.x;
-              f[8 * j + 2 * k + 1] += x.y;
-            }
+          if (p.epi & EPI_SAVE_PRE) store_chunk(static_cast<__nv_bfloat16*>(p.C2), p.ldc2, cb, f);
+          if (p.epi & EPI_GELU) {
+  #pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = gelu_erf(f[j]);
           }
-        }
-        if (p.epi & EPI_OUT_F32) {
-          // fp32 output: two passes of 16 columns through the exchange buffer (4 floats per 16-byte vector)
-          float* obase = static_cast<float*>(p.C) + gofs;
-          const bool vec_ok = ((reinterpret_cast<uintptr_t>(obase) & 15) == 0) && ((p.ldc & 3) == 0);
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              *reinterpret_cast<float4*>(xaddr(lane, j)) =
-                  make_float4(f[16 * hf + 4 * j], f[16 * hf + 4 * j + 1], f[16 * hf + 4 * j + 2], f[16 * hf + 4 * j + 3]);
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 t = *reinterpret_cast<const float4*>(xaddr(grow + 8 * i, gvec));
-              const int col = cb + 16 * hf + gvec * 4;
-              if (grows[i] < 0 || col >= ncols_out) continue;
-              float* o = obase + static_cast<long long>(grows[i]) * p.ldc + col;
-              if (PEERS && p.c_peers > 1)   // the row's owner accumulates it
-                o = static_cast<float*>(p.c_peer[grows[i] / p.c_rows]) + gofs +
-                    static_cast<long long>(grows[i] % p.c_rows) * p.ldc + col;
-              const bool full4 = vec_ok && col + 4 <= ncols_out;
-              if (p.epi & EPI_ATOMIC) {
-                if (full4) {
-                  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o), "f"(t.x), "f"(t.y), "f"(t.z),
-                               "f"(t.w)
-                               : "memory");
-                } else {
-                  const float tv[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-                  for (int e = 0; e < 4; ++e)
-                    if (col + e < ncols_out) atomicAdd(o + e, tv[e]);
-                }
-              } else {
-                if (full4) {
-                  *reinterpret_cast<float4*>(o) = t;
-                } else {
-                  const float tv[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-                  for (int e = 0; e < 4; ++e)
-                    if (col + e < ncols_out) o[e] = tv[e];
-                }
+          if (p.epi & EPI_MUL_DGELU) {
+            uint4 u[4];
+            turn_chunk(pre, u);
+  #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t w4[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+  #pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float2 x = unpack_bf16x2(w4[k]);
+                f[8 * j + 2 * k] *= gelu_erf_grad(x.x);
+                f[8 * j + 2 * k + 1] *= gelu_erf_grad(x.y);
               }
             }
           }
-        } else {
-          store_chunk(static_cast<__nv_bfloat16*>(p.C) + gofs, p.ldc, cb, f);
+          if (p.epi & EPI_RESIDUAL) {
+            uint4 u[4];
+            if (pre_res) {
+              turn_chunk(pre, u);
+            } else {
+              uint4 t[4];
+              fetch_chunk(p.residual, p.ldr, cb, t);
+              turn_chunk(t, u);
+            }
+  #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t w4[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+  #pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float2 x = unpack_bf16x2(w4[k]);
+                f[8 * j + 2 * k] += x.x;
+                f[8 * j + 2 * k + 1] += x.y;
+              }
+            }
+          }
+          if (p.epi & EPI_OUT_F32) {
+            // fp32 output: two passes of 16 columns through the exchange buffer (4 floats per 16-byte vector)
+            float* obase = static_cast<float*>(p.C) + gofs;
+            const bool vec_ok = ((reinterpret_cast<uintptr_t>(obase) & 15) == 0) && ((p.ldc & 3) == 0);
+  #pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+              __syncwarp();
+  #pragma unroll
+              for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float4*>(xaddr(lane, j)) =
+                    make_float4(f[16 * hf + 4 * j], f[16 * hf + 4 * j + 1], f[16 * hf + 4 * j + 2], f[16 * hf + 4 * j + 3]);
+              __syncwarp();
+  #pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float4 t = *reinterpret_cast<const float4*>(xaddr(grow + 8 * i, gvec));
+                const int col = cb + 16 * hf + gvec * 4;
+                if (grows[i] < 0 || col >= ncols_out) continue;
+                float* o = obase + static_cast<long long>(grows[i]) * p.ldc + col;
+                if (PEERS && p.c_peers > 1)   // the row's owner accumulates it
+                  o = static_cast<float*>(p.c_peer[grows[i] / p.c_rows]) + gofs +
+                      static_cast<long long>(grows[i] % p.c_rows) * p.ldc + col;
+                const bool full4 = vec_ok && col + 4 <= ncols_out;
+                if (p.epi & EPI_ATOMIC) {
+                  if (full4) {
+                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o), "f"(t.x), "f"(t.y), "f"(t.z),
+                                 "f"(t.w)
+                                 : "memory");
+                  } else {
+                    const float tv[4] = {t.x, t.y, t.z, t.w};
+  #pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                      if (col + e < ncols_out) atomicAdd(o + e, tv[e]);
+                  }
+                } else {
+                  if (full4) {
+                    *reinterpret_cast<float4*>(o) = t;
+                  } else {
+                    const float tv[4] = {t.x, t.y, t.z, t.w};
+  #pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                      if (col + e < ncols_out) o[e] = tv[e];
+                  }
+                }
+              }
+            }
+          } else {
+            store_chunk(static_cast<__nv_bfloat16*>(p.C) + gofs, p.ldc, cb, f);
+          }
+        }
+        if (Cfg::CAN_COLSUM && p.colsum != nullptr && part == 0 &&
+            first_sum_kb(p, tc, p.groups * p.num_n_tiles) < tc.kb_end) {
+          uint32_t v[32];   // column 0 of the sums accumulator: lane l holds the sum of A's column (row of D) q * 32 + l
+          tmem_ld_32x32(tmem_base + Cfg::SUM_COL0 + dcol * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
+          tmem_ld_wait();
+          const int g = tc.m_blk * GEMM_BM + q * 32 + lane;
+          if (g < p.M) atomicAdd(p.colsum + g, __uint_as_float(v[0]) * p.alpha);
         }
       }
-      if (Cfg::CAN_COLSUM && p.colsum != nullptr && tc.n_blk == 0 && tc.grp == 0 && part == 0) {
-        uint32_t v[32];   // column 0 of the sums accumulator: lane l holds the sum of A's column (row of D) q * 32 + l
-        tmem_ld_32x32(tmem_base + Cfg::SUM_COL0 + acc * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
-        tmem_ld_wait();
-        const int g = tc.m_blk * GEMM_BM + q * 32 + lane;
-        if (g < p.M) atomicAdd(p.colsum + g, __uint_as_float(v[0]) * p.alpha);
-      }
+      if (failed) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -836,18 +890,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 }
 
 // ------------------------------------------------------------------------------ host side
-template <int BN, int CTAS, bool PEERS = false>
+template <int BN, int CTAS, bool PEERS = false, int STACK = 1>
 static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t stream) {
-  using Cfg = GemmCfg<BN, CTAS>;
+  using Cfg = GemmCfg<BN, CTAS, STACK>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, PEERS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::MAX_SMEM);
     if (e != cudaSuccess) return e;
     configured = true;
   }
   GemmParams p = p_in;
-  if (PEERS) p.epi_tma = 0;
+  if (PEERS || STACK > 1) p.epi_tma = 0;
   const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
   p.epi_bufs = p.epi_tma ? Cfg::out_bufs(has_in) + (has_in ? 2 : 0) : 1;
   p.stages = Cfg::stages_for(p.epi_bufs);
@@ -857,7 +911,7 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   const int units = total < max_units ? total : max_units;
   if (units <= 0) return cudaSuccess;
   if (CTAS == 1) {
-    gemm_tcgen05_kernel<BN, CTAS, PEERS><<<units, GEMM_THREADS, p.smem_bytes, stream>>>(p);
+    gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK><<<units, GEMM_THREADS, p.smem_bytes, stream>>>(p);
     return cudaGetLastError();
   }
   cudaLaunchConfig_t cfg = {};
@@ -872,7 +926,7 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, PEERS>, p);
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, p);
 }
 
 cudaError_t gemm_read_stalls(unsigned long long* out8, bool reset) {
@@ -891,6 +945,14 @@ cudaError_t launch_gemm(const GemmParams& p, int bn, int ctas, int num_sms, cuda
       case 128: return launch_bn<128, 2>(p, num_sms, stream);
       case 192: return p.b_mode == OP_KMAJOR_2D ? launch_bn<192, 2>(p, num_sms, stream) : cudaErrorInvalidValue;
       case 256: return launch_bn<256, 2>(p, num_sms, stream);
+      default: return cudaErrorInvalidValue;
+    }
+  }
+  if (p.stack == 2) {
+    switch (bn) {
+      case 128: return launch_bn<128, 1, false, 2>(p, num_sms, stream);
+      case 192: return launch_bn<192, 1, false, 2>(p, num_sms, stream);
+      case 256: return p.colsum == nullptr ? launch_bn<256, 1, false, 2>(p, num_sms, stream) : cudaErrorInvalidValue;
       default: return cudaErrorInvalidValue;
     }
   }

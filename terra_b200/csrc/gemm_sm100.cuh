@@ -32,6 +32,7 @@ struct GemmParams {
   int num_m_tiles, num_n_tiles;
   int m_blocks;                // 128-row blocks of the output (a CTA pair's last tile may reach beyond them)
   int k_blocks;                // total 64-wide k-blocks
+  int stack;                   // 2: tiles of two row blocks (weight gradients), 0 / 1: of one
   int split_k;                 // >1: tiles are (m, n, split); needs EPI_ATOMIC
   int groups;                  // extra outermost tile dimension (conv taps for the weight gradient); >=1
   int a_mode, b_mode;

@@ -40,6 +40,7 @@ struct GemmEpilogue {
   // contraction (sum over tokens of dy[token][n], the bias gradient) into colsum[n] (fp32), from an extra
   // 16-column MMA against a tile of ones. Null: off. Tile widths up to 192.
   float* colsum;
+  int stack;          // weight-gradient form: 2 = tiles of two 128-row blocks that share a tile of B (widths 128, 192; 256 without colsum)
 };
 
 // Tensor-parallel fusions over peer memory. a_ptr[i]: GPU i's [a_rows, K] bf16 shard (K-major, leading dimension of
@@ -83,10 +84,10 @@ int convt2x2_fwd_bf16(const void* x, const void* w, const void* bias4, void* y, 
 int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, int W, int Cin, int Cout, void* status,
                         int num_sms, cudaStream_t stream);
 int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int split_k,
-                        void* status, int num_sms, cudaStream_t stream);
+                        void* status, int num_sms, cudaStream_t stream, int stack = 1);
 int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
                        int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo = nullptr,
-                       const void* halo_hi = nullptr, float* bias_grad = nullptr);   // bias_grad[Cout] += sums of dy
+                       const void* halo_hi = nullptr, float* bias_grad = nullptr, int stack = 1);   // bias_grad[Cout] += sums of dy
 
 // elementwise.cu -------------------------------------------------------------------------------
 // LayerNorm over the last dimension (C <= 8192, C % 8 == 0), bf16 in/out, fp32 statistics.

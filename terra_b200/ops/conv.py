@@ -121,17 +121,18 @@ class _Conv3x3Fn(torch.autograd.Function):
         Cout = weight.shape[0]
         # ---- weight / bias gradients (fp32); the halo rows received in forward serve the boundary taps
         gw, gb = _arena_grad(weight), _arena_grad(bias)
+        split, stack = _wgrad_split(B, H, W, stride, Cout, Cin)
         if gw is not None:
             # tap-major staging [9, Cout, Cin] (persistent, self-cleaning) folded into the arena's (Cout, Cin, 3, 3) view
             dw9 = _zero_scratch(x.device, (9, Cout, Cin), "conv3x3")
             # the bias gradient (column sums of dy) comes out of the same kernel
-            ext.conv3x3_wgrad(x, dy, dw9, stride, _wgrad_split(B, H, W, stride, Cout, Cin), status_word(x.device), lo, hi,
-                              bias_grad=gb if FUSE_BIAS_GRAD else None)
+            ext.conv3x3_wgrad(x, dy, dw9, stride, split, status_word(x.device), lo, hi,
+                              bias_grad=gb if FUSE_BIAS_GRAD else None, stack=stack)
             ext.strided_add(dw9, gw, 1, Cin * 9, 9, True)
             dw = None
         else:
             dw9 = torch.zeros(9, Cout, Cin, device=x.device, dtype=torch.float32)
-            ext.conv3x3_wgrad(x, dy, dw9, stride, _wgrad_split(B, H, W, stride, Cout, Cin), status_word(x.device), lo, hi)
+            ext.conv3x3_wgrad(x, dy, dw9, stride, split, status_word(x.device), lo, hi, stack=stack)
             dw = dw9.view(3, 3, Cout, Cin).permute(2, 3, 0, 1)
         if gb is not None:
             if gw is None or not FUSE_BIAS_GRAD:
@@ -165,12 +166,33 @@ def balanced_split(tiles: int, kblocks: int, sms: int = 148, limit: int = 64) ->
     return best
 
 
+def _stream_cost(heavy, light, bn, split, sms=148):
+    """KB through the most loaded CTA's shared-memory port (operand fill and tensor-core reads) per k-block of the whole
+    contraction, when ``heavy`` tiles of two row blocks are handed out before ``light`` ones of a single block."""
+    one = 2 * (16 + bn // 8)
+    two = 32 + bn // 8 + one
+    return (-(-heavy * split // sms) * (two - one) + -(-(heavy + light) * split // sms) * one) / split
+
+
+def _wgrad_plan(taps, M, N, kblocks):
+    """(split-K factor, row blocks per tile) of a convolution's weight gradient: ``taps`` products of ``M`` x ``N`` outputs.
+    Two row blocks share a tile of the other operand (15 % less traffic per output) where that also comes out ahead with the
+    single block an odd count leaves over and with whole rounds of CTAs; every split adds 0.2 % for its pass of atomics."""
+    bn = 192 if N % 192 == 0 else 128            # the tile width the kernel picks
+    blocks, n = (M + 127) // 128, taps * ((N + bn - 1) // bn)
+    best = balanced_split(blocks * n, kblocks)
+    plan, cost = (best, 1), _stream_cost(0, blocks * n, bn, best) * (1 + 0.002 * best)
+    if N > 64 and blocks >= 2 and (blocks + 1) // 2 * n * kblocks >= 148 * 8:
+        for s in range(1, max(1, min(kblocks, 64)) + 1):
+            c = _stream_cost(blocks // 2 * n, blocks % 2 * n, bn, s) * (1 + 0.002 * s)
+            if c < cost * 0.99:
+                plan, cost = (s, 2), c
+    return plan
+
+
 def _wgrad_split(B, H, W, stride, Cout, Cin):
     Ho, Wo = (H, W) if stride == 1 else ((H + 1) // 2, W // 2)
-    kblocks = B * Ho * ((Wo + 63) // 64)
-    bn = 192 if Cin % 192 == 0 else 128            # the tile width conv3x3_wgrad picks
-    tiles = 9 * ((Cout + 127) // 128) * ((Cin + bn - 1) // bn)
-    return balanced_split(tiles, kblocks)
+    return _wgrad_plan(9, Cout, Cin, B * Ho * ((Wo + 63) // 64))
 
 
 def _conv3x3_s2_dgrad(dy, w16, H, W, dom, weight=None):
@@ -259,9 +281,8 @@ class _ConvT2x2Fn(torch.autograd.Function):
         if tiled:
             # [tap, ci, co] staging -> (Cin, Cout, 2, 2)
             shape, layout = (4, Cin, Cout), (1, Cout * 4, 4)
-            tiles = 4 * ((Cin + 127) // 128) * ((Cout + 191) // 192 if Cout % 192 == 0 else (Cout + 127) // 128)
-            split = balanced_split(tiles, B * H * ((W + 63) // 64))
-            wgrad = lambda dwt: ext.convt2x2_wgrad(x.contiguous(), dy, dwt, split, status_word(x.device))
+            split, stack = _wgrad_plan(4, Cin, Cout, B * H * ((W + 63) // 64))
+            wgrad = lambda dwt: ext.convt2x2_wgrad(x.contiguous(), dy, dwt, split, status_word(x.device), stack)
         else:
             # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it. [tap, co, ci] staging
             dyu = dy.view(B, H, 2, W, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B * H * W, 4 * Cout)

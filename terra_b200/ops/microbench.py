@@ -149,8 +149,9 @@ def case_conv(a):
         dy = _rand(B, Ho, Wo, C, scale=0.1)
         dw = torch.zeros(9, C, C, device="cuda")
         from .conv import _wgrad_split
-        split = a.split if a.split else _wgrad_split(B, H, W, a.stride, C, C)      # the model's choice
-        fn = lambda: ext.conv3x3_wgrad(x, dy, dw, a.stride, split, status_word("cuda"), None, None)
+        split, stack = _wgrad_split(B, H, W, a.stride, C, C)      # the model's choice
+        split = a.split or split
+        fn = lambda: ext.conv3x3_wgrad(x, dy, dw, a.stride, split, status_word("cuda"), None, None, stack=stack)
         nbytes = (x.numel() + dy.numel()) * 2
     else:
         wp = pack_conv3x3_weight(w)

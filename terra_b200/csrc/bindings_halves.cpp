@@ -95,8 +95,10 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 // operand fill plus the tensor core's reads through the shared-memory port, in KB; the column sums add 40 KB per row block,
 // shared out over the column tiles. Every split pays its start and its pass of atomics (about 1000 KB a row block). Widths
 // of 256 leave no room for the sums' accumulators: dy is then read once more (5 TB/s against 3.7 us per 1000 KB).
-// Measured (139264 rows, us): 1152 x 384 unstacked / stacked 125 / 132, 1536 x 384 163 / 155, 384 x 1536 171 / 212 (three
-// row blocks stack badly).
+// Measured (139264 rows, us, sums in the first column tile): 1152 x 384 unstacked / stacked 125 / 132, 1536 x 384 163 / 155,
+// 384 x 1536 171 / 212 (three row blocks stack badly). By this rule, before -> now: 2976 x 384 over 557056 rows
+// 1322 -> 1104, 384 x 2976 1535 (128-wide) -> 1132, 1152 x 384 126 -> 116, 3072 x 1024 over 156672 rows 811 + 176 for the
+// sums -> 817, 3x3 convolution 384 -> 384 at 557056 pixels 1584 -> 1351.
 struct WgradPlan {
   int bn, stack, split;
 };

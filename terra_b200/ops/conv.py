@@ -16,6 +16,7 @@ Reference: models/utils.py:101-180 (``CreditDownBlock`` / ``CreditUpBlock``), cr
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -174,6 +175,7 @@ def _stream_cost(heavy, light, bn, split, sms=148):
     return (-(-heavy * split // sms) * (two - one) + -(-(heavy + light) * split // sms) * one) / split
 
 
+@functools.lru_cache(maxsize=256)
 def _wgrad_plan(taps, M, N, kblocks):
     """(split-K factor, row blocks per tile) of a convolution's weight gradient: ``taps`` products of ``M`` x ``N`` outputs.
     Two row blocks share a tile of the other operand (15 % less traffic per output) where that also comes out ahead with the

@@ -173,7 +173,7 @@ void conv3x3_s2_dgrad(const torch::Tensor& dy, const torch::Tensor& w, torch::Te
 }
 
 // The three products of the 2x2 / stride-2 transposed convolution, x [B, H, W, Cin] and y / dy [B, 2H, 2W, Cout]:
-// op 0: y from x (w: [4 * Cout, Cin_pad], bias [4 * Cout]); op 1: dx from dy (w: [Cin, 4 * Cout_pad])
+// op 0: y from x (w: [4 * Cout_pad, Cin_pad], bias [4 * Cout_pad]); op 1: dx from dy (w: [Cin, 4 * Cout_pad])
 void convt2x2(int64_t op, const torch::Tensor& in, const torch::Tensor& w, const c10::optional<torch::Tensor>& bias4,
               torch::Tensor& out, const c10::optional<torch::Tensor>& status) {
   check_image(in, "in");
@@ -181,10 +181,11 @@ void convt2x2(int64_t op, const torch::Tensor& in, const torch::Tensor& w, const
   const torch::Tensor &x = op == 0 ? in : out, &y = op == 0 ? out : in;
   TORCH_CHECK(x.size(0) == y.size(0) && 2 * x.size(1) == y.size(1) && 2 * x.size(2) == y.size(2), "convt2x2: grids");
   const int64_t Cin = x.size(3), Cout = y.size(3);
-  check_packed(w, op == 0 ? 4 * Cout : Cin, op == 0 ? 1 : 4, op == 0 ? Cin : Cout);
+  const int64_t phase = (Cout + 63) / 64 * 64;
+  check_packed(w, op == 0 ? 4 * phase : Cin, op == 0 ? 1 : 4, op == 0 ? Cin : Cout);
   TORCH_CHECK(op != 0 || (bias4.has_value() && bias4->scalar_type() == torch::kBFloat16 && bias4->is_contiguous() &&
-                          bias4->numel() == 4 * Cout),
-              "convt2x2: bias bf16 [4 * Cout]");
+                          bias4->numel() == 4 * phase),
+              "convt2x2: bias bf16 [4 * Cout_pad]");
   const c10::cuda::CUDAGuard guard(x.device());
   tb::note_launch();
   const int rc = op == 0 ? tb::convt2x2_fwd_bf16(x.data_ptr(), w.data_ptr(), opt_ptr(bias4), out.data_ptr(), x.size(0), x.size(1),

@@ -200,8 +200,9 @@ void unpatchify_crop(const torch::Tensor& patches, const c10::optional<torch::Te
 }
 
 // w: contiguous bf16 storage that every index of the packing stays inside; out: [N1 * N2, T * Cpad] bf16
+// (rows n2 >= valid2 are zero)
 void pack_taps(const torch::Tensor& w, torch::Tensor& out, int64_t n1, int64_t s1, int64_t n2, int64_t s2, int64_t channels,
-               int64_t sc, const std::vector<int64_t>& offsets) {
+               int64_t sc, const std::vector<int64_t>& offsets, int64_t valid2) {
   const int64_t T = static_cast<int64_t>(offsets.size());
   need(w.is_cuda() && w.is_contiguous() && w.scalar_type() == torch::kBFloat16, "pack_taps: w bf16 contiguous");
   need(T >= 1 && T <= 9 && out.is_contiguous() && out.scalar_type() == torch::kBFloat16 && out.dim() == 2 &&
@@ -213,10 +214,11 @@ void pack_taps(const torch::Tensor& w, torch::Tensor& out, int64_t n1, int64_t s
     off[t] = static_cast<int>(offsets[t]);
     top = off[t] > top ? off[t] : top;
   }
-  need(s1 >= 0 && s2 >= 0 && sc >= 0 && (n1 - 1) * s1 + (n2 - 1) * s2 + (channels - 1) * sc + top < w.numel(), "pack_taps: range");
+  need(s1 >= 0 && s2 >= 0 && sc >= 0 && valid2 >= 1 && valid2 <= n2 && (n1 - 1) * s1 + (valid2 - 1) * s2 + (channels - 1) * sc + top < w.numel(), "pack_taps: range");
   const c10::cuda::CUDAGuard guard(w.device());
   tb::note_launch();
-  rc_check(tb::pack_taps_bf16(w.data_ptr(), out.data_ptr(), static_cast<int>(n1), static_cast<int>(n2), static_cast<int>(T),
+  rc_check(tb::pack_taps_bf16(w.data_ptr(), out.data_ptr(), static_cast<int>(n1), static_cast<int>(n2),
+                              static_cast<int>(valid2), static_cast<int>(T),
                               static_cast<int>(channels), static_cast<int>(out.size(1) / T), s1, s2, sc, off, cur_stream()),
            "pack_taps");
 }

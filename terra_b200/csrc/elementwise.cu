@@ -743,10 +743,10 @@ __global__ void add_bf16_kernel(const uint4* __restrict__ a, const uint4* __rest
 }
 
 // Packed operands of the implicit GEMMs: out[(n1 * N2 + n2)][t][c] = w[n1 * s1 + n2 * s2 + c * sc + off[t]], zero for
-// c >= C. One launch per operand and optimizer step (zero fill, permutation, flip and copy were three to five); the reads
+// c >= C and for n2 >= V2 (rows that only pad). One launch per operand and optimizer step (zero fill, permutation, flip and copy were three to five); the reads
 // are strided by the taps, which the caches absorb (a weight is at most a few MB).
 struct PackTaps {
-  int N2, T, C, Cpad;
+  int N2, V2, T, C, Cpad;
   long long s1, s2, sc;
   int off[9];
 };
@@ -761,8 +761,9 @@ __global__ void __launch_bounds__(256) pack_taps_kernel(const __nv_bfloat16* __r
     const long long n = r / p.T;
     const __nv_bfloat16* src = w + n / p.N2 * p.s1 + n % p.N2 * p.s2 + p.off[t];
     __nv_bfloat162 v = __nv_bfloat162(__ushort_as_bfloat16(0), __ushort_as_bfloat16(0));
-    if (c < p.C) v.x = src[c * p.sc];
-    if (c + 1 < p.C) v.y = src[(c + 1) * p.sc];
+    const bool row = n % p.N2 < p.V2;
+    if (row && c < p.C) v.x = src[c * p.sc];
+    if (row && c + 1 < p.C) v.y = src[(c + 1) * p.sc];
     out[i] = *reinterpret_cast<const uint32_t*>(&v);
   }
 }
@@ -1143,10 +1144,10 @@ int patch_relayout(const void* image, const void* add, void* patches, void* imag
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int pack_taps_bf16(const void* w, void* out, int N1, int N2, int T, int C, int Cpad, long long s1, long long s2, long long sc,
+int pack_taps_bf16(const void* w, void* out, int N1, int N2, int V2, int T, int C, int Cpad, long long s1, long long s2, long long sc,
                    const int* offsets, cudaStream_t stream) {
   if (T < 1 || T > 9 || Cpad % 2 != 0 || C > Cpad || N1 < 1 || N2 < 1) return -1;
-  PackTaps p = {N2, T, C, Cpad, s1, s2, sc, {}};
+  PackTaps p = {N2, V2, T, C, Cpad, s1, s2, sc, {}};
   for (int t = 0; t < T; ++t) p.off[t] = offsets[t];
   const long long total = static_cast<long long>(N1) * N2 * T * (Cpad / 2);
   pack_taps_kernel<<<grid_for(total, 256), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(w), static_cast<uint32_t*>(out), p,

@@ -3,6 +3,7 @@
 #include "gemm_sm100.cuh"
 #include "host_api.h"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -33,18 +34,8 @@ static EncodeTiledFn get_encode_fn() {
 
 // rank <= 5, bf16 elements, 128-byte swizzle, zero fill outside the tensor.
 // dims/box are innermost first; strides (bytes) are for dims 1..rank-1.
-static int make_tensor_map_bf16_swizzled(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
-                                         const unsigned long long* strides_bytes, const unsigned int* box,
-                                         CUtensorMapSwizzle swizzle);
-
 int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
                          const unsigned long long* strides_bytes, const unsigned int* box) {
-  return make_tensor_map_bf16_swizzled(out, base, rank, dims, strides_bytes, box, CU_TENSOR_MAP_SWIZZLE_128B);
-}
-
-static int make_tensor_map_bf16_swizzled(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
-                                         const unsigned long long* strides_bytes, const unsigned int* box,
-                                         CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return -1;
   // cuTensorMapEncodeTiled is a driver call: it needs the primary context bound to THIS thread. A thread that
@@ -69,7 +60,7 @@ static int make_tensor_map_bf16_swizzled(CUtensorMap* out, const void* base, int
   for (int i = 0; i + 1 < rank; ++i)
     if (gstr[i] % 16 != 0) return -3;
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(base),
-                  gdim, gstr, bdim, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  gdim, gstr, bdim, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -100 - static_cast<int>(r);
 }
@@ -82,12 +73,12 @@ static int map_2d(CUtensorMap* out, const void* base, long long inner, long long
   return make_tensor_map_bf16(out, base, 2, dims, str, box);
 }
 
-// 32 x 32 chunk of a row-major bf16 matrix in the 64-byte-swizzled layout (the epilogue's staging format)
+// 32 x 64 unit of a row-major bf16 matrix in the 128-byte-swizzled layout (the epilogue's staging format)
 static int map_chunk(CUtensorMap* out, const void* base, long long cols, long long rows, long long ld_elems) {
   unsigned long long dims[2] = {static_cast<unsigned long long>(cols), static_cast<unsigned long long>(rows)};
   unsigned long long str[1] = {static_cast<unsigned long long>(ld_elems) * 2ull};
-  unsigned int box[2] = {32u, 32u};
-  return make_tensor_map_bf16_swizzled(out, base, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+  unsigned int box[2] = {64u, 32u};
+  return make_tensor_map_bf16(out, base, 2, dims, str, box);
 }
 
 // Plain row-major bf16 outputs leave through TMA stores (and the residual / GELU-input operand arrives through TMA
@@ -100,7 +91,7 @@ static void try_tma_epilogue(GemmParams& p, long long M, long long N) {
   p.epi_tma = 0;
   const int f = p.epi;
   if (!enabled || (f & (EPI_OUT_F32 | EPI_ATOMIC | EPI_ROW_CONV))) return;
-  if ((f & EPI_RESIDUAL) && (f & EPI_MUL_DGELU)) return;
+  if (((f & EPI_RESIDUAL) != 0) + ((f & EPI_MUL_DGELU) != 0) + ((f & EPI_SAVE_PRE) != 0) > 1) return;   // one second buffer
   // The input buffers cost the operand ring one or two stages. A long contraction hides the epilogue behind its main
   // loop anyway and wants the deeper ring instead (K = 1536 with a residual measured 15 % slower on three stages).
   if ((f & (EPI_RESIDUAL | EPI_MUL_DGELU)) && p.k_blocks > 12) return;
@@ -134,22 +125,28 @@ static bool pairs_enabled() {
   return on;
 }
 
-// Tile of a plain product with many tiles: the width and CTA count with the fewest cycles per 128 rows, a tile taking the
-// longer of its main loop (operand fill and tensor-core reads through the shared-memory port) and its epilogue (rounds of
-// 32-column chunks over three warps per lane quadrant, by what a chunk does). Measured on 139264 rows, pairs of 192 / 256:
-// 1152 x 384 with bias 126 / 130 us, 3072 x 1024 804 / 645 us; times GELU' 1536 x 384, single 192 / pairs 256: 352 / 364 us.
+// Tile of a plain product with many tiles: the width and CTA count with the fewest cycles per 128 rows. A tile takes the
+// longer of its main loop and its epilogue (rounds of 64-column units over three warps per lane quadrant, by what a unit
+// does). A k-block takes the longest of its MMAs (2 BN cycles), its bytes through the shared-memory port (fill and
+// tensor-core reads at 128 bytes a cycle) and about 450 cycles of hand-over. Measured on 139264 rows (us): pairs of 192 / 256
+// 1152 x 384 with bias 128 / 133, 384 x 384 with residual 66 / 86, 3072 x 1024 804 / 645; 2976 x 384 with residual on
+// 278528 rows 848 / 1038; times GELU', 1536 x 384, single 192 / pairs of 256 290 / 327.
 static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, int num_sms, int* bn_out, int* ctas_out) {
   *bn_out = pick_bn(N, 0);
   *ctas_out = 1;
+  const bool second = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU | EPI_SAVE_PRE)) != 0;
+  // the ring keeps too little beside two units per epilogue warp when single tiles are 256 wide
+  if (*bn_out == 256 && second && k_blocks <= 12) *bn_out = 192;
   if (!pairs_enabled() || N < 128 || ((m_blocks + 1) / 2) * ((N + 255) / 256) < 8LL * (num_sms / 2)) return;
-  const long long chunk = (flags & EPI_MUL_DGELU) ? 4500 : (flags & EPI_SAVE_PRE) ? 3800 : (flags & EPI_RESIDUAL) ? 3500 : 1800;
+  const long long unit = (flags & EPI_MUL_DGELU) ? 4500 : (flags & EPI_SAVE_PRE) ? 3500 : (flags & EPI_RESIDUAL) ? 2500 : 2000;
   long long best = 0;
   for (int ctas : {2, 1})
     for (int bn : {256, 192, 128}) {
       if (ctas == 2 && b_mn && bn == 192) continue;      // half of an MN-major B must be whole 64-row boxes
-      const long long loop = static_cast<long long>(k_blocks) * 16 * (16 + bn / (8 * ctas));
-      const long long epilogue = chunk * ((bn / 32 + 2) / 3);
-      const long long cost = (N + bn - 1) / bn * (loop > epilogue ? loop : epilogue);
+      if (ctas == 1 && bn == 256 && second) continue;
+      const long long port = 16 * (16 + bn / (8 * ctas));
+      const long long loop = k_blocks * std::max(450LL, std::max(2LL * bn, port));
+      const long long cost = (N + bn - 1) / bn * std::max(loop, unit * ((bn / 64 + 2) / 3));
       if (best == 0 || cost < best) {
         best = cost;
         *bn_out = bn;
@@ -385,14 +382,14 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   p.phase_cols = c.phase_cols;
   std::memcpy(p.out_off, c.out_off, sizeof(p.out_off));
   if (!(p.epi & ~(EPI_ROW_CONV | EPI_BIAS | EPI_BIAS_F32))) {
-    // 32 pixels x 32 channels per store; rows and channels outside the image are clipped
+    // 32 pixels x 64 channels per store; rows and channels outside the image are clipped
     const unsigned long long C = static_cast<unsigned long long>(c.out_c), mul = static_cast<unsigned long long>(c.out_mul);
     const unsigned long long row = C * 2ull * mul * c.out_w;
     unsigned long long dims[5] = {C, mul, static_cast<unsigned long long>(c.out_w), static_cast<unsigned long long>(c.out_h),
                                   static_cast<unsigned long long>(c.B)};
     unsigned long long str[4] = {C * 2ull, C * 2ull * mul, row, row * c.out_h};
-    unsigned int box[5] = {32, 1, 32, 1, 1};
-    rc = make_tensor_map_bf16_swizzled(&p.map_c, c.y, 5, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+    unsigned int box[5] = {64, 1, 32, 1, 1};
+    rc = make_tensor_map_bf16(&p.map_c, c.y, 5, dims, str, box);
     if (rc != 0) return rc - 5000;
     p.epi_tma = 2;
   } else if (c.out_mul != 1 || c.phase_cols != 0) {
@@ -439,13 +436,13 @@ int conv3x3_s2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H,
   return gather_conv(c, epi, num_sms, stream, nullptr, nullptr);
 }
 
-// 2x2 / stride-2 transposed convolution: x [B, H, W, Cin] -> y [B, 2H, 2W, Cout]; w: [4 * Cout, Cin_pad], rows (dy, dx, co);
-// bias: [4 * Cout]. One tap, the four output phases side by side in N.
+// 2x2 / stride-2 transposed convolution: x [B, H, W, Cin] -> y [B, 2H, 2W, Cout]; w: [4 * Cout_pad, Cin_pad], rows (dy, dx, co);
+// bias: [4 * Cout_pad] (padded to multiples of 64; the padding columns are clipped by the store). One tap, the four output phases side by side in N.
 int convt2x2_fwd_bf16(const void* x, const void* w, const void* bias4, void* y, int B, int H, int W, int Cin, int Cout,
                       void* status, int num_sms, cudaStream_t stream) {
-  if (Cout % 32 != 0) return -13;             // a 32-column chunk of the epilogue lies inside one phase
+  const int pad = (Cout + 63) / 64 * 64;      // a 64-column unit of the epilogue lies inside one phase
   const Tap tap = {0, 0, 0};
-  GatherConv c = {x, B, H, W, Cin, 1, H, W, 1, &tap, 1, 1, {0, 1}, w, 4 * Cout, y, 2 * H, W, Cout, 2, Cout,
+  GatherConv c = {x, B, H, W, Cin, 1, H, W, 1, &tap, 1, 1, {0, 1}, w, 4 * pad, y, 2 * H, W, Cout, 2, pad,
                   {{0, 0}, {0, 1}, {1, 0}, {1, 1}}};
   GemmEpilogue epi = {};
   epi.flags = EPI_BIAS;

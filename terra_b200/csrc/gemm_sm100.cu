@@ -55,9 +55,9 @@ struct GemmCfg {
   static constexpr int B_BYTES = B_ROWS * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   // After the operand ring: 512 bytes of barriers, the per-warp bias slots (together 2 KB), then `bufs` buffers of
-  // 2 KB per epilogue warp: one or two output staging buffers (one: also the exchange buffer of the per-lane epilogue),
-  // and two more for the operand the epilogue reads, loaded ahead by TMA. The ring takes what is left: the launcher
-  // passes the stage count to the kernel.
+  // 2 KB per epilogue warp: one (the exchange buffer of the per-lane epilogue), or two (a 32 x 64 unit of the output on its
+  // way to a TMA store), or four (another such unit: the saved pre-activation, or the operand the epilogue reads). The
+  // ring takes what is left: the launcher passes the stage count to the kernel.
   static constexpr int BAR_BYTES = 512;
   static constexpr int FIXED_BASE = 2048;
   static constexpr int EPI_BUF = 2048;
@@ -74,17 +74,11 @@ struct GemmCfg {
   static constexpr int SUM_COL0 = 2 * BN;
   static constexpr int TMEM_COLS = (2 * BN + 64 <= 256) ? 256 : 512;
   static constexpr bool CAN_COLSUM = CTAS == 1 && 2 * BN + 64 <= 512;
-  static_assert((STACK == 2 ? stages_for(1) : stages_for(3)) >= 3 && smem_bytes(1) <= MAX_SMEM && smem_bytes(3) <= MAX_SMEM, "shared memory budget");
+  static_assert((STACK == 2 ? stages_for(1) : stages_for(2)) >= 3 && smem_bytes(1) <= MAX_SMEM && smem_bytes(2) <= MAX_SMEM, "shared memory budget");
   static_assert(GEMM_EPI_WARPS * 32 * 4 + BAR_BYTES <= FIXED_BASE, "bias slots");
   // a CTA's half of an MN-major B must be whole 64-row boxes; K-major rows only need whole 8-row swizzle atoms
   static constexpr bool CAN_B_MN = B_ROWS % 64 == 0;
   static_assert(B_ROWS % 8 == 0 && B_BYTES % 1024 == 0, "B tile: whole swizzle atoms");
-  // Output staging buffers per epilogue warp. Two let a chunk be written while the store of the chunk before is still
-  // reading its buffer (that read takes several hundred cycles); not where they would cost an operand stage out of four.
-  static constexpr int out_bufs(bool has_in) {
-    const int in = has_in ? 2 : 0;
-    return (stages_for(2 + in) >= 4 || stages_for(2 + in) == stages_for(1 + in)) ? 2 : 1;
-  }
 };
 
 // Cycle counters of the three roles, summed over CTAs and launches since the last reset (read by gemm_read_stalls):
@@ -149,10 +143,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   uint64_t* tfull = empty + Cfg::MAX_STAGES;
   uint64_t* tempty = tfull + 2;
   uint64_t* pfull = tempty + 2;   // pair mode, leader CTA: "the peer's half of stage s has landed"
-  uint64_t* in_bar = pfull + Cfg::MAX_STAGES;   // two per epilogue warp: "the epilogue operand chunk has landed"
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(in_bar + 2 * GEMM_EPI_WARPS);
+  uint64_t* in_bar = pfull + Cfg::MAX_STAGES;   // one per epilogue warp: "the epilogue operand's unit has landed"
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(in_bar + GEMM_EPI_WARPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((3 * Cfg::MAX_STAGES + 4 + 2 * GEMM_EPI_WARPS) * 8 + 8 <= Cfg::BAR_BYTES, "barrier block");
+  static_assert((3 * Cfg::MAX_STAGES + 4 + GEMM_EPI_WARPS) * 8 + 8 <= Cfg::BAR_BYTES, "barrier block");
   float* bias_slots = reinterpret_cast<float*>(fixed + Cfg::BAR_BYTES);
   uint8_t* xchg = fixed + Cfg::FIXED_BASE;
   // The ring needs a 1024-byte aligned base (128-byte swizzle atoms). The dynamic window normally starts aligned; if
@@ -175,7 +169,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       mbar_init(&empty[s], 1);
       mbar_init(&pfull[s], 1);
     }
-    for (int i = 0; i < 2 * GEMM_EPI_WARPS; ++i) mbar_init(&in_bar[i], 1);
+    for (int i = 0; i < GEMM_EPI_WARPS; ++i) mbar_init(&in_bar[i], 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
       mbar_init(&tempty[a], GEMM_EPI_WARPS * CTAS);   // pair mode: both CTAs' epilogue warps release the leader's
@@ -438,90 +432,64 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
     };
     constexpr int CPW = (CHUNKS + GEMM_EPI_WARPS / 4 - 1) / (GEMM_EPI_WARPS / 4);   // chunks per warp
     if (!PEERS && STACK == 1 && p.epi_tma) {
-      // ---- plain row-major bf16 outputs: chunks leave (and the operand the epilogue reads arrives) through TMA.
-      // A chunk is 32 rows of 64 bytes in the 64-byte-swizzled layout, which is also conflict-free for the
-      // row-per-lane 16-byte accesses of the warp. The warp's first one or two buffers stage outputs in turn: one lane
-      // issues the store and, before a buffer is written again, waits until its store has read it. The last two receive
-      // the input operand two chunks ahead (across tiles), so its latency hides behind the chunks in between.
+      // ---- bf16 outputs through TMA, and the operand the epilogue reads. A warp works on units of 32 rows x 64 columns (128
+      // bytes per row in the 128-byte-swizzled layout, conflict-free for the row-per-lane 16-byte accesses). Tiles of 192
+      // columns are one unit per warp and tile, so a buffer has a whole tile's time to drain or fill. Against 32-column
+      // chunks (three uneven rounds at width 256, two at 192): 278528 x 2976 x 384 with residual 1061 -> 848 us, 139264 x
+      // 1536 x 384 times GELU' 352 -> 290, 139264 x 384 x 384 with residual 72 -> 66, 17280 x 768 x 192 with GELU 30 -> 24.
+      // The warp's first 4 KB stage the output; one lane issues the store and, before the buffer is written again, waits
+      // until the store has read it. The second 4 KB stage the saved pre-activation, or receive the input unit, loaded as
+      // soon as the unit before has been read (across tiles), so its latency hides behind the main loop.
+      constexpr int UNITS = BN / 64, WARPS_PER_Q = GEMM_EPI_WARPS / 4;
       const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
-      const bool two_out = p.epi_bufs == (has_in ? 4 : 2);
-      uint8_t* my_bufs = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
-      uint8_t* in_bufs = my_bufs + (two_out ? 2 : 1) * Cfg::EPI_BUF;
-      uint64_t* my_in = in_bar + (warp - 2) * 2;
-      const uint32_t row_off = static_cast<uint32_t>(lane) * 64u;
-      const uint32_t swz = (static_cast<uint32_t>(lane) >> 1) & 3u;
-      const uint32_t out_addr = smem_u32(my_bufs);
-      uint32_t issued = 0, consumed = 0, stored = 0;
-      int pf_tile = unit, pf_ci = 0, pf_n0 = 0, pf_row = 0;
-      auto prefetch_next = [&]() {   // issue the load of this warp's next input chunk, if there is one
+      uint8_t* my_out = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
+      uint8_t* my_second = my_out + 2 * Cfg::EPI_BUF;
+      uint64_t* my_in = in_bar + (warp - 2);
+      const uint32_t row_off = static_cast<uint32_t>(lane) * 128u;
+      const uint32_t swz = static_cast<uint32_t>(lane) & 7u;
+      uint32_t consumed = 0;
+      int pf_tile = unit, pf_u = part, pf_n0 = 0, pf_row = 0;
+      auto prefetch_next = [&]() {   // issue the load of this warp's next input unit, if there is one
         while (pf_tile < total_tiles) {
-          if (pf_ci == 0) {      // the divisions once per tile
+          if (pf_u == part) {        // the divisions once per tile
             const TileCoord t = decode_tile(p, pf_tile, CTAS, rank);
             pf_n0 = t.n_blk * BN;
             pf_row = t.m_blk * GEMM_BM + q * 32;
           }
-          const int c = part + pf_ci * (GEMM_EPI_WARPS / 4);
-          const int col = pf_n0 + c * 32, row = pf_row;
-          const bool ok = c < CHUNKS && col < p.N;
-          if (++pf_ci >= CPW) {
-            pf_ci = 0;
+          const int col = pf_n0 + pf_u * 64, row = pf_row;
+          const bool ok = pf_u < UNITS && col < p.N;
+          pf_u += WARPS_PER_Q;
+          if (pf_u >= UNITS) {
+            pf_u = part;
             pf_tile += units;
           }
           if (ok) {
             if (lane == 0) {
-              uint64_t* b = my_in + (issued & 1u);
-              mbar_expect_tx(b, Cfg::EPI_BUF);
-              tma_load_2d(in_bufs + Cfg::EPI_BUF * (issued & 1u), &p.map_in, b, col, row);
+              mbar_expect_tx(my_in, 2 * Cfg::EPI_BUF);
+              tma_load_2d(my_second, &p.map_in, my_in, col, row);
             }
-            ++issued;
             return;
           }
         }
       };
-      auto stage_store = [&](const CUtensorMap* map, const float (&f)[32], int col, int row, int at_tile) {
-        if (lane == 0) {
-          if (two_out) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
-        }
-        __syncwarp();
-        const uint32_t dst = out_addr + (two_out ? (stored & 1u) * Cfg::EPI_BUF : 0u);
-        ++stored;
+      auto stage_half = [&](uint8_t* buf, const float (&f)[32], int h) {
+        const uint32_t base = smem_u32(buf) + row_off;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const uint32_t a = dst + row_off + (((static_cast<uint32_t>(j) ^ swz) & 3u) << 4);
+          const uint32_t a = base + (((static_cast<uint32_t>(4 * h + j)) ^ swz) << 4);
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(pack_bf16x2(f[8 * j], f[8 * j + 1])),
                        "r"(pack_bf16x2(f[8 * j + 2], f[8 * j + 3])), "r"(pack_bf16x2(f[8 * j + 4], f[8 * j + 5])),
                        "r"(pack_bf16x2(f[8 * j + 6], f[8 * j + 7]))
                        : "memory");
         }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {   // a group per chunk, also where the rows lie outside the output: the waits count groups
-          if (p.epi_tma == 2) {
-            // 32 consecutive pixels of an image row (decoded again by this one lane: nothing of it is kept in registers)
-            const TileCoord t = decode_tile(p, at_tile, CTAS, rank);
-            const int phase = p.phase_cols > 0 ? col / p.phase_cols : t.grp;
-            const int w = (t.m_blk % p.tile_n0) * GEMM_BM + q * 32;
-            const int h = (t.m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0];
-            if (t.m_blk < p.m_blocks && w < p.out_w && h < p.out_h)
-              tma_store_5d(map, dst, p.phase_cols > 0 ? col - phase * p.phase_cols : col, p.out_off[phase][1], w, h,
-                           t.m_blk / (p.tile_n0 * p.tile_n1));
-          } else if (row < p.M) {
-            tma_store_2d(map, dst, col, row);
-          }
-          bulk_commit_group();
-        }
       };
-      if (has_in) {
-        prefetch_next();
-        prefetch_next();
-      }
+      if (has_in) prefetch_next();
       bool failed = false;
       for (int tile = unit; tile < total_tiles && !failed; tile += units, ++tcount) {
         const TileCoord tc = decode_tile(p, tile, CTAS, rank);
         const int acc = tcount & 1;
         const uint32_t aph = (tcount >> 1) & 1u;
         const int n0 = tc.n_blk * BN;
-        const int row0 = tc.m_blk * GEMM_BM + q * 32;
         const long long ew0 = clock64();
         const bool tile_ready = mbar_wait<PAIR>(&tfull[acc], aph, abort_flag, p.status, 0x400u + acc, mbar_budget);
         if (!__all_sync(0xffffffffu, tile_ready)) break;
@@ -535,88 +503,111 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             if (PAIR && rank == 1) mbar_arrive_remote(map_to_cta(&tempty[acc], 0));   // the leader's MMA thread waits
             else mbar_arrive(&tempty[acc]);
           }
+          released = true;
         };
-        // (not unrolled: one copy of the chunk's code stays in the instruction cache of the twelve warps)
 #pragma unroll 1
-        for (int ci = 0; ci < CPW; ++ci) {
-          const int c = part + ci * (GEMM_EPI_WARPS / 4);
-          if (c >= CHUNKS || n0 + c * 32 >= p.N) break;   // warp-uniform
-          const int nb = n0 + c * 32;
-          const bool last = (ci + 1 >= CPW) || (c + GEMM_EPI_WARPS / 4 >= CHUNKS) || (nb + 32 * (GEMM_EPI_WARPS / 4) >= p.N);
-          if (has_bias) {
-            float b = 0.f;
-            if (nb + lane < p.N)
-              b = (p.epi & EPI_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + nb + lane)
-                                         : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[nb + lane]);
-            __syncwarp();
-            my_bias[lane] = b;
-            __syncwarp();
-          }
-          uint32_t v[32];
-          tmem_ld_32x32(tmem_base + acc * BN + c * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
-          uint4 u[4];
+        for (int u = part; u < UNITS && n0 + u * 64 < p.N; u += WARPS_PER_Q) {   // warp-uniform
+          const int nb0 = n0 + u * 64;
+          const bool last = u + WARPS_PER_Q >= UNITS || nb0 + 64 * WARPS_PER_Q >= p.N;
+          if (lane == 0) bulk_wait_group_read<0>();
+          __syncwarp();
           if (has_in) {
-            const uint32_t b = consumed & 1u;
-            const bool in_ready =
-                mbar_wait<false>(&my_in[b], (consumed >> 1) & 1u, abort_flag, p.status, 0x600u + b, mbar_budget);
+            const bool in_ready = mbar_wait<false>(my_in, consumed & 1u, abort_flag, p.status, 0x600u, mbar_budget);
             if (!__all_sync(0xffffffffu, in_ready)) {
-              tmem_ld_wait();
               failed = true;
               break;
             }
-            const uint32_t src = smem_u32(in_bufs + Cfg::EPI_BUF * b) + row_off;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint32_t a = src + (((static_cast<uint32_t>(j) ^ swz) & 3u) << 4);
-              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(u[j].x), "=r"(u[j].y), "=r"(u[j].z), "=r"(u[j].w)
-                           : "r"(a)
-                           : "memory");
-            }
             ++consumed;
           }
-          tmem_ld_wait();
-          if (last) {
-            release();
-            released = true;
-          }
-          float f[32];
-          const f32x2 alpha2 = f2_pack(p.alpha, p.alpha);
-          if (has_bias) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 b4 = *reinterpret_cast<const float4*>(my_bias + j);
-              f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2, f2_pack(b4.x, b4.y)), f[j], f[j + 1]);
-              f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), alpha2, f2_pack(b4.z, b4.w)), f[j + 2], f[j + 3]);
+          // (one copy of the half's code stays in the instruction cache of the twelve warps)
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            const int nb = nb0 + 32 * h;
+            if (nb >= p.N) break;   // warp-uniform
+            if (has_bias) {
+              float b = 0.f;
+              if (nb + lane < p.N)
+                b = (p.epi & EPI_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + nb + lane)
+                                           : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[nb + lane]);
+              __syncwarp();
+              my_bias[lane] = b;
+              __syncwarp();
             }
-          } else {
+            uint32_t v[32];
+            tmem_ld_32x32(tmem_base + acc * BN + u * 64 + h * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
+            uint4 in[4];
+            if (has_in) {
+              const uint32_t base = smem_u32(my_second) + row_off;
 #pragma unroll
-            for (int j = 0; j < 32; j += 2)
-              f2_unpack(f2_mul(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2), f[j], f[j + 1]);
-          }
-          if (p.epi & EPI_SAVE_PRE) stage_store(&p.map_c2, f, nb, row0, tile);
-          if (p.epi & EPI_GELU) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) f2_unpack(gelu_erf2(f2_pack(f[j], f[j + 1])), f[j], f[j + 1]);
-          }
-          if (has_in) {
-            const bool dgelu = (p.epi & EPI_MUL_DGELU) != 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint32_t w4[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float2 x = unpack_bf16x2(w4[k]);
-                const f32x2 f2 = f2_pack(f[8 * j + 2 * k], f[8 * j + 2 * k + 1]), x2 = f2_pack(x.x, x.y);
-                f2_unpack(dgelu ? f2_mul(f2, gelu_erf_grad2(x2)) : f2_add(f2, x2), f[8 * j + 2 * k], f[8 * j + 2 * k + 1]);
+              for (int j = 0; j < 4; ++j) {
+                const uint32_t a = base + (((static_cast<uint32_t>(4 * h + j)) ^ swz) << 4);
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(in[j].x), "=r"(in[j].y), "=r"(in[j].z), "=r"(in[j].w)
+                             : "r"(a)
+                             : "memory");
               }
             }
-            __syncwarp();        // every lane holds its part of the input chunk: its buffer may be refilled
-            prefetch_next();
+            tmem_ld_wait();
+            if (last && (h == 1 || nb + 32 >= p.N)) release();
+            float f[32];
+            const f32x2 alpha2 = f2_pack(p.alpha, p.alpha);
+            if (has_bias) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 4) {
+                const float4 b4 = *reinterpret_cast<const float4*>(my_bias + j);
+                f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2, f2_pack(b4.x, b4.y)), f[j],
+                          f[j + 1]);
+                f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), alpha2, f2_pack(b4.z, b4.w)),
+                          f[j + 2], f[j + 3]);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; j += 2)
+                f2_unpack(f2_mul(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2), f[j], f[j + 1]);
+            }
+            if (p.epi & EPI_SAVE_PRE) stage_half(my_second, f, h);
+            if (p.epi & EPI_GELU) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 2) f2_unpack(gelu_erf2(f2_pack(f[j], f[j + 1])), f[j], f[j + 1]);
+            }
+            if (has_in) {
+              const bool dgelu = (p.epi & EPI_MUL_DGELU) != 0;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint32_t w4[4] = {in[j].x, in[j].y, in[j].z, in[j].w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const float2 x = unpack_bf16x2(w4[k]);
+                  const f32x2 f2 = f2_pack(f[8 * j + 2 * k], f[8 * j + 2 * k + 1]), x2 = f2_pack(x.x, x.y);
+                  f2_unpack(dgelu ? f2_mul(f2, gelu_erf_grad2(x2)) : f2_add(f2, x2), f[8 * j + 2 * k], f[8 * j + 2 * k + 1]);
+                }
+              }
+            }
+            stage_half(my_out, f, h);
           }
-          stage_store(&p.map_c, f, nb, row0, tile);
+          fence_proxy_async_smem();
+          __syncwarp();          // the unit is staged, and every lane holds its part of the input: its buffer may be refilled
+          if (lane == 0) {
+            if (p.epi_tma == 2) {
+              // 32 consecutive pixels of an image row (decoded by this one lane)
+              const int phase = p.phase_cols > 0 ? nb0 / p.phase_cols : tc.grp;
+              const int w = (tc.m_blk % p.tile_n0) * GEMM_BM + q * 32;
+              const int h = (tc.m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0];
+              if (tc.m_blk < p.m_blocks && w < p.out_w && h < p.out_h)
+                tma_store_5d(&p.map_c, smem_u32(my_out), p.phase_cols > 0 ? nb0 - phase * p.phase_cols : nb0, p.out_off[phase][1], w,
+                             h, tc.m_blk / (p.tile_n0 * p.tile_n1));
+            } else {
+              const int row0 = tc.m_blk * GEMM_BM + q * 32;
+              if (row0 < p.M) {
+                if (p.epi & EPI_SAVE_PRE) tma_store_2d(&p.map_c2, smem_u32(my_second), nb0, row0);
+                tma_store_2d(&p.map_c, smem_u32(my_out), nb0, row0);
+              }
+            }
+            bulk_commit_group();
+          }
+          if (has_in) prefetch_next();
         }
-        if (!released && !failed) release();   // a warp without a chunk in this tile (narrow last column tile)
+        if (!released && !failed) release();   // a warp without a unit in this tile
       }
       if (lane == 0) bulk_wait_group_read<0>();
     } else
@@ -902,8 +893,11 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   }
   GemmParams p = p_in;
   if (PEERS || STACK > 1) p.epi_tma = 0;
-  const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
-  p.epi_bufs = p.epi_tma ? Cfg::out_bufs(has_in) + (has_in ? 2 : 0) : 1;
+  p.epi_bufs = p.epi_tma == 0 ? 1 : ((p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU | EPI_SAVE_PRE)) ? 4 : 2);
+  if (p.epi_tma == 1 && Cfg::stages_for(p.epi_bufs) < 3) {   // single-CTA tiles 256 wide: the ring needs the room
+    p.epi_tma = 0;
+    p.epi_bufs = 1;
+  }
   p.stages = Cfg::stages_for(p.epi_bufs);
   p.smem_bytes = Cfg::smem_bytes(p.epi_bufs);
   const int total = p.groups * p.num_m_tiles * p.num_n_tiles * p.split_k;

@@ -65,10 +65,10 @@ struct GemmParams {
   int grp_kb[5];
   float alpha;
   KernelStatus* status;
-  // Epilogue through TMA (plain row-major bf16 outputs): every epilogue warp stages its 32 x 32 chunk in shared memory in
-  // the 64-byte-swizzled layout and one lane stores it through map_c / map_c2; the operand the epilogue reads (residual,
-  // or the GELU input of the backward pass) arrives through map_in, loaded two chunks ahead into per-warp buffers.
-  // epi_bufs = buffers of 2 KB per epilogue warp (1 or 2: output staging; + two where there is an input).
+  // Epilogue through TMA: every epilogue warp stages units of 32 rows x 64 columns in shared memory in the 128-byte-swizzled
+  // layout and one lane stores them through map_c / map_c2; the operand the epilogue reads (residual, or the GELU input of
+  // the backward pass) arrives through map_in. epi_bufs = buffers of 2 KB per epilogue warp (2: the output's unit; 4: and
+  // that of the pre-activation or the input; 1: no TMA).
   // stages / smem_bytes: the launcher sizes the operand ring with what the epilogue buffers leave.
   float* colsum;               // weight-gradient form: += column sums of operand A over the contraction (see GemmEpilogue)
   CUtensorMap map_c, map_c2, map_in;

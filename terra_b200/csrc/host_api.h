@@ -183,8 +183,8 @@ int window_attn_tc_bwd(const WindowAttnArgs& a, void* status, cudaStream_t strea
 // with `add` (an image, or null) added.
 int patch_relayout(const void* image, const void* add, void* patches, void* image_out, int to_patches, int B, int H, int W, int C,
                    int p, int Hp, int Wp, int top, int left, cudaStream_t stream);
-// out[n1 * N2 + n2][t][c] = w[n1 * s1 + n2 * s2 + c * sc + offsets[t]] (bf16), zeros for C <= c < Cpad
-int pack_taps_bf16(const void* w, void* out, int N1, int N2, int T, int C, int Cpad, long long s1, long long s2, long long sc,
+// out[n1 * N2 + n2][t][c] = w[n1 * s1 + n2 * s2 + c * sc + offsets[t]] (bf16), zeros for C <= c < Cpad and n2 >= V2
+int pack_taps_bf16(const void* w, void* out, int N1, int N2, int V2, int T, int C, int Cpad, long long s1, long long s2, long long sc,
                    const int* offsets, cudaStream_t stream);
 // drow[row, head] = sum over the head's channels of dO * O (bf16 [rows, C] inputs, fp32 [rows, heads] output).
 int attn_rowdot(const void* o, const void* dout, float* drow, long long rows, int C, int heads, cudaStream_t stream);

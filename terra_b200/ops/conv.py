@@ -34,19 +34,20 @@ _MAX_TAP_CHUNKS = 128       # (tap, 64-channel chunk) entries of the implicit GE
 
 
 # ------------------------------------------------------------------------------------------------ weight packing
-def _pack_taps(w, n1, s1, n2, s2, channels, sc, offsets):
+def _pack_taps(w, n1, s1, n2, s2, channels, sc, offsets, pad2=None):
     """bf16 ``[n1 * n2, taps * C_pad]`` with ``out[i * n2 + j, t, c] = w.flatten()[i * s1 + j * s2 + c * sc + offsets[t]]``, the
-    channels padded to a multiple of 64 with zeros."""
+    channels padded to a multiple of 64 with zeros, and the ``n2`` rows of every ``i`` to ``pad2``."""
+    valid2, n2 = n2, pad2 or n2
     cpad, taps = (channels + 63) // 64 * 64, len(offsets)
     if w.is_cuda and w.dtype == torch.bfloat16:
         out = torch.empty(n1 * n2, taps * cpad, device=w.device, dtype=torch.bfloat16)
-        _ext.load().pack_taps(w.contiguous(), out, n1, s1, n2, s2, channels, sc, list(offsets))
+        _ext.load().pack_taps(w.contiguous(), out, n1, s1, n2, s2, channels, sc, list(offsets), valid2)
         return out
-    steps = [(n1, s1), (n2, s2), (1, 0), (channels, sc)]
+    steps = [(n1, s1), (valid2, s2), (1, 0), (channels, sc)]
     at = sum(torch.arange(n, device=w.device).view([-1 if d == e else 1 for e in range(4)]) * s for d, (n, s) in enumerate(steps))
     at = at + torch.tensor(list(offsets), device=w.device).view(1, 1, -1, 1)
-    out = torch.zeros(n1 * n2, taps, cpad, device=w.device, dtype=torch.bfloat16)
-    out[:, :, :channels] = w.reshape(-1)[at.reshape(-1)].view(n1 * n2, taps, channels)
+    out = torch.zeros(n1, n2, taps, cpad, device=w.device, dtype=torch.bfloat16)
+    out[:, :valid2, :, :channels] = w.reshape(-1)[at.reshape(-1)].view(n1, valid2, taps, channels)
     return out.view(n1 * n2, taps * cpad)
 
 
@@ -245,9 +246,9 @@ def conv3x3(x, conv: torch.nn.Conv2d, stride: int = 1, dom=None):
 
 # ------------------------------------------------------------------------------------------------ transposed conv 2x2 / s2
 def _convt_tiled(Cin, Cout):
-    """The gathered forms: a 32-column chunk of the forward epilogue must lie in one (dy, dx) phase, and the (tap, channel
-    chunk) tables must hold the layer. Other channel counts go through a plain GEMM and permuted copies."""
-    return Cout % 32 == 0 and Cin % 8 == 0 and max(4 * ((Cout + 63) // 64), (Cin + 63) // 64) <= _MAX_TAP_CHUNKS
+    """The gathered forms: the (tap, channel chunk) tables must hold the layer. Larger channel counts go through a plain GEMM
+    and permuted copies."""
+    return Cout % 8 == 0 and Cin % 8 == 0 and max(4 * ((Cout + 63) // 64), (Cin + 63) // 64) <= _MAX_TAP_CHUNKS
 
 
 class _ConvT2x2Fn(torch.autograd.Function):
@@ -258,13 +259,15 @@ class _ConvT2x2Fn(torch.autograd.Function):
         Cout = weight.shape[1]
         w16 = weight.bf16 if getattr(weight, "bf16", None) is not None else weight.detach().to(torch.bfloat16)
         b16 = bias.bf16 if getattr(bias, "bf16", None) is not None else bias.detach().to(torch.bfloat16)
-        b4 = _packed(bias, b16, "convT_bias", lambda b: b.repeat(4))
         y = torch.empty(B, 2 * H, 2 * W, Cout, device=x.device, dtype=torch.bfloat16)
         if _convt_tiled(Cin, Cout):
-            # rows (dy, dx, co); the epilogue stores every phase to its pixels
-            wt = _packed(weight, w16, "convT", lambda w: _pack_taps(w, 4, 1, Cout, 4, Cin, 4 * Cout, (0,)))
+            # rows (dy, dx, co), every phase padded to whole units of the epilogue, which stores it to its pixels
+            pad = (Cout + 63) // 64 * 64
+            wt = _packed(weight, w16, "convT", lambda w: _pack_taps(w, 4, 1, Cout, 4, Cin, 4 * Cout, (0,), pad))
+            b4 = _packed(bias, b16, "convT_bias", lambda b: TF.pad(b, (0, pad - Cout)).repeat(4))
             ext.convt2x2(0, x.contiguous(), wt, b4, y, status_word(x.device))
         else:
+            b4 = _packed(bias, b16, "convT_bias_flat", lambda b: b.repeat(4))
             flat = gemm(x.view(-1, Cin), _convt_flat_weight(weight, w16), bias=b4)
             y.copy_(flat.view(B, H, W, 2, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B, 2 * H, 2 * W, Cout))
         ctx.save_for_backward(x)

@@ -41,7 +41,8 @@ def test_stride2_input_gradient(B, H, W, Cin, Cout):
 @pytest.mark.parametrize("B,H,W,Cin,Cout", [
     (1, 1, 1, 64, 64), (1, 16, 24, 96, 96), (2, 7, 130, 64, 64), (1, 5, 3, 128, 32), (1, 9, 33, 40, 96), (1, 20, 257, 192, 384),
     (1, 256, 256, 64, 192),                # CTA pairs
-    (1, 6, 10, 64, 40),                    # phases that a 32-column chunk would straddle: GEMM and permuted copy
+    (1, 6, 10, 64, 40),                    # phases that end inside a unit of the epilogue
+    (1, 3, 5, 64, 2056),                   # more channels than the tap table holds: GEMM and permuted copy
 ])
 def test_transposed_convolution(B, H, W, Cin, Cout):
     from terra_b200.ops.conv import conv_transpose2x2

@@ -38,5 +38,5 @@ def test_kernel(cout, cin):
     for pack in (conv.pack_conv3x3_weight, conv.pack_conv3x3_weight_dgrad, conv.pack_conv3x3_weight_s2_dgrad):
         assert torch.equal(pack(w.cuda()).cpu(), pack(w))
     v = _weights(cin, cout, 2)             # transposed convolution: (Cin, Cout, 2, 2)
-    for args in ((4, 1, cout, 4, cin, 4 * cout, (0,)), (1, 0, cin, 4 * cout, cout, 4, range(4))):
+    for args in ((4, 1, cout, 4, cin, 4 * cout, (0,)), (4, 1, cout, 4, cin, 4 * cout, (0,), cout + 56), (1, 0, cin, 4 * cout, cout, 4, range(4))):
         assert torch.equal(conv._pack_taps(v.cuda(), *args).cpu(), conv._pack_taps(v, *args))

@@ -2,8 +2,8 @@
 //
 //   D[M,N] (+)= A[M,K] * B[N,K]^T, fp32 accumulation in tensor memory.
 //
-// Roles inside a 448-thread CTA (one CTA per SM, tiles assigned round-robin):
-//   warp 0   one elected lane issues TMA loads (per-CTA, no cluster fan-out) into a ring of
+// Roles inside a 480-thread CTA (one CTA per SM, tiles assigned round-robin):
+//   warp 0, warp 14  one elected lane each issues the TMA loads of A and of B (per-CTA, no cluster fan-out) into a ring of
 //            128-byte-swizzled shared-memory stages, signalling `full[s]` by transaction bytes;
 //   warp 1   owns the TMEM allocation; one elected lane issues tcgen05.mma (M=128, N=BN, K=16)
 //            and commits to `empty[s]` (stage reusable) and `tfull[a]` (accumulator a complete);
@@ -31,11 +31,14 @@
 
 namespace tb {
 
-// warp 0: TMA, warp 1: MMA, warps 2..13: epilogue (three per TMEM lane quadrant, interleaved over the 32-column
-// chunks). 14 warps keep every scheduler at four warps or fewer, which allows 128 registers per thread: with 18 warps
+// warp 0: TMA of A, warp 1: MMA, warps 2..13: epilogue (three per TMEM lane quadrant, interleaved over the columns), warp 14:
+// TMA of B. 15 warps keep every scheduler at four warps or fewer, which allows 128 registers per thread: with 18 warps
 // the cap is 96 and the epilogue spills, and its reloads miss the small L1 left beside 227 KB of shared memory.
 constexpr int GEMM_EPI_WARPS = 12;
-constexpr int GEMM_THREADS = 64 + 32 * GEMM_EPI_WARPS;
+// The last warp issues the loads of B: one thread's chain of wait, expect and load instructions for both operands took about
+// as long per k-block as the loads themselves, and the MMA thread waited for it two thirds of its time (K = 384).
+constexpr int GEMM_B_WARP = 2 + GEMM_EPI_WARPS;
+constexpr int GEMM_THREADS = 32 * (GEMM_B_WARP + 1);
 
 // CTAS = 2: a cluster of two CTAs (two SMs of one TPC) computes a 256 x BN tile with one pair-wide MMA. Each CTA stages
 // its own 128 rows of A and its own half of B, so a k-block costs each SM (16 + BN / 8) KB of shared-memory fill instead
@@ -127,6 +130,17 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int tile, 
   return t;
 }
 
+// mbar_wait that adds the time spent to `waited`; a barrier that is complete costs one test and reads no clock.
+template <bool PAIR>
+__device__ __forceinline__ bool wait_counted(uint64_t* bar, uint32_t parity, volatile int* abort_flag, KernelStatus* st,
+                                             unsigned int where, uint32_t budget, long long& waited) {
+  if (mbar_test(bar, parity)) return true;
+  const long long begin = clock64();
+  const bool ok = mbar_wait<PAIR>(bar, parity, abort_flag, st, where, budget);
+  waited += clock64() - begin;
+  return ok;
+}
+
 // PEERS: the tensor-parallel variants (A gathered from peer buffers, output scattered to peer buffers). A separate
 // instantiation, so that the plain kernel carries none of their registers and branches.
 template <int BN, int CTAS, bool PEERS, int STACK = 1>
@@ -165,7 +179,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::MAX_STAGES; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], 2);         // both producers
       mbar_init(&empty[s], 1);
       mbar_init(&pfull[s], 1);
     }
@@ -218,7 +232,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   const uint32_t mbar_budget = PEERS ? 1u + 4u * static_cast<uint32_t>((p.a_budget_ns + 999999999ull) / 1000000000ull) : 1u;
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+    // ------------------------------------------------------------------ TMA producer of A
     if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
@@ -229,7 +243,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         const TileCoord tc = decode_tile(p, tile, CTAS, rank, STACK);
         const int m0 = tc.m_blk * GEMM_BM;
         const int blocks = STACK > 1 ? min(STACK, p.m_blocks - tc.m_blk) : 1;   // 128-row blocks of this tile
-        const int n0 = tc.n_blk * BN + rank * Cfg::B_ROWS;   // this CTA's rows of B
         int abase[5] = {0, 0, 0, 0, 0};
         if (p.a_mode == OP_TABLE_5D) {
           const int t0 = tc.m_blk % p.tile_n0;
@@ -239,14 +252,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           for (int d = 0; d < 5; ++d) abase[d] = t0 * p.a_mul0[d] + t1 * p.a_mul1[d] + t2 * p.a_mul2[d];
         }
         for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
-          const long long w0 = clock64();
-          if (!mbar_wait<PAIR>(&empty[s], ph ^ 1u, abort_flag, p.status, 0x100u + s, mbar_budget)) break;
-          t_wait += clock64() - w0;
+          if (!wait_counted<PAIR>(&empty[s], ph ^ 1u, abort_flag, p.status, 0x100u + s, mbar_budget, t_wait)) break;
           uint8_t* sA = smem + s * Cfg::STAGE_BYTES;
-          uint8_t* sB = sA + Cfg::A_BYTES;
-          mbar_expect_tx(&full[s], STACK > 1 ? Cfg::B_BYTES + blocks * Cfg::BLOCK_BYTES : Cfg::STAGE_BYTES);
+          mbar_expect_tx(&full[s], STACK > 1 ? blocks * Cfg::BLOCK_BYTES : Cfg::A_BYTES);
           int pw = 0, ph_ = 0, pb = 0;
-          if (p.a_mode == OP_PIXELS_5D || p.b_mode == OP_PIXELS_5D) {
+          if (p.a_mode == OP_PIXELS_5D) {
             pw = kb % p.pix_n0;
             ph_ = (kb / p.pix_n0) % p.pix_n1;
             pb = kb / (p.pix_n0 * p.pix_n1);
@@ -303,7 +313,30 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               if (STACK == 1 || j < blocks * (GEMM_BM / 64))
                 tma_load_5d(sA + j * (GEMM_BK * 128), &p.map_a, &full[s], m0 + j * 64, 0, pw * GEMM_BK, ph_, pb);
           }
-          // ---- operand B
+        }
+      }
+      atomicAdd(&g_gemm_stalls[3], static_cast<unsigned long long>(clock64() - t_begin));
+      atomicAdd(&g_gemm_stalls[4], static_cast<unsigned long long>(t_wait));
+    }
+  } else if (warp == GEMM_B_WARP) {
+    // ------------------------------------------------------------------ TMA producer of B
+    if (elect_one()) {
+      int s = 0;
+      uint32_t ph = 0;
+      long long t_wait = 0;
+      for (int tile = unit; tile < total_tiles && !*abort_flag; tile += units) {
+        const TileCoord tc = decode_tile(p, tile, CTAS, rank, STACK);
+        const int n0 = tc.n_blk * BN + rank * Cfg::B_ROWS;   // this CTA's rows of B
+        for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
+          if (!wait_counted<PAIR>(&empty[s], ph ^ 1u, abort_flag, p.status, 0x140u + s, mbar_budget, t_wait)) break;
+          uint8_t* sB = smem + s * Cfg::STAGE_BYTES + Cfg::A_BYTES;
+          mbar_expect_tx(&full[s], Cfg::B_BYTES);
+          int pw = 0, ph_ = 0, pb = 0;
+          if (p.b_mode == OP_PIXELS_5D) {
+            pw = kb % p.pix_n0;
+            ph_ = (kb / p.pix_n0) % p.pix_n1;
+            pb = kb / (p.pix_n0 * p.pix_n1);
+          }
           if (p.b_mode == OP_KMAJOR_2D) {
             tma_load_2d(sB, &p.map_b, &full[s], kb * GEMM_BK, n0);
           } else if (p.b_mode == OP_MNMAJOR_2D) {
@@ -327,8 +360,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           }
         }
       }
-      atomicAdd(&g_gemm_stalls[3], static_cast<unsigned long long>(clock64() - t_begin));
-      atomicAdd(&g_gemm_stalls[4], static_cast<unsigned long long>(t_wait));
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA in pair mode)
@@ -362,10 +393,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         const uint32_t d_sums = tmem_base + Cfg::SUM_COL0 + acc * 32;
         bool ok = true;
         for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
-          const long long w1 = clock64();
-          if (!mbar_wait<PAIR>(&full[s], ph, abort_flag, p.status, 0x300u + s, mbar_budget)) { ok = false; break; }
-          if (PAIR && !mbar_wait<PAIR>(&pfull[s], ph, abort_flag, p.status, 0x380u + s, mbar_budget)) { ok = false; break; }
-          t_ops += clock64() - w1;
+          if (!wait_counted<PAIR>(&full[s], ph, abort_flag, p.status, 0x300u + s, mbar_budget, t_ops)) { ok = false; break; }
+          if (PAIR && !wait_counted<PAIR>(&pfull[s], ph, abort_flag, p.status, 0x380u + s, mbar_budget, t_ops)) {
+            ok = false;
+            break;
+          }
           tc_fence_after();
           const uint32_t sA = smem_u32(smem + s * Cfg::STAGE_BYTES);
           const uint32_t sB = sA + Cfg::A_BYTES;

@@ -136,7 +136,8 @@ static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, 
   *ctas_out = 1;
   const bool second = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU | EPI_SAVE_PRE)) != 0;
   // the ring keeps too little beside two units per epilogue warp when single tiles are 256 wide
-  if (*bn_out == 256 && second && k_blocks <= 12) *bn_out = 192;
+  // (an input operand with a longer contraction takes the per-lane epilogue, which needs no such room)
+  if (*bn_out == 256 && second && (k_blocks <= 12 || (flags & EPI_SAVE_PRE))) *bn_out = 192;
   if (!pairs_enabled() || N < 128 || ((m_blocks + 1) / 2) * ((N + 255) / 256) < 8LL * (num_sms / 2)) return;
   const long long unit = (flags & EPI_MUL_DGELU) ? 4500 : (flags & EPI_SAVE_PRE) ? 3500 : (flags & EPI_RESIDUAL) ? 2500 : 2000;
   long long best = 0;

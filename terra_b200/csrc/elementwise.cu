@@ -1006,8 +1006,13 @@ struct GnShape {
   }
 };
 
+// (GnShape divides by the sizes: an empty batch or image is refused here, as an empty grid would be by the launch)
+static bool gn_sizes_ok(int B, long long HW, int C, int groups) {
+  return B >= 1 && HW >= 1 && C >= 8 && C % 8 == 0 && groups >= 1 && C % groups == 0;
+}
+
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {
-  if (C % 8 != 0 || C % groups != 0) return -1;
+  if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 512, 3, 4);
   groupnorm_stats_kernel<<<s.grid, s.block, 2 * C * sizeof(float), stream>>>(static_cast<const __nv_bfloat16*>(x), sums, HW,
                                                                              C, groups, s.pix);
@@ -1016,7 +1021,7 @@ int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int 
 
 int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, const void* beta, const void* res, void* y,
                          int B, long long HW, int C, int groups, cudaStream_t stream) {
-  if (C % 8 != 0 || C % groups != 0) return -1;
+  if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 6, 2);
   groupnorm_silu_apply_kernel<<<s.grid, s.block, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
@@ -1028,7 +1033,7 @@ int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, c
 int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats, const void* gamma, const void* beta,
                               float* red, float* dgamma, float* dbeta, int B, long long HW, int C, int groups,
                               cudaStream_t stream) {
-  if (C % 8 != 0 || C % groups != 0) return -1;
+  if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 3, 2);
   groupnorm_silu_bwd_reduce_kernel<<<s.grid, s.block, 2 * C * sizeof(float), stream>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
@@ -1054,7 +1059,7 @@ int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa
 int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, const float* red, const void* gamma,
                              const void* beta, void* dx, int B, long long HW, int C, int groups, float inv_count,
                              cudaStream_t stream) {
-  if (C % 8 != 0 || C % groups != 0) return -1;
+  if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 4, 2);
   groupnorm_silu_bwd_apply_kernel<<<s.grid, s.block, groups * 2 * sizeof(float), stream>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red,

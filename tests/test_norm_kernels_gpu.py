@@ -62,3 +62,21 @@ def test_groupnorm_silu(B, HW, C, groups, shortcut):
     rel = 2e-2 if HW == 1 else REL
     assert _rel(y, ref.detach() + (res.float() if shortcut else 0)) < REL
     assert _rel(got[0], xr.grad) < rel and _rel(got[1], gn.weight.grad) < rel and _rel(got[2], gn.bias.grad) < rel
+
+
+@pytest.mark.parametrize("B,HW", [(0, 16), (2, 0)])
+def test_groupnorm_refuses_empty_images(B, HW):
+    """The four launchers divide by the sizes; an empty batch or image is an error that Python sees."""
+    from terra_b200 import _ext
+    from terra_b200.ops.conv import groupnorm_silu
+
+    C, G, ext = 64, 8, _ext.load()
+    x, w = torch.empty(B, HW, C, device="cuda", dtype=torch.bfloat16), _rand(C)
+    stats, red = torch.zeros(B, G, 2, device="cuda"), torch.zeros(B, C, 2, device="cuda")
+    for call in (lambda: ext.groupnorm_stats(x, stats, G),
+                 lambda: ext.groupnorm_silu_apply(x, stats, w, w, None, x.clone(), G),
+                 lambda: ext.groupnorm_silu_bwd_reduce(x, x, stats, w, w, red, G, None, None),
+                 lambda: ext.groupnorm_silu_bwd_apply(x, x, stats, red, w, w, x.clone(), G, 1.0),
+                 lambda: groupnorm_silu(x.view(B, 1, HW, C), torch.nn.GroupNorm(G, C).cuda())):
+        with pytest.raises(RuntimeError):
+            call()

@@ -134,6 +134,7 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
            grad_w.is_contiguous() && grad_w.size(0) == dy.size(1) && grad_w.size(1) == x.size(1),
        "wgrad: dy [M, N], x [M, K] bf16, grad_w [N, K] fp32");
   need(!grad_b.has_value() || vec(*grad_b, torch::kFloat32, dy.size(1)), "wgrad: grad_b fp32 [N]");
+  need(dy.size(0) > 0 && dy.size(1) > 0 && x.size(1) > 0, "wgrad: empty operand");
   const c10::cuda::CUDAGuard guard(dy.device());
   const int64_t M = dy.size(0), N = dy.size(1), K = x.size(1);
   bool sums = grad_b.has_value();

@@ -52,3 +52,13 @@ def test_weight_gradient_of_pitched_rows():
     wgrad_accumulate(dy, x, gw, gb)
     ref = dy.float().t() @ x.float()
     assert _rel(gw, ref) < 1e-5 and _rel(gb, dy.float().sum(0)) < 1e-5
+
+
+@pytest.mark.parametrize("M,N,K", [(10, 64, 0), (10, 0, 64), (0, 64, 64)])
+def test_weight_gradient_refuses_empty_operands(M, N, K):
+    """The plan of the tiles divides by their number; an empty operand is an error that Python sees."""
+    from terra_b200.ops.blocks import wgrad_accumulate
+
+    dy, x = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16), torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        wgrad_accumulate(dy, x, torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda"))

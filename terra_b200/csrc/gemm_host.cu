@@ -138,7 +138,7 @@ static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, 
   // the ring keeps too little beside two units per epilogue warp when single tiles are 256 wide
   // (an input operand with a longer contraction takes the per-lane epilogue, which needs no such room)
   if (*bn_out == 256 && second && (k_blocks <= 12 || (flags & EPI_SAVE_PRE))) *bn_out = 192;
-  if (!pairs_enabled() || N < 128 || ((m_blocks + 1) / 2) * ((N + 255) / 256) < 8LL * (num_sms / 2)) return;
+  if (!pairs_enabled() || num_sms < 2 || N < 128 || ((m_blocks + 1) / 2) * ((N + 255) / 256) < 8LL * (num_sms / 2)) return;
   const long long unit = (flags & EPI_MUL_DGELU) ? 4500 : (flags & EPI_SAVE_PRE) ? 3500 : (flags & EPI_RESIDUAL) ? 2500 : 2000;
   long long best = 0;
   for (int ctas : {2, 1})
@@ -154,6 +154,10 @@ static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, 
         *ctas_out = ctas;
       }
     }
+}
+
+void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, int num_sms, int* bn, int* ctas) {
+  pick_tile((M + GEMM_BM - 1) / GEMM_BM, N, static_cast<int>((K + GEMM_BK - 1) / GEMM_BK), b_mn, flags, num_sms, bn, ctas);
 }
 
 static void fill_epilogue(GemmParams& p, const GemmEpilogue& e) {
@@ -198,8 +202,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
     bn_request -= 1000;
     if (bn_request != 128 && bn_request != 256 && !(bn_request == 192 && !B.mn_major)) return -11;
   } else if (bn_request == 0 && !A.mn_major && !gather_a && !scatter_c && split_k <= 1 && epi.colsum == nullptr) {
-    pick_tile((M + GEMM_BM - 1) / GEMM_BM, N, static_cast<int>((K + GEMM_BK - 1) / GEMM_BK), B.mn_major, epi.flags, num_sms,
-              &bn_request, &ctas);
+    gemm_tile(M, N, K, B.mn_major != 0, epi.flags, num_sms, &bn_request, &ctas);
   }
   if (epi.colsum != nullptr) {
     // column sums ride on the weight-gradient form only, and need room for their accumulators behind the tile's

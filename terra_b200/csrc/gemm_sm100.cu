@@ -934,8 +934,9 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   p.smem_bytes = Cfg::smem_bytes(p.epi_bufs);
   const int total = p.groups * p.num_m_tiles * p.num_n_tiles * p.split_k;
   const int max_units = num_sms / CTAS;
+  if (total <= 0) return cudaSuccess;
+  if (max_units < 1) return cudaErrorInvalidValue;   // a pair on one SM
   const int units = total < max_units ? total : max_units;
-  if (units <= 0) return cudaSuccess;
   if (CTAS == 1) {
     gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK><<<units, GEMM_THREADS, p.smem_bytes, stream>>>(p);
     return cudaGetLastError();

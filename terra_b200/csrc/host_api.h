@@ -72,6 +72,9 @@ int gemm_bf16(const GemmOperand& A, const GemmOperand& B, long long M, long long
 // Cycle counters of the GEMM kernel's roles summed over CTAs and launches since the last reset:
 // [0] MMA span, [1] MMA waiting for an accumulator, [2] MMA waiting for operands, [3] TMA span, [4] TMA waiting for
 // free stages, [5] epilogue span, [6] epilogue waiting for tiles. Synchronises the device.
+// The rule's tile of a plain product (no peers, no split, no column sums) when no width is asked for: columns, and CTAs per
+// tile of 128 rows each (2: a CTA pair).
+void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, int num_sms, int* bn, int* ctas);
 int gemm_stall_counters(unsigned long long* out8, int reset);
 
 int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin, int Cout, int stride,

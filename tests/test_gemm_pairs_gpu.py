@@ -92,3 +92,18 @@ def test_gelu_keeps_its_limits():
     assert torch.allclose(act[0].float()[fine], ref.to(torch.bfloat16).float()[fine], rtol=1e-2, atol=1e-4)
     x = bias.float()
     assert torch.allclose(grad[0].float()[x >= 9], torch.ones_like(x[x >= 9])) and grad[0].float()[x <= -9].abs().max() < 1e-3
+
+
+@pytest.mark.parametrize("sms", [1, 2, 3])
+def test_few_multiprocessors(sms):
+    """A product held to a few SMs computes every tile; one SM holds no pair, asked for or not."""
+    from terra_b200.ops.gemm import check_status, gemm
+
+    torch.manual_seed(4)
+    a, w = _rand(128 * 9 + 1, 64), _rand(384, 64, scale=0.125)
+    got = gemm(a, w, sms=sms)
+    check_status("cuda")
+    assert _rel(got, a.float() @ w.float().t()) < REL
+    if sms == 1:
+        with pytest.raises(RuntimeError):
+            gemm(a, w, sms=1, bn=1128)

@@ -6,6 +6,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include "check.h"
 #include "host_api.h"
 #include "launch_count.h"
 
@@ -51,7 +52,7 @@ void gemm(const torch::Tensor& a, bool a_mn, const torch::Tensor& b, bool b_mn, 
   const int64_t K = a_mn ? a.size(0) : a.size(1);
   const int64_t N = b_mn ? b.size(1) : b.size(0);
   const int64_t Kb = b_mn ? b.size(0) : b.size(1);
-  TORCH_CHECK(K == Kb, "gemm: contraction mismatch ", K, " vs ", Kb);
+  if (K != Kb) need(false, ("gemm: contraction mismatch " + std::to_string(K) + " vs " + std::to_string(Kb)).c_str());
   tb::GemmOperand A{a.data_ptr(), a.stride(0), a_mn ? 1 : 0};
   tb::GemmOperand B{b.data_ptr(), b.stride(0), b_mn ? 1 : 0};
   tb::GemmEpilogue e{};
@@ -95,7 +96,8 @@ void gemm(const torch::Tensor& a, bool a_mn, const torch::Tensor& b, bool b_mn, 
   }
   const int rc = tb::gemm_bf16_peers(A, B, M, N, K, e, peers, static_cast<int>(split_k), static_cast<int>(bn),
                                      sms > 0 ? static_cast<int>(sms) : sm_count(), cur_stream());
-  TORCH_CHECK(rc == 0, "terra_b200 gemm launch failed, code ", rc, " (M=", M, " N=", N, " K=", K, ")");
+  if (rc != 0)
+    rc_check(rc, ("gemm (M=" + std::to_string(M) + " N=" + std::to_string(N) + " K=" + std::to_string(K) + ") launch").c_str());
 }
 
 // x: [B,H,W,Cin] bf16 NHWC, w: [Cout, 9*Cin_pad] bf16, y: [B,Ho,Wo,Cout]
@@ -124,7 +126,7 @@ void conv3x3_fwd(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor& 
   const int rc = tb::conv3x3_fwd_bf16(x.data_ptr(), w.data_ptr(), x.size(0), x.size(1), x.size(2), x.size(3), w.size(0),
                                       static_cast<int>(stride), e, sm_count(), cur_stream(), opt_ptr(halo_lo),
                                       opt_ptr(halo_hi));
-  TORCH_CHECK(rc == 0, "terra_b200 conv3x3_fwd launch failed, code ", rc);
+  rc_check(rc, "conv3x3_fwd");
 }
 
 // dw: [9, Cout, Cin] fp32 (zeroed by the caller)
@@ -145,7 +147,7 @@ void conv3x3_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tenso
                                         sm_count(), cur_stream(), opt_ptr(halo_lo), opt_ptr(halo_hi),
                                         bias_grad.has_value() ? bias_grad->data_ptr<float>() : nullptr,
                                         static_cast<int>(stack));
-  TORCH_CHECK(rc == 0, "terra_b200 conv3x3_wgrad launch failed, code ", rc);
+  rc_check(rc, "conv3x3_wgrad");
 }
 
 void check_image(const torch::Tensor& t, const char* name) {
@@ -154,7 +156,7 @@ void check_image(const torch::Tensor& t, const char* name) {
 void check_packed(const torch::Tensor& w, int64_t rows, int64_t taps, int64_t channels) {
   TORCH_CHECK(w.scalar_type() == torch::kBFloat16 && w.is_contiguous() && w.dim() == 2 && w.size(0) == rows &&
                   w.size(1) == taps * ((channels + 63) / 64 * 64),
-              "packed weights: bf16 [", rows, ", ", taps, " * channels padded to 64]");
+              "packed weights: bf16 [rows, taps * channels padded to 64]");
 }
 void* status_ptr(const c10::optional<torch::Tensor>& s) { return s.has_value() ? s->data_ptr() : nullptr; }
 
@@ -170,7 +172,7 @@ void conv3x3_s2_dgrad(const torch::Tensor& dy, const torch::Tensor& w, torch::Te
   tb::note_launch();
   const int rc = tb::conv3x3_s2_dgrad_bf16(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), dx.size(0), dx.size(1), dx.size(2), dx.size(3),
                                            dy.size(3), status_ptr(status), sm_count(), cur_stream());
-  TORCH_CHECK(rc == 0, "terra_b200 conv3x3_s2_dgrad launch failed, code ", rc);
+  rc_check(rc, "conv3x3_s2_dgrad");
 }
 
 // The three products of the 2x2 / stride-2 transposed convolution, x [B, H, W, Cin] and y / dy [B, 2H, 2W, Cout]:
@@ -193,7 +195,7 @@ void convt2x2(int64_t op, const torch::Tensor& in, const torch::Tensor& w, const
                                                  x.size(2), Cin, Cout, status_ptr(status), sm_count(), cur_stream())
                          : tb::convt2x2_dgrad_bf16(y.data_ptr(), w.data_ptr(), out.data_ptr(), x.size(0), x.size(1), x.size(2), Cin,
                                                    Cout, status_ptr(status), sm_count(), cur_stream());
-  TORCH_CHECK(rc == 0, "terra_b200 convt2x2 launch failed, code ", rc);
+  rc_check(rc, "convt2x2");
 }
 
 // dw: [4, Cin, Cout] fp32, accumulated
@@ -209,7 +211,7 @@ void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tens
   const int rc = tb::convt2x2_wgrad_bf16(x.data_ptr(), dy.data_ptr(), dw.data_ptr<float>(), x.size(0), x.size(1), x.size(2),
                                          x.size(3), dy.size(3), static_cast<int>(split_k), status_ptr(status), sm_count(),
                                          cur_stream(), static_cast<int>(stack));
-  TORCH_CHECK(rc == 0, "terra_b200 convt2x2_wgrad launch failed, code ", rc);
+  rc_check(rc, "convt2x2_wgrad");
 }
 
 }  // namespace

@@ -5,6 +5,7 @@
 
 #include <cmath>
 
+#include "check.h"
 #include "comm_api.h"
 #include "launch_count.h"
 
@@ -89,7 +90,7 @@ void gather_shards_async(int64_t stream, int64_t dst, const std::vector<int64_t>
                                          reinterpret_cast<const unsigned int*>(signals_ptr),
                                          reinterpret_cast<unsigned int*>(ready_ptr), static_cast<unsigned int>(epoch),
                                          include_self ? 1 : 0);
-  TORCH_CHECK(rc == 0, "gather_shards_async failed with code ", rc);
+  rc_check(rc, "gather_shards_async");
 }
 
 void peer_gather_indexed(torch::Tensor& dst, const std::vector<int64_t>& src_ptrs, const torch::Tensor& src_slot,

@@ -2,13 +2,12 @@
 // (which the multi-rank layouts use), without the interpreter between them. A small layer is bound by its launches: on 512
 // rows of width 96 the Python form spent about 20 us per launch on the host against 1 to 10 us of kernel time.
 #include <algorithm>
-#include <stdexcept>
-#include <string>
 #include <vector>
 #include <torch/extension.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include "check.h"
 #include "host_api.h"
 #include "launch_count.h"
 
@@ -18,12 +17,6 @@ using torch::Tensor;
 using OptTensor = c10::optional<torch::Tensor>;
 
 cudaStream_t cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
-void need(bool ok, const char* what) {
-  if (!ok) throw std::runtime_error(std::string("terra_b200: ") + what);
-}
-void rc_check(int rc, const char* what) {
-  if (rc != 0) throw std::runtime_error(std::string("terra_b200: ") + what + " failed with code " + std::to_string(rc));
-}
 int sm_count() {
   static const int n = [] {
     int dev = 0, v = 148;

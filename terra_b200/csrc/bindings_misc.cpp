@@ -4,6 +4,7 @@
 
 #include <memory>
 
+#include "check.h"
 #include "copy_engine.h"
 
 namespace {
@@ -16,7 +17,7 @@ class PyCopyEngine {
   int64_t offload(const torch::Tensor& t) {
     TORCH_CHECK(t.is_cuda() && t.is_contiguous(), "offload: contiguous CUDA tensor");
     const int64_t id = eng_->offload(t.data_ptr(), t.nbytes(), cur_stream());
-    TORCH_CHECK(id > 0, "copy engine offload failed: ", id);
+    if (id <= 0) need(false, ("copy engine offload failed: " + std::to_string(id)).c_str());
     return id;
   }
   void restore(int64_t ticket, torch::Tensor& dst, bool wait) {

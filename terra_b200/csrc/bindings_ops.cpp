@@ -1,10 +1,9 @@
 // Bindings for the memory-bound kernels and window attention.
-#include <stdexcept>
-#include <string>
 #include <torch/extension.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include "check.h"
 #include "host_api.h"
 #include "launch_count.h"
 
@@ -14,13 +13,6 @@ cudaStream_t cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 const void* opt_ptr(const c10::optional<torch::Tensor>& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 void* opt_mut(const c10::optional<torch::Tensor>& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 
-// Plain std::runtime_error (pybind11 turns it into RuntimeError): no backtrace collection on the error path.
-void need(bool ok, const char* what) {
-  if (!ok) throw std::runtime_error(std::string("terra_b200: ") + what);
-}
-void rc_check(int rc, const char* what) {
-  if (rc != 0) throw std::runtime_error(std::string("terra_b200: ") + what + " failed with code " + std::to_string(rc));
-}
 
 void layernorm_fwd(const torch::Tensor& x, const torch::Tensor& g, const torch::Tensor& b, torch::Tensor& y,
                    torch::Tensor& mean, torch::Tensor& rstd, double eps) {

@@ -188,3 +188,14 @@ def test_gemm_cta_pair(bn):
     gemm(dy, a, a_mn=True, b_mn=True, out=gw, accumulate=True, split_k=3, bn=bn)
     check_status("cuda")
     _close(gw, dy.float().t() @ a.float())
+
+
+def test_refused_products_raise():
+    """A product that cannot be launched is an error that Python sees; its message holds the numbers."""
+    from terra_b200.ops.gemm import gemm
+
+    a, b = torch.zeros(8, 64, device="cuda", dtype=torch.bfloat16), torch.zeros(16, 72, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="64 vs 72"):
+        gemm(a, b)
+    with pytest.raises(RuntimeError, match="N=16"):
+        gemm(a, b[:, :64], bn=1064)          # no such width for a CTA pair

@@ -42,15 +42,27 @@ struct Epi {
   const Tensor* pre = nullptr;
 };
 
-// out [M, N] = epilogue(a [M, K] * w), w [N, K] or, with b_mn, [K, N]
+// an operand of the epilogue: rows like the output's
+bool like_out(const Tensor* t, const Tensor& out) {
+  return t == nullptr || (rows_pitched(*t) && t->sizes() == out.sizes() && t->device() == out.device());
+}
+
+// out [M, N] = epilogue(a [M, K] * w), w [N, K] or, with b_mn, [K, N]; the bias bf16 or fp32
 void product(const Tensor& a, const Tensor& w, bool b_mn, const Tensor& out, const Epi& e, const Tensor& status) {
+  need(rows_pitched(a) && rows_pitched(w) && rows_pitched(out) && a.device() == w.device() && a.device() == out.device(),
+       "block half: operands must be 2-D bf16 rows on one GPU");
+  need(a.size(1) == w.size(b_mn ? 0 : 1) && out.size(0) == a.size(0) && out.size(1) == w.size(b_mn ? 1 : 0), "block half: operand shapes");
+  need(like_out(e.residual, out) && like_out(e.aux, out) && like_out(e.pre, out), "block half: operands of the epilogue");
   tb::GemmOperand A{a.data_ptr(), a.stride(0), 0}, B{w.data_ptr(), w.stride(0), b_mn ? 1 : 0};
   tb::GemmEpilogue g{};
   g.flags = e.flags;
   g.C = out.data_ptr();
   g.ldc = out.stride(0);
   if (e.bias != nullptr) {
-    g.flags |= tb::EPI_BIAS;
+    const bool f32 = e.bias->scalar_type() == torch::kFloat32;
+    need(vec(*e.bias, f32 ? torch::kFloat32 : torch::kBFloat16, out.size(1)) && e.bias->device() == out.device(),
+         "block half: bias bf16 or fp32, one entry per column");
+    g.flags |= tb::EPI_BIAS | (f32 ? tb::EPI_BIAS_F32 : 0);
     g.bias = e.bias->data_ptr();
   }
   if (e.residual != nullptr) {
@@ -70,7 +82,6 @@ void product(const Tensor& a, const Tensor& w, bool b_mn, const Tensor& out, con
   }
   g.alpha = 1.0f;
   g.status = status.data_ptr();
-  need(a.size(1) == w.size(b_mn ? 0 : 1) && out.size(0) == a.size(0) && out.size(1) == w.size(b_mn ? 1 : 0), "block half: operand shapes");
   tb::note_launch();
   rc_check(tb::gemm_bf16(A, B, a.size(0), out.size(1), a.size(1), g, 1, 0, sm_count(), cur_stream()), "gemm");
 }
@@ -124,8 +135,8 @@ WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
 // 16-column MMA of the dy tiles against ones) where its accumulators fit beside the tile's (widths up to 192).
 void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTensor& grad_b, bool fuse_bias, const Tensor& status) {
   need(rows_pitched(dy) && rows_pitched(x) && dy.size(0) == x.size(0) && grad_w.scalar_type() == torch::kFloat32 && grad_w.dim() == 2 &&
-           grad_w.is_contiguous() && grad_w.size(0) == dy.size(1) && grad_w.size(1) == x.size(1),
-       "wgrad: dy [M, N], x [M, K] bf16, grad_w [N, K] fp32");
+           grad_w.is_cuda() && grad_w.stride(1) == 1 && grad_w.size(0) == dy.size(1) && grad_w.size(1) == x.size(1),
+       "wgrad: dy [M, N], x [M, K] bf16, grad_w [N, K] fp32 rows");
   need(!grad_b.has_value() || vec(*grad_b, torch::kFloat32, dy.size(1)), "wgrad: grad_b fp32 [N]");
   need(dy.size(0) > 0 && dy.size(1) > 0 && x.size(1) > 0, "wgrad: empty operand");
   const c10::cuda::CUDAGuard guard(dy.device());
@@ -170,6 +181,10 @@ Norm norm_fwd(const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
 }
 Tensor norm_bwd(const Tensor& dxn, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, const Tensor& gw,
                 const Tensor& gb, const Tensor& dres) {
+  need(rows_bf16(x) && rows_bf16(dxn) && rows_bf16(dres) && dxn.sizes() == x.sizes() && dres.sizes() == x.sizes(),
+       "block half: x and its gradients must be contiguous [rows, C]");
+  need(vec(w, torch::kBFloat16, x.size(1)) && vec(mean, torch::kFloat32, x.size(0)) && vec(rstd, torch::kFloat32, x.size(0)),
+       "block half: norm weight bf16, row statistics fp32");
   need(vec(gw, torch::kFloat32, x.size(1)) && vec(gb, torch::kFloat32, x.size(1)), "block half: norm gradients fp32");
   Tensor dx = torch::empty_like(x);
   tb::note_launch();
@@ -235,7 +250,9 @@ Tensor attn_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, cons
                      const Tensor& proj_bg, const OptTensor& table_g, const std::vector<int64_t>& geo, double scale, bool fuse_bias,
                      const Tensor& status) {
   const c10::cuda::CUDAGuard guard(x.device());
-  need(rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: dy like x");
+  // (the saved tensors come back through whatever hooks the caller has set, so their form is checked like any input's)
+  need(rows_bf16(x) && rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: x and dy contiguous [rows, C]");
+  need(rows_bf16(qkv) && qkv.size(0) == x.size(0) && qkv.size(1) == 3 * x.size(1), "block half: qkv contiguous [rows, 3 C]");
   tb::WindowAttnArgs a = window_args(geo, x.size(1), table, scale, x.size(0));
   wgrad(dy, o, proj_wg, proj_bg, fuse_bias, status);
   Tensor dout = torch::empty_like(x), dqkv = torch::empty_like(qkv), dxn = torch::empty_like(x);
@@ -277,9 +294,9 @@ Tensor mlp_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, const
                     const Tensor& ln_bg, const Tensor& fc1_wg, const Tensor& fc1_bg, const Tensor& fc2_wg, const Tensor& fc2_bg,
                     bool fuse_bias, const Tensor& status) {
   const c10::cuda::CUDAGuard guard(x.device());
-  need(rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: dy like x");
+  need(rows_bf16(x) && rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: x and dy contiguous [rows, C]");
   wgrad(dy, act, fc2_wg, fc2_bg, fuse_bias, status);
-  Tensor dpre = torch::empty_like(pre), dxn = torch::empty_like(x);
+  Tensor dpre = torch::empty({x.size(0), fc2_w.size(1)}, x.options()), dxn = torch::empty_like(x);
   Epi e;
   e.aux = &pre;
   product(dy, fc2_w, true, dpre, e, status);

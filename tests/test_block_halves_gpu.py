@@ -62,3 +62,89 @@ def test_weight_gradient_refuses_empty_operands(M, N, K):
     dy, x = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16), torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
     with pytest.raises(RuntimeError):
         wgrad_accumulate(dy, x, torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda"))
+
+
+def _mlp(dim, rows):
+    from terra_b200.models.layers import MlpHalf
+    from terra_b200.utils.flat_params import ParamArena
+
+    torch.manual_seed(2)
+    mod = MlpHalf(dim, 4 * dim).cuda()
+    return mod, ParamArena(mod), torch.randn(rows, dim, device="cuda").to(torch.bfloat16)
+
+
+def test_native_halves_refuse_other_operands():
+    """Weights and biases are read by raw pointers: types, sizes and strides that do not fit are errors."""
+    from terra_b200 import _ext
+    from terra_b200.ops.gemm import status_word
+
+    ext, C, H = _ext.load(), 64, 256
+    r = lambda *s, dt=torch.bfloat16: torch.randn(*s, device="cuda").to(dt)
+    good = dict(x=r(32, C), ln_w=r(C), ln_b=r(C), fc1_w=r(H, C), fc1_b=r(H), fc2_w=r(C, H), fc2_b=r(C))
+    run = lambda **kw: ext.mlp_half_fwd(*{**good, **kw}.values(), 1e-5, status_word("cuda"))[0]
+    y = run()
+    # an fp32 bias is taken by its type
+    assert torch.equal(run(fc1_b=good["fc1_b"].float(), fc2_b=good["fc2_b"].float()), y)
+    for bad in (dict(fc1_w=r(H, C, dt=torch.float32)), dict(fc1_w=r(C, H).t()), dict(fc2_w=r(C, H).cpu()), dict(fc1_b=r(H - 8)),
+                dict(fc2_b=r(2 * C)[::2]), dict(fc2_b=r(C, dt=torch.float16)), dict(x=r(32, 2 * C)[:, :C]), dict(ln_w=r(C).float())):
+        with pytest.raises(RuntimeError):
+            run(**bad)
+
+
+@pytest.mark.parametrize("half", ["attention", "mlp"])
+def test_saved_tensors_of_another_form(half):
+    """Hooks may hand the saved tensors back with another row pitch: products take that, what is read as dense rows is
+    refused."""
+    from terra_b200.models.layers import SwinAttentionHalf
+    from terra_b200.ops import blocks
+    from terra_b200.ops.attention import WindowGeometry
+    from terra_b200.utils.flat_params import ParamArena
+
+    if half == "attention":
+        torch.manual_seed(2)
+        geo = WindowGeometry(1, 2, 2, 8, 8)
+        mod = SwinAttentionHalf(1, 64, (8, 8), 2, use_relative_position_bias=True).cuda()
+        arena, x = ParamArena(mod), torch.randn(geo.rows_local, 64, device="cuda").to(torch.bfloat16)
+        run = lambda t: blocks.attention_half(t, mod, geo, True)
+        pitched_ok, dense = (3, 5), (0, 4)          # xn, o / x, qkv in the order of saving
+    else:
+        mod, arena, x = _mlp(64, 300)
+        run = lambda t: blocks.mlp_half(t, mod)
+        pitched_ok, dense = (3, 4, 5), (0,)         # xn, pre, act / x
+    dy = torch.randn_like(x)
+
+    def grads(pitched):
+        seen = []
+
+        def pack(t):
+            seen.append(len(seen))
+            return len(seen) - 1, t
+
+        def unpack(p):
+            i, t = p
+            return torch.cat([t, t], dim=1)[:, :t.shape[1]] if i in pitched else t
+
+        arena.zero_grad()
+        t = x.clone().requires_grad_(True)
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            y = run(t)
+        y.backward(dy)
+        return t.grad, arena.grad.clone()
+
+    dx, g = grads(())
+    dx2, g2 = grads(pitched_ok)
+    assert torch.equal(dx, dx2) and _rel(g2, g) < 1e-5
+    for i in dense:
+        with pytest.raises(RuntimeError):
+            grads((i,))
+
+
+def test_weight_gradient_into_pitched_rows():
+    from terra_b200.ops.blocks import wgrad_accumulate
+
+    torch.manual_seed(3)
+    dy, x = torch.randn(500, 136, device="cuda").to(torch.bfloat16), torch.randn(500, 72, device="cuda").to(torch.bfloat16)
+    wide = torch.ones(136, 200, device="cuda")
+    wgrad_accumulate(dy, x, wide[:, 64:136])
+    assert _rel(wide[:, 64:136] - 1, dy.float().t() @ x.float()) < 1e-5
+    assert (wide[:, :64] == 1).all() and (wide[:, 136:] == 1).all()

@@ -2,6 +2,7 @@
 // (which the multi-rank layouts use), without the interpreter between them. A small layer is bound by its launches: on 512
 // rows of width 96 the Python form spent about 20 us per launch on the host against 1 to 10 us of kernel time.
 #include <algorithm>
+#include <tuple>
 #include <vector>
 #include <torch/extension.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -308,6 +309,14 @@ Tensor mlp_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, const
 }  // namespace
 
 void bind_halves(pybind11::module_& m) {
+  m.def(
+      "wgrad_plan",
+      [](int64_t N, int64_t K, int64_t M, bool sums) {
+        need(N > 0 && K > 0 && M > 0, "wgrad_plan: empty operand");
+        const WgradPlan p = plan_wgrad(N, K, M, sums);
+        return std::make_tuple(p.bn, p.stack, p.split);
+      },
+      "tile width, row blocks per tile and split of the contraction that wgrad takes");
   m.def("wgrad", &wgrad, "weight (and bias) gradient of a linear layer, accumulated in fp32");
   m.def("attn_half_fwd", &attn_half_fwd);
   m.def("attn_half_bwd", &attn_half_bwd);

@@ -25,8 +25,10 @@ import torch.nn.functional as TF
 from .. import _ext
 from .attention import (MAX_KERNEL_WINDOW_TOKENS, WindowGeometry, attn_backward_impl, attn_forward_impl,
                         launch_window_attn_bwd, launch_window_attn_fwd, window_attention)
-from .gemm import gemm, status_word
+from . import _flags as F
+from .gemm import TRACE, gemm, status_word, trace_product
 from .packed import fp32_values
+from ..utils import nvtx
 from ..utils.nvtx import nvtx_range
 
 LN_EPS = 1e-5
@@ -37,10 +39,19 @@ LN_EPS = 1e-5
 FUSE_BIAS_GRAD = os.environ.get("TERRA_FUSED_BIAS_GRAD", "1") == "1"
 
 
+# TERRA_TRACE=1 / TERRA_NVTX=1 report single launches, so the halves are then launched one by one from Python
+_LAUNCHES_OBSERVED = TRACE or nvtx.ENABLED
+
+
+@nvtx_range("terra.gemm")
 def wgrad_accumulate(dy: torch.Tensor, x: torch.Tensor, grad_w: torch.Tensor, grad_b: torch.Tensor = None) -> None:
     """grad_w[N, K] (fp32) += dy[M, N]^T @ x[M, K]; with ``grad_b``: grad_b[N] (fp32) += column sums of dy, from the
     same kernel (a 16-column MMA of the dy tiles against ones), which saves the separate pass over dy."""
-    _ext.load().wgrad(dy, x, grad_w, grad_b, FUSE_BIAS_GRAD, status_word(dy.device))
+    ext = _ext.load()
+    if TRACE:
+        bn, _, split = ext.wgrad_plan(grad_w.shape[0], grad_w.shape[1], dy.shape[0], grad_b is not None and FUSE_BIAS_GRAD)
+        trace_product(dy, True, x, True, grad_w, F.EPI_OUT_F32 | F.EPI_ATOMIC, split, bn)
+    ext.wgrad(dy, x, grad_w, grad_b, FUSE_BIAS_GRAD, status_word(dy.device))
 
 
 def bias_grad_accumulate(dy: torch.Tensor, grad_b: torch.Tensor) -> None:
@@ -79,8 +90,9 @@ def _views(p: torch.nn.Parameter):
 
 def _native_half(comm, geo: WindowGeometry, impl: str) -> bool:
     """One native call runs the half when this rank owns every window and token and the small-window kernels are the
-    selected ones (not in the bounds-checked build, whose reports go through the Python launches)."""
-    return comm is None and impl == "mma" and geo.sp == 1 and geo.tp == 1 and geo.n_wg == 1 and not _ext.DEBUG_BOUNDS
+    selected ones (not in the bounds-checked build, whose reports go through the Python launches, nor when single launches
+    are to be observed)."""
+    return not _LAUNCHES_OBSERVED and comm is None and impl == "mma" and geo.sp == 1 and geo.tp == 1 and geo.n_wg == 1 and not _ext.DEBUG_BOUNDS
 
 
 def _native_geometry(geo: WindowGeometry, num_heads, shifted, use_mask):
@@ -154,8 +166,13 @@ class _AttnHalfFn(torch.autograd.Function):
 class _MlpHalfFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, anchor, pk: ParamPack):
-        y, mean, rstd, xn, pre, act = _ext.load().mlp_half_fwd(x, pk.ln_w, pk.ln_b, pk.fc1_w, pk.fc1_b, pk.fc2_w, pk.fc2_b, LN_EPS,
-                                                               status_word(x.device))
+        if _LAUNCHES_OBSERVED:
+            xn, mean, rstd = layernorm_cuda(x, pk.ln_w, pk.ln_b)
+            act, pre = gemm(xn, pk.fc1_w, bias=pk.fc1_b, gelu=True, save_pre=True)
+            y = gemm(act, pk.fc2_w, bias=pk.fc2_b, residual=x)
+        else:
+            y, mean, rstd, xn, pre, act = _ext.load().mlp_half_fwd(x, pk.ln_w, pk.ln_b, pk.fc1_w, pk.fc1_b, pk.fc2_w, pk.fc2_b,
+                                                                   LN_EPS, status_word(x.device))
         ctx.save_for_backward(x, mean, rstd, xn, pre, act)
         ctx.pk = pk
         return y
@@ -165,6 +182,12 @@ class _MlpHalfFn(torch.autograd.Function):
         x, mean, rstd, xn, pre, act = ctx.saved_tensors
         pk = ctx.pk
         dy = dy.contiguous()
+        if _LAUNCHES_OBSERVED:
+            wgrad_accumulate(dy, act, pk.fc2_wg, pk.fc2_bg)
+            dpre = gemm(dy, pk.fc2_w, b_mn=True, dgelu_aux=pre)
+            wgrad_accumulate(dpre, xn, pk.fc1_wg, pk.fc1_bg)
+            dxn = gemm(dpre, pk.fc1_w, b_mn=True)
+            return layernorm_bwd_cuda(dxn, x, pk.ln_w, mean, rstd, pk.ln_wg, pk.ln_bg, dres=dy), None, None
         dx = _ext.load().mlp_half_bwd(dy, x, mean, rstd, xn, pre, act, pk.ln_w, pk.fc1_w, pk.fc2_w, pk.ln_wg, pk.ln_bg, pk.fc1_wg,
                                       pk.fc1_bg, pk.fc2_wg, pk.fc2_bg, FUSE_BIAS_GRAD, status_word(x.device))
         return dx, None, None

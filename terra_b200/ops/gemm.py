@@ -24,7 +24,7 @@ from . import _flags as F
 from ..utils.nvtx import nvtx_range
 
 _status = {}
-_TRACE = os.environ.get("TERRA_TRACE", "0") == "1"
+TRACE = os.environ.get("TERRA_TRACE", "0") == "1"
 
 
 def status_word(device) -> torch.Tensor:
@@ -45,6 +45,15 @@ def check_status(device) -> None:
         raise RuntimeError(
             f"terra_b200 kernel reported error {st[0]} at site 0x{st[1] & 0xffffffff:x} (info {st[2]}, {st[3]})"
         )
+
+
+def trace_product(a, a_mn, b, b_mn, out, flags, split_k, bn, bias=None, residual=None) -> None:
+    """``TERRA_TRACE=1``: one line on stderr per product, before its launch."""
+    print(f"[terra trace] gemm a={tuple(a.shape)}/{a.dtype}/{a.stride()} a_mn={a_mn} b={tuple(b.shape)}/{b.dtype}/{b.stride()} "
+          f"b_mn={b_mn} out={tuple(out.shape)}/{out.dtype}/{out.stride()}/{out.device} flags={flags} split_k={split_k} bn={bn} "
+          f"bias={None if bias is None else (tuple(bias.shape), bias.dtype)} "
+          f"res={None if residual is None else (tuple(residual.shape), residual.dtype, residual.stride())}",
+          file=sys.stderr, flush=True)
 
 
 @nvtx_range("terra.gemm")
@@ -119,12 +128,8 @@ def gemm(
     if save_pre:
         flags |= F.EPI_SAVE_PRE
         pre = torch.empty(M, N, dtype=torch.bfloat16, device=a.device)
-    if _TRACE:
-        print(f"[terra trace] gemm a={tuple(a.shape)}/{a.dtype}/{a.stride()} a_mn={a_mn} b={tuple(b.shape)}/{b.dtype}/{b.stride()} "
-              f"b_mn={b_mn} out={tuple(out.shape)}/{out.dtype}/{out.stride()}/{out.device} flags={flags} split_k={split_k} bn={bn} "
-              f"bias={None if bias is None else (tuple(bias.shape), bias.dtype)} "
-              f"res={None if residual is None else (tuple(residual.shape), residual.dtype, residual.stride())}",
-              file=sys.stderr, flush=True)
+    if TRACE:
+        trace_product(a, a_mn, b, b_mn, out, flags, split_k, bn, bias, residual)
     ext.gemm(a, a_mn, b, b_mn, out, flags, bias, residual, dgelu_aux, pre, float(alpha), int(split_k), int(bn),
              status_word(a.device), int(sms), list(a_peers or []), int(rank), list(out_peers or []),
              int(a_flags), int(a_epoch), int(a_budget_ns), int(bool(a_interleave)), int(a_chunks), colsum)

@@ -1,6 +1,6 @@
 """The native attention half against the same launches made one by one from Python: outputs and input gradients bit for bit,
 parameter gradients to the order of their fp32 atomics (1e-5 of the norm); with and without a bias table, several samples,
-widths with partial tiles, rows given as a pitched weight-gradient operand."""
+widths with partial tiles, rows given as a pitched weight-gradient operand. The native MLP half likewise, and against fp32."""
 import pytest
 import torch
 
@@ -40,6 +40,69 @@ def test_attention_half(monkeypatch, B, nWh, nWw, window, dim, heads, shifted, t
         got.append((y.detach(), t.grad, arena.grad.clone()))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert _rel(got[0][2], got[1][2]) < 1e-5
+
+
+@pytest.mark.parametrize("dim,rows", [(96, 512), (64, 1), (72, 333), (192, 4001), (384, 20000)])
+def test_mlp_half(monkeypatch, dim, rows):
+    from terra_b200.ops import blocks
+    from terra_b200.ops.gemm import check_status
+
+    mod, arena, x = _mlp(dim, rows)
+    dy = torch.randn_like(x)
+    got = []
+    for native in (True, False):
+        monkeypatch.setattr(blocks, "_LAUNCHES_OBSERVED", not native)
+        arena.zero_grad()
+        t = x.clone().requires_grad_(True)
+        y = blocks.mlp_half(t, mod)
+        y.backward(dy)
+        check_status("cuda")
+        got.append((y.detach(), t.grad, arena.grad.clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert _rel(got[0][2], got[1][2]) < 1e-5
+    # and against the layer in fp32 (bf16 weights; three roundings of 2^-9 along the way, and the GELU fit's 2.6e-5)
+    m = {k: v.to(torch.bfloat16).float().requires_grad_(True) for k, v in mod.state_dict().items()}
+    t = x.float().requires_grad_(True)
+    xn = torch.nn.functional.layer_norm(t, (dim,), m["norm2.weight"], m["norm2.bias"], 1e-5)
+    act = torch.nn.functional.gelu(xn @ m["fc1.weight"].t() + m["fc1.bias"])
+    ref = t + act @ m["fc2.weight"].t() + m["fc2.bias"]
+    ref.backward(dy.float())
+    assert _rel(got[0][0].float(), ref.detach()) < 8e-3 and _rel(got[0][1].float(), t.grad) < 8e-3
+    for name, p in mod.named_parameters():
+        assert _rel(p.grad, m[name].grad) < 1e-2, name
+
+
+_OBSERVED = """
+import sys, torch
+names = []
+torch.cuda.nvtx.range_push, torch.cuda.nvtx.range_pop = names.append, lambda: None
+from terra_b200.models.layers import MlpHalf, SwinAttentionHalf
+from terra_b200.ops import blocks
+from terra_b200.ops.attention import WindowGeometry
+from terra_b200.utils.flat_params import ParamArena
+geo = WindowGeometry(1, 2, 2, 8, 8)
+attn, mlp = SwinAttentionHalf(1, 64, (8, 8), 2, use_relative_position_bias=True).cuda(), MlpHalf(64, 256).cuda()
+for m, run in ((attn, lambda x: blocks.attention_half(x, attn, geo, True)), (mlp, lambda x: blocks.mlp_half(x, mlp))):
+    ParamArena(m)
+    x = torch.randn(geo.rows_local, 64, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    run(x).backward(torch.ones_like(x))
+print(names.count("terra.gemm"), names.count("terra.layernorm"))
+"""
+
+
+def test_launches_can_be_observed():
+    """TERRA_TRACE=1 prints a line per product and TERRA_NVTX=1 opens a range per launch, in the halves too: two products
+    forward, two input and two weight gradients backward, one LayerNorm, each."""
+    import os
+    import subprocess
+    import sys
+
+    env = dict(os.environ, TERRA_TRACE="1", TERRA_NVTX="1")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _OBSERVED], cwd=root, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == ["12", "2"]
+    assert r.stderr.count("[terra trace] gemm") == 12
 
 
 def test_weight_gradient_of_pitched_rows():

@@ -246,6 +246,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       },
       "tile width and CTAs per tile that gemm takes when no width is asked for", py::arg("m"), py::arg("n"), py::arg("k"),
       py::arg("b_mn") = false, py::arg("flags") = 0, py::arg("sms") = 148);
+  m.def("gemm_tma_epilogue", &tb::gemm_tma_epilogue, "whether the epilogue may go through TMA (TERRA_GEMM_TMA_EPILOGUE)");
   m.def("conv3x3_fwd", &conv3x3_fwd, "implicit-GEMM 3x3 convolution (NHWC bf16)");
   m.def("conv3x3_wgrad", &conv3x3_wgrad, "3x3 convolution weight gradient (fp32 atomics)", py::arg("x"), py::arg("dy"),
         py::arg("dw"), py::arg("stride"), py::arg("split_k"), py::arg("status"), py::arg("halo_lo"), py::arg("halo_hi"),

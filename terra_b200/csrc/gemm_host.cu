@@ -81,16 +81,21 @@ static int map_chunk(CUtensorMap* out, const void* base, long long cols, long lo
   return make_tensor_map_bf16(out, base, 2, dims, str, box);
 }
 
-// Plain row-major bf16 outputs leave through TMA stores (and the residual / GELU-input operand arrives through TMA
-// loads) when every matrix qualifies for a tensor map; otherwise the epilogue keeps its per-lane global accesses.
-static void try_tma_epilogue(GemmParams& p, long long M, long long N) {
+// TERRA_GEMM_TMA_EPILOGUE=0: outputs are stored and epilogue operands read by the lanes themselves.
+bool gemm_tma_epilogue() {
   static const bool enabled = [] {
     const char* e = std::getenv("TERRA_GEMM_TMA_EPILOGUE");
     return e == nullptr || std::atoi(e) != 0;
   }();
+  return enabled;
+}
+
+// Plain row-major bf16 outputs leave through TMA stores (and the residual / GELU-input operand arrives through TMA
+// loads) when every matrix qualifies for a tensor map; otherwise the epilogue keeps its per-lane global accesses.
+static void try_tma_epilogue(GemmParams& p, long long M, long long N) {
   p.epi_tma = 0;
   const int f = p.epi;
-  if (!enabled || (f & (EPI_OUT_F32 | EPI_ATOMIC | EPI_ROW_CONV))) return;
+  if (!gemm_tma_epilogue() || (f & (EPI_OUT_F32 | EPI_ATOMIC | EPI_ROW_CONV))) return;
   if (((f & EPI_RESIDUAL) != 0) + ((f & EPI_MUL_DGELU) != 0) + ((f & EPI_SAVE_PRE) != 0) > 1) return;   // one second buffer
   // The input buffers cost the operand ring one or two stages. A long contraction hides the epilogue behind its main
   // loop anyway and wants the deeper ring instead (K = 1536 with a residual measured 15 % slower on three stages).
@@ -385,7 +390,10 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   p.out_mul = c.out_mul;
   p.phase_cols = c.phase_cols;
   std::memcpy(p.out_off, c.out_off, sizeof(p.out_off));
-  if (!(p.epi & ~(EPI_ROW_CONV | EPI_BIAS | EPI_BIAS_F32))) {
+  p.ldc = c.out_c;
+  // (outputs that go to every second pixel have no per-lane form)
+  const bool strided = c.out_mul != 1 || c.phase_cols != 0;
+  if (!(p.epi & ~(EPI_ROW_CONV | EPI_BIAS | EPI_BIAS_F32)) && (strided || gemm_tma_epilogue())) {
     // 32 pixels x 64 channels per store; rows and channels outside the image are clipped
     const unsigned long long C = static_cast<unsigned long long>(c.out_c), mul = static_cast<unsigned long long>(c.out_mul);
     const unsigned long long row = C * 2ull * mul * c.out_w;
@@ -396,7 +404,7 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
     rc = make_tensor_map_bf16(&p.map_c, c.y, 5, dims, str, box);
     if (rc != 0) return rc - 5000;
     p.epi_tma = 2;
-  } else if (c.out_mul != 1 || c.phase_cols != 0) {
+  } else if (strided) {
     return -16;
   }
   const cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);

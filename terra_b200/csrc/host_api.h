@@ -75,6 +75,7 @@ int gemm_bf16(const GemmOperand& A, const GemmOperand& B, long long M, long long
 // The rule's tile of a plain product (no peers, no split, no column sums) when no width is asked for: columns, and CTAs per
 // tile of 128 rows each (2: a CTA pair).
 void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, int num_sms, int* bn, int* ctas);
+bool gemm_tma_epilogue();   // whether the epilogue may go through TMA (environment switch)
 int gemm_stall_counters(unsigned long long* out8, int reset);
 
 int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin, int Cout, int stride,

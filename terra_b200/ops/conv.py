@@ -200,12 +200,12 @@ def _wgrad_split(B, H, W, stride, Cout, Cin):
 
 def _conv3x3_s2_dgrad(dy, w16, H, W, dom, weight=None):
     """Input gradient of the stride-2 convolution. One launch: the four parities of the input pixel are four tile groups
-    of the implicit GEMM, with the 1, 2, 2 or 4 taps that reach them. With halo rows to give back (multi-rank stripes), or
-    more channels than the tap table holds: dcol = dy @ W (tap-major columns) on the GEMM, then one gather kernel over the
+    of the implicit GEMM, with the 1, 2, 2 or 4 taps that reach them. With halo rows to give back (multi-rank stripes),
+    more channels than the tap table holds, or without the TMA epilogue: dcol = dy @ W (tap-major columns) on the GEMM, then one gather kernel over the
     taps that reach each input pixel."""
     B, Ho, Wo, Cout = dy.shape
     Cin = w16.shape[1]
-    if not (dom is not None and dom.world > 1) and 9 * ((Cout + 63) // 64) <= _MAX_TAP_CHUNKS:
+    if not (dom is not None and dom.world > 1) and 9 * ((Cout + 63) // 64) <= _MAX_TAP_CHUNKS and _ext.load().gemm_tma_epilogue():
         wp = _packed(weight, w16, "s2dgrad_taps", pack_conv3x3_weight_s2_dgrad) if weight is not None else \
             pack_conv3x3_weight_s2_dgrad(w16)
         out = torch.empty(B, H, W, Cin, device=dy.device, dtype=torch.bfloat16)
@@ -246,9 +246,9 @@ def conv3x3(x, conv: torch.nn.Conv2d, stride: int = 1, dom=None):
 
 # ------------------------------------------------------------------------------------------------ transposed conv 2x2 / s2
 def _convt_tiled(Cin, Cout):
-    """The gathered forms: the (tap, channel chunk) tables must hold the layer. Larger channel counts go through a plain GEMM
-    and permuted copies."""
-    return Cout % 8 == 0 and Cin % 8 == 0 and max(4 * ((Cout + 63) // 64), (Cin + 63) // 64) <= _MAX_TAP_CHUNKS
+    """The gathered forms: the (tap, channel chunk) tables must hold the layer, and their outputs leave through TMA. Otherwise
+    a plain GEMM and permuted copies."""
+    return _ext.load().gemm_tma_epilogue() and Cout % 8 == 0 and Cin % 8 == 0 and max(4 * ((Cout + 63) // 64), (Cin + 63) // 64) <= _MAX_TAP_CHUNKS
 
 
 class _ConvT2x2Fn(torch.autograd.Function):

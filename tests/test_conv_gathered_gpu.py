@@ -70,3 +70,45 @@ def test_transposed_convolution(B, H, W, Cin, Cout):
         check_status("cuda")
         assert _rel(y.permute(0, 3, 1, 2), yr) < REL and _rel(xc.grad.permute(0, 3, 1, 2), xr.grad) < REL
         assert _rel(m.weight.grad, ref.weight.grad) < REL and _rel(m.bias.grad, ref.bias.grad) < REL
+
+
+_BY_LANE = """
+import sys, torch
+from terra_b200 import _ext
+from terra_b200.ops import conv
+ext = _ext.load()
+assert not ext.gemm_tma_epilogue()
+torch.manual_seed(5)
+mods = [torch.nn.Conv2d(96, 72, 3, padding=1), torch.nn.Conv2d(96, 72, 3, stride=2, padding=1), torch.nn.ConvTranspose2d(96, 72, 2, stride=2)]
+out = []
+for m, op in zip(mods, (conv.conv3x3, lambda x, m: conv.conv3x3(x, m, 2), conv.conv_transpose2x2)):
+    m = m.cuda()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(p.to(torch.bfloat16).float())
+    x = torch.randn(2, 18, 140, 96, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    y = op(x, m)
+    dy = torch.randn(y.shape, device="cuda").to(torch.bfloat16)
+    y.backward(dy)
+    xr = x.detach().float().permute(0, 3, 1, 2).requires_grad_(True)
+    yr = m(xr)
+    yr.backward(dy.float().permute(0, 3, 1, 2))
+    rel = lambda a, b: ((a.float().permute(0, 3, 1, 2) - b).norm() / b.norm()).item()
+    out += [rel(y.detach(), yr.detach()), rel(x.grad, xr.grad)]
+print(*out)
+"""
+
+
+def test_convolutions_without_the_tma_epilogue():
+    """TERRA_GEMM_TMA_EPILOGUE=0 reaches the convolutions: per-lane stores, or the general path where there are none (columns
+    that are rounded to bf16 as well for the stride-2 input gradient)."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _BY_LANE], cwd=root, env=dict(os.environ, TERRA_GEMM_TMA_EPILOGUE="0"),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    errors = [float(v) for v in r.stdout.split()]
+    assert len(errors) == 6 and max(errors[:3] + errors[4:]) < REL and errors[3] < 2 * REL, errors

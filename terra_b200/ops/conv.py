@@ -202,7 +202,9 @@ def _conv3x3_s2_dgrad(dy, w16, H, W, dom, weight=None):
     """Input gradient of the stride-2 convolution. One launch: the four parities of the input pixel are four tile groups
     of the implicit GEMM, with the 1, 2, 2 or 4 taps that reach them. With halo rows to give back (multi-rank stripes),
     more channels than the tap table holds, or without the TMA epilogue: dcol = dy @ W (tap-major columns) on the GEMM, then one gather kernel over the
-    taps that reach each input pixel."""
+    taps that reach each input pixel. (Images of fewer than about 50 columns of ``dy`` would be faster by columns - 32768
+    pixels of 384 channels, us, one launch / columns: 2048 x 16 472 / 161, 682 x 48 166 / 159, 512 x 64 128 / 162 - but the
+    columns round every tap's share to bf16 where the one launch sums them in fp32.)"""
     B, Ho, Wo, Cout = dy.shape
     Cin = w16.shape[1]
     if not (dom is not None and dom.world > 1) and 9 * ((Cout + 63) // 64) <= _MAX_TAP_CHUNKS and _ext.load().gemm_tma_epilogue():
@@ -245,9 +247,14 @@ def conv3x3(x, conv: torch.nn.Conv2d, stride: int = 1, dom=None):
 
 
 # ------------------------------------------------------------------------------------------------ transposed conv 2x2 / s2
-def _convt_tiled(Cin, Cout):
+def _convt_tiled(B, H, W, Cin, Cout):
     """The gathered forms: the (tap, channel chunk) tables must hold the layer, and their outputs leave through TMA. Otherwise
-    a plain GEMM and permuted copies."""
+    a plain GEMM and permuted copies, as for images of fewer than 32 columns whose rows make more than one round of tiles: a
+    tile is 128 pixels of one row, so below a quarter of it the padding costs more than the copies. Forward + backward at
+    32768 pixels of 384 channels (us, gathered / general): 2048 x 16 658 / 440, 1365 x 24 466 / 442, 1024 x 32 368 / 441, 512 x 64
+    232 / 440; at 512 pixels, in one round, 32 x 16 53 / 77 (both forms round once: the sums are fp32)."""
+    if W < 32 and B * H > 148:
+        return False
     return _ext.load().gemm_tma_epilogue() and Cout % 8 == 0 and Cin % 8 == 0 and max(4 * ((Cout + 63) // 64), (Cin + 63) // 64) <= _MAX_TAP_CHUNKS
 
 
@@ -260,7 +267,7 @@ class _ConvT2x2Fn(torch.autograd.Function):
         w16 = weight.bf16 if getattr(weight, "bf16", None) is not None else weight.detach().to(torch.bfloat16)
         b16 = bias.bf16 if getattr(bias, "bf16", None) is not None else bias.detach().to(torch.bfloat16)
         y = torch.empty(B, 2 * H, 2 * W, Cout, device=x.device, dtype=torch.bfloat16)
-        if _convt_tiled(Cin, Cout):
+        if _convt_tiled(B, H, W, Cin, Cout):
             # rows (dy, dx, co), every phase padded to whole units of the epilogue, which stores it to its pixels
             pad = (Cout + 63) // 64 * 64
             wt = _packed(weight, w16, "convT", lambda w: _pack_taps(w, 4, 1, Cout, 4, Cin, 4 * Cout, (0,), pad))
@@ -268,8 +275,8 @@ class _ConvT2x2Fn(torch.autograd.Function):
             ext.convt2x2(0, x.contiguous(), wt, b4, y, status_word(x.device))
         else:
             b4 = _packed(bias, b16, "convT_bias_flat", lambda b: b.repeat(4))
-            flat = gemm(x.view(-1, Cin), _convt_flat_weight(weight, w16), bias=b4)
-            y.copy_(flat.view(B, H, W, 2, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B, 2 * H, 2 * W, Cout))
+            flat = gemm(x.reshape(-1, Cin), _convt_flat_weight(weight, w16), bias=b4)
+            y.view(B, H, 2, W, 2, Cout).copy_(flat.view(B, H, W, 2, 2, Cout).transpose(2, 3))
         ctx.save_for_backward(x)
         ctx.p = (w16, Cout, weight, bias)
         return y
@@ -280,7 +287,7 @@ class _ConvT2x2Fn(torch.autograd.Function):
         (x,) = ctx.saved_tensors
         w16, Cout, weight, bias = ctx.p
         B, H, W, Cin = x.shape
-        tiled = _convt_tiled(Cin, Cout)
+        tiled = _convt_tiled(B, H, W, Cin, Cout)
         dy = dy.contiguous()
         gw, gb = _arena_grad(weight), _arena_grad(bias)
         if tiled:
@@ -292,7 +299,7 @@ class _ConvT2x2Fn(torch.autograd.Function):
             # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it. [tap, co, ci] staging
             dyu = dy.view(B, H, 2, W, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B * H * W, 4 * Cout)
             shape, layout = (4, Cout, Cin), (1, 4, Cout * 4)
-            wgrad = lambda dwt: wgrad_accumulate(dyu, x.view(-1, Cin), dwt.view(4 * Cout, Cin))
+            wgrad = lambda dwt: wgrad_accumulate(dyu, x.reshape(-1, Cin), dwt.view(4 * Cout, Cin))
         if gw is not None:
             dwt = _zero_scratch(x.device, shape, "convT")
             wgrad(dwt)

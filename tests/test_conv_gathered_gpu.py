@@ -42,6 +42,7 @@ def test_stride2_input_gradient(B, H, W, Cin, Cout):
     (1, 1, 1, 64, 64), (1, 16, 24, 96, 96), (2, 7, 130, 64, 64), (1, 5, 3, 128, 32), (1, 9, 33, 40, 96), (1, 20, 257, 192, 384),
     (1, 256, 256, 64, 192),                # CTA pairs
     (1, 6, 10, 64, 40),                    # phases that end inside a unit of the epilogue
+    (1, 149, 24, 64, 64), (2, 80, 3, 64, 96),            # narrow images: GEMM and permuted copy
     (1, 3, 5, 64, 2056),                   # more channels than the tap table holds: GEMM and permuted copy
 ])
 def test_transposed_convolution(B, H, W, Cin, Cout):

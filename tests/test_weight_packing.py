@@ -40,3 +40,13 @@ def test_kernel(cout, cin):
     v = _weights(cin, cout, 2)             # transposed convolution: (Cin, Cout, 2, 2)
     for args in ((4, 1, cout, 4, cin, 4 * cout, (0,)), (4, 1, cout, 4, cin, 4 * cout, (0,), cout + 56), (1, 0, cin, 4 * cout, cout, 4, range(4))):
         assert torch.equal(conv._pack_taps(v.cuda(), *args).cpu(), conv._pack_taps(v, *args))
+
+
+def test_transposed_convolution_takes_wide_images_and_small_ones_gathered():
+    """The rule between the gathered transposed convolution and the general path (the kernel's tiles are 128 pixels of a row)."""
+    from terra_b200.ops import conv
+
+    tiled = lambda *a: bool(conv._convt_tiled(*a))
+    assert tiled(1, 5000, 32, 96, 96) and tiled(1, 4, 4, 96, 96) and tiled(1, 148, 31, 96, 96) and tiled(1, 256, 544, 384, 384)
+    assert not tiled(1, 149, 31, 96, 96) and not tiled(2, 75, 8, 96, 96)
+    assert not tiled(1, 64, 64, 60, 96) and not tiled(1, 64, 64, 96, 60) and not tiled(1, 64, 64, 96, 2056)

@@ -239,13 +239,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("a_interleave"), py::arg("a_chunks"), py::arg("colsum") = py::none());
   m.def(
       "gemm_tile",
-      [](int64_t M, int64_t N, int64_t K, bool b_mn, int64_t flags, int64_t sms) {
+      [](int64_t M, int64_t N, int64_t K, bool b_mn, int64_t flags, int64_t sms, bool gathered) {
         int bn = 0, ctas = 0;
-        tb::gemm_tile(M, N, K, b_mn, static_cast<int>(flags), static_cast<int>(sms), &bn, &ctas);
+        tb::gemm_tile(M, N, K, b_mn, static_cast<int>(flags), gathered, static_cast<int>(sms), &bn, &ctas);
         return std::make_pair(bn, ctas);
       },
       "tile width and CTAs per tile that gemm takes when no width is asked for", py::arg("m"), py::arg("n"), py::arg("k"),
-      py::arg("b_mn") = false, py::arg("flags") = 0, py::arg("sms") = 148);
+      py::arg("b_mn") = false, py::arg("flags") = 0, py::arg("sms") = 148, py::arg("gathered") = false);
   m.def("gemm_tma_epilogue", &tb::gemm_tma_epilogue, "whether the epilogue may go through TMA (TERRA_GEMM_TMA_EPILOGUE)");
   m.def("conv3x3_fwd", &conv3x3_fwd, "implicit-GEMM 3x3 convolution (NHWC bf16)");
   m.def("conv3x3_wgrad", &conv3x3_wgrad, "3x3 convolution weight gradient (fp32 atomics)", py::arg("x"), py::arg("dy"),

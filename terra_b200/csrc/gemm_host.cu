@@ -118,10 +118,8 @@ static int pick_bn(long long N, int requested) {
 
 // CTA pairs (256-row tiles, one MMA over two SMs). What bounds the main loop is the shared-memory port (128 B per clock
 // and SM): a k-block of a 128 x BN tile costs (16 + BN / 8) KB of operand fill and as much again for the tensor core's
-// reads. In a pair each CTA stages 128 rows of A and only half of B's BN rows, (16 + BN / 16) KB. Pairs are taken by
-// plain products (no peers, no split, no column sums) as soon as their tiles make eight rounds over the
-// pairs of SMs; with fewer rounds the larger tiles leave more of the last one empty (17280 rows, 576 x 192: 12 us with
-// single CTAs, 18 us with pairs; 139264 rows, 1152 x 384: 130 and 117 us).
+// reads. In a pair each CTA stages 128 rows of A and only half of B's BN rows, (16 + BN / 16) KB. A pair starts later (two
+// cluster barriers) and its larger tiles leave more of the last round empty.
 static bool pairs_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("TERRA_GEMM_2CTA");
@@ -130,39 +128,59 @@ static bool pairs_enabled() {
   return on;
 }
 
-// Tile of a plain product with many tiles: the width and CTA count with the fewest cycles per 128 rows. A tile takes the
-// longer of its main loop and its epilogue (rounds of 64-column units over three warps per lane quadrant, by what a unit
-// does). A k-block takes the longest of its MMAs (2 BN cycles), its bytes through the shared-memory port (fill and
-// tensor-core reads at 128 bytes a cycle) and about 450 cycles of hand-over. Measured on 139264 rows (us): pairs of 192 / 256
-// 1152 x 384 with bias 128 / 133, 384 x 384 with residual 66 / 86, 3072 x 1024 804 / 645; 2976 x 384 with residual on
-// 278528 rows 848 / 1038; times GELU', 1536 x 384, single 192 / pairs of 256 290 / 327.
-static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, int num_sms, int* bn_out, int* ctas_out) {
+// Tile of a plain product or gathered convolution (no peers, no split, no column sums): the width and CTA count with the
+// least time by a model, in us. Persistent CTAs (pairs) take rounds of tiles; a tile takes the longer of its main loop and its
+// epilogue (rounds of 64-column units over the three warps of a lane quadrant, or of 32-column chunks where the lanes store
+// themselves) and a fixed hand-over, and the shorter of the two shows once, before the first or after the last tile.
+//
+// The constants were fitted to measurements, passes back to back in a CUDA graph at 1.9 GHz, falling to about 1.4 GHz under the
+// power cap in the largest. Products: 64 to 278528 rows, 31 pairs of N and K between 96 and 4096, five epilogues, all six
+// tiles (6600 times). Convolutions: the five forms, 64 to 384 channels, 16 x 32 to 512 x 1088 pixels (1500 times). The choice is
+// 0.5 % (0.3 %) slower than the best tile on average, more than 10 % in one case of 80 (none).
+// Against a rule that weighed tiles without rounds and start (us, both in turn on one GPU, before / this): 80000 x 136 x 384
+// with bias 36 / 21, 17280 x 1000 x 1000 62 / 41, 17280 x 1024 x 1024 GELU 52 / 43, 512 x 1024 x 4096 26 / 18; no change beyond the
+// noise for the 139264-row products of width 384 and 1024.
+struct TileCosts {
+  double start[2], tile, tail, plain_unit;   // start: single CTAs, pairs
+  double kblock[2][3];                       // main loop per 64-wide k-block, widths 128, 192, 256
+};
+static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, bool gathered, int num_sms, int* bn_out,
+                      int* ctas_out) {
   *bn_out = pick_bn(N, 0);
   *ctas_out = 1;
-  const bool second = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU | EPI_SAVE_PRE)) != 0;
-  // the ring keeps too little beside two units per epilogue warp when single tiles are 256 wide
-  // (an input operand with a longer contraction takes the per-lane epilogue, which needs no such room)
-  if (*bn_out == 256 && second && (k_blocks <= 12 || (flags & EPI_SAVE_PRE))) *bn_out = 192;
-  if (!pairs_enabled() || num_sms < 2 || N < 128 || ((m_blocks + 1) / 2) * ((N + 255) / 256) < 8LL * (num_sms / 2)) return;
-  const long long unit = (flags & EPI_MUL_DGELU) ? 4500 : (flags & EPI_SAVE_PRE) ? 3500 : (flags & EPI_RESIDUAL) ? 2500 : 2000;
-  long long best = 0;
-  for (int ctas : {2, 1})
-    for (int bn : {256, 192, 128}) {
-      if (ctas == 2 && b_mn && bn == 192) continue;      // half of an MN-major B must be whole 64-row boxes
-      if (ctas == 1 && bn == 256 && second) continue;
-      const long long port = 16 * (16 + bn / (8 * ctas));
-      const long long loop = k_blocks * std::max(450LL, std::max(2LL * bn, port));
-      const long long cost = (N + bn - 1) / bn * std::max(loop, unit * ((bn / 64 + 2) / 3));
-      if (best == 0 || cost < best) {
-        best = cost;
+  if (N <= 64 || m_blocks < 1) return;
+  static const TileCosts rows = {{3.6, 6.1}, 0.95, 0.82, 0.83, {{0.29, 0.37, 0.45}, {0.215, 0.295, 0.39}}};
+  static const TileCosts image = {{4.5, 6.5}, 1.0, 0.62, 1.35, {{0.26, 0.31, 0.36}, {0.255, 0.286, 0.33}}};
+  const TileCosts& cost = gathered ? image : rows;
+  const bool input = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0, second = input || (flags & EPI_SAVE_PRE);
+  const double unit = (flags & EPI_MUL_DGELU) ? 2.9 : (flags & EPI_RESIDUAL) ? 1.88 : (flags & (EPI_GELU | EPI_SAVE_PRE)) ? 1.69 : cost.plain_unit;
+  const bool by_lane = !gemm_tma_epilogue() || (flags & (EPI_OUT_F32 | EPI_ATOMIC)) || (input && k_blocks > 12);
+  double least = 0.0;
+  for (int ctas : {1, 2}) {
+    if (ctas == 2 && (!pairs_enabled() || num_sms < 2)) continue;
+    for (int w = 0; w < 3; ++w) {
+      const int bn = 128 + 64 * w;
+      if (bn >= 2 * N || (ctas == 2 && b_mn && bn == 192)) continue;      // half of an MN-major B must be whole 64-row boxes
+      const long long tiles = (m_blocks + ctas - 1) / ctas * ((N + bn - 1) / bn), units = num_sms / ctas;
+      const long long cols = std::min<long long>(bn, N);
+      // (single tiles of 256 columns leave no room for a second staging buffer beside the operand ring)
+      const bool lanes = by_lane || (second && bn == 256 && ctas == 1);
+      const double loop = k_blocks * cost.kblock[ctas - 1][w] * (ctas == 2 && b_mn ? 0.82 : 1.0);
+      const double epilogue = unit * (lanes ? ((cols + 31) / 32 + 2) / 3 : ((cols + 63) / 64 + 2) / 3);
+      // (a tie goes to the pair, which loads less)
+      const double time = (cost.start[ctas - 1] + (tiles + units - 1) / units * (std::max(loop, epilogue) + cost.tile) +
+                           cost.tail * std::min(loop, epilogue)) * (ctas == 2 ? 0.99 : 1.0);
+      if (least == 0.0 || time < least) {
+        least = time;
         *bn_out = bn;
         *ctas_out = ctas;
       }
     }
+  }
 }
 
-void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, int num_sms, int* bn, int* ctas) {
-  pick_tile((M + GEMM_BM - 1) / GEMM_BM, N, static_cast<int>((K + GEMM_BK - 1) / GEMM_BK), b_mn, flags, num_sms, bn, ctas);
+void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, bool gathered, int num_sms, int* bn, int* ctas) {
+  pick_tile((M + GEMM_BM - 1) / GEMM_BM, N, static_cast<int>((K + GEMM_BK - 1) / GEMM_BK), b_mn, flags, gathered, num_sms, bn, ctas);
 }
 
 static void fill_epilogue(GemmParams& p, const GemmEpilogue& e) {
@@ -207,7 +225,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
     bn_request -= 1000;
     if (bn_request != 128 && bn_request != 256 && !(bn_request == 192 && !B.mn_major)) return -11;
   } else if (bn_request == 0 && !A.mn_major && !gather_a && !scatter_c && split_k <= 1 && epi.colsum == nullptr) {
-    gemm_tile(M, N, K, B.mn_major != 0, epi.flags, num_sms, &bn_request, &ctas);
+    gemm_tile(M, N, K, B.mn_major != 0, epi.flags, false, num_sms, &bn_request, &ctas);
   }
   if (epi.colsum != nullptr) {
     // column sums ride on the weight-gradient form only, and need room for their accumulators behind the tile's
@@ -346,7 +364,7 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   std::memset(&p, 0, sizeof(p));
   const long long m_blocks = static_cast<long long>((c.tiles_w + GEMM_BM - 1) / GEMM_BM) * c.tiles_h * c.B;
   int bn = 0, ctas = 1;
-  pick_tile(m_blocks * c.groups, c.N, c.ntaps * cchunks / c.groups, false, epi.flags, num_sms, &bn, &ctas);
+  pick_tile(m_blocks * c.groups, c.N, c.ntaps * cchunks / c.groups, false, epi.flags, true, num_sms, &bn, &ctas);
   p.M = c.B * c.tiles_h * c.tiles_w;
   p.N = c.N;
   p.K = c.ntaps * cchunks * 64;

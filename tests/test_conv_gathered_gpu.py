@@ -1,6 +1,6 @@
 """The strided forms of the implicit GEMM: input gradient of the stride-2 convolution and the three products of the 2x2
 transposed convolution, against fp32 PyTorch, at ragged widths (tiles are 128 pixels wide), odd heights, channel counts with
-a padded chunk, sizes that take CTA pairs, and the channel counts that keep the general path.
+a padded chunk, sizes that take CTA pairs (there the 3x3 forms as well), and the channel counts that keep the general path.
 
 Bound: bf16 operands are exact, sums fp32, one rounding of the result: 2^-9 = 0.2 % of the norm; the tests allow 0.4 %."""
 import pytest
@@ -21,7 +21,7 @@ def _rel(got, ref):
 
 @pytest.mark.parametrize("B,H,W,Cin,Cout", [
     (1, 2, 2, 64, 64), (1, 1, 4, 32, 64), (2, 13, 200, 96, 96), (1, 33, 258, 96, 192), (1, 8, 16, 40, 72), (1, 64, 300, 384, 384),
-    (1, 512, 512, 192, 64),                # CTA pairs
+    (1, 512, 512, 192, 64),                # two tiles per image row, many rounds
     (1, 6, 20, 64, 1024),                  # more channels than the tap table holds: columns and gather
 ])
 def test_stride2_input_gradient(B, H, W, Cin, Cout):
@@ -40,7 +40,7 @@ def test_stride2_input_gradient(B, H, W, Cin, Cout):
 
 @pytest.mark.parametrize("B,H,W,Cin,Cout", [
     (1, 1, 1, 64, 64), (1, 16, 24, 96, 96), (2, 7, 130, 64, 64), (1, 5, 3, 128, 32), (1, 9, 33, 40, 96), (1, 20, 257, 192, 384),
-    (1, 256, 256, 64, 192),                # CTA pairs
+    (1, 256, 256, 64, 192),                # two tiles per image row, many rounds
     (1, 6, 10, 64, 40),                    # phases that end inside a unit of the epilogue
     (1, 149, 24, 64, 64), (2, 80, 3, 64, 96),            # narrow images: GEMM and permuted copy
     (1, 3, 5, 64, 2056),                   # more channels than the tap table holds: GEMM and permuted copy
@@ -71,6 +71,75 @@ def test_transposed_convolution(B, H, W, Cin, Cout):
         check_status("cuda")
         assert _rel(y.permute(0, 3, 1, 2), yr) < REL and _rel(xc.grad.permute(0, 3, 1, 2), xr.grad) < REL
         assert _rel(m.weight.grad, ref.weight.grad) < REL and _rel(m.bias.grad, ref.bias.grad) < REL
+
+
+def _pairs(row_tiles, N, k_blocks):
+    from terra_b200 import _ext
+
+    return _ext.load().gemm_tile(128 * row_tiles, N, 64 * k_blocks, gathered=True)[1] == 2
+
+
+@pytest.mark.parametrize("B,H,W,stride,halos", [
+    (1, 1201, 100, 1, False), (1, 601, 200, 1, True), (3, 401, 100, 1, False),      # 1201, 1202, 1203 row tiles
+    (1, 2401, 200, 2, False), (3, 801, 200, 2, True),                                # 1201, 1203
+])
+def test_3x3_convolutions_on_pairs(B, H, W, stride, halos):
+    """Forward with bias, and the input gradient of stride 1 (the same kernel on other weights), on CTA pairs: counts of row tiles
+    that leave half a pair over, several samples, rows from a neighbour above and below."""
+    from terra_b200 import _ext
+    from terra_b200.ops.conv import pack_conv3x3_weight, pack_conv3x3_weight_dgrad
+    from terra_b200.ops.gemm import check_status, status_word
+
+    torch.manual_seed(6)
+    Cin, Cout, ext = 64, 192, _ext.load()
+    Ho, Wo = -(-H // stride), W // stride
+    assert _pairs(-(-Wo // 128) * Ho * B, Cout, 9)
+    x, w, bias = _rand(B, H, W, Cin), _rand(Cout, Cin, 3, 3, scale=0.04), _rand(Cout)
+    lo, hi = (_rand(B, 1, W, Cin), _rand(B, 1, W, Cin)) if halos else (None, None)
+    y = torch.empty(B, Ho, Wo, Cout, device="cuda", dtype=torch.bfloat16)
+    ext.conv3x3_fwd(x, pack_conv3x3_weight(w), y, stride, 1, bias, None, status_word("cuda"), lo, hi)     # 1: with bias
+    check_status("cuda")
+    zero = torch.zeros_like(x[:, :1])
+    whole = torch.cat([zero if lo is None else lo, x, zero if hi is None else hi], dim=1).float().permute(0, 3, 1, 2)
+    ref = TF.conv2d(whole, w.float(), bias.float(), stride=stride, padding=(0, 1))[:, :, :Ho]
+    assert _rel(y.permute(0, 3, 1, 2), ref) < REL
+    if stride == 1:
+        wt = _rand(Cin, Cout, 3, 3, scale=0.04)       # of the convolution whose input has the 192 channels
+        dx = torch.empty(B, H, W, Cout, device="cuda", dtype=torch.bfloat16)
+        ext.conv3x3_fwd(x, pack_conv3x3_weight_dgrad(wt), dx, 1, 0, None, None, status_word("cuda"), lo, hi)
+        check_status("cuda")
+        ref = TF.conv_transpose2d(whole, wt.float(), padding=1)[:, :, 1:-1]
+        assert _rel(dx.permute(0, 3, 1, 2), ref) < REL
+
+
+def test_strided_forms_on_pairs():
+    """The input gradient of the stride-2 convolution and the transposed convolution with half a pair left over."""
+    from terra_b200 import _ext
+    from terra_b200.ops import conv
+    from terra_b200.ops.gemm import check_status, status_word
+
+    torch.manual_seed(7)
+    ext, B, H, W = _ext.load(), 3, 401, 100              # 1203 row tiles
+    Cin, Cout = 192, 256
+    assert _pairs(4 * B * H, Cin, 9)
+    w, dy = _rand(Cout, Cin, 3, 3, scale=0.04), _rand(B, H, W, Cout)
+    dx = torch.empty(B, 2 * H, 2 * W, Cin, device="cuda", dtype=torch.bfloat16)
+    ext.conv3x3_s2_dgrad(dy, conv.pack_conv3x3_weight_s2_dgrad(w), dx, status_word("cuda"))
+    check_status("cuda")
+    ref = TF.conv_transpose2d(dy.float().permute(0, 3, 1, 2), w.float(), stride=2, padding=1, output_padding=1)
+    assert _rel(dx.permute(0, 3, 1, 2), ref) < REL
+    Cin, Cout = 384, 192
+    assert _pairs(B * H, 4 * Cout, Cin // 64) and _pairs(B * H, Cin, 4 * Cout // 64)
+    x, w, bias = _rand(B, H, W, Cin), _rand(Cin, Cout, 2, 2, scale=0.05), _rand(Cout)
+    y = torch.empty(B, 2 * H, 2 * W, Cout, device="cuda", dtype=torch.bfloat16)
+    ext.convt2x2(0, x, conv._pack_taps(w, 4, 1, Cout, 4, Cin, 4 * Cout, (0,)), bias.repeat(4), y, status_word("cuda"))
+    dx = torch.empty_like(x)
+    ext.convt2x2(1, y, conv._pack_taps(w, 1, 0, Cin, 4 * Cout, Cout, 4, range(4)), None, dx, status_word("cuda"))
+    check_status("cuda")
+    ref = TF.conv_transpose2d(x.float().permute(0, 3, 1, 2), w.float(), bias.float(), stride=2)
+    assert _rel(y.permute(0, 3, 1, 2), ref) < REL
+    ref = TF.conv2d(y.float().permute(0, 3, 1, 2), w.float(), stride=2)
+    assert _rel(dx.permute(0, 3, 1, 2), ref) < REL
 
 
 _BY_LANE = """

@@ -60,16 +60,23 @@ def test_untransposed_weights(bn, M, N, K):
     assert _rel(got, a.float() @ w.float()) < REL
 
 
-@pytest.mark.parametrize("N,K,b_mn", [(384, 64, False), (1152, 40, False), (384, 96, True)])
+@pytest.mark.parametrize("N,K,b_mn", [(1152, 320, False), (384, 320, True), (96, 384, False)])
 def test_rule_takes_pairs_for_many_tiles(N, K, b_mn):
-    """Row counts far above and just below the rule's line (eight rounds over the SM pairs) give the same products."""
+    """The smallest product for which the rule takes CTA pairs, the one below it, and one whose last pair holds a single row
+    block, each with a ragged last block: the rule's choice and the values."""
+    from terra_b200 import _ext
     from terra_b200.ops.gemm import check_status, gemm
 
     torch.manual_seed(3)
-    a = _rand(2 * 128 * 640 + 77, K)
+    pairs = lambda blocks: _ext.load().gemm_tile(128 * blocks - 51, N, K, b_mn)[1] == 2
+    line = next(b for b in range(1, 2000) if pairs(b))
+    odd = next(b for b in range(line | 1, 4000, 2) if pairs(b))
+    a = _rand(128 * max(line, odd) - 51, K)
     w = _rand(K, N, scale=K ** -0.5) if b_mn else _rand(N, K, scale=K ** -0.5)
     ref = a.float() @ (w.float() if b_mn else w.float().t())
-    for rows in (a.shape[0], 128 * 147 + 5):
+    for blocks in (line, line - 1, odd):
+        assert pairs(blocks) == (blocks != line - 1)
+        rows = 128 * blocks - 51
         got = gemm(a[:rows].contiguous(), w, b_mn=b_mn)
         check_status("cuda")
         assert _rel(got, ref[:rows]) < REL

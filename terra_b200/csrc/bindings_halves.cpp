@@ -98,12 +98,13 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 
 // Tile width, row blocks per tile and split of the contraction for N x K outputs over M rows. A k-block costs a CTA its
 // operand fill plus the tensor core's reads through the shared-memory port, in KB; the column sums add 40 KB per row block,
-// shared out over the column tiles. Every split pays its start and its pass of atomics (about 1000 KB a row block). Widths
-// of 256 leave no room for the sums' accumulators: dy is then read once more (5 TB/s against 3.7 us per 1000 KB).
-// Measured (139264 rows, us, sums in the first column tile): 1152 x 384 unstacked / stacked 125 / 132, 1536 x 384 163 / 155,
-// 384 x 1536 171 / 212 (three row blocks stack badly). By this rule, before -> now: 2976 x 384 over 557056 rows
-// 1322 -> 1104, 384 x 2976 1535 (128-wide) -> 1132, 1152 x 384 126 -> 116, 3072 x 1024 over 156672 rows 811 + 176 for the
-// sums -> 817, 3x3 convolution 384 -> 384 at 557056 pixels 1584 -> 1351.
+// shared out over the column tiles. Every split pays its start and its pass of atomics (1100 KB a row block, and 1.3 KB per
+// output block of the whole launch). Widths of 256 leave no room for the sums' accumulators: the column sums are then two
+// launches of their own, which read dy once more (10 us and 8.9 TB/s against 3.7 us per 1000 KB).
+// The constants were fitted to 11000 times: 64 to 557056 rows, 45 pairs of N and K between 96 and 4096, all widths, stacked or not, one
+// to four rounds (passes back to back in a CUDA graph); the choice is 2 % slower than the best plan on average. Without the 10 us the
+// separate sums were taken for few rows too (us, that / this rule): 512 rows of 384 x 1536 22 / 9, 2048 of 256 x 1024 19 / 9, 17280 of
+// 192 x 2208 39 / 23, 156672 of 3072 x 1024 839 / 799.
 struct WgradPlan {
   int bn, stack, split;
 };
@@ -116,12 +117,13 @@ WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
     for (int bn : {192, 128, 256}) {
       const int64_t n = (K + bn - 1) / bn, tiles = (m_blocks + stack - 1) / stack * n;
       const double kb = 16.0 * stack + bn / 8 + stack * (16.0 + bn / 8) + (sums && bn < 256 ? 40.0 * stack / n : 0.0);
-      const double extra = sums && bn == 256 ? 2.0 * M * N / 5e6 / 0.0037 : 0.0;
+      const double extra = sums && bn == 256 ? (10.0 + 2.0 * M * N / 8.9e6) / 0.0037 : 0.0;
       // whole rounds of CTAs: the largest split of one round, two rounds, ...
       for (int64_t rounds = 1; rounds <= 3; ++rounds) {
         const int64_t split = std::max<int64_t>(1, std::min(rounds * sms / tiles, k_blocks));
         const int64_t per = (k_blocks + split - 1) / split;
-        const double cost = static_cast<double>((tiles * split + sms - 1) / sms) * (per * kb + 1000.0 * stack) + extra;
+        const double cost = static_cast<double>((tiles * split + sms - 1) / sms) * (per * kb + 1100.0 * stack) +
+                            1.3 * tiles * split * stack * bn / 192 + extra;
         if (least < 0.0 || cost < least * 0.995) {
           least = cost;
           best = {bn, stack, static_cast<int>(split)};

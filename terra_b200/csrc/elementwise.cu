@@ -33,8 +33,8 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // would leave half of its lanes idle in the second vector. LPR is the largest power of two that divides the row's
 // vectors; rows of more than 3 odd vectors per lane fall back to 32 lanes with a bounds test. The backward kernel keeps its
 // operands packed and computes x-hat twice, which lets three blocks of four warps share an SM.
-// 139264 x 384, one row per warp -> this: forward 48.8 -> 38.4 us (32 us at 6.65 TB/s), backward with shortcut
-// 112 -> 80 us (64 us); 156672 x 1024 backward 292 -> 273 us (193 us).
+// 139264 x 384, one row per warp -> this: forward 49 -> 37 us (33 us at 6.5 TB/s), backward with shortcut 110 -> 79 us (65 us);
+// 139264 x 1024 backward 250 -> 234 us (175 us).
 template <int LPR>
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -43,7 +43,7 @@ __device__ __forceinline__ float group_sum(float v) {
 }
 
 template <int LPR, int VPL, bool EXACT>
-__global__ void __launch_bounds__(256, VPL <= 2 ? 6 : (VPL == 3 ? 4 : 1)) layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256, VPL == 1 ? 6 : (VPL == 2 ? 5 : (VPL <= 4 ? 4 : (VPL == 6 ? 3 : 2)))) layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ gamma,
                                                             const __nv_bfloat16* __restrict__ beta,
                                                             __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out,
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256, VPL <= 2 ? 6 : (VPL == 3 ? 4 : 1)) layern
   for (long long base = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * RPW; base < rows;
        base += step) {
     const long long row = base + lane / LPR;
-    const bool live = row < rows;
+    const bool live = RPW == 1 || row < rows;
     const uint4* xr = reinterpret_cast<const uint4*>(x + row * C);
     float v[VPL][8];
     float s = 0.f;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 
   for (long long base = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * RPW; base < rows;
        base += step) {
     const long long row = base + lane / LPR;
-    const bool live = row < rows;
+    const bool live = RPW == 1 || row < rows;
     const uint4* xr = reinterpret_cast<const uint4*>(x + row * C);
     const uint4* dr = reinterpret_cast<const uint4*>(dy + row * C);
     float mu = 0.f, rs = 0.f;
@@ -923,8 +923,9 @@ int grid_for(long long work_items, int block, int max_blocks = 148 * 16) {
 
 }  // namespace
 
-// CALL sees LPR, VPL and EXACT (see the LayerNorm kernels) for rows of NVEC 16-byte vectors. MANY: every warp gets several
-// rows even when it carries 32 / LPR of them; below that a row per warp finishes sooner (shorter chains, more warps).
+// CALL sees LPR, VPL and EXACT (see the LayerNorm kernels) for rows of NVEC 16-byte vectors. MANY: rows
+// enough that groups of 32 / LPR of them still make warps for every SM; below that a row per warp finishes sooner (shorter chains,
+// more warps).
 #define TB_LN_CASE(L, V, E, CALL) { constexpr int LPR = L; constexpr int VPL = V; constexpr bool EXACT = E; CALL; }
 #define TB_LN_DISPATCH(NVEC, MANY, CALL)                        \
   switch ((MANY) ? (NVEC) : 0) {                                               \
@@ -946,10 +947,23 @@ int grid_for(long long work_items, int block, int max_blocks = 148 * 16) {
       }                                                         \
   }
 
+// Blocks of the LayerNorm kernels. Forward: one resident wave where the rows of a warp are many vectors or few, more blocks than
+// that for wide rows (278528 rows, us, 4 / 6 / 16 blocks per SM: C = 384 70 / 77 / 71, 768 142 / 160 / 142, 1024 195 / 198 / 177).
+constexpr int ln_fwd_blocks(int vpl) { return 148 * (vpl == 1 ? 6 : (vpl == 2 ? 5 : (vpl == 3 ? 4 : (vpl == 8 ? 2 : 16)))); }
+// Backward: every block ends in 2 C atomics on the same addresses, so few rows take three blocks per SM and many rows one
+// resident wave (139264 rows with shortcut, us, 2 / 3 / resident: C = 72 70 / 55 / 42, 256 116 / 87 / 62, 512 158 / 124 / 108; 4096 rows
+// of 256 7.5 / 9 / 15). Rows of five vectors per lane and more have room for two blocks; a third waits for both (2048 columns
+// 1186 / 1452).
+inline int ln_bwd_blocks(int vpl, bool exact, long long rows) {
+  if (vpl > 4) return 148 * 2;
+  const bool many = rows >= 148LL * 3 * 4 * 32;       // 32 rows for every warp of three blocks per SM
+  return 148 * (many && vpl == 1 ? (exact ? 5 : 6) : (many && vpl == 2 ? 4 : 3));
+}
+
 int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                   long long rows, int C, float eps, cudaStream_t stream) {
   if (C % 8 != 0 || C > 2048) return -1;
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 16, (layernorm_fwd_kernel<LPR, VPL, EXACT><<<grid_for(rows, 8 * (32 / LPR), VPL > 3 ? 148 * 16 : 148 * 6), 256, 0, stream>>>(
+  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 16, (layernorm_fwd_kernel<LPR, VPL, EXACT><<<grid_for(rows, 8 * (32 / LPR), ln_fwd_blocks(VPL)), 256, 0, stream>>>(
                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
                             static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(y), mean, rstd, rows, C,
                             eps)));
@@ -960,8 +974,7 @@ int layernorm_bwd(const void* dy, const void* x, const void* gamma, const float*
                   float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream) {
   if (C % 8 != 0 || C > 2048) return -1;
   const size_t sh = 2 * C * sizeof(float);
-  // three resident blocks per SM: every block ends in 2 C atomics on the same addresses
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (layernorm_bwd_kernel<LPR, VPL, EXACT><<<grid_for(rows, 4 * (32 / LPR), 148 * 3), 128, sh, stream>>>(
+  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (layernorm_bwd_kernel<LPR, VPL, EXACT><<<grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh, stream>>>(
                             static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
                             static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma,
                             dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C)));

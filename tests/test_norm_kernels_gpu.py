@@ -39,6 +39,12 @@ def test_layernorm(C, rows, shortcut):
     assert _rel(gw - 1, wr.grad) < REL and _rel(gb - 1, br.grad) < REL          # accumulated on top of what was there
 
 
+@pytest.mark.parametrize("C", [40, 64, 256, 512, 1536])
+def test_layernorm_of_many_rows(C):
+    """Row counts that take the larger grids of the backward kernel."""
+    test_layernorm(C, 57001, True)
+
+
 @pytest.mark.parametrize("B,HW,C,groups", [(1, 1, 96, 32), (2, 7, 384, 32), (1, 1000, 64, 32), (3, 20011, 96, 32), (1, 16385, 384, 32),
                                            (2, 333, 1024, 32), (1, 4097, 520, 5)])
 @pytest.mark.parametrize("shortcut", [False, True])

@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 // keeps several independent 16-byte loads in flight. blockIdx.y is the sample; the pixel range of a sample is split over
 // blockIdx.x so that the grid is about one resident wave. (Before, the apply kernels divided to find every vector's channel
 // and loaded its constants again, and one load per thread was in flight. 557056 pixels x 384, before -> now: statistics
-// 98 -> 96 us, apply with shortcut 355 -> 225, backward sums 366 -> 258, backward apply 406 -> 264; one copy of the image
+// 98 -> 90 us, apply with shortcut 355 -> 225, backward sums 366 -> 258, backward apply 406 -> 264; one copy of the image
 // each way at 6.65 TB/s is 129 us.)
 //
 // Statistics: per-channel partials in shared memory, folded to groups, two atomics per (block, group).
@@ -999,9 +999,10 @@ int colsum_bf16(const void* x, float* out, float* partials, long long rows, int 
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// Launch shape of the GroupNorm kernels: `threads` per block as (column vectors) x (pixels), pixels split over about
-// `waves` blocks per SM in all (at least two loop rounds of `unroll` pixels per thread, so that tiny images do not pay for
-// more blocks than they fill).
+// Launch shape of the GroupNorm kernels: `threads` per block as (column vectors) x (pixels), pixels split over at most `waves`
+// blocks per SM in all (one block beyond a resident wave would double the time: eight samples of 17280 x 384 rounded up made 448
+// blocks of 444, 106 us instead of 70 in the backward sums) and at least one loop round of `unroll` pixels per thread, so that
+// tiny images do not pay for more blocks than they fill.
 struct GnShape {
   dim3 block, grid;
   int pix;
@@ -1010,7 +1011,7 @@ struct GnShape {
     const int bx = nvec < 64 ? nvec : 64;
     const int by = threads / bx > 0 ? threads / bx : 1;
     block = dim3(bx, by);
-    const long long blocks = (148LL * waves + B - 1) / B;
+    const long long blocks = B < 148 * waves ? 148LL * waves / B : 1;
     const long long least = static_cast<long long>(by) * unroll;
     long long p = (HW + blocks - 1) / blocks;
     p = (p + least - 1) / least * least;
@@ -1026,7 +1027,11 @@ static bool gn_sizes_ok(int B, long long HW, int C, int groups) {
 
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
-  const GnShape s(B, HW, C, 512, 3, 4);
+  // Every block ends in two atomics per group on the same addresses, and its warps meet in shared memory before. While the image
+  // is L2-sized the passes over it are shorter than that, and one block per SM is enough (us, 1 / 3 blocks per SM: 64800 x 192 13 / 21,
+  // 139264 x 128 15 / 22, 139264 x 256 20 / 23, 139264 x 384 52 / 29).
+  const bool small = static_cast<long long>(B) * HW * C * 2 <= 72000000LL;
+  const GnShape s(B, HW, C, 512, small ? 1 : 3, 4);
   groupnorm_stats_kernel<<<s.grid, s.block, 2 * C * sizeof(float), stream>>>(static_cast<const __nv_bfloat16*>(x), sums, HW,
                                                                              C, groups, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -23,8 +23,8 @@
 //     shared memory allows it); the token tables are computed two windows ahead;
 //   * a window's results are staged over its own dead operand rows and leave as 16-byte vectors, warp by warp.
 //   * elementwise work on neighbouring columns goes through the two-wide fp32 instructions.
-// 2176 shifted windows of 8 x 8, 12 heads of 32 channels: forward 126 us (a version with four-warp blocks that walked over
-// heads and looked every bias up took 324 us; 64 us of HBM traffic), backward 246 us (586 us; 113 us).
+// 2176 shifted windows of 8 x 8, 12 heads of 32 channels: forward 105 us (a version with four-warp blocks that walked over
+// heads and looked every bias up took 324 us; 66 us of HBM traffic), backward 246 us (586 us; 115 us).
 #include <atomic>
 #include "common.cuh"
 #include "host_api.h"
@@ -76,14 +76,20 @@ struct WaCfg {
   static constexpr bool ACC_REGS = NPAD == 64;                   // bias-gradient sums: registers or shared memory
   static constexpr int ACC = (BWD && !ACC_REGS) ? NPAD * NPAD : 0;   // floats
   static constexpr int FIXED = (STASH + DQ) * 2 + ACC * 4 + 3 * NPAD * 8 + NPAD * 4;
-  // Two stages unless the second one would cost resident CTAs: 56 KB lets four CTAs of four warps share an SM, the
-  // backward kernel is held to three (NPAD = 64) or fewer by its registers anyway.
-  static constexpr int TWO = FIXED + 2 * STAGE * 2;
-  static constexpr int STAGES = TWO <= (BWD ? (NPAD == 64 ? 74 : 110) : (NPAD == 64 ? 57 : 100)) * 1024 ? 2 : 1;
+  // Resident CTAs that shared memory allows, with the kilobyte that every CTA reserves and a small bias table (that of an 8 x 8
+  // window makes three of four where 64 channels are staged). Two stages where three (two for windows above 64 tokens) fit.
+  static constexpr int fits(int stages) { return 228 * 1024 / (FIXED + stages * STAGE * 2 + 1024); }
+  static constexpr int STAGES = fits(2) >= (NPAD == 64 ? 3 : 2) ? 2 : 1;
   static constexpr size_t bytes(int nrel) { return static_cast<size_t>(FIXED) + STAGES * STAGE * 2 + HPC * nrel * 4; }
-  // resident CTAs per SM asked of the compiler: bounds the registers per thread
-  static constexpr int MIN_CTAS = NPAD > 96 ? 1 : (BWD ? (NPAD > 64 ? (HD > 64 ? 1 : 2) : (HD > 64 ? 2 : 3))
-                                                       : (NPAD > 64 ? 2 : (HD > 64 ? 4 : 5)));
+  // Resident CTAs asked of the compiler, which bounds the registers per thread: no more than shared memory allows. (Asked for
+  // five where two stages of 64 channels let four or three fit, the compiler spilled for nothing: 2176 windows of 8 x 8, 12 heads
+  // of 32 channels, forward without / with shift 116 / 125 us, for four 96 / 105. For three it would be 94 / 103, but then
+  // 4 x 4 windows lose the fourth: 6 heads of 64 channels 67 / 71 us, for four 65 / 70, for three 75 / 80. One stage and five
+  // CTAs: 100 / 109.)
+  static constexpr int WANTED = NPAD > 96 ? 1 : (BWD ? (NPAD > 64 ? (HD > 64 ? 1 : 2) : (HD > 64 ? 2 : 3))
+                                                     : (NPAD > 64 ? 2 : (HD > 64 ? 4 : 5)));
+  // (128-token windows of 128-channel heads do not fit backward at all: their launch is refused)
+  static constexpr int MIN_CTAS = fits(STAGES) < 1 ? 1 : (WANTED < fits(STAGES) ? WANTED : fits(STAGES));
 };
 
 struct WaItem {

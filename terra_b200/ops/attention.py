@@ -159,7 +159,7 @@ def window_attention_reference(qkv_all: torch.Tensor, geo: WindowGeometry, num_h
 def attn_forward_impl(N: int) -> str:
     """Which forward kernel runs: ``tc`` (tcgen05 / TMEM, any window size) or ``mma`` (warp-level mma.sync, windows of
     at most 128 tokens, several CTAs per SM). Windows above 128 tokens always take ``tc``; below, ``mma`` is the default
-    because it measures faster there (0.13 against 0.49 ms on the 2176-window stage with head dim 32): one softmax warp
+    because it measures faster there (0.10 against 0.49 ms on the 2176-window stage with head dim 32): one softmax warp
     per scheduler leaves the tensor-core kernel latency bound on 64-token windows. ``TERRA_ATTN_FWD=tc`` selects it
     anyway."""
     import os

@@ -408,9 +408,9 @@ __device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
 }
 __device__ __forceinline__ f32x2 f2_both(float v) { return f2_pack(v, v); }
 
-// GELU and its derivative on two elements: the expressions of gelu_erf / gelu_erf_grad operation by operation, 5 and 9
-// issue slots per element instead of 9 and 14. The value needs no clamp of x itself: beyond the fit's range the clamped
-// polynomial times x keeps the sign of x and grows, and tanh has saturated.
+// GELU and its derivative on two elements: the expressions of gelu_erf / gelu_erf_grad, 5 and 9 issue slots per element
+// instead of 9 and 14. The derivative is operation by operation the same; the value clamps x * x to 64 instead of x to 8: beyond
+// the fit's range the clamped polynomial times x keeps the sign of x and grows, and tanh has saturated.
 __device__ __forceinline__ f32x2 gelu_erf2(f32x2 x) {
 #ifdef TERRA_GELU_EXACT_ERF
   float a, b;

@@ -820,8 +820,8 @@ __global__ void conv_s2_col2im_kernel(const uint4* __restrict__ dcol, void* __re
 // contiguous copies, bound by HBM; V (16, 8, 4 or 2 bytes) divides the byte length of a patch row, of an image row and of
 // the left padding, so that no vector crosses the edge of the image. `row_units` = vectors of a padded row,
 // `seg_units` = vectors of a patch row. Thread block: one padded row (blockIdx.y) and PATCH_UNROLL vectors per thread.
-// 720 x 1440 x 138 padded to 768 rows: 87 us in (89 us at 6.65 TB/s), 126 us out with the addition (132 us); the tensor
-// operators took 1100 us for both.
+// 720 x 1440 x 138 padded to 768 rows, L2 flushed before: 94 us in (591 MB, 90 us at 6.54 TB/s), 132 us out with the addition
+// (858 MB, 131 us; the padding is not read); the tensor operators took 1100 us for both.
 constexpr int PATCH_UNROLL = 4;
 template <class V>
 __global__ void __launch_bounds__(256) pad_patchify_kernel(const V* __restrict__ x, V* __restrict__ patches, int H, int p, int hn,

@@ -7,9 +7,9 @@
 //            128-byte-swizzled shared-memory stages, signalling `full[s]` by transaction bytes;
 //   warp 1   owns the TMEM allocation; one elected lane issues tcgen05.mma (M=128, N=BN, K=16)
 //            and commits to `empty[s]` (stage reusable) and `tfull[a]` (accumulator a complete);
-//   warps 2-13 epilogue (three per 32-lane TMEM quadrant, interleaved over the column chunks): tcgen05.ld, fused
-//            bias / GELU / residual / GELU-gradient / pixel-shuffle / split-K atomics; global transfers coalesced
-//            through shared memory.
+//   warps 2-13 epilogue (three per 32-lane TMEM quadrant, interleaved over the columns): tcgen05.ld, fused bias / GELU /
+//            residual / GELU-gradient; bf16 outputs leave as units of 32 rows (or pixels) x 64 columns through TMA stores,
+//            fp32 split-K atomics and what does not fit a tensor map as 32-column chunks through an exchange buffer.
 // Two accumulators (2*BN TMEM columns) let the epilogue of tile i overlap the main loop of tile i+1.
 //
 // Operand addressing is data driven (see gemm_sm100.cuh) so that the same kernel serves
@@ -41,8 +41,8 @@ constexpr int GEMM_B_WARP = 2 + GEMM_EPI_WARPS;
 constexpr int GEMM_THREADS = 32 * (GEMM_B_WARP + 1);
 
 // CTAS = 2: a cluster of two CTAs (two SMs of one TPC) computes a 256 x BN tile with one pair-wide MMA. Each CTA stages
-// its own 128 rows of A and its own half of B, so a k-block costs each SM (16 + BN / 8) KB of shared-memory fill instead
-// of (16 + BN / 4) KB: the operand traffic per flop through shared memory, which bounds the single-CTA main loop, drops
+// its own 128 rows of A and its own half of B, so a k-block costs each SM (16 + BN / 16) KB of shared-memory fill instead
+// of (16 + BN / 8) KB: the operand traffic per flop through shared memory, which bounds the single-CTA main loop, drops
 // by a third at BN = 256.
 //
 // STACK = 2 (weight gradients, one CTA): two 128-row blocks of A share a tile of B, 256 x BN outputs in both accumulators.
@@ -444,13 +444,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..13)
     // tcgen05.ld hands lane l the 32 columns of accumulator row l. Global memory wants the opposite: neighbouring
-    // lanes on neighbouring addresses. Every transfer of a 32 x 32 chunk (output, saved pre-activation, residual,
-    // GELU input) therefore goes through the warp's 2 KB exchange buffer: row-per-lane on one side, four lanes per
+    // lanes on neighbouring addresses. The TMA form (first branch below) stages units for bulk stores. In the other form
+    // (fp32 output, peers, stacked tiles, matrices or operand mixes without a tensor map, TERRA_GEMM_TMA_EPILOGUE=0) every
+    // transfer of a 32 x 32 chunk goes through the warp's 2 KB exchange buffer: row-per-lane on one side, four lanes per
     // row (eight rows, 64 contiguous bytes each, per instruction) on the global side. 16-byte vectors are XOR
     // swizzled by (row >> 1); the profiler still counts about two wavefronts per ideal one on the row-gathering
     // side (a padded 80-byte pitch measured worse), which costs a few percent of the short-K GEMMs.
     const int q = warp & 3;               // TMEM lane quadrant this warp may read
-    const int part = (warp - 2) >> 2;     // chunks part, part + 4, ... of the tile's 32-column chunks
+    const int part = (warp - 2) >> 2;     // chunks (units) part, part + 3, ... of the tile's columns
     constexpr int CHUNKS = BN / 32;
     float* my_bias = bias_slots + (warp - 2) * 32;
     uint8_t* my_x = xchg + (warp - 2) * 2048;

@@ -23,7 +23,6 @@ enum : int {
   EPI_ATOMIC = 1 << 6,     // fp32 atomic accumulate into C (split-K)
   EPI_ROW_CONV = 1 << 7,   // rows are (w-chunk, h, b) tiles of an image of width out_w
   EPI_BIAS_F32 = 1 << 9,   // bias pointer is fp32
-  EPI_SILU_MUL = 1 << 10,  // reserved
 };
 
 struct GemmEpilogue {

@@ -149,6 +149,8 @@ class _AttnHalfFn(torch.autograd.Function):
             gemm(dy, pk.proj_w, b_mn=True, out=do)
             dqkv, qkv_ptrs, dout_ptrs, dqkv_ptrs = comm.attn_backward_buffers(qkv, do, shifted)
         else:
+            if not qkv.is_contiguous():      # (saved-tensor hooks may hand it back in another form)
+                raise RuntimeError("attention half: qkv must be contiguous [rows, 3 C]")
             do = gemm(dy, pk.proj_w, b_mn=True)
             dqkv = torch.empty_like(qkv)
             qkv_ptrs, dout_ptrs, dqkv_ptrs = [qkv.data_ptr()], [do.data_ptr()], [dqkv.data_ptr()]

@@ -155,7 +155,8 @@ def test_native_halves_refuse_other_operands():
 
 
 @pytest.mark.parametrize("half", ["attention", "mlp"])
-def test_saved_tensors_of_another_form(half):
+@pytest.mark.parametrize("native", [True, False])
+def test_saved_tensors_of_another_form(monkeypatch, half, native):
     """Hooks may hand the saved tensors back with another row pitch: products take that, what is read as dense rows is
     refused."""
     from terra_b200.models.layers import SwinAttentionHalf
@@ -163,6 +164,7 @@ def test_saved_tensors_of_another_form(half):
     from terra_b200.ops.attention import WindowGeometry
     from terra_b200.utils.flat_params import ParamArena
 
+    monkeypatch.setattr(blocks, "_LAUNCHES_OBSERVED", not native)
     if half == "attention":
         torch.manual_seed(2)
         geo = WindowGeometry(1, 2, 2, 8, 8)

@@ -192,6 +192,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* m, uin
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
       : "memory");
 }
+// a box of global memory into L2 only
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1)
+               : "memory");
+}
 __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1,
                                             int c2, int c3, int c4) {
   asm volatile(
@@ -408,8 +413,22 @@ __device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
 }
 __device__ __forceinline__ f32x2 f2_both(float v) { return f2_pack(v, v); }
 
-// GELU and its derivative on two elements: the expressions of gelu_erf / gelu_erf_grad, 5 and 9 issue slots per element
-// instead of 9 and 14. The derivative is operation by operation the same; the value clamps x * x to 64 instead of x to 8: beyond
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+__device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
+  __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
+  return __bfloat1622float2(v);
+}
+__device__ __forceinline__ uint32_t f2_to_bf16x2(f32x2 v) {
+  float lo, hi;
+  f2_unpack(v, lo, hi);
+  return pack_bf16x2(lo, hi);
+}
+
+// GELU and its derivative on two elements: the expressions of gelu_erf / gelu_erf_grad, 5 and 8 issue slots per element
+// instead of 9 and 14. The value clamps x * x to 64 instead of x to 8: beyond
 // the fit's range the clamped polynomial times x keeps the sign of x and grows, and tanh has saturated.
 __device__ __forceinline__ f32x2 gelu_erf2(f32x2 x) {
 #ifdef TERRA_GELU_EXACT_ERF
@@ -426,28 +445,25 @@ __device__ __forceinline__ f32x2 gelu_erf2(f32x2 x) {
   return f2_fma(h, f2_pack(tanh_fast(a), tanh_fast(b)), h);
 #endif
 }
-__device__ __forceinline__ f32x2 gelu_erf_grad2(f32x2 x) {
-  float a, b;
-  f2_unpack(x, a, b);
+// The derivative at two bf16 values (the saved pre-activation): the clamp is taken on the pair, and the factors -1 and 0.5 of
+// the scalar expression are folded into constants, which changes no rounding.
+__device__ __forceinline__ f32x2 gelu_erf_grad2_bf16(uint32_t x) {
 #ifdef TERRA_GELU_EXACT_ERF
-  return f2_pack(gelu_erf_grad(a), gelu_erf_grad(b));
+  const float2 v = unpack_bf16x2(x);
+  return f2_pack(gelu_erf_grad(v.x), gelu_erf_grad(v.y));
 #else
-  const f32x2 xc = f2_pack(fminf(fmaxf(a, -8.0f), 8.0f), fminf(fmaxf(b, -8.0f), 8.0f));
+  uint32_t c;
+  asm("{\n.reg .b32 t;\nmax.bf16x2 t, %1, %2;\nmin.bf16x2 %0, t, %3;\n}" : "=r"(c) : "r"(x), "r"(0xC100C100u), "r"(0x41004100u));   // -8, 8
+  const float2 v = unpack_bf16x2(c);
+  const f32x2 xc = f2_pack(v.x, v.y);
   const f32x2 x2 = f2_mul(xc, xc);
+  float a, b;
   f2_unpack(f2_mul(xc, f2_fma(x2, f2_fma(x2, f2_both(GELU_C2), f2_both(GELU_C1)), f2_both(GELU_C0))), a, b);
   const f32x2 t = f2_pack(tanh_fast(a), tanh_fast(b));
-  const f32x2 du = f2_fma(x2, f2_fma(x2, f2_both(5.0f * GELU_C2), f2_both(3.0f * GELU_C1)), f2_both(GELU_C0));
-  const f32x2 sech2 = f2_fma(f2_mul(t, f2_both(-1.0f)), t, f2_both(1.0f));
-  return f2_fma(f2_mul(f2_mul(f2_both(0.5f), xc), sech2), du, f2_fma(f2_both(0.5f), t, f2_both(0.5f)));
+  const f32x2 du = f2_fma(x2, f2_fma(x2, f2_both(-2.5f * GELU_C2), f2_both(-1.5f * GELU_C1)), f2_both(-0.5f * GELU_C0));   // -u'(x) / 2
+  const f32x2 sech2 = f2_fma(t, t, f2_both(-1.0f));                                                                  // tanh^2 - 1
+  return f2_fma(f2_mul(xc, sech2), du, f2_fma(f2_both(0.5f), t, f2_both(0.5f)));
 #endif
-}
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-__device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
-  __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
-  return __bfloat1622float2(v);
 }
 
 }  // namespace tb

@@ -97,9 +97,6 @@ static void try_tma_epilogue(GemmParams& p, long long M, long long N) {
   const int f = p.epi;
   if (!gemm_tma_epilogue() || (f & (EPI_OUT_F32 | EPI_ATOMIC | EPI_ROW_CONV))) return;
   if (((f & EPI_RESIDUAL) != 0) + ((f & EPI_MUL_DGELU) != 0) + ((f & EPI_SAVE_PRE) != 0) > 1) return;   // one second buffer
-  // The input buffers cost the operand ring one or two stages. A long contraction hides the epilogue behind its main
-  // loop anyway and wants the deeper ring instead (K = 1536 with a residual measured 15 % slower on three stages).
-  if ((f & (EPI_RESIDUAL | EPI_MUL_DGELU)) && p.k_blocks > 12) return;
   if (p.a_peers > 1 || p.c_peers > 1 || p.groups != 1 || p.C == nullptr) return;
   if (map_chunk(&p.map_c, p.C, N, M, p.ldc) != 0) return;
   if ((f & EPI_SAVE_PRE) && map_chunk(&p.map_c2, p.C2, N, M, p.ldc2) != 0) return;

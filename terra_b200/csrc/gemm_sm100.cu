@@ -27,6 +27,7 @@
 //
 // Every wait is bounded; on expiry the CTA sets its abort flag, records the site in the
 // KernelStatus word, drains, releases TMEM and returns.
+#include <type_traits>
 #include "gemm_sm100.cuh"
 
 namespace tb {
@@ -57,12 +58,12 @@ struct GemmCfg {
   static constexpr int B_ROWS = BN / CTAS;                 // rows of B staged by one CTA
   static constexpr int B_BYTES = B_ROWS * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  // After the operand ring: 512 bytes of barriers, the per-warp bias slots (together 2 KB), then `bufs` buffers of
+  // After the operand ring: 512 bytes of barriers, the per-warp bias slots (together 4 KB), then `bufs` buffers of
   // 2 KB per epilogue warp: one (the exchange buffer of the per-lane epilogue), or two (a 32 x 64 unit of the output on its
   // way to a TMA store), or four (another such unit: the saved pre-activation, or the operand the epilogue reads). The
   // ring takes what is left: the launcher passes the stage count to the kernel.
   static constexpr int BAR_BYTES = 512;
-  static constexpr int FIXED_BASE = 2048;
+  static constexpr int FIXED_BASE = 4096;
   static constexpr int EPI_BUF = 2048;
   static constexpr int MAX_SMEM = 232448;   // 227 KB, the per-block limit of sm_100
   static constexpr int MAX_STAGES = 8;
@@ -78,7 +79,7 @@ struct GemmCfg {
   static constexpr int TMEM_COLS = (2 * BN + 64 <= 256) ? 256 : 512;
   static constexpr bool CAN_COLSUM = CTAS == 1 && 2 * BN + 64 <= 512;
   static_assert((STACK == 2 ? stages_for(1) : stages_for(2)) >= 3 && smem_bytes(1) <= MAX_SMEM && smem_bytes(2) <= MAX_SMEM, "shared memory budget");
-  static_assert(GEMM_EPI_WARPS * 32 * 4 + BAR_BYTES <= FIXED_BASE, "bias slots");
+  static_assert(GEMM_EPI_WARPS * 64 * 4 + BAR_BYTES <= FIXED_BASE, "bias slots");
   // a CTA's half of an MN-major B must be whole 64-row boxes; K-major rows only need whole 8-row swizzle atoms
   static constexpr bool CAN_B_MN = B_ROWS % 64 == 0;
   static_assert(B_ROWS % 8 == 0 && B_BYTES % 1024 == 0, "B tile: whole swizzle atoms");
@@ -157,10 +158,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   uint64_t* tfull = empty + Cfg::MAX_STAGES;
   uint64_t* tempty = tfull + 2;
   uint64_t* pfull = tempty + 2;   // pair mode, leader CTA: "the peer's half of stage s has landed"
-  uint64_t* in_bar = pfull + Cfg::MAX_STAGES;   // one per epilogue warp: "the epilogue operand's unit has landed"
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(in_bar + GEMM_EPI_WARPS);
+  uint64_t* in_bar = pfull + Cfg::MAX_STAGES;   // two per epilogue warp: "the epilogue operand's unit has landed"
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(in_bar + 2 * GEMM_EPI_WARPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((3 * Cfg::MAX_STAGES + 4 + GEMM_EPI_WARPS) * 8 + 8 <= Cfg::BAR_BYTES, "barrier block");
+  static_assert((3 * Cfg::MAX_STAGES + 4 + 2 * GEMM_EPI_WARPS) * 8 + 8 <= Cfg::BAR_BYTES, "barrier block");
   float* bias_slots = reinterpret_cast<float*>(fixed + Cfg::BAR_BYTES);
   uint8_t* xchg = fixed + Cfg::FIXED_BASE;
   // The ring needs a 1024-byte aligned base (128-byte swizzle atoms). The dynamic window normally starts aligned; if
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       mbar_init(&empty[s], 1);
       mbar_init(&pfull[s], 1);
     }
-    for (int i = 0; i < GEMM_EPI_WARPS; ++i) mbar_init(&in_bar[i], 1);
+    for (int i = 0; i < 2 * GEMM_EPI_WARPS; ++i) mbar_init(&in_bar[i], 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
       mbar_init(&tempty[a], GEMM_EPI_WARPS * CTAS);   // pair mode: both CTAs' epilogue warps release the leader's
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
     const int q = warp & 3;               // TMEM lane quadrant this warp may read
     const int part = (warp - 2) >> 2;     // chunks (units) part, part + 3, ... of the tile's columns
     constexpr int CHUNKS = BN / 32;
-    float* my_bias = bias_slots + (warp - 2) * 32;
+    float* my_bias = bias_slots + (warp - 2) * 64;
     uint8_t* my_x = xchg + (warp - 2) * 2048;
     const bool has_bias = (p.epi & EPI_BIAS) != 0;
     const int grow = lane >> 2, gvec = lane & 3;      // global side: rows grow + 8 i, vector gvec
@@ -467,182 +468,224 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
     if (!PEERS && STACK == 1 && p.epi_tma) {
       // ---- bf16 outputs through TMA, and the operand the epilogue reads. A warp works on units of 32 rows x 64 columns (128
       // bytes per row in the 128-byte-swizzled layout, conflict-free for the row-per-lane 16-byte accesses). Tiles of 192
-      // columns are one unit per warp and tile, so a buffer has a whole tile's time to drain or fill. Against 32-column
-      // chunks (three uneven rounds at width 256, two at 192): 278528 x 2976 x 384 with residual 1061 -> 848 us, 139264 x
-      // 1536 x 384 times GELU' 352 -> 290, 139264 x 384 x 384 with residual 72 -> 66, 17280 x 768 x 192 with GELU 30 -> 24.
-      // The warp's first 4 KB stage the output; one lane issues the store and, before the buffer is written again, waits
-      // until the store has read it. The second 4 KB stage the saved pre-activation, or receive the input unit, loaded as
-      // soon as the unit before has been read (across tiles), so its latency hides behind the main loop.
+      // columns are one unit per warp and tile.
+      //
+      // What bounds a unit is latency, three warps per scheduler being all there is to hide it. So the form of the epilogue is a
+      // compile-time constant (with the flags tested inside, every pair of elements became a basic block of its own), a unit's
+      // two tensor-memory loads are issued together, the bias of a unit is fetched while the accumulator is waited for and spread
+      // through shared memory once, and the input unit arrives in the buffer its output is staged in: a lane reads and writes
+      // the same 16 bytes. With two such buffers the next unit's load has this unit's processing time to arrive (and the one
+      // after it is already on its way from HBM to L2); with one (long contractions, which want the ring and hide the epilogue)
+      // it is issued when the store has read the buffer.
+      // The first buffer (4 KB) stages the output; the second takes the saved pre-activation, or alternates with the first.
+      // Cycles per unit with the flags tested inside / this: bias 2400, bias and residual 3400 + 800 waiting for the input, GELU
+      // with the pre-activation 4500, times GELU' 6100 + 800. 139264 x 1536 x 384 times GELU' 334 -> 261 us, the same with GELU 260
+      // -> 243, 139264 x 384 x 384 63 -> 54, 156672 x 1024 x 1024 with residual 316 -> 279, 17280 x 576 x 192 12.4 -> 10.0.
       constexpr int UNITS = BN / 64, WARPS_PER_Q = GEMM_EPI_WARPS / 4;
-      const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
       uint8_t* my_out = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
-      uint8_t* my_second = my_out + 2 * Cfg::EPI_BUF;
-      uint64_t* my_in = in_bar + (warp - 2);
-      const uint32_t row_off = static_cast<uint32_t>(lane) * 128u;
-      const uint32_t swz = static_cast<uint32_t>(lane) & 7u;
-      uint32_t consumed = 0;
-      int pf_tile = unit, pf_u = part, pf_n0 = 0, pf_row = 0;
-      auto prefetch_next = [&]() {   // issue the load of this warp's next input unit, if there is one
-        while (pf_tile < total_tiles) {
-          if (pf_u == part) {        // the divisions once per tile
-            const TileCoord t = decode_tile(p, pf_tile, CTAS, rank);
-            pf_n0 = t.n_blk * BN;
-            pf_row = t.m_blk * GEMM_BM + q * 32;
-          }
-          const int col = pf_n0 + pf_u * 64, row = pf_row;
-          const bool ok = pf_u < UNITS && col < p.N;
-          pf_u += WARPS_PER_Q;
-          if (pf_u >= UNITS) {
-            pf_u = part;
-            pf_tile += units;
-          }
-          if (ok) {
-            if (lane == 0) {
-              mbar_expect_tx(my_in, 2 * Cfg::EPI_BUF);
-              tma_load_2d(my_second, &p.map_in, my_in, col, row);
-            }
-            return;
-          }
-        }
+      uint64_t* my_in = in_bar + 2 * (warp - 2);
+      const uint32_t out_base = smem_u32(my_out) + static_cast<uint32_t>(lane) * 128u;
+      const uint32_t swz = (static_cast<uint32_t>(lane) & 7u) << 4;
+      const uint32_t bias_base = smem_u32(my_bias);
+      // coordinates of this warp's units, in the order it works on them
+      struct Walk {
+        int tile, u, n0, row;
       };
-      auto stage_half = [&](uint8_t* buf, const float (&f)[32], int h) {
-        const uint32_t base = smem_u32(buf) + row_off;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t a = base + (((static_cast<uint32_t>(4 * h + j)) ^ swz) << 4);
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(pack_bf16x2(f[8 * j], f[8 * j + 1])),
-                       "r"(pack_bf16x2(f[8 * j + 2], f[8 * j + 3])), "r"(pack_bf16x2(f[8 * j + 4], f[8 * j + 5])),
-                       "r"(pack_bf16x2(f[8 * j + 6], f[8 * j + 7]))
-                       : "memory");
-        }
-      };
-      if (has_in) prefetch_next();
-      bool failed = false;
-      for (int tile = unit; tile < total_tiles && !failed; tile += units, ++tcount) {
-        const TileCoord tc = decode_tile(p, tile, CTAS, rank);
-        const int acc = tcount & 1;
-        const uint32_t aph = (tcount >> 1) & 1u;
-        const int n0 = tc.n_blk * BN;
-        const long long ew0 = clock64();
-        const bool tile_ready = mbar_wait<PAIR>(&tfull[acc], aph, abort_flag, p.status, 0x400u + acc, mbar_budget);
-        if (!__all_sync(0xffffffffu, tile_ready)) break;
-        e_wait += clock64() - ew0;
-        tc_fence_after();
-        bool released = false;
-        auto release = [&]() {   // the accumulator has been read: the MMA thread may start the tile after next
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (PAIR && rank == 1) mbar_arrive_remote(map_to_cta(&tempty[acc], 0));   // the leader's MMA thread waits
-            else mbar_arrive(&tempty[acc]);
+      auto walk_next = [&](Walk& w, int& col, int& row) -> bool {
+        if (part >= UNITS) return false;
+        while (w.tile < total_tiles) {
+          if (w.u == part) {        // the divisions once per tile
+            const TileCoord t = decode_tile(p, w.tile, CTAS, rank);
+            w.n0 = t.n_blk * BN;
+            w.row = t.m_blk * GEMM_BM + q * 32;
           }
-          released = true;
+          col = w.n0 + w.u * 64;
+          row = w.row;
+          const bool ok = w.u < UNITS && col < p.N;
+          w.u += WARPS_PER_Q;
+          if (w.u >= UNITS) {
+            w.u = part;
+            w.tile += units;
+          }
+          if (ok) return true;
+        }
+        return false;
+      };
+
+      auto run = [&](auto form_const) {
+        constexpr int FORM = decltype(form_const)::value;      // EPI_* flags of the form, or -1: tested at run time
+        const int flags = FORM >= 0 ? FORM : p.epi;
+        const bool with_bias = (flags & EPI_BIAS) != 0, gelu = (flags & EPI_GELU) != 0, save_pre = (flags & EPI_SAVE_PRE) != 0;
+        const bool has_in = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0, dgelu = (flags & EPI_MUL_DGELU) != 0;
+        const f32x2 alpha2 = f2_both(p.alpha);
+        const int in_bufs = p.epi_bufs / 2;
+        Walk load = {unit, part, 0, 0}, ahead = load;
+        auto fetch_in = [&](int buf) {       // this warp's next input unit into `buf`; the unit after it into L2
+          int col, row;
+          if (walk_next(load, col, row) && lane == 0) {
+            mbar_expect_tx(my_in + buf, 2 * Cfg::EPI_BUF);
+            tma_load_2d(my_out + buf * 2 * Cfg::EPI_BUF, &p.map_in, my_in + buf, col, row);
+          }
+          if (walk_next(ahead, col, row) && lane == 0) tma_prefetch_l2_2d(&p.map_in, col, row);
         };
-#pragma unroll 1
-        for (int u = part; u < UNITS && n0 + u * 64 < p.N; u += WARPS_PER_Q) {   // warp-uniform
-          const int nb0 = n0 + u * 64;
-          const bool last = u + WARPS_PER_Q >= UNITS || nb0 + 64 * WARPS_PER_Q >= p.N;
-          if (lane == 0) bulk_wait_group_read<0>();
-          __syncwarp();
-          if (has_in) {
-            const bool in_ready = mbar_wait<false>(my_in, consumed & 1u, abort_flag, p.status, 0x600u, mbar_budget);
-            if (!__all_sync(0xffffffffu, in_ready)) {
-              failed = true;
-              break;
-            }
-            ++consumed;
-          }
-          // (one copy of the half's code stays in the instruction cache of the twelve warps)
-#pragma unroll 1
-          for (int h = 0; h < 2; ++h) {
-            const int nb = nb0 + 32 * h;
-            if (nb >= p.N) break;   // warp-uniform
-            if (has_bias) {
-              float b = 0.f;
-              if (nb + lane < p.N)
-                b = (p.epi & EPI_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + nb + lane)
-                                           : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[nb + lane]);
-              __syncwarp();
-              my_bias[lane] = b;
-              __syncwarp();
-            }
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + acc * BN + u * 64 + h * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
-            uint4 in[4];
-            if (has_in) {
-              const uint32_t base = smem_u32(my_second) + row_off;
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint32_t a = base + (((static_cast<uint32_t>(4 * h + j)) ^ swz) << 4);
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(in[j].x), "=r"(in[j].y), "=r"(in[j].z), "=r"(in[j].w)
-                             : "r"(a)
-                             : "memory");
-              }
-            }
-            tmem_ld_wait();
-            if (last && (h == 1 || nb + 32 >= p.N)) release();
-            float f[32];
-            const f32x2 alpha2 = f2_pack(p.alpha, p.alpha);
-            if (has_bias) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                const float4 b4 = *reinterpret_cast<const float4*>(my_bias + j);
-                f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2, f2_pack(b4.x, b4.y)), f[j],
-                          f[j + 1]);
-                f2_unpack(f2_fma(f2_pack(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), alpha2, f2_pack(b4.z, b4.w)),
-                          f[j + 2], f[j + 3]);
-              }
+        if (has_in) {
+          int col, row;
+          walk_next(ahead, col, row);        // `ahead` runs one unit in front of `load`
+          fetch_in(0);
+        }
+        uint32_t count = 0;                  // units of this warp so far
+        bool failed = false;
+        for (int tile = unit; tile < total_tiles && !failed; tile += units, ++tcount) {
+          const TileCoord tc = decode_tile(p, tile, CTAS, rank);
+          const int acc = tcount & 1;
+          const uint32_t aph = (tcount >> 1) & 1u;
+          const int n0 = tc.n_blk * BN;
+          auto bias_pair = [&](int col) -> float2 {     // columns col, col + 1 (col even)
+            float2 b = make_float2(0.f, 0.f);
+            if (p.epi & EPI_BIAS_F32) {
+              if (col < p.N) b.x = __ldg(static_cast<const float*>(p.bias) + col);
+              if (col + 1 < p.N) b.y = __ldg(static_cast<const float*>(p.bias) + col + 1);
             } else {
-#pragma unroll
-              for (int j = 0; j < 32; j += 2)
-                f2_unpack(f2_mul(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), alpha2), f[j], f[j + 1]);
+              if (col < p.N) b.x = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
+              if (col + 1 < p.N) b.y = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col + 1]);
             }
-            if (p.epi & EPI_SAVE_PRE) stage_half(my_second, f, h);
-            if (p.epi & EPI_GELU) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 2) f2_unpack(gelu_erf2(f2_pack(f[j], f[j + 1])), f[j], f[j + 1]);
+            return b;
+          };
+          float2 bias_here = make_float2(0.f, 0.f);
+          if (with_bias && part < UNITS) bias_here = bias_pair(n0 + part * 64 + 2 * lane);
+          const long long ew0 = clock64();
+          const bool tile_ready = mbar_wait<PAIR>(&tfull[acc], aph, abort_flag, p.status, 0x400u + acc, mbar_budget);
+          if (!__all_sync(0xffffffffu, tile_ready)) break;
+          e_wait += clock64() - ew0;
+          tc_fence_after();
+          bool released = false;
+          auto release = [&]() {   // the accumulator has been read: the MMA thread may start the tile after next
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if (PAIR && rank == 1) mbar_arrive_remote(map_to_cta(&tempty[acc], 0));   // the leader's MMA thread waits
+              else mbar_arrive(&tempty[acc]);
+            }
+            released = true;
+          };
+#pragma unroll 1
+          for (int u = part; u < UNITS && n0 + u * 64 < p.N; u += WARPS_PER_Q) {   // warp-uniform
+            const int nb0 = n0 + u * 64;
+            const bool last = u + WARPS_PER_Q >= UNITS || nb0 + 64 * WARPS_PER_Q >= p.N;
+            const int buf = has_in && in_bufs == 2 ? static_cast<int>(count & 1u) : 0;
+            uint32_t v[2][32];
+            const uint32_t tcol = tmem_base + acc * BN + u * 64 + (static_cast<uint32_t>(q * 32) << 16);
+            tmem_ld_32x32(tcol, v[0]);
+            tmem_ld_32x32(tcol + 32, v[1]);
+            if (with_bias) {
+              __syncwarp();
+              asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(bias_base + lane * 8), "f"(bias_here.x), "f"(bias_here.y) : "memory");
+              if (!last) bias_here = bias_pair(nb0 + 64 * WARPS_PER_Q + 2 * lane);
             }
             if (has_in) {
-              const bool dgelu = (p.epi & EPI_MUL_DGELU) != 0;
+              const bool in_ready = mbar_wait<false>(my_in + buf, (in_bufs == 2 ? count >> 1 : count) & 1u, abort_flag, p.status, 0x600u,
+                                                     mbar_budget);
+              if (!__all_sync(0xffffffffu, in_ready)) {
+                tmem_ld_wait();
+                failed = true;
+                break;
+              }
+            }
+            ++count;
+            tmem_ld_wait();
+            if (last) release();
+            if (lane == 0) bulk_wait_group_read<0>();     // the unit before has left its buffer
+            __syncwarp();
+            if (has_in && in_bufs == 2) fetch_in(buf ^ 1);
+            const uint32_t row_out = out_base + buf * 2 * Cfg::EPI_BUF;
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint32_t w4[4] = {in[j].x, in[j].y, in[j].z, in[j].w};
+            for (int g = 0; g < 8; ++g) {      // 8 columns: 16 bytes of the output row
+              const uint32_t at = (static_cast<uint32_t>(g) << 4) ^ swz;
+              f32x2 f[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                f[k] = f2_pack(__uint_as_float(v[g >> 2][(g & 3) * 8 + 2 * k]), __uint_as_float(v[g >> 2][(g & 3) * 8 + 2 * k + 1]));
+              if (with_bias) {
+#pragma unroll
+                for (int k = 0; k < 4; k += 2) {
+                  float b0, b1, b2, b3;
+                  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                               : "=f"(b0), "=f"(b1), "=f"(b2), "=f"(b3)
+                               : "r"(bias_base + g * 32 + k * 8));
+                  f[k] = FORM >= 0 ? f2_add(f[k], f2_pack(b0, b1)) : f2_fma(f[k], alpha2, f2_pack(b0, b1));
+                  f[k + 1] = FORM >= 0 ? f2_add(f[k + 1], f2_pack(b2, b3)) : f2_fma(f[k + 1], alpha2, f2_pack(b2, b3));
+                }
+              } else if (FORM < 0) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) f[k] = f2_mul(f[k], alpha2);
+              }
+              if (save_pre)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_out + 2 * Cfg::EPI_BUF + at), "r"(f2_to_bf16x2(f[0])),
+                             "r"(f2_to_bf16x2(f[1])), "r"(f2_to_bf16x2(f[2])), "r"(f2_to_bf16x2(f[3]))
+                             : "memory");
+              if (gelu) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) f[k] = gelu_erf2(f[k]);
+              }
+              if (has_in) {
+                uint32_t in[4];
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(in[0]), "=r"(in[1]), "=r"(in[2]), "=r"(in[3])
+                             : "r"(row_out + at)
+                             : "memory");
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                  const float2 x = unpack_bf16x2(w4[k]);
-                  const f32x2 f2 = f2_pack(f[8 * j + 2 * k], f[8 * j + 2 * k + 1]), x2 = f2_pack(x.x, x.y);
-                  f2_unpack(dgelu ? f2_mul(f2, gelu_erf_grad2(x2)) : f2_add(f2, x2), f[8 * j + 2 * k], f[8 * j + 2 * k + 1]);
+                  if (dgelu) {
+                    f[k] = f2_mul(f[k], gelu_erf_grad2_bf16(in[k]));
+                  } else {
+                    const float2 x = unpack_bf16x2(in[k]);
+                    f[k] = f2_add(f[k], f2_pack(x.x, x.y));
+                  }
                 }
               }
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_out + at), "r"(f2_to_bf16x2(f[0])), "r"(f2_to_bf16x2(f[1])),
+                           "r"(f2_to_bf16x2(f[2])), "r"(f2_to_bf16x2(f[3]))
+                           : "memory");
             }
-            stage_half(my_out, f, h);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();          // the unit is staged, and every lane holds its part of the input: its buffer may be refilled
-          if (lane == 0) {
-            if (p.epi_tma == 2) {
-              // 32 consecutive pixels of an image row (decoded by this one lane)
-              const int phase = p.phase_cols > 0 ? nb0 / p.phase_cols : tc.grp;
-              const int w = (tc.m_blk % p.tile_n0) * GEMM_BM + q * 32;
-              const int h = (tc.m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0];
-              if (tc.m_blk < p.m_blocks && w < p.out_w && h < p.out_h)
-                tma_store_5d(&p.map_c, smem_u32(my_out), p.phase_cols > 0 ? nb0 - phase * p.phase_cols : nb0, p.out_off[phase][1], w,
-                             h, tc.m_blk / (p.tile_n0 * p.tile_n1));
-            } else {
-              const int row0 = tc.m_blk * GEMM_BM + q * 32;
-              if (row0 < p.M) {
-                if (p.epi & EPI_SAVE_PRE) tma_store_2d(&p.map_c2, smem_u32(my_second), nb0, row0);
-                tma_store_2d(&p.map_c, smem_u32(my_out), nb0, row0);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              const uint32_t src = smem_u32(my_out) + buf * 2 * Cfg::EPI_BUF;
+              if (p.epi_tma == 2) {
+                // 32 consecutive pixels of an image row (decoded by this one lane)
+                const int phase = p.phase_cols > 0 ? nb0 / p.phase_cols : tc.grp;
+                const int w = (tc.m_blk % p.tile_n0) * GEMM_BM + q * 32;
+                const int h = (tc.m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0];
+                if (tc.m_blk < p.m_blocks && w < p.out_w && h < p.out_h)
+                  tma_store_5d(&p.map_c, src, p.phase_cols > 0 ? nb0 - phase * p.phase_cols : nb0, p.out_off[phase][1], w, h,
+                               tc.m_blk / (p.tile_n0 * p.tile_n1));
+              } else {
+                const int row0 = tc.m_blk * GEMM_BM + q * 32;
+                if (row0 < p.M) {
+                  if (save_pre) tma_store_2d(&p.map_c2, src + 2 * Cfg::EPI_BUF, nb0, row0);
+                  tma_store_2d(&p.map_c, src, nb0, row0);
+                }
               }
+              bulk_commit_group();
             }
-            bulk_commit_group();
+            if (has_in && in_bufs == 1) {
+              if (lane == 0) bulk_wait_group_read<0>();
+              __syncwarp();
+              fetch_in(0);
+            }
           }
-          if (has_in) prefetch_next();
+          if (!released && !failed) release();   // a warp without a unit in this tile
         }
-        if (!released && !failed) release();   // a warp without a unit in this tile
-      }
-      if (lane == 0) bulk_wait_group_read<0>();
+        if (lane == 0) bulk_wait_group_read<0>();
+      };
+      const int form = p.epi & (EPI_BIAS | EPI_GELU | EPI_RESIDUAL | EPI_MUL_DGELU | EPI_SAVE_PRE);
+      if (p.alpha != 1.0f) run(std::integral_constant<int, -1>{});
+      else if (form == 0) run(std::integral_constant<int, 0>{});
+      else if (form == EPI_BIAS) run(std::integral_constant<int, EPI_BIAS>{});
+      else if (form == (EPI_BIAS | EPI_GELU | EPI_SAVE_PRE)) run(std::integral_constant<int, EPI_BIAS | EPI_GELU | EPI_SAVE_PRE>{});
+      else if (form == (EPI_BIAS | EPI_RESIDUAL)) run(std::integral_constant<int, EPI_BIAS | EPI_RESIDUAL>{});
+      else if (form == EPI_MUL_DGELU) run(std::integral_constant<int, EPI_MUL_DGELU>{});
+      else run(std::integral_constant<int, -1>{});
     } else
     for (int tile = unit; tile < total_tiles; tile += units, ++tcount) {
       const TileCoord first = decode_tile(p, tile, CTAS, rank, STACK);
@@ -926,7 +969,10 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   }
   GemmParams p = p_in;
   if (PEERS || STACK > 1) p.epi_tma = 0;
-  p.epi_bufs = p.epi_tma == 0 ? 1 : ((p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU | EPI_SAVE_PRE)) ? 4 : 2);
+  // (a long contraction hides the epilogue behind its main loop and wants the deeper ring: one buffer for input and output)
+  const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
+  p.epi_bufs = p.epi_tma == 0 ? 1 : ((p.epi & EPI_SAVE_PRE) || (has_in && p.k_blocks <= 12) ? 4 : 2);
+  if (p.epi_bufs == 4 && has_in && Cfg::stages_for(4) < 3) p.epi_bufs = 2;
   if (p.epi_tma == 1 && Cfg::stages_for(p.epi_bufs) < 3) {   // single-CTA tiles 256 wide: the ring needs the room
     p.epi_tma = 0;
     p.epi_bufs = 1;

@@ -101,10 +101,13 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 // shared out over the column tiles. Every split pays its start and its pass of atomics (1100 KB a row block, and 1.3 KB per
 // output block of the whole launch). Widths of 256 leave no room for the sums' accumulators: the column sums are then two
 // launches of their own, which read dy once more (10 us and 8.9 TB/s against 3.7 us per 1000 KB).
+// A pair of CTAs (request 1000 + width: 256 x 256 or 256 x 384 outputs) halves B's share and is bound by the tensor core instead: 512 or
+// 768 cycles per k-block, 74 and 140 KB of that measure as timed. Only the 384-wide tile has room for the sums (16 KB, shared out alike).
 // The constants were fitted to 11000 times: 64 to 557056 rows, 45 pairs of N and K between 96 and 4096, all widths, stacked or not, one
 // to four rounds (passes back to back in a CUDA graph); the choice is 2 % slower than the best plan on average. Without the 10 us the
 // separate sums were taken for few rows too (us, that / this rule): 512 rows of 384 x 1536 22 / 9, 2048 of 256 x 1024 19 / 9, 17280 of
-// 192 x 2208 39 / 23, 156672 of 3072 x 1024 839 / 799.
+// 192 x 2208 39 / 23, 156672 of 3072 x 1024 839 / 799. Pairs (us, best single / pair): 557056 rows of 2976 x 384 with sums 1184 / 1032,
+// without 1047 / 935, 139264 of 1536 x 384 231 / 202, 156672 of 3072 x 1024 without sums 704 / 647.
 struct WgradPlan {
   int bn, stack, split;
 };
@@ -112,24 +115,32 @@ WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   const int64_t m_blocks = (N + 127) / 128, k_blocks = (M + 63) / 64, sms = sm_count();
   WgradPlan best{128, 1, 1};
   double least = -1.0;
-  for (int stack : {1, 2}) {
-    if (stack > m_blocks) continue;
-    for (int bn : {192, 128, 256}) {
-      const int64_t n = (K + bn - 1) / bn, tiles = (m_blocks + stack - 1) / stack * n;
-      const double kb = 16.0 * stack + bn / 8 + stack * (16.0 + bn / 8) + (sums && bn < 256 ? 40.0 * stack / n : 0.0);
-      const double extra = sums && bn == 256 ? (10.0 + 2.0 * M * N / 8.9e6) / 0.0037 : 0.0;
-      // whole rounds of CTAs: the largest split of one round, two rounds, ...
-      for (int64_t rounds = 1; rounds <= 3; ++rounds) {
-        const int64_t split = std::max<int64_t>(1, std::min(rounds * sms / tiles, k_blocks));
-        const int64_t per = (k_blocks + split - 1) / split;
-        const double cost = static_cast<double>((tiles * split + sms - 1) / sms) * (per * kb + 1100.0 * stack) +
-                            1.3 * tiles * split * stack * bn / 192 + extra;
-        if (least < 0.0 || cost < least * 0.995) {
-          least = cost;
-          best = {bn, stack, static_cast<int>(split)};
-        }
+  // `width` columns, `blocks` 128-row blocks a tile, `kb` KB a k-block, on `units` CTAs or pairs; `pair`: two CTAs share the blocks
+  auto consider = [&](int request, int width, int stack, bool pair, double kb, double extra) {
+    const int64_t blocks = pair ? 2 : stack, units = pair ? sms / 2 : sms;
+    const int64_t n = (K + width - 1) / width, tiles = (m_blocks + blocks - 1) / blocks * n;
+    if (sums && extra == 0.0) kb += (pair ? 16.0 : 40.0 * stack) / n;
+    // whole rounds of CTAs: the largest split of one round, two rounds, ...
+    for (int64_t rounds = 1; rounds <= 3; ++rounds) {
+      const int64_t split = std::max<int64_t>(1, std::min(rounds * units / tiles, k_blocks));
+      const int64_t per = (k_blocks + split - 1) / split;
+      const double cost = static_cast<double>((tiles * split + units - 1) / units) * (per * kb + 1100.0 * (pair ? width / 128.0 : stack)) +
+                          1.3 * tiles * split * blocks * width / 192 + (pair ? 600.0 : 0.0) + extra;   // (a pair starts 2 us later)
+      if (least < 0.0 || cost < least * 0.995) {
+        least = cost;
+        best = {request, stack, static_cast<int>(split)};
       }
     }
+  };
+  const double separate = sums ? (10.0 + 2.0 * M * N / 5.6e6) / 0.0037 : 0.0;
+  for (int stack : {1, 2}) {
+    if (stack > m_blocks) continue;
+    for (int bn : {192, 128, 256})
+      consider(bn, bn, stack, false, 16.0 * stack + bn / 8 + stack * (16.0 + bn / 8), bn == 256 ? separate : 0.0);
+  }
+  if (tb::gemm_pairs() && sms >= 2 && m_blocks >= 2) {
+    if (K > 256) consider(1384, 384, 1, true, 140.0, 0.0);
+    if (K > 128) consider(1256, 256, 1, true, 74.0, separate);
   }
   return best;
 }
@@ -150,7 +161,7 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
     sums = false;
   }
   const WgradPlan plan = plan_wgrad(N, K, M, sums);
-  if (sums && plan.bn == 256) {
+  if (sums && plan.bn % 1000 == 256) {
     column_sums(dy, *grad_b);
     sums = false;
   }

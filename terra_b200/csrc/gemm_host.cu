@@ -117,7 +117,7 @@ static int pick_bn(long long N, int requested) {
 // and SM): a k-block of a 128 x BN tile costs (16 + BN / 8) KB of operand fill and as much again for the tensor core's
 // reads. In a pair each CTA stages 128 rows of A and only half of B's BN rows, (16 + BN / 16) KB. A pair starts later (two
 // cluster barriers) and its larger tiles leave more of the last round empty.
-static bool pairs_enabled() {
+bool gemm_pairs() {
   static const bool on = [] {
     const char* e = std::getenv("TERRA_GEMM_2CTA");
     return e == nullptr || std::atoi(e) != 0;
@@ -128,45 +128,49 @@ static bool pairs_enabled() {
 // Tile of a plain product or gathered convolution (no peers, no split, no column sums): the width and CTA count with the
 // least time by a model, in us. Persistent CTAs (pairs) take rounds of tiles; a tile takes the longer of its main loop and its
 // epilogue (rounds of 64-column units over the three warps of a lane quadrant, or of 32-column chunks where the lanes store
-// themselves) and a fixed hand-over, and the shorter of the two shows once, before the first or after the last tile.
+// themselves) and a fixed hand-over, and the shorter of the two shows once, before the first or after the last tile. Tiles of 384
+// columns (pairs) have one accumulator: main loop and most of the epilogue follow one another, for 40 KB of operands per k-block where
+// two tiles of 192 read 56 (128 wide, the only even width of a pair with an MN-major B and N = 384: 72).
 //
-// The constants were fitted to measurements, passes back to back in a CUDA graph at 1.9 GHz, falling to about 1.4 GHz under the
-// power cap in the largest. Products: 64 to 278528 rows, 31 pairs of N and K between 96 and 4096, five epilogues, all six
-// tiles (6600 times). Convolutions: the five forms, 64 to 384 channels, 16 x 32 to 512 x 1088 pixels (1500 times). The choice is
-// 0.5 % (0.3 %) slower than the best tile on average, more than 10 % in one case of 80 (none).
-// Against a rule that weighed tiles without rounds and start (us, both in turn on one GPU, before / this): 80000 x 136 x 384
-// with bias 36 / 21, 17280 x 1000 x 1000 62 / 41, 17280 x 1024 x 1024 GELU 52 / 43, 512 x 1024 x 4096 26 / 18; no change beyond the
-// noise for the 139264-row products of width 384 and 1024.
+// The constants were fitted to measurements, passes in a CUDA graph at 1.9 GHz, falling to about 1.4 GHz under the
+// power cap in the largest. Products: 512 to 139264 rows, 25 pairs of N and K between 96 and 3072, five epilogues, all seven
+// tiles (3100 times). Convolutions: the five forms, 96 to 384 channels, 16 x 32 to 512 x 1088 pixels (1300 times). The choice is
+// 0.5 % (0.4 %) slower than the best tile on average, more than 10 % in one case of 200. Before the fit and the 384-wide tiles (us, before /
+// this, on one GPU): input gradients 139264 x 384 x 1152 118 / 104, 139264 x 384 x 1536 153 / 132, 557056 x 384 x 2976 1113 / 1054;
+// patch embedding 557056 x 384 x 2976 1041 / 931, recovery 557056 x 2976 x 384 1662 / 1576.
 struct TileCosts {
-  double start[2], tile, tail, plain_unit;   // start: single CTAs, pairs
-  double kblock[2][3];                       // main loop per 64-wide k-block, widths 128, 192, 256
+  double start[2], tile, tail, plain_unit, bias_unit, drain;   // start: single CTAs, pairs
+  double kblock[2][4];                                         // main loop per 64-wide k-block, widths 128, 192, 256, 384
 };
 static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, bool gathered, int num_sms, int* bn_out,
                       int* ctas_out) {
   *bn_out = pick_bn(N, 0);
   *ctas_out = 1;
   if (N <= 64 || m_blocks < 1) return;
-  static const TileCosts rows = {{3.6, 6.1}, 0.95, 0.82, 0.83, {{0.29, 0.37, 0.45}, {0.215, 0.295, 0.39}}};
-  static const TileCosts image = {{4.5, 6.5}, 1.0, 0.62, 1.35, {{0.26, 0.31, 0.36}, {0.255, 0.286, 0.33}}};
+  static const TileCosts rows = {{4.04, 5.57}, 0.575, 0.93, 0.378, 0.806, 0.894, {{0.221, 0.320, 0.439}, {0.200, 0.274, 0.340, 0.535}}};
+  static const TileCosts image = {{4.24, 6.3}, 0.754, 0.404, 0.925, 0.925, 0.830, {{0.267, 0.306, 0.372}, {0.255, 0.278, 0.320, 0.490}}};
   const TileCosts& cost = gathered ? image : rows;
-  const bool input = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0, second = input || (flags & EPI_SAVE_PRE);
-  const double unit = (flags & EPI_MUL_DGELU) ? 2.9 : (flags & EPI_RESIDUAL) ? 1.88 : (flags & (EPI_GELU | EPI_SAVE_PRE)) ? 1.69 : cost.plain_unit;
-  const bool by_lane = !gemm_tma_epilogue() || (flags & (EPI_OUT_F32 | EPI_ATOMIC)) || (input && k_blocks > 12);
+  const bool input = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
+  const double unit = (flags & EPI_MUL_DGELU) ? 2.14 : (flags & EPI_RESIDUAL) ? 1.77 : (flags & (EPI_GELU | EPI_SAVE_PRE)) ? 2.19
+                      : (flags & EPI_BIAS) ? cost.bias_unit : cost.plain_unit;
+  const bool by_lane = !gemm_tma_epilogue() || (flags & (EPI_OUT_F32 | EPI_ATOMIC));
   double least = 0.0;
   for (int ctas : {1, 2}) {
-    if (ctas == 2 && (!pairs_enabled() || num_sms < 2)) continue;
-    for (int w = 0; w < 3; ++w) {
-      const int bn = 128 + 64 * w;
-      if (bn >= 2 * N || (ctas == 2 && b_mn && bn == 192)) continue;      // half of an MN-major B must be whole 64-row boxes
+    if (ctas == 2 && (!gemm_pairs() || num_sms < 2)) continue;
+    for (int w = 0; w < 2 + ctas; ++w) {
+      const int bn = w == 3 ? 384 : 128 + 64 * w;
+      if (bn >= 2 * N || (bn == 384 && N <= 256)) continue;
+      if (ctas == 2 && b_mn && bn == 192) continue;      // half of an MN-major B must be whole 64-row boxes
       const long long tiles = (m_blocks + ctas - 1) / ctas * ((N + bn - 1) / bn), units = num_sms / ctas;
-      const long long cols = std::min<long long>(bn, N);
-      // (single tiles of 256 columns leave no room for a second staging buffer beside the operand ring)
-      const bool lanes = by_lane || (second && bn == 256 && ctas == 1);
-      const double loop = k_blocks * cost.kblock[ctas - 1][w] * (ctas == 2 && b_mn ? 0.82 : 1.0);
+      const long long cols = std::min<long long>(bn, N), rounds = (tiles + units - 1) / units;
+      // (single tiles of 256 columns leave no room for the pre-activation's staging buffer beside the operand ring)
+      const bool lanes = by_lane || ((flags & EPI_SAVE_PRE) && !input && bn == 256 && ctas == 1);
+      const double loop = k_blocks * cost.kblock[ctas - 1][w];
       const double epilogue = unit * (lanes ? ((cols + 31) / 32 + 2) / 3 : ((cols + 63) / 64 + 2) / 3);
-      // (a tie goes to the pair, which loads less)
-      const double time = (cost.start[ctas - 1] + (tiles + units - 1) / units * (std::max(loop, epilogue) + cost.tile) +
-                           cost.tail * std::min(loop, epilogue)) * (ctas == 2 ? 0.99 : 1.0);
+      double time = cost.start[ctas - 1];
+      if (bn == 384) time += rounds * (std::max(loop + epilogue * cost.drain, epilogue) + cost.tile) + (1.0 - cost.drain) * epilogue;
+      else time += rounds * (std::max(loop, epilogue) + cost.tile) + cost.tail * std::min(loop, epilogue);
+      if (ctas == 2) time *= 0.99;      // (a tie goes to the pair, which loads less)
       if (least == 0.0 || time < least) {
         least = time;
         *bn_out = bn;
@@ -220,16 +224,16 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   if (bn_request >= 1000) {
     ctas = 2;
     bn_request -= 1000;
-    if (bn_request != 128 && bn_request != 256 && !(bn_request == 192 && !B.mn_major)) return -11;
+    if (bn_request != 128 && bn_request != 256 && !(bn_request == 192 && !B.mn_major) && bn_request != 384) return -11;
   } else if (bn_request == 0 && !A.mn_major && !gather_a && !scatter_c && split_k <= 1 && epi.colsum == nullptr) {
     gemm_tile(M, N, K, B.mn_major != 0, epi.flags, false, num_sms, &bn_request, &ctas);
   }
   if (epi.colsum != nullptr) {
     // column sums ride on the weight-gradient form only, and need room for their accumulators behind the tile's
-    if (!A.mn_major || (epi.flags & EPI_BIAS) || !(epi.flags & EPI_ATOMIC) || ctas != 1 || gather_a || scatter_c) return -15;
+    if (!A.mn_major || (epi.flags & EPI_BIAS) || !(epi.flags & EPI_ATOMIC) || (ctas != 1 && bn_request != 384) || gather_a || scatter_c) return -15;
     if (bn_request == 256 || (bn_request == 0 && pick_bn(N, 0) == 256)) bn_request = (N % 192 == 0) ? 192 : 128;
   }
-  const int bn = pick_bn(N, bn_request);
+  const int bn = bn_request == 384 ? 384 : pick_bn(N, bn_request);
   p.M = static_cast<int>(M);
   p.N = static_cast<int>(N);
   p.K = static_cast<int>(K);
@@ -284,7 +288,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   else rc = map_2d(&p.map_a, gather_a ? peers.a_ptr[p.a_first] : A.ptr, K, gather_a ? peers.a_rows : M, A.ld, GEMM_BK, GEMM_BM);
   if (rc != 0) return rc;
   if (B.mn_major) rc = map_2d(&p.map_b, B.ptr, N, K, B.ld, 64, GEMM_BK);
-  else rc = map_2d(&p.map_b, B.ptr, K, N, B.ld, GEMM_BK, bn / ctas);   // a CTA of a pair stages half of B's rows
+  else rc = map_2d(&p.map_b, B.ptr, K, N, B.ld, GEMM_BK, bn == 384 ? 64 : bn / ctas);   // a CTA of a pair stages half of B's rows
   if (rc != 0) return rc - 1000;
   fill_epilogue(p, epi);
   p.tile_n0 = 1;
@@ -381,7 +385,7 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   p.b_mode = OP_KMAJOR_2D;
   int rc = image_map(&p.map_a, c.x, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
   if (rc != 0) return rc;
-  rc = map_2d(&p.map_b, c.w, p.K, c.N, p.K, GEMM_BK, bn / ctas);
+  rc = map_2d(&p.map_b, c.w, p.K, c.N, p.K, GEMM_BK, bn == 384 ? 64 : bn / ctas);
   if (rc != 0) return rc - 1000;
   rc = attach_halos(p, halo_lo, halo_hi, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
   if (rc != 0) return rc;

@@ -50,19 +50,24 @@ constexpr int GEMM_THREADS = 32 * (GEMM_B_WARP + 1);
 // The operand stream through L2 bounds those products (12 TB/s measured with 128 x 192 tiles: 40 KB per k-block); stacked, a
 // k-block costs 56 KB for twice the outputs. There is no second accumulator set to overlap the epilogue with the next
 // tile, which a contraction over thousands of k-blocks does not need.
+//
+// BN = 384 (pairs): one tile of A meets 384 columns of B, as two MMAs of 256 and 128 columns (their halves are whole 64-column boxes in
+// either orientation of B).
 template <int BN, int CTAS, int STACK = 1>
 struct GemmCfg {
+  static constexpr bool WIDE = BN == 384;
+  static_assert(!WIDE || (CTAS == 2 && STACK == 1), "wide tiles: pairs");
   static constexpr int BLOCK_BYTES = GEMM_BM * GEMM_BK * 2;   // one 128-row block of A
   static constexpr int A_BYTES = STACK * BLOCK_BYTES;
-  static constexpr int ACCS = STACK == 1 ? 2 : 1;          // accumulator sets
+  static constexpr int ACCS = STACK == 1 && !WIDE ? 2 : 1;          // accumulator sets
   static constexpr int B_ROWS = BN / CTAS;                 // rows of B staged by one CTA
   static constexpr int B_BYTES = B_ROWS * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  // After the operand ring: 512 bytes of barriers, the per-warp bias slots (together 4 KB), then `bufs` buffers of
+  // After the operand ring: 1 KB of barriers, the per-warp bias slots (together 4 KB), then `bufs` buffers of
   // 2 KB per epilogue warp: one (the exchange buffer of the per-lane epilogue), or two (a 32 x 64 unit of the output on its
   // way to a TMA store), or four (another such unit: the saved pre-activation, or the operand the epilogue reads). The
   // ring takes what is left: the launcher passes the stage count to the kernel.
-  static constexpr int BAR_BYTES = 512;
+  static constexpr int BAR_BYTES = 1024;
   static constexpr int FIXED_BASE = 4096;
   static constexpr int EPI_BUF = 2048;
   static constexpr int MAX_SMEM = 232448;   // 227 KB, the per-block limit of sm_100
@@ -75,9 +80,9 @@ struct GemmCfg {
   static constexpr int smem_bytes(int bufs) { return stages_for(bufs) * STAGE_BYTES + fixed_bytes(bufs) + 1024; }   // + alignment slack
   // two accumulators (of alternating tiles, or of a tile's two row blocks); the allocation must be a power of two
   // behind them two 32-column accumulators of the column sums (weight-gradient form with a bias gradient, BN <= 192)
-  static constexpr int SUM_COL0 = 2 * BN;
-  static constexpr int TMEM_COLS = (2 * BN + 64 <= 256) ? 256 : 512;
-  static constexpr bool CAN_COLSUM = CTAS == 1 && 2 * BN + 64 <= 512;
+  static constexpr int SUM_COL0 = WIDE ? BN : 2 * BN;
+  static constexpr int TMEM_COLS = (SUM_COL0 + 64 <= 256) ? 256 : 512;
+  static constexpr bool CAN_COLSUM = (CTAS == 1 || WIDE) && SUM_COL0 + 64 <= 512;
   static_assert((STACK == 2 ? stages_for(1) : stages_for(2)) >= 3 && smem_bytes(1) <= MAX_SMEM && smem_bytes(2) <= MAX_SMEM, "shared memory budget");
   static_assert(GEMM_EPI_WARPS * 64 * 4 + BAR_BYTES <= FIXED_BASE, "bias slots");
   // a CTA's half of an MN-major B must be whole 64-row boxes; K-major rows only need whole 8-row swizzle atoms
@@ -104,32 +109,63 @@ __device__ __forceinline__ int first_sum_kb(const GemmParams& p, const TileCoord
   return t.kb_begin + (place + ways - t.kb_begin % ways) % ways;
 }
 
-// p.num_m_tiles counts tiles of ctas * 128 rows; m_blk is returned in units of 128 rows for CTA `rank` of the pair.
+// Walks over the tiles of a CTA (pair): tile t is the mixed-radix number (split, n, m, group) with the split varying fastest, and
+// a step adds the digits of the tile step. (Decoded by divisions a tile cost every role about 600 cycles, once per tile for the
+// loads and the MMAs and three times for the epilogue: as long as two k-blocks.)
+// p.num_m_tiles counts tiles of ctas * 128 rows; m_blk is in units of 128 rows for CTA `rank` of the pair.
 // Stacked tiles (p.stack = 2 blocks of rows): the row tile varies slowest, so that the last one, which may hold a single
 // block, is handed out last.
-__device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int tile, int ctas = 1, int rank = 0, int stack = 1) {
-  TileCoord t;
-  t.split = tile % p.split_k;
-  int r = tile / p.split_k;
-  t.n_blk = r % p.num_n_tiles;
-  r /= p.num_n_tiles;
-  if (stack > 1) {
-    t.grp = r % p.groups;
-    t.m_blk = r / p.groups * stack;
-  } else {
-    t.m_blk = (r % p.num_m_tiles) * ctas + rank;
-    t.grp = r / p.num_m_tiles;
+template <int CTAS, int STACK>
+struct TileWalk {
+  int tile, split, n, lo, hi;          // (lo, hi) = (m, group), stacked tiles (group, m)
+  int step, d_split, d_n, d_lo, d_hi;
+  __device__ __forceinline__ TileWalk(const GemmParams& p, int first, int by) : tile(first), step(by) {
+    digits(p, first, split, n, lo, hi);
+    digits(p, by, d_split, d_n, d_lo, d_hi);
   }
-  if (p.grp_ranges) {
-    t.kb_begin = p.grp_kb[t.grp];
-    t.kb_end = p.grp_kb[t.grp + 1];
-  } else {
-    const int per = (p.k_blocks + p.split_k - 1) / p.split_k;
-    t.kb_begin = t.split * per;
-    t.kb_end = min(p.k_blocks, t.kb_begin + per);
+  static __device__ __forceinline__ void digits(const GemmParams& p, int t, int& split, int& n, int& lo, int& hi) {
+    const int radix = STACK > 1 ? p.groups : p.num_m_tiles;
+    split = 0;
+    if (p.split_k > 1) {
+      split = t % p.split_k;
+      t /= p.split_k;
+    }
+    n = t % p.num_n_tiles;
+    t /= p.num_n_tiles;
+    lo = t % radix;
+    hi = t / radix;
   }
-  return t;
-}
+  __device__ __forceinline__ void next(const GemmParams& p) {
+    tile += step;
+    split += d_split;
+    int carry = split >= p.split_k;
+    split -= carry ? p.split_k : 0;
+    n += d_n + carry;
+    carry = n >= p.num_n_tiles;
+    n -= carry ? p.num_n_tiles : 0;
+    lo += d_lo + carry;
+    const int radix = STACK > 1 ? p.groups : p.num_m_tiles;
+    carry = lo >= radix;
+    lo -= carry ? radix : 0;
+    hi += d_hi + carry;
+  }
+  __device__ __forceinline__ int m_blk(int rank) const { return STACK > 1 ? hi * STACK : lo * CTAS + rank; }
+  __device__ __forceinline__ TileCoord coord(const GemmParams& p, int rank, int per_split) const {
+    TileCoord t;
+    t.split = split;
+    t.n_blk = n;
+    t.m_blk = m_blk(rank);
+    t.grp = STACK > 1 ? lo : hi;
+    if (p.grp_ranges) {
+      t.kb_begin = p.grp_kb[t.grp];
+      t.kb_end = p.grp_kb[t.grp + 1];
+    } else {
+      t.kb_begin = split * per_split;
+      t.kb_end = min(p.k_blocks, t.kb_begin + per_split);
+    }
+    return t;
+  }
+};
 
 // mbar_wait that adds the time spent to `waited`; a barrier that is complete costs one test and reads no clock.
 template <bool PAIR>
@@ -148,7 +184,7 @@ template <int BN, int CTAS, bool PEERS, int STACK = 1>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   static_assert(STACK == 1 || (CTAS == 1 && !PEERS), "stacked tiles: one CTA, no peers");
   using Cfg = GemmCfg<BN, CTAS, STACK>;
-  constexpr bool PAIR = CTAS == 2;
+  constexpr bool PAIR = CTAS == 2, WIDE = Cfg::WIDE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int stages = p.stages;
@@ -157,11 +193,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   uint64_t* empty = full + Cfg::MAX_STAGES;
   uint64_t* tfull = empty + Cfg::MAX_STAGES;
   uint64_t* tempty = tfull + 2;
-  uint64_t* pfull = tempty + 2;   // pair mode, leader CTA: "the peer's half of stage s has landed"
-  uint64_t* in_bar = pfull + Cfg::MAX_STAGES;   // two per epilogue warp: "the epilogue operand's unit has landed"
+  uint64_t* in_bar = tempty + 2;   // two per epilogue warp: "the epilogue operand's unit has landed"
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(in_bar + 2 * GEMM_EPI_WARPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((3 * Cfg::MAX_STAGES + 4 + 2 * GEMM_EPI_WARPS) * 8 + 8 <= Cfg::BAR_BYTES, "barrier block");
+  static_assert((2 * Cfg::MAX_STAGES + 4 + 2 * GEMM_EPI_WARPS) * 8 + 8 <= Cfg::BAR_BYTES, "barrier block");
   float* bias_slots = reinterpret_cast<float*>(fixed + Cfg::BAR_BYTES);
   uint8_t* xchg = fixed + Cfg::FIXED_BASE;
   // The ring needs a 1024-byte aligned base (128-byte swizzle atoms). The dynamic window normally starts aligned; if
@@ -180,9 +215,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::MAX_STAGES; ++s) {
-      mbar_init(&full[s], 2);         // both producers
+      mbar_init(&full[s], 2);         // both producers (a pair: the leader's, for the loads of both CTAs)
       mbar_init(&empty[s], 1);
-      mbar_init(&pfull[s], 1);
     }
     for (int i = 0; i < 2 * GEMM_EPI_WARPS; ++i) mbar_init(&in_bar[i], 1);
     for (int a = 0; a < 2; ++a) {
@@ -226,6 +260,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   }
 
   const int total_tiles = p.groups * p.num_m_tiles * p.num_n_tiles * p.split_k;
+  const int per_split = p.split_k > 1 ? (p.k_blocks + p.split_k - 1) / p.split_k : p.k_blocks;
+  using Walk = TileWalk<CTAS, STACK>;
   // Bound of the CTA-internal waits, in units of about a second of polling. The producer of the tensor-parallel form
   // may wait a_budget_ns (global timer) for a peer's shard; the roles that consume its stages must outlast that wait,
   // or ordinary rank skew would abort a tile whose data arrives in time. Measured polling rates put one unit between
@@ -240,8 +276,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       const long long t_begin = clock64();
       long long t_wait = 0;
       unsigned int peers_ready = 0u;   // bit per (peer, chunk) whose flag has been seen
-      for (int tile = unit; tile < total_tiles && !*abort_flag; tile += units) {
-        const TileCoord tc = decode_tile(p, tile, CTAS, rank, STACK);
+      for (Walk walk(p, unit, units); walk.tile < total_tiles && !*abort_flag; walk.next(p)) {
+        const TileCoord tc = walk.coord(p, rank, per_split);
         const int m0 = tc.m_blk * GEMM_BM;
         const int blocks = STACK > 1 ? min(STACK, p.m_blocks - tc.m_blk) : 1;   // 128-row blocks of this tile
         int abase[5] = {0, 0, 0, 0, 0};
@@ -255,7 +291,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
           if (!wait_counted<PAIR>(&empty[s], ph ^ 1u, abort_flag, p.status, 0x100u + s, mbar_budget, t_wait)) break;
           uint8_t* sA = smem + s * Cfg::STAGE_BYTES;
-          mbar_expect_tx(&full[s], STACK > 1 ? blocks * Cfg::BLOCK_BYTES : Cfg::A_BYTES);
+          if (rank == 0) mbar_expect_tx(&full[s], STACK > 1 ? blocks * Cfg::BLOCK_BYTES : CTAS * Cfg::BLOCK_BYTES);
+          const uint32_t bar = PAIR ? map_to_cta(&full[s], 0) : smem_u32(&full[s]);
           int pw = 0, ph_ = 0, pb = 0;
           if (p.a_mode == OP_PIXELS_5D) {
             pw = kb % p.pix_n0;
@@ -287,15 +324,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
                 fence_proxy_async_all();   // order the acquire before the asynchronous-proxy reads of the shard
                 peers_ready |= 1u << fidx;
               }
-              tma_load_2d(sA, &p.map_a_peer[peer], &full[s], kb * GEMM_BK, lm * GEMM_BM);
+              tma_load_2d<PAIR>(sA, &p.map_a_peer[peer], bar, kb * GEMM_BK, lm * GEMM_BM);
             } else {
-              tma_load_2d(sA, &p.map_a, &full[s], kb * GEMM_BK, m0);
+              tma_load_2d<PAIR>(sA, &p.map_a, bar, kb * GEMM_BK, m0);
             }
           } else if (p.a_mode == OP_MNMAJOR_2D) {
 #pragma unroll
             for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
               if (STACK == 1 || j < blocks * (GEMM_BM / 64))
-                tma_load_2d(sA + j * (GEMM_BK * 128), &p.map_a, &full[s], m0 + j * 64, kb * GEMM_BK);
+                tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, kb * GEMM_BK);
           } else if (p.a_mode == OP_TABLE_5D) {
             const short* e = p.ktable[kb];
             int h = abase[3] + e[3];
@@ -307,12 +344,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               m = &p.map_halo_hi;
               h -= p.img_h;
             }
-            tma_load_5d(sA, m, &full[s], abase[0] + e[0], abase[1] + e[1], abase[2] + e[2], h, abase[4]);
+            tma_load_5d<PAIR>(sA, m, bar, abase[0] + e[0], abase[1] + e[1], abase[2] + e[2], h, abase[4]);
           } else {  // OP_PIXELS_5D: {channels, 1, w, h, b}
 #pragma unroll
             for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
               if (STACK == 1 || j < blocks * (GEMM_BM / 64))
-                tma_load_5d(sA + j * (GEMM_BK * 128), &p.map_a, &full[s], m0 + j * 64, 0, pw * GEMM_BK, ph_, pb);
+                tma_load_5d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, 0, pw * GEMM_BK, ph_, pb);
           }
         }
       }
@@ -325,13 +362,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       int s = 0;
       uint32_t ph = 0;
       long long t_wait = 0;
-      for (int tile = unit; tile < total_tiles && !*abort_flag; tile += units) {
-        const TileCoord tc = decode_tile(p, tile, CTAS, rank, STACK);
-        const int n0 = tc.n_blk * BN + rank * Cfg::B_ROWS;   // this CTA's rows of B
+      for (Walk walk(p, unit, units); walk.tile < total_tiles && !*abort_flag; walk.next(p)) {
+        const TileCoord tc = walk.coord(p, rank, per_split);
+        // this CTA's rows of B, in boxes of 64 where they are not one (wide tiles: its halves of 256 and of 128)
+        const int n0 = tc.n_blk * BN + rank * (WIDE ? 128 : Cfg::B_ROWS);
+        auto box_at = [&](int j) { return WIDE && j == 2 ? tc.n_blk * BN + 256 + rank * 64 : n0 + j * 64; };
         for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
           if (!wait_counted<PAIR>(&empty[s], ph ^ 1u, abort_flag, p.status, 0x140u + s, mbar_budget, t_wait)) break;
           uint8_t* sB = smem + s * Cfg::STAGE_BYTES + Cfg::A_BYTES;
-          mbar_expect_tx(&full[s], Cfg::B_BYTES);
+          if (rank == 0) mbar_expect_tx(&full[s], CTAS * Cfg::B_BYTES);
+          const uint32_t bar = PAIR ? map_to_cta(&full[s], 0) : smem_u32(&full[s]);
           int pw = 0, ph_ = 0, pb = 0;
           if (p.b_mode == OP_PIXELS_5D) {
             pw = kb % p.pix_n0;
@@ -339,11 +379,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             pb = kb / (p.pix_n0 * p.pix_n1);
           }
           if (p.b_mode == OP_KMAJOR_2D) {
-            tma_load_2d(sB, &p.map_b, &full[s], kb * GEMM_BK, n0);
+            if (WIDE) {
+#pragma unroll
+              for (int j = 0; j < 3; ++j) tma_load_2d<PAIR>(sB + j * (64 * 128), &p.map_b, bar, kb * GEMM_BK, box_at(j));
+            } else {
+              tma_load_2d<PAIR>(sB, &p.map_b, bar, kb * GEMM_BK, n0);
+            }
           } else if (p.b_mode == OP_MNMAJOR_2D) {
 #pragma unroll
             for (int j = 0; Cfg::CAN_B_MN && j < Cfg::B_ROWS / 64; ++j)
-              tma_load_2d(sB + j * (GEMM_BK * 128), &p.map_b, &full[s], n0 + j * 64, kb * GEMM_BK);
+              tma_load_2d<PAIR>(sB + j * (GEMM_BK * 128), &p.map_b, bar, box_at(j), kb * GEMM_BK);
           } else {  // OP_PIXELS_5D with per-group (tap) displacement
             const short* g = p.grp_off[tc.grp];
             int h = ph_ * p.pix_hmul + g[2];
@@ -356,8 +401,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               h -= p.img_h;
             }
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_5d(sB + j * (GEMM_BK * 128), m, &full[s], n0 + j * 64, g[0], pw * GEMM_BK + g[1], h, pb);
+            for (int j = 0; j < Cfg::B_ROWS / 64; ++j)
+              tma_load_5d<PAIR>(sB + j * (GEMM_BK * 128), m, bar, box_at(j), g[0], pw * GEMM_BK + g[1], h, pb);
           }
         }
       }
@@ -365,21 +410,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA in pair mode)
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(GEMM_BM * CTAS, BN, p.a_mode == OP_MNMAJOR_2D || p.a_mode == OP_PIXELS_5D,
-                                             p.b_mode == OP_MNMAJOR_2D || p.b_mode == OP_PIXELS_5D);
       const bool a_mn = (p.a_mode == OP_MNMAJOR_2D || p.a_mode == OP_PIXELS_5D);
       const bool b_mn = (p.b_mode == OP_MNMAJOR_2D || p.b_mode == OP_PIXELS_5D);
+      const uint32_t idesc = make_idesc_bf16(GEMM_BM * CTAS, WIDE ? 256 : BN, a_mn, b_mn);
+      const uint32_t idesc_rest = make_idesc_bf16(GEMM_BM * CTAS, 128, a_mn, b_mn);      // wide tiles: columns 256 to 383
       const uint32_t a_lbo = a_mn ? GEMM_BK * 128 : 16, b_lbo = b_mn ? GEMM_BK * 128 : 16;
       const uint32_t a_kstep = a_mn ? (16 * 128) >> 4 : 32 >> 4;   // descriptor units of 16 bytes
       const uint32_t b_kstep = b_mn ? (16 * 128) >> 4 : 32 >> 4;
-      const uint32_t idesc_sums = make_idesc_bf16(GEMM_BM, 16, a_mn, 0);
+      const uint32_t idesc_sums = make_idesc_bf16(GEMM_BM * CTAS, PAIR ? 32 : 16, a_mn, 0);   // (16 rows of ones per CTA)
       const uint64_t d_ones = make_smem_desc_plain(smem_u32(bias_slots), 128, 256);
       int s = 0;
+      bool landed = false;                   // the next stage has been seen full
       uint32_t ph = 0, tcount = 0;
       const long long t_begin = clock64();
       long long t_acc = 0, t_ops = 0;
-      for (int tile = unit; tile < total_tiles && !*abort_flag; tile += units, ++tcount) {
-        const TileCoord tc = decode_tile(p, tile, CTAS, rank, STACK);
+      for (Walk walk(p, unit, units); walk.tile < total_tiles && !*abort_flag; walk.next(p), ++tcount) {
+        const TileCoord tc = walk.coord(p, rank, per_split);
         const int acc = tcount % Cfg::ACCS;
         const uint32_t aph = (tcount / Cfg::ACCS) & 1u;
         const int blocks = STACK > 1 ? min(STACK, p.m_blocks - tc.m_blk) : 1;
@@ -388,38 +434,55 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         t_acc += clock64() - w0;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        const int ways = p.groups * p.num_n_tiles;
-        const int sum_first = Cfg::CAN_COLSUM && p.colsum != nullptr ? first_sum_kb(p, tc, ways) : tc.kb_end;
-        int sum_kb = sum_first;
-        const uint32_t d_sums = tmem_base + Cfg::SUM_COL0 + acc * 32;
         bool ok = true;
-        for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
-          if (!wait_counted<PAIR>(&full[s], ph, abort_flag, p.status, 0x300u + s, mbar_budget, t_ops)) { ok = false; break; }
-          if (PAIR && !wait_counted<PAIR>(&pfull[s], ph, abort_flag, p.status, 0x380u + s, mbar_budget, t_ops)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sA = smem_u32(smem + s * Cfg::STAGE_BYTES);
-          const uint32_t sB = sA + Cfg::A_BYTES;
-          const uint64_t da = make_smem_desc(sA, a_lbo, 1024);
-          const uint64_t db = make_smem_desc(sB, b_lbo, 1024);
-#pragma unroll
-          for (int mb = 0; mb < STACK; ++mb) {
-            if (STACK > 1 && mb >= blocks) break;
-            const uint64_t dm = da + mb * (Cfg::BLOCK_BYTES >> 4);
-#pragma unroll
-            for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
-              umma_bf16<CTAS>(d_tmem + mb * BN, dm + kk * a_kstep, db + kk * b_kstep, idesc, (kb > tc.kb_begin || kk > 0) ? 1u : 0u);
+        // (Column sums have a loop of their own: with their test inside, the four MMAs of a k-block took 200 to 280 cycles to issue
+        // instead of 60.)
+        auto k_loop = [&](auto with_sums) {
+          constexpr bool SUMS = decltype(with_sums)::value;
+          const int ways = p.groups * p.num_n_tiles;
+          const int sum_first = SUMS ? first_sum_kb(p, tc, ways) : 0;
+          int sum_kb = sum_first;
+          const uint32_t d_sums = tmem_base + Cfg::SUM_COL0 + acc * 32;
+          for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb) {
+            if (!landed && !wait_counted<PAIR>(&full[s], ph, abort_flag, p.status, 0x300u + s, mbar_budget, t_ops)) {
+              ok = false;
+              break;
             }
-            if (Cfg::CAN_COLSUM && kb == sum_kb) {   // column sums of A: the same A tiles against 16 columns of ones
+            tc_fence_after();
+            const uint32_t sA = smem_u32(smem + s * Cfg::STAGE_BYTES);
+            const uint32_t sB = sA + Cfg::A_BYTES;
+            uint64_t* const freed = &empty[s];
+            ph ^= (s + 1 == stages);
+            s = (s + 1 == stages) ? 0 : s + 1;
+            landed = mbar_test(&full[s], ph);       // (a look at the next stage, whose latency the MMAs cover)
+            const uint64_t da = make_smem_desc(sA, a_lbo, 1024);
+            const uint64_t db = make_smem_desc(sB, b_lbo, 1024);
 #pragma unroll
-              for (int kk = 0; kk < GEMM_BK / 16; ++kk)
-                umma_bf16<CTAS>(d_sums + mb * 32, dm + kk * a_kstep, d_ones, idesc_sums, (kb > sum_first || kk > 0) ? 1u : 0u);
+            for (int mb = 0; mb < STACK; ++mb) {
+              if (STACK > 1 && mb >= blocks) break;
+              const uint64_t dm = da + mb * (Cfg::BLOCK_BYTES >> 4);
+#pragma unroll
+              for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
+                umma_bf16<CTAS>(d_tmem + mb * BN, dm + kk * a_kstep, db + kk * b_kstep, idesc, (kb > tc.kb_begin || kk > 0) ? 1u : 0u);
+                if (WIDE)
+                  umma_bf16<CTAS>(d_tmem + 256, dm + kk * a_kstep, db + (128 * 128 >> 4) + kk * b_kstep, idesc_rest,
+                                  (kb > tc.kb_begin || kk > 0) ? 1u : 0u);
+              }
+              if (SUMS && kb == sum_kb) {   // column sums of A: the same A tiles against columns of ones
+#pragma unroll
+                for (int kk = 0; kk < GEMM_BK / 16; ++kk)
+                  umma_bf16<CTAS>(d_sums + mb * 32, dm + kk * a_kstep, d_ones, idesc_sums, (kb > sum_first || kk > 0) ? 1u : 0u);
+              }
             }
+            if (SUMS && kb == sum_kb) sum_kb += ways;
+            umma_commit<CTAS>(freed);     // frees the stage (in both CTAs of a pair)
           }
-          if (kb == sum_kb) sum_kb += ways;
-          umma_commit<CTAS>(&empty[s]);     // frees stage s (in both CTAs of a pair)
+        };
+        if constexpr (Cfg::CAN_COLSUM) {
+          if (p.colsum != nullptr) k_loop(std::true_type{});
+          else k_loop(std::false_type{});
+        } else {
+          k_loop(std::false_type{});
         }
         if (!ok) break;
         umma_commit<CTAS>(&tfull[acc]);     // accumulator complete (in both CTAs of a pair)
@@ -427,20 +490,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       atomicAdd(&g_gemm_stalls[0], static_cast<unsigned long long>(clock64() - t_begin));
       atomicAdd(&g_gemm_stalls[1], static_cast<unsigned long long>(t_acc));
       atomicAdd(&g_gemm_stalls[2], static_cast<unsigned long long>(t_ops));
-    } else if (PAIR && rank == 1 && elect_one()) {
-      // Peer CTA: its MMA warp has nothing to issue. It forwards "my half of stage s has landed" to the leader, whose
-      // MMA thread waits for both halves before it issues.
-      int s = 0;
-      uint32_t ph = 0;
-      for (int tile = unit; tile < total_tiles && !*abort_flag; tile += units) {
-        const TileCoord tc = decode_tile(p, tile, CTAS, rank);
-        bool ok = true;
-        for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
-          if (!mbar_wait<PAIR>(&full[s], ph, abort_flag, p.status, 0x3c0u + s, mbar_budget)) { ok = false; break; }
-          mbar_arrive_remote(map_to_cta(&pfull[s], 0));
-        }
-        if (!ok) break;
-      }
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..13)
@@ -488,24 +537,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       const uint32_t swz = (static_cast<uint32_t>(lane) & 7u) << 4;
       const uint32_t bias_base = smem_u32(my_bias);
       // coordinates of this warp's units, in the order it works on them
-      struct Walk {
-        int tile, u, n0, row;
+      struct Units {
+        Walk walk;
+        int u;
       };
-      auto walk_next = [&](Walk& w, int& col, int& row) -> bool {
-        if (part >= UNITS) return false;
-        while (w.tile < total_tiles) {
-          if (w.u == part) {        // the divisions once per tile
-            const TileCoord t = decode_tile(p, w.tile, CTAS, rank);
-            w.n0 = t.n_blk * BN;
-            w.row = t.m_blk * GEMM_BM + q * 32;
-          }
-          col = w.n0 + w.u * 64;
-          row = w.row;
-          const bool ok = w.u < UNITS && col < p.N;
+      auto next_unit = [&](Units& w, int& col, int& row) -> bool {
+        while (part < UNITS && w.walk.tile < total_tiles) {
+          col = w.walk.n * BN + w.u * 64;
+          row = w.walk.m_blk(rank) * GEMM_BM + q * 32;
+          const bool ok = col < p.N;
           w.u += WARPS_PER_Q;
           if (w.u >= UNITS) {
             w.u = part;
-            w.tile += units;
+            w.walk.next(p);
           }
           if (ok) return true;
         }
@@ -519,26 +563,26 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         const bool has_in = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0, dgelu = (flags & EPI_MUL_DGELU) != 0;
         const f32x2 alpha2 = f2_both(p.alpha);
         const int in_bufs = p.epi_bufs / 2;
-        Walk load = {unit, part, 0, 0}, ahead = load;
+        Units load = {Walk(p, unit, units), part}, ahead = load;
         auto fetch_in = [&](int buf) {       // this warp's next input unit into `buf`; the unit after it into L2
           int col, row;
-          if (walk_next(load, col, row) && lane == 0) {
+          if (next_unit(load, col, row) && lane == 0) {
             mbar_expect_tx(my_in + buf, 2 * Cfg::EPI_BUF);
             tma_load_2d(my_out + buf * 2 * Cfg::EPI_BUF, &p.map_in, my_in + buf, col, row);
           }
-          if (walk_next(ahead, col, row) && lane == 0) tma_prefetch_l2_2d(&p.map_in, col, row);
+          if (next_unit(ahead, col, row) && lane == 0) tma_prefetch_l2_2d(&p.map_in, col, row);
         };
         if (has_in) {
           int col, row;
-          walk_next(ahead, col, row);        // `ahead` runs one unit in front of `load`
+          next_unit(ahead, col, row);        // `ahead` runs one unit in front of `load`
           fetch_in(0);
         }
         uint32_t count = 0;                  // units of this warp so far
         bool failed = false;
-        for (int tile = unit; tile < total_tiles && !failed; tile += units, ++tcount) {
-          const TileCoord tc = decode_tile(p, tile, CTAS, rank);
-          const int acc = tcount & 1;
-          const uint32_t aph = (tcount >> 1) & 1u;
+        for (Walk walk(p, unit, units); walk.tile < total_tiles && !failed; walk.next(p), ++tcount) {
+          const TileCoord tc = walk.coord(p, rank, per_split);
+          const int acc = tcount % Cfg::ACCS;
+          const uint32_t aph = (tcount / Cfg::ACCS) & 1u;
           const int n0 = tc.n_blk * BN;
           auto bias_pair = [&](int col) -> float2 {     // columns col, col + 1 (col even)
             float2 b = make_float2(0.f, 0.f);
@@ -598,6 +642,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             __syncwarp();
             if (has_in && in_bufs == 2) fetch_in(buf ^ 1);
             const uint32_t row_out = out_base + buf * 2 * Cfg::EPI_BUF;
+            const int row0 = tc.m_blk * GEMM_BM + q * 32;
 #pragma unroll
             for (int g = 0; g < 8; ++g) {      // 8 columns: 16 bytes of the output row
               const uint32_t at = (static_cast<uint32_t>(g) << 4) ^ swz;
@@ -660,7 +705,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
                   tma_store_5d(&p.map_c, src, p.phase_cols > 0 ? nb0 - phase * p.phase_cols : nb0, p.out_off[phase][1], w, h,
                                tc.m_blk / (p.tile_n0 * p.tile_n1));
               } else {
-                const int row0 = tc.m_blk * GEMM_BM + q * 32;
                 if (row0 < p.M) {
                   if (save_pre) tma_store_2d(&p.map_c2, src + 2 * Cfg::EPI_BUF, nb0, row0);
                   tma_store_2d(&p.map_c, src, nb0, row0);
@@ -687,8 +731,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       else if (form == EPI_MUL_DGELU) run(std::integral_constant<int, EPI_MUL_DGELU>{});
       else run(std::integral_constant<int, -1>{});
     } else
-    for (int tile = unit; tile < total_tiles; tile += units, ++tcount) {
-      const TileCoord first = decode_tile(p, tile, CTAS, rank, STACK);
+    for (Walk walk(p, unit, units); walk.tile < total_tiles; walk.next(p), ++tcount) {
+      const TileCoord first = walk.coord(p, rank, per_split);
       const int acc = tcount % Cfg::ACCS;
       const uint32_t aph = (tcount / Cfg::ACCS) & 1u;
       const int n0 = first.n_blk * BN;
@@ -1016,6 +1060,7 @@ cudaError_t gemm_read_stalls(unsigned long long* out8, bool reset) {
 cudaError_t launch_gemm(const GemmParams& p, int bn, int ctas, int num_sms, cudaStream_t stream) {
   if (ctas == 2) {
     switch (bn) {
+      case 384: return launch_bn<384, 2>(p, num_sms, stream);
       case 128: return launch_bn<128, 2>(p, num_sms, stream);
       case 192: return p.b_mode == OP_KMAJOR_2D ? launch_bn<192, 2>(p, num_sms, stream) : cudaErrorInvalidValue;
       case 256: return launch_bn<256, 2>(p, num_sms, stream);

@@ -73,6 +73,7 @@ int gemm_bf16(const GemmOperand& A, const GemmOperand& B, long long M, long long
 // free stages, [5] epilogue span, [6] epilogue waiting for tiles. Synchronises the device.
 // The rule's tile of a plain product (no peers, no split, no column sums) when no width is asked for: columns, and CTAs per
 // tile of 128 rows each (2: a CTA pair). `gathered`: of a convolution with M / 128 row tiles and K / 64 taps x channel chunks.
+bool gemm_pairs();   // CTA pairs are allowed (TERRA_GEMM_2CTA)
 void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, bool gathered, int num_sms, int* bn, int* ctas);
 bool gemm_tma_epilogue();   // whether the epilogue may go through TMA (environment switch)
 int gemm_stall_counters(unsigned long long* out8, int reset);

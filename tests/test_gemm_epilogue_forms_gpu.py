@@ -18,7 +18,7 @@ def _data(m, n, k, seed=0):
     return r(m, k), r(n, k) * k ** -0.5, r(n), r(m, n) * 3
 
 
-@pytest.mark.parametrize("bn", [0, 128, 192, 256, 1128, 1192, 1256])
+@pytest.mark.parametrize("bn", [0, 128, 192, 256, 1128, 1192, 1256, 1384])
 @pytest.mark.parametrize("form", FORMS)
 def test_forms_against_64_bits(form, bn):
     for m, n, k in SIZES:
@@ -68,3 +68,28 @@ def test_gelu_derivative_outside_the_fit():
     got = gemm(torch.ones(8, 8, device="cuda").to(torch.bfloat16), eye, dgelu_aux=x.repeat(8, 1)).float()
     want = (x.float() > 0).float().repeat(8, 1)
     assert (got - want).abs().max() < 1e-3
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 64), (255, 264, 64), (256, 384, 128), (1000, 392, 1000), (20000, 768, 200), (40000, 384, 1160)])
+def test_tiles_384_wide_with_the_weight_as_stored(m, n, k):
+    """Input gradients: B MN-major, whose halves of 256 and of 128 columns are whole boxes."""
+    a, w, _, _ = _data(m, n, k, 1)
+    got = gemm(a, w.t().contiguous(), b_mn=True, bn=1384)
+    want = a.double() @ w.double().t()
+    assert ((got.double() - want).abs() <= want.abs() * 2 ** -8 + 1e-5).all()      # half a bf16 step, fp32 sums of values near 1
+    check_status("cuda")
+
+
+@pytest.mark.parametrize("rows,n,k,split", [(64, 8, 264, 1), (1000, 256, 384, 3), (5000, 400, 392, 7), (30000, 1528, 768, 11)])
+@pytest.mark.parametrize("bn,sums", [(1384, True), (1384, False), (1256, False)])
+def test_weight_gradients_of_pairs(rows, n, k, split, bn, sums):
+    """Both operands MN-major, the column sums from a 32-column MMA over the pair. fp32 sums in another order: 1e-5 of the norm."""
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    dy, x = (torch.randn(rows, c, generator=gen, device="cuda").to(torch.bfloat16) for c in (n, k))
+    gw, gb = torch.ones(n, k, device="cuda"), torch.ones(n, device="cuda")
+    gemm(dy, x, a_mn=True, b_mn=True, out=gw, accumulate=True, split_k=split, bn=bn, colsum=gb if sums else None)
+    check_status("cuda")
+    rel = lambda got, want: ((got.double() - want).norm() / want.norm()).item()
+    assert rel(gw - 1, dy.double().t() @ x.double()) < 1e-5
+    if sums:
+        assert rel(gb, 1 + dy.double().sum(0)) < 1e-5

@@ -1,6 +1,7 @@
 // Memory-bound kernels: LayerNorm, GroupNorm(+SiLU), column sums, masked loss, fused AdamW.
 // All are single-pass over HBM where the math allows it, with 16-byte vector accesses.
 #include <cstdlib>
+#include "chained_launch.cuh"
 #include "common.cuh"
 #include "host_api.h"
 
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(256, VPL == 1 ? 6 : (VPL == 2 ? 5 : (VPL <= 4 
                                                             __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out,
                                                             float* __restrict__ rstd_out, long long rows, int C,
                                                             float eps) {
+  chain_begin();
   constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31, sub = lane % LPR;
   const int nvec = EXACT ? LPR * VPL : C >> 3;
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 
                                                             __nv_bfloat16* __restrict__ dx, float* __restrict__ dgamma,
                                                             float* __restrict__ dbeta, const __nv_bfloat16* __restrict__ dres,
                                                             long long rows, int C) {
+  chain_begin();
   constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31, sub = lane % LPR;
   const int nvec = EXACT ? LPR * VPL : C >> 3;
@@ -232,6 +235,7 @@ __global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 
 // ------------------------------------------------------------------------------------------ column sums
 __global__ void __launch_bounds__(256) colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ partials,
                                                      long long rows, int C, long long ld, int rows_per_block) {
+  chain_begin();
   // thread -> one 8-wide column vector; blockDim.y rows in flight. blockDim.x spans the whole row when it has at most
   // 64 vectors (a row is then one contiguous read), otherwise 32 vectors per block column.
   const int nvec = C >> 3;
@@ -283,6 +287,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const __nv_bfloat16* __rest
 // out[c] += sum over r of partials[r][c]. Block = 32 columns x 32 row lanes.
 __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __restrict__ partials, float* __restrict__ out,
                                                              int nparts, int C) {
+  chain_begin();
   __shared__ float sh[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
@@ -311,6 +316,7 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat16* __restrict__ x,
                                                               float* __restrict__ sums, long long HW, int C, int groups,
                                                               int pix_per_block) {
+  chain_begin();
   extern __shared__ float sh[];  // [2][C]
   const int nvec = C >> 3;
   const int b = blockIdx.y;
@@ -383,6 +389,7 @@ __global__ void __launch_bounds__(256, 3) groupnorm_silu_apply_kernel(const __nv
                                                                       const __nv_bfloat16* __restrict__ res,
                                                                       __nv_bfloat16* __restrict__ y, long long HW, int C,
                                                                       int groups, int pix_per_block) {
+  chain_begin();
   const int nvec = C >> 3;
   const int b = blockIdx.y;
   const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
@@ -430,6 +437,7 @@ __global__ void __launch_bounds__(256, 3) groupnorm_silu_bwd_reduce_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta, float* __restrict__ red,
     long long HW, int C, int groups, int pix_per_block, float* __restrict__ dgamma, float* __restrict__ dbeta) {
+  chain_begin();
   extern __shared__ float sh[];  // [2][C]
   const int nvec = C >> 3;
   const int b = blockIdx.y;
@@ -502,6 +510,7 @@ __global__ void __launch_bounds__(256, 3) groupnorm_silu_bwd_reduce_kernel(
 // {sum, sum of squares} per (sample, group) -> {mean, rstd}; the sums are cleared for their next use
 __global__ void groupnorm_finalize_kernel(float* __restrict__ sums, float* __restrict__ stats, int cells, float inv_count,
                                           float eps, int clear) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < cells) {
     const float mean = sums[2 * i] * inv_count;
@@ -520,6 +529,7 @@ __global__ void groupnorm_finalize_kernel(float* __restrict__ sums, float* __res
 // gradients into the (Cout, Cin, kh, kw) layout of the gradient arena.
 __global__ void __launch_bounds__(256) strided_add_kernel(float* __restrict__ src, float* __restrict__ dst, int na, int nb,
                                                           int nc, long long sa, long long sb, long long sc, int clear) {
+  chain_begin();
   const long long total = static_cast<long long>(na) * nb * nc;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -537,6 +547,7 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const float* __restrict__ red, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
     __nv_bfloat16* __restrict__ dx, long long HW, int C, int groups, float inv_count, int pix_per_block) {
+  chain_begin();
   extern __shared__ float gs[];  // [groups][2] of this block's sample
   const int cpg = C / groups, nvec = C >> 3;
   const int b = blockIdx.y;
@@ -602,6 +613,7 @@ __global__ void __launch_bounds__(256) masked_loss_kernel(const __nv_bfloat16* _
                                                           const __nv_bfloat16* __restrict__ mask, long long nvec,
                                                           long long mask_period_vec, int kind, float grad_scale,
                                                           float* __restrict__ loss_sum, __nv_bfloat16* __restrict__ grad) {
+  chain_begin();
   float acc = 0.f;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -644,6 +656,7 @@ __global__ void __launch_bounds__(256) masked_loss_kernel(const __nv_bfloat16* _
 __global__ void __launch_bounds__(256) attn_rowdot_kernel(const uint4* __restrict__ o, const uint4* __restrict__ dout,
                                                           float* __restrict__ drow, long long rows, int vec_per_row,
                                                           int vec_per_head, int heads) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -669,6 +682,7 @@ __global__ void __launch_bounds__(256) attn_rowdot_kernel(const uint4* __restric
 // One pass over a flat fp32 gradient buffer for the loss-scaling path: out[0] += sum of squares (for the clipping
 // norm), out[1] becomes non-zero when any element is inf or nan (the step is then skipped and the scale backed off).
 __global__ void __launch_bounds__(256) grad_inspect_kernel(const float* __restrict__ g, long long n, float* __restrict__ out) {
+  chain_begin();
   float acc = 0.f;
   bool bad = false;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -705,6 +719,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ master, 
                                                     __nv_bfloat16* __restrict__ param, long long n, float lr, float b1,
                                                     float b2, float eps, float wd, float bc1, float bc2s,
                                                     float gscale) {
+  chain_begin();
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float g = GRAD_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(grad)[i])
@@ -724,6 +739,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ master, 
 }
 
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ d, long long n) {
+  chain_begin();
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
     d[i] = __float2bfloat16(s[i]);
@@ -731,6 +747,7 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ s, __nv_bfloat16*
 
 __global__ void add_bf16_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, uint4* __restrict__ o,
                                 long long nvec) {
+  chain_begin();
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float x[8], y[8];
@@ -752,6 +769,7 @@ struct PackTaps {
 };
 __global__ void __launch_bounds__(256) pack_taps_kernel(const __nv_bfloat16* __restrict__ w, uint32_t* __restrict__ out,
                                                         PackTaps p, long long total) {
+  chain_begin();
   const int half = p.Cpad >> 1;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -775,6 +793,7 @@ __global__ void __launch_bounds__(256) pack_taps_kernel(const __nv_bfloat16* __r
 template <bool F32>
 __global__ void conv_s2_col2im_kernel(const uint4* __restrict__ dcol, void* __restrict__ out, int B, int Ho, int Wo, int W,
                                       int cvec, int r0, int rows) {
+  chain_begin();
   const long long total = static_cast<long long>(B) * rows * W * cvec;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -826,6 +845,7 @@ constexpr int PATCH_UNROLL = 4;
 template <class V>
 __global__ void __launch_bounds__(256) pad_patchify_kernel(const V* __restrict__ x, V* __restrict__ patches, int H, int p, int hn,
                                                            int top, int left_units, int img_units, int row_units, int seg_units) {
+  chain_begin();
   const int yy = blockIdx.y % (hn * p), b = blockIdx.y / (hn * p);
   const int y = yy - top;
   const V* src = x + (static_cast<long long>(b) * H + y) * img_units - left_units;
@@ -862,6 +882,7 @@ template <class V>
 __global__ void __launch_bounds__(256) unpatchify_crop_kernel(const V* __restrict__ patches, const V* __restrict__ add,
                                                               V* __restrict__ out, int H, int p, int hn, int top, int left_units,
                                                               int img_units, int row_units, int seg_units) {
+  chain_begin();
   const int y = blockIdx.y % H, b = blockIdx.y / H;
   const int yy = y + top;
   const V* src = patches + (static_cast<long long>(b) * hn + yy / p) * p * row_units + static_cast<long long>(yy % p) * seg_units;
@@ -888,6 +909,7 @@ __global__ void __launch_bounds__(256) unpatchify_crop_kernel(const V* __restric
 // reduce-scatter with the row-parallel layer's bias and the block's shortcut folded in.
 __global__ void sum_slots_bf16_kernel(const uint4* __restrict__ src, uint4* __restrict__ o, int slots, long long nvec,
                                       const uint4* __restrict__ bias, const uint4* __restrict__ res, int cvec) {
+  chain_begin();
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float acc[8];
@@ -963,8 +985,7 @@ inline int ln_bwd_blocks(int vpl, bool exact, long long rows) {
 int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                   long long rows, int C, float eps, cudaStream_t stream) {
   if (C % 8 != 0 || C > 2048) return -1;
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 16, (layernorm_fwd_kernel<LPR, VPL, EXACT><<<grid_for(rows, 8 * (32 / LPR), ln_fwd_blocks(VPL)), 256, 0, stream>>>(
-                            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
+  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 16, (launch_chained(layernorm_fwd_kernel<LPR, VPL, EXACT>, grid_for(rows, 8 * (32 / LPR), ln_fwd_blocks(VPL)), 256, 0, stream, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
                             static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(y), mean, rstd, rows, C,
                             eps)));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -974,8 +995,7 @@ int layernorm_bwd(const void* dy, const void* x, const void* gamma, const float*
                   float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream) {
   if (C % 8 != 0 || C > 2048) return -1;
   const size_t sh = 2 * C * sizeof(float);
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (layernorm_bwd_kernel<LPR, VPL, EXACT><<<grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh, stream>>>(
-                            static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (launch_chained(layernorm_bwd_kernel<LPR, VPL, EXACT>, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh, stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
                             static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma,
                             dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C)));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -994,8 +1014,8 @@ int colsum_bf16(const void* x, float* out, float* partials, long long rows, int 
   const int nparts = static_cast<int>((rows + rows_per_block - 1) / rows_per_block);
   dim3 grid(static_cast<unsigned>(nparts), (nvec + bx - 1) / bx);
   const size_t sh = static_cast<size_t>(by) * (bx * 8 + 1) * sizeof(float);
-  colsum_kernel<<<grid, block, sh, stream>>>(static_cast<const __nv_bfloat16*>(x), partials, rows, C, ld, rows_per_block);
-  colsum_finish_kernel<<<(C + 31) / 32, dim3(32, 32), 0, stream>>>(partials, out, nparts, C);
+  launch_chained(colsum_kernel, grid, block, sh, stream, static_cast<const __nv_bfloat16*>(x), partials, rows, C, ld, rows_per_block);
+  launch_chained(colsum_finish_kernel, (C + 31) / 32, dim3(32, 32), 0, stream, partials, out, nparts, C);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1032,7 +1052,7 @@ int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int 
   // 139264 x 128 15 / 22, 139264 x 256 20 / 23, 139264 x 384 52 / 29).
   const bool small = static_cast<long long>(B) * HW * C * 2 <= 72000000LL;
   const GnShape s(B, HW, C, 512, small ? 1 : 3, 4);
-  groupnorm_stats_kernel<<<s.grid, s.block, 2 * C * sizeof(float), stream>>>(static_cast<const __nv_bfloat16*>(x), sums, HW,
+  launch_chained(groupnorm_stats_kernel, s.grid, s.block, 2 * C * sizeof(float), stream, static_cast<const __nv_bfloat16*>(x), sums, HW,
                                                                              C, groups, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1041,8 +1061,7 @@ int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, c
                          int B, long long HW, int C, int groups, cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 6, 2);
-  groupnorm_silu_apply_kernel<<<s.grid, s.block, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
+  launch_chained(groupnorm_silu_apply_kernel, s.grid, s.block, 0, stream, static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
       static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(y), HW,
       C, groups, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1053,8 +1072,7 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
                               cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 3, 2);
-  groupnorm_silu_bwd_reduce_kernel<<<s.grid, s.block, 2 * C * sizeof(float), stream>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
+  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, 2 * C * sizeof(float), stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
       static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups,
       s.pix, dgamma, dbeta);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1062,7 +1080,7 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
 
 int groupnorm_finalize(float* sums, float* stats, int cells, float inv_count, float eps, int clear, cudaStream_t stream) {
   if (cells <= 0) return 0;
-  groupnorm_finalize_kernel<<<(cells + 255) / 256, 256, 0, stream>>>(sums, stats, cells, inv_count, eps, clear);
+  launch_chained(groupnorm_finalize_kernel, (cells + 255) / 256, 256, 0, stream, sums, stats, cells, inv_count, eps, clear);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1070,7 +1088,7 @@ int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa
                     cudaStream_t stream) {
   const long long total = static_cast<long long>(na) * nb * nc;
   if (total <= 0) return 0;
-  strided_add_kernel<<<grid_for(total, 256), 256, 0, stream>>>(src, dst, na, nb, nc, sa, sb, sc, clear);
+  launch_chained(strided_add_kernel, grid_for(total, 256), 256, 0, stream, src, dst, na, nb, nc, sa, sb, sc, clear);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1079,8 +1097,7 @@ int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, 
                              cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 4, 2);
-  groupnorm_silu_bwd_apply_kernel<<<s.grid, s.block, groups * 2 * sizeof(float), stream>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red,
+  launch_chained(groupnorm_silu_bwd_apply_kernel, s.grid, s.block, groups * 2 * sizeof(float), stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red,
       static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
       static_cast<__nv_bfloat16*>(dx), HW, C, groups, inv_count, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1090,8 +1107,7 @@ int masked_loss_fwd_bwd(const void* pred, const void* label, const void* mask, l
                         int kind, float grad_scale, float* loss_sum, void* grad, cudaStream_t stream) {
   if (n % 8 != 0 || (mask != nullptr && mask_period % 8 != 0)) return -1;
   const long long nvec = n / 8;
-  masked_loss_kernel<<<grid_for(nvec, 256), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(pred), static_cast<const __nv_bfloat16*>(label),
+  launch_chained(masked_loss_kernel, grid_for(nvec, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(pred), static_cast<const __nv_bfloat16*>(label),
       static_cast<const __nv_bfloat16*>(mask), nvec, mask != nullptr ? mask_period / 8 : 1, kind, grad_scale, loss_sum,
       static_cast<__nv_bfloat16*>(grad));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1102,24 +1118,24 @@ int adamw_step(float* master, float* exp_avg, float* exp_avg_sq, const void* gra
                float bias_corr2_sqrt, float grad_scale, cudaStream_t stream) {
   const int grid = grid_for(n, 256);
   if (grad_is_bf16)
-    adamw_kernel<true><<<grid, 256, 0, stream>>>(master, exp_avg, exp_avg_sq, grad,
+    launch_chained(adamw_kernel<true>, grid, 256, 0, stream, master, exp_avg, exp_avg_sq, grad,
                                                  static_cast<__nv_bfloat16*>(param_bf16), n, lr, beta1, beta2, eps,
                                                  weight_decay, bias_corr1, bias_corr2_sqrt, grad_scale);
   else
-    adamw_kernel<false><<<grid, 256, 0, stream>>>(master, exp_avg, exp_avg_sq, grad,
+    launch_chained(adamw_kernel<false>, grid, 256, 0, stream, master, exp_avg, exp_avg_sq, grad,
                                                   static_cast<__nv_bfloat16*>(param_bf16), n, lr, beta1, beta2, eps,
                                                   weight_decay, bias_corr1, bias_corr2_sqrt, grad_scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int cast_f32_to_bf16(const float* src, void* dst, long long n, cudaStream_t stream) {
-  cast_f32_bf16_kernel<<<grid_for(n, 256), 256, 0, stream>>>(src, static_cast<__nv_bfloat16*>(dst), n);
+  launch_chained(cast_f32_bf16_kernel, grid_for(n, 256), 256, 0, stream, src, static_cast<__nv_bfloat16*>(dst), n);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int add_bf16(const void* a, const void* b, void* out, long long n, cudaStream_t stream) {
   if (n % 8 != 0) return -1;
-  add_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>(static_cast<const uint4*>(a), static_cast<const uint4*>(b),
+  launch_chained(add_bf16_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const uint4*>(a), static_cast<const uint4*>(b),
                                                             static_cast<uint4*>(out), n / 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1129,10 +1145,10 @@ int conv_s2_col2im(const void* dcol, void* out, int B, int Ho, int Wo, int W, in
   if (C % 8 != 0 || rows <= 0) return -1;
   const long long total = static_cast<long long>(B) * rows * W * (C / 8);
   if (out_f32)
-    conv_s2_col2im_kernel<true><<<grid_for(total, 256), 256, 0, stream>>>(static_cast<const uint4*>(dcol), out, B, Ho, Wo, W,
+    launch_chained(conv_s2_col2im_kernel<true>, grid_for(total, 256), 256, 0, stream, static_cast<const uint4*>(dcol), out, B, Ho, Wo, W,
                                                                           C / 8, r0, rows);
   else
-    conv_s2_col2im_kernel<false><<<grid_for(total, 256), 256, 0, stream>>>(static_cast<const uint4*>(dcol), out, B, Ho, Wo, W,
+    launch_chained(conv_s2_col2im_kernel<false>, grid_for(total, 256), 256, 0, stream, static_cast<const uint4*>(dcol), out, B, Ho, Wo, W,
                                                                            C / 8, r0, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1154,10 +1170,10 @@ int patch_relayout(const void* image, const void* add, void* patches, void* imag
     const int span = to_patches ? row_units : img_units;
     const dim3 grid((span + 256 * PATCH_UNROLL - 1) / (256 * PATCH_UNROLL), static_cast<unsigned>(rows));
     if (to_patches)
-      pad_patchify_kernel<V><<<grid, 256, 0, stream>>>(static_cast<const V*>(image), static_cast<V*>(patches), H, p, hn, top, lu,
+      launch_chained(pad_patchify_kernel<V>, grid, 256, 0, stream, static_cast<const V*>(image), static_cast<V*>(patches), H, p, hn, top, lu,
                                                        img_units, row_units, seg);
     else
-      unpatchify_crop_kernel<V><<<grid, 256, 0, stream>>>(static_cast<const V*>(patches), static_cast<const V*>(add),
+      launch_chained(unpatchify_crop_kernel<V>, grid, 256, 0, stream, static_cast<const V*>(patches), static_cast<const V*>(add),
                                                           static_cast<V*>(image_out), H, p, hn, top, lu, img_units, row_units, seg);
   };
   if (bytes % 16 == 0) launch(uint4{});
@@ -1173,7 +1189,7 @@ int pack_taps_bf16(const void* w, void* out, int N1, int N2, int V2, int T, int 
   PackTaps p = {N2, V2, T, C, Cpad, s1, s2, sc, {}};
   for (int t = 0; t < T; ++t) p.off[t] = offsets[t];
   const long long total = static_cast<long long>(N1) * N2 * T * (Cpad / 2);
-  pack_taps_kernel<<<grid_for(total, 256), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(w), static_cast<uint32_t*>(out), p,
+  launch_chained(pack_taps_kernel, grid_for(total, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(w), static_cast<uint32_t*>(out), p,
                                                              total);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1183,14 +1199,14 @@ int attn_rowdot(const void* o, const void* dout, float* drow, long long rows, in
   if (heads <= 0 || C % heads != 0) return -1;
   const int hd = C / heads;
   if (hd != 16 && hd != 32 && hd != 64 && hd != 128) return -1;
-  attn_rowdot_kernel<<<grid_for(rows * 32, 256), 256, 0, stream>>>(static_cast<const uint4*>(o), static_cast<const uint4*>(dout),
+  launch_chained(attn_rowdot_kernel, grid_for(rows * 32, 256), 256, 0, stream, static_cast<const uint4*>(o), static_cast<const uint4*>(dout),
                                                                   drow, rows, C / 8, hd / 8, heads);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int grad_inspect(const float* grad, long long n, float* out2, cudaStream_t stream) {
   if (n <= 0) return 0;
-  grad_inspect_kernel<<<grid_for(n, 256 * 8, 148 * 8), 256, 0, stream>>>(grad, n, out2);
+  launch_chained(grad_inspect_kernel, grid_for(n, 256 * 8, 148 * 8), 256, 0, stream, grad, n, out2);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1198,7 +1214,7 @@ int sum_slots_bf16(const void* src, void* out, int slots, long long n, cudaStrea
                    const void* residual, int cols) {
   if (n % 8 != 0 || slots < 1) return -1;
   if (bias != nullptr && (cols <= 0 || cols % 8 != 0 || n % cols != 0)) return -1;
-  sum_slots_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>(static_cast<const uint4*>(src), static_cast<uint4*>(out),
+  launch_chained(sum_slots_bf16_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const uint4*>(src), static_cast<uint4*>(out),
                                                                   slots, n / 8, static_cast<const uint4*>(bias),
                                                                   static_cast<const uint4*>(residual), cols > 0 ? cols / 8 : 1);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

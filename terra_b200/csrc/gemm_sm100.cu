@@ -28,6 +28,7 @@
 // Every wait is bounded; on expiry the CTA sets its abort flag, records the site in the
 // KernelStatus word, drains, releases TMEM and returns.
 #include <type_traits>
+#include "chained_launch.cuh"
 #include "gemm_sm100.cuh"
 
 namespace tb {
@@ -203,6 +204,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   // the alignment shift does not fit into the slack the launch is refused as a whole, before any barrier exists.
   if (stages < 1 || stages > Cfg::MAX_STAGES ||
       xchg + GEMM_EPI_WARPS * p.epi_bufs * Cfg::EPI_BUF > smem_raw + p.smem_bytes) {
+    chain_begin();
     if (threadIdx.x == 0) report_error(p.status, TB_ERR_BAD_ARG, 0x700u, blockIdx.x, 0u);
     return;
   }
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   if (PAIR) cluster_sync_all(); else __syncthreads();   // barriers and allocations of both CTAs exist from here on
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();        // global memory is touched from here on
   if (PAIR) {
     // the pair-wide MMA names one tensor-memory address for both CTAs: the two allocations must coincide
     if (threadIdx.x == 0 && ld_shared_cluster_u32(map_to_cta(tmem_slot, rank ^ 1)) != tmem_base) {
@@ -1028,22 +1031,25 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   if (total <= 0) return cudaSuccess;
   if (max_units < 1) return cudaErrorInvalidValue;   // a pair on one SM
   const int units = total < max_units ? total : max_units;
-  if (CTAS == 1) {
-    gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK><<<units, GEMM_THREADS, p.smem_bytes, stream>>>(p);
-    return cudaGetLastError();
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(units * CTAS);
   cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = p.smem_bytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  int attrs = 0;
+  if (!PEERS) {      // (kernels that wait for another GPU are not chained)
+    attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (CTAS > 1) {
+    attr[attrs].id = cudaLaunchAttributeClusterDimension;
+    attr[attrs].val.clusterDim.x = CTAS;
+    attr[attrs].val.clusterDim.y = 1;
+    attr[attrs++].val.clusterDim.z = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = attrs;
   return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, p);
 }
 

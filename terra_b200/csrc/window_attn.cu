@@ -26,6 +26,7 @@
 // 2176 shifted windows of 8 x 8, 12 heads of 32 channels: forward 105 us (a version with four-warp blocks that walked over
 // heads and looked every bias up took 324 us; 66 us of HBM traffic), backward 246 us (586 us; 115 us).
 #include <atomic>
+#include "chained_launch.cuh"
 #include "common.cuh"
 #include "host_api.h"
 #include "window_geo.cuh"
@@ -376,10 +377,6 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
   const float scale2 = a.scale * WA_LOG2E;
   const int ti = tid / a.ww, tj = tid % a.ww;                    // token `tid` of a window
 
-  for (int i = tid; i < HPC * geo.nrel; i += Cfg::THREADS) {
-    const int h = i / geo.nrel, r = i % geo.nrel;
-    bias_s[i] = use_bias ? a.bias_table[r * a.num_heads + head0 + h] * WA_LOG2E : 0.f;
-  }
   if (tid < NPAD) {
     cofs[tid] = ti * (2 * a.ww - 1) + tj;
     if (tid >= N)
@@ -407,7 +404,12 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
   WaItem cur = next;
   if (tid < N) wa_table(a, geo, next, ti, tj, tabs + tid);
   __syncthreads();
+  chain_begin();        // global memory is touched from here on
   if (STAGES == 2) wa_gather<Cfg, BWD>(a, tabs, smem_u32(stages), ch0, tid, q0, q1);
+  for (int i = tid; i < HPC * geo.nrel; i += Cfg::THREADS) {
+    const int h = i / geo.nrel, r = i % geo.nrel;
+    bias_s[i] = use_bias ? a.bias_table[r * a.num_heads + head0 + h] * WA_LOG2E : 0.f;
+  }      // (seen after the barrier that opens the first window)
   if (static_cast<int>(blockIdx.x) + step < items) {
     next = wa_item(a, blockIdx.x + step, my_nw);
     if (tid < N) wa_table(a, geo, next, ti, tj, tabs + NPAD + tid);
@@ -620,7 +622,9 @@ int launch(WindowAttnArgs a, cudaStream_t stream) {
   int gx = sms * occupancy / groups;             // one resident wave: a CTA of a second wave would repeat the set-up
   if (gx < 1) gx = 1;
   if (gx > items) gx = items;
-  kernel<<<dim3(gx, groups), Cfg::THREADS, sb, stream>>>(a);
+  // (with peers a neighbour's flags order the buffers: launched plainly)
+  if (a.n_wg * a.sp * a.tp == 1) launch_chained(kernel, dim3(gx, groups), dim3(Cfg::THREADS), sb, stream, a);
+  else kernel<<<dim3(gx, groups), Cfg::THREADS, sb, stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -22;
 }
 

@@ -1,0 +1,294 @@
+// The layers as autograd nodes in C++: the same launches as the Python nodes (which the multi-rank layouts, tracing and function
+// transforms use), without the interpreter in the backward pass. A small layer is bound by the host: a Python node costs about
+// 50 us of interpreter, argument lists and hand-over of the interpreter lock for its two directions, around 40 us of launches.
+//
+// A node keeps the operands that belong to the layer (bf16 weights, gradient accumulators, packed weights) beside the tensors
+// saved for the backward pass, which go through whatever saved-tensor hooks are set. Parameter gradients are accumulated in place; the
+// parameter among the inputs (`anchor`) only makes autograd call the node when the activation needs no gradient.
+// Us per pass, Python node / this: attention half of 512 rows of width 96 @@A@@, residual convolution and GroupNorm of 96 x 180 pixels
+// @@B@@, a training step of 19 such layers @@C@@.
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/extension.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include "check.h"
+#include "torch_ops.h"
+
+namespace {
+
+using torch::Tensor;
+using OptTensor = c10::optional<torch::Tensor>;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+
+template <class T>
+using Held = c10::intrusive_ptr<T>;
+
+template <class T>
+void hold(AutogradContext* ctx, const Held<T>& layer) {
+  ctx->saved_data["layer"] = c10::IValue::make_capsule(layer);
+}
+template <class T>
+Held<T> held(AutogradContext* ctx) {
+  return c10::static_intrusive_pointer_cast<T>(ctx->saved_data["layer"].toCapsule());
+}
+
+// ------------------------------------------------------------------------------------------------ attention half
+struct AttnLayer : torch::CustomClassHolder {
+  Tensor ln_w, ln_b, qkv_w, qkv_b, proj_w, proj_b, ln_wg, ln_bg, qkv_wg, qkv_bg, proj_wg, proj_bg, status;
+  OptTensor table, table_g;
+  std::vector<int64_t> geo;
+  double scale, eps;
+  bool fuse_bias;
+};
+
+struct AttnHalf : Function<AttnHalf> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& anchor, const Held<AttnLayer>& l) {
+    auto r = terra_ops::attn_half_fwd(x, l->ln_w, l->ln_b, l->qkv_w, l->qkv_b, l->proj_w, l->proj_b, l->table, l->geo, l->scale, l->eps,
+                                      l->status);
+    ctx->save_for_backward({x, r[1], r[2], r[3], r[4], r[5]});
+    hold(ctx, l);
+    return r[0];
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list dy) {
+    const auto s = ctx->get_saved_variables();
+    const auto l = held<AttnLayer>(ctx);
+    return {terra_ops::attn_half_bwd(dy[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5], l->ln_w, l->qkv_w, l->proj_w, l->table, l->ln_wg,
+                                     l->ln_bg, l->qkv_wg, l->qkv_bg, l->proj_wg, l->proj_bg, l->table_g, l->geo, l->scale, l->fuse_bias,
+                                     l->status),
+            Tensor(), Tensor()};
+  }
+};
+
+Tensor attn_half(const Tensor& x, const Tensor& anchor, const std::vector<Tensor>& w, const std::vector<Tensor>& g, const OptTensor& table,
+                 const OptTensor& table_g, std::vector<int64_t> geo, double scale, double eps, bool fuse_bias, const Tensor& status) {
+  need(w.size() == 6 && g.size() == 6, "attention half: six weights and their gradients");
+  auto l = c10::make_intrusive<AttnLayer>();
+  l->ln_w = w[0], l->ln_b = w[1], l->qkv_w = w[2], l->qkv_b = w[3], l->proj_w = w[4], l->proj_b = w[5];
+  l->ln_wg = g[0], l->ln_bg = g[1], l->qkv_wg = g[2], l->qkv_bg = g[3], l->proj_wg = g[4], l->proj_bg = g[5];
+  l->table = table, l->table_g = table_g, l->geo = std::move(geo), l->scale = scale, l->eps = eps, l->fuse_bias = fuse_bias;
+  l->status = status;
+  return AttnHalf::apply(x, anchor, l);
+}
+
+// ------------------------------------------------------------------------------------------------ MLP half
+struct MlpLayer : torch::CustomClassHolder {
+  Tensor ln_w, ln_b, fc1_w, fc1_b, fc2_w, fc2_b, ln_wg, ln_bg, fc1_wg, fc1_bg, fc2_wg, fc2_bg, status;
+  double eps;
+  bool fuse_bias;
+};
+
+struct MlpHalf : Function<MlpHalf> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& anchor, const Held<MlpLayer>& l) {
+    auto r = terra_ops::mlp_half_fwd(x, l->ln_w, l->ln_b, l->fc1_w, l->fc1_b, l->fc2_w, l->fc2_b, l->eps, l->status);
+    ctx->save_for_backward({x, r[1], r[2], r[3], r[4], r[5]});
+    hold(ctx, l);
+    return r[0];
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list dy) {
+    const auto s = ctx->get_saved_variables();
+    const auto l = held<MlpLayer>(ctx);
+    return {terra_ops::mlp_half_bwd(dy[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5], l->ln_w, l->fc1_w, l->fc2_w, l->ln_wg, l->ln_bg,
+                                    l->fc1_wg, l->fc1_bg, l->fc2_wg, l->fc2_bg, l->fuse_bias, l->status),
+            Tensor(), Tensor()};
+  }
+};
+
+Tensor mlp_half(const Tensor& x, const Tensor& anchor, const std::vector<Tensor>& w, const std::vector<Tensor>& g, double eps, bool fuse_bias,
+                const Tensor& status) {
+  need(w.size() == 6 && g.size() == 6, "MLP half: six weights and their gradients");
+  auto l = c10::make_intrusive<MlpLayer>();
+  l->ln_w = w[0], l->ln_b = w[1], l->fc1_w = w[2], l->fc1_b = w[3], l->fc2_w = w[4], l->fc2_b = w[5];
+  l->ln_wg = g[0], l->ln_bg = g[1], l->fc1_wg = g[2], l->fc1_bg = g[3], l->fc2_wg = g[4], l->fc2_bg = g[5];
+  l->eps = eps, l->fuse_bias = fuse_bias, l->status = status;
+  return MlpHalf::apply(x, anchor, l);
+}
+
+// ------------------------------------------------------------------------------------------------ linear
+struct LinearLayer : torch::CustomClassHolder {
+  Tensor w, wg, status;
+  OptTensor b, bg;
+  bool need_dx, fuse_bias, has_res;
+};
+
+struct Linear : Function<Linear> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& anchor, const OptTensor& residual, const Held<LinearLayer>& l) {
+    Tensor y = terra_ops::linear_product(x, l->w, false, l->b, residual, l->status);
+    ctx->save_for_backward({x});
+    hold(ctx, l);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const auto l = held<LinearLayer>(ctx);
+    const Tensor dy = grads[0].contiguous();
+    terra_ops::wgrad(dy, s[0], l->wg, l->bg, l->fuse_bias, l->status);
+    Tensor dx;
+    if (l->need_dx) dx = terra_ops::linear_product(dy, l->w, true, c10::nullopt, c10::nullopt, l->status);
+    return {dx, Tensor(), l->has_res ? dy : Tensor(), Tensor()};
+  }
+};
+
+Tensor linear(const Tensor& x, const Tensor& anchor, const Tensor& w, const OptTensor& b, const Tensor& wg, const OptTensor& bg,
+              const OptTensor& residual, bool need_dx, bool fuse_bias, const Tensor& status) {
+  auto l = c10::make_intrusive<LinearLayer>();
+  l->w = w, l->b = b, l->wg = wg, l->bg = bg, l->need_dx = need_dx, l->fuse_bias = fuse_bias, l->has_res = residual.has_value();
+  l->status = status;
+  return Linear::apply(x, anchor, residual, l);
+}
+
+// ------------------------------------------------------------------------------------------------ 3x3 convolution
+struct ConvLayer : torch::CustomClassHolder {
+  Tensor w_fwd, b, wg, bg, staging, status;   // staging: fp32 [9, Cout, Cin], zero between uses
+  OptTensor w_dgrad;                           // given where the input needs a gradient
+  int64_t stride, split, stack;
+  bool fuse_bias;
+};
+
+struct Conv3x3 : Function<Conv3x3> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, const Held<ConvLayer>& l) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t st = l->stride;
+    Tensor y = torch::empty({x.size(0), st == 1 ? x.size(1) : (x.size(1) + 1) / 2, x.size(2) / st, l->w_fwd.size(0)},
+                            x.options().dtype(torch::kBFloat16));
+    terra_ops::conv3x3_fwd(x, l->w_fwd, y, st, 1 /* with bias */, l->b, c10::nullopt, l->status, c10::nullopt, c10::nullopt);
+    ctx->save_for_backward({x});
+    hold(ctx, l);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const auto l = held<ConvLayer>(ctx);
+    const Tensor& x = s[0];
+    const Tensor dy = grads[0].contiguous();
+    const c10::cuda::CUDAGuard guard(dy.device());
+    const int64_t cin = l->staging.size(2);
+    terra_ops::conv3x3_wgrad(x, dy, l->staging, l->stride, l->split, l->status, c10::nullopt, c10::nullopt,
+                             l->fuse_bias ? OptTensor(l->bg) : OptTensor(), l->stack);
+    terra_ops::strided_add(l->staging, l->wg, 1, cin * 9, 9, true);
+    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, dy.size(3)}), l->bg);
+    Tensor dx;
+    if (l->w_dgrad.has_value()) {
+      dx = torch::empty_like(x);
+      if (l->stride == 1)
+        terra_ops::conv3x3_fwd(dy, *l->w_dgrad, dx, 1, 0, c10::nullopt, c10::nullopt, l->status, c10::nullopt, c10::nullopt);
+      else
+        terra_ops::conv3x3_s2_dgrad(dy, *l->w_dgrad, dx, l->status);
+    }
+    return {dx, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor conv3x3(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad, const Tensor& b,
+               const Tensor& wg, const Tensor& bg, const Tensor& staging, int64_t stride, int64_t split, int64_t stack, bool fuse_bias,
+               const Tensor& status) {
+  auto l = c10::make_intrusive<ConvLayer>();
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b = b, l->wg = wg, l->bg = bg, l->staging = staging, l->stride = stride, l->split = split;
+  l->stack = stack, l->fuse_bias = fuse_bias, l->status = status;
+  return Conv3x3::apply(x, weight, bias, l);
+}
+
+// ------------------------------------------------------------------------------------------------ transposed 2x2 convolution
+struct ConvTLayer : torch::CustomClassHolder {
+  Tensor w_fwd, b4, wg, bg, staging, status;   // staging: fp32 [4, Cin, Cout], zero between uses
+  OptTensor w_dgrad;
+  int64_t split, stack;
+};
+
+struct ConvT2x2 : Function<ConvT2x2> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, const Held<ConvTLayer>& l) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor y = torch::empty({x.size(0), 2 * x.size(1), 2 * x.size(2), l->staging.size(2)}, x.options().dtype(torch::kBFloat16));
+    terra_ops::convt2x2(0, x.contiguous(), l->w_fwd, l->b4, y, l->status);
+    ctx->save_for_backward({x});
+    hold(ctx, l);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const auto l = held<ConvTLayer>(ctx);
+    const Tensor x = s[0].contiguous(), dy = grads[0].contiguous();
+    const c10::cuda::CUDAGuard guard(dy.device());
+    const int64_t cout = l->staging.size(2);
+    terra_ops::convt2x2_wgrad(x, dy, l->staging, l->split, l->status, l->stack);
+    terra_ops::strided_add(l->staging, l->wg, 1, cout * 4, 4, true);
+    terra_ops::colsum(dy.view({-1, cout}), l->bg);
+    Tensor dx;
+    if (l->w_dgrad.has_value()) {
+      dx = torch::empty(x.sizes(), x.options());
+      terra_ops::convt2x2(1, dy, *l->w_dgrad, c10::nullopt, dx, l->status);
+    }
+    return {dx, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor conv_transpose2x2(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad,
+                         const Tensor& b4, const Tensor& wg, const Tensor& bg, const Tensor& staging, int64_t split, int64_t stack,
+                         const Tensor& status) {
+  auto l = c10::make_intrusive<ConvTLayer>();
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->wg = wg, l->bg = bg, l->staging = staging, l->split = split, l->stack = stack;
+  l->status = status;
+  return ConvT2x2::apply(x, weight, bias, l);
+}
+
+// ------------------------------------------------------------------------------------------------ GroupNorm + SiLU
+struct NormLayer : torch::CustomClassHolder {
+  Tensor g, b, gg, bg, sums;                   // sums: fp32 [B, groups, 2], zero between uses
+  int64_t groups;
+  double eps;
+  bool has_res;
+};
+
+struct GroupNormSilu : Function<GroupNormSilu> {
+  static double inverse_count(const Tensor& x, int64_t groups) {
+    return 1.0 / (static_cast<double>(x.size(1)) * x.size(2) * (x.size(3) / groups));
+  }
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& gamma, const Tensor& beta, const OptTensor& residual,
+                        const Held<NormLayer>& l) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
+    const Tensor x3 = x.view(flat);
+    Tensor stats = torch::empty({x.size(0), l->groups, 2}, x.options().dtype(torch::kFloat32));
+    terra_ops::groupnorm_stats(x3, l->sums, l->groups);
+    terra_ops::groupnorm_finalize(l->sums, stats, inverse_count(x, l->groups), l->eps, true);
+    Tensor y = torch::empty_like(x), y3 = y.view(flat);
+    terra_ops::groupnorm_silu_apply(x3, stats, l->g, l->b, residual.has_value() ? OptTensor(residual->view(flat)) : residual, y3, l->groups);
+    ctx->save_for_backward({x, stats, l->g, l->b});
+    hold(ctx, l);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const auto l = held<NormLayer>(ctx);
+    const Tensor& x = s[0];
+    const Tensor dy = grads[0].contiguous();
+    const c10::cuda::CUDAGuard guard(dy.device());
+    const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
+    const Tensor x3 = x.view(flat), dy3 = dy.view(flat);
+    Tensor red = torch::zeros({x.size(0), x.size(3), 2}, x.options().dtype(torch::kFloat32));
+    terra_ops::groupnorm_silu_bwd_reduce(dy3, x3, s[1], s[2], s[3], red, l->groups, l->gg, l->bg);
+    Tensor dx = torch::empty_like(x), dx3 = dx.view(flat);
+    terra_ops::groupnorm_silu_bwd_apply(dy3, x3, s[1], red, s[2], s[3], dx3, l->groups, inverse_count(x, l->groups));
+    return {dx, Tensor(), Tensor(), l->has_res ? dy : Tensor(), Tensor()};
+  }
+};
+
+Tensor groupnorm_silu(const Tensor& x, const Tensor& gamma, const Tensor& beta, const OptTensor& residual, const Tensor& g, const Tensor& b,
+                      const Tensor& gg, const Tensor& bg, const Tensor& sums, int64_t groups, double eps) {
+  auto l = c10::make_intrusive<NormLayer>();
+  l->g = g, l->b = b, l->gg = gg, l->bg = bg, l->sums = sums, l->groups = groups, l->eps = eps, l->has_res = residual.has_value();
+  return GroupNormSilu::apply(x, gamma, beta, residual, l);
+}
+
+}  // namespace
+
+void bind_nodes(pybind11::module_& m) {
+  auto n = m.def_submodule("nodes", "layers as autograd nodes");
+  n.def("attn_half", &attn_half);
+  n.def("mlp_half", &mlp_half);
+  n.def("linear", &linear);
+  n.def("conv3x3", &conv3x3);
+  n.def("conv_transpose2x2", &conv_transpose2x2);
+  n.def("groupnorm_silu", &groupnorm_silu);
+}

@@ -8,6 +8,7 @@
 
 #include "check.h"
 #include "host_api.h"
+#include "torch_ops.h"
 #include "launch_count.h"
 
 namespace {
@@ -100,6 +101,10 @@ void gemm(const torch::Tensor& a, bool a_mn, const torch::Tensor& b, bool b_mn, 
     rc_check(rc, ("gemm (M=" + std::to_string(M) + " N=" + std::to_string(N) + " K=" + std::to_string(K) + ") launch").c_str());
 }
 
+}  // namespace
+
+namespace terra_ops {
+
 // x: [B,H,W,Cin] bf16 NHWC, w: [Cout, 9*Cin_pad] bf16, y: [B,Ho,Wo,Cout]
 void conv3x3_fwd(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor& y, int64_t stride, int64_t flags,
                  const c10::optional<torch::Tensor>& bias, const c10::optional<torch::Tensor>& residual,
@@ -150,15 +155,15 @@ void conv3x3_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tenso
   rc_check(rc, "conv3x3_wgrad");
 }
 
-void check_image(const torch::Tensor& t, const char* name) {
+static void check_image(const torch::Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.is_contiguous() && t.dim() == 4, name, ": NHWC bf16 contiguous");
 }
-void check_packed(const torch::Tensor& w, int64_t rows, int64_t taps, int64_t channels) {
+static void check_packed(const torch::Tensor& w, int64_t rows, int64_t taps, int64_t channels) {
   TORCH_CHECK(w.scalar_type() == torch::kBFloat16 && w.is_contiguous() && w.dim() == 2 && w.size(0) == rows &&
                   w.size(1) == taps * ((channels + 63) / 64 * 64),
               "packed weights: bf16 [rows, taps * channels padded to 64]");
 }
-void* status_ptr(const c10::optional<torch::Tensor>& s) { return s.has_value() ? s->data_ptr() : nullptr; }
+static void* status_ptr(const c10::optional<torch::Tensor>& s) { return s.has_value() ? s->data_ptr() : nullptr; }
 
 // dy: [B, Ho, Wo, Cout], dx: [B, H, W, Cin] with Ho = (H + 1) / 2, Wo = W / 2; w: [Cin, 9 * Cout_pad]
 void conv3x3_s2_dgrad(const torch::Tensor& dy, const torch::Tensor& w, torch::Tensor& dx,
@@ -214,11 +219,14 @@ void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tens
   rc_check(rc, "convt2x2_wgrad");
 }
 
-}  // namespace
+}  // namespace terra_ops
+
+using namespace terra_ops;
 
 void bind_elementwise(pybind11::module_& m);
 void bind_attention(pybind11::module_& m);
 void bind_halves(pybind11::module_& m);
+void bind_nodes(pybind11::module_& m);
 void bind_copy_engine(pybind11::module_& m);
 void bind_comm(pybind11::module_& m);
 
@@ -259,6 +267,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   bind_elementwise(m);
   bind_attention(m);
   bind_halves(m);
+  bind_nodes(m);
   bind_copy_engine(m);
   bind_comm(m);
 }

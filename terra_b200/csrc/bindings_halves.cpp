@@ -11,6 +11,7 @@
 #include "check.h"
 #include "host_api.h"
 #include "launch_count.h"
+#include "torch_ops.h"
 
 namespace {
 
@@ -145,6 +146,10 @@ WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   return best;
 }
 
+}  // namespace
+
+namespace terra_ops {
+
 // grad_w [N, K] (fp32) += dy [M, N]^T x [M, K]; grad_b [N] += column sums of dy, from the same kernel (`fuse_bias`: a
 // 16-column MMA of the dy tiles against ones) where its accumulators fit beside the tile's (widths up to 192).
 void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTensor& grad_b, bool fuse_bias, const Tensor& status) {
@@ -177,6 +182,12 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
   tb::note_launch();
   rc_check(tb::gemm_bf16(A, B, N, K, M, g, plan.split, plan.bn, sm_count(), cur_stream()), "gemm (weight gradient)");
 }
+
+}  // namespace terra_ops
+
+using namespace terra_ops;
+
+namespace {
 
 struct Norm {
   Tensor xn, mean, rstd;
@@ -233,6 +244,21 @@ tb::WindowAttnArgs window_args(const std::vector<int64_t>& g, int64_t C, const O
     a.bias_table = table->data_ptr<float>();
   }
   return a;
+}
+
+}  // namespace
+
+namespace terra_ops {
+
+// y [M, N] = x [M, K] W^T (+ bias) (+ residual), or with `transposed` dx = dy W
+Tensor linear_product(const Tensor& x, const Tensor& w, bool transposed, const OptTensor& bias, const OptTensor& residual, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor y = torch::empty({x.size(0), w.size(transposed ? 1 : 0)}, x.options());
+  Epi e;
+  if (bias.has_value()) e.bias = &*bias;
+  if (residual.has_value()) e.residual = &*residual;
+  product(x, w, transposed, y, e, status);
+  return y;
 }
 
 // -> y, mean, rstd, xn, qkv, o
@@ -319,7 +345,7 @@ Tensor mlp_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, const
   return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy);
 }
 
-}  // namespace
+}  // namespace terra_ops
 
 void bind_halves(pybind11::module_& m) {
   m.def(

@@ -5,6 +5,7 @@
 
 #include "check.h"
 #include "host_api.h"
+#include "torch_ops.h"
 #include "launch_count.h"
 
 namespace {
@@ -37,6 +38,10 @@ void layernorm_bwd(const torch::Tensor& dy, const torch::Tensor& x, const torch:
                              cur_stream()),
            "layernorm_bwd");
 }
+
+}  // namespace
+
+namespace terra_ops {
 
 void colsum(const torch::Tensor& x, torch::Tensor& out) {
   need(x.dim() == 2 && x.stride(1) == 1 && x.scalar_type() == torch::kBFloat16, "colsum: 2-D bf16");
@@ -117,6 +122,12 @@ void groupnorm_silu_bwd_apply(const torch::Tensor& dy, const torch::Tensor& x, c
                                         groups, static_cast<float>(inv_count), cur_stream()),
            "groupnorm_silu_bwd_apply");
 }
+
+}  // namespace terra_ops
+
+using namespace terra_ops;
+
+namespace {
 
 void masked_loss(const torch::Tensor& pred, const torch::Tensor& label, const c10::optional<torch::Tensor>& mask,
                  int64_t kind, double grad_scale, torch::Tensor& loss_sum, const c10::optional<torch::Tensor>& grad) {

@@ -88,6 +88,14 @@ def _views(p: torch.nn.Parameter):
     return p.bf16, p.grad
 
 
+def native_node(grads=()) -> bool:
+    """Whether a layer may be a node in C++: not while a trace is recorded or a function transform is active (the Python nodes
+    are recorded by the first and refuse the second), when single launches are to be observed, or without gradient
+    accumulators (which only a backward pass asks for)."""
+    return (not _LAUNCHES_OBSERVED and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
+            and all(g is not None for g in grads))
+
+
 def _native_half(comm, geo: WindowGeometry, impl: str) -> bool:
     """One native call runs the half when this rank owns every window and token and the small-window kernels are the
     selected ones (not in the bounds-checked build, whose reports go through the Python launches, nor when single launches
@@ -255,6 +263,14 @@ def attention_half(x, mod, geo: WindowGeometry, shifted: bool, comm=None):
         proj_w, proj_b = attn.proj.weight, attn.proj.bias
         qkv_w, qkv_b = fused["qkv_weight"], fused["qkv_bias"]
         table = attn.relative_position_bias_table if attn.use_relative_position_bias else None
+        grads = [ln_w.grad, ln_b.grad, qkv_w.grad, qkv_b.grad, proj_w.grad, proj_b.grad]
+        if (_native_half(comm, geo, attn_forward_impl(geo.N)) and native_node(grads)
+                and attn_backward_impl(geo.N, x.shape[1] // attn.num_heads) == "mma"):
+            return _ext.load().nodes.attn_half(
+                x, ln_w, [ln_w.bf16, ln_b.bf16, qkv_w.bf16, qkv_b.bf16, proj_w.bf16, proj_b.bf16], grads,
+                None if table is None else fp32_values(table), None if table is None else table.grad,
+                _native_geometry(geo, attn.num_heads, shifted, mod.use_attn_mask), attn.scale, LN_EPS, FUSE_BIAS_GRAD,
+                status_word(x.device))
         pk = ParamPack(
             ln_w=ln_w.bf16, ln_b=ln_b.bf16, ln_wg=ln_w.grad, ln_bg=ln_b.grad,
             qkv_w=qkv_w.bf16, qkv_b=qkv_b.bf16, qkv_wg=qkv_w.grad, qkv_bg=qkv_b.grad,
@@ -275,6 +291,10 @@ def mlp_half(x, mod):
     if x.is_cuda:
         ln_w, ln_b, fc1, fc2 = mod.norm2.weight, mod.norm2.bias, mod.fc1, mod.fc2
         w1, b1, w2, b2 = fc1.weight, fc1.bias, fc2.weight, fc2.bias
+        grads = [ln_w.grad, ln_b.grad, w1.grad, b1.grad, w2.grad, b2.grad]
+        if native_node(grads):
+            return _ext.load().nodes.mlp_half(x, ln_w, [ln_w.bf16, ln_b.bf16, w1.bf16, b1.bf16, w2.bf16, b2.bf16], grads, LN_EPS,
+                                              FUSE_BIAS_GRAD, status_word(x.device))
         pk = ParamPack(
             ln_w=ln_w.bf16, ln_b=ln_b.bf16, ln_wg=ln_w.grad, ln_bg=ln_b.grad,
             fc1_w=w1.bf16, fc1_b=b1.bf16, fc1_wg=w1.grad, fc1_bg=b1.grad,
@@ -289,6 +309,8 @@ def linear(x, lin: torch.nn.Linear, residual=None, need_dx=True):
     if x.is_cuda:
         w16, wg = _views(lin.weight)
         b16, bg = _views(lin.bias) if lin.bias is not None else (None, None)
+        if native_node((wg,)):
+            return _ext.load().nodes.linear(x, lin.weight, w16, b16, wg, bg, residual, need_dx, FUSE_BIAS_GRAD, status_word(x.device))
         return _LinearFn.apply(x, lin.weight, w16, b16, wg, bg, residual, need_dx)
     y = TF.linear(x, lin.weight, lin.bias)
     return y if residual is None else y + residual

@@ -26,7 +26,7 @@ from .. import _ext
 from . import _flags as F
 from .gemm import gemm, status_word
 from .packed import PACK_EPOCH, _packed, fp32_values, invalidate_packed_weights  # noqa: F401  (re-exported)
-from .blocks import FUSE_BIAS_GRAD, wgrad_accumulate, bias_grad_accumulate
+from .blocks import FUSE_BIAS_GRAD, native_node, wgrad_accumulate, bias_grad_accumulate
 from ..utils.nvtx import nvtx_range
 
 GN_EPS = 1e-5
@@ -230,11 +230,38 @@ def _conv3x3_s2_dgrad(dy, w16, H, W, dom, weight=None):
     return out
 
 
+def _layer_grads(a, b):
+    """The arena gradients of two parameters where a native node may stand for their layer, else None."""
+    if not native_node():
+        return None
+    ga, gb = _arena_grad(a), _arena_grad(b)
+    return None if ga is None or gb is None else (ga, gb)
+
+
+def _conv3x3_node(x, weight, bias, stride, dom):
+    """The convolution of one rank as a native autograd node; None where it is not one."""
+    grads = None if dom is not None and dom.world > 1 else _layer_grads(weight, bias)
+    if grads is None or x.dim() != 4:
+        return None
+    ext = _ext.load()
+    (B, H, W, Cin), Cout, w16 = x.shape, weight.shape[0], weight.bf16
+    if stride != 1 and not (9 * ((Cout + 63) // 64) <= _MAX_TAP_CHUNKS and ext.gemm_tma_epilogue()):
+        return None
+    wd = None
+    if x.requires_grad and torch.is_grad_enabled():
+        wd = _packed(weight, w16, "dgrad", pack_conv3x3_weight_dgrad) if stride == 1 else \
+            _packed(weight, w16, "s2dgrad_taps", pack_conv3x3_weight_s2_dgrad)
+    split, stack = _wgrad_split(B, H, W, stride, Cout, Cin)
+    return ext.nodes.conv3x3(x, weight, bias, _packed(weight, w16, "fwd", pack_conv3x3_weight), wd, bias.bf16, *grads,
+                             _zero_scratch(x.device, (9, Cout, Cin), "conv3x3"), stride, split, stack, FUSE_BIAS_GRAD, status_word(x.device))
+
+
 @nvtx_range("terra.conv3x3")
 def conv3x3(x, conv: torch.nn.Conv2d, stride: int = 1, dom=None):
     """x NHWC -> NHWC. ``conv`` holds a (Cout, Cin, 3, 3) weight and a bias."""
     if x.is_cuda:
-        return _Conv3x3Fn.apply(x, conv.weight, conv.bias, stride, dom)
+        y = _conv3x3_node(x, conv.weight, conv.bias, stride, dom)
+        return _Conv3x3Fn.apply(x, conv.weight, conv.bias, stride, dom) if y is None else y
     xin = x.permute(0, 3, 1, 2)
     if dom is not None and dom.world > 1:
         xin = dom.halo_exchange_cpu(xin, 1)
@@ -268,10 +295,8 @@ class _ConvT2x2Fn(torch.autograd.Function):
         b16 = bias.bf16 if getattr(bias, "bf16", None) is not None else bias.detach().to(torch.bfloat16)
         y = torch.empty(B, 2 * H, 2 * W, Cout, device=x.device, dtype=torch.bfloat16)
         if _convt_tiled(B, H, W, Cin, Cout):
-            # rows (dy, dx, co), every phase padded to whole units of the epilogue, which stores it to its pixels
-            pad = (Cout + 63) // 64 * 64
-            wt = _packed(weight, w16, "convT", lambda w: _pack_taps(w, 4, 1, Cout, 4, Cin, 4 * Cout, (0,), pad))
-            b4 = _packed(bias, b16, "convT_bias", lambda b: TF.pad(b, (0, pad - Cout)).repeat(4))
+            wt = _packed(weight, w16, "convT", _pack_convt)
+            b4 = _packed(bias, b16, "convT_bias", _pack_convt_bias)
             ext.convt2x2(0, x.contiguous(), wt, b4, y, status_word(x.device))
         else:
             b4 = _packed(bias, b16, "convT_bias_flat", lambda b: b.repeat(4))
@@ -319,11 +344,41 @@ class _ConvT2x2Fn(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             if tiled:
                 dx = torch.empty(B, H, W, Cin, device=x.device, dtype=torch.bfloat16)
-                wd = _packed(weight, w16, "convT_dgrad", lambda w: _pack_taps(w, 1, 0, Cin, 4 * Cout, Cout, 4, range(4)))
+                wd = _packed(weight, w16, "convT_dgrad", _pack_convt_dgrad)
                 ext.convt2x2(1, dy, wd, None, dx, status_word(x.device))
             else:
                 dx = gemm(dyu, _convt_flat_weight(weight, w16), b_mn=True).view(B, H, W, Cin)
         return dx, dw, db
+
+
+def _pack_convt(w):
+    """Rows (dy, dx, co), every phase padded to whole units of the epilogue, which stores it to its pixels."""
+    cin, cout = w.shape[:2]
+    return _pack_taps(w, 4, 1, cout, 4, cin, 4 * cout, (0,), (cout + 63) // 64 * 64)
+
+
+def _pack_convt_bias(b):
+    return TF.pad(b, (0, -b.shape[0] % 64)).repeat(4)
+
+
+def _pack_convt_dgrad(w):
+    cin, cout = w.shape[:2]
+    return _pack_taps(w, 1, 0, cin, 4 * cout, cout, 4, range(4))
+
+
+def _conv_transpose2x2_node(x, weight, bias):
+    """The transposed convolution as a native autograd node (the gathered forms); None where it is not one."""
+    grads = _layer_grads(weight, bias)
+    if grads is None or x.dim() != 4:
+        return None
+    (B, H, W, Cin), Cout, w16 = x.shape, weight.shape[1], weight.bf16
+    if not _convt_tiled(B, H, W, Cin, Cout):
+        return None
+    wd = _packed(weight, w16, "convT_dgrad", _pack_convt_dgrad) if x.requires_grad and torch.is_grad_enabled() else None
+    split, stack = _wgrad_plan(4, Cin, Cout, B * H * ((W + 63) // 64))
+    return _ext.load().nodes.conv_transpose2x2(
+        x, weight, bias, _packed(weight, w16, "convT", _pack_convt), wd, _packed(bias, bias.bf16, "convT_bias", _pack_convt_bias), *grads,
+        _zero_scratch(x.device, (4, Cin, Cout), "convT"), split, stack, status_word(x.device))
 
 
 def _convt_flat_weight(weight, w16):
@@ -334,7 +389,8 @@ def _convt_flat_weight(weight, w16):
 
 def conv_transpose2x2(x, convt: torch.nn.ConvTranspose2d):
     if x.is_cuda:
-        return _ConvT2x2Fn.apply(x, convt.weight, convt.bias)
+        y = _conv_transpose2x2_node(x, convt.weight, convt.bias)
+        return _ConvT2x2Fn.apply(x, convt.weight, convt.bias) if y is None else y
     return TF.conv_transpose2d(x.permute(0, 3, 1, 2), convt.weight, convt.bias, stride=2).permute(0, 2, 3, 1)
 
 
@@ -393,6 +449,11 @@ class _GroupNormSiluFn(torch.autograd.Function):
 def groupnorm_silu(x, gn: torch.nn.GroupNorm, residual=None, dom=None):
     """silu(group_norm(x)) [+ residual] on NHWC; statistics span the whole (global) image."""
     if x.is_cuda:
+        grads = None if dom is not None and dom.world > 1 else _layer_grads(gn.weight, gn.bias)
+        if grads is not None and x.dim() == 4:
+            return _ext.load().nodes.groupnorm_silu(
+                x, gn.weight, gn.bias, residual, gn.weight.bf16, gn.bias.bf16, *grads,
+                _zero_scratch(x.device, (x.shape[0], gn.num_groups, 2), "gn_sums"), gn.num_groups, GN_EPS)
         return _GroupNormSiluFn.apply(x, gn.weight, gn.bias, residual, gn.num_groups, dom)
     xc = x.permute(0, 3, 1, 2)
     if dom is not None and dom.world > 1:

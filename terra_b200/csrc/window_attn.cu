@@ -23,8 +23,14 @@
 //     shared memory allows it); the token tables are computed two windows ahead;
 //   * a window's results are staged over its own dead operand rows and leave as 16-byte vectors, warp by warp.
 //   * elementwise work on neighbouring columns goes through the two-wide fp32 instructions.
-// 2176 shifted windows of 8 x 8, 12 heads of 32 channels: forward 105 us (a version with four-warp blocks that walked over
-// heads and looked every bias up took 324 us; 66 us of HBM traffic), backward 246 us (586 us; 115 us).
+//   * where a block holds two heads (forward, 16 and 32 channels) a warp takes 32 rows of one head, not 16 of both: two independent
+//     chains to issue from, and half the reads of K and V through the shared-memory port;
+//   * accumulator tiles go to shared memory four 8 x 8 tiles an instruction;
+//   * windows of at most 32 tokens have blocks of their own size, and padding columns cost a comparison, not the masked form.
+// Us, before these three / now (shifted, with bias): 2176 windows of 8 x 8, 12 heads of 32 channels, forward 105 / 92 (66 of HBM
+// traffic), backward 236 / 233 (115); 2448 of 8 x 8, 8 heads of 128 channels 237 / 233 and 626 / 608; 180 of 8 x 12, 12 heads of 16
+// channels 26 / 25 and 50 / 49; 1020 of 7 x 7, 12 heads of 32 channels 93 / 57 and 140 / 119; 1800 of 4 x 8, 8 heads of 32 channels
+// 89 / 25 and 120 / 54. What is left is issue and latency: the shared-memory port is busy 50 (forward) and 70 % (backward) of the time.
 #include <atomic>
 #include "chained_launch.cuh"
 #include "common.cuh"
@@ -51,6 +57,12 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
                : "r"(smem_u32(p)));
 }
 
+// four 8 x 8 tiles of the accumulator layout (bf16 pairs) to rows of shared memory, lane l giving the address of row l & 7 of tile l >> 3
+__device__ __forceinline__ void stsm_x4(void* p, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(p)), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+               : "memory");
+}
+
 // 16-byte asynchronous copy global -> shared
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -67,6 +79,7 @@ struct WaCfg {
   static constexpr int PITCH = G + 8;
   static constexpr int PP = NPAD + 8;                            // pitch of the P / dS stash (backward)
   static constexpr int THREADS = NPAD * 2;                       // a warp per 16 rows
+  static constexpr int MT = !BWD && HPC == 2 ? 2 : 1;            // 16-row tiles of a warp (two: half of the warps per head)
   static constexpr int MATS = BWD ? 4 : 3;                       // q, k, v [, dO]
   static constexpr int MAT = NPAD * PITCH;                       // elements
   static constexpr int STAGE = MATS * MAT;
@@ -74,20 +87,21 @@ struct WaCfg {
   // dQ is staged in the warp's own stash rows before P and dS go there; a 128-channel head does not fit into them
   static constexpr bool DQ_IN_STASH = HD <= NPAD;
   static constexpr int DQ = (BWD && !DQ_IN_STASH) ? MAT : 0;
-  static constexpr bool ACC_REGS = NPAD == 64;                   // bias-gradient sums: registers or shared memory
+  static constexpr bool ACC_REGS = NPAD <= 64;                   // bias-gradient sums: registers or shared memory
   static constexpr int ACC = (BWD && !ACC_REGS) ? NPAD * NPAD : 0;   // floats
   static constexpr int FIXED = (STASH + DQ) * 2 + ACC * 4 + 3 * NPAD * 8 + NPAD * 4;
   // Resident CTAs that shared memory allows, with the kilobyte that every CTA reserves and a small bias table (that of an 8 x 8
   // window makes three of four where 64 channels are staged). Two stages where three (two for windows above 64 tokens) fit.
   static constexpr int fits(int stages) { return 228 * 1024 / (FIXED + stages * STAGE * 2 + 1024); }
-  static constexpr int STAGES = fits(2) >= (NPAD == 64 ? 3 : 2) ? 2 : 1;
+  static constexpr int STAGES = fits(2) >= (NPAD <= 64 ? 3 : 2) ? 2 : 1;
   static constexpr size_t bytes(int nrel) { return static_cast<size_t>(FIXED) + STAGES * STAGE * 2 + HPC * nrel * 4; }
   // Resident CTAs asked of the compiler, which bounds the registers per thread: no more than shared memory allows. (Asked for
   // five where two stages of 64 channels let four or three fit, the compiler spilled for nothing: 2176 windows of 8 x 8, 12 heads
   // of 32 channels, forward without / with shift 116 / 125 us, for four 96 / 105. For three it would be 94 / 103, but then
   // 4 x 4 windows lose the fourth: 6 heads of 64 channels 67 / 71 us, for four 65 / 70, for three 75 / 80. One stage and five
   // CTAs: 100 / 109.)
-  static constexpr int WANTED = NPAD > 96 ? 1 : (BWD ? (NPAD > 64 ? (HD > 64 ? 1 : 2) : (HD > 64 ? 2 : 3))
+  // (Two tiles a warp: three blocks of 160 registers instead of four of 128, 96 / 102 us for the 2176 windows above.)
+  static constexpr int WANTED = MT == 2 && NPAD <= 64 ? (NPAD == 64 ? 3 : 8) : NPAD == 32 ? (BWD ? (HD > 64 ? 4 : 6) : 8) : NPAD > 96 ? 1 : (BWD ? (NPAD > 64 ? (HD > 64 ? 1 : 2) : (HD > 64 ? 2 : 3))
                                                      : (NPAD > 64 ? 2 : (HD > 64 ? 4 : 5)));
   // (128-token windows of 128-channel heads do not fit backward at all: their launch is refused)
   static constexpr int MIN_CTAS = fits(STAGES) < 1 ? 1 : (WANTED < fits(STAGES) ? WANTED : fits(STAGES));
@@ -184,119 +198,158 @@ __device__ __forceinline__ void wa_set(float (&v)[4], int i, f32x2 x) { f2_unpac
 // cofs(r) - cofs(c) + rel0 with cofs(t) = (t / ww) (2 ww - 1) + t % ww. For windows 8 (12) wide the columns of a thread
 // repeat every 1 (3) blocks of 8, so an index is one of 1 (3) per-thread bases plus a compile-time constant; other
 // widths read cofs from shared memory.
-template <int NPAD, int WW>
-__device__ __forceinline__ void wa_scores(float (&s)[NPAD / 8][4], float scale2, const float* tb, int rel0, const int* cofs,
-                                          const int2* tab, int r0, int tq, int N, bool general, bool use_mask, float& mx0,
-                                          float& mx1) {
-  const int r1 = r0 + 8;
+// A warp's block is MT tiles of 16 rows (rows r0 + 16 t and r0 + 16 t + 8 of this thread).
+template <int NPAD, int WW, int MT>
+__device__ __forceinline__ void wa_scores(float (&s)[MT][NPAD / 8][4], float scale2, const float* tb, int rel0, const int* cofs,
+                                          const int2* tab, int r0, int tq, int N, bool general, bool use_mask, float (&mx)[MT][2]) {
   if (!general) {
     if constexpr (WW == 8) {
-      // row r1 = r0 + 8 is the next window row, same column: its bias at key block nb is row r0's at block nb - 1
+      // row r0 + 8 is the next window row, same column: its bias at key block nb is row r0's at block nb - 1, and so on for the rows below
       const float* p = tb + ((r0 >> 3) * 15 + (r0 & 7) - 2 * tq + rel0);
-      float b0 = p[15], b1 = p[14];
+      float b[2 * MT][2];      // this key block's bias of rows r0, r0 + 8, ...
+#pragma unroll
+      for (int i = 1; i < 2 * MT; ++i) b[i][0] = p[15 * i], b[i][1] = p[15 * i - 1];
 #pragma unroll
       for (int nb = 0; nb < NPAD / 8; ++nb) {
-        wa_set(s[nb], 2, f2_fma(wa_pair(s[nb], 2), f2_both(scale2), f2_pack(b0, b1)));
-        b0 = p[-15 * nb];
-        b1 = p[-15 * nb - 1];
-        wa_set(s[nb], 0, f2_fma(wa_pair(s[nb], 0), f2_both(scale2), f2_pack(b0, b1)));
-        mx0 = fmaxf(mx0, fmaxf(s[nb][0], s[nb][1]));
-        mx1 = fmaxf(mx1, fmaxf(s[nb][2], s[nb][3]));
+        b[0][0] = p[-15 * nb];
+        b[0][1] = p[-15 * nb - 1];
+#pragma unroll
+        for (int t = 0; t < MT; ++t)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            wa_set(s[t][nb], 2 * h, f2_fma(wa_pair(s[t][nb], 2 * h), f2_both(scale2), f2_pack(b[2 * t + h][0], b[2 * t + h][1])));
+            mx[t][h] = fmaxf(mx[t][h], fmaxf(s[t][nb][2 * h], s[t][nb][2 * h + 1]));
+          }
+#pragma unroll
+        for (int i = 2 * MT - 1; i > 0; --i) b[i][0] = b[i - 1][0], b[i][1] = b[i - 1][1];
       }
     } else if constexpr (WW == 12) {
-      const int ro0 = cofs[r0] + rel0, dr = cofs[r1] - cofs[r0];
-      // columns 8 m + 2 tq of the first three blocks, m = 0, 1, 2; later blocks are whole window rows (2 per 3 blocks) on
-      const float* p[3];
-      p[0] = tb + ro0 - 2 * tq;
-      p[1] = tb + ro0 - (tq < 2 ? 8 + 2 * tq : 23 + 2 * tq - 4);
-      p[2] = tb + ro0 - (23 + 4 + 2 * tq);
 #pragma unroll
-      for (int nb = 0; nb < NPAD / 8; ++nb) {
-        const float* c = p[nb % 3] - (nb / 3) * 46;
-        wa_set(s[nb], 0, f2_fma(wa_pair(s[nb], 0), f2_both(scale2), f2_pack(c[0], c[-1])));
-        wa_set(s[nb], 2, f2_fma(wa_pair(s[nb], 2), f2_both(scale2), f2_pack(c[dr], c[dr - 1])));
-        mx0 = fmaxf(mx0, fmaxf(s[nb][0], s[nb][1]));
-        mx1 = fmaxf(mx1, fmaxf(s[nb][2], s[nb][3]));
+      for (int t = 0; t < MT; ++t) {
+        const int ra = r0 + 16 * t;
+        const int ro0 = cofs[ra] + rel0, dr = cofs[ra + 8] - cofs[ra];
+        // columns 8 m + 2 tq of the first three blocks, m = 0, 1, 2; later blocks are whole window rows (2 per 3 blocks) on
+        const float* p[3];
+        p[0] = tb + ro0 - 2 * tq;
+        p[1] = tb + ro0 - (tq < 2 ? 8 + 2 * tq : 23 + 2 * tq - 4);
+        p[2] = tb + ro0 - (23 + 4 + 2 * tq);
+#pragma unroll
+        for (int nb = 0; nb < NPAD / 8; ++nb) {
+          const float* c = p[nb % 3] - (nb / 3) * 46;
+          wa_set(s[t][nb], 0, f2_fma(wa_pair(s[t][nb], 0), f2_both(scale2), f2_pack(c[0], c[-1])));
+          wa_set(s[t][nb], 2, f2_fma(wa_pair(s[t][nb], 2), f2_both(scale2), f2_pack(c[dr], c[dr - 1])));
+          mx[t][0] = fmaxf(mx[t][0], fmaxf(s[t][nb][0], s[t][nb][1]));
+          mx[t][1] = fmaxf(mx[t][1], fmaxf(s[t][nb][2], s[t][nb][3]));
+        }
       }
     } else {
-      const float *t0 = tb + cofs[r0] + rel0, *t1 = tb + cofs[r1] + rel0;
 #pragma unroll
-      for (int nb = 0; nb < NPAD / 8; ++nb) {
-        const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
-        s[nb][0] = fmaf(s[nb][0], scale2, t0[-co.x]);
-        s[nb][1] = fmaf(s[nb][1], scale2, t0[-co.y]);
-        s[nb][2] = fmaf(s[nb][2], scale2, t1[-co.x]);
-        s[nb][3] = fmaf(s[nb][3], scale2, t1[-co.y]);
-        mx0 = fmaxf(mx0, fmaxf(s[nb][0], s[nb][1]));
-        mx1 = fmaxf(mx1, fmaxf(s[nb][2], s[nb][3]));
+      for (int t = 0; t < MT; ++t) {
+        const float *t0 = tb + cofs[r0 + 16 * t] + rel0, *t1 = tb + cofs[r0 + 16 * t + 8] + rel0;
+#pragma unroll
+        for (int nb = 0; nb < NPAD / 8; ++nb) {
+          const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
+          s[t][nb][0] = fmaf(s[t][nb][0], scale2, t0[-co.x]);
+          s[t][nb][1] = fmaf(s[t][nb][1], scale2, t0[-co.y]);
+          s[t][nb][2] = fmaf(s[t][nb][2], scale2, t1[-co.x]);
+          s[t][nb][3] = fmaf(s[t][nb][3], scale2, t1[-co.y]);
+          if (nb * 8 + 8 > N) {      // padding columns: their scores are lowest, their probabilities zero
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (nb * 8 + tq * 2 + (k & 1) >= N) s[t][nb][k] = -1e30f;
+          }
+          mx[t][0] = fmaxf(mx[t][0], fmaxf(s[t][nb][0], s[t][nb][1]));
+          mx[t][1] = fmaxf(mx[t][1], fmaxf(s[t][nb][2], s[t][nb][3]));
+        }
       }
     }
   } else {
-    // windows that the mask cuts, and windows with padding columns (their scores are lowest, their probabilities zero)
-    const int reg0 = tab[r0].y >> 8, reg1 = tab[r1].y >> 8;
-    const bool row0 = r0 < N, row1 = r1 < N;
-    const float *t0 = tb + (row0 ? cofs[r0] + rel0 : 0), *t1 = tb + (row1 ? cofs[r1] + rel0 : 0);
+    // windows that the mask cuts
 #pragma unroll
-    for (int nb = 0; nb < NPAD / 8; ++nb) {
-      const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
+    for (int t = 0; t < MT; ++t) {
+      const int ra = r0 + 16 * t, rb = ra + 8;
+      const int reg0 = tab[ra].y >> 8, reg1 = tab[rb].y >> 8;
+      const bool row0 = ra < N, row1 = rb < N;
+      const float *t0 = tb + (row0 ? cofs[ra] + rel0 : 0), *t1 = tb + (row1 ? cofs[rb] + rel0 : 0);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int col = nb * 8 + tq * 2 + (k & 1);
-        const bool lo = k < 2;
-        float v = s[nb][k] * scale2;
-        if (col < N) {
-          if (lo ? row0 : row1) v += (lo ? t0 : t1)[-((k & 1) ? co.y : co.x)];
-          if (use_mask && (tab[col].y >> 8) != (lo ? reg0 : reg1)) v += -100.f * WA_LOG2E;
-        } else {
-          v = -1e30f;
+      for (int nb = 0; nb < NPAD / 8; ++nb) {
+        const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int col = nb * 8 + tq * 2 + (k & 1);
+          const bool lo = k < 2;
+          float v = s[t][nb][k] * scale2;
+          if (col < N) {
+            if (lo ? row0 : row1) v += (lo ? t0 : t1)[-((k & 1) ? co.y : co.x)];
+            if (use_mask && (tab[col].y >> 8) != (lo ? reg0 : reg1)) v += -100.f * WA_LOG2E;
+          } else {
+            v = -1e30f;
+          }
+          s[t][nb][k] = v;
+          mx[t][lo ? 0 : 1] = fmaxf(mx[t][lo ? 0 : 1], v);
         }
-        s[nb][k] = v;
-        if (lo) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
       }
     }
   }
 }
 
-// d[nb] += A(16 rows at `arow`, HD channels) * B(NPAD rows at `bmat`)^T, both row-major bf16 in shared memory
-template <int HD, int NPAD, int PITCH>
-__device__ __forceinline__ void wa_mma_nt(float (&d)[NPAD / 8][4], const __nv_bfloat16* arow, const __nv_bfloat16* bmat, int lane) {
+// d[t] = A(16 rows at `arow` + 16 t, HD channels) * B(NPAD rows at `bmat`)^T, both row-major bf16 in shared memory
+template <int HD, int NPAD, int PITCH, int MT>
+__device__ __forceinline__ void wa_mma_nt(float (&d)[MT][NPAD / 8][4], const __nv_bfloat16* arow, const __nv_bfloat16* bmat, int lane) {
 #pragma unroll
-  for (int nb = 0; nb < NPAD / 8; ++nb)
+  for (int t = 0; t < MT; ++t)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) d[nb][k] = 0.f;
+    for (int nb = 0; nb < NPAD / 8; ++nb)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) d[t][nb][k] = 0.f;
 #pragma unroll
   for (int kk = 0; kk < HD / 16; ++kk) {
-    uint32_t af[4];
-    ldsm_x4(af, arow + (lane & 15) * PITCH + kk * 16 + (lane >> 4) * 8);
+    uint32_t af[MT][4];
+#pragma unroll
+    for (int t = 0; t < MT; ++t) ldsm_x4(af[t], arow + (16 * t + (lane & 15)) * PITCH + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
     for (int nb = 0; nb < NPAD / 8; nb += 2) {
       uint32_t bf[4];
       ldsm_x4(bf, bmat + (nb * 8 + (lane & 7) + (lane >> 4) * 8) * PITCH + kk * 16 + ((lane >> 3) & 1) * 8);
       const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
-      mma_bf16_16816(d[nb], af, b0);
-      mma_bf16_16816(d[nb + 1], af, b1);
+#pragma unroll
+      for (int t = 0; t < MT; ++t) {
+        mma_bf16_16816(d[t][nb], af[t], b0);
+        mma_bf16_16816(d[t][nb + 1], af[t], b1);
+      }
     }
   }
 }
 
-// o = P (16 x NPAD, fp32 accumulator layout, rounded to bf16) * B (NPAD rows, HD channels, row-major in shared memory)
-template <int HD, int NPAD, int PITCH>
-__device__ __forceinline__ void wa_mma_pn(float (&o)[HD / 8][4], const float (&p)[NPAD / 8][4], const __nv_bfloat16* bmat, int lane) {
+// o[t] = P[t] (16 x NPAD, fp32 accumulator layout, rounded to bf16) * B (NPAD rows, HD channels, row-major in shared memory)
+template <int HD, int NPAD, int PITCH, int MT>
+__device__ __forceinline__ void wa_mma_pn(float (&o)[MT][HD / 8][4], const float (&p)[MT][NPAD / 8][4], const __nv_bfloat16* bmat, int lane) {
 #pragma unroll
-  for (int nb = 0; nb < HD / 8; ++nb)
+  for (int t = 0; t < MT; ++t)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) o[nb][k] = 0.f;
+    for (int nb = 0; nb < HD / 8; ++nb)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[t][nb][k] = 0.f;
 #pragma unroll
   for (int j = 0; j < NPAD / 16; ++j) {
-    const uint32_t pf[4] = {pack_bf16x2(p[2 * j][0], p[2 * j][1]), pack_bf16x2(p[2 * j][2], p[2 * j][3]),
-                            pack_bf16x2(p[2 * j + 1][0], p[2 * j + 1][1]), pack_bf16x2(p[2 * j + 1][2], p[2 * j + 1][3])};
+    uint32_t pf[MT][4];
+#pragma unroll
+    for (int t = 0; t < MT; ++t) {
+      pf[t][0] = pack_bf16x2(p[t][2 * j][0], p[t][2 * j][1]);
+      pf[t][1] = pack_bf16x2(p[t][2 * j][2], p[t][2 * j][3]);
+      pf[t][2] = pack_bf16x2(p[t][2 * j + 1][0], p[t][2 * j + 1][1]);
+      pf[t][3] = pack_bf16x2(p[t][2 * j + 1][2], p[t][2 * j + 1][3]);
+    }
 #pragma unroll
     for (int nb = 0; nb < HD / 8; nb += 2) {
       uint32_t bf[4];
       ldsm_x4_t(bf, bmat + (j * 16 + (lane & 15)) * PITCH + nb * 8 + (lane >> 4) * 8);
       const uint32_t b0[2] = {bf[0], bf[1]}, b1[2] = {bf[2], bf[3]};
-      mma_bf16_16816(o[nb], pf, b0);
-      mma_bf16_16816(o[nb + 1], pf, b1);
+#pragma unroll
+      for (int t = 0; t < MT; ++t) {
+        mma_bf16_16816(o[t][nb], pf[t], b0);
+        mma_bf16_16816(o[t][nb + 1], pf[t], b1);
+      }
     }
   }
 }
@@ -331,14 +384,23 @@ __device__ __forceinline__ void wa_softmax(float (&s)[NPAD / 8][4], float mx0, f
   inv1 = 1.f / sum1;
 }
 
-// A warp's 16 x HD accumulator tile, scaled per row, to bf16 rows in shared memory (rows r0 = gq and r0 + 8 of the tile).
-template <int HD>
-__device__ __forceinline__ void wa_stage(__nv_bfloat16* dst, int pitch, const float (&o)[HD / 8][4], float f0, float f1, int gq,
-                                         int tq, bool ok0, bool ok1) {
+// A warp's 16 x W accumulator tile, scaled per row (r0 = gq and r0 + 8), to bf16 rows in shared memory.
+template <int W>
+__device__ __forceinline__ void wa_stage(__nv_bfloat16* dst, int pitch, const float (&o)[W / 8][4], float f0, float f1, int lane) {
+  __nv_bfloat16* at = dst + (lane & 15) * pitch + (lane >> 4) * 8;
 #pragma unroll
-  for (int nb = 0; nb < HD / 8; ++nb) {
-    if (ok0) *reinterpret_cast<uint32_t*>(dst + gq * pitch + nb * 8 + tq * 2) = pack_bf16x2(o[nb][0] * f0, o[nb][1] * f0);
-    if (ok1) *reinterpret_cast<uint32_t*>(dst + (gq + 8) * pitch + nb * 8 + tq * 2) = pack_bf16x2(o[nb][2] * f1, o[nb][3] * f1);
+  for (int nb = 0; nb < W / 8; nb += 2)
+    stsm_x4(at + nb * 8, pack_bf16x2(o[nb][0] * f0, o[nb][1] * f0), pack_bf16x2(o[nb][2] * f1, o[nb][3] * f1),
+            pack_bf16x2(o[nb + 1][0] * f0, o[nb + 1][1] * f0), pack_bf16x2(o[nb + 1][2] * f1, o[nb + 1][3] * f1));
+}
+// The same where rows may be padding, which stays as it is (K and V rows of later windows must find zeros there).
+template <int W>
+__device__ __forceinline__ void wa_stage_rows(__nv_bfloat16* dst, int pitch, const float (&o)[W / 8][4], float f, int lane, bool ok0, bool ok1) {
+  const int gq = lane >> 2, tq = lane & 3;
+#pragma unroll
+  for (int nb = 0; nb < W / 8; ++nb) {
+    if (ok0) *reinterpret_cast<uint32_t*>(dst + gq * pitch + nb * 8 + tq * 2) = pack_bf16x2(o[nb][0] * f, o[nb][1] * f);
+    if (ok1) *reinterpret_cast<uint32_t*>(dst + (gq + 8) * pitch + nb * 8 + tq * 2) = pack_bf16x2(o[nb][2] * f, o[nb][3] * f);
   }
 }
 
@@ -347,7 +409,7 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
     window_attn_kernel(const __grid_constant__ WindowAttnArgs a) {
   using Cfg = WaCfg<HD, NPAD, HPC, BWD>;
   static_assert(!BWD || HPC == 1, "the backward kernel keeps one head's bias-gradient sums");
-  constexpr int G = Cfg::G, PITCH = Cfg::PITCH, PP = Cfg::PP, STAGES = Cfg::STAGES, NB = NPAD / 8;
+  constexpr int G = Cfg::G, PITCH = Cfg::PITCH, PP = Cfg::PP, STAGES = Cfg::STAGES, NB = NPAD / 8, MT = Cfg::MT;
   extern __shared__ __align__(16) uint8_t smem[];
   __nv_bfloat16* stages = reinterpret_cast<__nv_bfloat16*>(smem);
   __nv_bfloat16* Ps = stages + STAGES * Cfg::STAGE;             // backward: [NPAD][PP] each
@@ -378,7 +440,7 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
   const int ti = tid / a.ww, tj = tid % a.ww;                    // token `tid` of a window
 
   if (tid < NPAD) {
-    cofs[tid] = ti * (2 * a.ww - 1) + tj;
+    cofs[tid] = tid < N ? ti * (2 * a.ww - 1) + tj : 0;      // (a padding token's bias is read, from inside the table, and not used)
     if (tid >= N)
       for (int k = 0; k < 3; ++k) tabs[k * NPAD + tid] = make_int2(-1, 15 << 8);
   }
@@ -396,8 +458,8 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
     for (int k = 0; k < 4; ++k) acc[nb][k] = 0.f;
 
   const int step = gridDim.x;
-  const int row0 = warp * 16, r0 = row0 + gq, r1 = r0 + 8;
-  const bool in0 = r0 < N, in1 = r1 < N;
+  const int my_head = MT == 1 ? 0 : warp / (NPAD / (16 * MT));
+  const int row0 = (MT == 1 ? warp : warp % (NPAD / (16 * MT))) * 16 * MT, r0 = row0 + gq, r1 = r0 + 8;
   const float own0 = (r0 >= q0 && r0 < q1) ? 1.f : 0.f, own1 = (r1 >= q0 && r1 < q1) ? 1.f : 0.f;   // this rank's query rows
 
   WaItem next = wa_item(a, blockIdx.x, my_nw);      // the item whose table was written last
@@ -435,36 +497,47 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
       next = wa_item(a, item + 2 * step, my_nw);
       if (tid < N) wa_table(a, geo, next, ti, tj, tabs + slot2 * NPAD + tid);
     }
-    const bool general = N != NPAD || (a.use_mask && ((a.sh > 0 && mine.ii == a.nWh - 1) || (a.sw > 0 && mine.jj == a.nWw - 1)));
+    const bool general = (WW != 0 && N != NPAD) || (a.use_mask && ((a.sh > 0 && mine.ii == a.nWh - 1) || (a.sw > 0 && mine.jj == a.nWw - 1)));
 
     if constexpr (!BWD) {
-      if (row0 < q1 && row0 + 16 > q0) {
+      if (row0 < q1 && row0 + 16 * MT > q0) {
 #pragma unroll 1
-        for (int hh = 0; hh < HPC; ++hh) {
-          float s[NB][4];
-          wa_mma_nt<HD, NPAD, PITCH>(s, Qs + row0 * PITCH + hh * HD, Ks + hh * HD, lane);
-          float mx0 = -1e30f, mx1 = -1e30f, inv0, inv1;
-          wa_scores<NPAD, WW>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx0, mx1);
-          wa_softmax<NPAD>(s, mx0, mx1, inv0, inv1);
+        for (int hh = MT == 1 ? 0 : my_head; hh < (MT == 1 ? HPC : my_head + 1); ++hh) {
+          float s[MT][NB][4];
+          wa_mma_nt<HD, NPAD, PITCH, MT>(s, Qs + row0 * PITCH + hh * HD, Ks + hh * HD, lane);
+          float mx[MT][2], inv[MT][2];
+#pragma unroll
+          for (int t = 0; t < MT; ++t) mx[t][0] = mx[t][1] = -1e30f;
+          wa_scores<NPAD, WW, MT>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx);
+#pragma unroll
+          for (int t = 0; t < MT; ++t) wa_softmax<NPAD>(s[t], mx[t][0], mx[t][1], inv[t][0], inv[t][1]);
           // O = P V with the numerators as P, the row normalisation applied to the (smaller) output; staged over this
           // warp's own Q rows, which no other warp reads
-          float o[HD / 8][4];
-          wa_mma_pn<HD, NPAD, PITCH>(o, s, Vs + hh * HD, lane);
+          float o[MT][HD / 8][4];
+          wa_mma_pn<HD, NPAD, PITCH, MT>(o, s, Vs + hh * HD, lane);
           __syncwarp();
-          wa_stage<HD>(Qs + row0 * PITCH + hh * HD, PITCH, o, inv0, inv1, gq, tq, in0, in1);
+#pragma unroll
+          for (int t = 0; t < MT; ++t)
+            wa_stage<HD>(Qs + (row0 + 16 * t) * PITCH + hh * HD, PITCH, o[t], inv[t][0], inv[t][1], lane);
         }
         __syncwarp();
-        wa_store<G>(a.out, a.C, ch0, Qs + row0 * PITCH, PITCH, tab, row0, lane, q0, q1);
+        if constexpr (MT == 1) {
+          wa_store<G>(a.out, a.C, ch0, Qs + row0 * PITCH, PITCH, tab, row0, lane, q0, q1);
+        } else {
+#pragma unroll
+          for (int t = 0; t < MT; ++t)
+            wa_store<HD>(a.out, a.C, ch0 + my_head * HD, Qs + (row0 + 16 * t) * PITCH + my_head * HD, PITCH, tab, row0 + 16 * t, lane, q0, q1);
+        }
       }
     } else {
       // ---- phase 1, a warp per 16 query rows: P, dS, dQ
       if (row0 < N) {
-        float s[NB][4], dp[NB][4];
-        wa_mma_nt<HD, NPAD, PITCH>(s, Qs + row0 * PITCH, Ks, lane);
-        float mx0 = -1e30f, mx1 = -1e30f, inv0, inv1;
-        wa_scores<NPAD, WW>(s, scale2, bias_s, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx0, mx1);
-        wa_softmax<NPAD>(s, mx0, mx1, inv0, inv1);
-        wa_mma_nt<HD, NPAD, PITCH>(dp, dOs + row0 * PITCH, Vs, lane);        // dP = dO V^T
+        float s1[1][NB][4], dp1[1][NB][4], mx[1][2] = {{-1e30f, -1e30f}}, inv0, inv1;
+        float(&s)[NB][4] = s1[0], (&dp)[NB][4] = dp1[0];
+        wa_mma_nt<HD, NPAD, PITCH, 1>(s1, Qs + row0 * PITCH, Ks, lane);
+        wa_scores<NPAD, WW, 1>(s1, scale2, bias_s, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx);
+        wa_softmax<NPAD>(s, mx[0][0], mx[0][1], inv0, inv1);
+        wa_mma_nt<HD, NPAD, PITCH, 1>(dp1, dOs + row0 * PITCH, Vs, lane);        // dP = dO V^T
         f32x2 e0 = f2_both(0.f), e1 = f2_both(0.f);
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
@@ -501,36 +574,37 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
           }
         }
         {
-          float dq[HD / 8][4];
-          wa_mma_pn<HD, NPAD, PITCH>(dq, dp, Ks, lane);
+          float dq1[1][HD / 8][4];
+          float(&dq)[HD / 8][4] = dq1[0];
+          wa_mma_pn<HD, NPAD, PITCH, 1>(dq1, dp1, Ks, lane);
           // the stash rows of this block were last read before the barrier that opened this window
           __nv_bfloat16* st = Cfg::DQ_IN_STASH ? Ps + row0 * PP : dQs + row0 * PITCH;
           constexpr int stp = Cfg::DQ_IN_STASH ? PP : PITCH;
-          wa_stage<HD>(st, stp, dq, a.scale, a.scale, gq, tq, true, true);
+          wa_stage<HD>(st, stp, dq, a.scale, a.scale, lane);
           __syncwarp();
           wa_store<HD>(a.dqkv, 3LL * a.C, ch0, st, stp, tab, row0, lane, q0, q1);
           __syncwarp();
         }
-#pragma unroll
-        for (int nb = 0; nb < NB; ++nb) {
-          const int col = nb * 8 + tq * 2;
-          *reinterpret_cast<uint32_t*>(Ps + r0 * PP + col) = pack_bf16x2(s[nb][0], s[nb][1]);
-          *reinterpret_cast<uint32_t*>(Ps + r1 * PP + col) = pack_bf16x2(s[nb][2], s[nb][3]);
-          *reinterpret_cast<uint32_t*>(dSs + r0 * PP + col) = pack_bf16x2(dp[nb][0], dp[nb][1]);
-          *reinterpret_cast<uint32_t*>(dSs + r1 * PP + col) = pack_bf16x2(dp[nb][2], dp[nb][3]);
+        if constexpr (HD == 64 && NPAD == 64) {      // (the compiler spills here with the tile stores: 127 us instead of 114)
+          wa_stage_rows<NPAD>(Ps + row0 * PP, PP, s, 1.f, lane, true, true);
+          wa_stage_rows<NPAD>(dSs + row0 * PP, PP, dp, 1.f, lane, true, true);
+        } else {
+          wa_stage<NPAD>(Ps + row0 * PP, PP, s, 1.f, 1.f, lane);
+          wa_stage<NPAD>(dSs + row0 * PP, PP, dp, 1.f, 1.f, lane);
         }
       }
       __syncthreads();
-      // ---- phase 2, a warp per 16 keys: dV = P^T dO, dK = scale dS^T Q. K and V are dead: their rows stage the results.
-      // With sequence parallelism every rank of the window recomputes the whole window (cheap) and keeps only the
-      // gradients of its own token shard, so no cross-rank reduction of dK / dV is needed.
+      // ---- phase 2, a warp per 16 keys: dV = P^T dO, dK = scale dS^T Q. (Half of the warps for dV and half for dK, 32 keys each, read
+      // less of dO and Q but measured up to 6 % slower at 64 tokens.) K and V are dead: their rows stage the results. With sequence parallelism every
+      // rank of the window recomputes the whole window (cheap) and keeps only the gradients of its own token shard, so no
+      // cross-rank reduction of dK / dV is needed.
+      const int qblocks = (N + 15) >> 4;
       if (row0 < N) {
         float dv[HD / 8][4], dk[HD / 8][4];
 #pragma unroll
         for (int nb = 0; nb < HD / 8; ++nb)
 #pragma unroll
           for (int k = 0; k < 4; ++k) dv[nb][k] = dk[nb][k] = 0.f;
-        const int qblocks = (N + 15) >> 4;
 #pragma unroll
         for (int j = 0; j < NPAD / 16; ++j) {   // query blocks (contraction); blocks without a token were not stashed
           if (j >= qblocks) break;
@@ -552,8 +626,13 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
             mma_bf16_16816(dk[nb + 1], sa, c1);
           }
         }
-        wa_stage<HD>(Ks + row0 * PITCH, PITCH, dk, a.scale, a.scale, gq, tq, in0, in1);
-        wa_stage<HD>(Vs + row0 * PITCH, PITCH, dv, 1.f, 1.f, gq, tq, in0, in1);
+        if (WW != 0 || N == NPAD) {
+          wa_stage<HD>(Ks + row0 * PITCH, PITCH, dk, a.scale, a.scale, lane);
+          wa_stage<HD>(Vs + row0 * PITCH, PITCH, dv, 1.f, 1.f, lane);
+        } else {
+          wa_stage_rows<HD>(Ks + row0 * PITCH, PITCH, dk, a.scale, lane, r0 < N, r1 < N);
+          wa_stage_rows<HD>(Vs + row0 * PITCH, PITCH, dv, 1.f, lane, r0 < N, r1 < N);
+        }
         __syncwarp();
         wa_store<HD>(a.dqkv, 3LL * a.C, a.C + ch0, Ks + row0 * PITCH, PITCH, tab, row0, lane, q0, q1);
         wa_store<HD>(a.dqkv, 3LL * a.C, 2 * a.C + ch0, Vs + row0 * PITCH, PITCH, tab, row0, lane, q0, q1);
@@ -637,8 +716,9 @@ int launch_hd(const WindowAttnArgs& a, cudaStream_t stream) {
 #define TB_WA_WIDTH(WW_)                                                                       \
   return grouped ? launch<HD, NPAD, HPC, WW_, BWD>(a, stream) : launch<HD, NPAD, 1, WW_, BWD>(a, stream)
   // (the specialised widths serve windows without padding tokens; 96 = 8 x 12 or 12 x 8)
-  if constexpr (NPAD != 96) { if (a.ww == 8) { TB_WA_WIDTH(8); } }
-  if constexpr (NPAD == 96) { if (a.ww == 12) { TB_WA_WIDTH(12); } }
+  const bool whole = a.wh * a.ww == NPAD;
+  if constexpr (NPAD != 96) { if (whole && a.ww == 8) { TB_WA_WIDTH(8); } }
+  if constexpr (NPAD == 96) { if (whole && a.ww == 12) { TB_WA_WIDTH(12); } }
   TB_WA_WIDTH(0);
 #undef TB_WA_WIDTH
 }
@@ -650,9 +730,10 @@ int dispatch(const WindowAttnArgs& a, cudaStream_t stream) {
   const int hd = a.C / a.num_heads;
   if (N > 128) return -11;
   if (a.sp < 1 || a.shardN < 1 || a.n_wg < 1 || a.n_wg > 8 || a.n_wg * a.sp > WA_MAX_PEERS) return -12;
-  const int npad = N <= 64 ? 64 : (N <= 96 ? 96 : 128);
+  const int npad = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 96 ? 96 : 128));
 #define TB_WA_CASE(HD_, NP_) \
   if (hd == HD_ && npad == NP_) return launch_hd<HD_, NP_, BWD>(a, stream);
+  TB_WA_CASE(16, 32) TB_WA_CASE(32, 32) TB_WA_CASE(64, 32) TB_WA_CASE(128, 32)
   TB_WA_CASE(16, 64) TB_WA_CASE(32, 64) TB_WA_CASE(64, 64) TB_WA_CASE(128, 64)
   TB_WA_CASE(16, 96) TB_WA_CASE(32, 96) TB_WA_CASE(64, 96) TB_WA_CASE(128, 96)
   TB_WA_CASE(16, 128) TB_WA_CASE(32, 128) TB_WA_CASE(64, 128) TB_WA_CASE(128, 128)

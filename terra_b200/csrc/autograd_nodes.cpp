@@ -191,15 +191,16 @@ Tensor conv3x3(const Tensor& x, const Tensor& weight, const Tensor& bias, const 
 
 // ------------------------------------------------------------------------------------------------ transposed 2x2 convolution
 struct ConvTLayer : torch::CustomClassHolder {
-  Tensor w_fwd, b4, wg, bg, staging, status;   // staging: fp32 [4, Cin, Cout], zero between uses
+  Tensor w_fwd, b4, wg, bg, staging, status;   // staging: fp32 [4, Cout, Cin], zero between uses
   OptTensor w_dgrad;
   int64_t split, stack;
+  bool fuse_bias;
 };
 
 struct ConvT2x2 : Function<ConvT2x2> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, const Held<ConvTLayer>& l) {
     const c10::cuda::CUDAGuard guard(x.device());
-    Tensor y = torch::empty({x.size(0), 2 * x.size(1), 2 * x.size(2), l->staging.size(2)}, x.options().dtype(torch::kBFloat16));
+    Tensor y = torch::empty({x.size(0), 2 * x.size(1), 2 * x.size(2), l->staging.size(1)}, x.options().dtype(torch::kBFloat16));
     terra_ops::convt2x2(0, x.contiguous(), l->w_fwd, l->b4, y, l->status);
     ctx->save_for_backward({x});
     hold(ctx, l);
@@ -210,10 +211,10 @@ struct ConvT2x2 : Function<ConvT2x2> {
     const auto l = held<ConvTLayer>(ctx);
     const Tensor x = s[0].contiguous(), dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
-    const int64_t cout = l->staging.size(2);
-    terra_ops::convt2x2_wgrad(x, dy, l->staging, l->split, l->status, l->stack);
-    terra_ops::strided_add(l->staging, l->wg, 1, cout * 4, 4, true);
-    terra_ops::colsum(dy.view({-1, cout}), l->bg);
+    const int64_t cout = l->staging.size(1);
+    terra_ops::convt2x2_wgrad(x, dy, l->staging, l->split, l->status, l->stack, l->fuse_bias ? OptTensor(l->bg) : OptTensor());
+    terra_ops::strided_add(l->staging, l->wg, 1, 4, cout * 4, true);
+    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, cout}), l->bg);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
       dx = torch::empty(x.sizes(), x.options());
@@ -225,10 +226,10 @@ struct ConvT2x2 : Function<ConvT2x2> {
 
 Tensor conv_transpose2x2(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad,
                          const Tensor& b4, const Tensor& wg, const Tensor& bg, const Tensor& staging, int64_t split, int64_t stack,
-                         const Tensor& status) {
+                         bool fuse_bias, const Tensor& status) {
   auto l = c10::make_intrusive<ConvTLayer>();
   l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->wg = wg, l->bg = bg, l->staging = staging, l->split = split, l->stack = stack;
-  l->status = status;
+  l->fuse_bias = fuse_bias, l->status = status;
   return ConvT2x2::apply(x, weight, bias, l);
 }
 

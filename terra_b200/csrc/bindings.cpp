@@ -203,19 +203,24 @@ void convt2x2(int64_t op, const torch::Tensor& in, const torch::Tensor& w, const
   rc_check(rc, "convt2x2");
 }
 
-// dw: [4, Cin, Cout] fp32, accumulated
+// dw: [4, Cout, Cin] fp32 and bias_grad: [Cout] fp32, accumulated
 void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tensor& dw, int64_t split_k,
-                    const c10::optional<torch::Tensor>& status, int64_t stack) {
+                    const c10::optional<torch::Tensor>& status, int64_t stack,
+                    const c10::optional<torch::Tensor>& bias_grad) {
   check_image(x, "x");
   check_image(dy, "dy");
   TORCH_CHECK(x.size(0) == dy.size(0) && 2 * x.size(1) == dy.size(1) && 2 * x.size(2) == dy.size(2), "convt2x2_wgrad: grids");
   TORCH_CHECK(dw.scalar_type() == torch::kFloat32 && dw.is_contiguous() && dw.numel() == 4 * x.size(3) * dy.size(3),
-              "dw: fp32 [4, Cin, Cout]");
+              "dw: fp32 [4, Cout, Cin]");
+  TORCH_CHECK(!bias_grad.has_value() || (bias_grad->scalar_type() == torch::kFloat32 && bias_grad->is_contiguous() &&
+                                         bias_grad->numel() == dy.size(3)),
+              "bias_grad: contiguous fp32 [Cout]");
   const c10::cuda::CUDAGuard guard(x.device());
   tb::note_launch();
   const int rc = tb::convt2x2_wgrad_bf16(x.data_ptr(), dy.data_ptr(), dw.data_ptr<float>(), x.size(0), x.size(1), x.size(2),
                                          x.size(3), dy.size(3), static_cast<int>(split_k), status_ptr(status), sm_count(),
-                                         cur_stream(), static_cast<int>(stack));
+                                         cur_stream(), static_cast<int>(stack),
+                                         bias_grad.has_value() ? bias_grad->data_ptr<float>() : nullptr);
   rc_check(rc, "convt2x2_wgrad");
 }
 
@@ -263,7 +268,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("convt2x2", &convt2x2, "2x2 / stride-2 transposed convolution: forward (op 0), input gradient (op 1)", py::arg("op"),
         py::arg("input"), py::arg("w"), py::arg("bias4"), py::arg("out"), py::arg("status"));
   m.def("convt2x2_wgrad", &convt2x2_wgrad, "2x2 / stride-2 transposed convolution: weight gradient (fp32 atomics)",
-        py::arg("x"), py::arg("dy"), py::arg("dw"), py::arg("split_k"), py::arg("status"), py::arg("stack") = 1);
+        py::arg("x"), py::arg("dy"), py::arg("dw"), py::arg("split_k"), py::arg("status"), py::arg("stack") = 1, py::arg("bias_grad") = py::none());
   bind_elementwise(m);
   bind_attention(m);
   bind_halves(m);

@@ -495,10 +495,11 @@ int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, i
 }
 
 // Weight gradients: dw[tap][M][N] (fp32, atomically accumulated) = sum over the pixels of `a` [B, Ho, Wo, M] of a[pix]^T
-// times `b` [B, H, W, N] at the pixel's tap (hmul = par = stride of the grid of `a` in `b`).
+// times `b` [B, H, W, N] at the pixel's tap (hmul = par = stride of the grid of `a` in `b`). With disp_a the pixels are those of
+// `b` [B, Ho, Wo, N], and `a` [B, H, W, M] is taken at the tap: its column sums then ride on the product.
 static int gather_wgrad(const void* a, const void* b, float* dw, int B, int Ho, int Wo, int M, int H, int W, int N, int stride,
                         const Tap* taps, int ntaps, int split_k, void* status, int num_sms, cudaStream_t stream,
-                        const void* halo_lo, const void* halo_hi, float* colsum, int stack) {
+                        const void* halo_lo, const void* halo_hi, float* colsum, int stack, bool disp_a = false) {
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
   const int bn = pick_bn(N, N % 192 == 0 ? 192 : 128);   // 384 columns: two tiles of 192, a fifth less operand traffic per flop
@@ -523,9 +524,10 @@ static int gather_wgrad(const void* a, const void* b, float* dw, int B, int Ho, 
   p.split_k = split_k;
   p.a_mode = OP_PIXELS_5D;
   p.b_mode = OP_PIXELS_5D;
-  int rc = image_map(&p.map_a, a, M, 1, Wo, Ho, B, GEMM_BK);
+  p.disp_a = disp_a ? 1 : 0;
+  int rc = disp_a ? image_map(&p.map_a, a, M, stride, W, H, B, GEMM_BK) : image_map(&p.map_a, a, M, 1, Wo, Ho, B, GEMM_BK);
   if (rc != 0) return rc;
-  rc = image_map(&p.map_b, b, N, stride, W, H, B, GEMM_BK);
+  rc = disp_a ? image_map(&p.map_b, b, N, 1, Wo, Ho, B, GEMM_BK) : image_map(&p.map_b, b, N, stride, W, H, B, GEMM_BK);
   if (rc != 0) return rc - 1000;
   rc = attach_halos(p, halo_lo, halo_hi, N, stride, W, H, B, GEMM_BK);
   if (rc != 0) return rc;
@@ -566,13 +568,15 @@ int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, i
                       halo_hi, bias_grad, stack);
 }
 
-// 2x2 / stride-2 transposed convolution: dw[tap][Cin][Cout] (pre-zeroed) from x [B, H, W, Cin] and dy [B, 2H, 2W, Cout].
+// 2x2 / stride-2 transposed convolution: dw[tap][Cout][Cin] (pre-zeroed) from x [B, H, W, Cin] and dy [B, 2H, 2W, Cout], and
+// bias_grad[Cout] += the sums of dy from the same kernel: dy is operand A, displaced by the tap. (As operand B its sums were two launches
+// of their own, 90 of 290 us for 139264 pixels of 384 channels.)
 int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int split_k,
-                        void* status, int num_sms, cudaStream_t stream, int stack) {
+                        void* status, int num_sms, cudaStream_t stream, int stack, float* bias_grad) {
   if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
   const Tap taps[4] = {{0, 0, 0}, {1, 0, 0}, {0, 0, 1}, {1, 0, 1}};
-  return gather_wgrad(x, dy, dw, B, H, W, Cin, 2 * H, 2 * W, Cout, 2, taps, 4, split_k, status, num_sms, stream, nullptr,
-                      nullptr, nullptr, stack);
+  return gather_wgrad(dy, x, dw, B, H, W, Cout, 2 * H, 2 * W, Cin, 2, taps, 4, split_k, status, num_sms, stream, nullptr,
+                      nullptr, bias_grad, stack, true);
 }
 
 int gemm_stall_counters(unsigned long long* out8, int reset) {

@@ -102,11 +102,11 @@ struct TileCoord {
 };
 
 // Column sums of A (weight-gradient form): every tile of a row block streams the same A tiles, so the sums are shared out by
-// k-block, kb % ways == the tile's place among its row block's `ways` tiles. (A 16-column MMA costs as much of the
+// k-block, kb % ways == the tile's place among its row block's `ways` tiles (with a displaced A those of its group). (A 16-column MMA costs as much of the
 // tensor pipe and of the shared-memory port as 40 KB of operand stream: left to the first column tile it made that tile
 // half as slow again, and the launch waits for the slowest.) Returns this tile's first such k-block.
 __device__ __forceinline__ int first_sum_kb(const GemmParams& p, const TileCoord& t, int ways) {
-  const int place = t.grp * p.num_n_tiles + t.n_blk;
+  const int place = p.disp_a ? t.n_blk : t.grp * p.num_n_tiles + t.n_blk;
   return t.kb_begin + (place + ways - t.kb_begin % ways) % ways;
 }
 
@@ -348,11 +348,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               h -= p.img_h;
             }
             tma_load_5d<PAIR>(sA, m, bar, abase[0] + e[0], abase[1] + e[1], abase[2] + e[2], h, abase[4]);
-          } else {  // OP_PIXELS_5D: {channels, 1, w, h, b}
+          } else {  // OP_PIXELS_5D: {channels, parity, w, h, b}
+            const short* g = p.grp_off[tc.grp];
+            const int par = p.disp_a ? g[0] : 0, w = pw * GEMM_BK + (p.disp_a ? g[1] : 0), h = p.disp_a ? ph_ * p.pix_hmul + g[2] : ph_;
 #pragma unroll
             for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
               if (STACK == 1 || j < blocks * (GEMM_BM / 64))
-                tma_load_5d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, 0, pw * GEMM_BK, ph_, pb);
+                tma_load_5d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, par, w, h, pb);
           }
         }
       }
@@ -394,7 +396,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               tma_load_2d<PAIR>(sB + j * (GEMM_BK * 128), &p.map_b, bar, box_at(j), kb * GEMM_BK);
           } else {  // OP_PIXELS_5D with per-group (tap) displacement
             const short* g = p.grp_off[tc.grp];
-            int h = ph_ * p.pix_hmul + g[2];
+            const int par = p.disp_a ? 0 : g[0], w = pw * GEMM_BK + (p.disp_a ? 0 : g[1]);
+            int h = p.disp_a ? ph_ : ph_ * p.pix_hmul + g[2];
             const CUtensorMap* m = &p.map_b;
             if (h < 0 && (p.halo_flags & 1)) {
               m = &p.map_halo_lo;
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             }
 #pragma unroll
             for (int j = 0; j < Cfg::B_ROWS / 64; ++j)
-              tma_load_5d<PAIR>(sB + j * (GEMM_BK * 128), m, bar, box_at(j), g[0], pw * GEMM_BK + g[1], h, pb);
+              tma_load_5d<PAIR>(sB + j * (GEMM_BK * 128), m, bar, box_at(j), par, w, h, pb);
           }
         }
       }
@@ -442,7 +445,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         // instead of 60.)
         auto k_loop = [&](auto with_sums) {
           constexpr bool SUMS = decltype(with_sums)::value;
-          const int ways = p.groups * p.num_n_tiles;
+          const int ways = p.disp_a ? p.num_n_tiles : p.groups * p.num_n_tiles;
           const int sum_first = SUMS ? first_sum_kb(p, tc, ways) : 0;
           int sum_kb = sum_first;
           const uint32_t d_sums = tmem_base + Cfg::SUM_COL0 + acc * 32;
@@ -967,7 +970,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           }
         }
         if (Cfg::CAN_COLSUM && p.colsum != nullptr && part == 0 &&
-            first_sum_kb(p, tc, p.groups * p.num_n_tiles) < tc.kb_end) {
+            first_sum_kb(p, tc, p.disp_a ? p.num_n_tiles : p.groups * p.num_n_tiles) < tc.kb_end) {
           uint32_t v[32];   // column 0 of the sums accumulator: lane l holds the sum of A's column (row of D) q * 32 + l
           tmem_ld_32x32(tmem_base + Cfg::SUM_COL0 + dcol * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
           tmem_ld_wait();

@@ -43,8 +43,9 @@ struct GemmParams {
   short ktable[GEMM_MAX_KTABLE][4];
   // OP_PIXELS_5D: k-block -> (wc, h, b) with extents (pix_n0 = chunks per row, pix_n1 = rows).
   int pix_n0, pix_n1;
-  int pix_hmul;                // input row = h * pix_hmul + dh   (2 for the stride-2 convolution)
-  short grp_off[16][4];        // per group (tap): {parity, dw, dh, unused} applied to operand B
+  int pix_hmul;                // row of the displaced image = h * pix_hmul + dh   (2 for the stride-2 convolution)
+  short grp_off[16][4];        // per group (tap): {parity, dw, dh, unused} applied to operand B, or A
+  int disp_a;                  // the displaced image is operand A (and the column sums add up over the groups)
   long long grp_c_stride;      // output offset (elements) between groups
   // epilogue
   int epi;

@@ -88,7 +88,7 @@ int convt2x2_fwd_bf16(const void* x, const void* w, const void* bias4, void* y, 
 int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, int W, int Cin, int Cout, void* status,
                         int num_sms, cudaStream_t stream);
 int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int split_k,
-                        void* status, int num_sms, cudaStream_t stream, int stack = 1);
+                        void* status, int num_sms, cudaStream_t stream, int stack, float* bias_grad);
 int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
                        int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo = nullptr,
                        const void* halo_hi = nullptr, float* bias_grad = nullptr, int stack = 1);   // bias_grad[Cout] += sums of dy

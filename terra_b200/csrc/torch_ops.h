@@ -14,7 +14,8 @@ void conv3x3_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t stride
                    const OptTensor& halo_lo, const OptTensor& halo_hi, const OptTensor& bias_grad, int64_t stack);
 void conv3x3_s2_dgrad(const Tensor& dy, const Tensor& w, Tensor& dx, const OptTensor& status);
 void convt2x2(int64_t op, const Tensor& in, const Tensor& w, const OptTensor& bias4, Tensor& out, const OptTensor& status);
-void convt2x2_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t split_k, const OptTensor& status, int64_t stack);
+void convt2x2_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t split_k, const OptTensor& status, int64_t stack,
+                    const OptTensor& bias_grad);
 
 void colsum(const Tensor& x, Tensor& out);
 void groupnorm_stats(const Tensor& x, Tensor& sums, int64_t groups);

@@ -315,15 +315,15 @@ class _ConvT2x2Fn(torch.autograd.Function):
         tiled = _convt_tiled(B, H, W, Cin, Cout)
         dy = dy.contiguous()
         gw, gb = _arena_grad(weight), _arena_grad(bias)
+        # [tap, co, ci] staging -> (Cin, Cout, 2, 2)
+        shape, layout = (4, Cout, Cin), (1, 4, Cout * 4)
+        fused = tiled and gb is not None and FUSE_BIAS_GRAD
         if tiled:
-            # [tap, ci, co] staging -> (Cin, Cout, 2, 2)
-            shape, layout = (4, Cin, Cout), (1, Cout * 4, 4)
-            split, stack = _wgrad_plan(4, Cin, Cout, B * H * ((W + 63) // 64))
-            wgrad = lambda dwt: ext.convt2x2_wgrad(x.contiguous(), dy, dwt, split, status_word(x.device), stack)
+            split, stack = _wgrad_plan(4, Cout, Cin, B * H * ((W + 63) // 64))
+            wgrad = lambda dwt: ext.convt2x2_wgrad(x.contiguous(), dy, dwt, split, status_word(x.device), stack, gb if fused else None)
         else:
-            # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it. [tap, co, ci] staging
+            # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it
             dyu = dy.view(B, H, 2, W, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B * H * W, 4 * Cout)
-            shape, layout = (4, Cout, Cin), (1, 4, Cout * 4)
             wgrad = lambda dwt: wgrad_accumulate(dyu, x.reshape(-1, Cin), dwt.view(4 * Cout, Cin))
         if gw is not None:
             dwt = _zero_scratch(x.device, shape, "convT")
@@ -333,9 +333,10 @@ class _ConvT2x2Fn(torch.autograd.Function):
         else:
             dwt = torch.zeros(*shape, device=x.device, dtype=torch.float32)
             wgrad(dwt)
-            dw = dwt.view(2, 2, *shape[1:]).permute(*((2, 3, 0, 1) if tiled else (3, 2, 0, 1)))
+            dw = dwt.view(2, 2, *shape[1:]).permute(3, 2, 0, 1)
         if gb is not None:
-            ext.colsum(dy.view(-1, Cout), gb)
+            if not fused:
+                ext.colsum(dy.view(-1, Cout), gb)
             db = None
         else:
             db = torch.zeros(Cout, device=x.device, dtype=torch.float32)
@@ -375,10 +376,10 @@ def _conv_transpose2x2_node(x, weight, bias):
     if not _convt_tiled(B, H, W, Cin, Cout):
         return None
     wd = _packed(weight, w16, "convT_dgrad", _pack_convt_dgrad) if x.requires_grad and torch.is_grad_enabled() else None
-    split, stack = _wgrad_plan(4, Cin, Cout, B * H * ((W + 63) // 64))
+    split, stack = _wgrad_plan(4, Cout, Cin, B * H * ((W + 63) // 64))
     return _ext.load().nodes.conv_transpose2x2(
         x, weight, bias, _packed(weight, w16, "convT", _pack_convt), wd, _packed(bias, bias.bf16, "convT_bias", _pack_convt_bias), *grads,
-        _zero_scratch(x.device, (4, Cin, Cout), "convT"), split, stack, status_word(x.device))
+        _zero_scratch(x.device, (4, Cout, Cin), "convT"), split, stack, FUSE_BIAS_GRAD, status_word(x.device))
 
 
 def _convt_flat_weight(weight, w16):

@@ -98,6 +98,8 @@ struct MlpHalf : Function<MlpHalf> {
 Tensor mlp_half(const Tensor& x, const Tensor& anchor, const std::vector<Tensor>& w, const std::vector<Tensor>& g, double eps, bool fuse_bias,
                 const Tensor& status) {
   need(w.size() == 6 && g.size() == 6, "MLP half: six weights and their gradients");
+  if (!c10::GradMode::is_enabled() && !x._fw_grad(0).defined())
+    return terra_ops::mlp_half_infer(x, w[0], w[1], w[2], w[3], w[4], w[5], eps, status);
   auto l = c10::make_intrusive<MlpLayer>();
   l->ln_w = w[0], l->ln_b = w[1], l->fc1_w = w[2], l->fc1_b = w[3], l->fc2_w = w[4], l->fc2_b = w[5];
   l->ln_wg = g[0], l->ln_bg = g[1], l->fc1_wg = g[2], l->fc1_bg = g[3], l->fc2_wg = g[4], l->fc2_bg = g[5];
@@ -235,7 +237,7 @@ Tensor conv_transpose2x2(const Tensor& x, const Tensor& weight, const Tensor& bi
 
 // ------------------------------------------------------------------------------------------------ GroupNorm + SiLU
 struct NormLayer : torch::CustomClassHolder {
-  Tensor g, b, gg, bg, sums;                   // sums: fp32 [B, groups, 2], zero between uses
+  Tensor g, b, gg, bg, sums;                   // sums: fp32 [B * groups * 2 + 1] (a ticket), zero between uses
   int64_t groups;
   double eps;
   bool has_res;
@@ -251,8 +253,7 @@ struct GroupNormSilu : Function<GroupNormSilu> {
     const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
     const Tensor x3 = x.view(flat);
     Tensor stats = torch::empty({x.size(0), l->groups, 2}, x.options().dtype(torch::kFloat32));
-    terra_ops::groupnorm_stats(x3, l->sums, l->groups);
-    terra_ops::groupnorm_finalize(l->sums, stats, inverse_count(x, l->groups), l->eps, true);
+    terra_ops::groupnorm_mean_rstd(x3, l->sums, stats, l->groups, inverse_count(x, l->groups), l->eps);
     Tensor y = torch::empty_like(x), y3 = y.view(flat);
     terra_ops::groupnorm_silu_apply(x3, stats, l->g, l->b, residual.has_value() ? OptTensor(residual->view(flat)) : residual, y3, l->groups);
     ctx->save_for_backward({x, stats, l->g, l->b});

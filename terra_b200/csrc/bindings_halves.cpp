@@ -311,6 +311,23 @@ Tensor attn_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, cons
   return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy);
 }
 
+// y alone, where no backward pass follows: the pre-activation is not written
+Tensor mlp_half_infer(const Tensor& x, const Tensor& ln_w, const Tensor& ln_b, const Tensor& fc1_w, const Tensor& fc1_b, const Tensor& fc2_w,
+                      const Tensor& fc2_b, double eps, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  Norm n = norm_fwd(x, ln_w, ln_b, eps);
+  Tensor act = torch::empty({x.size(0), fc1_w.size(0)}, x.options()), y = torch::empty_like(x);
+  Epi e;
+  e.flags = tb::EPI_GELU;
+  e.bias = &fc1_b;
+  product(n.xn, fc1_w, false, act, e, status);
+  Epi r;
+  r.bias = &fc2_b;
+  r.residual = &x;
+  product(act, fc2_w, false, y, r, status);
+  return y;
+}
+
 // -> y, mean, rstd, xn, pre, act
 std::vector<Tensor> mlp_half_fwd(const Tensor& x, const Tensor& ln_w, const Tensor& ln_b, const Tensor& fc1_w, const Tensor& fc1_b,
                                  const Tensor& fc2_w, const Tensor& fc2_b, double eps, const Tensor& status) {

@@ -312,22 +312,54 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 // 98 -> 90 us, apply with shortcut 355 -> 225, backward sums 366 -> 258, backward apply 406 -> 264; one copy of the image
 // each way at 6.65 TB/s is 129 us.)
 //
-// Statistics: per-channel partials in shared memory, folded to groups, two atomics per (block, group).
+// Adds a thread's 16 sums (s, q of its eight channels) over the block's threadIdx.y and leaves them in sh[c] and sh[C + c]. Every thread of
+// the block takes part. Through a buffer of the block's own rather than by shared-memory atomics, which
+// are compare-and-swap loops for floats and met `blockDim.y` at a time on one address: they were half of the time of images of some MB.
+__device__ __forceinline__ void gn_block_sums(float* sh, float* buf, const float (&s)[8], const float (&q)[8], int C, int vi) {
+  const int bx = blockDim.x, t = threadIdx.y * bx + threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    buf[(threadIdx.y * 16 + j) * bx + threadIdx.x] = s[j];
+    buf[(threadIdx.y * 16 + 8 + j) * bx + threadIdx.x] = q[j];
+  }
+  __syncthreads();
+  for (int i = t; i < 16 * bx; i += bx * blockDim.y) {
+    float sum = 0.f;
+    for (int y = 0; y < static_cast<int>(blockDim.y); ++y) sum += buf[y * 16 * bx + i];
+    const int j = i / bx, c = (vi - static_cast<int>(threadIdx.x) + i % bx) * 8 + (j & 7);
+    if (c < C) sh[(j >> 3) * C + c] = sum;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void gn_finalize_cell(float* sums, float* stats, int i, float inv_count, float eps, bool clear) {
+  const float mean = __ldcg(sums + 2 * i) * inv_count;
+  const float var = fmaxf(__ldcg(sums + 2 * i + 1) * inv_count - mean * mean, 0.f);
+  stats[2 * i] = mean;
+  stats[2 * i + 1] = rsqrtf(var + eps);
+  if (clear) {
+    sums[2 * i] = 0.f;
+    sums[2 * i + 1] = 0.f;
+  }
+}
+
+// Statistics: per-channel sums of the block, folded to groups, two atomics per (block, group). With `stats` the last block to finish turns
+// the sums into mean and reciprocal deviation and clears them (and the ticket counter) for their next use.
 __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat16* __restrict__ x,
                                                               float* __restrict__ sums, long long HW, int C, int groups,
-                                                              int pix_per_block) {
+                                                              int pix_per_block, float* __restrict__ stats, unsigned int* __restrict__ ticket,
+                                                              float inv_count, float eps) {
   chain_begin();
-  extern __shared__ float sh[];  // [2][C]
+  extern __shared__ float sh[];  // [2][C], then the threads' sums
   const int nvec = C >> 3;
   const int b = blockIdx.y;
-  for (int c = threadIdx.y * blockDim.x + threadIdx.x; c < 2 * C; c += blockDim.x * blockDim.y) sh[c] = 0.f;
-  __syncthreads();
   const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
   const long long p1 = min(HW, p0 + pix_per_block);
-  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
+  for (int v0 = 0; v0 < nvec; v0 += blockDim.x) {
+    const int vi = v0 + threadIdx.x;
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const uint4* src = reinterpret_cast<const uint4*>(x) + static_cast<long long>(b) * HW * nvec + vi;
-    for (long long p = p0 + threadIdx.y; p < p1; p += 4 * blockDim.y) {
+    for (long long p = p0 + threadIdx.y; vi < nvec && p < p1; p += 4 * blockDim.y) {
       uint4 t[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -345,15 +377,10 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
         }
       }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      atomicAdd(&sh[vi * 8 + j], s[j]);
-      atomicAdd(&sh[C + vi * 8 + j], q[j]);
-    }
+    gn_block_sums(sh, sh + 2 * C, s, q, C, vi);
   }
-  __syncthreads();
-  const int cpg = C / groups;
-  for (int g = threadIdx.y * blockDim.x + threadIdx.x; g < groups; g += blockDim.x * blockDim.y) {
+  const int cpg = C / groups, tid = threadIdx.y * blockDim.x + threadIdx.x;
+  for (int g = tid; g < groups; g += blockDim.x * blockDim.y) {
     float s = 0.f, q = 0.f;
     for (int c = g * cpg; c < (g + 1) * cpg; ++c) {
       s += sh[c];
@@ -361,6 +388,17 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
     }
     atomicAdd(&sums[(b * groups + g) * 2 + 0], s);
     atomicAdd(&sums[(b * groups + g) * 2 + 1], q);
+  }
+  if (stats == nullptr) return;
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(ticket, 1u) + 1u == gridDim.x * gridDim.y;
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    for (int i = tid; i < static_cast<int>(gridDim.y) * groups; i += blockDim.x * blockDim.y) gn_finalize_cell(sums, stats, i, inv_count, eps, true);
+    if (tid == 0) *ticket = 0u;
   }
 }
 
@@ -432,72 +470,94 @@ __global__ void __launch_bounds__(256, 3) groupnorm_silu_apply_kernel(const __nv
   }
 }
 
-// pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}
+// Two channels' constants, and SiLU's derivative part of them: xhat and dz = dy * silu'(z), z = xhat * gamma + beta.
+struct GnPair {
+  f32x2 nmu, rs, g, bt;      // minus the mean, reciprocal deviation, affine parameters
+};
+__device__ __forceinline__ GnPair gn_pair(const float* __restrict__ stats, uint32_t gamma2, uint32_t beta2, int b, int c, int cpg, int groups) {
+  const float* s0 = stats + (b * groups + c / cpg) * 2;
+  const float* s1 = stats + (b * groups + (c + 1) / cpg) * 2;
+  const float2 g = unpack_bf16x2(gamma2), bt = unpack_bf16x2(beta2);
+  return {f2_pack(-s0[0], -s1[0]), f2_pack(s0[1], s1[1]), f2_pack(g.x, g.y), f2_pack(bt.x, bt.y)};
+}
+__device__ __forceinline__ f32x2 f2_of_bf16x2(uint32_t v) {
+  const float2 f = unpack_bf16x2(v);
+  return f2_pack(f.x, f.y);
+}
+// (two elements per instruction; the same operations as sigmoidf_ in the same order)
+__device__ __forceinline__ f32x2 f2_sigmoid(f32x2 z) {
+  float a, b;
+  f2_unpack(f2_mul(z, f2_both(-1.4426950408889634f)), a, b);
+  f2_unpack(f2_add(f2_pack(exp2f(a), exp2f(b)), f2_both(1.f)), a, b);
+  return f2_pack(__fdividef(1.f, a), __fdividef(1.f, b));
+}
+__device__ __forceinline__ f32x2 gn_dz(const GnPair& c, f32x2 x, f32x2 dy, f32x2& xh) {
+  xh = f2_mul(f2_add(x, c.nmu), c.rs);
+  const f32x2 z = f2_fma(xh, c.g, c.bt), sg = f2_sigmoid(z);
+  return f2_mul(f2_mul(dy, sg), f2_fma(z, f2_fma(sg, f2_both(-1.f), f2_both(1.f)), f2_both(1.f)));
+}
+
+// pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}. Bound by issue and the latency of its loads beside HBM: two channels per instruction
+// and no shared-memory atomics (us, before / this: 557056 pixels x 384 257 / 248, 17280 x 192 17.4 / 13.3; statistics of 17280 x 192 10.1 + 1.4
+// for a launch that finished them / 7.1).
 __global__ void __launch_bounds__(256, 3) groupnorm_silu_bwd_reduce_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta, float* __restrict__ red,
     long long HW, int C, int groups, int pix_per_block, float* __restrict__ dgamma, float* __restrict__ dbeta) {
   chain_begin();
-  extern __shared__ float sh[];  // [2][C]
+  extern __shared__ float sh[];  // [2][C], then the threads' sums
   const int nvec = C >> 3;
   const int b = blockIdx.y;
-  for (int c = threadIdx.y * blockDim.x + threadIdx.x; c < 2 * C; c += blockDim.x * blockDim.y) sh[c] = 0.f;
-  __syncthreads();
   const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
   const long long p1 = min(HW, p0 + pix_per_block);
-  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
-    // (the affine parameters stay packed: 16 registers less)
-    float rs[8], mu[8];
-    const uint4 gq = reinterpret_cast<const uint4*>(gamma)[vi], bq = reinterpret_cast<const uint4*>(beta)[vi];
-    {
-      GnChannels c;
-      gn_channels(c, stats, gamma, beta, b, vi, C / groups, groups);
+  for (int v0 = 0; v0 < nvec; v0 += blockDim.x) {
+    const int vi = v0 + threadIdx.x;
+    f32x2 s2[4], q2[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        rs[j] = c.rs[j];
-        mu[j] = c.mu[j];
+    for (int j = 0; j < 4; ++j) s2[j] = q2[j] = f2_both(0.f);
+    if (vi < nvec) {
+      GnPair c[4];
+      {
+        const uint4 gq = reinterpret_cast<const uint4*>(gamma)[vi], bq = reinterpret_cast<const uint4*>(beta)[vi];
+        const uint32_t g4[4] = {gq.x, gq.y, gq.z, gq.w}, b4[4] = {bq.x, bq.y, bq.z, bq.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = gn_pair(stats, g4[j], b4[j], b, vi * 8 + 2 * j, C / groups, groups);
       }
-    }
-    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const long long first = static_cast<long long>(b) * HW * nvec + vi;
-    const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
-    const uint4* ds = reinterpret_cast<const uint4*>(dy) + first;
-    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
-      uint4 t[2], d2[2];
+      const long long first = static_cast<long long>(b) * HW * nvec + vi;
+      const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
+      const uint4* ds = reinterpret_cast<const uint4*>(dy) + first;
+      for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
+        uint4 t[2], d2[2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        t[u] = d2[u] = make_uint4(0u, 0u, 0u, 0u);     // dz = 0 behind the range
-        if (p + u * blockDim.y < p1) {
-          t[u] = xs[(p + u * blockDim.y) * nvec];
-          d2[u] = ds[(p + u * blockDim.y) * nvec];
+        for (int u = 0; u < 2; ++u) {
+          t[u] = d2[u] = make_uint4(0u, 0u, 0u, 0u);
+          if (p + u * blockDim.y < p1) {
+            t[u] = xs[(p + u * blockDim.y) * nvec];
+            d2[u] = ds[(p + u * blockDim.y) * nvec];
+          }
         }
-      }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        float f[8], d[8], g[8], bt[8];
-        unpack8(t[u], f);
-        unpack8(d2[u], d);
-        unpack8(gq, g);
-        unpack8(bq, bt);
-        if (p + u * blockDim.y >= p1) break;
+        for (int u = 0; u < 2; ++u) {
+          if (p + u * blockDim.y >= p1) break;
+          const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, d4[4] = {d2[u].x, d2[u].y, d2[u].z, d2[u].w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh = (f[j] - mu[j]) * rs[j];
-          const float z = xh * g[j] + bt[j];
-          const float sg = sigmoidf_(z);
-          const float dz = d[j] * sg * (1.f + z * (1.f - sg));
-          s[j] += dz;
-          q[j] += dz * xh;
+          for (int j = 0; j < 4; ++j) {
+            f32x2 xh;
+            const f32x2 dz = gn_dz(c[j], f2_of_bf16x2(x4[j]), f2_of_bf16x2(d4[j]), xh);
+            s2[j] = f2_add(s2[j], dz);
+            q2[j] = f2_fma(dz, xh, q2[j]);
+          }
         }
       }
     }
+    float s[8], q[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      atomicAdd(&sh[vi * 8 + j], s[j]);
-      atomicAdd(&sh[C + vi * 8 + j], q[j]);
+    for (int j = 0; j < 4; ++j) {
+      f2_unpack(s2[j], s[2 * j], s[2 * j + 1]);
+      f2_unpack(q2[j], q[2 * j], q[2 * j + 1]);
     }
+    gn_block_sums(sh, sh + 2 * C, s, q, C, vi);
   }
-  __syncthreads();
   for (int c = threadIdx.y * blockDim.x + threadIdx.x; c < C; c += blockDim.x * blockDim.y) {
     atomicAdd(&red[(static_cast<long long>(b) * C + c) * 2 + 0], sh[c]);
     atomicAdd(&red[(static_cast<long long>(b) * C + c) * 2 + 1], sh[C + c]);
@@ -512,16 +572,7 @@ __global__ void groupnorm_finalize_kernel(float* __restrict__ sums, float* __res
                                           float eps, int clear) {
   chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < cells) {
-    const float mean = sums[2 * i] * inv_count;
-    const float var = fmaxf(sums[2 * i + 1] * inv_count - mean * mean, 0.f);
-    stats[2 * i] = mean;
-    stats[2 * i + 1] = rsqrtf(var + eps);
-    if (clear) {
-      sums[2 * i] = 0.f;
-      sums[2 * i + 1] = 0.f;
-    }
-  }
+  if (i < cells) gn_finalize_cell(sums, stats, i, inv_count, eps, clear != 0);
 }
 
 // dst[a * sa + b * sb + c * sc] += src[(a * nb + b) * nc + c] (fp32); with `clear` the source is zeroed behind the read,
@@ -566,13 +617,18 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
   const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
   const long long p1 = min(HW, p0 + pix_per_block);
   for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
-    GnChannels c;
-    gn_channels(c, stats, gamma, beta, b, vi, cpg, groups);
-    float m1[8], m2[8];
+    GnPair c[4];
+    f32x2 nm1[4], nm2[4];
+    {
+      const uint4 gq = reinterpret_cast<const uint4*>(gamma)[vi], bq = reinterpret_cast<const uint4*>(beta)[vi];
+      const uint32_t g4[4] = {gq.x, gq.y, gq.z, gq.w}, b4[4] = {bq.x, bq.y, bq.z, bq.w};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      m1[j] = gs[(vi * 8 + j) / cpg * 2];
-      m2[j] = gs[(vi * 8 + j) / cpg * 2 + 1];
+      for (int j = 0; j < 4; ++j) {
+        const int ch = vi * 8 + 2 * j;
+        c[j] = gn_pair(stats, g4[j], b4[j], b, ch, cpg, groups);
+        nm1[j] = f2_pack(-gs[ch / cpg * 2], -gs[(ch + 1) / cpg * 2]);
+        nm2[j] = f2_pack(-gs[ch / cpg * 2 + 1], -gs[(ch + 1) / cpg * 2 + 1]);
+      }
     }
     const long long first = static_cast<long long>(b) * HW * nvec + vi;
     const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
@@ -590,18 +646,15 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         if (p + u * blockDim.y >= p1) break;
-        float f[8], d[8], o[8];
-        unpack8(t[u], f);
-        unpack8(d2[u], d);
+        const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, d4[4] = {d2[u].x, d2[u].y, d2[u].z, d2[u].w};
+        uint32_t o[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh = (f[j] - c.mu[j]) * c.rs[j];
-          const float z = xh * c.g[j] + c.bt[j];
-          const float sg = sigmoidf_(z);
-          const float dz = d[j] * sg * (1.f + z * (1.f - sg));
-          o[j] = c.rs[j] * (dz * c.g[j] - m1[j] - xh * m2[j]);
+        for (int j = 0; j < 4; ++j) {
+          f32x2 xh;
+          const f32x2 dz = gn_dz(c[j], f2_of_bf16x2(x4[j]), f2_of_bf16x2(d4[j]), xh);
+          o[j] = f2_to_bf16x2(f2_mul(c[j].rs, f2_fma(xh, nm2[j], f2_fma(dz, c[j].g, nm1[j]))));
         }
-        dst[(p + u * blockDim.y) * nvec] = pack8(o);
+        dst[(p + u * blockDim.y) * nvec] = make_uint4(o[0], o[1], o[2], o[3]);
       }
     }
   }
@@ -1045,16 +1098,34 @@ static bool gn_sizes_ok(int B, long long HW, int C, int groups) {
   return B >= 1 && HW >= 1 && C >= 8 && C % 8 == 0 && groups >= 1 && C % groups == 0;
 }
 
-int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {
-  if (!gn_sizes_ok(B, HW, C, groups)) return -1;
+// [2][C] sums of the block and 16 per thread. Beyond the 48 KB that every launch may have (C >= 2048) the kernel is asked for more.
+constexpr int GN_MAX_CHANNELS = 6144;
+template <class Kernel>
+static size_t gn_smem(Kernel kernel, const GnShape& s, int C) {
+  const size_t bytes = (2 * static_cast<size_t>(C) + 16 * static_cast<size_t>(s.block.x) * s.block.y) * sizeof(float);
+  if (bytes > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+  return bytes;
+}
+
+static int groupnorm_stats_launch(const void* x, float* sums, int B, long long HW, int C, int groups, float* stats, unsigned int* ticket,
+                                  float inv_count, float eps, cudaStream_t stream) {
+  if (!gn_sizes_ok(B, HW, C, groups) || C > GN_MAX_CHANNELS) return -1;
   // Every block ends in two atomics per group on the same addresses, and its warps meet in shared memory before. While the image
   // is L2-sized the passes over it are shorter than that, and one block per SM is enough (us, 1 / 3 blocks per SM: 64800 x 192 13 / 21,
   // 139264 x 128 15 / 22, 139264 x 256 20 / 23, 139264 x 384 52 / 29).
   const bool small = static_cast<long long>(B) * HW * C * 2 <= 72000000LL;
   const GnShape s(B, HW, C, 512, small ? 1 : 3, 4);
-  launch_chained(groupnorm_stats_kernel, s.grid, s.block, 2 * C * sizeof(float), stream, static_cast<const __nv_bfloat16*>(x), sums, HW,
-                                                                             C, groups, s.pix);
+  launch_chained(groupnorm_stats_kernel, s.grid, s.block, gn_smem(groupnorm_stats_kernel, s, C), stream, static_cast<const __nv_bfloat16*>(x),
+                 sums, HW, C, groups, s.pix, stats, ticket, inv_count, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {
+  return groupnorm_stats_launch(x, sums, B, HW, C, groups, nullptr, nullptr, 0.f, 0.f, stream);
+}
+// Mean and reciprocal deviation in one launch; sums [B * groups * 2] and the ticket behind them zero before and after.
+int groupnorm_mean_rstd(const void* x, float* sums, float* stats, int B, long long HW, int C, int groups, float inv_count, float eps,
+                        cudaStream_t stream) {
+  return groupnorm_stats_launch(x, sums, B, HW, C, groups, stats, reinterpret_cast<unsigned int*>(sums + 2LL * B * groups), inv_count, eps, stream);
 }
 
 int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, const void* beta, const void* res, void* y,
@@ -1070,9 +1141,9 @@ int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, c
 int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats, const void* gamma, const void* beta,
                               float* red, float* dgamma, float* dbeta, int B, long long HW, int C, int groups,
                               cudaStream_t stream) {
-  if (!gn_sizes_ok(B, HW, C, groups)) return -1;
+  if (!gn_sizes_ok(B, HW, C, groups) || C > GN_MAX_CHANNELS) return -1;
   const GnShape s(B, HW, C, 256, 3, 2);
-  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, 2 * C * sizeof(float), stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
+  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, gn_smem(groupnorm_silu_bwd_reduce_kernel, s, C), stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
       static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups,
       s.pix, dgamma, dbeta);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

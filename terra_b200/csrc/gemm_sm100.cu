@@ -733,6 +733,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       else if (form == 0) run(std::integral_constant<int, 0>{});
       else if (form == EPI_BIAS) run(std::integral_constant<int, EPI_BIAS>{});
       else if (form == (EPI_BIAS | EPI_GELU | EPI_SAVE_PRE)) run(std::integral_constant<int, EPI_BIAS | EPI_GELU | EPI_SAVE_PRE>{});
+      else if (form == (EPI_BIAS | EPI_GELU)) run(std::integral_constant<int, EPI_BIAS | EPI_GELU>{});
       else if (form == (EPI_BIAS | EPI_RESIDUAL)) run(std::integral_constant<int, EPI_BIAS | EPI_RESIDUAL>{});
       else if (form == EPI_MUL_DGELU) run(std::integral_constant<int, EPI_MUL_DGELU>{});
       else run(std::integral_constant<int, -1>{});

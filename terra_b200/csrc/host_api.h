@@ -105,6 +105,8 @@ int colsum_rows_per_block();
 // out[c] += column sums of the bf16 matrix x; partials: fp32 scratch of ceil(rows / colsum_rows_per_block()) x C
 int colsum_bf16(const void* x, float* out, float* partials, long long rows, int C, long long ld, cudaStream_t stream);
 // GroupNorm statistics over NHWC bf16 [B, HW, C]: accumulates per (b, group) sum and sum of squares (fp32, zeroed).
+int groupnorm_mean_rstd(const void* x, float* sums, float* stats, int B, long long HW, int C, int groups, float inv_count, float eps,
+                        cudaStream_t stream);
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream);
 // y = silu((x - mean) * rstd * gamma + beta) [+ res]; `stats` holds {mean, rstd} per (b, group).
 int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, const void* beta, const void* res, void* y,

@@ -18,6 +18,7 @@ void convt2x2_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t split
                     const OptTensor& bias_grad);
 
 void colsum(const Tensor& x, Tensor& out);
+void groupnorm_mean_rstd(const Tensor& x, Tensor& scratch, Tensor& stats, int64_t groups, double inv_count, double eps);
 void groupnorm_stats(const Tensor& x, Tensor& sums, int64_t groups);
 void groupnorm_silu_apply(const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, const OptTensor& res, Tensor& y,
                           int64_t groups);
@@ -40,6 +41,8 @@ Tensor attn_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, cons
                      const Tensor& status);
 std::vector<Tensor> mlp_half_fwd(const Tensor& x, const Tensor& ln_w, const Tensor& ln_b, const Tensor& fc1_w, const Tensor& fc1_b,
                                  const Tensor& fc2_w, const Tensor& fc2_b, double eps, const Tensor& status);
+Tensor mlp_half_infer(const Tensor& x, const Tensor& ln_w, const Tensor& ln_b, const Tensor& fc1_w, const Tensor& fc1_b, const Tensor& fc2_w,
+                      const Tensor& fc2_b, double eps, const Tensor& status);
 Tensor mlp_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, const Tensor& rstd, const Tensor& xn, const Tensor& pre,
                     const Tensor& act, const Tensor& ln_w, const Tensor& fc1_w, const Tensor& fc2_w, const Tensor& ln_wg,
                     const Tensor& ln_bg, const Tensor& fc1_wg, const Tensor& fc1_bg, const Tensor& fc2_wg, const Tensor& fc2_bg,

@@ -454,7 +454,7 @@ def groupnorm_silu(x, gn: torch.nn.GroupNorm, residual=None, dom=None):
         if grads is not None and x.dim() == 4:
             return _ext.load().nodes.groupnorm_silu(
                 x, gn.weight, gn.bias, residual, gn.weight.bf16, gn.bias.bf16, *grads,
-                _zero_scratch(x.device, (x.shape[0], gn.num_groups, 2), "gn_sums"), gn.num_groups, GN_EPS)
+                _zero_scratch(x.device, (x.shape[0] * gn.num_groups * 2 + 1,), "gn_sums"), gn.num_groups, GN_EPS)
         return _GroupNormSiluFn.apply(x, gn.weight, gn.bias, residual, gn.num_groups, dom)
     xc = x.permute(0, 3, 1, 2)
     if dom is not None and dom.world > 1:

@@ -111,16 +111,18 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 // without 1047 / 935, 139264 of 1536 x 384 231 / 202, 156672 of 3072 x 1024 without sums 704 / 647.
 struct WgradPlan {
   int bn, stack, split;
+  bool swapped;      // the transpose: rows are x's columns
 };
 WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   const int64_t m_blocks = (N + 127) / 128, k_blocks = (M + 63) / 64, sms = sm_count();
-  WgradPlan best{128, 1, 1};
+  WgradPlan best{128, 1, 1, false};
   double least = -1.0;
   // `width` columns, `blocks` 128-row blocks a tile, `kb` KB a k-block, on `units` CTAs or pairs; `pair`: two CTAs share the blocks
-  auto consider = [&](int request, int width, int stack, bool pair, double kb, double extra) {
+  auto consider = [&](int request, int width, int stack, bool pair, double kb, double extra, bool swapped = false) {
     const int64_t blocks = pair ? 2 : stack, units = pair ? sms / 2 : sms;
-    const int64_t n = (K + width - 1) / width, tiles = (m_blocks + blocks - 1) / blocks * n;
-    if (sums && extra == 0.0) kb += (pair ? 16.0 : 40.0 * stack) / n;
+    const int64_t rows = swapped ? (K + 127) / 128 : m_blocks;
+    const int64_t n = ((swapped ? N : K) + width - 1) / width, tiles = (rows + blocks - 1) / blocks * n;
+    if (sums && extra == 0.0 && !swapped) kb += (pair ? 16.0 : 40.0 * stack) / n;
     // whole rounds of CTAs: the largest split of one round, two rounds, ...
     for (int64_t rounds = 1; rounds <= 3; ++rounds) {
       const int64_t split = std::max<int64_t>(1, std::min(rounds * units / tiles, k_blocks));
@@ -129,7 +131,7 @@ WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
                           1.3 * tiles * split * blocks * width / 192 + (pair ? 600.0 : 0.0) + extra;   // (a pair starts 2 us later)
       if (least < 0.0 || cost < least * 0.995) {
         least = cost;
-        best = {request, stack, static_cast<int>(split)};
+        best = {request, stack, static_cast<int>(split), swapped};
       }
     }
   };
@@ -143,6 +145,8 @@ WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
     if (K > 256) consider(1384, 384, 1, true, 140.0, 0.0);
     if (K > 128) consider(1256, 256, 1, true, 74.0, separate);
   }
+  // few outputs of a wide layer (patch embedding: 384 x 2976): 384 rows fill one and a half pairs, 384 columns one tile
+  if (tb::gemm_pairs() && sms >= 2 && N > 256 && K > 2 * N) consider(1384, 384, 1, true, 140.0, separate, true);
   return best;
 }
 
@@ -166,13 +170,14 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
     sums = false;
   }
   const WgradPlan plan = plan_wgrad(N, K, M, sums);
-  if (sums && plan.bn % 1000 == 256) {
+  if (sums && (plan.bn % 1000 == 256 || plan.swapped)) {
     column_sums(dy, *grad_b);
     sums = false;
   }
   tb::GemmOperand A{dy.data_ptr(), dy.stride(0), 1}, B{x.data_ptr(), x.stride(0), 1};
+  if (plan.swapped) std::swap(A, B);
   tb::GemmEpilogue g{};
-  g.flags = tb::EPI_OUT_F32 | tb::EPI_ATOMIC;
+  g.flags = tb::EPI_OUT_F32 | tb::EPI_ATOMIC | (plan.swapped ? tb::EPI_TRANSPOSE : 0);
   g.C = grad_w.data_ptr();
   g.ldc = grad_w.stride(0);
   g.alpha = 1.0f;
@@ -180,7 +185,8 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
   g.colsum = sums ? grad_b->data_ptr<float>() : nullptr;
   g.stack = plan.stack;
   tb::note_launch();
-  rc_check(tb::gemm_bf16(A, B, N, K, M, g, plan.split, plan.bn, sm_count(), cur_stream()), "gemm (weight gradient)");
+  rc_check(tb::gemm_bf16(A, B, plan.swapped ? K : N, plan.swapped ? N : K, M, g, plan.split, plan.bn, sm_count(), cur_stream()),
+           "gemm (weight gradient)");
 }
 
 }  // namespace terra_ops
@@ -205,19 +211,28 @@ Norm norm_fwd(const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
   return n;
 }
 Tensor norm_bwd(const Tensor& dxn, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, const Tensor& gw,
-                const Tensor& gb, const Tensor& dres) {
+                const Tensor& gb, const Tensor& dres, const OptTensor& dres_sum) {
   need(rows_bf16(x) && rows_bf16(dxn) && rows_bf16(dres) && dxn.sizes() == x.sizes() && dres.sizes() == x.sizes(),
        "block half: x and its gradients must be contiguous [rows, C]");
   need(vec(w, torch::kBFloat16, x.size(1)) && vec(mean, torch::kFloat32, x.size(0)) && vec(rstd, torch::kFloat32, x.size(0)),
        "block half: norm weight bf16, row statistics fp32");
   need(vec(gw, torch::kFloat32, x.size(1)) && vec(gb, torch::kFloat32, x.size(1)), "block half: norm gradients fp32");
+  need(!dres_sum.has_value() || vec(*dres_sum, torch::kFloat32, x.size(1)), "block half: bias gradient fp32, one entry per column");
   Tensor dx = torch::empty_like(x);
   tb::note_launch();
   rc_check(tb::layernorm_bwd(dxn.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(),
                              gw.data_ptr<float>(), gb.data_ptr<float>(), dres.data_ptr(), x.size(0), static_cast<int>(x.size(1)),
-                             cur_stream()),
+                             cur_stream(), dres_sum.has_value() ? dres_sum->data_ptr<float>() : nullptr),
            "layernorm_bwd");
   return dx;
+}
+
+// The bias gradient of a half's last product is the column sums of dy, which the LayerNorm's backward pass reads for the shortcut. For
+// wide rows they are taken there: the weight gradient may then use tiles 256 wide, which have no room for them, without two launches that
+// read dy once more (attention half of 156672 x 1024 4845 -> 4794 us). Narrower rows gain nothing (MLP half of 139264 x 384 1388 / 1401: the
+// kernel spills), few rows would pay for half as many atomics again at the end of the kernel, and above 1024 columns it spills more.
+bool sums_beside_norm(const Tensor& dy, bool fuse_bias) {
+  return fuse_bias && dy.size(0) >= 32768 && dy.size(1) > 512 && dy.size(1) <= 1024;
 }
 
 // Window geometry of a rank that owns every window and token: {B, nWh, nWw, wh, ww, heads, sh, sw, use_mask}
@@ -294,7 +309,8 @@ Tensor attn_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, cons
   need(rows_bf16(x) && rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: x and dy contiguous [rows, C]");
   need(rows_bf16(qkv) && qkv.size(0) == x.size(0) && qkv.size(1) == 3 * x.size(1), "block half: qkv contiguous [rows, 3 C]");
   tb::WindowAttnArgs a = window_args(geo, x.size(1), table, scale, x.size(0));
-  wgrad(dy, o, proj_wg, proj_bg, fuse_bias, status);
+  const bool beside = sums_beside_norm(dy, fuse_bias);
+  wgrad(dy, o, proj_wg, beside ? OptTensor() : OptTensor(proj_bg), fuse_bias, status);
   Tensor dout = torch::empty_like(x), dqkv = torch::empty_like(qkv), dxn = torch::empty_like(x);
   product(dy, proj_w, true, dout, Epi(), status);
   a.qkv[0] = qkv.data_ptr();
@@ -308,7 +324,7 @@ Tensor attn_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, cons
   rc_check(tb::window_attn_bwd(a, cur_stream()), "window_attn_bwd");
   wgrad(dqkv, xn, qkv_wg, qkv_bg, fuse_bias, status);
   product(dqkv, qkv_w, true, dxn, Epi(), status);
-  return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy);
+  return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy, beside ? OptTensor(proj_bg) : OptTensor());
 }
 
 // y alone, where no backward pass follows: the pre-activation is not written
@@ -352,14 +368,15 @@ Tensor mlp_half_bwd(const Tensor& dy, const Tensor& x, const Tensor& mean, const
                     bool fuse_bias, const Tensor& status) {
   const c10::cuda::CUDAGuard guard(x.device());
   need(rows_bf16(x) && rows_bf16(dy) && dy.sizes() == x.sizes(), "block half: x and dy contiguous [rows, C]");
-  wgrad(dy, act, fc2_wg, fc2_bg, fuse_bias, status);
+  const bool beside = sums_beside_norm(dy, fuse_bias);
+  wgrad(dy, act, fc2_wg, beside ? OptTensor() : OptTensor(fc2_bg), fuse_bias, status);
   Tensor dpre = torch::empty({x.size(0), fc2_w.size(1)}, x.options()), dxn = torch::empty_like(x);
   Epi e;
   e.aux = &pre;
   product(dy, fc2_w, true, dpre, e, status);
   wgrad(dpre, xn, fc1_wg, fc1_bg, fuse_bias, status);
   product(dpre, fc1_w, true, dxn, Epi(), status);
-  return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy);
+  return norm_bwd(dxn, x, ln_w, mean, rstd, ln_wg, ln_bg, dy, beside ? OptTensor(fc2_bg) : OptTensor());
 }
 
 }  // namespace terra_ops

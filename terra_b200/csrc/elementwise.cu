@@ -110,14 +110,15 @@ __global__ void __launch_bounds__(256, VPL == 1 ? 6 : (VPL == 2 ? 5 : (VPL <= 4 
   }
 }
 
-template <int LPR, int VPL, bool EXACT>
-__global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 ? 3 : 2))) layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
+// SUMS: dsum += the column sums of dres as well, which passes through here anyway (the bias gradient of the layer before the shortcut).
+template <int LPR, int VPL, bool EXACT, bool SUMS>
+__global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= (SUMS ? 3 : 4) ? 3 : 2))) layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                             const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ gamma,
                                                             const float* __restrict__ mean, const float* __restrict__ rstd,
                                                             __nv_bfloat16* __restrict__ dx, float* __restrict__ dgamma,
                                                             float* __restrict__ dbeta, const __nv_bfloat16* __restrict__ dres,
-                                                            long long rows, int C) {
+                                                            long long rows, int C, float* __restrict__ dsum) {
   chain_begin();
   constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31, sub = lane % LPR;
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 
   for (int i = 0; i < VPL; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) ag[i][j] = ab[i][j] = 0.f;
+  float as[SUMS ? VPL : 1][8] = {};
   uint4 gq[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
@@ -199,6 +201,10 @@ __global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] += rr[j];
           }
+          if constexpr (SUMS) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) as[i][j] += rr[j];
+          }
           or_[vi] = pack8(o);
         }
       }
@@ -206,14 +212,19 @@ __global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 
   }
   // the warp's row groups first (lanes sub, sub + LPR, ... hold the same columns), then the block's warps through shared
   // memory, then one atomic per column
-  extern __shared__ float sh[];   // [2][C]
-  for (int c = threadIdx.x; c < 2 * C; c += blockDim.x) sh[c] = 0.f;
+  extern __shared__ float sh[];   // [2 or 3][C]
+  for (int c = threadIdx.x; c < (SUMS ? 3 : 2) * C; c += blockDim.x) sh[c] = 0.f;
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     const int vi = sub + i * LPR;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+      if constexpr (SUMS) {
+#pragma unroll
+        for (int o = LPR; o < 32; o <<= 1) as[i][j] += __shfl_xor_sync(0xffffffffu, as[i][j], o);
+        if (lane < LPR && (EXACT || vi < nvec)) atomicAdd(&sh[2 * C + vi * 8 + j], as[i][j]);
+      }
 #pragma unroll
       for (int o = LPR; o < 32; o <<= 1) {
         ag[i][j] += __shfl_xor_sync(0xffffffffu, ag[i][j], o);
@@ -229,6 +240,7 @@ __global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
     atomicAdd(&dgamma[c], sh[c]);
     atomicAdd(&dbeta[c], sh[C + c]);
+    if constexpr (SUMS) atomicAdd(&dsum[c], sh[2 * C + c]);
   }
 }
 
@@ -1045,12 +1057,20 @@ int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, f
 }
 
 int layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
-                  float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream) {
-  if (C % 8 != 0 || C > 2048) return -1;
+                  float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream, float* dres_sum) {
+  if (C % 8 != 0 || C > 2048 || (dres_sum != nullptr && dres == nullptr)) return -1;
+  if (dres_sum != nullptr) {
+    const size_t sh3 = 3 * C * sizeof(float);
+    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (launch_chained(layernorm_bwd_kernel<LPR, VPL, EXACT, true>, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh3, stream,
+                              static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+                              static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma,
+                              dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C, dres_sum)));
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
   const size_t sh = 2 * C * sizeof(float);
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (launch_chained(layernorm_bwd_kernel<LPR, VPL, EXACT>, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh, stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (launch_chained(layernorm_bwd_kernel<LPR, VPL, EXACT, false>, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh, stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
                             static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma,
-                            dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C)));
+                            dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C, nullptr)));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

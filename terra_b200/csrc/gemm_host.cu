@@ -281,6 +281,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   }
   p.split_k = split_k;
   if (split_k > 1 && !((epi.flags & EPI_ATOMIC) && (epi.flags & EPI_OUT_F32))) return -10;
+  if ((epi.flags & EPI_TRANSPOSE) && (!(epi.flags & EPI_ATOMIC) || !(epi.flags & EPI_OUT_F32) || !A.mn_major || scatter_c)) return -18;
   p.a_mode = A.mn_major ? OP_MNMAJOR_2D : OP_KMAJOR_2D;
   p.b_mode = B.mn_major ? OP_MNMAJOR_2D : OP_KMAJOR_2D;
   int rc;

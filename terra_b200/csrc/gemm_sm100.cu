@@ -4,13 +4,13 @@
 //
 // Roles inside a 480-thread CTA (one CTA per SM, tiles assigned round-robin):
 //   warp 0, warp 14  one elected lane each issues the TMA loads of A and of B (per-CTA, no cluster fan-out) into a ring of
-//            128-byte-swizzled shared-memory stages, signalling `full[s]` by transaction bytes;
+//            128-byte-swizzled shared-memory stages, signalling `full[s]` (of a pair: the leader's) by transaction bytes;
 //   warp 1   owns the TMEM allocation; one elected lane issues tcgen05.mma (M=128, N=BN, K=16)
 //            and commits to `empty[s]` (stage reusable) and `tfull[a]` (accumulator a complete);
 //   warps 2-13 epilogue (three per 32-lane TMEM quadrant, interleaved over the columns): tcgen05.ld, fused bias / GELU /
 //            residual / GELU-gradient; bf16 outputs leave as units of 32 rows (or pixels) x 64 columns through TMA stores,
 //            fp32 split-K atomics and what does not fit a tensor map as 32-column chunks through an exchange buffer.
-// Two accumulators (2*BN TMEM columns) let the epilogue of tile i overlap the main loop of tile i+1.
+// Two accumulators (2*BN TMEM columns) let the epilogue of tile i overlap the main loop of tile i+1 (tiles 384 wide have one).
 //
 // Operand addressing is data driven (see gemm_sm100.cuh) so that the same kernel serves
 //   * linear layers forward (K-major x K-major),
@@ -921,7 +921,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               }
             }
           }
-          if (p.epi & EPI_OUT_F32) {
+          if (p.epi & EPI_TRANSPOSE) {
+            // a column of the chunk is 32 consecutive rows, one per lane: 128 bytes of the transposed output
+            const int g = static_cast<int>(out_row(q * 32 + lane));
+            float* o = static_cast<float*>(p.C) + g;
+            if (g >= 0) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (cb + j < ncols_out) atomicAdd(o + static_cast<long long>(cb + j) * p.ldc, f[j]);
+            }
+          } else if (p.epi & EPI_OUT_F32) {
             // fp32 output: two passes of 16 columns through the exchange buffer (4 floats per 16-byte vector)
             float* obase = static_cast<float*>(p.C) + gofs;
             const bool vec_ok = ((reinterpret_cast<uintptr_t>(obase) & 15) == 0) && ((p.ldc & 3) == 0);

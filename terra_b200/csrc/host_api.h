@@ -22,6 +22,7 @@ enum : int {
   EPI_OUT_F32 = 1 << 5,    // C is fp32
   EPI_ATOMIC = 1 << 6,     // fp32 atomic accumulate into C (split-K)
   EPI_ROW_CONV = 1 << 7,   // rows are (w-chunk, h, b) tiles of an image of width out_w
+  EPI_TRANSPOSE = 1 << 8,  // fp32 atomic output stored as its transpose: C[col * ldc + row]
   EPI_BIAS_F32 = 1 << 9,   // bias pointer is fp32
 };
 
@@ -99,7 +100,7 @@ int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, f
                   long long rows, int C, float eps, cudaStream_t stream);
 // dx (bf16, plus `dres` when given); dgamma/dbeta accumulated atomically into fp32 buffers that the caller zeroed.
 int layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
-                  float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream);
+                  float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream, float* dres_sum = nullptr);
 // Column sums of a bf16 [rows, C] matrix into fp32 out[C] (atomic accumulate; caller zeroes out).
 int colsum_rows_per_block();
 // out[c] += column sums of the bf16 matrix x; partials: fp32 scratch of ceil(rows / colsum_rows_per_block()) x C

@@ -36,6 +36,33 @@ def test_groupnorm_silu_backward_and_statistics(B, HW, C, groups):
         assert rel(gn.weight.grad, p64[0].grad) < 1e-4 and rel(gn.bias.grad, p64[1].grad) < 1e-4
 
 
+@pytest.mark.parametrize("rows,dim", [(32767, 1024), (32768, 1024), (33000, 512), (33000, 520), (40001, 768), (33000, 1032)])
+@pytest.mark.parametrize("half", ["mlp", "attention"])
+def test_bias_gradient_beside_the_norm(rows, dim, half):
+    """Both sides of the row and width rule; fp32 sums of 3e4 values in another order: 1e-5 of the norm."""
+    from terra_b200.models.layers import MlpHalf, SwinAttentionHalf
+    from terra_b200.ops import blocks
+    from terra_b200.ops.attention import WindowGeometry
+    from terra_b200.utils.flat_params import ParamArena
+
+    torch.manual_seed(1)
+    if half == "attention":
+        if dim not in (512, 768, 1024):
+            pytest.skip("head widths are 16 to 128")
+        geo = WindowGeometry(1, 2, rows // 128, 8, 8)
+        mod = SwinAttentionHalf(0, dim, (8, 8), dim // 32).cuda()
+        rows, bias, run = geo.rows_local, mod.attn.proj.bias, lambda t: blocks.attention_half(t, mod, geo, False)
+    else:
+        mod = MlpHalf(dim, 256).cuda()
+        bias, run = mod.fc2.bias, lambda t: blocks.mlp_half(t, mod)
+    ParamArena(mod).zero_grad()
+    x = torch.randn(rows, dim, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(rows, dim, device="cuda").to(torch.bfloat16)
+    run(x).backward(dy)
+    want = dy.double().sum(0)
+    assert (bias.grad.double() - want).norm() <= 1e-5 * want.norm()
+
+
 def test_inference_skips_the_pre_activation_only():
     from terra_b200.models.layers import MlpHalf
     from terra_b200.ops import blocks

@@ -10,6 +10,8 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime.h>
 
 #include "check.h"
 #include "torch_ops.h"
@@ -268,7 +270,9 @@ struct GroupNormSilu : Function<GroupNormSilu> {
     const c10::cuda::CUDAGuard guard(dy.device());
     const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
     const Tensor x3 = x.view(flat), dy3 = dy.view(flat);
-    Tensor red = torch::zeros({x.size(0), x.size(3), 2}, x.options().dtype(torch::kFloat32));
+    // (cleared by a memory operation: half of the host time of a fill)
+    Tensor red = torch::empty({x.size(0), x.size(3), 2}, x.options().dtype(torch::kFloat32));
+    need(cudaMemsetAsync(red.data_ptr(), 0, red.nbytes(), c10::cuda::getCurrentCUDAStream().stream()) == cudaSuccess, "groupnorm: clearing the sums");
     terra_ops::groupnorm_silu_bwd_reduce(dy3, x3, s[1], s[2], s[3], red, l->groups, l->gg, l->bg);
     Tensor dx = torch::empty_like(x), dx3 = dx.view(flat);
     terra_ops::groupnorm_silu_bwd_apply(dy3, x3, s[1], red, s[2], s[3], dx3, l->groups, inverse_count(x, l->groups));

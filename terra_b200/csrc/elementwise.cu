@@ -509,10 +509,11 @@ __device__ __forceinline__ f32x2 gn_dz(const GnPair& c, f32x2 x, f32x2 dy, f32x2
   return f2_mul(f2_mul(dy, sg), f2_fma(z, f2_fma(sg, f2_both(-1.f), f2_both(1.f)), f2_both(1.f)));
 }
 
-// pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}. Bound by issue and the latency of its loads beside HBM: two channels per instruction
-// and no shared-memory atomics (us, before / this: 557056 pixels x 384 257 / 248, 17280 x 192 17.4 / 13.3; statistics of 17280 x 192 10.1 + 1.4
-// for a launch that finished them / 7.1).
-__global__ void __launch_bounds__(256, 3) groupnorm_silu_bwd_reduce_kernel(
+// pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}. Bound by issue and the latency of its loads beside HBM: two channels per instruction,
+// no shared-memory atomics, eight loads in flight per thread of two blocks (us, before / these two / eight loads: 557056 pixels x 384 257 / 244 /
+// 193, 139264 x 384 - / 68 / 54, 64800 x 192 - / 19 / 15, 17280 x 192 17.4 / 12.9 / 8.3; with three blocks the registers do not reach: 236).
+// Statistics of 17280 x 192: 10.1 and 1.4 for a launch that finished them / 7.1.
+__global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_reduce_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta, float* __restrict__ red,
     long long HW, int C, int groups, int pix_per_block, float* __restrict__ dgamma, float* __restrict__ dbeta) {
@@ -538,10 +539,10 @@ __global__ void __launch_bounds__(256, 3) groupnorm_silu_bwd_reduce_kernel(
       const long long first = static_cast<long long>(b) * HW * nvec + vi;
       const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
       const uint4* ds = reinterpret_cast<const uint4*>(dy) + first;
-      for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
-        uint4 t[2], d2[2];
+      for (long long p = p0 + threadIdx.y; p < p1; p += 4 * blockDim.y) {
+        uint4 t[4], d2[4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < 4; ++u) {
           t[u] = d2[u] = make_uint4(0u, 0u, 0u, 0u);
           if (p + u * blockDim.y < p1) {
             t[u] = xs[(p + u * blockDim.y) * nvec];
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(256, 3) groupnorm_silu_bwd_reduce_kernel(
           }
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < 4; ++u) {
           if (p + u * blockDim.y >= p1) break;
           const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, d4[4] = {d2[u].x, d2[u].y, d2[u].z, d2[u].w};
 #pragma unroll
@@ -1162,7 +1163,7 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
                               float* red, float* dgamma, float* dbeta, int B, long long HW, int C, int groups,
                               cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups) || C > GN_MAX_CHANNELS) return -1;
-  const GnShape s(B, HW, C, 256, 3, 2);
+  const GnShape s(B, HW, C, 256, 2, 4);
   launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, gn_smem(groupnorm_silu_bwd_reduce_kernel, s, C), stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
       static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups,
       s.pix, dgamma, dbeta);

@@ -36,6 +36,14 @@ Held<T> held(AutogradContext* ctx) {
   return c10::static_intrusive_pointer_cast<T>(ctx->saved_data["layer"].toCapsule());
 }
 
+// fp32 zeros that belong to one call. From the allocator, so that calls on other streams, in other threads and in captures have their own;
+// cleared by a memory operation, half of the host time of a fill kernel.
+Tensor zeroed(const Tensor& like, at::IntArrayRef sizes, const char* what) {
+  Tensor t = torch::empty(sizes, like.options().dtype(torch::kFloat32));
+  need(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), c10::cuda::getCurrentCUDAStream().stream()) == cudaSuccess, what);
+  return t;
+}
+
 // ------------------------------------------------------------------------------------------------ attention half
 struct AttnLayer : torch::CustomClassHolder {
   Tensor ln_w, ln_b, qkv_w, qkv_b, proj_w, proj_b, ln_wg, ln_bg, qkv_wg, qkv_bg, proj_wg, proj_bg, status;
@@ -144,8 +152,8 @@ Tensor linear(const Tensor& x, const Tensor& anchor, const Tensor& w, const OptT
 
 // ------------------------------------------------------------------------------------------------ 3x3 convolution
 struct ConvLayer : torch::CustomClassHolder {
-  Tensor w_fwd, b, wg, bg, staging, status;   // staging: fp32 [9, Cout, Cin], zero between uses
-  OptTensor w_dgrad;                           // given where the input needs a gradient
+  Tensor w_fwd, b, wg, bg, status;
+  OptTensor w_dgrad;      // given where the input needs a gradient
   int64_t stride, split, stack;
   bool fuse_bias;
 };
@@ -167,10 +175,12 @@ struct Conv3x3 : Function<Conv3x3> {
     const Tensor& x = s[0];
     const Tensor dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
-    const int64_t cin = l->staging.size(2);
-    terra_ops::conv3x3_wgrad(x, dy, l->staging, l->stride, l->split, l->status, c10::nullopt, c10::nullopt,
+    const int64_t cin = x.size(3);
+    // tap-major [9, Cout, Cin], folded into the (Cout, Cin, 3, 3) accumulator
+    Tensor dw9 = zeroed(x, {9, dy.size(3), cin}, "conv3x3: clearing the weight gradient");
+    terra_ops::conv3x3_wgrad(x, dy, dw9, l->stride, l->split, l->status, c10::nullopt, c10::nullopt,
                              l->fuse_bias ? OptTensor(l->bg) : OptTensor(), l->stack);
-    terra_ops::strided_add(l->staging, l->wg, 1, cin * 9, 9, true);
+    terra_ops::strided_add(dw9, l->wg, 1, cin * 9, 9);
     if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, dy.size(3)}), l->bg);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
@@ -185,26 +195,26 @@ struct Conv3x3 : Function<Conv3x3> {
 };
 
 Tensor conv3x3(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad, const Tensor& b,
-               const Tensor& wg, const Tensor& bg, const Tensor& staging, int64_t stride, int64_t split, int64_t stack, bool fuse_bias,
+               const Tensor& wg, const Tensor& bg, int64_t stride, int64_t split, int64_t stack, bool fuse_bias,
                const Tensor& status) {
   auto l = c10::make_intrusive<ConvLayer>();
-  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b = b, l->wg = wg, l->bg = bg, l->staging = staging, l->stride = stride, l->split = split;
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b = b, l->wg = wg, l->bg = bg, l->stride = stride, l->split = split;
   l->stack = stack, l->fuse_bias = fuse_bias, l->status = status;
   return Conv3x3::apply(x, weight, bias, l);
 }
 
 // ------------------------------------------------------------------------------------------------ transposed 2x2 convolution
 struct ConvTLayer : torch::CustomClassHolder {
-  Tensor w_fwd, b4, wg, bg, staging, status;   // staging: fp32 [4, Cout, Cin], zero between uses
+  Tensor w_fwd, b4, wg, bg, status;
   OptTensor w_dgrad;
-  int64_t split, stack;
+  int64_t cout, split, stack;
   bool fuse_bias;
 };
 
 struct ConvT2x2 : Function<ConvT2x2> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, const Held<ConvTLayer>& l) {
     const c10::cuda::CUDAGuard guard(x.device());
-    Tensor y = torch::empty({x.size(0), 2 * x.size(1), 2 * x.size(2), l->staging.size(1)}, x.options().dtype(torch::kBFloat16));
+    Tensor y = torch::empty({x.size(0), 2 * x.size(1), 2 * x.size(2), l->cout}, x.options().dtype(torch::kBFloat16));
     terra_ops::convt2x2(0, x.contiguous(), l->w_fwd, l->b4, y, l->status);
     ctx->save_for_backward({x});
     hold(ctx, l);
@@ -215,10 +225,10 @@ struct ConvT2x2 : Function<ConvT2x2> {
     const auto l = held<ConvTLayer>(ctx);
     const Tensor x = s[0].contiguous(), dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
-    const int64_t cout = l->staging.size(1);
-    terra_ops::convt2x2_wgrad(x, dy, l->staging, l->split, l->status, l->stack, l->fuse_bias ? OptTensor(l->bg) : OptTensor());
-    terra_ops::strided_add(l->staging, l->wg, 1, 4, cout * 4, true);
-    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, cout}), l->bg);
+    Tensor dw4 = zeroed(x, {4, l->cout, x.size(3)}, "conv_transpose2x2: clearing the weight gradient");
+    terra_ops::convt2x2_wgrad(x, dy, dw4, l->split, l->status, l->stack, l->fuse_bias ? OptTensor(l->bg) : OptTensor());
+    terra_ops::strided_add(dw4, l->wg, 1, 4, l->cout * 4);
+    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, l->cout}), l->bg);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
       dx = torch::empty(x.sizes(), x.options());
@@ -229,17 +239,17 @@ struct ConvT2x2 : Function<ConvT2x2> {
 };
 
 Tensor conv_transpose2x2(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad,
-                         const Tensor& b4, const Tensor& wg, const Tensor& bg, const Tensor& staging, int64_t split, int64_t stack,
+                         const Tensor& b4, const Tensor& wg, const Tensor& bg, int64_t cout, int64_t split, int64_t stack,
                          bool fuse_bias, const Tensor& status) {
   auto l = c10::make_intrusive<ConvTLayer>();
-  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->wg = wg, l->bg = bg, l->staging = staging, l->split = split, l->stack = stack;
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->wg = wg, l->bg = bg, l->cout = cout, l->split = split, l->stack = stack;
   l->fuse_bias = fuse_bias, l->status = status;
   return ConvT2x2::apply(x, weight, bias, l);
 }
 
 // ------------------------------------------------------------------------------------------------ GroupNorm + SiLU
 struct NormLayer : torch::CustomClassHolder {
-  Tensor g, b, gg, bg, sums;                   // sums: fp32 [B * groups * 2 + 1] (a ticket), zero between uses
+  Tensor g, b, gg, bg;
   int64_t groups;
   double eps;
   bool has_res;
@@ -255,7 +265,8 @@ struct GroupNormSilu : Function<GroupNormSilu> {
     const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
     const Tensor x3 = x.view(flat);
     Tensor stats = torch::empty({x.size(0), l->groups, 2}, x.options().dtype(torch::kFloat32));
-    terra_ops::groupnorm_mean_rstd(x3, l->sums, stats, l->groups, inverse_count(x, l->groups), l->eps);
+    Tensor sums = zeroed(x, {x.size(0) * l->groups * 2 + 1}, "groupnorm: clearing the sums");      // (and the ticket behind them)
+    terra_ops::groupnorm_mean_rstd(x3, sums, stats, l->groups, inverse_count(x, l->groups), l->eps);
     Tensor y = torch::empty_like(x), y3 = y.view(flat);
     terra_ops::groupnorm_silu_apply(x3, stats, l->g, l->b, residual.has_value() ? OptTensor(residual->view(flat)) : residual, y3, l->groups);
     ctx->save_for_backward({x, stats, l->g, l->b});
@@ -270,9 +281,7 @@ struct GroupNormSilu : Function<GroupNormSilu> {
     const c10::cuda::CUDAGuard guard(dy.device());
     const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
     const Tensor x3 = x.view(flat), dy3 = dy.view(flat);
-    // (cleared by a memory operation: half of the host time of a fill)
-    Tensor red = torch::empty({x.size(0), x.size(3), 2}, x.options().dtype(torch::kFloat32));
-    need(cudaMemsetAsync(red.data_ptr(), 0, red.nbytes(), c10::cuda::getCurrentCUDAStream().stream()) == cudaSuccess, "groupnorm: clearing the sums");
+    Tensor red = zeroed(x, {x.size(0), x.size(3), 2}, "groupnorm: clearing the gradient's sums");
     terra_ops::groupnorm_silu_bwd_reduce(dy3, x3, s[1], s[2], s[3], red, l->groups, l->gg, l->bg);
     Tensor dx = torch::empty_like(x), dx3 = dx.view(flat);
     terra_ops::groupnorm_silu_bwd_apply(dy3, x3, s[1], red, s[2], s[3], dx3, l->groups, inverse_count(x, l->groups));
@@ -281,9 +290,9 @@ struct GroupNormSilu : Function<GroupNormSilu> {
 };
 
 Tensor groupnorm_silu(const Tensor& x, const Tensor& gamma, const Tensor& beta, const OptTensor& residual, const Tensor& g, const Tensor& b,
-                      const Tensor& gg, const Tensor& bg, const Tensor& sums, int64_t groups, double eps) {
+                      const Tensor& gg, const Tensor& bg, int64_t groups, double eps) {
   auto l = c10::make_intrusive<NormLayer>();
-  l->g = g, l->b = b, l->gg = gg, l->bg = bg, l->sums = sums, l->groups = groups, l->eps = eps, l->has_res = residual.has_value();
+  l->g = g, l->b = b, l->gg = gg, l->bg = bg, l->groups = groups, l->eps = eps, l->has_res = residual.has_value();
   return GroupNormSilu::apply(x, gamma, beta, residual, l);
 }
 

@@ -100,25 +100,25 @@ void groupnorm_silu_bwd_reduce(const torch::Tensor& dy, const torch::Tensor& x, 
            "groupnorm_silu_bwd_reduce");
 }
 
-void groupnorm_finalize(torch::Tensor& sums, torch::Tensor& stats, double inv_count, double eps, bool clear) {
+void groupnorm_finalize(torch::Tensor& sums, torch::Tensor& stats, double inv_count, double eps) {
   need(sums.is_cuda() && sums.is_contiguous() && stats.is_contiguous() && sums.scalar_type() == torch::kFloat32 &&
            stats.scalar_type() == torch::kFloat32 && sums.numel() == stats.numel() && sums.numel() % 2 == 0,
        "groupnorm_finalize: fp32 [cells, 2] sums and stats");
   const c10::cuda::CUDAGuard guard(sums.device());
   tb::note_launch();
   rc_check(tb::groupnorm_finalize(sums.data_ptr<float>(), stats.data_ptr<float>(), static_cast<int>(sums.numel() / 2),
-                                  static_cast<float>(inv_count), static_cast<float>(eps), clear ? 1 : 0, cur_stream()),
+                                  static_cast<float>(inv_count), static_cast<float>(eps), cur_stream()),
            "groupnorm_finalize");
 }
 
-void strided_add(torch::Tensor& src, torch::Tensor& dst, int64_t sa, int64_t sb, int64_t sc, bool clear) {
+void strided_add(const torch::Tensor& src, torch::Tensor& dst, int64_t sa, int64_t sb, int64_t sc) {
   need(src.is_cuda() && src.is_contiguous() && src.dim() == 3 && src.scalar_type() == torch::kFloat32 &&
            dst.scalar_type() == torch::kFloat32 && dst.is_contiguous() && dst.numel() == src.numel(),
        "strided_add: fp32 src [a, b, c] contiguous, dst contiguous with as many elements");
   const c10::cuda::CUDAGuard guard(src.device());
   tb::note_launch();
   rc_check(tb::strided_add_f32(src.data_ptr<float>(), dst.data_ptr<float>(), static_cast<int>(src.size(0)),
-                               static_cast<int>(src.size(1)), static_cast<int>(src.size(2)), sa, sb, sc, clear ? 1 : 0,
+                               static_cast<int>(src.size(1)), static_cast<int>(src.size(2)), sa, sb, sc,
                                cur_stream()),
            "strided_add");
 }

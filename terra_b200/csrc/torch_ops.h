@@ -24,8 +24,8 @@ void groupnorm_silu_apply(const Tensor& x, const Tensor& stats, const Tensor& g,
                           int64_t groups);
 void groupnorm_silu_bwd_reduce(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, Tensor& red,
                                int64_t groups, const OptTensor& dgamma, const OptTensor& dbeta);
-void groupnorm_finalize(Tensor& sums, Tensor& stats, double inv_count, double eps, bool clear);
-void strided_add(Tensor& src, Tensor& dst, int64_t sa, int64_t sb, int64_t sc, bool clear);
+void groupnorm_finalize(Tensor& sums, Tensor& stats, double inv_count, double eps);
+void strided_add(const Tensor& src, Tensor& dst, int64_t sa, int64_t sb, int64_t sc);
 void groupnorm_silu_bwd_apply(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& red, const Tensor& g, const Tensor& b,
                               Tensor& dx, int64_t groups, double inv_count);
 

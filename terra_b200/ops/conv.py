@@ -72,20 +72,6 @@ def pack_conv3x3_weight_dgrad(w: torch.Tensor) -> torch.Tensor:
     return _pack_taps(w, 1, 0, cin, 9, cout, cin * 9, range(8, -1, -1))
 
 
-_SCRATCH = {}
-
-
-def _zero_scratch(device, shape, tag):
-    """Persistent fp32 staging that is handed out zeroed and comes back zeroed (its consumer clears it behind the
-    read), so that no fill kernel runs per use."""
-    key = (torch.device(device).index, tuple(shape), tag)
-    buf = _SCRATCH.get(key)
-    if buf is None:
-        buf = torch.zeros(*shape, device=device, dtype=torch.float32)
-        _SCRATCH[key] = buf
-    return buf
-
-
 def _arena_grad(p):
     """The parameter's fp32 gradient view in the flat arena (accumulated into in place), or None."""
     g = getattr(p, "grad", None)
@@ -125,12 +111,12 @@ class _Conv3x3Fn(torch.autograd.Function):
         gw, gb = _arena_grad(weight), _arena_grad(bias)
         split, stack = _wgrad_split(B, H, W, stride, Cout, Cin)
         if gw is not None:
-            # tap-major staging [9, Cout, Cin] (persistent, self-cleaning) folded into the arena's (Cout, Cin, 3, 3) view
-            dw9 = _zero_scratch(x.device, (9, Cout, Cin), "conv3x3")
+            # tap-major staging [9, Cout, Cin] folded into the arena's (Cout, Cin, 3, 3) view
+            dw9 = torch.zeros(9, Cout, Cin, device=x.device, dtype=torch.float32)
             # the bias gradient (column sums of dy) comes out of the same kernel
             ext.conv3x3_wgrad(x, dy, dw9, stride, split, status_word(x.device), lo, hi,
                               bias_grad=gb if FUSE_BIAS_GRAD else None, stack=stack)
-            ext.strided_add(dw9, gw, 1, Cin * 9, 9, True)
+            ext.strided_add(dw9, gw, 1, Cin * 9, 9)
             dw = None
         else:
             dw9 = torch.zeros(9, Cout, Cin, device=x.device, dtype=torch.float32)
@@ -253,7 +239,7 @@ def _conv3x3_node(x, weight, bias, stride, dom):
             _packed(weight, w16, "s2dgrad_taps", pack_conv3x3_weight_s2_dgrad)
     split, stack = _wgrad_split(B, H, W, stride, Cout, Cin)
     return ext.nodes.conv3x3(x, weight, bias, _packed(weight, w16, "fwd", pack_conv3x3_weight), wd, bias.bf16, *grads,
-                             _zero_scratch(x.device, (9, Cout, Cin), "conv3x3"), stride, split, stack, FUSE_BIAS_GRAD, status_word(x.device))
+                             stride, split, stack, FUSE_BIAS_GRAD, status_word(x.device))
 
 
 @nvtx_range("terra.conv3x3")
@@ -325,14 +311,12 @@ class _ConvT2x2Fn(torch.autograd.Function):
             # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it
             dyu = dy.view(B, H, 2, W, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B * H * W, 4 * Cout)
             wgrad = lambda dwt: wgrad_accumulate(dyu, x.reshape(-1, Cin), dwt.view(4 * Cout, Cin))
+        dwt = torch.zeros(*shape, device=x.device, dtype=torch.float32)
+        wgrad(dwt)
         if gw is not None:
-            dwt = _zero_scratch(x.device, shape, "convT")
-            wgrad(dwt)
-            ext.strided_add(dwt, gw, *layout, True)
+            ext.strided_add(dwt, gw, *layout)
             dw = None
         else:
-            dwt = torch.zeros(*shape, device=x.device, dtype=torch.float32)
-            wgrad(dwt)
             dw = dwt.view(2, 2, *shape[1:]).permute(3, 2, 0, 1)
         if gb is not None:
             if not fused:
@@ -379,7 +363,7 @@ def _conv_transpose2x2_node(x, weight, bias):
     split, stack = _wgrad_plan(4, Cout, Cin, B * H * ((W + 63) // 64))
     return _ext.load().nodes.conv_transpose2x2(
         x, weight, bias, _packed(weight, w16, "convT", _pack_convt), wd, _packed(bias, bias.bf16, "convT_bias", _pack_convt_bias), *grads,
-        _zero_scratch(x.device, (4, Cout, Cin), "convT"), split, stack, FUSE_BIAS_GRAD, status_word(x.device))
+        Cout, split, stack, FUSE_BIAS_GRAD, status_word(x.device))
 
 
 def _convt_flat_weight(weight, w16):
@@ -405,15 +389,11 @@ class _GroupNormSiluFn(torch.autograd.Function):
         multi = dom is not None and dom.world > 1
         count = float(H * W * (C // groups)) * (dom.world if multi else 1)
         stats = torch.empty(B, groups, 2, device=x.device, dtype=torch.float32)
+        sums = torch.zeros(B, groups, 2, device=x.device, dtype=torch.float32)
+        ext.groupnorm_stats(x3, sums, groups)
         if multi:
-            sums = torch.zeros(B, groups, 2, device=x.device, dtype=torch.float32)
-            ext.groupnorm_stats(x3, sums, groups)
             sums = dom.all_reduce_small(sums)
-            ext.groupnorm_finalize(sums, stats, 1.0 / count, GN_EPS, False)
-        else:
-            sums = _zero_scratch(x.device, (B, groups, 2), "gn_sums")          # cleared again by the finalize kernel
-            ext.groupnorm_stats(x3, sums, groups)
-            ext.groupnorm_finalize(sums, stats, 1.0 / count, GN_EPS, True)
+        ext.groupnorm_finalize(sums, stats, 1.0 / count, GN_EPS)
         g16 = gamma.bf16 if getattr(gamma, "bf16", None) is not None else gamma.detach().to(torch.bfloat16)
         b16 = beta.bf16 if getattr(beta, "bf16", None) is not None else beta.detach().to(torch.bfloat16)
         y = torch.empty_like(x)
@@ -454,7 +434,7 @@ def groupnorm_silu(x, gn: torch.nn.GroupNorm, residual=None, dom=None):
         if grads is not None and x.dim() == 4:
             return _ext.load().nodes.groupnorm_silu(
                 x, gn.weight, gn.bias, residual, gn.weight.bf16, gn.bias.bf16, *grads,
-                _zero_scratch(x.device, (x.shape[0] * gn.num_groups * 2 + 1,), "gn_sums"), gn.num_groups, GN_EPS)
+                gn.num_groups, GN_EPS)
         return _GroupNormSiluFn.apply(x, gn.weight, gn.bias, residual, gn.num_groups, dom)
     xc = x.permute(0, 3, 1, 2)
     if dom is not None and dom.world > 1:

@@ -2,9 +2,11 @@
 // transforms use), without the interpreter in the backward pass. A small layer is bound by the host: a Python node costs about
 // 50 us of interpreter, argument lists and hand-over of the interpreter lock for its two directions, around 40 us of launches.
 //
-// A node keeps the operands that belong to the layer (bf16 weights, gradient accumulators, packed weights) beside the tensors
-// saved for the backward pass, which go through whatever saved-tensor hooks are set. Parameter gradients are accumulated in place; the
-// parameter among the inputs (`anchor`) only makes autograd call the node when the activation needs no gradient.
+// A node keeps the operands that belong to the layer (bf16 weights, packed weights) beside the tensors saved for the backward pass, which go
+// through whatever saved-tensor hooks are set. Parameter gradients are accumulated in place: the halves and linear layers into the
+// accumulators that the forward call was given, the others into the parameter's `.grad` at the time of the backward pass, or returned to
+// autograd where it has none by then. A parameter among the inputs (`anchor`) makes autograd call the node also when the activation needs no
+// gradient.
 // Us per pass, Python node / this: attention half of 512 rows of width 96 199 / 167, residual convolution and GroupNorm of 96 x 180 pixels
 // 229 / 178, a training step of 19 such layers 2408 / 1994.
 #include <torch/csrc/autograd/custom_function.h>
@@ -43,6 +45,17 @@ Tensor zeroed(const Tensor& like, at::IntArrayRef sizes, const char* what) {
   need(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), c10::cuda::getCurrentCUDAStream().stream()) == cudaSuccess, what);
   return t;
 }
+
+// Where a parameter's gradient goes: into its fp32 accumulator, or, where there is none to add into (dropped since the forward pass),
+// into zeros that the node returns.
+struct ParamGrad {
+  Tensor into, returned;
+  ParamGrad(const Tensor& param, const char* what) {
+    const Tensor& g = param.grad();
+    if (g.defined() && g.is_cuda() && g.scalar_type() == torch::kFloat32 && g.is_contiguous()) into = g;
+    else into = returned = zeroed(param, param.sizes(), what);
+  }
+};
 
 // ------------------------------------------------------------------------------------------------ attention half
 struct AttnLayer : torch::CustomClassHolder {
@@ -152,7 +165,7 @@ Tensor linear(const Tensor& x, const Tensor& anchor, const Tensor& w, const OptT
 
 // ------------------------------------------------------------------------------------------------ 3x3 convolution
 struct ConvLayer : torch::CustomClassHolder {
-  Tensor w_fwd, b, wg, bg, status;
+  Tensor w_fwd, b, weight, bias, status;
   OptTensor w_dgrad;      // given where the input needs a gradient
   int64_t stride, split, stack;
   bool fuse_bias;
@@ -176,12 +189,13 @@ struct Conv3x3 : Function<Conv3x3> {
     const Tensor dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
     const int64_t cin = x.size(3);
-    // tap-major [9, Cout, Cin], folded into the (Cout, Cin, 3, 3) accumulator
-    Tensor dw9 = zeroed(x, {9, dy.size(3), cin}, "conv3x3: clearing the weight gradient");
+    ParamGrad gw(l->weight, "conv3x3: clearing the weight gradient"), gb(l->bias, "conv3x3: clearing the bias gradient");
+    // tap-major [9, Cout, Cin], folded into the (Cout, Cin, 3, 3) gradient
+    Tensor dw9 = zeroed(x, {9, dy.size(3), cin}, "conv3x3: clearing the weight gradient's staging");
     terra_ops::conv3x3_wgrad(x, dy, dw9, l->stride, l->split, l->status, c10::nullopt, c10::nullopt,
-                             l->fuse_bias ? OptTensor(l->bg) : OptTensor(), l->stack);
-    terra_ops::strided_add(dw9, l->wg, 1, cin * 9, 9);
-    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, dy.size(3)}), l->bg);
+                             l->fuse_bias ? OptTensor(gb.into) : OptTensor(), l->stack);
+    terra_ops::strided_add(dw9, gw.into, 1, cin * 9, 9);
+    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, dy.size(3)}), gb.into);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
       dx = torch::empty_like(x);
@@ -190,31 +204,30 @@ struct Conv3x3 : Function<Conv3x3> {
       else
         terra_ops::conv3x3_s2_dgrad(dy, *l->w_dgrad, dx, l->status);
     }
-    return {dx, Tensor(), Tensor(), Tensor()};
+    return {dx, gw.returned, gb.returned, Tensor()};
   }
 };
 
 Tensor conv3x3(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad, const Tensor& b,
-               const Tensor& wg, const Tensor& bg, int64_t stride, int64_t split, int64_t stack, bool fuse_bias,
-               const Tensor& status) {
+               int64_t stride, int64_t split, int64_t stack, bool fuse_bias, const Tensor& status) {
   auto l = c10::make_intrusive<ConvLayer>();
-  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b = b, l->wg = wg, l->bg = bg, l->stride = stride, l->split = split;
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b = b, l->weight = weight, l->bias = bias, l->stride = stride, l->split = split;
   l->stack = stack, l->fuse_bias = fuse_bias, l->status = status;
   return Conv3x3::apply(x, weight, bias, l);
 }
 
 // ------------------------------------------------------------------------------------------------ transposed 2x2 convolution
 struct ConvTLayer : torch::CustomClassHolder {
-  Tensor w_fwd, b4, wg, bg, status;
+  Tensor w_fwd, b4, weight, bias, status;
   OptTensor w_dgrad;
-  int64_t cout, split, stack;
+  int64_t split, stack;
   bool fuse_bias;
 };
 
 struct ConvT2x2 : Function<ConvT2x2> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, const Held<ConvTLayer>& l) {
     const c10::cuda::CUDAGuard guard(x.device());
-    Tensor y = torch::empty({x.size(0), 2 * x.size(1), 2 * x.size(2), l->cout}, x.options().dtype(torch::kBFloat16));
+    Tensor y = torch::empty({x.size(0), 2 * x.size(1), 2 * x.size(2), l->weight.size(1)}, x.options().dtype(torch::kBFloat16));
     terra_ops::convt2x2(0, x.contiguous(), l->w_fwd, l->b4, y, l->status);
     ctx->save_for_backward({x});
     hold(ctx, l);
@@ -225,31 +238,32 @@ struct ConvT2x2 : Function<ConvT2x2> {
     const auto l = held<ConvTLayer>(ctx);
     const Tensor x = s[0].contiguous(), dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
-    Tensor dw4 = zeroed(x, {4, l->cout, x.size(3)}, "conv_transpose2x2: clearing the weight gradient");
-    terra_ops::convt2x2_wgrad(x, dy, dw4, l->split, l->status, l->stack, l->fuse_bias ? OptTensor(l->bg) : OptTensor());
-    terra_ops::strided_add(dw4, l->wg, 1, 4, l->cout * 4);
-    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, l->cout}), l->bg);
+    const int64_t cout = dy.size(3);
+    ParamGrad gw(l->weight, "conv_transpose2x2: clearing the weight gradient"), gb(l->bias, "conv_transpose2x2: clearing the bias gradient");
+    Tensor dw4 = zeroed(x, {4, cout, x.size(3)}, "conv_transpose2x2: clearing the weight gradient's staging");
+    terra_ops::convt2x2_wgrad(x, dy, dw4, l->split, l->status, l->stack, l->fuse_bias ? OptTensor(gb.into) : OptTensor());
+    terra_ops::strided_add(dw4, gw.into, 1, 4, cout * 4);
+    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, cout}), gb.into);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
       dx = torch::empty(x.sizes(), x.options());
       terra_ops::convt2x2(1, dy, *l->w_dgrad, c10::nullopt, dx, l->status);
     }
-    return {dx, Tensor(), Tensor(), Tensor()};
+    return {dx, gw.returned, gb.returned, Tensor()};
   }
 };
 
 Tensor conv_transpose2x2(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad,
-                         const Tensor& b4, const Tensor& wg, const Tensor& bg, int64_t cout, int64_t split, int64_t stack,
-                         bool fuse_bias, const Tensor& status) {
+                         const Tensor& b4, int64_t split, int64_t stack, bool fuse_bias, const Tensor& status) {
   auto l = c10::make_intrusive<ConvTLayer>();
-  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->wg = wg, l->bg = bg, l->cout = cout, l->split = split, l->stack = stack;
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->weight = weight, l->bias = bias, l->split = split, l->stack = stack;
   l->fuse_bias = fuse_bias, l->status = status;
   return ConvT2x2::apply(x, weight, bias, l);
 }
 
 // ------------------------------------------------------------------------------------------------ GroupNorm + SiLU
 struct NormLayer : torch::CustomClassHolder {
-  Tensor g, b, gg, bg;
+  Tensor g, b, gamma, beta;
   int64_t groups;
   double eps;
   bool has_res;
@@ -281,18 +295,19 @@ struct GroupNormSilu : Function<GroupNormSilu> {
     const c10::cuda::CUDAGuard guard(dy.device());
     const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
     const Tensor x3 = x.view(flat), dy3 = dy.view(flat);
+    ParamGrad gg(l->gamma, "groupnorm: clearing the gradient"), gb(l->beta, "groupnorm: clearing the gradient");
     Tensor red = zeroed(x, {x.size(0), x.size(3), 2}, "groupnorm: clearing the gradient's sums");
-    terra_ops::groupnorm_silu_bwd_reduce(dy3, x3, s[1], s[2], s[3], red, l->groups, l->gg, l->bg);
+    terra_ops::groupnorm_silu_bwd_reduce(dy3, x3, s[1], s[2], s[3], red, l->groups, gg.into, gb.into);
     Tensor dx = torch::empty_like(x), dx3 = dx.view(flat);
     terra_ops::groupnorm_silu_bwd_apply(dy3, x3, s[1], red, s[2], s[3], dx3, l->groups, inverse_count(x, l->groups));
-    return {dx, Tensor(), Tensor(), l->has_res ? dy : Tensor(), Tensor()};
+    return {dx, gg.returned, gb.returned, l->has_res ? dy : Tensor(), Tensor()};
   }
 };
 
 Tensor groupnorm_silu(const Tensor& x, const Tensor& gamma, const Tensor& beta, const OptTensor& residual, const Tensor& g, const Tensor& b,
-                      const Tensor& gg, const Tensor& bg, int64_t groups, double eps) {
+                      int64_t groups, double eps) {
   auto l = c10::make_intrusive<NormLayer>();
-  l->g = g, l->b = b, l->gg = gg, l->bg = bg, l->groups = groups, l->eps = eps, l->has_res = residual.has_value();
+  l->g = g, l->b = b, l->gamma = gamma, l->beta = beta, l->groups = groups, l->eps = eps, l->has_res = residual.has_value();
   return GroupNormSilu::apply(x, gamma, beta, residual, l);
 }
 

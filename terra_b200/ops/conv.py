@@ -216,18 +216,14 @@ def _conv3x3_s2_dgrad(dy, w16, H, W, dom, weight=None):
     return out
 
 
-def _layer_grads(a, b):
-    """The arena gradients of two parameters where a native node may stand for their layer, else None."""
-    if not native_node():
-        return None
-    ga, gb = _arena_grad(a), _arena_grad(b)
-    return None if ga is None or gb is None else (ga, gb)
+def _native_layer(a, b) -> bool:
+    """Whether a native node may stand for the layer of two parameters (it reads their gradients again when it runs backward)."""
+    return native_node() and _arena_grad(a) is not None and _arena_grad(b) is not None
 
 
 def _conv3x3_node(x, weight, bias, stride, dom):
     """The convolution of one rank as a native autograd node; None where it is not one."""
-    grads = None if dom is not None and dom.world > 1 else _layer_grads(weight, bias)
-    if grads is None or x.dim() != 4:
+    if (dom is not None and dom.world > 1) or x.dim() != 4 or not _native_layer(weight, bias):
         return None
     ext = _ext.load()
     (B, H, W, Cin), Cout, w16 = x.shape, weight.shape[0], weight.bf16
@@ -238,7 +234,7 @@ def _conv3x3_node(x, weight, bias, stride, dom):
         wd = _packed(weight, w16, "dgrad", pack_conv3x3_weight_dgrad) if stride == 1 else \
             _packed(weight, w16, "s2dgrad_taps", pack_conv3x3_weight_s2_dgrad)
     split, stack = _wgrad_split(B, H, W, stride, Cout, Cin)
-    return ext.nodes.conv3x3(x, weight, bias, _packed(weight, w16, "fwd", pack_conv3x3_weight), wd, bias.bf16, *grads,
+    return ext.nodes.conv3x3(x, weight, bias, _packed(weight, w16, "fwd", pack_conv3x3_weight), wd, bias.bf16,
                              stride, split, stack, FUSE_BIAS_GRAD, status_word(x.device))
 
 
@@ -353,8 +349,7 @@ def _pack_convt_dgrad(w):
 
 def _conv_transpose2x2_node(x, weight, bias):
     """The transposed convolution as a native autograd node (the gathered forms); None where it is not one."""
-    grads = _layer_grads(weight, bias)
-    if grads is None or x.dim() != 4:
+    if x.dim() != 4 or not _native_layer(weight, bias):
         return None
     (B, H, W, Cin), Cout, w16 = x.shape, weight.shape[1], weight.bf16
     if not _convt_tiled(B, H, W, Cin, Cout):
@@ -362,8 +357,8 @@ def _conv_transpose2x2_node(x, weight, bias):
     wd = _packed(weight, w16, "convT_dgrad", _pack_convt_dgrad) if x.requires_grad and torch.is_grad_enabled() else None
     split, stack = _wgrad_plan(4, Cout, Cin, B * H * ((W + 63) // 64))
     return _ext.load().nodes.conv_transpose2x2(
-        x, weight, bias, _packed(weight, w16, "convT", _pack_convt), wd, _packed(bias, bias.bf16, "convT_bias", _pack_convt_bias), *grads,
-        Cout, split, stack, FUSE_BIAS_GRAD, status_word(x.device))
+        x, weight, bias, _packed(weight, w16, "convT", _pack_convt), wd, _packed(bias, bias.bf16, "convT_bias", _pack_convt_bias),
+        split, stack, FUSE_BIAS_GRAD, status_word(x.device))
 
 
 def _convt_flat_weight(weight, w16):
@@ -430,11 +425,8 @@ class _GroupNormSiluFn(torch.autograd.Function):
 def groupnorm_silu(x, gn: torch.nn.GroupNorm, residual=None, dom=None):
     """silu(group_norm(x)) [+ residual] on NHWC; statistics span the whole (global) image."""
     if x.is_cuda:
-        grads = None if dom is not None and dom.world > 1 else _layer_grads(gn.weight, gn.bias)
-        if grads is not None and x.dim() == 4:
-            return _ext.load().nodes.groupnorm_silu(
-                x, gn.weight, gn.bias, residual, gn.weight.bf16, gn.bias.bf16, *grads,
-                gn.num_groups, GN_EPS)
+        if not (dom is not None and dom.world > 1) and x.dim() == 4 and _native_layer(gn.weight, gn.bias):
+            return _ext.load().nodes.groupnorm_silu(x, gn.weight, gn.bias, residual, gn.weight.bf16, gn.bias.bf16, gn.num_groups, GN_EPS)
         return _GroupNormSiluFn.apply(x, gn.weight, gn.bias, residual, gn.num_groups, dom)
     xc = x.permute(0, 3, 1, 2)
     if dom is not None and dom.world > 1:

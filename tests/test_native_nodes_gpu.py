@@ -107,3 +107,37 @@ def test_inference_without_gradient_accumulators():
         p.grad = None
     with torch.no_grad():
         assert torch.equal(run(x, None), want)
+
+
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("change", ["dropped", "one dropped", "bound anew"])
+@pytest.mark.parametrize("kind", ["conv", "conv_s2", "up", "gn"])
+def test_gradients_go_where_the_parameters_point_in_the_backward_pass(monkeypatch, kind, change, fused):
+    """`zero_grad(set_to_none=True)` or another accumulator between the forward and the backward pass."""
+    monkeypatch.setattr(conv, "FUSE_BIAS_GRAD", fused)
+    m, x, _, run = _layer(kind)
+    arena = ParamArena(m)
+
+    def backward(t, between):
+        arena.zero_grad()
+        y = run(t, None)
+        between()
+        torch.manual_seed(4)
+        y.backward(torch.randn_like(y))
+        return [p.grad.clone() for p in m.parameters()]
+
+    def drop():
+        for p in list(m.parameters())[:1 if change == "one dropped" else 2]:
+            p.grad = None
+
+    def rebind():
+        for p in m.parameters():
+            p.grad = torch.full_like(p, 2.0)
+
+    want = backward(x.clone().requires_grad_(True), lambda: None)
+    got = backward(x.clone().requires_grad_(True), rebind if change == "bound anew" else drop)
+    for p, a, b in zip(m.parameters(), got, want):
+        assert a.shape == p.shape and _rel(a - (2.0 if change == "bound anew" else 0.0), b) < 1e-5
+    if change != "one dropped":
+        assert not arena.grad.any()      # what the parameters no longer point to stays as it was
+    check_status("cuda")

@@ -5,15 +5,20 @@
 // completed and its writes are visible, so nothing that an earlier kernel wrote or still reads may be touched before that call, and
 // every thread of every chained kernel makes it (a block that left without it could let the kernel after next start too early).
 // What it saves is the gap between two dependent launches: about 4 us between GEMMs of one stream (2 us of it the set-up of a CTA
-// pair), in chains of kernels of 5 to 50 us. Kernels that wait for another GPU are launched plainly.
+// pair), in chains of kernels of 5 to 50 us.
+//
+// Kernels that may wait for another GPU are launched plainly and call `chain_wait` instead, so that their successor starts when they have
+// ended. Let in early it would hold every SM that they leave free (a GEMM: all of its shared memory) for as long as the peer is late, and
+// work of other streams, which the peer may be waiting for in turn, would have none.
 #pragma once
 #include <cuda_runtime.h>
 #include <utility>
 
 namespace tb {
 
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  chain_wait();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 

@@ -186,6 +186,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   static_assert(STACK == 1 || (CTAS == 1 && !PEERS), "stacked tiles: one CTA, no peers");
   using Cfg = GemmCfg<BN, CTAS, STACK>;
   constexpr bool PAIR = CTAS == 2, WIDE = Cfg::WIDE;
+  auto start = []() {
+    if constexpr (PEERS) chain_wait();
+    else chain_begin();
+  };
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int stages = p.stages;
@@ -204,7 +208,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   // the alignment shift does not fit into the slack the launch is refused as a whole, before any barrier exists.
   if (stages < 1 || stages > Cfg::MAX_STAGES ||
       xchg + GEMM_EPI_WARPS * p.epi_bufs * Cfg::EPI_BUF > smem_raw + p.smem_bytes) {
-    chain_begin();
+    start();
     if (threadIdx.x == 0) report_error(p.status, TB_ERR_BAD_ARG, 0x700u, blockIdx.x, 0u);
     return;
   }
@@ -250,7 +254,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   if (PAIR) cluster_sync_all(); else __syncthreads();   // barriers and allocations of both CTAs exist from here on
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  chain_begin();        // global memory is touched from here on
+  start();        // global memory is touched from here on
   if (PAIR) {
     // the pair-wide MMA names one tensor-memory address for both CTAs: the two allocations must coincide
     if (threadIdx.x == 0 && ld_shared_cluster_u32(map_to_cta(tmem_slot, rank ^ 1)) != tmem_base) {

@@ -404,6 +404,8 @@ __device__ __forceinline__ void wa_stage_rows(__nv_bfloat16* dst, int pitch, con
   }
 }
 
+__host__ __device__ __forceinline__ bool one_rank(const WindowAttnArgs& a) { return a.n_wg * a.sp * a.tp == 1; }
+
 template <int HD, int NPAD, int HPC, int WW, bool BWD>
 __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD, NPAD, HPC, BWD>::MIN_CTAS))
     window_attn_kernel(const __grid_constant__ WindowAttnArgs a) {
@@ -466,7 +468,7 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
   WaItem cur = next;
   if (tid < N) wa_table(a, geo, next, ti, tj, tabs + tid);
   __syncthreads();
-  chain_begin();        // global memory is touched from here on
+  if (one_rank(a)) chain_begin(); else chain_wait();        // global memory is touched from here on
   if (STAGES == 2) wa_gather<Cfg, BWD>(a, tabs, smem_u32(stages), ch0, tid, q0, q1);
   for (int i = tid; i < HPC * geo.nrel; i += Cfg::THREADS) {
     const int h = i / geo.nrel, r = i % geo.nrel;
@@ -702,7 +704,7 @@ int launch(WindowAttnArgs a, cudaStream_t stream) {
   if (gx < 1) gx = 1;
   if (gx > items) gx = items;
   // (with peers a neighbour's flags order the buffers: launched plainly)
-  if (a.n_wg * a.sp * a.tp == 1) launch_chained(kernel, dim3(gx, groups), dim3(Cfg::THREADS), sb, stream, a);
+  if (one_rank(a)) launch_chained(kernel, dim3(gx, groups), dim3(Cfg::THREADS), sb, stream, a);
   else kernel<<<dim3(gx, groups), Cfg::THREADS, sb, stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -22;
 }

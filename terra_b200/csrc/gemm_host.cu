@@ -233,7 +233,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
     if (!A.mn_major || (epi.flags & EPI_BIAS) || !(epi.flags & EPI_ATOMIC) || (ctas != 1 && bn_request != 384) || gather_a || scatter_c) return -15;
     if (bn_request == 256 || (bn_request == 0 && pick_bn(N, 0) == 256)) bn_request = (N % 192 == 0) ? 192 : 128;
   }
-  const int bn = bn_request == 384 ? 384 : pick_bn(N, bn_request);
+  const int bn = ctas == 2 && bn_request == 384 ? 384 : pick_bn(N, bn_request);      // (single CTAs have no such tile: as any other width)
   p.M = static_cast<int>(M);
   p.N = static_cast<int>(N);
   p.K = static_cast<int>(K);

@@ -97,3 +97,15 @@ def test_weight_gradients_of_pairs(rows, n, k, split, bn, sums):
     assert rel(gw - 1, dy.double().t() @ x.double()) < 1e-5
     if sums:
         assert rel(gb, 1 + dy.double().sum(0)) < 1e-5
+
+
+@pytest.mark.parametrize("m,n,k", [(104, 64, 64), (1000, 384, 136), (304, 1024, 200)])      # (rows a multiple of 8: a pitch)
+@pytest.mark.parametrize("bn", [384, 100])
+def test_a_width_that_single_tiles_do_not_have_falls_back_to_the_rule(m, n, k, bn):
+    """Only a pair (1384) has tiles of 384 columns; any other width asked for is left to the rule, forward and for weight gradients."""
+    a, w, _, _ = _data(m, n, k, 1)
+    want = a.double() @ w.double().t()
+    assert ((gemm(a, w, bn=bn).double() - want).abs() <= want.abs() * 2 ** -8 + 1e-5).all()      # half a bf16 step, fp32 sums
+    gw = gemm(a.t().contiguous(), w.t().contiguous(), a_mn=True, b_mn=True, out_f32=True, accumulate=True, bn=bn)
+    assert ((gw.double() - want).norm() / want.norm()).item() < 1e-5
+    check_status("cuda")

@@ -390,6 +390,13 @@ void bind_halves(pybind11::module_& m) {
         return std::make_tuple(p.bn, p.stack, p.split);
       },
       "tile width, row blocks per tile and split of the contraction that wgrad takes");
+  m.def(
+      "wgrad_swapped",
+      [](int64_t N, int64_t K, int64_t M, bool sums) {
+        need(N > 0 && K > 0 && M > 0, "wgrad_swapped: empty operand");
+        return plan_wgrad(N, K, M, sums).swapped;
+      },
+      "whether wgrad computes x^T dy and stores its transpose (the plan is then that of K x N outputs)");
   m.def("wgrad", &wgrad, "weight (and bias) gradient of a linear layer, accumulated in fp32");
   m.def("attn_half_fwd", &attn_half_fwd);
   m.def("attn_half_bwd", &attn_half_bwd);

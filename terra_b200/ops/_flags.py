@@ -7,4 +7,5 @@ EPI_MUL_DGELU = 1 << 4
 EPI_OUT_F32 = 1 << 5
 EPI_ATOMIC = 1 << 6
 EPI_ROW_CONV = 1 << 7
+EPI_TRANSPOSE = 1 << 8      # fp32 atomic output stored as its transpose
 EPI_BIAS_F32 = 1 << 9

@@ -49,8 +49,12 @@ def wgrad_accumulate(dy: torch.Tensor, x: torch.Tensor, grad_w: torch.Tensor, gr
     same kernel (a 16-column MMA of the dy tiles against ones), which saves the separate pass over dy."""
     ext = _ext.load()
     if TRACE:
-        bn, _, split = ext.wgrad_plan(grad_w.shape[0], grad_w.shape[1], dy.shape[0], grad_b is not None and FUSE_BIAS_GRAD)
-        trace_product(dy, True, x, True, grad_w, F.EPI_OUT_F32 | F.EPI_ATOMIC, split, bn)
+        sizes = (grad_w.shape[0], grad_w.shape[1], dy.shape[0], grad_b is not None and FUSE_BIAS_GRAD)
+        bn, _, split = ext.wgrad_plan(*sizes)
+        if ext.wgrad_swapped(*sizes):
+            trace_product(x, True, dy, True, grad_w, F.EPI_OUT_F32 | F.EPI_ATOMIC | F.EPI_TRANSPOSE, split, bn)
+        else:
+            trace_product(dy, True, x, True, grad_w, F.EPI_OUT_F32 | F.EPI_ATOMIC, split, bn)
     ext.wgrad(dy, x, grad_w, grad_b, FUSE_BIAS_GRAD, status_word(dy.device))
 
 

@@ -314,6 +314,8 @@ def linear(x, lin: torch.nn.Linear, residual=None, need_dx=True):
         w16, wg = _views(lin.weight)
         b16, bg = _views(lin.bias) if lin.bias is not None else (None, None)
         if native_node((wg,)):
+            if residual is not None and residual.dim() != 2:
+                residual = residual.reshape(-1, w16.shape[0])
             return _ext.load().nodes.linear(x, lin.weight, w16, b16, wg, bg, residual, need_dx, FUSE_BIAS_GRAD, status_word(x.device))
         return _LinearFn.apply(x, lin.weight, w16, b16, wg, bg, residual, need_dx)
     y = TF.linear(x, lin.weight, lin.bias)

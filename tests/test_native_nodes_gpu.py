@@ -141,3 +141,19 @@ def test_gradients_go_where_the_parameters_point_in_the_backward_pass(monkeypatc
     if change != "one dropped":
         assert not arena.grad.any()      # what the parameters no longer point to stays as it was
     check_status("cuda")
+
+
+def test_a_residual_with_the_rows_of_several_samples():
+    m, x, res, _ = _layer("linear_res")
+    ParamArena(m)
+    x, res = x[:330], res[:330]
+    want = blocks.linear(x, m, residual=res)
+    u = res.view(2, 165, 72).detach().requires_grad_(True)
+    y = blocks.linear(x, m, residual=u)
+    assert torch.equal(y, want)
+    y.backward(torch.ones_like(y))
+    assert u.grad.shape == u.shape and (u.grad == 1).all()
+    for wrong in (res[:200], res.view(2, 165, 72)[:, :100]):      # (rows that are not there are not read)
+        with pytest.raises(RuntimeError):
+            blocks.linear(x, m, residual=wrong)
+    check_status("cuda")

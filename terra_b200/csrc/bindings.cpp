@@ -16,12 +16,12 @@ namespace {
 cudaStream_t cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
+  static const int n = [] {      // (once, whichever thread comes first)
+    int dev = 0, v = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  }
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
   return n;
 }
 

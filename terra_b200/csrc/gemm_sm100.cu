@@ -27,6 +27,7 @@
 //
 // Every wait is bounded; on expiry the CTA sets its abort flag, records the site in the
 // KernelStatus word, drains, releases TMEM and returns.
+#include <atomic>
 #include <type_traits>
 #include "chained_launch.cuh"
 #include "gemm_sm100.cuh"
@@ -1024,12 +1025,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 template <int BN, int CTAS, bool PEERS = false, int STACK = 1>
 static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t stream) {
   using Cfg = GemmCfg<BN, CTAS, STACK>;
-  static bool configured = false;
-  if (!configured) {
+  static std::atomic<bool> configured{false};      // (the backward pass launches without the interpreter's lock)
+  if (!configured.load(std::memory_order_relaxed)) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::MAX_SMEM);
     if (e != cudaSuccess) return e;
-    configured = true;
+    configured.store(true, std::memory_order_relaxed);
   }
   GemmParams p = p_in;
   if (PEERS || STACK > 1) p.epi_tma = 0;

@@ -59,6 +59,34 @@ def test_streams_side_by_side(monkeypatch, native, B, H, W, dim):
     check_status("cuda")
 
 
+def test_threads_with_streams_of_their_own():
+    """Backward passes run without the interpreter's lock while other threads go forward."""
+    import threading
+
+    from terra_b200.ops.gemm import check_status
+
+    sets = [_layers(72, s) for s in range(3)]
+    xs = [(torch.randn(1, 33, 40, 72, device="cuda") * (1 + s)).to(torch.bfloat16) for s in range(3)]
+    want = [_pass(m, a, x) for (m, a), x in zip(sets, xs)]
+    torch.cuda.synchronize()
+    got = [None] * 3
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got[i] = [_pass(*sets[i], xs[i]) for _ in range(10)]
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for w, results in zip(want, got):
+        for g in results:
+            _close(g, w)
+    check_status("cuda")
+
+
 def test_first_use_inside_a_capture():
     """Nothing that a capture only records is used by the calls beside it."""
     from terra_b200.ops import conv

@@ -101,12 +101,13 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 // operand fill plus the tensor core's reads through the shared-memory port, in KB; the column sums add 40 KB per row block,
 // shared out over the column tiles. Every split pays its start and its pass of atomics (1100 KB a row block, and 1.3 KB per
 // output block of the whole launch). Widths of 256 leave no room for the sums' accumulators: the column sums are then two
-// launches of their own, which read dy once more (10 us and 8.9 TB/s against 3.7 us per 1000 KB).
+// launches of their own, which read dy once more (10 us and 5.6 TB/s against 3.7 us per 1000 KB).
 // A pair of CTAs (request 1000 + width: 256 x 256 or 256 x 384 outputs) halves B's share and is bound by the tensor core instead: 512 or
 // 768 cycles per k-block, 74 and 140 KB of that measure as timed. Only the 384-wide tile has room for the sums (16 KB, shared out alike).
-// The constants were fitted to 11000 times: 64 to 557056 rows, 45 pairs of N and K between 96 and 4096, all widths, stacked or not, one
-// to four rounds (passes back to back in a CUDA graph); the choice is 2 % slower than the best plan on average. Without the 10 us the
-// separate sums were taken for few rows too (us, that / this rule): 512 rows of 384 x 1536 22 / 9, 2048 of 256 x 1024 19 / 9, 17280 of
+// The constants of single CTAs were fitted to 11000 times: 64 to 557056 rows, 45 pairs of N and K between 96 and 4096, all widths, stacked
+// or not, one to four rounds (passes back to back in a CUDA graph); the choice among them is 2 % slower than the best plan on average. Those of
+// pairs are not part of that fit: the figures at the end are what they were set by. Without the 10 us the separate sums were taken for few rows
+// too (us, that / this rule): 512 rows of 384 x 1536 22 / 9, 2048 of 256 x 1024 19 / 9, 17280 of
 // 192 x 2208 39 / 23, 156672 of 3072 x 1024 839 / 799. Pairs (us, best single / pair): 557056 rows of 2976 x 384 with sums 1184 / 1032,
 // without 1047 / 935, 139264 of 1536 x 384 231 / 202, 156672 of 3072 x 1024 without sums 704 / 647.
 struct WgradPlan {
@@ -155,7 +156,7 @@ WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
 namespace terra_ops {
 
 // grad_w [N, K] (fp32) += dy [M, N]^T x [M, K]; grad_b [N] += column sums of dy, from the same kernel (`fuse_bias`: a
-// 16-column MMA of the dy tiles against ones) where its accumulators fit beside the tile's (widths up to 192).
+// MMA of the dy tiles against ones) where its accumulators fit beside the tile's (single CTAs up to 192 columns, pairs of 384).
 void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTensor& grad_b, bool fuse_bias, const Tensor& status) {
   need(rows_pitched(dy) && rows_pitched(x) && dy.size(0) == x.size(0) && grad_w.scalar_type() == torch::kFloat32 && grad_w.dim() == 2 &&
            grad_w.is_cuda() && grad_w.stride(1) == 1 && grad_w.size(0) == dy.size(1) && grad_w.size(1) == x.size(1),

@@ -507,7 +507,7 @@ __device__ __forceinline__ f32x2 gn_dz(const GnPair& c, f32x2 x, f32x2 dy, f32x2
 
 // pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}. Bound by issue and the latency of its loads beside HBM: two channels per instruction,
 // no shared-memory atomics, eight loads in flight per thread of two blocks (us, before / these two / eight loads: 557056 pixels x 384 257 / 244 /
-// 193, 139264 x 384 - / 68 / 54, 64800 x 192 - / 19 / 15, 17280 x 192 17.4 / 12.9 / 8.3; with three blocks the registers do not reach: 236).
+// 193, 139264 x 384 - / 68 / 54, 64800 x 192 - / 19 / 15, 17280 x 192 17.4 / - / 8.3; with three blocks the registers do not reach: 236).
 // Statistics of 17280 x 192: 10.1 and 1.4 for a launch that finished them / 7.1.
 __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_reduce_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
@@ -1044,27 +1044,30 @@ inline int ln_bwd_blocks(int vpl, bool exact, long long rows) {
 int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                   long long rows, int C, float eps, cudaStream_t stream) {
   if (C % 8 != 0 || C > 2048) return -1;
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 16, (launch_chained(layernorm_fwd_kernel<LPR, VPL, EXACT>, grid_for(rows, 8 * (32 / LPR), ln_fwd_blocks(VPL)), 256, 0, stream, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
-                            static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(y), mean, rstd, rows, C,
-                            eps)));
+  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 16,
+                 launch_chained(layernorm_fwd_kernel<LPR, VPL, EXACT>, grid_for(rows, 8 * (32 / LPR), ln_fwd_blocks(VPL)), 256, 0, stream,
+                                static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
+                                static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(y), mean, rstd, rows, C, eps));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
                   float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream, float* dres_sum) {
   if (C % 8 != 0 || C > 2048 || (dres_sum != nullptr && dres == nullptr)) return -1;
+  auto go = [&](auto kernel, int blocks, int rows_per_block, int sums) {
+    launch_chained(kernel, grid_for(rows, rows_per_block, blocks), 128, sums * C * sizeof(float), stream,
+                   static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), mean,
+                   rstd, static_cast<__nv_bfloat16*>(dx), dgamma, dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C, dres_sum);
+  };
   if (dres_sum != nullptr) {
-    const size_t sh3 = 3 * C * sizeof(float);
-    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (launch_chained(layernorm_bwd_kernel<LPR, VPL, EXACT, true>, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh3, stream,
-                              static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
-                              static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma,
-                              dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C, dres_sum)));
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    // (of the widths that gain by it: bindings_halves.cpp, sums_beside_norm)
+    if (C <= 512 || C > 1024) return -1;
+    if (C <= 768) go(layernorm_bwd_kernel<32, 3, false, true>, ln_bwd_blocks(3, false, rows), 4, 3);
+    else go(layernorm_bwd_kernel<32, 4, false, true>, ln_bwd_blocks(4, false, rows), 4, 3);
+  } else {
+    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8,
+                   go(layernorm_bwd_kernel<LPR, VPL, EXACT, false>, ln_bwd_blocks(VPL, EXACT, rows), 4 * (32 / LPR), 2));
   }
-  const size_t sh = 2 * C * sizeof(float);
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, (launch_chained(layernorm_bwd_kernel<LPR, VPL, EXACT, false>, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, EXACT, rows)), 128, sh, stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
-                            static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma,
-                            dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C, nullptr)));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1146,9 +1149,9 @@ int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, c
                          int B, long long HW, int C, int groups, cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 6, 2);
-  launch_chained(groupnorm_silu_apply_kernel, s.grid, s.block, 0, stream, static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
-      static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(y), HW,
-      C, groups, s.pix);
+  launch_chained(groupnorm_silu_apply_kernel, s.grid, s.block, 0, stream, static_cast<const __nv_bfloat16*>(x), stats,
+                 static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
+                 static_cast<__nv_bfloat16*>(y), HW, C, groups, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1157,9 +1160,9 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
                               cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups) || C > GN_MAX_CHANNELS) return -1;
   const GnShape s(B, HW, C, 256, 2, 4);
-  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, gn_smem(groupnorm_silu_bwd_reduce_kernel, s, C), stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
-      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups,
-      s.pix, dgamma, dbeta);
+  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, gn_smem(groupnorm_silu_bwd_reduce_kernel, s, C), stream,
+                 static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
+                 static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups, s.pix, dgamma, dbeta);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1181,9 +1184,9 @@ int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, 
                              cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, 4, 2);
-  launch_chained(groupnorm_silu_bwd_apply_kernel, s.grid, s.block, groups * 2 * sizeof(float), stream, static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red,
-      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
-      static_cast<__nv_bfloat16*>(dx), HW, C, groups, inv_count, s.pix);
+  launch_chained(groupnorm_silu_bwd_apply_kernel, s.grid, s.block, groups * 2 * sizeof(float), stream,
+                 static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red, static_cast<const __nv_bfloat16*>(gamma),
+                 static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(dx), HW, C, groups, inv_count, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1191,9 +1194,9 @@ int masked_loss_fwd_bwd(const void* pred, const void* label, const void* mask, l
                         int kind, float grad_scale, float* loss_sum, void* grad, cudaStream_t stream) {
   if (n % 8 != 0 || (mask != nullptr && mask_period % 8 != 0)) return -1;
   const long long nvec = n / 8;
-  launch_chained(masked_loss_kernel, grid_for(nvec, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(pred), static_cast<const __nv_bfloat16*>(label),
-      static_cast<const __nv_bfloat16*>(mask), nvec, mask != nullptr ? mask_period / 8 : 1, kind, grad_scale, loss_sum,
-      static_cast<__nv_bfloat16*>(grad));
+  launch_chained(masked_loss_kernel, grid_for(nvec, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(pred),
+                 static_cast<const __nv_bfloat16*>(label), static_cast<const __nv_bfloat16*>(mask), nvec, mask != nullptr ? mask_period / 8 : 1, kind,
+                 grad_scale, loss_sum, static_cast<__nv_bfloat16*>(grad));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1202,13 +1205,11 @@ int adamw_step(float* master, float* exp_avg, float* exp_avg_sq, const void* gra
                float bias_corr2_sqrt, float grad_scale, cudaStream_t stream) {
   const int grid = grid_for(n, 256);
   if (grad_is_bf16)
-    launch_chained(adamw_kernel<true>, grid, 256, 0, stream, master, exp_avg, exp_avg_sq, grad,
-                                                 static_cast<__nv_bfloat16*>(param_bf16), n, lr, beta1, beta2, eps,
-                                                 weight_decay, bias_corr1, bias_corr2_sqrt, grad_scale);
+    launch_chained(adamw_kernel<true>, grid, 256, 0, stream, master, exp_avg, exp_avg_sq, grad, static_cast<__nv_bfloat16*>(param_bf16), n,
+                   lr, beta1, beta2, eps, weight_decay, bias_corr1, bias_corr2_sqrt, grad_scale);
   else
-    launch_chained(adamw_kernel<false>, grid, 256, 0, stream, master, exp_avg, exp_avg_sq, grad,
-                                                  static_cast<__nv_bfloat16*>(param_bf16), n, lr, beta1, beta2, eps,
-                                                  weight_decay, bias_corr1, bias_corr2_sqrt, grad_scale);
+    launch_chained(adamw_kernel<false>, grid, 256, 0, stream, master, exp_avg, exp_avg_sq, grad, static_cast<__nv_bfloat16*>(param_bf16), n,
+                   lr, beta1, beta2, eps, weight_decay, bias_corr1, bias_corr2_sqrt, grad_scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1220,7 +1221,7 @@ int cast_f32_to_bf16(const float* src, void* dst, long long n, cudaStream_t stre
 int add_bf16(const void* a, const void* b, void* out, long long n, cudaStream_t stream) {
   if (n % 8 != 0) return -1;
   launch_chained(add_bf16_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const uint4*>(a), static_cast<const uint4*>(b),
-                                                            static_cast<uint4*>(out), n / 8);
+                 static_cast<uint4*>(out), n / 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1230,10 +1231,10 @@ int conv_s2_col2im(const void* dcol, void* out, int B, int Ho, int Wo, int W, in
   const long long total = static_cast<long long>(B) * rows * W * (C / 8);
   if (out_f32)
     launch_chained(conv_s2_col2im_kernel<true>, grid_for(total, 256), 256, 0, stream, static_cast<const uint4*>(dcol), out, B, Ho, Wo, W,
-                                                                          C / 8, r0, rows);
+                   C / 8, r0, rows);
   else
     launch_chained(conv_s2_col2im_kernel<false>, grid_for(total, 256), 256, 0, stream, static_cast<const uint4*>(dcol), out, B, Ho, Wo, W,
-                                                                           C / 8, r0, rows);
+                   C / 8, r0, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1254,11 +1255,11 @@ int patch_relayout(const void* image, const void* add, void* patches, void* imag
     const int span = to_patches ? row_units : img_units;
     const dim3 grid((span + 256 * PATCH_UNROLL - 1) / (256 * PATCH_UNROLL), static_cast<unsigned>(rows));
     if (to_patches)
-      launch_chained(pad_patchify_kernel<V>, grid, 256, 0, stream, static_cast<const V*>(image), static_cast<V*>(patches), H, p, hn, top, lu,
-                                                       img_units, row_units, seg);
+      launch_chained(pad_patchify_kernel<V>, grid, 256, 0, stream, static_cast<const V*>(image), static_cast<V*>(patches), H, p, hn, top,
+                     lu, img_units, row_units, seg);
     else
       launch_chained(unpatchify_crop_kernel<V>, grid, 256, 0, stream, static_cast<const V*>(patches), static_cast<const V*>(add),
-                                                          static_cast<V*>(image_out), H, p, hn, top, lu, img_units, row_units, seg);
+                     static_cast<V*>(image_out), H, p, hn, top, lu, img_units, row_units, seg);
   };
   if (bytes % 16 == 0) launch(uint4{});
   else if (bytes % 8 == 0) launch(uint2{});
@@ -1273,8 +1274,8 @@ int pack_taps_bf16(const void* w, void* out, int N1, int N2, int V2, int T, int 
   PackTaps p = {N2, V2, T, C, Cpad, s1, s2, sc, {}};
   for (int t = 0; t < T; ++t) p.off[t] = offsets[t];
   const long long total = static_cast<long long>(N1) * N2 * T * (Cpad / 2);
-  launch_chained(pack_taps_kernel, grid_for(total, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(w), static_cast<uint32_t*>(out), p,
-                                                             total);
+  launch_chained(pack_taps_kernel, grid_for(total, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(w), static_cast<uint32_t*>(out),
+                 p, total);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1283,8 +1284,8 @@ int attn_rowdot(const void* o, const void* dout, float* drow, long long rows, in
   if (heads <= 0 || C % heads != 0) return -1;
   const int hd = C / heads;
   if (hd != 16 && hd != 32 && hd != 64 && hd != 128) return -1;
-  launch_chained(attn_rowdot_kernel, grid_for(rows * 32, 256), 256, 0, stream, static_cast<const uint4*>(o), static_cast<const uint4*>(dout),
-                                                                  drow, rows, C / 8, hd / 8, heads);
+  launch_chained(attn_rowdot_kernel, grid_for(rows * 32, 256), 256, 0, stream, static_cast<const uint4*>(o),
+                 static_cast<const uint4*>(dout), drow, rows, C / 8, hd / 8, heads);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1299,8 +1300,7 @@ int sum_slots_bf16(const void* src, void* out, int slots, long long n, cudaStrea
   if (n % 8 != 0 || slots < 1) return -1;
   if (bias != nullptr && (cols <= 0 || cols % 8 != 0 || n % cols != 0)) return -1;
   launch_chained(sum_slots_bf16_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const uint4*>(src), static_cast<uint4*>(out),
-                                                                  slots, n / 8, static_cast<const uint4*>(bias),
-                                                                  static_cast<const uint4*>(residual), cols > 0 ? cols / 8 : 1);
+                 slots, n / 8, static_cast<const uint4*>(bias), static_cast<const uint4*>(residual), cols > 0 ? cols / 8 : 1);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -81,7 +81,8 @@ struct GemmCfg {
   }
   static constexpr int smem_bytes(int bufs) { return stages_for(bufs) * STAGE_BYTES + fixed_bytes(bufs) + 1024; }   // + alignment slack
   // two accumulators (of alternating tiles, or of a tile's two row blocks); the allocation must be a power of two
-  // behind them two 32-column accumulators of the column sums (weight-gradient form with a bias gradient, BN <= 192)
+  // behind them two 32-column accumulators of the column sums (weight-gradient form with a bias gradient; single
+  // CTAs up to 192 columns, and pairs of 384 behind their one accumulator)
   static constexpr int SUM_COL0 = WIDE ? BN : 2 * BN;
   static constexpr int TMEM_COLS = (SUM_COL0 + 64 <= 256) ? 256 : 512;
   static constexpr bool CAN_COLSUM = (CTAS == 1 || WIDE) && SUM_COL0 + 64 <= 512;
@@ -538,8 +539,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       // after it is already on its way from HBM to L2); with one (long contractions, which want the ring and hide the epilogue)
       // it is issued when the store has read the buffer.
       // The first buffer (4 KB) stages the output; the second takes the saved pre-activation, or alternates with the first.
-      // Cycles per unit with the flags tested inside / this: bias 2400, bias and residual 3400 + 800 waiting for the input, GELU
-      // with the pre-activation 4500, times GELU' 6100 + 800. 139264 x 1536 x 384 times GELU' 334 -> 261 us, the same with GELU 260
+      // Cycles per unit with the flags tested inside: bias 2400 (now under 1300), bias and residual 3400 + 800 waiting for the input, GELU
+      // with the pre-activation 4500, times GELU' 6100 + 800. Launches, before / now: 139264 x 1536 x 384 times GELU' 334 -> 261 us, the same with GELU 260
       // -> 243, 139264 x 384 x 384 63 -> 54, 156672 x 1024 x 1024 with residual 316 -> 279, 17280 x 576 x 192 12.4 -> 10.0.
       constexpr int UNITS = BN / 64, WARPS_PER_Q = GEMM_EPI_WARPS / 4;
       uint8_t* my_out = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;

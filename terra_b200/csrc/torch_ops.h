@@ -19,12 +19,10 @@ void convt2x2_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t split
 
 void colsum(const Tensor& x, Tensor& out);
 void groupnorm_mean_rstd(const Tensor& x, Tensor& scratch, Tensor& stats, int64_t groups, double inv_count, double eps);
-void groupnorm_stats(const Tensor& x, Tensor& sums, int64_t groups);
 void groupnorm_silu_apply(const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, const OptTensor& res, Tensor& y,
                           int64_t groups);
 void groupnorm_silu_bwd_reduce(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, Tensor& red,
                                int64_t groups, const OptTensor& dgamma, const OptTensor& dbeta);
-void groupnorm_finalize(Tensor& sums, Tensor& stats, double inv_count, double eps);
 void strided_add(const Tensor& src, Tensor& dst, int64_t sa, int64_t sb, int64_t sc);
 void groupnorm_silu_bwd_apply(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& red, const Tensor& g, const Tensor& b,
                               Tensor& dx, int64_t groups, double inv_count);

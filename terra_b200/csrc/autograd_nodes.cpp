@@ -38,8 +38,7 @@ Held<T> held(AutogradContext* ctx) {
   return c10::static_intrusive_pointer_cast<T>(ctx->saved_data["layer"].toCapsule());
 }
 
-// fp32 zeros that belong to one call. From the allocator, so that calls on other streams, in other threads and in captures have their own;
-// cleared by a memory operation, half of the host time of a fill kernel.
+// fp32 zeros, cleared by a memory operation (half of the host time of a fill kernel)
 Tensor zeroed(const Tensor& like, at::IntArrayRef sizes, const char* what) {
   Tensor t = torch::empty(sizes, like.options().dtype(torch::kFloat32));
   need(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), c10::cuda::getCurrentCUDAStream().stream()) == cudaSuccess, what);
@@ -191,10 +190,11 @@ struct Conv3x3 : Function<Conv3x3> {
     const int64_t cin = x.size(3);
     ParamGrad gw(l->weight, "conv3x3: clearing the weight gradient"), gb(l->bias, "conv3x3: clearing the bias gradient");
     // tap-major [9, Cout, Cin], folded into the (Cout, Cin, 3, 3) gradient
-    Tensor dw9 = zeroed(x, {9, dy.size(3), cin}, "conv3x3: clearing the weight gradient's staging");
+    Tensor dw9 = terra_ops::scratch_take(x, {9, dy.size(3), cin});
     terra_ops::conv3x3_wgrad(x, dy, dw9, l->stride, l->split, l->status, c10::nullopt, c10::nullopt,
                              l->fuse_bias ? OptTensor(gb.into) : OptTensor(), l->stack);
     terra_ops::strided_add(dw9, gw.into, 1, cin * 9, 9);
+    terra_ops::scratch_give(dw9);
     if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, dy.size(3)}), gb.into);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
@@ -240,9 +240,10 @@ struct ConvT2x2 : Function<ConvT2x2> {
     const c10::cuda::CUDAGuard guard(dy.device());
     const int64_t cout = dy.size(3);
     ParamGrad gw(l->weight, "conv_transpose2x2: clearing the weight gradient"), gb(l->bias, "conv_transpose2x2: clearing the bias gradient");
-    Tensor dw4 = zeroed(x, {4, cout, x.size(3)}, "conv_transpose2x2: clearing the weight gradient's staging");
+    Tensor dw4 = terra_ops::scratch_take(x, {4, cout, x.size(3)});
     terra_ops::convt2x2_wgrad(x, dy, dw4, l->split, l->status, l->stack, l->fuse_bias ? OptTensor(gb.into) : OptTensor());
     terra_ops::strided_add(dw4, gw.into, 1, 4, cout * 4);
+    terra_ops::scratch_give(dw4);
     if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, cout}), gb.into);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
@@ -279,8 +280,9 @@ struct GroupNormSilu : Function<GroupNormSilu> {
     const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
     const Tensor x3 = x.view(flat);
     Tensor stats = torch::empty({x.size(0), l->groups, 2}, x.options().dtype(torch::kFloat32));
-    Tensor sums = zeroed(x, {x.size(0) * l->groups * 2 + 1}, "groupnorm: clearing the sums");      // (and the ticket behind them)
+    Tensor sums = terra_ops::scratch_take(x, {x.size(0) * l->groups * 2 + 1});      // (and the ticket behind them)
     terra_ops::groupnorm_mean_rstd(x3, sums, stats, l->groups, inverse_count(x, l->groups), l->eps);
+    terra_ops::scratch_give(sums);
     Tensor y = torch::empty_like(x), y3 = y.view(flat);
     terra_ops::groupnorm_silu_apply(x3, stats, l->g, l->b, residual.has_value() ? OptTensor(residual->view(flat)) : residual, y3, l->groups);
     ctx->save_for_backward({x, stats, l->g, l->b});

@@ -111,7 +111,7 @@ void groupnorm_finalize(torch::Tensor& sums, torch::Tensor& stats, double inv_co
            "groupnorm_finalize");
 }
 
-void strided_add(const torch::Tensor& src, torch::Tensor& dst, int64_t sa, int64_t sb, int64_t sc) {
+void strided_add(torch::Tensor& src, torch::Tensor& dst, int64_t sa, int64_t sb, int64_t sc) {
   need(src.is_cuda() && src.is_contiguous() && src.dim() == 3 && src.scalar_type() == torch::kFloat32 &&
            dst.scalar_type() == torch::kFloat32 && dst.is_contiguous() && dst.numel() == src.numel(),
        "strided_add: fp32 src [a, b, c] contiguous, dst contiguous with as many elements");
@@ -415,6 +415,8 @@ void bind_elementwise(pybind11::module_& m) {
         pybind11::arg("dgamma") = pybind11::none(), pybind11::arg("dbeta") = pybind11::none());
   m.def("groupnorm_finalize", &groupnorm_finalize);
   m.def("strided_add", &strided_add);
+  m.def("scratch_take", [](const torch::Tensor& like, const std::vector<int64_t>& sizes) { return scratch_take(like, sizes); });
+  m.def("scratch_give", &scratch_give);
   m.def("groupnorm_silu_bwd_apply", &groupnorm_silu_bwd_apply);
   m.def("masked_loss", &masked_loss);
   m.def("adamw_step", &adamw_step);

@@ -344,16 +344,18 @@ __device__ __forceinline__ void gn_block_sums(float* sh, float* buf, const float
   __syncthreads();
 }
 
-__device__ __forceinline__ void gn_finalize_cell(const float* sums, float* stats, int i, float inv_count, float eps) {
+__device__ __forceinline__ void gn_finalize_cell(float* sums, float* stats, int i, float inv_count, float eps) {
   const float mean = __ldcg(sums + 2 * i) * inv_count;
   const float var = fmaxf(__ldcg(sums + 2 * i + 1) * inv_count - mean * mean, 0.f);
   stats[2 * i] = mean;
   stats[2 * i + 1] = rsqrtf(var + eps);
+  sums[2 * i] = 0.f;
+  sums[2 * i + 1] = 0.f;
 }
 
 // Statistics: per-channel sums of the block, folded to groups, two atomics per (block, group). With `stats` the last block to finish turns
-// the sums into mean and reciprocal deviation. Sums and ticket counter belong to this launch alone and are zero before it: shared by two
-// launches, one would finalize what the other still adds to, and a ticket left at a remainder would spoil every launch after them.
+// the sums into mean and reciprocal deviation and clears them and the ticket counter. They belong to this launch alone while it runs: shared
+// by two launches at once, one would finalize what the other still adds to, and a ticket left at a remainder would spoil every launch after them.
 __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat16* __restrict__ x,
                                                               float* __restrict__ sums, long long HW, int C, int groups,
                                                               int pix_per_block, float* __restrict__ stats, unsigned int* __restrict__ ticket,
@@ -407,6 +409,7 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
   if (last) {
     __threadfence();
     for (int i = tid; i < static_cast<int>(gridDim.y) * groups; i += blockDim.x * blockDim.y) gn_finalize_cell(sums, stats, i, inv_count, eps);
+    if (tid == 0) *ticket = 0u;
   }
 }
 
@@ -576,17 +579,17 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_reduce_kernel(
   }
 }
 
-// {sum, sum of squares} per (sample, group) -> {mean, rstd}
-__global__ void groupnorm_finalize_kernel(const float* __restrict__ sums, float* __restrict__ stats, int cells, float inv_count,
+// {sum, sum of squares} per (sample, group) -> {mean, rstd}; the sums are cleared
+__global__ void groupnorm_finalize_kernel(float* __restrict__ sums, float* __restrict__ stats, int cells, float inv_count,
                                           float eps) {
   chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < cells) gn_finalize_cell(sums, stats, i, inv_count, eps);
 }
 
-// dst[a * sa + b * sb + c * sc] += src[(a * nb + b) * nc + c] (fp32). Used to fold tap-major convolution weight gradients into the
-// (Cout, Cin, kh, kw) layout of the gradient arena.
-__global__ void __launch_bounds__(256) strided_add_kernel(const float* __restrict__ src, float* __restrict__ dst, int na, int nb,
+// dst[a * sa + b * sb + c * sc] += src[(a * nb + b) * nc + c] (fp32); the source is zeroed behind the read. Used to fold tap-major convolution
+// weight gradients into the (Cout, Cin, kh, kw) layout of the gradient arena.
+__global__ void __launch_bounds__(256) strided_add_kernel(float* __restrict__ src, float* __restrict__ dst, int na, int nb,
                                                           int nc, long long sa, long long sb, long long sc) {
   chain_begin();
   const long long total = static_cast<long long>(na) * nb * nc;
@@ -596,6 +599,7 @@ __global__ void __launch_bounds__(256) strided_add_kernel(const float* __restric
     const long long t = i / nc;
     const int b = static_cast<int>(t % nb), a2 = static_cast<int>(t / nb);
     dst[a2 * sa + b * sb + c * sc] += src[i];
+    src[i] = 0.f;
   }
 }
 
@@ -1139,7 +1143,7 @@ static int groupnorm_stats_launch(const void* x, float* sums, int B, long long H
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {
   return groupnorm_stats_launch(x, sums, B, HW, C, groups, nullptr, nullptr, 0.f, 0.f, stream);
 }
-// Mean and reciprocal deviation in one launch; sums [B * groups * 2] and the ticket behind them zero before it.
+// Mean and reciprocal deviation in one launch; sums [B * groups * 2] and the ticket behind them zero before and after.
 int groupnorm_mean_rstd(const void* x, float* sums, float* stats, int B, long long HW, int C, int groups, float inv_count, float eps,
                         cudaStream_t stream) {
   return groupnorm_stats_launch(x, sums, B, HW, C, groups, stats, reinterpret_cast<unsigned int*>(sums + 2LL * B * groups), inv_count, eps, stream);
@@ -1166,13 +1170,13 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int groupnorm_finalize(const float* sums, float* stats, int cells, float inv_count, float eps, cudaStream_t stream) {
+int groupnorm_finalize(float* sums, float* stats, int cells, float inv_count, float eps, cudaStream_t stream) {
   if (cells <= 0) return 0;
   launch_chained(groupnorm_finalize_kernel, (cells + 255) / 256, 256, 0, stream, sums, stats, cells, inv_count, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int strided_add_f32(const float* src, float* dst, int na, int nb, int nc, long long sa, long long sb, long long sc, cudaStream_t stream) {
+int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa, long long sb, long long sc, cudaStream_t stream) {
   const long long total = static_cast<long long>(na) * nb * nc;
   if (total <= 0) return 0;
   launch_chained(strided_add_kernel, grid_for(total, 256), 256, 0, stream, src, dst, na, nb, nc, sa, sb, sc);

@@ -106,7 +106,7 @@ int colsum_rows_per_block();
 // out[c] += column sums of the bf16 matrix x; partials: fp32 scratch of ceil(rows / colsum_rows_per_block()) x C
 int colsum_bf16(const void* x, float* out, float* partials, long long rows, int C, long long ld, cudaStream_t stream);
 // GroupNorm statistics over NHWC bf16 [B, HW, C]: accumulates per (b, group) sum and sum of squares (fp32, zeroed).
-// `mean_rstd` finishes them in the same launch: sums [B * groups * 2] and a ticket word behind them, this call's own, zero before it.
+// `mean_rstd` finishes them in the same launch: sums [B * groups * 2] and a ticket word behind them, this call's own, zero before and after.
 int groupnorm_mean_rstd(const void* x, float* sums, float* stats, int B, long long HW, int C, int groups, float inv_count, float eps,
                         cudaStream_t stream);
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream);
@@ -121,10 +121,10 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
 int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, const float* red, const void* gamma,
                              const void* beta, void* dx, int B, long long HW, int C, int groups, float inv_count,
                              cudaStream_t stream);
-// {sum, sumsq} per (sample, group) cell -> {mean, rstd}.
-int groupnorm_finalize(const float* sums, float* stats, int cells, float inv_count, float eps, cudaStream_t stream);
-// dst[a*sa + b*sb + c*sc] += src[a][b][c] (fp32, src contiguous [na][nb][nc]).
-int strided_add_f32(const float* src, float* dst, int na, int nb, int nc, long long sa, long long sb, long long sc, cudaStream_t stream);
+// {sum, sumsq} per (sample, group) cell -> {mean, rstd}; the sums are cleared.
+int groupnorm_finalize(float* sums, float* stats, int cells, float inv_count, float eps, cudaStream_t stream);
+// dst[a*sa + b*sb + c*sc] += src[a][b][c] (fp32, src contiguous [na][nb][nc]); src is zeroed behind the read.
+int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa, long long sb, long long sc, cudaStream_t stream);
 // Masked loss: loss_sum += sum(f(pred * mask - label)), f = |.| (kind 0) or square (kind 1);
 // grad = mask * f'(.) * scale (bf16). `mask` may be null. Partial sums are fp32 atomics on loss_sum[0].
 int masked_loss_fwd_bwd(const void* pred, const void* label, const void* mask, long long n, long long mask_period,

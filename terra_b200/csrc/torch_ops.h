@@ -17,13 +17,17 @@ void convt2x2(int64_t op, const Tensor& in, const Tensor& w, const OptTensor& bi
 void convt2x2_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t split_k, const OptTensor& status, int64_t stack,
                     const OptTensor& bias_grad);
 
+// fp32 scratch that a call takes zeroed, for itself, and gives back zeroed once everything it launches with it is queued (zero_scratch.cpp)
+Tensor scratch_take(const Tensor& like, at::IntArrayRef sizes);
+void scratch_give(const Tensor& scratch);
+
 void colsum(const Tensor& x, Tensor& out);
 void groupnorm_mean_rstd(const Tensor& x, Tensor& scratch, Tensor& stats, int64_t groups, double inv_count, double eps);
 void groupnorm_silu_apply(const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, const OptTensor& res, Tensor& y,
                           int64_t groups);
 void groupnorm_silu_bwd_reduce(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, Tensor& red,
                                int64_t groups, const OptTensor& dgamma, const OptTensor& dbeta);
-void strided_add(const Tensor& src, Tensor& dst, int64_t sa, int64_t sb, int64_t sc);
+void strided_add(Tensor& src, Tensor& dst, int64_t sa, int64_t sb, int64_t sc);
 void groupnorm_silu_bwd_apply(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& red, const Tensor& g, const Tensor& b,
                               Tensor& dx, int64_t groups, double inv_count);
 

@@ -112,11 +112,12 @@ class _Conv3x3Fn(torch.autograd.Function):
         split, stack = _wgrad_split(B, H, W, stride, Cout, Cin)
         if gw is not None:
             # tap-major staging [9, Cout, Cin] folded into the arena's (Cout, Cin, 3, 3) view
-            dw9 = torch.zeros(9, Cout, Cin, device=x.device, dtype=torch.float32)
+            dw9 = ext.scratch_take(x, [9, Cout, Cin])
             # the bias gradient (column sums of dy) comes out of the same kernel
             ext.conv3x3_wgrad(x, dy, dw9, stride, split, status_word(x.device), lo, hi,
                               bias_grad=gb if FUSE_BIAS_GRAD else None, stack=stack)
             ext.strided_add(dw9, gw, 1, Cin * 9, 9)
+            ext.scratch_give(dw9)
             dw = None
         else:
             dw9 = torch.zeros(9, Cout, Cin, device=x.device, dtype=torch.float32)
@@ -307,12 +308,15 @@ class _ConvT2x2Fn(torch.autograd.Function):
             # un-shuffle dy to [pixels, (dy, dx, co)] once; both products read it
             dyu = dy.view(B, H, 2, W, 2, Cout).permute(0, 1, 3, 2, 4, 5).reshape(B * H * W, 4 * Cout)
             wgrad = lambda dwt: wgrad_accumulate(dyu, x.reshape(-1, Cin), dwt.view(4 * Cout, Cin))
-        dwt = torch.zeros(*shape, device=x.device, dtype=torch.float32)
-        wgrad(dwt)
         if gw is not None:
+            dwt = ext.scratch_take(x, shape)
+            wgrad(dwt)
             ext.strided_add(dwt, gw, *layout)
+            ext.scratch_give(dwt)
             dw = None
         else:
+            dwt = torch.zeros(*shape, device=x.device, dtype=torch.float32)
+            wgrad(dwt)
             dw = dwt.view(2, 2, *shape[1:]).permute(3, 2, 0, 1)
         if gb is not None:
             if not fused:
@@ -384,11 +388,15 @@ class _GroupNormSiluFn(torch.autograd.Function):
         multi = dom is not None and dom.world > 1
         count = float(H * W * (C // groups)) * (dom.world if multi else 1)
         stats = torch.empty(B, groups, 2, device=x.device, dtype=torch.float32)
-        sums = torch.zeros(B, groups, 2, device=x.device, dtype=torch.float32)
-        ext.groupnorm_stats(x3, sums, groups)
         if multi:
-            sums = dom.all_reduce_small(sums)
-        ext.groupnorm_finalize(sums, stats, 1.0 / count, GN_EPS)
+            sums = torch.zeros(B, groups, 2, device=x.device, dtype=torch.float32)
+            ext.groupnorm_stats(x3, sums, groups)
+            ext.groupnorm_finalize(dom.all_reduce_small(sums), stats, 1.0 / count, GN_EPS)
+        else:
+            sums = ext.scratch_take(x, [B, groups, 2])
+            ext.groupnorm_stats(x3, sums, groups)
+            ext.groupnorm_finalize(sums, stats, 1.0 / count, GN_EPS)
+            ext.scratch_give(sums)
         g16 = gamma.bf16 if getattr(gamma, "bf16", None) is not None else gamma.detach().to(torch.bfloat16)
         b16 = beta.bf16 if getattr(beta, "bf16", None) is not None else beta.detach().to(torch.bfloat16)
         y = torch.empty_like(x)

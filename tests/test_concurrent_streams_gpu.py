@@ -105,3 +105,44 @@ def test_first_use_inside_a_capture():
         graph.replay()
         torch.cuda.synchronize()
     assert rel(eager) < 5e-3 and rel(out) < 5e-3      # (outputs are rounded to bf16: 2^-9)
+
+
+def test_scratch_belongs_to_one_call_and_one_stream():
+    from terra_b200 import _ext
+
+    ext = _ext.load()
+    like = torch.zeros(1, device="cuda")
+    a, b = ext.scratch_take(like, [2, 331]), ext.scratch_take(like, [331, 2])      # two calls at once
+    assert a.shape == (2, 331) and a.data_ptr() != b.data_ptr() and not a.any() and not b.any()
+    at = a.data_ptr()
+    ext.scratch_give(a)
+    other = torch.cuda.Stream()
+    with torch.cuda.stream(other):
+        c = ext.scratch_take(like, [662])
+        assert c.data_ptr() != at
+    d = ext.scratch_take(like, [662])
+    assert d.data_ptr() == at and ext.scratch_take(like, [662]).data_ptr() not in (at, b.data_ptr())
+    ext.scratch_give(d)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):      # neither taken from the pool nor kept in it
+        e = ext.scratch_take(like, [662])
+        assert e.data_ptr() != at
+        ext.scratch_give(e)
+        f = ext.scratch_take(like, [662])
+        assert f.data_ptr() not in (e.data_ptr(), at)
+    assert ext.scratch_take(like, [662]).data_ptr() == at
+
+
+def test_idle_scratch_is_bounded():
+    from terra_b200 import _ext
+
+    ext = _ext.load()
+    like = torch.zeros(1, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    for n in range(200):      # 200 sizes of 4 MB: no more than 256 MB of them stay
+        ext.scratch_give(ext.scratch_take(like, [(1 << 20) + 8 * n]))
+    assert torch.cuda.memory_allocated() - before <= 260 << 20
+    ext.scratch_give(ext.scratch_take(like, [65 << 20]))      # larger than all that may lie idle
+    assert torch.cuda.memory_allocated() - before <= 260 << 20

@@ -166,7 +166,7 @@ Tensor linear(const Tensor& x, const Tensor& anchor, const Tensor& w, const OptT
 struct ConvLayer : torch::CustomClassHolder {
   Tensor w_fwd, b, weight, bias, status;
   OptTensor w_dgrad;      // given where the input needs a gradient
-  int64_t stride, split, stack;
+  int64_t stride, split;
   bool fuse_bias;
 };
 
@@ -187,15 +187,11 @@ struct Conv3x3 : Function<Conv3x3> {
     const Tensor& x = s[0];
     const Tensor dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
-    const int64_t cin = x.size(3);
     ParamGrad gw(l->weight, "conv3x3: clearing the weight gradient"), gb(l->bias, "conv3x3: clearing the bias gradient");
-    // tap-major [9, Cout, Cin], folded into the (Cout, Cin, 3, 3) gradient
-    Tensor dw9 = terra_ops::scratch_take(x, {9, dy.size(3), cin});
-    terra_ops::conv3x3_wgrad(x, dy, dw9, l->stride, l->split, l->status, c10::nullopt, c10::nullopt,
-                             l->fuse_bias ? OptTensor(gb.into) : OptTensor(), l->stack);
-    terra_ops::strided_add(dw9, gw.into, 1, cin * 9, 9);
+    Tensor dw9 = terra_ops::scratch_take(x, {9, x.size(3), dy.size(3)});
+    terra_ops::conv3x3_wgrad_taps(x, dy, dw9, l->stride, l->status, gb.into, l->fuse_bias, l->split);
+    terra_ops::fold_taps(dw9, gw.into);
     terra_ops::scratch_give(dw9);
-    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, dy.size(3)}), gb.into);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
       dx = torch::empty_like(x);
@@ -209,10 +205,10 @@ struct Conv3x3 : Function<Conv3x3> {
 };
 
 Tensor conv3x3(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad, const Tensor& b,
-               int64_t stride, int64_t split, int64_t stack, bool fuse_bias, const Tensor& status) {
+               int64_t stride, int64_t split, bool fuse_bias, const Tensor& status) {
   auto l = c10::make_intrusive<ConvLayer>();
-  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b = b, l->weight = weight, l->bias = bias, l->stride = stride, l->split = split;
-  l->stack = stack, l->fuse_bias = fuse_bias, l->status = status;
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b = b, l->weight = weight, l->bias = bias, l->stride = stride, l->split = split, l->fuse_bias = fuse_bias;
+  l->status = status;
   return Conv3x3::apply(x, weight, bias, l);
 }
 
@@ -220,7 +216,7 @@ Tensor conv3x3(const Tensor& x, const Tensor& weight, const Tensor& bias, const 
 struct ConvTLayer : torch::CustomClassHolder {
   Tensor w_fwd, b4, weight, bias, status;
   OptTensor w_dgrad;
-  int64_t split, stack;
+  int64_t split;
   bool fuse_bias;
 };
 
@@ -241,10 +237,9 @@ struct ConvT2x2 : Function<ConvT2x2> {
     const int64_t cout = dy.size(3);
     ParamGrad gw(l->weight, "conv_transpose2x2: clearing the weight gradient"), gb(l->bias, "conv_transpose2x2: clearing the bias gradient");
     Tensor dw4 = terra_ops::scratch_take(x, {4, cout, x.size(3)});
-    terra_ops::convt2x2_wgrad(x, dy, dw4, l->split, l->status, l->stack, l->fuse_bias ? OptTensor(gb.into) : OptTensor());
-    terra_ops::strided_add(dw4, gw.into, 1, 4, cout * 4);
+    terra_ops::convt2x2_wgrad_taps(x, dy, dw4, l->status, gb.into, l->fuse_bias, l->split);
+    terra_ops::fold_taps(dw4, gw.into);
     terra_ops::scratch_give(dw4);
-    if (!l->fuse_bias) terra_ops::colsum(dy.view({-1, cout}), gb.into);
     Tensor dx;
     if (l->w_dgrad.has_value()) {
       dx = torch::empty(x.sizes(), x.options());
@@ -255,9 +250,9 @@ struct ConvT2x2 : Function<ConvT2x2> {
 };
 
 Tensor conv_transpose2x2(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& w_fwd, const OptTensor& w_dgrad,
-                         const Tensor& b4, int64_t split, int64_t stack, bool fuse_bias, const Tensor& status) {
+                         const Tensor& b4, int64_t split, bool fuse_bias, const Tensor& status) {
   auto l = c10::make_intrusive<ConvTLayer>();
-  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->weight = weight, l->bias = bias, l->split = split, l->stack = stack;
+  l->w_fwd = w_fwd, l->w_dgrad = w_dgrad, l->b4 = b4, l->weight = weight, l->bias = bias, l->split = split;
   l->fuse_bias = fuse_bias, l->status = status;
   return ConvT2x2::apply(x, weight, bias, l);
 }

@@ -224,6 +224,69 @@ void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tens
   rc_check(rc, "convt2x2_wgrad");
 }
 
+static tb::TapPlan tap_plan(const TapPlanRequest& request, int taps, int64_t channels, int64_t N, int64_t k_blocks, bool row_sums, bool column_sums,
+                            int64_t least_split) {
+  if (!request.has_value())
+    return tb::plan_tap_wgrad(taps, static_cast<int>(channels), static_cast<int>(N), k_blocks, row_sums, column_sums, static_cast<int>(least_split),
+                              sm_count());
+  const auto& r = *request;
+  TORCH_CHECK(r.size() == 4 && r[3] >= 1 && (r[1] == 1 ? (r[0] == 128 || r[0] == 192) && (r[2] == 1 || r[2] == 2)
+                                                        : r[1] == 2 && r[2] == 1 && (r[0] == 384 || (r[0] == 256 && !column_sums))),
+              "tap plan: {columns, CTAs, row blocks, split}");
+  return {static_cast<int>(r[0]), static_cast<int>(r[1]), static_cast<int>(r[2]), static_cast<int>(r[3])};
+}
+static float* grad_ptr(const OptTensor& g, int64_t n) {
+  TORCH_CHECK(!g.has_value() || (g->is_cuda() && g->scalar_type() == torch::kFloat32 && g->is_contiguous() && g->numel() == n),
+              "bias_grad: contiguous fp32 [Cout]");
+  return g.has_value() ? g->data_ptr<float>() : nullptr;
+}
+
+void conv3x3_wgrad_taps(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t stride, const OptTensor& status, const OptTensor& bias_grad,
+                        bool fuse_bias, int64_t least_split, const TapPlanRequest& request) {
+  check_image(x, "x");
+  check_image(dy, "dy");
+  const int64_t Cin = x.size(3), Cout = dy.size(3), pixels = dy.numel() / std::max<int64_t>(Cout, 1);
+  TORCH_CHECK((stride == 1 || (stride == 2 && x.size(2) % 2 == 0)) && x.size(0) == dy.size(0) && dy.size(1) == (x.size(1) + stride - 1) / stride &&
+                  dy.size(2) == x.size(2) / stride && pixels > 0,
+              "conv3x3_wgrad_taps: grids");
+  TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == torch::kFloat32 && dw.is_contiguous() && dw.numel() == 9 * Cin * Cout, "dw: fp32 [9, Cin, Cout]");
+  float* const sums = grad_ptr(bias_grad, Cout);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t k_blocks = (dy.size(2) + 63) / 64 * dy.size(1) * dy.size(0);
+  const bool fused = fuse_bias && sums != nullptr;
+  const tb::TapPlan plan = tap_plan(request, 9, Cin, Cout, k_blocks, fused, false, least_split);
+  tb::note_launch();
+  const int rc = tb::conv3x3_wgrad_taps_bf16(x.data_ptr(), dy.data_ptr(), dw.data_ptr<float>(), x.size(0), x.size(1), x.size(2), Cin, Cout,
+                                             static_cast<int>(stride), plan, status_ptr(status), sm_count(), cur_stream(), fused ? sums : nullptr);
+  rc_check(rc, "conv3x3_wgrad_taps");
+  if (sums != nullptr && !fused) {
+    Tensor out = *bias_grad;
+    colsum(dy.view({-1, Cout}), out);
+  }
+}
+
+void convt2x2_wgrad_taps(const Tensor& x, const Tensor& dy, Tensor& dw, const OptTensor& status, const OptTensor& bias_grad, bool fuse_bias,
+                         int64_t least_split, const TapPlanRequest& request) {
+  check_image(x, "x");
+  check_image(dy, "dy");
+  const int64_t Cin = x.size(3), Cout = dy.size(3), pixels = x.numel() / std::max<int64_t>(Cin, 1);
+  TORCH_CHECK(x.size(0) == dy.size(0) && 2 * x.size(1) == dy.size(1) && 2 * x.size(2) == dy.size(2) && pixels > 0, "convt2x2_wgrad_taps: grids");
+  TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == torch::kFloat32 && dw.is_contiguous() && dw.numel() == 4 * Cin * Cout, "dw: fp32 [4, Cout, Cin]");
+  float* const sums = grad_ptr(bias_grad, Cout);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t k_blocks = (x.size(2) + 63) / 64 * x.size(1) * x.size(0);
+  const bool fused = fuse_bias && sums != nullptr;
+  const tb::TapPlan plan = tap_plan(request, 4, Cout, Cin, k_blocks, false, fused, least_split);
+  tb::note_launch();
+  const int rc = tb::convt2x2_wgrad_taps_bf16(x.data_ptr(), dy.data_ptr(), dw.data_ptr<float>(), x.size(0), x.size(1), x.size(2), Cin, Cout,
+                                              plan, status_ptr(status), sm_count(), cur_stream(), fused ? sums : nullptr);
+  rc_check(rc, "convt2x2_wgrad_taps");
+  if (sums != nullptr && !fused) {
+    Tensor out = *bias_grad;
+    colsum(dy.view({-1, Cout}), out);
+  }
+}
+
 }  // namespace terra_ops
 
 using namespace terra_ops;
@@ -269,6 +332,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("input"), py::arg("w"), py::arg("bias4"), py::arg("out"), py::arg("status"));
   m.def("convt2x2_wgrad", &convt2x2_wgrad, "2x2 / stride-2 transposed convolution: weight gradient (fp32 atomics)",
         py::arg("x"), py::arg("dy"), py::arg("dw"), py::arg("split_k"), py::arg("status"), py::arg("stack") = 1, py::arg("bias_grad") = py::none());
+  m.def("conv3x3_wgrad_taps", &conv3x3_wgrad_taps, "3x3 convolution: weight gradients of all taps as one product", py::arg("x"), py::arg("dy"),
+        py::arg("dw"), py::arg("stride"), py::arg("status"), py::arg("bias_grad") = py::none(), py::arg("fuse_bias") = true,
+        py::arg("least_split") = 1, py::arg("plan") = py::none());
+  m.def("convt2x2_wgrad_taps", &convt2x2_wgrad_taps, "2x2 / stride-2 transposed convolution: weight gradients of all taps as one product",
+        py::arg("x"), py::arg("dy"), py::arg("dw"), py::arg("status"), py::arg("bias_grad") = py::none(), py::arg("fuse_bias") = true,
+        py::arg("least_split") = 1, py::arg("plan") = py::none());
+  m.def(
+      "tap_wgrad_plan",
+      [](int64_t taps, int64_t channels, int64_t N, int64_t k_blocks, bool row_sums, bool column_sums, int64_t least_split) {
+        const tb::TapPlan p = tb::plan_tap_wgrad(static_cast<int>(taps), static_cast<int>(channels), static_cast<int>(N), k_blocks, row_sums,
+                                                 column_sums, static_cast<int>(least_split), 148);
+        return std::vector<int64_t>{p.bn, p.ctas, p.stack, p.split};
+      },
+      "the rule's plan on 148 SMs: columns, CTAs, row blocks, split", py::arg("taps"), py::arg("channels"), py::arg("n"), py::arg("k_blocks"),
+      py::arg("row_sums"), py::arg("column_sums"), py::arg("least_split") = 1);
   bind_elementwise(m);
   bind_attention(m);
   bind_halves(m);

@@ -123,6 +123,17 @@ void strided_add(torch::Tensor& src, torch::Tensor& dst, int64_t sa, int64_t sb,
            "strided_add");
 }
 
+void fold_taps(torch::Tensor& src, torch::Tensor& dst) {
+  need(src.is_cuda() && src.is_contiguous() && src.dim() == 3 && src.scalar_type() == torch::kFloat32 && src.size(0) >= 1 && src.size(0) <= 9 &&
+           dst.scalar_type() == torch::kFloat32 && dst.is_contiguous() && dst.numel() == src.numel(),
+       "fold_taps: fp32 src [taps <= 9, rows, cols] contiguous, dst contiguous with as many elements");
+  const c10::cuda::CUDAGuard guard(src.device());
+  tb::note_launch();
+  rc_check(tb::fold_taps_f32(src.data_ptr<float>(), dst.data_ptr<float>(), static_cast<int>(src.size(0)), static_cast<int>(src.size(1)),
+                             static_cast<int>(src.size(2)), cur_stream()),
+           "fold_taps");
+}
+
 void groupnorm_silu_bwd_apply(const torch::Tensor& dy, const torch::Tensor& x, const torch::Tensor& stats,
                               const torch::Tensor& red, const torch::Tensor& g, const torch::Tensor& b,
                               torch::Tensor& dx, int64_t groups, double inv_count) {
@@ -415,6 +426,7 @@ void bind_elementwise(pybind11::module_& m) {
         pybind11::arg("dgamma") = pybind11::none(), pybind11::arg("dbeta") = pybind11::none());
   m.def("groupnorm_finalize", &groupnorm_finalize);
   m.def("strided_add", &strided_add);
+  m.def("fold_taps", &fold_taps, "dst[c][r][t] += src[t][r][c], src zeroed");
   m.def("scratch_take", [](const torch::Tensor& like, const std::vector<int64_t>& sizes) { return scratch_take(like, sizes); });
   m.def("scratch_give", &scratch_give);
   m.def("groupnorm_silu_bwd_apply", &groupnorm_silu_bwd_apply);

@@ -603,6 +603,47 @@ __global__ void __launch_bounds__(256) strided_add_kernel(float* __restrict__ sr
   }
 }
 
+// dst[c][r][t] += src[t][r][c] (fp32), the source zeroed behind the read: weight gradients of all taps ([tap][displaced channel][column]) into
+// the parameter's layout. Both sides move whole lines, through a tile of 32 columns x 16 rows x taps in shared memory.
+constexpr int FOLD_COLS = 32, FOLD_ROWS = 16, FOLD_TAPS = 9;
+__global__ void __launch_bounds__(256) fold_taps_kernel(float* __restrict__ src, float* __restrict__ dst, int taps, int rows, int cols) {
+  chain_begin();
+  __shared__ float tile[FOLD_COLS][FOLD_ROWS * FOLD_TAPS + 1];
+  const int c0 = blockIdx.x * FOLD_COLS, r0 = blockIdx.y * FOLD_ROWS;
+  const int nr = min(FOLD_ROWS, rows - r0), nc = min(FOLD_COLS, cols - c0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // all loads of a thread are issued before the first use: 2 rows of every tap, 4 columns of the destination
+  constexpr int RUN = (FOLD_ROWS * FOLD_TAPS + 31) / 32;
+  float v[FOLD_ROWS / 8][FOLD_TAPS], old[FOLD_COLS / 8][RUN];
+  float* const s = src + static_cast<long long>(r0) * cols + c0 + lane;
+#pragma unroll
+  for (int k = 0; k < FOLD_ROWS / 8; ++k)
+#pragma unroll
+    for (int t = 0; t < FOLD_TAPS; ++t)
+      if (t < taps && warp + 8 * k < nr && lane < nc) v[k][t] = s[(static_cast<long long>(t) * rows + warp + 8 * k) * cols];
+#pragma unroll
+  for (int k = 0; k < FOLD_COLS / 8; ++k)
+#pragma unroll
+    for (int i = 0; i < RUN; ++i)
+      if (warp + 8 * k < nc && lane + 32 * i < nr * taps)
+        old[k][i] = dst[(static_cast<long long>(c0 + warp + 8 * k) * rows + r0) * taps + lane + 32 * i];
+#pragma unroll
+  for (int k = 0; k < FOLD_ROWS / 8; ++k)
+#pragma unroll
+    for (int t = 0; t < FOLD_TAPS; ++t)
+      if (t < taps && warp + 8 * k < nr && lane < nc) {
+        tile[lane][(warp + 8 * k) * taps + t] = v[k][t];
+        s[(static_cast<long long>(t) * rows + warp + 8 * k) * cols] = 0.f;
+      }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < FOLD_COLS / 8; ++k)
+#pragma unroll
+    for (int i = 0; i < RUN; ++i)
+      if (warp + 8 * k < nc && lane + 32 * i < nr * taps)
+        dst[(static_cast<long long>(c0 + warp + 8 * k) * rows + r0) * taps + lane + 32 * i] = old[k][i] + tile[warp + 8 * k][lane + 32 * i];
+}
+
 // pass 2: dx = rstd * (dz*gamma - s1/n - xhat * s2/n), s1 = sum_c gamma_c red[b][c][0], s2 likewise with [1]
 __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
@@ -1180,6 +1221,14 @@ int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa
   const long long total = static_cast<long long>(na) * nb * nc;
   if (total <= 0) return 0;
   launch_chained(strided_add_kernel, grid_for(total, 256), 256, 0, stream, src, dst, na, nb, nc, sa, sb, sc);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+int fold_taps_f32(float* src, float* dst, int taps, int rows, int cols, cudaStream_t stream) {
+  if (taps < 1 || taps > FOLD_TAPS) return -1;
+  if (rows <= 0 || cols <= 0) return 0;
+  const dim3 grid((cols + FOLD_COLS - 1) / FOLD_COLS, (rows + FOLD_ROWS - 1) / FOLD_ROWS);
+  launch_chained(fold_taps_kernel, grid, dim3(256), 0, stream, src, dst, taps, rows, cols);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

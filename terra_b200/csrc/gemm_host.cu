@@ -13,6 +13,7 @@ namespace tb {
 
 cudaError_t launch_gemm(const GemmParams& p, int bn, int ctas, int num_sms, cudaStream_t stream);
 cudaError_t gemm_read_stalls(unsigned long long* out8, bool reset);
+cudaError_t gemm_ones_tile(void** ptr);
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -431,19 +432,23 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
 
+static void conv3x3_taps(Tap (&taps)[9], int stride) {
+  for (int tap = 0; tap < 9; ++tap) {
+    const int dyy = tap / 3, dxx = tap % 3;
+    // stride 2: w_in = 2 wo + dxx - 1, so dxx = 0 -> parity 1 of column wo - 1; 1 -> parity 0 of wo; 2 -> parity 1 of wo
+    taps[tap].parity = static_cast<short>(stride == 1 || dxx == 1 ? 0 : 1);
+    taps[tap].dw = static_cast<short>(stride == 1 ? dxx - 1 : (dxx == 0 ? -1 : 0));
+    taps[tap].dh = static_cast<short>(dyy - 1);
+  }
+}
+
 int conv3x3_fwd_bf16(const void* x, const void* w, int B, int H, int W, int Cin, int Cout, int stride,
                      const GemmEpilogue& epi, int num_sms, cudaStream_t stream, const void* halo_lo,
                      const void* halo_hi) {
   if (stride != 1 && stride != 2) return -11;
   if (stride == 2 && (W % 2 != 0)) return -12;
   Tap taps[9];
-  for (int tap = 0; tap < 9; ++tap) {
-    const int dy = tap / 3, dx = tap % 3;
-    // stride 2: w_in = 2 wo + dx - 1, so dx = 0 -> parity 1 of column wo - 1; 1 -> parity 0 of wo; 2 -> parity 1 of wo
-    taps[tap].parity = static_cast<short>(stride == 1 || dx == 1 ? 0 : 1);
-    taps[tap].dw = static_cast<short>(stride == 1 ? dx - 1 : (dx == 0 ? -1 : 0));
-    taps[tap].dh = static_cast<short>(dy - 1);
-  }
+  conv3x3_taps(taps, stride);
   const int Ho = (stride == 1) ? H : (H + 1) / 2, Wo = (stride == 1) ? W : W / 2;
   GatherConv c = {x, B, H, W, Cin, stride, Ho, Wo, stride, taps, 9, 1, {0, 9}, w, Cout, epi.C, Ho, Wo, Cout, 1, 0, {}};
   return gather_conv(c, epi, num_sms, stream, halo_lo, halo_hi);
@@ -558,12 +563,7 @@ int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, i
   if (stride == 2 && (W % 2 != 0)) return -12;
   if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
   Tap taps[9];
-  for (int tap = 0; tap < 9; ++tap) {
-    const int dyy = tap / 3, dxx = tap % 3;
-    taps[tap].parity = static_cast<short>(stride == 1 || dxx == 1 ? 0 : 1);
-    taps[tap].dw = static_cast<short>(stride == 1 ? dxx - 1 : (dxx == 0 ? -1 : 0));
-    taps[tap].dh = static_cast<short>(dyy - 1);
-  }
+  conv3x3_taps(taps, stride);
   const int Ho = (stride == 1) ? H : (H + 1) / 2, Wo = (stride == 1) ? W : W / 2;
   return gather_wgrad(dy, x, dw, B, Ho, Wo, Cout, H, W, Cin, stride, taps, 9, split_k, status, num_sms, stream, halo_lo,
                       halo_hi, bias_grad, stack);
@@ -578,6 +578,129 @@ int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, 
   const Tap taps[4] = {{0, 0, 0}, {1, 0, 0}, {0, 0, 1}, {1, 0, 1}};
   return gather_wgrad(dy, x, dw, B, H, W, Cout, 2 * H, 2 * W, Cin, 2, taps, 4, split_k, status, num_sms, stream, nullptr,
                       nullptr, bias_grad, stack, true);
+}
+
+// All taps' weight gradients as one product (one rank): the channels of the displaced image, box after box of 64 and tap after tap, are the
+// rows, and the other image's channels the columns, so that tiles of 256 rows need no whole number of them in a tap (9 x 384 rows are 13.5 of
+// a pair's, 9 x 192 seven stacked ones where two per tap made nine). With the undisplaced image as operand B its column sums, the bias gradient of
+// a convolution, are one more row, that of a box of ones.
+//
+// The plan is the one with the least time by a model, in us: rounds of tiles over the CTAs (pairs), each its k-blocks and a hand-over with the
+// epilogue, and the atomics of all splits. Fitted to 900 passes in CUDA graphs: the two layers at 512 to 557056 pixels, 96 to 384 channels, all
+// tiles, half a round to three and more; the choice is 0.5 % slower than the best plan on average, at most 8 %.
+// Us, a product per tap (two row blocks stacked where that was ahead) / this: 557056 pixels of 384 channels 1251 / 951, of 192 383 / 275, 80000 of
+// 256 104 / 85, 17280 of 192 25 / 21; transposed, 139264 of 384 186 / 161, of 192 69 / 57, of 96 45 / 35. (Of 96 and 128 channels the row of ones
+// costs a tile in ten: 17280 pixels 12.6 / 13.5 and 16.4 / 17.2; folding the gradients takes 2 to 10 us less than it did.)
+// `least_split`: the contraction is cut into so many parts at least (the error of the tensor core's fp32 sums grows with their length: 139264
+// pixels of 384 channels, 18 parts 8.6e-6, 12 parts 13.0e-6), unless they are down to 24 k-blocks (1.6e-6).
+TapPlan plan_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool row_sums, bool column_sums, int least_split, int num_sms) {
+  struct Tile {
+    int width, ctas, stack;
+    double kblock, tile;
+  };
+  static const Tile tiles[] = {{128, 1, 1, 0.265, 2.99}, {192, 1, 1, 0.299, 2.93}, {128, 1, 2, 0.433, 6.09}, {192, 1, 2, 0.566, 5.38},
+                               {256, 2, 1, 0.345, 2.26}, {384, 2, 1, 0.515, 6.82}};
+  least_split = static_cast<int>(std::min<long long>(least_split, (k_blocks + 23) / 24));
+  const long long boxes = static_cast<long long>(taps) * ((channels + 63) / 64) + (row_sums ? 1 : 0);
+  TapPlan best = {128, 1, 1, 1};
+  double least = -1.0;
+  for (const Tile& t : tiles) {
+    if (t.ctas == 2 && (!gemm_pairs() || num_sms < 2 || t.width >= 2 * N || (t.width == 384 && N <= 256) || (t.width == 256 && column_sums))) continue;
+    if (t.width == 192 && N <= 128) continue;
+    const long long units = num_sms / t.ctas, n = (N + t.width - 1) / t.width;
+    const long long blocks = (boxes + 1) / 2, count = (blocks + t.stack * t.ctas - 1) / (t.stack * t.ctas) * n;
+    const long long least_halves = 2 * ((std::min<long long>(least_split, k_blocks) * count + units - 1) / units);      // whole rounds
+    for (long long halves : {1LL, 2LL, 4LL, 6LL, least_halves}) {      // half a round of CTAs, one, two, three, as many as it takes
+      const long long want = std::max<long long>({1, least_split, halves * units / 2 / count});
+      const long long per = (k_blocks + std::min(want, k_blocks) - 1) / std::min(want, k_blocks);
+      const long long split = (k_blocks + per - 1) / per;
+      const double outputs = static_cast<double>(count) * split * t.stack * t.ctas * 128 * std::min(t.width, N) * 4e-6;      // MB
+      const double kblock = t.kblock + (column_sums ? 0.155 * t.stack / n : 0.0);
+      const double time = static_cast<double>((count * split + units - 1) / units) * (per * kblock + t.tile) + 0.119 * outputs + (t.ctas == 2 ? 4.6 : 0.0);
+      if (least < 0.0 || time < least) {
+        least = time;
+        best = {t.width, t.ctas, t.stack, static_cast<int>(split)};
+      }
+    }
+  }
+  return best;
+}
+
+// dw[tap][channels][N] (fp32, accumulated) = sum over the pixels of b [B, Ho, Wo, N] of a [B, H, W, channels] at the pixel's tap, times b.
+// row_sums [N] += the sums of b, colsum [channels] += those of a over all taps.
+static int tap_wgrad(const void* a, const void* b, float* dw, int B, int Ho, int Wo, int channels, int H, int W, int N, int stride,
+                     const Tap* taps, int ntaps, const TapPlan& plan, void* status, int num_sms, cudaStream_t stream, float* row_sums,
+                     float* colsum) {
+  GemmParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.M = channels;
+  p.N = N;
+  p.pix_n0 = (Wo + GEMM_BK - 1) / GEMM_BK;
+  p.pix_n1 = Ho;
+  p.pix_hmul = stride;
+  p.k_blocks = p.pix_n0 * Ho * B;
+  p.K = p.k_blocks * GEMM_BK;
+  p.taps = ntaps;
+  p.tap_boxes = (channels + 63) / 64;
+  p.tap_channels = channels;
+  p.row_sums = row_sums;
+  p.m_blocks = (ntaps * p.tap_boxes + (row_sums != nullptr ? 1 : 0) + 1) / 2;
+  p.stack = plan.stack;
+  p.num_m_tiles = (p.m_blocks + plan.stack * plan.ctas - 1) / (plan.stack * plan.ctas);
+  p.num_n_tiles = (N + plan.bn - 1) / plan.bn;
+  p.groups = 1;
+  int split = std::max(1, std::min(plan.split, p.k_blocks));
+  {
+    const int per = (p.k_blocks + split - 1) / split;
+    split = (p.k_blocks + per - 1) / per;      // no empty split
+  }
+  p.split_k = split;
+  p.a_mode = OP_PIXELS_5D;
+  p.b_mode = OP_PIXELS_5D;
+  p.disp_a = 1;
+  int rc = image_map(&p.map_a, a, channels, stride, W, H, B, GEMM_BK);
+  if (rc != 0) return rc;
+  rc = image_map(&p.map_b, b, N, 1, Wo, Ho, B, GEMM_BK);
+  if (rc != 0) return rc - 1000;
+  void* ones = nullptr;      // (boxes behind the last tap are read in any case)
+  if (gemm_ones_tile(&ones) != cudaSuccess) return -20;
+  rc = map_2d(&p.map_in, ones, 64, 64, 64, 64, 64);
+  if (rc != 0) return rc - 2000;
+  for (int t = 0; t < ntaps; ++t) {
+    p.grp_off[t][0] = taps[t].parity;
+    p.grp_off[t][1] = taps[t].dw;
+    p.grp_off[t][2] = taps[t].dh;
+  }
+  p.epi = EPI_OUT_F32 | EPI_ATOMIC;
+  p.colsum = colsum;
+  p.C = dw;
+  p.ldc = N;
+  p.alpha = 1.0f;
+  p.status = static_cast<KernelStatus*>(status);
+  p.tile_n0 = 1;
+  p.tile_n1 = 1;
+  const cudaError_t e = launch_gemm(p, plan.bn, plan.ctas, num_sms, stream);
+  return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+}
+
+// 3x3 convolution on one rank: dw[tap][Cin][Cout] += ..., and bias_grad[Cout] += the sums of dy.
+int conv3x3_wgrad_taps_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride, const TapPlan& plan,
+                            void* status, int num_sms, cudaStream_t stream, float* bias_grad) {
+  if (stride != 1 && stride != 2) return -11;
+  if (stride == 2 && (W % 2 != 0)) return -12;
+  if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
+  Tap taps[9];
+  conv3x3_taps(taps, stride);
+  const int Ho = (stride == 1) ? H : (H + 1) / 2, Wo = (stride == 1) ? W : W / 2;
+  return tap_wgrad(x, dy, dw, B, Ho, Wo, Cin, H, W, Cout, stride, taps, 9, plan, status, num_sms, stream, bias_grad, nullptr);
+}
+
+// 2x2 / stride-2 transposed convolution: dw[tap][Cout][Cin] += ..., bias_grad[Cout] += the sums of dy
+int convt2x2_wgrad_taps_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, const TapPlan& plan,
+                             void* status, int num_sms, cudaStream_t stream, float* bias_grad) {
+  if (Cin % 8 != 0 || Cout % 8 != 0) return -13;
+  const Tap taps[4] = {{0, 0, 0}, {1, 0, 0}, {0, 0, 1}, {1, 0, 1}};
+  return tap_wgrad(dy, x, dw, B, H, W, Cout, 2 * H, 2 * W, Cin, 2, taps, 4, plan, status, num_sms, stream, nullptr, bias_grad);
 }
 
 int gemm_stall_counters(unsigned long long* out8, int reset) {

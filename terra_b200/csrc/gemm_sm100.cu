@@ -98,6 +98,14 @@ struct GemmCfg {
 // [3] TMA thread span, [4] of it waiting for free stages, [5] first epilogue warp span, [6] of it waiting for tiles.
 __device__ unsigned long long g_gemm_stalls[8];
 
+// 64 x 64 bf16 ones: operand rows whose product with B is B's column sums (GemmParams::tap_boxes)
+#define TB_ONES_8(v) v, v, v, v, v, v, v, v
+#define TB_ONES_64(v) TB_ONES_8(TB_ONES_8(v))
+__device__ __align__(1024) uint32_t g_ones_tile[2048] = {TB_ONES_8(TB_ONES_64(0x3F803F80u)), TB_ONES_8(TB_ONES_64(0x3F803F80u)),
+                                                         TB_ONES_8(TB_ONES_64(0x3F803F80u)), TB_ONES_8(TB_ONES_64(0x3F803F80u))};
+#undef TB_ONES_8
+#undef TB_ONES_64
+
 struct TileCoord {
   int grp, m_blk, n_blk, split;
   int kb_begin, kb_end;
@@ -112,12 +120,13 @@ __device__ __forceinline__ int first_sum_kb(const GemmParams& p, const TileCoord
   return t.kb_begin + (place + ways - t.kb_begin % ways) % ways;
 }
 
-// Walks over the tiles of a CTA (pair): tile t is the mixed-radix number (split, n, m, group) with the split varying fastest, and
-// a step adds the digits of the tile step. (Decoded by divisions a tile cost every role about 600 cycles, once per tile for the
-// loads and the MMAs and three times for the epilogue: as long as two k-blocks.)
+// Walks over the tiles of a CTA (pair): tile t is a mixed-radix number, and a step adds the digits of the tile step. (Decoded by
+// divisions a tile cost every role about 600 cycles, once per tile for the loads and the MMAs and three times for the epilogue: as long as
+// two k-blocks.) The digits are, from the fastest, (n, m, group, split): the tiles of one part of the contraction run side by side and share
+// its operands in L2, where a launch has more of them than CTAs.
 // p.num_m_tiles counts tiles of ctas * 128 rows; m_blk is in units of 128 rows for CTA `rank` of the pair.
-// Stacked tiles (p.stack = 2 blocks of rows): the row tile varies slowest, so that the last one, which may hold a single
-// block, is handed out last.
+// Stacked tiles (p.stack = 2 blocks of rows) go by (split, n, group, m): the row tile varies slowest, so that the last one, which may hold a
+// single block, is handed out last.
 template <int CTAS, int STACK>
 struct TileWalk {
   int tile, split, n, lo, hi;          // (lo, hi) = (m, group), stacked tiles (group, m)
@@ -127,22 +136,29 @@ struct TileWalk {
     digits(p, by, d_split, d_n, d_lo, d_hi);
   }
   static __device__ __forceinline__ void digits(const GemmParams& p, int t, int& split, int& n, int& lo, int& hi) {
-    const int radix = STACK > 1 ? p.groups : p.num_m_tiles;
     split = 0;
-    if (p.split_k > 1) {
+    if (STACK > 1 && p.split_k > 1) {
       split = t % p.split_k;
       t /= p.split_k;
     }
     n = t % p.num_n_tiles;
     t /= p.num_n_tiles;
+    const int radix = STACK > 1 ? p.groups : p.num_m_tiles;
     lo = t % radix;
     hi = t / radix;
+    if (STACK == 1 && p.split_k > 1) {
+      split = hi / p.groups;
+      hi -= split * p.groups;
+    }
   }
   __device__ __forceinline__ void next(const GemmParams& p) {
     tile += step;
-    split += d_split;
-    int carry = split >= p.split_k;
-    split -= carry ? p.split_k : 0;
+    int carry = 0;
+    if (STACK > 1) {
+      split += d_split;
+      carry = split >= p.split_k;
+      split -= carry ? p.split_k : 0;
+    }
     n += d_n + carry;
     carry = n >= p.num_n_tiles;
     n -= carry ? p.num_n_tiles : 0;
@@ -151,6 +167,11 @@ struct TileWalk {
     carry = lo >= radix;
     lo -= carry ? radix : 0;
     hi += d_hi + carry;
+    if (STACK == 1 && p.split_k > 1) {
+      carry = hi >= p.groups;
+      hi -= carry ? p.groups : 0;
+      split += d_split + carry;
+    }
   }
   __device__ __forceinline__ int m_blk(int rank) const { return STACK > 1 ? hi * STACK : lo * CTAS + rank; }
   __device__ __forceinline__ TileCoord coord(const GemmParams& p, int rank, int per_split) const {
@@ -167,6 +188,25 @@ struct TileWalk {
       t.kb_end = min(p.k_blocks, t.kb_begin + per_split);
     }
     return t;
+  }
+};
+
+// Image position of a k-block of 64 pixels (OP_PIXELS_5D). Stepped: its four divisions per k-block kept the producers at 800 to 1030 cycles
+// a k-block, above the 384 to 768 that the tensor core needs.
+struct PixelWalk {
+  int w, h, b;
+  __device__ __forceinline__ void start(const GemmParams& p, int kb) {
+    w = kb % p.pix_n0;
+    kb /= p.pix_n0;
+    h = kb % p.pix_n1;
+    b = kb / p.pix_n1;
+  }
+  __device__ __forceinline__ void next(const GemmParams& p) {
+    if (++w < p.pix_n0) return;
+    w = 0;
+    if (++h < p.pix_n1) return;
+    h = 0;
+    ++b;
   }
 };
 
@@ -297,17 +337,27 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 #pragma unroll
           for (int d = 0; d < 5; ++d) abase[d] = t0 * p.a_mul0[d] + t1 * p.a_mul1[d] + t2 * p.a_mul2[d];
         }
+        // rows over all taps: channel and displacement of this tile's boxes of 64 rows (channel < 0: ones)
+        constexpr int BOXES = PEERS ? 1 : STACK * GEMM_BM / 64;
+        short box_c[BOXES], box_p[BOXES], box_w[BOXES], box_h[BOXES];
+        if (!PEERS && p.tap_boxes > 0) {
+#pragma unroll
+          for (int j = 0; j < BOXES; ++j) {
+            const int box = tc.m_blk * (GEMM_BM / 64) + j, tap = box / p.tap_boxes;
+            const short* g = p.grp_off[min(tap, p.taps - 1)];
+            box_c[j] = tap < p.taps ? static_cast<short>((box - tap * p.tap_boxes) * 64) : -1;
+            box_p[j] = g[0];
+            box_w[j] = g[1];
+            box_h[j] = g[2];
+          }
+        }
+        PixelWalk pix = {};
+        if (p.a_mode == OP_PIXELS_5D) pix.start(p, tc.kb_begin);
         for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
           if (!wait_counted<PAIR>(&empty[s], ph ^ 1u, abort_flag, p.status, 0x100u + s, mbar_budget, t_wait)) break;
           uint8_t* sA = smem + s * Cfg::STAGE_BYTES;
           if (rank == 0) mbar_expect_tx(&full[s], STACK > 1 ? blocks * Cfg::BLOCK_BYTES : CTAS * Cfg::BLOCK_BYTES);
           const uint32_t bar = PAIR ? map_to_cta(&full[s], 0) : smem_u32(&full[s]);
-          int pw = 0, ph_ = 0, pb = 0;
-          if (p.a_mode == OP_PIXELS_5D) {
-            pw = kb % p.pix_n0;
-            ph_ = (kb / p.pix_n0) % p.pix_n1;
-            pb = kb / (p.pix_n0 * p.pix_n1);
-          }
           // ---- operand A
           if (p.a_mode == OP_KMAJOR_2D) {
             if (PEERS && p.a_peers > 1) {
@@ -354,13 +404,26 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               h -= p.img_h;
             }
             tma_load_5d<PAIR>(sA, m, bar, abase[0] + e[0], abase[1] + e[1], abase[2] + e[2], h, abase[4]);
+          } else if (!PEERS && p.tap_boxes > 0) {   // OP_PIXELS_5D, a tap per box
+#pragma unroll
+            for (int j = 0; j < BOXES; ++j) {
+              if (STACK > 1 && j >= blocks * (GEMM_BM / 64)) break;
+              if (box_c[j] >= 0)
+                tma_load_5d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, box_c[j], box_p[j], pix.w * GEMM_BK + box_w[j],
+                                  pix.h * p.pix_hmul + box_h[j], pix.b);
+              else
+                tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_in, bar, 0, 0);
+            }
+            pix.next(p);
           } else {  // OP_PIXELS_5D: {channels, parity, w, h, b}
             const short* g = p.grp_off[tc.grp];
-            const int par = p.disp_a ? g[0] : 0, w = pw * GEMM_BK + (p.disp_a ? g[1] : 0), h = p.disp_a ? ph_ * p.pix_hmul + g[2] : ph_;
+            const int par = p.disp_a ? g[0] : 0, w = pix.w * GEMM_BK + (p.disp_a ? g[1] : 0);
+            const int h = p.disp_a ? pix.h * p.pix_hmul + g[2] : pix.h;
 #pragma unroll
             for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
               if (STACK == 1 || j < blocks * (GEMM_BM / 64))
-                tma_load_5d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, par, w, h, pb);
+                tma_load_5d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, par, w, h, pix.b);
+            pix.next(p);
           }
         }
       }
@@ -378,17 +441,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         // this CTA's rows of B, in boxes of 64 where they are not one (wide tiles: its halves of 256 and of 128)
         const int n0 = tc.n_blk * BN + rank * (WIDE ? 128 : Cfg::B_ROWS);
         auto box_at = [&](int j) { return WIDE && j == 2 ? tc.n_blk * BN + 256 + rank * 64 : n0 + j * 64; };
+        PixelWalk pix = {};
+        if (p.b_mode == OP_PIXELS_5D) pix.start(p, tc.kb_begin);
         for (int kb = tc.kb_begin; kb < tc.kb_end; ++kb, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
           if (!wait_counted<PAIR>(&empty[s], ph ^ 1u, abort_flag, p.status, 0x140u + s, mbar_budget, t_wait)) break;
           uint8_t* sB = smem + s * Cfg::STAGE_BYTES + Cfg::A_BYTES;
           if (rank == 0) mbar_expect_tx(&full[s], CTAS * Cfg::B_BYTES);
           const uint32_t bar = PAIR ? map_to_cta(&full[s], 0) : smem_u32(&full[s]);
-          int pw = 0, ph_ = 0, pb = 0;
-          if (p.b_mode == OP_PIXELS_5D) {
-            pw = kb % p.pix_n0;
-            ph_ = (kb / p.pix_n0) % p.pix_n1;
-            pb = kb / (p.pix_n0 * p.pix_n1);
-          }
           if (p.b_mode == OP_KMAJOR_2D) {
             if (WIDE) {
 #pragma unroll
@@ -402,8 +461,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               tma_load_2d<PAIR>(sB + j * (GEMM_BK * 128), &p.map_b, bar, box_at(j), kb * GEMM_BK);
           } else {  // OP_PIXELS_5D with per-group (tap) displacement
             const short* g = p.grp_off[tc.grp];
-            const int par = p.disp_a ? 0 : g[0], w = pw * GEMM_BK + (p.disp_a ? 0 : g[1]);
-            int h = p.disp_a ? ph_ : ph_ * p.pix_hmul + g[2];
+            const int par = p.disp_a ? 0 : g[0], w = pix.w * GEMM_BK + (p.disp_a ? 0 : g[1]);
+            int h = p.disp_a ? pix.h : pix.h * p.pix_hmul + g[2];
             const CUtensorMap* m = &p.map_b;
             if (h < 0 && (p.halo_flags & 1)) {
               m = &p.map_halo_lo;
@@ -414,7 +473,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             }
 #pragma unroll
             for (int j = 0; j < Cfg::B_ROWS / 64; ++j)
-              tma_load_5d<PAIR>(sB + j * (GEMM_BK * 128), m, bar, box_at(j), par, w, h, pb);
+              tma_load_5d<PAIR>(sB + j * (GEMM_BK * 128), m, bar, box_at(j), par, w, h, pix.b);
+            pix.next(p);
           }
         }
       }
@@ -769,6 +829,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             const int peer = (slot + p.a_first) % p.a_peers;
             const int lr = (p.a_interleave ? tc.m_blk / p.a_peers : tc.m_blk % p.a_tiles) * GEMM_BM + r;
             return (lr < p.a_rows) ? static_cast<long long>(peer) * p.a_rows + lr : -1;
+          } else if (!PEERS && p.tap_boxes > 0) {
+            const int g = tc.m_blk * GEMM_BM + r, tap = (g >> 6) / p.tap_boxes, c = g - tap * p.tap_boxes * 64;
+            if (tap >= p.taps) return tap == p.taps && c == 0 ? -2 : -1;      // -2: the column sums of B
+            return c < p.tap_channels ? static_cast<long long>(tap) * p.tap_channels + c : -1;
           } else {
             const long long g = static_cast<long long>(tc.m_blk) * GEMM_BM + r;
             return (g < p.M) ? g : -1;
@@ -952,6 +1016,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               for (int i = 0; i < 4; ++i) {
                 const float4 t = *reinterpret_cast<const float4*>(xaddr(grow + 8 * i, gvec));
                 const int col = cb + 16 * hf + gvec * 4;
+                if (!PEERS && grows[i] == -2 && p.row_sums != nullptr) {
+                  const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+                  for (int e = 0; e < 4; ++e)
+                    if (col + e < ncols_out) atomicAdd(p.row_sums + col + e, tv[e]);
+                  continue;
+                }
                 if (grows[i] < 0 || col >= ncols_out) continue;
                 float* o = obase + static_cast<long long>(grows[i]) * p.ldc + col;
                 if (PEERS && p.c_peers > 1)   // the row's owner accumulates it
@@ -990,7 +1061,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           uint32_t v[32];   // column 0 of the sums accumulator: lane l holds the sum of A's column (row of D) q * 32 + l
           tmem_ld_32x32(tmem_base + Cfg::SUM_COL0 + dcol * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
           tmem_ld_wait();
-          const int g = tc.m_blk * GEMM_BM + q * 32 + lane;
+          int g = tc.m_blk * GEMM_BM + q * 32 + lane;
+          if (p.tap_boxes > 0) {      // (the taps' sums add up)
+            const int tap = (g >> 6) / p.tap_boxes;
+            g = tap < p.taps ? g - tap * p.tap_boxes * 64 : p.M;
+          }
           if (g < p.M) atomicAdd(p.colsum + g, __uint_as_float(v[0]) * p.alpha);
         }
       }
@@ -1071,6 +1146,8 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   cfg.numAttrs = attrs;
   return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, p);
 }
+
+cudaError_t gemm_ones_tile(void** ptr) { return cudaGetSymbolAddress(ptr, g_ones_tile); }
 
 cudaError_t gemm_read_stalls(unsigned long long* out8, bool reset) {
   cudaError_t e = cudaMemcpyFromSymbol(out8, g_gemm_stalls, 8 * sizeof(unsigned long long));

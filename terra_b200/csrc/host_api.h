@@ -93,6 +93,17 @@ int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, 
 int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
                        int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo = nullptr,
                        const void* halo_hi = nullptr, float* bias_grad = nullptr, int stack = 1);   // bias_grad[Cout] += sums of dy
+// Weight gradients of all taps as one product (one rank): tile width, CTAs per tile, row blocks per tile, split of the contraction.
+struct TapPlan {
+  int bn, ctas, stack, split;
+};
+// `taps` times `channels` rows, N columns, `k_blocks` blocks of 64 pixels of an image row; the bias gradient as the sums of the columns'
+// operand (`row_sums`) or of the rows' (`column_sums`); at least `least_split` parts of the contraction.
+TapPlan plan_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool row_sums, bool column_sums, int least_split, int num_sms);
+int conv3x3_wgrad_taps_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride, const TapPlan& plan,
+                            void* status, int num_sms, cudaStream_t stream, float* bias_grad);      // dw [9, Cin, Cout]
+int convt2x2_wgrad_taps_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, const TapPlan& plan,
+                             void* status, int num_sms, cudaStream_t stream, float* bias_grad);     // dw [4, Cout, Cin]
 
 // elementwise.cu -------------------------------------------------------------------------------
 // LayerNorm over the last dimension (C <= 8192, C % 8 == 0), bf16 in/out, fp32 statistics.
@@ -125,6 +136,8 @@ int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, 
 int groupnorm_finalize(float* sums, float* stats, int cells, float inv_count, float eps, cudaStream_t stream);
 // dst[a*sa + b*sb + c*sc] += src[a][b][c] (fp32, src contiguous [na][nb][nc]); src is zeroed behind the read.
 int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa, long long sb, long long sc, cudaStream_t stream);
+// dst[c][r][t] += src[t][r][c] (fp32, both contiguous, taps <= 9); src is zeroed behind the read.
+int fold_taps_f32(float* src, float* dst, int taps, int rows, int cols, cudaStream_t stream);
 // Masked loss: loss_sum += sum(f(pred * mask - label)), f = |.| (kind 0) or square (kind 1);
 // grad = mask * f'(.) * scale (bf16). `mask` may be null. Partial sums are fp32 atomics on loss_sum[0].
 int masked_loss_fwd_bwd(const void* pred, const void* label, const void* mask, long long n, long long mask_period,

@@ -16,6 +16,14 @@ void conv3x3_s2_dgrad(const Tensor& dy, const Tensor& w, Tensor& dx, const OptTe
 void convt2x2(int64_t op, const Tensor& in, const Tensor& w, const OptTensor& bias4, Tensor& out, const OptTensor& status);
 void convt2x2_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t split_k, const OptTensor& status, int64_t stack,
                     const OptTensor& bias_grad);
+// The weight gradients of one rank, all taps in one product: dw [9, Cin, Cout] or [4, Cout, Cin], accumulated, for fold_taps; bias_grad [Cout]
+// accumulated, by launches of its own unless `fuse_bias`. The contraction is cut into `least_split` parts at least. `plan` ({columns, CTAs, row blocks, split}): instead of the rule's
+using TapPlanRequest = c10::optional<std::vector<int64_t>>;
+void conv3x3_wgrad_taps(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t stride, const OptTensor& status, const OptTensor& bias_grad,
+                        bool fuse_bias, int64_t least_split, const TapPlanRequest& plan = c10::nullopt);
+void convt2x2_wgrad_taps(const Tensor& x, const Tensor& dy, Tensor& dw, const OptTensor& status, const OptTensor& bias_grad, bool fuse_bias,
+                         int64_t least_split, const TapPlanRequest& plan = c10::nullopt);
+void fold_taps(Tensor& src, Tensor& dst);
 
 // fp32 scratch that a call takes zeroed, for itself, and gives back zeroed once everything it launches with it is queued (zero_scratch.cpp)
 Tensor scratch_take(const Tensor& like, at::IntArrayRef sizes);

@@ -234,9 +234,8 @@ def _conv3x3_node(x, weight, bias, stride, dom):
     if x.requires_grad and torch.is_grad_enabled():
         wd = _packed(weight, w16, "dgrad", pack_conv3x3_weight_dgrad) if stride == 1 else \
             _packed(weight, w16, "s2dgrad_taps", pack_conv3x3_weight_s2_dgrad)
-    split, stack = _wgrad_split(B, H, W, stride, Cout, Cin)
     return ext.nodes.conv3x3(x, weight, bias, _packed(weight, w16, "fwd", pack_conv3x3_weight), wd, bias.bf16,
-                             stride, split, stack, FUSE_BIAS_GRAD, status_word(x.device))
+                             stride, _wgrad_split(B, H, W, stride, Cout, Cin)[0], FUSE_BIAS_GRAD, status_word(x.device))
 
 
 @nvtx_range("terra.conv3x3")
@@ -359,10 +358,9 @@ def _conv_transpose2x2_node(x, weight, bias):
     if not _convt_tiled(B, H, W, Cin, Cout):
         return None
     wd = _packed(weight, w16, "convT_dgrad", _pack_convt_dgrad) if x.requires_grad and torch.is_grad_enabled() else None
-    split, stack = _wgrad_plan(4, Cout, Cin, B * H * ((W + 63) // 64))
     return _ext.load().nodes.conv_transpose2x2(
         x, weight, bias, _packed(weight, w16, "convT", _pack_convt), wd, _packed(bias, bias.bf16, "convT_bias", _pack_convt_bias),
-        split, stack, FUSE_BIAS_GRAD, status_word(x.device))
+        _wgrad_plan(4, Cout, Cin, B * H * ((W + 63) // 64))[0], FUSE_BIAS_GRAD, status_word(x.device))
 
 
 def _convt_flat_weight(weight, w16):

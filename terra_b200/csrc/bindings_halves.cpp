@@ -11,6 +11,7 @@
 #include "check.h"
 #include "host_api.h"
 #include "launch_count.h"
+#include "size_memo.h"
 #include "torch_ops.h"
 
 namespace {
@@ -97,58 +98,74 @@ void column_sums(const Tensor& dy, const Tensor& out) {
            "colsum");
 }
 
-// Tile width, row blocks per tile and split of the contraction for N x K outputs over M rows. A k-block costs a CTA its
-// operand fill plus the tensor core's reads through the shared-memory port, in KB; the column sums add 40 KB per row block,
-// shared out over the column tiles. Every split pays its start and its pass of atomics (1100 KB a row block, and 1.3 KB per
-// output block of the whole launch). Widths of 256 leave no room for the sums' accumulators: the column sums are then two
-// launches of their own, which read dy once more (10 us and 5.6 TB/s against 3.7 us per 1000 KB).
-// A pair of CTAs (request 1000 + width: 256 x 256 or 256 x 384 outputs) halves B's share and is bound by the tensor core instead: 512 or
-// 768 cycles per k-block, 74 and 140 KB of that measure as timed. Only the 384-wide tile has room for the sums (16 KB, shared out alike).
-// The constants of single CTAs were fitted to 11000 times: 64 to 557056 rows, 45 pairs of N and K between 96 and 4096, all widths, stacked
-// or not, one to four rounds (passes back to back in a CUDA graph); the choice among them is 2 % slower than the best plan on average. Those of
-// pairs are not part of that fit: the figures at the end are what they were set by. Without the 10 us the separate sums were taken for few rows
-// too (us, that / this rule): 512 rows of 384 x 1536 22 / 9, 2048 of 256 x 1024 19 / 9, 17280 of
-// 192 x 2208 39 / 23, 156672 of 3072 x 1024 839 / 799. Pairs (us, best single / pair): 557056 rows of 2976 x 384 with sums 1184 / 1032,
-// without 1047 / 935, 139264 of 1536 x 384 231 / 202, 156672 of 3072 x 1024 without sums 704 / 647.
+// Tile width, row blocks per tile and split of the contraction for N x K outputs over M rows: the plan of least time by a model, in us. Rounds of
+// tiles over the CTAs (or pairs: request 1000 + width), each its k-blocks and a hand-over with the epilogue. A k-block costs less where fewer
+// CTAs than there are SMs share L2's bandwidth; the column sums (the bias gradient) are more MMAs, shared out over the column tiles. Widths of
+// 256 and transposed plans have no room for the sums' accumulators, or the wrong operand: there the sums are two launches that read dy once more.
+// Transposed: few outputs of a wide layer (patch embedding: 384 x 2976), 384 rows filling one and a half pairs, 384 columns one tile.
+//
+// Fitted to 9000 passes in CUDA graphs: 200 to 557056 rows, 22 pairs of N and K between 96 and 4096, with and without sums, all tiles, half a
+// round to three; the choice is 0.9 % slower than the best plan on average, 9 % at most. The plans of the fit before, which was made with
+// epilogues through the lanes, were 3.7 % slower than the best on average. Us, those plans / this: 17280 rows of 1024 x 1024 44 / 32, 40000 of 3072 x 1024
+// with sums 220 / 186, 139264 of 1536 x 384 134 / 120, of 768 x 768 with sums 169 / 125, 156672 of 3072 x 1024 with sums 820 / 730.
+//
+// Among plans within 3 % the one with most parts is taken, and a part is longer than 32 k-blocks only where 128 x 256 tiles in one round would have it
+// so: the error of the tensor core's fp32 sums grows with their length (128 k-blocks 8.6e-6 of the norm, 192 13e-6).
 struct WgradPlan {
   int bn, stack, split;
   bool swapped;      // the transpose: rows are x's columns
 };
-WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
-  const int64_t m_blocks = (N + 127) / 128, k_blocks = (M + 63) / 64, sms = sm_count();
-  WgradPlan best{128, 1, 1, false};
-  double least = -1.0;
-  // `width` columns, `blocks` 128-row blocks a tile, `kb` KB a k-block, on `units` CTAs or pairs; `pair`: two CTAs share the blocks
-  auto consider = [&](int request, int width, int stack, bool pair, double kb, double extra, bool swapped = false) {
-    const int64_t blocks = pair ? 2 : stack, units = pair ? sms / 2 : sms;
-    const int64_t rows = swapped ? (K + 127) / 128 : m_blocks;
-    const int64_t n = ((swapped ? N : K) + width - 1) / width, tiles = (rows + blocks - 1) / blocks * n;
-    if (sums && extra == 0.0 && !swapped) kb += (pair ? 16.0 : 40.0 * stack) / n;
-    // whole rounds of CTAs: the largest split of one round, two rounds, ...
-    for (int64_t rounds = 1; rounds <= 3; ++rounds) {
-      const int64_t split = std::max<int64_t>(1, std::min(rounds * units / tiles, k_blocks));
-      const int64_t per = (k_blocks + split - 1) / split;
-      const double cost = static_cast<double>((tiles * split + units - 1) / units) * (per * kb + 1100.0 * (pair ? width / 128.0 : stack)) +
-                          1.3 * tiles * split * blocks * width / 192 + (pair ? 600.0 : 0.0) + extra;   // (a pair starts 2 us later)
-      if (least < 0.0 || cost < least * 0.995) {
-        least = cost;
-        best = {request, stack, static_cast<int>(split), swapped};
+WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
+  struct Tile {
+    int request, stack;
+    double kblock, tile;
+  };
+  static const Tile tiles[] = {{128, 1, 0.224, 1.91}, {192, 1, 0.307, 2.43}, {256, 1, 0.468, 2.42}, {128, 2, 0.523, 3.59}, {192, 2, 0.608, 4.73},
+                               {256, 2, 0.682, 13.4}, {1256, 1, 0.342, 3.52}, {1384, 1, 0.512, 4.93}};
+  const int64_t k_blocks = (M + 63) / 64, sms = sm_count();
+  const int64_t blocks_256 = ((N + 127) / 128) * ((K + 255) / 256);
+  const int64_t least_split = std::max<int64_t>(1, std::min((k_blocks + 31) / 32, sms / blocks_256));
+  const double separate = sums ? 8.5 + 2e-6 * M * N / 4.71 : 0.0;
+  const bool pairs = tb::gemm_pairs() && sms >= 2;
+  struct Choice {
+    WgradPlan plan;
+    double time;
+  };
+  std::vector<Choice> choices;
+  for (const Tile& t : tiles) {
+    const bool pair = t.request >= 1000;
+    const int width = t.request % 1000;
+    for (bool swapped : {false, true}) {
+      if (swapped && !(t.request == 1384 && N > 256 && K > 2 * N)) continue;
+      const int64_t rows = swapped ? K : N, cols = swapped ? N : K;
+      if ((pair && (!pairs || rows <= 128 || width >= 2 * cols || (width == 384 && cols <= 256))) || (t.stack == 2 && rows <= 128) ||
+          (width > 128 && !pair && cols <= width - 64))
+        continue;
+      const int64_t high = pair ? 2 : t.stack, units = pair ? sms / 2 : sms, n = (cols + width - 1) / width;
+      const int64_t count = ((rows + 127) / 128 + high - 1) / high * n;
+      const bool fused = sums && width != 256 && !swapped;
+      const double sum_cost = fused ? (pair ? 0.128 : 0.158 * t.stack) / n : 0.0;
+      for (int halves : {1, 2, 4, 6}) {
+        const int64_t want = std::min(std::max(least_split, halves * units / 2 / count), k_blocks), per = (k_blocks + want - 1) / want;
+        const int64_t split = (k_blocks + per - 1) / per, rounds = (count * split + units - 1) / units;
+        const double full = std::min(1.0, static_cast<double>(count * split) / units);
+        const double time = rounds * (per * (t.kblock * (0.77 + 0.23 * full) + sum_cost) + t.tile) + (pair ? 1.3 : 0.0) +
+                            0.008 * 4e-6 * count * split * high * 128 * std::min<int64_t>(width, cols) + 3.4 + (fused ? 0.0 : separate);
+        choices.push_back({{t.request, t.stack, static_cast<int>(split), swapped}, time});
       }
     }
-  };
-  const double separate = sums ? (10.0 + 2.0 * M * N / 5.6e6) / 0.0037 : 0.0;
-  for (int stack : {1, 2}) {
-    if (stack > m_blocks) continue;
-    for (int bn : {192, 128, 256})
-      consider(bn, bn, stack, false, 16.0 * stack + bn / 8 + stack * (16.0 + bn / 8), bn == 256 ? separate : 0.0);
   }
-  if (tb::gemm_pairs() && sms >= 2 && m_blocks >= 2) {
-    if (K > 256) consider(1384, 384, 1, true, 140.0, 0.0);
-    if (K > 128) consider(1256, 256, 1, true, 74.0, separate);
-  }
-  // few outputs of a wide layer (patch embedding: 384 x 2976): 384 rows fill one and a half pairs, 384 columns one tile
-  if (tb::gemm_pairs() && sms >= 2 && N > 256 && K > 2 * N) consider(1384, 384, 1, true, 140.0, separate, true);
-  return best;
+  double least = choices.front().time;
+  for (const Choice& c : choices) least = std::min(least, c.time);
+  const Choice* best = nullptr;
+  for (const Choice& c : choices)
+    if (c.time <= 1.03 * least && (best == nullptr || c.plan.split > best->plan.split || (c.plan.split == best->plan.split && c.time < best->time)))
+      best = &c;
+  return best->plan;
+}
+WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
+  static thread_local tb::SizeMemo<WgradPlan, 4> known;
+  return known.get({N, K, M, sums}, [&] { return model_wgrad(N, K, M, sums); });
 }
 
 }  // namespace

@@ -2,6 +2,7 @@
 // No allocation happens here: callers pass every buffer.
 #include "gemm_sm100.cuh"
 #include "host_api.h"
+#include "size_memo.h"
 
 #include <algorithm>
 #include <cstdio>
@@ -33,10 +34,10 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// rank <= 5, bf16 elements, 128-byte swizzle, zero fill outside the tensor.
+// rank <= 5, 128-byte swizzle, zero fill outside the tensor.
 // dims/box are innermost first; strides (bytes) are for dims 1..rank-1.
-int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
-                         const unsigned long long* strides_bytes, const unsigned int* box) {
+static int make_tensor_map(CUtensorMap* out, CUtensorMapDataType type, const void* base, int rank, const unsigned long long* dims,
+                           const unsigned long long* strides_bytes, const unsigned int* box) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return -1;
   // cuTensorMapEncodeTiled is a driver call: it needs the primary context bound to THIS thread. A thread that
@@ -60,10 +61,15 @@ int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const uns
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return -2;
   for (int i = 0; i + 1 < rank; ++i)
     if (gstr[i] % 16 != 0) return -3;
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(base),
+  CUresult r = fn(out, type, static_cast<cuuint32_t>(rank), const_cast<void*>(base),
                   gdim, gstr, bdim, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -100 - static_cast<int>(r);
+}
+
+int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
+                         const unsigned long long* strides_bytes, const unsigned int* box) {
+  return make_tensor_map(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, rank, dims, strides_bytes, box);
 }
 
 static int map_2d(CUtensorMap* out, const void* base, long long inner, long long outer, long long ld_elems,
@@ -106,6 +112,18 @@ static void try_tma_epilogue(GemmParams& p, long long M, long long N) {
   p.epi_tma = 1;
 }
 
+// Accumulated fp32 outputs leave as TMA reductions of 32 x 32 units where they qualify: `groups` (taps) of `rows` x N, or the transpose of one.
+static void try_tma_reduce(GemmParams& p, long long rows, long long N, long long groups, long long group_stride) {
+  if (!gemm_tma_epilogue() || (p.epi & ~EPI_TRANSPOSE) != (EPI_OUT_F32 | EPI_ATOMIC) || p.a_peers > 1 || p.c_peers > 1 || p.C == nullptr) return;
+  const bool turned = (p.epi & EPI_TRANSPOSE) != 0;
+  unsigned long long dims[3] = {static_cast<unsigned long long>(turned ? rows : N), static_cast<unsigned long long>(turned ? N : rows),
+                                static_cast<unsigned long long>(groups)};
+  if (p.ldc < 0 || static_cast<unsigned long long>(p.ldc) < dims[0]) return;
+  unsigned long long str[2] = {static_cast<unsigned long long>(p.ldc) * 4ull, static_cast<unsigned long long>(groups > 1 ? group_stride : p.ldc) * 4ull};
+  unsigned int box[3] = {32u, 32u, 1u};
+  if (make_tensor_map(&p.map_c, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.C, 3, dims, str, box) == 0) p.epi_tma = 3;
+}
+
 static int pick_bn(long long N, int requested) {
   if (requested == 64 || requested == 128 || requested == 192 || requested == 256) return requested;
   if (N <= 64) return 64;
@@ -143,8 +161,8 @@ struct TileCosts {
   double start[2], tile, tail, plain_unit, bias_unit, drain;   // start: single CTAs, pairs
   double kblock[2][4];                                         // main loop per 64-wide k-block, widths 128, 192, 256, 384
 };
-static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, bool gathered, int num_sms, int* bn_out,
-                      int* ctas_out) {
+static void model_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, bool gathered, int num_sms, int* bn_out,
+                       int* ctas_out) {
   *bn_out = pick_bn(N, 0);
   *ctas_out = 1;
   if (N <= 64 || m_blocks < 1) return;
@@ -179,6 +197,21 @@ static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, 
       }
     }
   }
+}
+
+static void pick_tile(long long m_blocks, long long N, int k_blocks, bool b_mn, int flags, bool gathered, int num_sms, int* bn_out,
+                      int* ctas_out) {
+  struct Choice {
+    int bn, ctas;
+  };
+  static thread_local SizeMemo<Choice, 7> known;
+  const Choice& c = known.get({m_blocks, N, k_blocks, b_mn, flags, gathered, num_sms}, [&] {
+    Choice made;
+    model_tile(m_blocks, N, k_blocks, b_mn, flags, gathered, num_sms, &made.bn, &made.ctas);
+    return made;
+  });
+  *bn_out = c.bn;
+  *ctas_out = c.ctas;
 }
 
 void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, bool gathered, int num_sms, int* bn, int* ctas) {
@@ -296,6 +329,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   p.tile_n0 = 1;
   p.tile_n1 = 1;
   try_tma_epilogue(p, M, N);
+  try_tma_reduce(p, M, N, 1, 0);
   cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
@@ -551,6 +585,7 @@ static int gather_wgrad(const void* a, const void* b, float* dw, int B, int Ho, 
   p.status = static_cast<KernelStatus*>(status);
   p.tile_n0 = 1;
   p.tile_n1 = 1;
+  try_tma_reduce(p, M, N, ntaps, p.grp_c_stride);
   const cudaError_t e = launch_gemm(p, bn, 1, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
@@ -586,20 +621,20 @@ int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, 
 // a convolution, are one more row, that of a box of ones.
 //
 // The plan is the one with the least time by a model, in us: rounds of tiles over the CTAs (pairs), each its k-blocks and a hand-over with the
-// epilogue, and the atomics of all splits. Fitted to 900 passes in CUDA graphs: the two layers at 512 to 557056 pixels, 96 to 384 channels, all
-// tiles, half a round to three and more; the choice is 0.5 % slower than the best plan on average, at most 8 %.
+// epilogue. Fitted to 900 passes in CUDA graphs: the two layers at 512 to 557056 pixels, 96 to 384 channels, all tiles, half a round to three
+// and more; the choice is 0.1 % slower than the best plan on average, at most 3 %.
 // Us, a product per tap (two row blocks stacked where that was ahead) / this: 557056 pixels of 384 channels 1251 / 951, of 192 383 / 275, 80000 of
 // 256 104 / 85, 17280 of 192 25 / 21; transposed, 139264 of 384 186 / 161, of 192 69 / 57, of 96 45 / 35. (Of 96 and 128 channels the row of ones
 // costs a tile in ten: 17280 pixels 12.6 / 13.5 and 16.4 / 17.2; folding the gradients takes 2 to 10 us less than it did.)
 // `least_split`: the contraction is cut into so many parts at least (the error of the tensor core's fp32 sums grows with their length: 139264
 // pixels of 384 channels, 18 parts 8.6e-6, 12 parts 13.0e-6), unless they are down to 24 k-blocks (1.6e-6).
-TapPlan plan_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool row_sums, bool column_sums, int least_split, int num_sms) {
+static TapPlan model_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool row_sums, bool column_sums, int least_split, int num_sms) {
   struct Tile {
     int width, ctas, stack;
     double kblock, tile;
   };
-  static const Tile tiles[] = {{128, 1, 1, 0.265, 2.99}, {192, 1, 1, 0.299, 2.93}, {128, 1, 2, 0.433, 6.09}, {192, 1, 2, 0.566, 5.38},
-                               {256, 2, 1, 0.345, 2.26}, {384, 2, 1, 0.515, 6.82}};
+  static const Tile tiles[] = {{128, 1, 1, 0.269, 1.56}, {192, 1, 1, 0.321, 1.92}, {128, 1, 2, 0.495, 3.34}, {192, 1, 2, 0.502, 4.65},
+                               {256, 2, 1, 0.334, 2.84}, {384, 2, 1, 0.461, 5.38}};
   least_split = static_cast<int>(std::min<long long>(least_split, (k_blocks + 23) / 24));
   const long long boxes = static_cast<long long>(taps) * ((channels + 63) / 64) + (row_sums ? 1 : 0);
   TapPlan best = {128, 1, 1, 1};
@@ -614,9 +649,9 @@ TapPlan plan_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool r
       const long long want = std::max<long long>({1, least_split, halves * units / 2 / count});
       const long long per = (k_blocks + std::min(want, k_blocks) - 1) / std::min(want, k_blocks);
       const long long split = (k_blocks + per - 1) / per;
-      const double outputs = static_cast<double>(count) * split * t.stack * t.ctas * 128 * std::min(t.width, N) * 4e-6;      // MB
-      const double kblock = t.kblock + (column_sums ? 0.155 * t.stack / n : 0.0);
-      const double time = static_cast<double>((count * split + units - 1) / units) * (per * kblock + t.tile) + 0.119 * outputs + (t.ctas == 2 ? 4.6 : 0.0);
+      const double full = std::min(1.0, static_cast<double>(count * split) / units);      // (fewer CTAs share L2's bandwidth)
+      const double kblock = (t.kblock * (0.57 + 0.43 * full)) + (column_sums ? 0.151 * t.stack / n : 0.0);
+      const double time = static_cast<double>((count * split + units - 1) / units) * (per * kblock + t.tile) + (t.ctas == 2 ? 1.0 : 0.0);
       if (least < 0.0 || time < least) {
         least = time;
         best = {t.width, t.ctas, t.stack, static_cast<int>(split)};
@@ -624,6 +659,12 @@ TapPlan plan_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool r
     }
   }
   return best;
+}
+
+TapPlan plan_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool row_sums, bool column_sums, int least_split, int num_sms) {
+  static thread_local SizeMemo<TapPlan, 8> known;
+  return known.get({taps, channels, N, k_blocks, row_sums, column_sums, least_split, num_sms},
+                   [&] { return model_tap_wgrad(taps, channels, N, k_blocks, row_sums, column_sums, least_split, num_sms); });
 }
 
 // dw[tap][channels][N] (fp32, accumulated) = sum over the pixels of b [B, Ho, Wo, N] of a [B, H, W, channels] at the pixel's tap, times b.
@@ -679,6 +720,7 @@ static int tap_wgrad(const void* a, const void* b, float* dw, int B, int Ho, int
   p.status = static_cast<KernelStatus*>(status);
   p.tile_n0 = 1;
   p.tile_n1 = 1;
+  try_tma_reduce(p, channels, N, ntaps, static_cast<long long>(channels) * N);
   const cudaError_t e = launch_gemm(p, plan.bn, plan.ctas, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

@@ -9,7 +9,8 @@
 //            and commits to `empty[s]` (stage reusable) and `tfull[a]` (accumulator a complete);
 //   warps 2-13 epilogue (three per 32-lane TMEM quadrant, interleaved over the columns): tcgen05.ld, fused bias / GELU /
 //            residual / GELU-gradient; bf16 outputs leave as units of 32 rows (or pixels) x 64 columns through TMA stores,
-//            fp32 split-K atomics and what does not fit a tensor map as 32-column chunks through an exchange buffer.
+//            accumulated fp32 outputs as TMA reductions of 32 x 32 units, what does not fit a tensor map as 32-column chunks through an
+//            exchange buffer.
 // Two accumulators (2*BN TMEM columns) let the epilogue of tile i overlap the main loop of tile i+1 (tiles 384 wide have one).
 //
 // Operand addressing is data driven (see gemm_sm100.cuh) so that the same kernel serves
@@ -586,7 +587,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       return reinterpret_cast<uint4*>(my_x + rr * 64 + (((vec ^ (rr >> 1)) & 3) << 4));
     };
     constexpr int CPW = (CHUNKS + GEMM_EPI_WARPS / 4 - 1) / (GEMM_EPI_WARPS / 4);   // chunks per warp
-    if (!PEERS && STACK == 1 && p.epi_tma) {
+    // the bias gradient that rides on a weight gradient: column 0 of the sums accumulator, lane l holding the sum of A's column (row of D) q * 32 + l
+    auto add_column_sums = [&](const TileCoord& tc, int dcol) {
+      if (!Cfg::CAN_COLSUM || p.colsum == nullptr || part != 0 ||
+          first_sum_kb(p, tc, p.disp_a ? p.num_n_tiles : p.groups * p.num_n_tiles) >= tc.kb_end)
+        return;
+      uint32_t v[32];
+      tmem_ld_32x32(tmem_base + Cfg::SUM_COL0 + dcol * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
+      tmem_ld_wait();
+      int g = tc.m_blk * GEMM_BM + q * 32 + lane;
+      if (p.tap_boxes > 0) {      // (the taps' sums add up)
+        const int tap = (g >> 6) / p.tap_boxes;
+        g = tap < p.taps ? g - tap * p.tap_boxes * 64 : p.M;
+      }
+      if (g < p.M) atomicAdd(p.colsum + g, __uint_as_float(v[0]) * p.alpha);
+    };
+    if (!PEERS && STACK == 1 && p.epi_tma && p.epi_tma != 3) {
       // ---- bf16 outputs through TMA, and the operand the epilogue reads. A warp works on units of 32 rows x 64 columns (128
       // bytes per row in the 128-byte-swizzled layout, conflict-free for the row-per-lane 16-byte accesses). Tiles of 192
       // columns are one unit per warp and tile.
@@ -628,7 +644,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         return false;
       };
 
-      auto run = [&](auto form_const) {
+      auto run = [&](auto form_const) __attribute__((always_inline)) {
         constexpr int FORM = decltype(form_const)::value;      // EPI_* flags of the form, or -1: tested at run time
         const int flags = FORM >= 0 ? FORM : p.epi;
         const bool with_bias = (flags & EPI_BIAS) != 0, gelu = (flags & EPI_GELU) != 0, save_pre = (flags & EPI_SAVE_PRE) != 0;
@@ -803,6 +819,84 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       else if (form == (EPI_BIAS | EPI_RESIDUAL)) run(std::integral_constant<int, EPI_BIAS | EPI_RESIDUAL>{});
       else if (form == EPI_MUL_DGELU) run(std::integral_constant<int, EPI_MUL_DGELU>{});
       else run(std::integral_constant<int, -1>{});
+    } else if (!PEERS && p.epi_tma == 3) {
+      // ---- accumulated fp32 outputs as TMA reductions of 32 x 32 units, 128 bytes a row in the 128-byte-swizzled layout. (By the lanes, as
+      // vector reductions behind the exchange buffer, an SM got 16 bytes per clock to L2: 14500 cycles for a tile of 256 x 192, which
+      // nothing hides where a tile is the CTA's only one.) Weight gradients, us, lanes / this, the same plans: 2048 rows of 384 x 384 10.4 / 6.9,
+      // 17280 of 192 x 192 11.4 / 8.8, 139264 of 384 x 384 49.6 / 46.3; convolution of 17280 pixels, 192 channels 20.8 / 18.
+      uint8_t* my_out = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
+      const uint32_t out_base = smem_u32(my_out);
+      for (Walk walk(p, unit, units); walk.tile < total_tiles; walk.next(p), ++tcount) {
+        const TileCoord first = walk.coord(p, rank, per_split);
+        const int acc = tcount % Cfg::ACCS, n0 = first.n_blk * BN;
+        const long long ew0 = clock64();
+        const bool tile_ready = mbar_wait<PAIR>(&tfull[acc], (tcount / Cfg::ACCS) & 1u, abort_flag, p.status, 0x400u + acc, mbar_budget);
+        if (!__all_sync(0xffffffffu, tile_ready)) break;
+        e_wait += clock64() - ew0;
+        tc_fence_after();
+#pragma unroll 1
+        for (int mb = 0; mb < STACK; ++mb) {
+          TileCoord tc = first;
+          tc.m_blk += mb;
+          if (STACK > 1 && tc.m_blk >= p.m_blocks) break;
+          const int dcol = STACK > 1 ? mb : acc;
+          int row = tc.m_blk * GEMM_BM + q * 32, group = tc.grp, rows = p.M;      // this warp's rows of the group (tap)
+          bool ones = false;
+          if (p.tap_boxes > 0) {
+            group = (row >> 6) / p.tap_boxes;
+            row -= group * p.tap_boxes * 64;
+            ones = group == p.taps && row == 0 && p.row_sums != nullptr;
+            if (group >= p.taps) rows = 0;
+          }
+          if (row < rows || ones) {
+#pragma unroll 1
+            for (int c = part; c < CHUNKS && n0 + c * 32 < p.N; c += GEMM_EPI_WARPS / 4) {      // warp-uniform
+              const int cb = n0 + c * 32;
+              uint32_t v[32];
+              tmem_ld_32x32(tmem_base + dcol * BN + c * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
+              if (lane == 0) bulk_wait_group_read<0>();      // the unit before has left the buffer
+              tmem_ld_wait();
+              if (p.alpha != 1.0f) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * p.alpha);
+              }
+              __syncwarp();
+              if (p.epi & EPI_TRANSPOSE) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  asm volatile("st.shared.b32 [%0], %1;" ::"r"(out_base + j * 128 + (((lane >> 2) ^ (j & 7)) << 4) + ((lane & 3) << 2)), "r"(v[j])
+                               : "memory");
+              } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out_base + lane * 128 + ((j ^ (lane & 7)) << 4)), "r"(v[4 * j]),
+                               "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
+                               : "memory");
+              }
+              if (ones) {      // row 0: the column sums of B
+                __syncwarp();
+                if (cb + lane < p.N) atomicAdd(p.row_sums + cb + lane, *reinterpret_cast<const float*>(my_out + lane * 4));
+                continue;
+              }
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                if (p.epi & EPI_TRANSPOSE) tma_reduce_add_3d(&p.map_c, out_base, row, cb, 0);
+                else tma_reduce_add_3d(&p.map_c, out_base, cb, row, group);
+                bulk_commit_group();
+              }
+            }
+          }
+          add_column_sums(tc, dcol);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (PAIR && rank == 1) mbar_arrive_remote(map_to_cta(&tempty[acc], 0));   // the leader's MMA thread waits
+          else mbar_arrive(&tempty[acc]);
+        }
+      }
+      if (lane == 0) bulk_wait_group_read<0>();
     } else
     for (Walk walk(p, unit, units); walk.tile < total_tiles; walk.next(p), ++tcount) {
       const TileCoord first = walk.coord(p, rank, per_split);
@@ -1056,18 +1150,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             store_chunk(static_cast<__nv_bfloat16*>(p.C) + gofs, p.ldc, cb, f);
           }
         }
-        if (Cfg::CAN_COLSUM && p.colsum != nullptr && part == 0 &&
-            first_sum_kb(p, tc, p.disp_a ? p.num_n_tiles : p.groups * p.num_n_tiles) < tc.kb_end) {
-          uint32_t v[32];   // column 0 of the sums accumulator: lane l holds the sum of A's column (row of D) q * 32 + l
-          tmem_ld_32x32(tmem_base + Cfg::SUM_COL0 + dcol * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
-          tmem_ld_wait();
-          int g = tc.m_blk * GEMM_BM + q * 32 + lane;
-          if (p.tap_boxes > 0) {      // (the taps' sums add up)
-            const int tap = (g >> 6) / p.tap_boxes;
-            g = tap < p.taps ? g - tap * p.tap_boxes * 64 : p.M;
-          }
-          if (g < p.M) atomicAdd(p.colsum + g, __uint_as_float(v[0]) * p.alpha);
-        }
+        add_column_sums(tc, dcol);
       }
       if (failed) break;
       tc_fence_before();
@@ -1109,7 +1192,7 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
     configured.store(true, std::memory_order_relaxed);
   }
   GemmParams p = p_in;
-  if (PEERS || STACK > 1) p.epi_tma = 0;
+  if (PEERS || (STACK > 1 && p.epi_tma != 3) || (p.epi_tma == 3 && Cfg::stages_for(2) < 3)) p.epi_tma = 0;
   // (a long contraction hides the epilogue behind its main loop and wants the deeper ring: one buffer for input and output)
   const bool has_in = (p.epi & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
   p.epi_bufs = p.epi_tma == 0 ? 1 : ((p.epi & EPI_SAVE_PRE) || (has_in && p.k_blocks <= 12) ? 4 : 2);
@@ -1147,7 +1230,17 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, p);
 }
 
-cudaError_t gemm_ones_tile(void** ptr) { return cudaGetSymbolAddress(ptr, g_ones_tile); }
+cudaError_t gemm_ones_tile(void** ptr) {
+  static std::atomic<void*> known[64];      // per device: the look-up takes a microsecond
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  *ptr = dev < 64 ? known[dev].load(std::memory_order_relaxed) : nullptr;
+  if (*ptr != nullptr) return cudaSuccess;
+  e = cudaGetSymbolAddress(ptr, g_ones_tile);
+  if (e == cudaSuccess && dev < 64) known[dev].store(*ptr, std::memory_order_relaxed);
+  return e;
+}
 
 cudaError_t gemm_read_stalls(unsigned long long* out8, bool reset) {
   cudaError_t e = cudaMemcpyFromSymbol(out8, g_gemm_stalls, 8 * sizeof(unsigned long long));

@@ -79,7 +79,8 @@ struct GemmParams {
   // stages / smem_bytes: the launcher sizes the operand ring with what the epilogue buffers leave.
   float* colsum;               // weight-gradient form: += column sums of operand A over the contraction (see GemmEpilogue)
   CUtensorMap map_c, map_c2, map_in;
-  int epi_tma;                 // 0: per-lane global accesses, 1: 2-D boxes of rows, 2: 5-D boxes of pixels (EPI_ROW_CONV)
+  int epi_tma;                 // 0: per-lane global accesses, 1: 2-D boxes of rows, 2: 5-D boxes of pixels (EPI_ROW_CONV), 3: reductions of
+                               // 32 x 32 fp32 units (map_c: {columns, rows, groups or taps}, EPI_TRANSPOSE: {rows, columns})
   int epi_bufs;
   int stages;
   int smem_bytes;

@@ -27,10 +27,10 @@
 //     chains to issue from, and half the reads of K and V through the shared-memory port;
 //   * accumulator tiles go to shared memory four 8 x 8 tiles an instruction;
 //   * windows of at most 32 tokens have blocks of their own size, and padding columns cost a comparison, not the masked form.
-// Us, before these three / now (shifted, with bias): 2176 windows of 8 x 8, 12 heads of 32 channels, forward 105 / 92 (66 of HBM
-// traffic), backward 236 / 233 (115); 2448 of 8 x 8, 8 heads of 128 channels 237 / 233 and 626 / 608; 180 of 8 x 12, 12 heads of 16
-// channels 26 / 25 and 50 / 49; 1020 of 7 x 7, 12 heads of 32 channels 93 / 57 and 140 / 119; 1800 of 4 x 8, 8 heads of 32 channels
-// 89 / 25 and 120 / 54. What is left is issue and latency: the shared-memory port is busy 50 (forward) and 70 % (backward) of the time.
+// Us, before these three / now (shifted, with bias): 2176 windows of 8 x 8, 12 heads of 32 channels, forward 105 / 88 (66 of HBM
+// traffic), backward 236 / 226 (115); 2448 of 8 x 8, 8 heads of 128 channels 237 / 235 and 626 / 612; 180 of 8 x 12, 12 heads of 16
+// channels 26 / 17 and 50 / 43; 1020 of 7 x 7, 12 heads of 32 channels 93 / 53 and 140 / 120; 1800 of 4 x 8, 8 heads of 32 channels
+// 89 / 22 and 120 / 54. What is left is issue and latency: the shared-memory port is busy 50 (forward) and 70 % (backward) of the time.
 #include <atomic>
 #include "chained_launch.cuh"
 #include "common.cuh"
@@ -193,7 +193,7 @@ __device__ __forceinline__ void wa_store(void* const* bases, long long ld, int c
 __device__ __forceinline__ f32x2 wa_pair(const float (&v)[4], int i) { return f2_pack(v[i], v[i + 1]); }
 __device__ __forceinline__ void wa_set(float (&v)[4], int i, f32x2 x) { f2_unpack(x, v[i], v[i + 1]); }
 
-// Scores of a 16-row block: s <- s * scale + bias (+ mask), base-2 domain, and the row maxima of this thread's columns.
+// Scores of a 16-row block: s <- s * scale + bias, base-2 domain, and the row maxima of this thread's columns.
 // `tb` is the head's table in shared memory, pre-multiplied by log2(e). The table index of (query r, key c) is
 // cofs(r) - cofs(c) + rel0 with cofs(t) = (t / ww) (2 ww - 1) + t % ww. For windows 8 (12) wide the columns of a thread
 // repeat every 1 (3) blocks of 8, so an index is one of 1 (3) per-thread bases plus a compile-time constant; other
@@ -201,107 +201,107 @@ __device__ __forceinline__ void wa_set(float (&v)[4], int i, f32x2 x) { f2_unpac
 // A warp's block is MT tiles of 16 rows (rows r0 + 16 t and r0 + 16 t + 8 of this thread).
 template <int NPAD, int WW, int MT>
 __device__ __forceinline__ void wa_scores(float (&s)[MT][NPAD / 8][4], float scale2, const float* tb, int rel0, const int* cofs,
-                                          const int2* tab, int r0, int tq, int N, bool general, bool use_mask, float (&mx)[MT][2]) {
-  if (!general) {
-    if constexpr (WW == 8) {
-      // row r0 + 8 is the next window row, same column: its bias at key block nb is row r0's at block nb - 1, and so on for the rows below
-      const float* p = tb + ((r0 >> 3) * 15 + (r0 & 7) - 2 * tq + rel0);
-      float b[2 * MT][2];      // this key block's bias of rows r0, r0 + 8, ...
+                                          int r0, int tq, int N, float (&mx)[MT][2]) {
+  if constexpr (WW == 8) {
+    // row r0 + 8 is the next window row, same column: its bias at key block nb is row r0's at block nb - 1, and so on for the rows below
+    const float* p = tb + ((r0 >> 3) * 15 + (r0 & 7) - 2 * tq + rel0);
+    float b[2 * MT][2];      // this key block's bias of rows r0, r0 + 8, ...
 #pragma unroll
-      for (int i = 1; i < 2 * MT; ++i) b[i][0] = p[15 * i], b[i][1] = p[15 * i - 1];
+    for (int i = 1; i < 2 * MT; ++i) b[i][0] = p[15 * i], b[i][1] = p[15 * i - 1];
+#pragma unroll
+    for (int nb = 0; nb < NPAD / 8; ++nb) {
+      b[0][0] = p[-15 * nb];
+      b[0][1] = p[-15 * nb - 1];
+#pragma unroll
+      for (int t = 0; t < MT; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          wa_set(s[t][nb], 2 * h, f2_fma(wa_pair(s[t][nb], 2 * h), f2_both(scale2), f2_pack(b[2 * t + h][0], b[2 * t + h][1])));
+          mx[t][h] = fmaxf(mx[t][h], fmaxf(s[t][nb][2 * h], s[t][nb][2 * h + 1]));
+        }
+#pragma unroll
+      for (int i = 2 * MT - 1; i > 0; --i) b[i][0] = b[i - 1][0], b[i][1] = b[i - 1][1];
+    }
+  } else if constexpr (WW == 12) {
+#pragma unroll
+    for (int t = 0; t < MT; ++t) {
+      const int ra = r0 + 16 * t;
+      const int ro0 = cofs[ra] + rel0, dr = cofs[ra + 8] - cofs[ra];
+      // columns 8 m + 2 tq of the first three blocks, m = 0, 1, 2; later blocks are whole window rows (2 per 3 blocks) on
+      const float* p[3];
+      p[0] = tb + ro0 - 2 * tq;
+      p[1] = tb + ro0 - (tq < 2 ? 8 + 2 * tq : 23 + 2 * tq - 4);
+      p[2] = tb + ro0 - (23 + 4 + 2 * tq);
 #pragma unroll
       for (int nb = 0; nb < NPAD / 8; ++nb) {
-        b[0][0] = p[-15 * nb];
-        b[0][1] = p[-15 * nb - 1];
-#pragma unroll
-        for (int t = 0; t < MT; ++t)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            wa_set(s[t][nb], 2 * h, f2_fma(wa_pair(s[t][nb], 2 * h), f2_both(scale2), f2_pack(b[2 * t + h][0], b[2 * t + h][1])));
-            mx[t][h] = fmaxf(mx[t][h], fmaxf(s[t][nb][2 * h], s[t][nb][2 * h + 1]));
-          }
-#pragma unroll
-        for (int i = 2 * MT - 1; i > 0; --i) b[i][0] = b[i - 1][0], b[i][1] = b[i - 1][1];
-      }
-    } else if constexpr (WW == 12) {
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const int ra = r0 + 16 * t;
-        const int ro0 = cofs[ra] + rel0, dr = cofs[ra + 8] - cofs[ra];
-        // columns 8 m + 2 tq of the first three blocks, m = 0, 1, 2; later blocks are whole window rows (2 per 3 blocks) on
-        const float* p[3];
-        p[0] = tb + ro0 - 2 * tq;
-        p[1] = tb + ro0 - (tq < 2 ? 8 + 2 * tq : 23 + 2 * tq - 4);
-        p[2] = tb + ro0 - (23 + 4 + 2 * tq);
-#pragma unroll
-        for (int nb = 0; nb < NPAD / 8; ++nb) {
-          const float* c = p[nb % 3] - (nb / 3) * 46;
-          wa_set(s[t][nb], 0, f2_fma(wa_pair(s[t][nb], 0), f2_both(scale2), f2_pack(c[0], c[-1])));
-          wa_set(s[t][nb], 2, f2_fma(wa_pair(s[t][nb], 2), f2_both(scale2), f2_pack(c[dr], c[dr - 1])));
-          mx[t][0] = fmaxf(mx[t][0], fmaxf(s[t][nb][0], s[t][nb][1]));
-          mx[t][1] = fmaxf(mx[t][1], fmaxf(s[t][nb][2], s[t][nb][3]));
-        }
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const float *t0 = tb + cofs[r0 + 16 * t] + rel0, *t1 = tb + cofs[r0 + 16 * t + 8] + rel0;
-#pragma unroll
-        for (int nb = 0; nb < NPAD / 8; ++nb) {
-          const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
-          s[t][nb][0] = fmaf(s[t][nb][0], scale2, t0[-co.x]);
-          s[t][nb][1] = fmaf(s[t][nb][1], scale2, t0[-co.y]);
-          s[t][nb][2] = fmaf(s[t][nb][2], scale2, t1[-co.x]);
-          s[t][nb][3] = fmaf(s[t][nb][3], scale2, t1[-co.y]);
-          if (nb * 8 + 8 > N) {      // padding columns: their scores are lowest, their probabilities zero
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (nb * 8 + tq * 2 + (k & 1) >= N) s[t][nb][k] = -1e30f;
-          }
-          mx[t][0] = fmaxf(mx[t][0], fmaxf(s[t][nb][0], s[t][nb][1]));
-          mx[t][1] = fmaxf(mx[t][1], fmaxf(s[t][nb][2], s[t][nb][3]));
-        }
+        const float* c = p[nb % 3] - (nb / 3) * 46;
+        wa_set(s[t][nb], 0, f2_fma(wa_pair(s[t][nb], 0), f2_both(scale2), f2_pack(c[0], c[-1])));
+        wa_set(s[t][nb], 2, f2_fma(wa_pair(s[t][nb], 2), f2_both(scale2), f2_pack(c[dr], c[dr - 1])));
+        mx[t][0] = fmaxf(mx[t][0], fmaxf(s[t][nb][0], s[t][nb][1]));
+        mx[t][1] = fmaxf(mx[t][1], fmaxf(s[t][nb][2], s[t][nb][3]));
       }
     }
   } else {
-    // windows that the mask cuts
 #pragma unroll
     for (int t = 0; t < MT; ++t) {
-      const int ra = r0 + 16 * t, rb = ra + 8;
-      const int reg0 = tab[ra].y >> 8, reg1 = tab[rb].y >> 8;
-      const bool row0 = ra < N, row1 = rb < N;
-      const float *t0 = tb + (row0 ? cofs[ra] + rel0 : 0), *t1 = tb + (row1 ? cofs[rb] + rel0 : 0);
+      const float *t0 = tb + cofs[r0 + 16 * t] + rel0, *t1 = tb + cofs[r0 + 16 * t + 8] + rel0;
 #pragma unroll
       for (int nb = 0; nb < NPAD / 8; ++nb) {
         const int2 co = *reinterpret_cast<const int2*>(cofs + nb * 8 + tq * 2);
+        s[t][nb][0] = fmaf(s[t][nb][0], scale2, t0[-co.x]);
+        s[t][nb][1] = fmaf(s[t][nb][1], scale2, t0[-co.y]);
+        s[t][nb][2] = fmaf(s[t][nb][2], scale2, t1[-co.x]);
+        s[t][nb][3] = fmaf(s[t][nb][3], scale2, t1[-co.y]);
+        if (nb * 8 + 8 > N) {      // padding columns: their scores are lowest, their probabilities zero
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int col = nb * 8 + tq * 2 + (k & 1);
-          const bool lo = k < 2;
-          float v = s[t][nb][k] * scale2;
-          if (col < N) {
-            if (lo ? row0 : row1) v += (lo ? t0 : t1)[-((k & 1) ? co.y : co.x)];
-            if (use_mask && (tab[col].y >> 8) != (lo ? reg0 : reg1)) v += -100.f * WA_LOG2E;
-          } else {
-            v = -1e30f;
-          }
-          s[t][nb][k] = v;
-          mx[t][lo ? 0 : 1] = fmaxf(mx[t][lo ? 0 : 1], v);
+          for (int k = 0; k < 4; ++k)
+            if (nb * 8 + tq * 2 + (k & 1) >= N) s[t][nb][k] = -1e30f;
         }
+        mx[t][0] = fmaxf(mx[t][0], fmaxf(s[t][nb][0], s[t][nb][1]));
+        mx[t][1] = fmaxf(mx[t][1], fmaxf(s[t][nb][2], s[t][nb][3]));
       }
     }
   }
 }
 
-// d[t] = A(16 rows at `arow` + 16 t, HD channels) * B(NPAD rows at `bmat`)^T, both row-major bf16 in shared memory
-template <int HD, int NPAD, int PITCH, int MT>
-__device__ __forceinline__ void wa_mma_nt(float (&d)[MT][NPAD / 8][4], const __nv_bfloat16* arow, const __nv_bfloat16* bmat, int lane) {
+template <int NPAD, int MT>
+__device__ __forceinline__ void wa_zero(float (&d)[MT][NPAD / 8][4]) {
 #pragma unroll
   for (int t = 0; t < MT; ++t)
 #pragma unroll
     for (int nb = 0; nb < NPAD / 8; ++nb)
 #pragma unroll
       for (int k = 0; k < 4; ++k) d[t][nb][k] = 0.f;
+}
+
+// What the products of q and k are added to: zero, or in a window that the mask cuts (few: the last row and column of the shifted frame) the
+// mask over the scale where query and key lie in different regions. There it costs a comparison an element and no register beyond the
+// sums' own; a score path of its own took three times as long, and the blocks that met it finished last. Us, such a path / this: 180
+// shifted windows of 8 x 12, 12 heads of 16 channels forward 24.5 / 16.5,
+// backward 49.1 / 42.9; 2176 of 8 x 8, 12 heads of 32 92.4 / 87.8 and 232.8 / 225.9. (Rounding: a masked
+// product loses its low bits to the mask's, which its probability of e^-100 hides.)
+template <int NPAD, int MT>
+__device__ __forceinline__ void wa_start_scores(float (&s)[MT][NPAD / 8][4], bool masked, float scale2, const int2* tab, int r0, int tq) {
+  wa_zero<NPAD, MT>(s);
+  if (!masked) return;
+  const float off = __fdividef(-100.f * WA_LOG2E, scale2);
+#pragma unroll
+  for (int t = 0; t < MT; ++t) {
+    const int reg0 = tab[r0 + 16 * t].y, reg1 = tab[r0 + 16 * t + 8].y;
+#pragma unroll
+    for (int nb = 0; nb < NPAD / 8; ++nb) {
+      const int e0 = tab[nb * 8 + tq * 2].y, e1 = tab[nb * 8 + tq * 2 + 1].y;      // regions in bits 8 and up
+      if ((e0 ^ reg0) >> 8) s[t][nb][0] = off;
+      if ((e1 ^ reg0) >> 8) s[t][nb][1] = off;
+      if ((e0 ^ reg1) >> 8) s[t][nb][2] = off;
+      if ((e1 ^ reg1) >> 8) s[t][nb][3] = off;
+    }
+  }
+}
+
+// d[t] += A(16 rows at `arow` + 16 t, HD channels) * B(NPAD rows at `bmat`)^T, both row-major bf16 in shared memory
+template <int HD, int NPAD, int PITCH, int MT>
+__device__ __forceinline__ void wa_mma_nt(float (&d)[MT][NPAD / 8][4], const __nv_bfloat16* arow, const __nv_bfloat16* bmat, int lane) {
 #pragma unroll
   for (int kk = 0; kk < HD / 16; ++kk) {
     uint32_t af[MT][4];
@@ -438,7 +438,8 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
   const int items = a.B * my_nw;
   const int q0 = a.my_sp * a.shardN;
   const int q1 = min(N, q0 + a.shardN);
-  const float scale2 = a.scale * WA_LOG2E;
+  // (no scale at all: one that leaves nothing of the products, so that the mask can be divided by it)
+  const float scale2 = a.scale == 0.f ? 1e-30f : a.scale * WA_LOG2E;
   const int ti = tid / a.ww, tj = tid % a.ww;                    // token `tid` of a window
 
   if (tid < NPAD) {
@@ -499,18 +500,19 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
       next = wa_item(a, item + 2 * step, my_nw);
       if (tid < N) wa_table(a, geo, next, ti, tj, tabs + slot2 * NPAD + tid);
     }
-    const bool general = (WW != 0 && N != NPAD) || (a.use_mask && ((a.sh > 0 && mine.ii == a.nWh - 1) || (a.sw > 0 && mine.jj == a.nWw - 1)));
+    const bool masked = a.use_mask && ((a.sh > 0 && mine.ii == a.nWh - 1) || (a.sw > 0 && mine.jj == a.nWw - 1));
 
     if constexpr (!BWD) {
       if (row0 < q1 && row0 + 16 * MT > q0) {
 #pragma unroll 1
         for (int hh = MT == 1 ? 0 : my_head; hh < (MT == 1 ? HPC : my_head + 1); ++hh) {
           float s[MT][NB][4];
+          wa_start_scores<NPAD, MT>(s, masked, scale2, tab, r0, tq);
           wa_mma_nt<HD, NPAD, PITCH, MT>(s, Qs + row0 * PITCH + hh * HD, Ks + hh * HD, lane);
           float mx[MT][2], inv[MT][2];
 #pragma unroll
           for (int t = 0; t < MT; ++t) mx[t][0] = mx[t][1] = -1e30f;
-          wa_scores<NPAD, WW, MT>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx);
+          wa_scores<NPAD, WW, MT>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, r0, tq, N, mx);
 #pragma unroll
           for (int t = 0; t < MT; ++t) wa_softmax<NPAD>(s[t], mx[t][0], mx[t][1], inv[t][0], inv[t][1]);
           // O = P V with the numerators as P, the row normalisation applied to the (smaller) output; staged over this
@@ -536,9 +538,11 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
       if (row0 < N) {
         float s1[1][NB][4], dp1[1][NB][4], mx[1][2] = {{-1e30f, -1e30f}}, inv0, inv1;
         float(&s)[NB][4] = s1[0], (&dp)[NB][4] = dp1[0];
+        wa_start_scores<NPAD, 1>(s1, masked, scale2, tab, r0, tq);
         wa_mma_nt<HD, NPAD, PITCH, 1>(s1, Qs + row0 * PITCH, Ks, lane);
-        wa_scores<NPAD, WW, 1>(s1, scale2, bias_s, rel0, cofs, tab, r0, tq, N, general, a.use_mask, mx);
+        wa_scores<NPAD, WW, 1>(s1, scale2, bias_s, rel0, cofs, r0, tq, N, mx);
         wa_softmax<NPAD>(s, mx[0][0], mx[0][1], inv0, inv1);
+        wa_zero<NPAD, 1>(dp1);
         wa_mma_nt<HD, NPAD, PITCH, 1>(dp1, dOs + row0 * PITCH, Vs, lane);        // dP = dO V^T
         f32x2 e0 = f2_both(0.f), e1 = f2_both(0.f);
 #pragma unroll

@@ -1,5 +1,6 @@
 // Memory-bound kernels: LayerNorm, GroupNorm(+SiLU), column sums, masked loss, fused AdamW.
 // All are single-pass over HBM where the math allows it, with 16-byte vector accesses.
+#include <algorithm>
 #include <cstdlib>
 #include "chained_launch.cuh"
 #include "common.cuh"
@@ -27,6 +28,49 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 }
+
+// A thread's own 16-byte vectors on their way through shared memory: K tensors, S steps ahead, read two steps at a time (instructions of one issue
+// between those of the other). What kernels over HBM lack beside bandwidth is loads in flight: held in registers, a round's loads are issued,
+// waited for and used in turn, while cp.async fetches the next rounds meanwhile and costs no register. Every thread reads only what it fetched,
+// so there is no barrier.
+template <int K, int S>
+struct LaneRing {
+  static_assert(S % 2 == 0 && S >= 4, "rounds of two steps");
+  uint32_t at, stride;      // this thread's slot; bytes between slots
+  int s = 0;                // the step to be read next
+  static constexpr int bytes(int threads) { return K * S * 16 * threads; }
+  __device__ __forceinline__ LaneRing(void* smem, int thread, int threads) : at(smem_u32(smem) + thread * 16), stride(threads * 16) {}
+  __device__ __forceinline__ void put(int slot, int k, const void* src) const {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + (slot * K + k) * stride), "l"(src) : "memory");
+  }
+  // the vectors of round `p`, two pixels `by` apart, into the slots read last (or, at the start, slots `slot` and `slot` + 1)
+  template <class Src>
+  __device__ __forceinline__ void fetch(int slot, long long p, long long by, long long end, long long pitch, const Src* const* src) const {
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (p + u * by < end) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          put(slot + u, k, src[k] + (p + u * by) * pitch);
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  template <class Src>
+  __device__ __forceinline__ void start(long long p, long long by, long long end, long long pitch, const Src* const* src) const {
+#pragma unroll
+    for (int u = 0; u < S; u += 2) fetch(u, p + u * by, by, end, pitch, src);
+  }
+  __device__ __forceinline__ void wait() const { asm volatile("cp.async.wait_group %0;" ::"n"(S / 2 - 1) : "memory"); }
+  __device__ __forceinline__ uint4 read(int u, int k) const {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(at + ((s + u) * K + k) * stride)
+                 : "memory");
+    return v;
+  }
+  __device__ __forceinline__ void next() { s = s + 2 == S ? 0 : s + 2; }
+};
 
 // ------------------------------------------------------------------------------------------ LayerNorm
 // Both kernels are bound by HBM. A row is held in registers by LPR lanes of VPL 16-byte vectors each, so that a warp
@@ -344,6 +388,10 @@ __device__ __forceinline__ void gn_block_sums(float* sh, float* buf, const float
   __syncthreads();
 }
 
+constexpr int GN_AHEAD = 4;      // pixels in flight per thread
+using GnStatsRing = LaneRing<1, GN_AHEAD>;
+using GnPairRing = LaneRing<2, GN_AHEAD>;
+
 __device__ __forceinline__ void gn_finalize_cell(float* sums, float* stats, int i, float inv_count, float eps) {
   const float mean = __ldcg(sums + 2 * i) * inv_count;
   const float var = fmaxf(__ldcg(sums + 2 * i + 1) * inv_count - mean * mean, 0.f);
@@ -369,25 +417,32 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
   for (int v0 = 0; v0 < nvec; v0 += blockDim.x) {
     const int vi = v0 + threadIdx.x;
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const uint4* src = reinterpret_cast<const uint4*>(x) + static_cast<long long>(b) * HW * nvec + vi;
-    for (long long p = p0 + threadIdx.y; vi < nvec && p < p1; p += 4 * blockDim.y) {
-      uint4 t[4];
+    if (vi < nvec) {
+      const uint4* src = reinterpret_cast<const uint4*>(x) + static_cast<long long>(b) * HW * nvec + vi;
+      const uint4* const from[1] = {src};
+      GnStatsRing ring(sh + 2 * C, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
+      const long long by = blockDim.y;
+      ring.start(p0 + threadIdx.y, by, p1, nvec, from);
+#pragma unroll 1
+      for (long long p = p0 + threadIdx.y; p < p1; p += 2 * by) {
+        ring.wait();
+        const uint4 t[2] = {ring.read(0, 0), ring.read(1, 0)};
+        ring.fetch(ring.s, p + GN_AHEAD * by, by, p1, nvec, from);
+        ring.next();
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        t[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (p + u * blockDim.y < p1) t[u] = src[(p + u * blockDim.y) * nvec];
-      }
+        for (int u = 0; u < 2; ++u) {
+          if (u == 1 && p + by >= p1) break;
+          float f[8];
+          unpack8(t[u], f);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float f[8];
-        unpack8(t[u], f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          s[j] += f[j];
-          q[j] += f[j] * f[j];
+          for (int j = 0; j < 8; ++j) {
+            s[j] += f[j];
+            q[j] += f[j] * f[j];
+          }
         }
       }
     }
+    __syncthreads();      // (the sums' buffer lies where the rings were)
     gn_block_sums(sh, sh + 2 * C, s, q, C, vi);
   }
   const int cpg = C / groups, tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -413,74 +468,6 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
   }
 }
 
-__device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + __expf(-z)); }
-
-// A thread's eight channels: statistics of their groups and affine parameters.
-struct GnChannels {
-  float mu[8], rs[8], g[8], bt[8];
-};
-__device__ __forceinline__ void gn_channels(GnChannels& c, const float* __restrict__ stats, const __nv_bfloat16* __restrict__ gamma,
-                                            const __nv_bfloat16* __restrict__ beta, int b, int vi, int cpg, int groups) {
-  unpack8(reinterpret_cast<const uint4*>(gamma)[vi], c.g);
-  unpack8(reinterpret_cast<const uint4*>(beta)[vi], c.bt);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int grp = (vi * 8 + j) / cpg;
-    c.mu[j] = stats[(b * groups + grp) * 2];
-    c.rs[j] = stats[(b * groups + grp) * 2 + 1];
-  }
-}
-
-__global__ void __launch_bounds__(256, 3) groupnorm_silu_apply_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                      const float* __restrict__ stats,
-                                                                      const __nv_bfloat16* __restrict__ gamma,
-                                                                      const __nv_bfloat16* __restrict__ beta,
-                                                                      const __nv_bfloat16* __restrict__ res,
-                                                                      __nv_bfloat16* __restrict__ y, long long HW, int C,
-                                                                      int groups, int pix_per_block) {
-  chain_begin();
-  const int nvec = C >> 3;
-  const int b = blockIdx.y;
-  const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
-  const long long p1 = min(HW, p0 + pix_per_block);
-  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
-    GnChannels c;
-    gn_channels(c, stats, gamma, beta, b, vi, C / groups, groups);
-    const long long first = static_cast<long long>(b) * HW * nvec + vi;
-    const uint4* src = reinterpret_cast<const uint4*>(x) + first;
-    const uint4* add = reinterpret_cast<const uint4*>(res) + first;
-    uint4* dst = reinterpret_cast<uint4*>(y) + first;
-    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
-      uint4 t[2], r[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (p + u * blockDim.y < p1) {
-          t[u] = src[(p + u * blockDim.y) * nvec];
-          if (res != nullptr) r[u] = add[(p + u * blockDim.y) * nvec];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (p + u * blockDim.y >= p1) break;
-        float f[8], o[8];
-        unpack8(t[u], f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float z = (f[j] - c.mu[j]) * c.rs[j] * c.g[j] + c.bt[j];
-          o[j] = z * sigmoidf_(z);
-        }
-        if (res != nullptr) {
-          float rr[8];
-          unpack8(r[u], rr);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += rr[j];
-        }
-        dst[(p + u * blockDim.y) * nvec] = pack8(o);
-      }
-    }
-  }
-}
-
 // Two channels' constants, and SiLU's derivative part of them: xhat and dz = dy * silu'(z), z = xhat * gamma + beta.
 struct GnPair {
   f32x2 nmu, rs, g, bt;      // minus the mean, reciprocal deviation, affine parameters
@@ -491,17 +478,78 @@ __device__ __forceinline__ GnPair gn_pair(const float* __restrict__ stats, uint3
   const float2 g = unpack_bf16x2(gamma2), bt = unpack_bf16x2(beta2);
   return {f2_pack(-s0[0], -s1[0]), f2_pack(s0[1], s1[1]), f2_pack(g.x, g.y), f2_pack(bt.x, bt.y)};
 }
+// a thread's eight channels
+__device__ __forceinline__ void gn_pairs(GnPair (&c)[4], const float* __restrict__ stats, const __nv_bfloat16* __restrict__ gamma,
+                                         const __nv_bfloat16* __restrict__ beta, int b, int vi, int cpg, int groups) {
+  const uint4 gq = reinterpret_cast<const uint4*>(gamma)[vi], bq = reinterpret_cast<const uint4*>(beta)[vi];
+  const uint32_t g4[4] = {gq.x, gq.y, gq.z, gq.w}, b4[4] = {bq.x, bq.y, bq.z, bq.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) c[j] = gn_pair(stats, g4[j], b4[j], b, vi * 8 + 2 * j, cpg, groups);
+}
 __device__ __forceinline__ f32x2 f2_of_bf16x2(uint32_t v) {
   const float2 f = unpack_bf16x2(v);
   return f2_pack(f.x, f.y);
 }
-// (two elements per instruction; the same operations as sigmoidf_ in the same order)
+// 1 / (1 + exp(-z)), two elements per instruction
 __device__ __forceinline__ f32x2 f2_sigmoid(f32x2 z) {
   float a, b;
   f2_unpack(f2_mul(z, f2_both(-1.4426950408889634f)), a, b);
   f2_unpack(f2_add(f2_pack(exp2f(a), exp2f(b)), f2_both(1.f)), a, b);
   return f2_pack(__fdividef(1.f, a), __fdividef(1.f, b));
 }
+// RES: a shortcut is added (without it twice the pixels ahead make up for the second tensor's loads)
+template <bool RES>
+__global__ void __launch_bounds__(256, 2) groupnorm_silu_apply_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                      const float* __restrict__ stats,
+                                                                      const __nv_bfloat16* __restrict__ gamma,
+                                                                      const __nv_bfloat16* __restrict__ beta,
+                                                                      const __nv_bfloat16* __restrict__ res,
+                                                                      __nv_bfloat16* __restrict__ y, long long HW, int C,
+                                                                      int groups, int pix_per_block) {
+  chain_begin();
+  extern __shared__ uint4 gn_ring[];
+  const int nvec = C >> 3;
+  const int b = blockIdx.y;
+  const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
+  const long long p1 = min(HW, p0 + pix_per_block);
+  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
+    GnPair c[4];
+    gn_pairs(c, stats, gamma, beta, b, vi, C / groups, groups);
+    const long long first = static_cast<long long>(b) * HW * nvec + vi;
+    const uint4* from[RES ? 2 : 1];
+    from[0] = reinterpret_cast<const uint4*>(x) + first;
+    if constexpr (RES) from[1] = reinterpret_cast<const uint4*>(res) + first;
+    uint4* dst = reinterpret_cast<uint4*>(y) + first;
+    constexpr int AHEAD = RES ? GN_AHEAD : 2 * GN_AHEAD;
+    LaneRing<RES ? 2 : 1, AHEAD> ring(gn_ring, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
+    const long long by = blockDim.y;
+    ring.start(p0 + threadIdx.y, by, p1, nvec, from);
+#pragma unroll 1
+    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * by) {
+      ring.wait();
+      const uint4 t[2] = {ring.read(0, 0), ring.read(1, 0)};
+      uint4 r[2] = {};
+      if constexpr (RES) r[0] = ring.read(0, 1), r[1] = ring.read(1, 1);
+      ring.fetch(ring.s, p + AHEAD * by, by, p1, nvec, from);
+      ring.next();
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (u == 1 && p + by >= p1) break;
+        const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, r4[4] = {r[u].x, r[u].y, r[u].z, r[u].w};
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 z = f2_fma(f2_mul(f2_add(f2_of_bf16x2(x4[j]), c[j].nmu), c[j].rs), c[j].g, c[j].bt);
+          f32x2 v = f2_mul(z, f2_sigmoid(z));
+          if constexpr (RES) v = f2_add(v, f2_of_bf16x2(r4[j]));
+          o[j] = f2_to_bf16x2(v);
+        }
+        dst[(p + u * by) * nvec] = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    }
+  }
+}
+
 __device__ __forceinline__ f32x2 gn_dz(const GnPair& c, f32x2 x, f32x2 dy, f32x2& xh) {
   xh = f2_mul(f2_add(x, c.nmu), c.rs);
   const f32x2 z = f2_fma(xh, c.g, c.bt), sg = f2_sigmoid(z);
@@ -512,7 +560,7 @@ __device__ __forceinline__ f32x2 gn_dz(const GnPair& c, f32x2 x, f32x2 dy, f32x2
 // no shared-memory atomics, eight loads in flight per thread of two blocks (us, before / these two / eight loads: 557056 pixels x 384 257 / 244 /
 // 193, 139264 x 384 - / 68 / 54, 64800 x 192 - / 19 / 15, 17280 x 192 17.4 / - / 8.3; with three blocks the registers do not reach: 236).
 // Statistics of 17280 x 192: 10.1 and 1.4 for a launch that finished them / 7.1.
-__global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_reduce_kernel(
+__global__ void __launch_bounds__(512, 1) groupnorm_silu_bwd_reduce_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta, float* __restrict__ red,
     long long HW, int C, int groups, int pix_per_block, float* __restrict__ dgamma, float* __restrict__ dbeta) {
@@ -529,29 +577,24 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_reduce_kernel(
     for (int j = 0; j < 4; ++j) s2[j] = q2[j] = f2_both(0.f);
     if (vi < nvec) {
       GnPair c[4];
-      {
-        const uint4 gq = reinterpret_cast<const uint4*>(gamma)[vi], bq = reinterpret_cast<const uint4*>(beta)[vi];
-        const uint32_t g4[4] = {gq.x, gq.y, gq.z, gq.w}, b4[4] = {bq.x, bq.y, bq.z, bq.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = gn_pair(stats, g4[j], b4[j], b, vi * 8 + 2 * j, C / groups, groups);
-      }
+      gn_pairs(c, stats, gamma, beta, b, vi, C / groups, groups);
       const long long first = static_cast<long long>(b) * HW * nvec + vi;
       const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
       const uint4* ds = reinterpret_cast<const uint4*>(dy) + first;
-      for (long long p = p0 + threadIdx.y; p < p1; p += 4 * blockDim.y) {
-        uint4 t[4], d2[4];
+      const uint4* const from[2] = {xs, ds};
+      GnPairRing ring(sh + 2 * C, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
+      const long long by = blockDim.y;
+      ring.start(p0 + threadIdx.y, by, p1, nvec, from);
+#pragma unroll 1
+      for (long long p = p0 + threadIdx.y; p < p1; p += 2 * by) {
+        ring.wait();
+        const uint4 t[2] = {ring.read(0, 0), ring.read(1, 0)}, d[2] = {ring.read(0, 1), ring.read(1, 1)};
+        ring.fetch(ring.s, p + GN_AHEAD * by, by, p1, nvec, from);
+        ring.next();
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          t[u] = d2[u] = make_uint4(0u, 0u, 0u, 0u);
-          if (p + u * blockDim.y < p1) {
-            t[u] = xs[(p + u * blockDim.y) * nvec];
-            d2[u] = ds[(p + u * blockDim.y) * nvec];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (p + u * blockDim.y >= p1) break;
-          const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, d4[4] = {d2[u].x, d2[u].y, d2[u].z, d2[u].w};
+        for (int u = 0; u < 2; ++u) {
+          if (u == 1 && p + by >= p1) break;
+          const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, d4[4] = {d[u].x, d[u].y, d[u].z, d[u].w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             f32x2 xh;
@@ -562,6 +605,7 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_reduce_kernel(
         }
       }
     }
+    __syncthreads();      // (the sums' buffer lies where the rings were)
     float s[8], q[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -671,12 +715,10 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
     GnPair c[4];
     f32x2 nm1[4], nm2[4];
     {
-      const uint4 gq = reinterpret_cast<const uint4*>(gamma)[vi], bq = reinterpret_cast<const uint4*>(beta)[vi];
-      const uint32_t g4[4] = {gq.x, gq.y, gq.z, gq.w}, b4[4] = {bq.x, bq.y, bq.z, bq.w};
+      gn_pairs(c, stats, gamma, beta, b, vi, cpg, groups);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int ch = vi * 8 + 2 * j;
-        c[j] = gn_pair(stats, g4[j], b4[j], b, ch, cpg, groups);
         nm1[j] = f2_pack(-gs[ch / cpg * 2], -gs[(ch + 1) / cpg * 2]);
         nm2[j] = f2_pack(-gs[ch / cpg * 2 + 1], -gs[(ch + 1) / cpg * 2 + 1]);
       }
@@ -685,19 +727,20 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
     const uint4* xs = reinterpret_cast<const uint4*>(x) + first;
     const uint4* ds = reinterpret_cast<const uint4*>(dy) + first;
     uint4* dst = reinterpret_cast<uint4*>(dx) + first;
-    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * blockDim.y) {
-      uint4 t[2], d2[2];
+    const uint4* const from[2] = {xs, ds};
+    GnPairRing ring(gs + (groups * 2 + 3) / 4 * 4, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
+    const long long by = blockDim.y;
+    ring.start(p0 + threadIdx.y, by, p1, nvec, from);
+#pragma unroll 1
+    for (long long p = p0 + threadIdx.y; p < p1; p += 2 * by) {
+      ring.wait();
+      const uint4 t[2] = {ring.read(0, 0), ring.read(1, 0)}, d[2] = {ring.read(0, 1), ring.read(1, 1)};
+      ring.fetch(ring.s, p + GN_AHEAD * by, by, p1, nvec, from);
+      ring.next();
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        if (p + u * blockDim.y < p1) {
-          t[u] = xs[(p + u * blockDim.y) * nvec];
-          d2[u] = ds[(p + u * blockDim.y) * nvec];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (p + u * blockDim.y >= p1) break;
-        const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, d4[4] = {d2[u].x, d2[u].y, d2[u].z, d2[u].w};
+        if (u == 1 && p + by >= p1) break;
+        const uint32_t x4[4] = {t[u].x, t[u].y, t[u].z, t[u].w}, d4[4] = {d[u].x, d[u].y, d[u].z, d[u].w};
         uint32_t o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -705,7 +748,7 @@ __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
           const f32x2 dz = gn_dz(c[j], f2_of_bf16x2(x4[j]), f2_of_bf16x2(d4[j]), xh);
           o[j] = f2_to_bf16x2(f2_mul(c[j].rs, f2_fma(xh, nm2[j], f2_fma(dz, c[j].g, nm1[j]))));
         }
-        dst[(p + u * blockDim.y) * nvec] = make_uint4(o[0], o[1], o[2], o[3]);
+        dst[(p + u * by) * nvec] = make_uint4(o[0], o[1], o[2], o[3]);
       }
     }
   }
@@ -1160,11 +1203,15 @@ static bool gn_sizes_ok(int B, long long HW, int C, int groups) {
   return B >= 1 && HW >= 1 && C >= 8 && C % 8 == 0 && groups >= 1 && C % groups == 0;
 }
 
-// [2][C] sums of the block and 16 per thread. Beyond the 48 KB that every launch may have (C >= 2048) the kernel is asked for more.
+// Images that stay in L2 are through before a second wave's blocks have paid for their set-up.
+static bool gn_small(int B, long long HW, int C) { return static_cast<long long>(B) * HW * C * 2 <= 72000000LL; }
+
+// [2][C] sums of the block, and 16 per thread where the threads' rings were. Beyond the 48 KB that every launch may have the kernel is asked for more.
 constexpr int GN_MAX_CHANNELS = 6144;
-template <class Kernel>
+template <class Ring, class Kernel>
 static size_t gn_smem(Kernel kernel, const GnShape& s, int C) {
-  const size_t bytes = (2 * static_cast<size_t>(C) + 16 * static_cast<size_t>(s.block.x) * s.block.y) * sizeof(float);
+  const int threads = s.block.x * s.block.y;
+  const size_t bytes = 2 * static_cast<size_t>(C) * sizeof(float) + std::max<size_t>(16 * sizeof(float) * threads, Ring::bytes(threads));
   if (bytes > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
   return bytes;
 }
@@ -1175,9 +1222,8 @@ static int groupnorm_stats_launch(const void* x, float* sums, int B, long long H
   // Every block ends in two atomics per group on the same addresses, and its warps meet in shared memory before. While the image
   // is L2-sized the passes over it are shorter than that, and one block per SM is enough (us, 1 / 3 blocks per SM: 64800 x 192 13 / 21,
   // 139264 x 128 15 / 22, 139264 x 256 20 / 23, 139264 x 384 52 / 29).
-  const bool small = static_cast<long long>(B) * HW * C * 2 <= 72000000LL;
-  const GnShape s(B, HW, C, 512, small ? 1 : 3, 4);
-  launch_chained(groupnorm_stats_kernel, s.grid, s.block, gn_smem(groupnorm_stats_kernel, s, C), stream, static_cast<const __nv_bfloat16*>(x),
+  const GnShape s(B, HW, C, 512, gn_small(B, HW, C) ? 1 : 3, 2);
+  launch_chained(groupnorm_stats_kernel, s.grid, s.block, gn_smem<GnStatsRing>(groupnorm_stats_kernel, s, C), stream, static_cast<const __nv_bfloat16*>(x),
                  sums, HW, C, groups, s.pix, stats, ticket, inv_count, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1193,8 +1239,9 @@ int groupnorm_mean_rstd(const void* x, float* sums, float* stats, int B, long lo
 int groupnorm_silu_apply(const void* x, const float* stats, const void* gamma, const void* beta, const void* res, void* y,
                          int B, long long HW, int C, int groups, cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
-  const GnShape s(B, HW, C, 256, 6, 2);
-  launch_chained(groupnorm_silu_apply_kernel, s.grid, s.block, 0, stream, static_cast<const __nv_bfloat16*>(x), stats,
+  const GnShape s(B, HW, C, 256, gn_small(B, HW, C) ? 2 : 4, 2);
+  launch_chained(res != nullptr ? groupnorm_silu_apply_kernel<true> : groupnorm_silu_apply_kernel<false>, s.grid, s.block,
+                 GnPairRing::bytes(s.block.x * s.block.y), stream, static_cast<const __nv_bfloat16*>(x), stats,
                  static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
                  static_cast<__nv_bfloat16*>(y), HW, C, groups, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1204,8 +1251,9 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
                               float* red, float* dgamma, float* dbeta, int B, long long HW, int C, int groups,
                               cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups) || C > GN_MAX_CHANNELS) return -1;
-  const GnShape s(B, HW, C, 256, 2, 4);
-  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, gn_smem(groupnorm_silu_bwd_reduce_kernel, s, C), stream,
+  const bool tiny = static_cast<long long>(B) * HW * C <= 1500000LL;      // (not enough pixels for larger blocks)
+  const GnShape s(B, HW, C, tiny ? 256 : 512, tiny ? 2 : 1, 2);
+  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, gn_smem<GnPairRing>(groupnorm_silu_bwd_reduce_kernel, s, C), stream,
                  static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
                  static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups, s.pix, dgamma, dbeta);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1236,8 +1284,9 @@ int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, 
                              const void* beta, void* dx, int B, long long HW, int C, int groups, float inv_count,
                              cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
-  const GnShape s(B, HW, C, 256, 4, 2);
-  launch_chained(groupnorm_silu_bwd_apply_kernel, s.grid, s.block, groups * 2 * sizeof(float), stream,
+  const GnShape s(B, HW, C, 256, gn_small(B, HW, C) ? 2 : 4, 2);
+  launch_chained(groupnorm_silu_bwd_apply_kernel, s.grid, s.block,
+                 (groups * 2 + 3) / 4 * 4 * sizeof(float) + GnPairRing::bytes(s.block.x * s.block.y), stream,
                  static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red, static_cast<const __nv_bfloat16*>(gamma),
                  static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(dx), HW, C, groups, inv_count, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -1,6 +1,7 @@
 // Memory-bound kernels: LayerNorm, GroupNorm(+SiLU), column sums, masked loss, fused AdamW.
 // All are single-pass over HBM where the math allows it, with 16-byte vector accesses.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include "chained_launch.cuh"
 #include "common.cuh"
@@ -16,6 +17,18 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// += of four neighbouring values, as one vector reduction where they are a whole 16-byte vector
+__device__ __forceinline__ void add4(float* to, const float4& v) {
+  if ((reinterpret_cast<uintptr_t>(to) & 15u) == 0) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+  } else {
+    atomicAdd(to, v.x);
+    atomicAdd(to + 1, v.y);
+    atomicAdd(to + 2, v.z);
+    atomicAdd(to + 3, v.w);
+  }
+}
+
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -27,6 +40,11 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
 }
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+
+__device__ __forceinline__ f32x2 f2_of_bf16x2(uint32_t v) {
+  const float2 f = unpack_bf16x2(v);
+  return f2_pack(f.x, f.y);
 }
 
 // A thread's own 16-byte vectors on their way through shared memory: K tensors, S steps ahead, read two steps at a time (instructions of one issue
@@ -76,10 +94,12 @@ struct LaneRing {
 // Both kernels are bound by HBM. A row is held in registers by LPR lanes of VPL 16-byte vectors each, so that a warp
 // carries 32 / LPR rows: a row of 48 vectors (C = 384) takes 16 lanes x 3 vectors, with no idle lane, where a whole warp
 // would leave half of its lanes idle in the second vector. LPR is the largest power of two that divides the row's
-// vectors; rows of more than 3 odd vectors per lane fall back to 32 lanes with a bounds test. The backward kernel keeps its
-// operands packed and computes x-hat twice, which lets three blocks of four warps share an SM.
-// 139264 x 384, one row per warp -> this: forward 49 -> 37 us (33 us at 6.5 TB/s), backward with shortcut 110 -> 79 us (65 us);
-// 139264 x 1024 backward 250 -> 234 us (175 us).
+// vectors; rows of more than 3 odd vectors per lane fall back to 32 lanes with a bounds test. The backward kernel has the next rows on their way
+// through shared memory, reads a row there twice (three blocks of four warps then share an SM), works on two columns per instruction and ends
+// in vector reductions without shared-memory atomics, which are compare-and-swap loops for floats.
+// 139264 x 384, one row per warp -> this: forward 49 -> 37 us (33 us at 6.5 TB/s). Backward with shortcut, us, rows in registers and scalar
+// atomics / the rest of this / those ends too: 139264 x 384 79 / 69 / 65 (65 at 6.5 TB/s), 156672 x 1024 262 / 204 / 202 (196), 17280 x 192 11.4 / 11.2 / 8.4, 2048 x 384
+// 10.8 / 10.8 / 6.4, 20000 x 512 23.6 / 21.5 / 15.5; with the shortcut's sums 156672 x 1024 380 / 262 / -.
 template <int LPR>
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -154,138 +174,176 @@ __global__ void __launch_bounds__(256, VPL == 1 ? 6 : (VPL == 2 ? 5 : (VPL <= 4 
   }
 }
 
-// SUMS: dsum += the column sums of dres as well, which passes through here anyway (the bias gradient of the layer before the shortcut).
-template <int LPR, int VPL, bool EXACT, bool SUMS>
-__global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= (SUMS ? 3 : 4) ? 3 : 2))) layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
+// Rows in flight per warp of the backward kernel beside the one in its registers, through shared memory by cp.async (see LaneRing; here the
+// K = vectors of x, dy and the shortcut's gradient that a lane has of a row).
+__host__ __device__ constexpr int ln_bwd_ahead(int vpl) { return vpl <= 4 ? 3 : 2; }
+
+// RES: dres is added. SUMS: dsum += the column sums of dres as well, which passes through here anyway (the bias gradient of the layer before the
+// shortcut).
+template <int LPR, int VPL, bool EXACT, bool RES, bool SUMS>
+__global__ void __launch_bounds__(128, VPL == 1 ? 5 : (VPL == 2 ? 4 : (VPL <= 4 ? 3 : 2))) layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                             const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ gamma,
                                                             const float* __restrict__ mean, const float* __restrict__ rstd,
                                                             __nv_bfloat16* __restrict__ dx, float* __restrict__ dgamma,
                                                             float* __restrict__ dbeta, const __nv_bfloat16* __restrict__ dres,
                                                             long long rows, int C, float* __restrict__ dsum) {
+  static_assert(RES || !SUMS, "the sums are of dres");
   chain_begin();
-  constexpr int RPW = 32 / LPR;
+  constexpr int RPW = 32 / LPR, K = (RES ? 3 : 2) * VPL, S = ln_bwd_ahead(VPL);
+  extern __shared__ __align__(16) float sh[];   // the lanes' rows in flight, then [warp][2 or 3][C] sums
   const int lane = threadIdx.x & 31, sub = lane % LPR;
   const int nvec = EXACT ? LPR * VPL : C >> 3;
   const long long step = static_cast<long long>(gridDim.x) * (blockDim.x >> 5) * RPW;
-  float ag[VPL][8], ab[VPL][8];
+  // (two columns per instruction)
+  f32x2 ag[VPL][4], ab[VPL][4], as[SUMS ? VPL : 1][4];
 #pragma unroll
   for (int i = 0; i < VPL; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ag[i][j] = ab[i][j] = 0.f;
-  float as[SUMS ? VPL : 1][8] = {};
+    for (int j = 0; j < 4; ++j) {
+      ag[i][j] = ab[i][j] = f2_both(0.f);
+      if (SUMS) as[i][j] = f2_both(0.f);
+    }
   uint4 gq[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     const int vi = sub + i * LPR;
     if (EXACT || vi < nvec) gq[i] = reinterpret_cast<const uint4*>(gamma)[vi];
   }
-  for (long long base = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * RPW; base < rows;
-       base += step) {
-    const long long row = base + lane / LPR;
-    const bool live = RPW == 1 || row < rows;
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * C);
-    const uint4* dr = reinterpret_cast<const uint4*>(dy + row * C);
-    float mu = 0.f, rs = 0.f;
-    // all of the row's loads (x, dy and the residual-path gradient) are issued before the first use
-    uint4 xq[VPL], dq[VPL], rq[VPL];
+  const uint32_t ring = smem_u32(sh) + threadIdx.x * 16;
+  constexpr uint32_t SLOT = 128 * 16;
+  auto fetch = [&](int slot, long long row) {
+    if (row < rows) {
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int vi = sub + i * LPR;
-      xq[i] = dq[i] = rq[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (live && (EXACT || vi < nvec)) {
-        xq[i] = xr[vi];
-        dq[i] = dr[vi];
-        if (dres != nullptr) rq[i] = reinterpret_cast<const uint4*>(dres + row * C)[vi];
+      for (int i = 0; i < VPL; ++i) {
+        const int vi = sub + i * LPR;
+        if (!EXACT && vi >= nvec) break;
+        const __nv_bfloat16* from[3] = {x, dy, dres};
+#pragma unroll
+        for (int t = 0; t < (RES ? 3 : 2); ++t)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring + (slot * K + t * VPL + i) * SLOT), "l"(from[t] + row * C + vi * 8)
+                       : "memory");
       }
     }
-    if (live) {
-      mu = mean[row];
-      rs = rstd[row];
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto read = [&](int slot, int k) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(ring + (slot * K + k) * SLOT) : "memory");
+    return v;
+  };
+  const long long first = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * RPW;
+  int slot = 0;
+#pragma unroll
+  for (int u = 0; u < S; ++u) fetch(u, first + u * step + lane / LPR);
+  float mu_next = 0.f, rs_next = 0.f;
+  if (first + lane / LPR < rows) {
+    mu_next = mean[first + lane / LPR];
+    rs_next = rstd[first + lane / LPR];
+  }
+#pragma unroll 1
+  for (long long base = first; base < rows; base += step) {
+    const long long row = base + lane / LPR;
+    const bool live = RPW == 1 || row < rows;
+    const float mu = mu_next, rs = rs_next;
+    if (row + step < rows) {
+      mu_next = mean[row + step];
+      rs_next = rstd[row + step];
     }
-    float s1 = 0.f, s2 = 0.f;
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 1) : "memory");
+    const f32x2 nmu = f2_both(-mu), rs2 = f2_both(rs);
+    f32x2 t1 = f2_both(0.f), t2 = f2_both(0.f);
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-      if (EXACT || sub + i * LPR < nvec) {
-        float xv[8], dyv[8], g[8];
-        unpack8(xq[i], xv);
-        unpack8(dq[i], dyv);
-        unpack8(gq[i], g);
+      if (live && (EXACT || sub + i * LPR < nvec)) {
+        const uint4 xq = read(slot, i), dq = read(slot, VPL + i);
+        const uint32_t x4[4] = {xq.x, xq.y, xq.z, xq.w}, d4[4] = {dq.x, dq.y, dq.z, dq.w}, g4[4] = {gq[i].x, gq[i].y, gq[i].z, gq[i].w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh = (xv[j] - mu) * rs;
-          ag[i][j] += dyv[j] * xh;
-          ab[i][j] += dyv[j];
-          const float dv = dyv[j] * g[j];
-          s1 += dv;
-          s2 += dv * xh;
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 xh = f2_mul(f2_add(f2_of_bf16x2(x4[j]), nmu), rs2), d = f2_of_bf16x2(d4[j]), dv = f2_mul(d, f2_of_bf16x2(g4[j]));
+          ag[i][j] = f2_fma(d, xh, ag[i][j]);
+          ab[i][j] = f2_add(ab[i][j], d);
+          t1 = f2_add(t1, dv);
+          t2 = f2_fma(dv, xh, t2);
         }
       }
     }
-    s1 = group_sum<LPR>(s1) / C;
-    s2 = group_sum<LPR>(s2) / C;
+    float s1, s2, odd1, odd2;
+    f2_unpack(t1, s1, odd1);
+    f2_unpack(t2, s2, odd2);
+    s1 = group_sum<LPR>(s1 + odd1) / C;
+    s2 = group_sum<LPR>(s2 + odd2) / C;
     if (live) {
       uint4* or_ = reinterpret_cast<uint4*>(dx + row * C);
+      const f32x2 n1 = f2_both(-s1), n2 = f2_both(-s2);
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
         const int vi = sub + i * LPR;
         if (EXACT || vi < nvec) {
-          // (recomputed from the packed operands: keeping x-hat and dy * gamma would cost 16 registers per vector)
-          float xv[8], dyv[8], g[8], rr[8], o[8];
-          unpack8(xq[i], xv);
-          unpack8(dq[i], dyv);
-          unpack8(gq[i], g);
-          unpack8(rq[i], rr);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xh = (xv[j] - mu) * rs;
-            o[j] = rs * (dyv[j] * g[j] - s1 - xh * s2);
+          // (read again: held in registers the operands would spill, or take a block's place)
+          const uint4 xq = read(slot, i), dq = read(slot, VPL + i);
+          const uint32_t x4[4] = {xq.x, xq.y, xq.z, xq.w}, d4[4] = {dq.x, dq.y, dq.z, dq.w}, g4[4] = {gq[i].x, gq[i].y, gq[i].z, gq[i].w};
+          uint32_t r4[4] = {}, o[4];
+          if constexpr (RES) {
+            const uint4 rq = read(slot, 2 * VPL + i);
+            r4[0] = rq.x, r4[1] = rq.y, r4[2] = rq.z, r4[3] = rq.w;
           }
-          if (dres != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += rr[j];
+          for (int j = 0; j < 4; ++j) {
+            const f32x2 xh = f2_mul(f2_add(f2_of_bf16x2(x4[j]), nmu), rs2), dv = f2_mul(f2_of_bf16x2(d4[j]), f2_of_bf16x2(g4[j]));
+            f32x2 v = f2_mul(rs2, f2_fma(xh, n2, f2_add(dv, n1)));
+            if constexpr (RES) {
+              const f32x2 r = f2_of_bf16x2(r4[j]);
+              v = f2_add(v, r);
+              if constexpr (SUMS) as[i][j] = f2_add(as[i][j], r);
+            }
+            o[j] = f2_to_bf16x2(v);
           }
-          if constexpr (SUMS) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) as[i][j] += rr[j];
-          }
-          or_[vi] = pack8(o);
+          or_[vi] = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
     }
+    fetch(slot, row + S * step);
+    slot = slot + 1 == S ? 0 : slot + 1;
   }
-  // the warp's row groups first (lanes sub, sub + LPR, ... hold the same columns), then the block's warps through shared
-  // memory, then one atomic per column
-  extern __shared__ float sh[];   // [2 or 3][C]
-  for (int c = threadIdx.x; c < (SUMS ? 3 : 2) * C; c += blockDim.x) sh[c] = 0.f;
+  // the warp's row groups first (lanes sub, sub + LPR, ... hold the same columns), then the block's warps through shared memory where the rows
+  // were, then one vector reduction per four columns: the blocks' ends meet on the same addresses, and take turns there
+  constexpr int SETS = SUMS ? 3 : 2;
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     const int vi = sub + i * LPR;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if constexpr (SUMS) {
+    for (int j = 0; j < 4; ++j) {
+      auto fold = [&](f32x2 v, int set) {
+        float e0, e1;
+        f2_unpack(v, e0, e1);
 #pragma unroll
-        for (int o = LPR; o < 32; o <<= 1) as[i][j] += __shfl_xor_sync(0xffffffffu, as[i][j], o);
-        if (lane < LPR && (EXACT || vi < nvec)) atomicAdd(&sh[2 * C + vi * 8 + j], as[i][j]);
-      }
-#pragma unroll
-      for (int o = LPR; o < 32; o <<= 1) {
-        ag[i][j] += __shfl_xor_sync(0xffffffffu, ag[i][j], o);
-        ab[i][j] += __shfl_xor_sync(0xffffffffu, ab[i][j], o);
-      }
-      if (lane < LPR && (EXACT || vi < nvec)) {
-        atomicAdd(&sh[vi * 8 + j], ag[i][j]);
-        atomicAdd(&sh[C + vi * 8 + j], ab[i][j]);
-      }
+        for (int o = LPR; o < 32; o <<= 1) {
+          e0 += __shfl_xor_sync(0xffffffffu, e0, o);
+          e1 += __shfl_xor_sync(0xffffffffu, e1, o);
+        }
+        if (lane < LPR && (EXACT || vi < nvec))
+          *reinterpret_cast<float2*>(sh + ((threadIdx.x >> 5) * SETS + set) * C + vi * 8 + 2 * j) = make_float2(e0, e1);
+      };
+      fold(ag[i][j], 0);
+      fold(ab[i][j], 1);
+      if constexpr (SUMS) fold(as[i][j], 2);
     }
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    atomicAdd(&dgamma[c], sh[c]);
-    atomicAdd(&dbeta[c], sh[C + c]);
-    if constexpr (SUMS) atomicAdd(&dsum[c], sh[2 * C + c]);
-  }
+  float* const out[3] = {dgamma, dbeta, dsum};
+#pragma unroll
+  for (int set = 0; set < SETS; ++set)
+    for (int c = threadIdx.x * 4; c < C; c += blockDim.x * 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float4 t = *reinterpret_cast<const float4*>(sh + (w * SETS + set) * C + c);
+        v.x += t.x, v.y += t.y, v.z += t.z, v.w += t.w;
+      }
+      add4(out[set] + c, v);
+    }
 }
 
 // ------------------------------------------------------------------------------------------ column sums
@@ -362,11 +420,13 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 // ------------------------------------------------------------------------------------------ GroupNorm
 // x: [B, HW, C] bf16. Every kernel is one pass over the image, bound by HBM: a block is (column vectors) x (pixels in
 // flight), so a thread's column constants (statistics, affine parameters) are loaded once for all of its pixels, and it
-// keeps several independent 16-byte loads in flight. blockIdx.y is the sample; the pixel range of a sample is split over
+// keeps several independent 16-byte loads in flight (LaneRing). blockIdx.y is the sample; the pixel range of a sample is split over
 // blockIdx.x so that the grid is about one resident wave. (Before, the apply kernels divided to find every vector's channel
 // and loaded its constants again, and one load per thread was in flight. 557056 pixels x 384, before -> now: statistics
 // 98 -> 90 us, apply with shortcut 355 -> 225, backward sums 366 -> 258, backward apply 406 -> 264; one copy of the image
-// each way at 6.65 TB/s is 129 us.)
+// each way at 6.65 TB/s is 129 us. Then, loads in registers -> in shared memory: apply 228 -> 212 with the shortcut and 190 -> 143 without, backward sums 192 -> 160,
+// backward apply 264 -> 199; 17280 x 192, with one wave of blocks for images that stay in L2: 6.4 -> 4.9, 6.0 -> 4.7, 8.6 -> 8.3, 7.3 -> 6.3, statistics
+// 5.0 -> 4.2.)
 //
 // Adds a thread's 16 sums (s, q of its eight channels) over the block's threadIdx.y and leaves them in sh[c] and sh[C + c]. Every thread of
 // the block takes part. Through a buffer of the block's own rather than by shared-memory atomics, which
@@ -409,7 +469,7 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
                                                               int pix_per_block, float* __restrict__ stats, unsigned int* __restrict__ ticket,
                                                               float inv_count, float eps) {
   chain_begin();
-  extern __shared__ float sh[];  // [2][C], then the threads' sums
+  extern __shared__ __align__(16) float sh[];  // [2][C], then the threads' sums
   const int nvec = C >> 3;
   const int b = blockIdx.y;
   const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
@@ -446,14 +506,23 @@ __global__ void __launch_bounds__(512) groupnorm_stats_kernel(const __nv_bfloat1
     gn_block_sums(sh, sh + 2 * C, s, q, C, vi);
   }
   const int cpg = C / groups, tid = threadIdx.y * blockDim.x + threadIdx.x;
-  for (int g = tid; g < groups; g += blockDim.x * blockDim.y) {
-    float s = 0.f, q = 0.f;
-    for (int c = g * cpg; c < (g + 1) * cpg; ++c) {
-      s += sh[c];
-      q += sh[C + c];
+  for (int g = 2 * tid; g < groups; g += 2 * blockDim.x * blockDim.y) {      // two groups: their four sums lie side by side
+    const bool two = g + 1 < groups;
+    float s[2] = {0.f, 0.f}, q[2] = {0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (k == 0 || two)
+        for (int c = (g + k) * cpg; c < (g + k + 1) * cpg; ++c) {
+          s[k] += sh[c];
+          q[k] += sh[C + c];
+        }
+    float* to = sums + (b * groups + g) * 2;
+    if (two) {
+      add4(to, make_float4(s[0], q[0], s[1], q[1]));
+    } else {
+      atomicAdd(to, s[0]);
+      atomicAdd(to + 1, q[0]);
     }
-    atomicAdd(&sums[(b * groups + g) * 2 + 0], s);
-    atomicAdd(&sums[(b * groups + g) * 2 + 1], q);
   }
   if (stats == nullptr) return;
   __shared__ bool last;
@@ -485,10 +554,6 @@ __device__ __forceinline__ void gn_pairs(GnPair (&c)[4], const float* __restrict
   const uint32_t g4[4] = {gq.x, gq.y, gq.z, gq.w}, b4[4] = {bq.x, bq.y, bq.z, bq.w};
 #pragma unroll
   for (int j = 0; j < 4; ++j) c[j] = gn_pair(stats, g4[j], b4[j], b, vi * 8 + 2 * j, cpg, groups);
-}
-__device__ __forceinline__ f32x2 f2_of_bf16x2(uint32_t v) {
-  const float2 f = unpack_bf16x2(v);
-  return f2_pack(f.x, f.y);
 }
 // 1 / (1 + exp(-z)), two elements per instruction
 __device__ __forceinline__ f32x2 f2_sigmoid(f32x2 z) {
@@ -556,16 +621,15 @@ __device__ __forceinline__ f32x2 gn_dz(const GnPair& c, f32x2 x, f32x2 dy, f32x2
   return f2_mul(f2_mul(dy, sg), f2_fma(z, f2_fma(sg, f2_both(-1.f), f2_both(1.f)), f2_both(1.f)));
 }
 
-// pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}. Bound by issue and the latency of its loads beside HBM: two channels per instruction,
-// no shared-memory atomics, eight loads in flight per thread of two blocks (us, before / these two / eight loads: 557056 pixels x 384 257 / 244 /
-// 193, 139264 x 384 - / 68 / 54, 64800 x 192 - / 19 / 15, 17280 x 192 17.4 / - / 8.3; with three blocks the registers do not reach: 236).
-// Statistics of 17280 x 192: 10.1 and 1.4 for a launch that finished them / 7.1.
+// pass 1 of the backward: red[b][c] = {sum dz, sum dz * xhat}. Bound by issue and the special functions beside HBM: two channels per instruction,
+// no shared-memory atomics, one block of 16 warps (us, 557056 pixels x 384: two blocks of 8 warps with eight loads in registers 192, three with
+// the ring and one pixel at a time 168, this 160; HBM alone 131).
 __global__ void __launch_bounds__(512, 1) groupnorm_silu_bwd_reduce_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
     const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta, float* __restrict__ red,
     long long HW, int C, int groups, int pix_per_block, float* __restrict__ dgamma, float* __restrict__ dbeta) {
   chain_begin();
-  extern __shared__ float sh[];  // [2][C], then the threads' sums
+  extern __shared__ __align__(16) float sh[];  // [2][C], then the threads' sums
   const int nvec = C >> 3;
   const int b = blockIdx.y;
   const long long p0 = static_cast<long long>(blockIdx.x) * pix_per_block;
@@ -614,12 +678,15 @@ __global__ void __launch_bounds__(512, 1) groupnorm_silu_bwd_reduce_kernel(
     }
     gn_block_sums(sh, sh + 2 * C, s, q, C, vi);
   }
-  for (int c = threadIdx.y * blockDim.x + threadIdx.x; c < C; c += blockDim.x * blockDim.y) {
-    atomicAdd(&red[(static_cast<long long>(b) * C + c) * 2 + 0], sh[c]);
-    atomicAdd(&red[(static_cast<long long>(b) * C + c) * 2 + 1], sh[C + c]);
+  // (vector reductions: the blocks' ends meet on the same addresses)
+  for (int c = 4 * (threadIdx.y * blockDim.x + threadIdx.x); c < C; c += 4 * blockDim.x * blockDim.y) {
+    const float4 dz = *reinterpret_cast<const float4*>(sh + c), dzx = *reinterpret_cast<const float4*>(sh + C + c);
+    float* r = red + (static_cast<long long>(b) * C + c) * 2;
+    add4(r, make_float4(dz.x, dzx.x, dz.y, dzx.y));
+    add4(r + 4, make_float4(dz.z, dzx.z, dz.w, dzx.w));
     // the affine parameters' gradients are the same sums taken over the batch as well
-    if (dbeta != nullptr) atomicAdd(&dbeta[c], sh[c]);
-    if (dgamma != nullptr) atomicAdd(&dgamma[c], sh[C + c]);
+    if (dbeta != nullptr) add4(dbeta + c, dz);
+    if (dgamma != nullptr) add4(dgamma + c, dzx);
   }
 }
 
@@ -1095,23 +1162,23 @@ int grid_for(long long work_items, int block, int max_blocks = 148 * 16) {
 // CALL sees LPR, VPL and EXACT (see the LayerNorm kernels) for rows of NVEC 16-byte vectors. MANY: rows
 // enough that groups of 32 / LPR of them still make warps for every SM; below that a row per warp finishes sooner (shorter chains,
 // more warps).
-#define TB_LN_CASE(L, V, E, CALL) { constexpr int LPR = L; constexpr int VPL = V; constexpr bool EXACT = E; CALL; }
-#define TB_LN_DISPATCH(NVEC, MANY, CALL)                        \
+#define TB_LN_CASE(L, V, E, ...) { constexpr int LPR = L; constexpr int VPL = V; constexpr bool EXACT = E; __VA_ARGS__; }
+#define TB_LN_DISPATCH(NVEC, MANY, ...)                         \
   switch ((MANY) ? (NVEC) : 0) {                                               \
-    case 4: TB_LN_CASE(4, 1, true, CALL) break;                 \
-    case 8: TB_LN_CASE(8, 1, true, CALL) break;                 \
-    case 12: TB_LN_CASE(4, 3, true, CALL) break;                \
-    case 16: TB_LN_CASE(16, 1, true, CALL) break;               \
-    case 24: TB_LN_CASE(8, 3, true, CALL) break;                \
-    case 48: TB_LN_CASE(16, 3, true, CALL) break;               \
+    case 4: TB_LN_CASE(4, 1, true, __VA_ARGS__) break;                 \
+    case 8: TB_LN_CASE(8, 1, true, __VA_ARGS__) break;                 \
+    case 12: TB_LN_CASE(4, 3, true, __VA_ARGS__) break;                \
+    case 16: TB_LN_CASE(16, 1, true, __VA_ARGS__) break;               \
+    case 24: TB_LN_CASE(8, 3, true, __VA_ARGS__) break;                \
+    case 48: TB_LN_CASE(16, 3, true, __VA_ARGS__) break;               \
     default:                                                    \
       switch (((NVEC) + 31) / 32) {                             \
-        case 1: TB_LN_CASE(32, 1, false, CALL) break;           \
-        case 2: TB_LN_CASE(32, 2, false, CALL) break;           \
-        case 3: TB_LN_CASE(32, 3, false, CALL) break;           \
-        case 4: TB_LN_CASE(32, 4, false, CALL) break;           \
-        case 5: case 6: TB_LN_CASE(32, 6, false, CALL) break;   \
-        case 7: case 8: TB_LN_CASE(32, 8, false, CALL) break;   \
+        case 1: TB_LN_CASE(32, 1, false, __VA_ARGS__) break;           \
+        case 2: TB_LN_CASE(32, 2, false, __VA_ARGS__) break;           \
+        case 3: TB_LN_CASE(32, 3, false, __VA_ARGS__) break;           \
+        case 4: TB_LN_CASE(32, 4, false, __VA_ARGS__) break;           \
+        case 5: case 6: TB_LN_CASE(32, 6, false, __VA_ARGS__) break;   \
+        case 7: case 8: TB_LN_CASE(32, 8, false, __VA_ARGS__) break;   \
         default: return -1;                                     \
       }                                                         \
   }
@@ -1123,10 +1190,10 @@ constexpr int ln_fwd_blocks(int vpl) { return 148 * (vpl == 1 ? 6 : (vpl == 2 ? 
 // resident wave (139264 rows with shortcut, us, 2 / 3 / resident: C = 72 70 / 55 / 42, 256 116 / 87 / 62, 512 158 / 124 / 108; 4096 rows
 // of 256 7.5 / 9 / 15). Rows of five vectors per lane and more have room for two blocks; a third waits for both (2048 columns
 // 1186 / 1452).
-inline int ln_bwd_blocks(int vpl, bool exact, long long rows) {
+inline int ln_bwd_blocks(int vpl, long long rows) {
   if (vpl > 4) return 148 * 2;
   const bool many = rows >= 148LL * 3 * 4 * 32;       // 32 rows for every warp of three blocks per SM
-  return 148 * (many && vpl == 1 ? (exact ? 5 : 6) : (many && vpl == 2 ? 4 : 3));
+  return 148 * (many && vpl == 1 ? 5 : (many && vpl == 2 ? 4 : 3));
 }
 
 int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
@@ -1139,24 +1206,40 @@ int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, f
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+template <int LPR, int VPL, bool EXACT, bool RES, bool SUMS>
+static int ln_bwd_launch(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* gamma, const float* mean, const float* rstd,
+                         __nv_bfloat16* dx, float* dgamma, float* dbeta, const __nv_bfloat16* dres, long long rows, int C, float* dsum,
+                         cudaStream_t stream) {
+  const size_t bytes = std::max<size_t>(4 * (SUMS ? 3 : 2) * C * sizeof(float), static_cast<size_t>(RES ? 3 : 2) * VPL * ln_bwd_ahead(VPL) * 128 * 16);
+  auto kernel = layernorm_bwd_kernel<LPR, VPL, EXACT, RES, SUMS>;
+  static std::atomic<bool> configured{false};      // (more than the 48 KB that every launch may have)
+  if (bytes > 48 * 1024 && !configured.load(std::memory_order_relaxed)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess) return -3;
+    configured.store(true, std::memory_order_relaxed);
+  }
+  launch_chained(kernel, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, rows)), 128, bytes, stream, dy, x, gamma, mean, rstd, dx, dgamma,
+                 dbeta, dres, rows, C, dsum);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
 int layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
                   float* dgamma, float* dbeta, const void* dres, long long rows, int C, cudaStream_t stream, float* dres_sum) {
   if (C % 8 != 0 || C > 2048 || (dres_sum != nullptr && dres == nullptr)) return -1;
-  auto go = [&](auto kernel, int blocks, int rows_per_block, int sums) {
-    launch_chained(kernel, grid_for(rows, rows_per_block, blocks), 128, sums * C * sizeof(float), stream,
-                   static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), mean,
-                   rstd, static_cast<__nv_bfloat16*>(dx), dgamma, dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C, dres_sum);
+  auto go = [&](auto launch) {
+    return launch(static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), mean, rstd,
+                  static_cast<__nv_bfloat16*>(dx), dgamma, dbeta, static_cast<const __nv_bfloat16*>(dres), rows, C, dres_sum, stream);
   };
   if (dres_sum != nullptr) {
     // (of the widths that gain by it: bindings_halves.cpp, sums_beside_norm)
     if (C <= 512 || C > 1024) return -1;
-    if (C <= 768) go(layernorm_bwd_kernel<32, 3, false, true>, ln_bwd_blocks(3, false, rows), 4, 3);
-    else go(layernorm_bwd_kernel<32, 4, false, true>, ln_bwd_blocks(4, false, rows), 4, 3);
-  } else {
-    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8,
-                   go(layernorm_bwd_kernel<LPR, VPL, EXACT, false>, ln_bwd_blocks(VPL, EXACT, rows), 4 * (32 / LPR), 2));
+    return C <= 768 ? go(ln_bwd_launch<32, 3, false, true, true>) : go(ln_bwd_launch<32, 4, false, true, true>);
   }
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  if (dres != nullptr) {
+    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, return go(ln_bwd_launch<LPR, VPL, EXACT, true, false>));
+  } else {
+    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, return go(ln_bwd_launch<LPR, VPL, EXACT, false, false>));
+  }
+  return -1;
 }
 
 int colsum_rows_per_block() { return 256; }

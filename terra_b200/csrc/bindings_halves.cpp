@@ -101,7 +101,8 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 // Tile width, row blocks per tile and split of the contraction for N x K outputs over M rows: the plan of least time by a model, in us. Rounds of
 // tiles over the CTAs (or pairs: request 1000 + width), each its k-blocks and a hand-over with the epilogue. A k-block costs less where fewer
 // CTAs than there are SMs share L2's bandwidth; the column sums (the bias gradient) are more MMAs, shared out over the column tiles. Widths of
-// 256 and transposed plans have no room for the sums' accumulators, or the wrong operand: there the sums are two launches that read dy once more.
+// 256 and transposed plans have no room for the sums' accumulators, or the wrong operand: there the sums are two launches that read dy once
+// more, or a row of ones behind x's columns where the last pair has room for it (557056 rows of 384 x 2976 1003 / 890 us).
 // Transposed: few outputs of a wide layer (patch embedding: 384 x 2976), 384 rows filling one and a half pairs, 384 columns one tile.
 //
 // Fitted to 9000 passes in CUDA graphs: 200 to 557056 rows, 22 pairs of N and K between 96 and 4096, with and without sums, all tiles, half a
@@ -126,6 +127,7 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   const int64_t blocks_256 = ((N + 127) / 128) * ((K + 255) / 256);
   const int64_t least_split = std::max<int64_t>(1, std::min((k_blocks + 31) / 32, sms / blocks_256));
   const double separate = sums ? 8.5 + 2e-6 * M * N / 4.71 : 0.0;
+  const bool ones_row = tb::gemm_row_sums_fit(K, 2);      // (of a transposed plan: the sums are a row of ones behind x's columns)
   const bool pairs = tb::gemm_pairs() && sms >= 2;
   struct Choice {
     WgradPlan plan;
@@ -150,7 +152,7 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
         const int64_t split = (k_blocks + per - 1) / per, rounds = (count * split + units - 1) / units;
         const double full = std::min(1.0, static_cast<double>(count * split) / units);
         const double time = rounds * (per * (t.kblock * (0.77 + 0.23 * full) + sum_cost) + t.tile) + (pair ? 1.3 : 0.0) +
-                            0.008 * 4e-6 * count * split * high * 128 * std::min<int64_t>(width, cols) + 3.4 + (fused ? 0.0 : separate);
+                            0.008 * 4e-6 * count * split * high * 128 * std::min<int64_t>(width, cols) + 3.4 + (fused || (swapped && ones_row) ? 0.0 : separate);
         choices.push_back({{t.request, t.stack, static_cast<int>(split), swapped}, time});
       }
     }
@@ -188,7 +190,9 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
     sums = false;
   }
   const WgradPlan plan = plan_wgrad(N, K, M, sums);
-  if (sums && (plan.bn % 1000 == 256 || plan.swapped)) {
+  const bool ones_row = sums && plan.swapped && tb::gemm_row_sums_fit(K, 2) && tb::gemm_tma_epilogue() && grad_w.stride(0) % 4 == 0 &&
+                        reinterpret_cast<uintptr_t>(grad_w.data_ptr()) % 16 == 0;
+  if (sums && !ones_row && (plan.bn % 1000 == 256 || plan.swapped)) {
     column_sums(dy, *grad_b);
     sums = false;
   }
@@ -200,7 +204,8 @@ void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTen
   g.ldc = grad_w.stride(0);
   g.alpha = 1.0f;
   g.status = status.data_ptr();
-  g.colsum = sums ? grad_b->data_ptr<float>() : nullptr;
+  g.colsum = sums && !ones_row ? grad_b->data_ptr<float>() : nullptr;
+  g.row_sums = ones_row ? grad_b->data_ptr<float>() : nullptr;
   g.stack = plan.stack;
   tb::note_launch();
   rc_check(tb::gemm_bf16(A, B, plan.swapped ? K : N, plan.swapped ? N : K, M, g, plan.split, plan.bn, sm_count(), cur_stream()),

@@ -218,6 +218,8 @@ void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, bool
   pick_tile((M + GEMM_BM - 1) / GEMM_BM, N, static_cast<int>((K + GEMM_BK - 1) / GEMM_BK), b_mn, flags, gathered, num_sms, bn, ctas);
 }
 
+bool gemm_row_sums_fit(long long rows, int blocks) { return (rows + 63) / 64 % (2 * blocks) != 0; }
+
 static void fill_epilogue(GemmParams& p, const GemmEpilogue& e) {
   p.epi = e.flags;
   p.C = e.C;
@@ -330,6 +332,15 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   p.tile_n1 = 1;
   try_tma_epilogue(p, M, N);
   try_tma_reduce(p, M, N, 1, 0);
+  if (epi.row_sums != nullptr) {
+    if (!gemm_row_sums_fit(M, ctas * (p.stack == 2 ? 2 : 1)) || p.epi_tma != 3 || !A.mn_major) return -21;
+    void* ones = nullptr;
+    if (gemm_ones_tile(&ones) != cudaSuccess) return -20;
+    rc = map_2d(&p.map_in, ones, 64, 64, 64, 64, 64);
+    if (rc != 0) return rc - 2000;
+    p.row_sums = epi.row_sums;
+    p.ones_row = static_cast<int>((M + 63) / 64 * 64);
+  }
   cudaError_t e = launch_gemm(p, bn, ctas, num_sms, stream);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
@@ -685,6 +696,7 @@ static int tap_wgrad(const void* a, const void* b, float* dw, int B, int Ho, int
   p.tap_boxes = (channels + 63) / 64;
   p.tap_channels = channels;
   p.row_sums = row_sums;
+  p.ones_row = ntaps * p.tap_boxes * 64;
   p.m_blocks = (ntaps * p.tap_boxes + (row_sums != nullptr ? 1 : 0) + 1) / 2;
   p.stack = plan.stack;
   p.num_m_tiles = (p.m_blocks + plan.stack * plan.ctas - 1) / (plan.stack * plan.ctas);

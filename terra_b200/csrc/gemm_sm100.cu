@@ -391,8 +391,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           } else if (p.a_mode == OP_MNMAJOR_2D) {
 #pragma unroll
             for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
-              if (STACK == 1 || j < blocks * (GEMM_BM / 64))
-                tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, kb * GEMM_BK);
+              if (STACK == 1 || j < blocks * (GEMM_BM / 64)) {
+                if (!PEERS && p.row_sums != nullptr && m0 + j * 64 == p.ones_row) tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_in, bar, 0, 0);
+                else tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, kb * GEMM_BK);
+              }
           } else if (p.a_mode == OP_TABLE_5D) {
             const short* e = p.ktable[kb];
             int h = abase[3] + e[3];
@@ -841,11 +843,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           if (STACK > 1 && tc.m_blk >= p.m_blocks) break;
           const int dcol = STACK > 1 ? mb : acc;
           int row = tc.m_blk * GEMM_BM + q * 32, group = tc.grp, rows = p.M;      // this warp's rows of the group (tap)
-          bool ones = false;
+          const bool ones = p.row_sums != nullptr && row == p.ones_row;
           if (p.tap_boxes > 0) {
             group = (row >> 6) / p.tap_boxes;
             row -= group * p.tap_boxes * 64;
-            ones = group == p.taps && row == 0 && p.row_sums != nullptr;
             if (group >= p.taps) rows = 0;
           }
           if (row < rows || ones) {
@@ -875,7 +876,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               }
               if (ones) {      // row 0: the column sums of B
                 __syncwarp();
-                if (cb + lane < p.N) atomicAdd(p.row_sums + cb + lane, *reinterpret_cast<const float*>(my_out + lane * 4));
+                const int at = (p.epi & EPI_TRANSPOSE) ? lane * 128 + ((lane & 7) << 4) : lane * 4;
+                if (cb + lane < p.N) atomicAdd(p.row_sums + cb + lane, *reinterpret_cast<const float*>(my_out + at));
                 continue;
               }
               fence_proxy_async_smem();
@@ -925,7 +927,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             return (lr < p.a_rows) ? static_cast<long long>(peer) * p.a_rows + lr : -1;
           } else if (!PEERS && p.tap_boxes > 0) {
             const int g = tc.m_blk * GEMM_BM + r, tap = (g >> 6) / p.tap_boxes, c = g - tap * p.tap_boxes * 64;
-            if (tap >= p.taps) return tap == p.taps && c == 0 ? -2 : -1;      // -2: the column sums of B
+            if (tap >= p.taps) return g == p.ones_row ? -2 : -1;      // -2: the column sums of B
             return c < p.tap_channels ? static_cast<long long>(tap) * p.tap_channels + c : -1;
           } else {
             const long long g = static_cast<long long>(tc.m_blk) * GEMM_BM + r;

@@ -47,10 +47,12 @@ struct GemmParams {
   short grp_off[16][4];        // per group (tap): {parity, dw, dh, unused} applied to operand B, or A
   // Weight gradients of all taps as one product (tap_boxes > 0, groups = 1): the rows of A are tap_boxes boxes of 64 channels per tap, one
   // tap after the other, so that tiles of 128, 256 or a pair's 2 x 128 rows run on across taps; row (tap, channel) of the output is
-  // row tap * tap_channels + channel. Boxes behind the last tap are ones (map_in: a 64 x 64 tile of them); the first of these rows is
-  // then the column sums of B, accumulated into row_sums.
+  // row tap * tap_channels + channel. Boxes behind the last tap are ones (map_in: a 64 x 64 tile of them).
   int taps, tap_boxes, tap_channels;
+  // Weight gradients: with row_sums, the box of A from row ones_row on (behind its own) is ones, and the first of these rows, the column sums of
+  // B, is accumulated into row_sums.
   float* row_sums;
+  int ones_row;
   int disp_a;                  // the displaced image is operand A (and the column sums add up over the groups)
   long long grp_c_stride;      // output offset (elements) between groups
   // epilogue

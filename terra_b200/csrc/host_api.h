@@ -40,6 +40,7 @@ struct GemmEpilogue {
   // contraction (sum over tokens of dy[token][n], the bias gradient) into colsum[n] (fp32), from an extra
   // 16-column MMA against a tile of ones. Null: off. Tile widths up to 192.
   float* colsum;
+  float* row_sums;    // weight-gradient form, output stored by TMA reductions: += the column sums of B, as a row of ones in A (gemm_row_sums_fit)
   int stack;          // weight-gradient form: 2 = tiles of two 128-row blocks that share a tile of B (widths 128, 192; 256 without colsum)
 };
 
@@ -76,6 +77,8 @@ int gemm_bf16(const GemmOperand& A, const GemmOperand& B, long long M, long long
 // tile of 128 rows each (2: a CTA pair). `gathered`: of a convolution with M / 128 row tiles and K / 64 taps x channel chunks.
 bool gemm_pairs();   // CTA pairs are allowed (TERRA_GEMM_2CTA)
 void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, bool gathered, int num_sms, int* bn, int* ctas);
+// whether tiles of `blocks` 128-row blocks leave room for a row of ones behind `rows` rows (GemmEpilogue::row_sums)
+bool gemm_row_sums_fit(long long rows, int blocks);
 bool gemm_tma_epilogue();   // whether the epilogue may go through TMA (environment switch)
 int gemm_stall_counters(unsigned long long* out8, int reset);
 

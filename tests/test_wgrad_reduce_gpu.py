@@ -28,3 +28,22 @@ def test_forms(bn, M, N, K, split, offset, extra, turned):
     want = 0.5 * dy.double().t() @ x.double()
     assert ((out - 1).double() - want).norm() <= 1e-5 * want.norm()
     assert (wide[:, :offset] == 1).all() and (wide[:, offset + K:] == 1).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(60001, 384, 2976), (40000, 376, 2208), (50000, 264, 1096), (450001, 384, 2304)])      # the last: no room behind 36 boxes
+@pytest.mark.parametrize("offset", [0, 2])      # 2: a gradient without a tensor map
+def test_bias_sums_as_a_row_of_ones(M, N, K, offset):
+    """Transposed weight gradients with the bias gradient in the rows that the last pair has to spare, or apart. Sums of 1e4 values: 1e-4."""
+    from terra_b200 import _ext
+    from terra_b200.ops.blocks import wgrad_accumulate
+    from terra_b200.ops.gemm import check_status
+
+    assert _ext.load().wgrad_swapped(N, K, M, True)
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    dy, x = (torch.randn(M, c, generator=gen, device="cuda", dtype=torch.bfloat16) for c in (N, K))
+    wide, gb = torch.ones(N, K + 8, device="cuda"), torch.ones(N, device="cuda")
+    wgrad_accumulate(dy, x, wide[:, offset:offset + K], gb)
+    check_status("cuda")
+    want, sums = dy.double().t() @ x.double(), dy.double().sum(0)
+    assert ((wide[:, offset:offset + K] - 1).double() - want).norm() <= 1e-4 * want.norm() and (gb - 1 - sums).norm() <= 1e-4 * sums.norm()
+    assert (wide[:, :offset] == 1).all() and (wide[:, offset + K:] == 1).all()

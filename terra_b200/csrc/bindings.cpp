@@ -224,6 +224,44 @@ void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tens
   rc_check(rc, "convt2x2_wgrad");
 }
 
+static void check_patches(const Tensor& image, const Tensor& grid, int64_t p, int64_t top, int64_t left) {
+  check_image(image, "image");
+  check_image(grid, "patches");
+  TORCH_CHECK(image.numel() > 0 && image.size(0) == grid.size(0) && p >= 1 && p <= 4 && image.size(1) % p == 0 && image.size(2) % p == 0 && top >= 0 &&
+                  left >= 0 && top + image.size(1) / p <= grid.size(1) && left + image.size(2) / p <= grid.size(2) && p * image.size(3) % 8 == 0 &&
+                  grid.size(3) % 8 == 0 && p * ((p * image.size(3) + 63) / 64) <= 128 && (grid.size(3) + 63) / 64 <= 128,
+              "patches: an image of whole patches inside the grid");
+}
+
+// image [B, H, W, C] -> y [B, rows, cols, N]; w [N, p * (p * C padded to 64)], bias [N]; top and left in patches
+void embed_image(const Tensor& image, const Tensor& w, const Tensor& bias, Tensor& y, int64_t p, int64_t top, int64_t left, const OptTensor& status) {
+  check_patches(image, y, p, top, left);
+  check_packed(w, y.size(3), p, p * image.size(3));
+  TORCH_CHECK(bias.scalar_type() == torch::kBFloat16 && bias.is_contiguous() && bias.numel() == y.size(3), "embed_image: bias bf16 [N]");
+  const c10::cuda::CUDAGuard guard(image.device());
+  tb::note_launch();
+  rc_check(tb::embed_image_bf16(image.data_ptr(), w.data_ptr(), bias.data_ptr(), y.data_ptr(), image.size(0), image.size(1), image.size(2),
+                                image.size(3), p, top, left, y.size(1), y.size(2), y.size(3), status_ptr(status), sm_count(), cur_stream()),
+           "embed_image");
+}
+
+// out = image + the patches of t [B, rows, cols, D] inside it; w [p * (p * C padded to 64), D padded to 64], bias alike
+void recover_image(const Tensor& t, const Tensor& w, const Tensor& bias, const Tensor& image, Tensor& out, int64_t p, int64_t top, int64_t left,
+                   const OptTensor& status) {
+  check_patches(image, t, p, top, left);
+  check_image(out, "out");
+  const int64_t run = (p * image.size(3) + 63) / 64 * 64;
+  check_packed(w, p * run, 1, t.size(3));
+  TORCH_CHECK(out.sizes() == image.sizes() && bias.scalar_type() == torch::kBFloat16 && bias.is_contiguous() && bias.numel() == p * run,
+              "recover_image: out like the image, bias bf16, a run padded to 64 per image row");
+  const c10::cuda::CUDAGuard guard(image.device());
+  tb::note_launch();
+  rc_check(tb::recover_image_bf16(t.data_ptr(), w.data_ptr(), bias.data_ptr(), image.data_ptr(), out.data_ptr(), image.size(0), image.size(1),
+                                  image.size(2), image.size(3), p, top, left, t.size(1), t.size(2), t.size(3), status_ptr(status), sm_count(),
+                                  cur_stream()),
+           "recover_image");
+}
+
 static tb::TapPlan tap_plan(const TapPlanRequest& request, int taps, int64_t channels, int64_t N, int64_t k_blocks, bool row_sums, bool column_sums,
                             int64_t least_split) {
   if (!request.has_value())
@@ -332,6 +370,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("input"), py::arg("w"), py::arg("bias4"), py::arg("out"), py::arg("status"));
   m.def("convt2x2_wgrad", &convt2x2_wgrad, "2x2 / stride-2 transposed convolution: weight gradient (fp32 atomics)",
         py::arg("x"), py::arg("dy"), py::arg("dw"), py::arg("split_k"), py::arg("status"), py::arg("stack") = 1, py::arg("bias_grad") = py::none());
+  m.def("embed_image", &embed_image, "patch embedding that reads the image itself");
+  m.def("recover_image", &recover_image, "patch recovery that adds to the image itself");
   m.def("conv3x3_wgrad_taps", &conv3x3_wgrad_taps, "3x3 convolution: weight gradients of all taps as one product", py::arg("x"), py::arg("dy"),
         py::arg("dw"), py::arg("stride"), py::arg("status"), py::arg("bias_grad") = py::none(), py::arg("fuse_bias") = true,
         py::arg("least_split") = 1, py::arg("plan") = py::none());

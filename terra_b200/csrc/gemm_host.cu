@@ -401,7 +401,20 @@ struct GatherConv {
   int out_h, out_w, out_c, out_mul; // output image; out_w = columns of one parity
   int phase_cols;                   // > 0: phases side by side in N
   short out_off[4][2];
+  // other layouts of the input and of the output (and the residual, which lies like the output): dimensions {channels, parity or row of a
+  // patch, columns, rows, samples} with their strides in elements
+  const struct ImageLayout* in_layout;
+  const struct ImageLayout* out_layout;
 };
+struct ImageLayout {
+  unsigned long long dims[5], strides[4];
+};
+static int layout_map(CUtensorMap* out, const void* base, const ImageLayout& l, int box_w) {
+  unsigned long long str[4];
+  for (int i = 0; i < 4; ++i) str[i] = 2 * l.strides[i];
+  unsigned int box[5] = {64, 1, static_cast<unsigned int>(box_w), 1, 1};
+  return make_tensor_map_bf16(out, base, 5, l.dims, str, box);
+}
 
 static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms, cudaStream_t stream, const void* halo_lo,
                        const void* halo_hi) {
@@ -430,7 +443,7 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   }
   p.a_mode = OP_TABLE_5D;
   p.b_mode = OP_KMAJOR_2D;
-  int rc = image_map(&p.map_a, c.x, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
+  int rc = c.in_layout != nullptr ? layout_map(&p.map_a, c.x, *c.in_layout, GEMM_BM) : image_map(&p.map_a, c.x, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
   if (rc != 0) return rc;
   rc = map_2d(&p.map_b, c.w, p.K, c.N, p.K, GEMM_BK, bn == 384 ? 64 : bn / ctas);
   if (rc != 0) return rc - 1000;
@@ -459,7 +472,12 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   p.ldc = c.out_c;
   // (outputs that go to every second pixel have no per-lane form)
   const bool strided = c.out_mul != 1 || c.phase_cols != 0;
-  if (!(p.epi & ~(EPI_ROW_CONV | EPI_BIAS | EPI_BIAS_F32)) && (strided || gemm_tma_epilogue())) {
+  if (c.out_layout != nullptr) {
+    rc = layout_map(&p.map_c, c.y, *c.out_layout, 32);
+    if (rc == 0 && (p.epi & EPI_RESIDUAL)) rc = layout_map(&p.map_in, p.residual, *c.out_layout, 32);
+    if (rc != 0) return rc - 5000;
+    p.epi_tma = 2;
+  } else if (!(p.epi & ~(EPI_ROW_CONV | EPI_BIAS | EPI_BIAS_F32)) && (strided || gemm_tma_epilogue())) {
     // 32 pixels x 64 channels per store; rows and channels outside the image are clipped
     const unsigned long long C = static_cast<unsigned long long>(c.out_c), mul = static_cast<unsigned long long>(c.out_mul);
     const unsigned long long row = C * 2ull * mul * c.out_w;
@@ -540,6 +558,52 @@ int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, i
   const Tap taps[4] = {{0, 0, 0}, {1, 0, 0}, {0, 0, 1}, {1, 0, 1}};
   GatherConv c = {dy, B, 2 * H, 2 * W, Cout, 2, H, W, 2, taps, 4, 1, {0, 4}, w, Cin, dx, H, W, Cin, 1, 0, {}};
   GemmEpilogue epi = {};
+  epi.alpha = 1.0f;
+  epi.status = status;
+  return gather_conv(c, epi, num_sms, stream, nullptr, nullptr);
+}
+
+// Patches of an image [B, H, W, C] (top and left patches of zeros before it, rows x cols of them in all) times w: y [B, rows, cols, N]. A patch's
+// features are p runs of p * C neighbouring elements, one per image row, so that the products read the image itself: 32 bytes of k-block
+// padding per run instead of a copy of the field in patch order. w: [N, p * (p * C padded to 64)].
+// Us, 64800 patches of 16 x 138 features to 192 channels: copy and product 104 + 69, this 68.
+int embed_image_bf16(const void* x, const void* w, const void* bias, void* y, int B, int H, int W, int C, int p, int top, int left, int rows,
+                     int cols, int N, void* status, int num_sms, cudaStream_t stream) {
+  if (p < 1 || p > 4 || H % p != 0 || W % p != 0 || (p * C) % 8 != 0 || N % 8 != 0) return -13;
+  Tap taps[4];
+  for (int r = 0; r < p; ++r) taps[r] = {static_cast<short>(r), static_cast<short>(-left), static_cast<short>(-top)};
+  const unsigned long long run = static_cast<unsigned long long>(p) * C, line = static_cast<unsigned long long>(W) * C;
+  const ImageLayout in = {{run, static_cast<unsigned long long>(p), static_cast<unsigned long long>(W / p), static_cast<unsigned long long>(H / p),
+                           static_cast<unsigned long long>(B)},
+                          {line, run, line * p, line * H}};
+  GatherConv c = {x, B, H / p, W / p, static_cast<int>(run), 1, rows, cols, 1, taps, p, 1, {0, p}, w, N, y, rows, cols, N, 1, 0, {}, &in, nullptr};
+  GemmEpilogue epi = {};
+  epi.flags = EPI_BIAS;
+  epi.bias = bias;
+  epi.alpha = 1.0f;
+  epi.status = status;
+  return gather_conv(c, epi, num_sms, stream, nullptr, nullptr);
+}
+
+// The way back: t [B, rows, cols, D] times w, the patches inside the image [B, H, W, C] (top and left of them outside) plus the image x: out. The
+// p runs of a patch are phases side by side in N. w: [p * (p * C padded to 64), D padded to 64], bias alike.
+// Us, 64800 patches of 192 channels: product and copy with the sum 72 + 166, this 170 (floor of the fields 88; the epilogue with a residual takes
+// 3400 cycles a unit).
+int recover_image_bf16(const void* t, const void* w, const void* bias, const void* x, void* out, int B, int H, int W, int C, int p, int top,
+                       int left, int rows, int cols, int D, void* status, int num_sms, cudaStream_t stream) {
+  if (p < 1 || p > 4 || H % p != 0 || W % p != 0 || (p * C) % 8 != 0 || D % 8 != 0) return -13;
+  const Tap tap = {0, static_cast<short>(left), static_cast<short>(top)};
+  const unsigned long long run = static_cast<unsigned long long>(p) * C, line = static_cast<unsigned long long>(W) * C;
+  const int pad = (p * C + 63) / 64 * 64;
+  const ImageLayout image = {{run, static_cast<unsigned long long>(p), static_cast<unsigned long long>(W / p), static_cast<unsigned long long>(H / p),
+                              static_cast<unsigned long long>(B)},
+                             {line, run, line * p, line * H}};
+  GatherConv c = {t, B, rows, cols, D, 1, H / p, W / p, 1, &tap, 1, 1, {0, 1}, w, p * pad, out, H / p, W / p, p * C, 1, pad,
+                  {{0, 0}, {0, 1}, {0, 2}, {0, 3}}, nullptr, &image};
+  GemmEpilogue epi = {};
+  epi.flags = EPI_BIAS | EPI_RESIDUAL;
+  epi.bias = bias;
+  epi.residual = x;
   epi.alpha = 1.0f;
   epi.status = status;
   return gather_conv(c, epi, num_sms, stream, nullptr, nullptr);

@@ -211,6 +211,16 @@ struct PixelWalk {
   }
 };
 
+// A unit of 32 consecutive pixels of an image row (EPI_ROW_CONV): coordinates in the output image, and in an operand that lies like it.
+struct PixelUnit {
+  int c, par, w, h, b;
+};
+__device__ __forceinline__ PixelUnit pixel_unit(const GemmParams& p, int m_blk, int q, int col, int grp) {
+  const int phase = p.phase_cols > 0 ? col / p.phase_cols : grp;
+  return {p.phase_cols > 0 ? col - phase * p.phase_cols : col, p.out_off[phase][1], (m_blk % p.tile_n0) * GEMM_BM + q * 32,
+          (m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0], m_blk / (p.tile_n0 * p.tile_n1)};
+}
+
 // mbar_wait that adds the time spent to `waited`; a barrier that is complete costs one test and reads no clock.
 template <bool PAIR>
 __device__ __forceinline__ bool wait_counted(uint64_t* bar, uint32_t parity, volatile int* abort_flag, KernelStatus* st,
@@ -658,9 +668,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           int col, row;
           if (next_unit(load, col, row) && lane == 0) {
             mbar_expect_tx(my_in + buf, 2 * Cfg::EPI_BUF);
-            tma_load_2d(my_out + buf * 2 * Cfg::EPI_BUF, &p.map_in, my_in + buf, col, row);
+            if (p.epi_tma == 2) {
+              const PixelUnit u = pixel_unit(p, row >> 7, q, col, 0);
+              tma_load_5d(my_out + buf * 2 * Cfg::EPI_BUF, &p.map_in, smem_u32(my_in + buf), u.c, u.par, u.w, u.h, u.b);
+            } else {
+              tma_load_2d(my_out + buf * 2 * Cfg::EPI_BUF, &p.map_in, my_in + buf, col, row);
+            }
           }
-          if (next_unit(ahead, col, row) && lane == 0) tma_prefetch_l2_2d(&p.map_in, col, row);
+          if (next_unit(ahead, col, row) && lane == 0) {
+            if (p.epi_tma == 2) {
+              const PixelUnit u = pixel_unit(p, row >> 7, q, col, 0);
+              tma_prefetch_l2_5d(&p.map_in, u.c, u.par, u.w, u.h, u.b);
+            } else {
+              tma_prefetch_l2_2d(&p.map_in, col, row);
+            }
+          }
         };
         if (has_in) {
           int col, row;
@@ -787,13 +809,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             if (lane == 0) {
               const uint32_t src = smem_u32(my_out) + buf * 2 * Cfg::EPI_BUF;
               if (p.epi_tma == 2) {
-                // 32 consecutive pixels of an image row (decoded by this one lane)
-                const int phase = p.phase_cols > 0 ? nb0 / p.phase_cols : tc.grp;
-                const int w = (tc.m_blk % p.tile_n0) * GEMM_BM + q * 32;
-                const int h = (tc.m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0];
-                if (tc.m_blk < p.m_blocks && w < p.out_w && h < p.out_h)
-                  tma_store_5d(&p.map_c, src, p.phase_cols > 0 ? nb0 - phase * p.phase_cols : nb0, p.out_off[phase][1], w, h,
-                               tc.m_blk / (p.tile_n0 * p.tile_n1));
+                // (decoded by this one lane)
+                const PixelUnit o = pixel_unit(p, tc.m_blk, q, nb0, tc.grp);
+                if (tc.m_blk < p.m_blocks && o.w < p.out_w && o.h < p.out_h) tma_store_5d(&p.map_c, src, o.c, o.par, o.w, o.h, o.b);
               } else {
                 if (row0 < p.M) {
                   if (save_pre) tma_store_2d(&p.map_c2, src + 2 * Cfg::EPI_BUF, nb0, row0);

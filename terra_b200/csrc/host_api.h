@@ -96,6 +96,12 @@ int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, 
 int conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, int W, int Cin, int Cout, int stride,
                        int split_k, void* status, int num_sms, cudaStream_t stream, const void* halo_lo = nullptr,
                        const void* halo_hi = nullptr, float* bias_grad = nullptr, int stack = 1);   // bias_grad[Cout] += sums of dy
+// Linear layers between an image [B, H, W, C] and its p x p patches (rows x cols of them, top and left before the image's own):
+// y [B, rows, cols, N] from x, and out = x + the patches of t [B, rows, cols, D] inside the image. Packed weights: gemm_host.cu.
+int embed_image_bf16(const void* x, const void* w, const void* bias, void* y, int B, int H, int W, int C, int p, int top, int left, int rows,
+                     int cols, int N, void* status, int num_sms, cudaStream_t stream);
+int recover_image_bf16(const void* t, const void* w, const void* bias, const void* x, void* out, int B, int H, int W, int C, int p, int top,
+                       int left, int rows, int cols, int D, void* status, int num_sms, cudaStream_t stream);
 // Weight gradients of all taps as one product (one rank): tile width, CTAs per tile, row blocks per tile, split of the contraction.
 struct TapPlan {
   int bn, ctas, stack, split;

@@ -21,7 +21,7 @@ from ..global_env_config import ON_H200
 from ..memory.activation import activation_checkpoint, activation_config_for_sampling
 from ..ops import blocks as B
 from ..ops.conv import conv3x3, conv_transpose2x2, groupnorm_silu
-from ..ops.patch import pad_patchify, patch_kernels_apply, unpatchify_add
+from ..ops.patch import direct_patches_apply, embed_image, pad_patchify, patch_kernels_apply, recover_image, unpatchify_add
 from ..parallel.context import ParallelContext
 from ..profiler.memory_timeline import mark_memory_timeline
 from ..utils.padding import get_padded_shape
@@ -253,6 +253,9 @@ class SequentialHierarchicalSwin(_SwinBase):
         fits = (raw_h + top + bottom, raw_w + left + right) == tuple(self.padded_shape)
         if fits and patch_kernels_apply(xin, self.padded_shape):
             p = self.patch_size
+            if direct_patches_apply(xin, p, top, left, self.embedding_dim):
+                y = self._forward_image(xin, top, left)
+                return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y
             y = unpatchify_add(self._core(pad_patchify(xin, p, self.padded_shape, top, left), None), xin, p, top, left)
             return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y
         if self.need_padding:
@@ -263,6 +266,23 @@ class SequentialHierarchicalSwin(_SwinBase):
             y = y[:, top:top + raw_h, left:left + raw_w, :]
         y = y + x.to(y.dtype)
         return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y
+
+
+    def _forward_image(self, xin, top, left):
+        """``_core`` where nothing is kept for a backward pass (recomputation has no part in it): patch layers on the image itself."""
+        p = self.patch_size
+        mark_memory_timeline("sampling_down_enter", "none")
+        x = self._in_unit(self.patch_embed, lambda t: embed_image(t, self._embed_linear(), p, self.padded_shape, top, left), xin)
+        if self.has_sampling:
+            x = self._down_block(x)
+        mark_memory_timeline("sampling_down_exit", "none")
+        x = self.pctx.windows_to_stripe(self.layers(self.pctx.stripe_to_windows(x)), xin.shape[0])
+        mark_memory_timeline("sampling_up_enter", "none")
+        if self.has_sampling:
+            x = self._up_block(x)
+        y = self._in_unit(self.patch_recovery, lambda t, r: recover_image(t, self._recovery_linear(), r, p, top, left), x, xin)
+        mark_memory_timeline("sampling_up_exit", "none")
+        return y
 
 
 class SequentialSwinReference(SequentialHierarchicalSwin):

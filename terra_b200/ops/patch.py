@@ -1,12 +1,16 @@
 """Padding and patch rearrangement of the sequential builds on CUDA: image [B, H, W, C] to patches [B, h, w, p*p*C] (feature
 order p1, p2, c) and back, one copy kernel each way where ``pad`` + ``permute`` + ``reshape`` (+ crop + add) took four passes
-over the field. The reference pads and rearranges with tensor operators (models/reference_model/
-sequential_hierarchical_swin.py:25-449)."""
+over the field; in inference, where whole patches lie inside the image, the patch layers read and write it themselves. The
+reference pads and rearranges with tensor operators (models/reference_model/sequential_hierarchical_swin.py:25-449)."""
 from __future__ import annotations
 
 import torch
 
 from .. import _ext
+from . import blocks
+from .conv import _pack_taps
+from .gemm import status_word
+from .packed import _packed
 
 MAX_ROWS = 65535        # batch x padded rows of one launch
 
@@ -62,3 +66,45 @@ def pad_patchify(x, p, padded_shape, top, left):
 def unpatchify_add(patches, x, p, top, left):
     """The image inside ``patches``, plus ``x``."""
     return _UnpatchifyAddFn.apply(patches.contiguous(), x, p, top, left)
+
+
+# ------------------------------------------------------------------------------------------------ without the copies (inference)
+def direct_patches_apply(x: torch.Tensor, p, top, left, dim) -> bool:
+    """Whether the patch layers may read and write the field ``x`` itself, in a call that keeps nothing for a backward pass: whole patches
+    inside the image and outside it, runs of whole 16-byte vectors, the product's tables and phases."""
+    _, H, W, C = x.shape
+    return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0 and blocks.native_node()
+            and 1 <= p <= 4 and H % p == W % p == top % p == left % p == 0 and p * C % 8 == 0 and dim % 8 == 0
+            and p * ((p * C + 63) // 64) <= 128 and (dim + 63) // 64 <= 128 and _ext.load().gemm_tma_epilogue())
+
+
+def _pack_embed(w, p):
+    run = w.shape[1] // p
+    return _pack_taps(w, 1, 0, w.shape[0], w.shape[1], run, 1, [r * run for r in range(p)])
+
+
+def _pack_recover(w, p):
+    run, dim = w.shape[0] // p, w.shape[1]
+    return _pack_taps(w, p, run * dim, run, dim, dim, 1, (0,), (run + 63) // 64 * 64)
+
+
+def _pack_recover_bias(b, p):
+    run = b.shape[0] // p
+    return torch.nn.functional.pad(b.view(p, run), (0, -run % 64)).reshape(-1)
+
+
+def embed_image(x, lin, p, padded_shape, top, left):
+    """``linear(pad_patchify(x))`` for ``direct_patches_apply`` fields: ``[B, rows, cols, N]``."""
+    w16, y = lin.weight.bf16, torch.empty(x.shape[0], padded_shape[0] // p, padded_shape[1] // p, lin.weight.shape[0], device=x.device, dtype=x.dtype)
+    _ext.load().embed_image(x, _packed(lin.weight, w16, f"embed{p}", lambda w: _pack_embed(w, p)), lin.bias.bf16, y, p, top // p, left // p,
+                            status_word(x.device))
+    return y
+
+
+def recover_image(t, lin, x, p, top, left):
+    """``unpatchify_add(linear(t), x)`` for ``direct_patches_apply`` fields; the sum is rounded once."""
+    out = torch.empty_like(x)
+    w = _packed(lin.weight, lin.weight.bf16, f"recover{p}", lambda v: _pack_recover(v, p))
+    b = _packed(lin.bias, lin.bias.bf16, f"recover{p}", lambda v: _pack_recover_bias(v, p))
+    _ext.load().recover_image(t.contiguous(), w, b, x, out, p, top // p, left // p, status_word(x.device))
+    return out

@@ -621,39 +621,26 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       //
       // What bounds a unit is latency, three warps per scheduler being all there is to hide it. So the form of the epilogue is a
       // compile-time constant (with the flags tested inside, every pair of elements became a basic block of its own), a unit's
-      // two tensor-memory loads are issued together, the bias of a unit is fetched while the accumulator is waited for and spread
-      // through shared memory once, and the input unit arrives in the buffer its output is staged in: a lane reads and writes
-      // the same 16 bytes. With two such buffers the next unit's load has this unit's processing time to arrive (and the one
-      // after it is already on its way from HBM to L2); with one (long contractions, which want the ring and hide the epilogue)
-      // it is issued when the store has read the buffer.
+      // two tensor-memory loads are issued together, the bias of a unit is spread through shared memory once, and the input unit arrives in the buffer its output is staged in: a lane reads and writes
+      // the same 16 bytes. With two such buffers the next unit's load has this unit's processing time to arrive; with one (long contractions,
+      // which want the ring and hide the epilogue) it is on its way from HBM to L2 meanwhile and issued when the store has read the buffer.
       // The first buffer (4 KB) stages the output; the second takes the saved pre-activation, or alternates with the first.
       // Cycles per unit with the flags tested inside: bias 2400 (now under 1300), bias and residual 3400 + 800 waiting for the input, GELU
       // with the pre-activation 4500, times GELU' 6100 + 800. Launches, before / now: 139264 x 1536 x 384 times GELU' 334 -> 261 us, the same with GELU 260
       // -> 243, 139264 x 384 x 384 63 -> 54, 156672 x 1024 x 1024 with residual 316 -> 279, 17280 x 576 x 192 12.4 -> 10.0.
+      // Where the epilogue bounds the launch no wait for a tile hides a latency, so the next unit's bias is loaded and its input asked for before this one is
+      // worked on, at coordinates that the walk over the tiles has anyway (two walks of units of their own took about 500 cycles a unit, a bias
+      // loaded with its tile 600): times GELU' 254 -> 217 us and 139264 x 2976 x 384 503 -> 440, with residual 388 -> 375 and x 2208 x 192 366 -> 277.
       constexpr int UNITS = BN / 64, WARPS_PER_Q = GEMM_EPI_WARPS / 4;
       uint8_t* my_out = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
       uint64_t* my_in = in_bar + 2 * (warp - 2);
       const uint32_t out_base = smem_u32(my_out) + static_cast<uint32_t>(lane) * 128u;
       const uint32_t swz = (static_cast<uint32_t>(lane) & 7u) << 4;
       const uint32_t bias_base = smem_u32(my_bias);
-      // coordinates of this warp's units, in the order it works on them
-      struct Units {
-        Walk walk;
-        int u;
-      };
-      auto next_unit = [&](Units& w, int& col, int& row) -> bool {
-        while (part < UNITS && w.walk.tile < total_tiles) {
-          col = w.walk.n * BN + w.u * 64;
-          row = w.walk.m_blk(rank) * GEMM_BM + q * 32;
-          const bool ok = col < p.N;
-          w.u += WARPS_PER_Q;
-          if (w.u >= UNITS) {
-            w.u = part;
-            w.walk.next(p);
-          }
-          if (ok) return true;
-        }
-        return false;
+      // column of this warp's first unit in the tile that a walk stands at, or -1
+      auto first_col = [&](const Walk& w) -> int {
+        const int col = w.n * BN + part * 64;
+        return part < UNITS && w.tile < total_tiles && col < p.N ? col : -1;
       };
 
       auto run = [&](auto form_const) __attribute__((always_inline)) {
@@ -662,53 +649,51 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         const bool with_bias = (flags & EPI_BIAS) != 0, gelu = (flags & EPI_GELU) != 0, save_pre = (flags & EPI_SAVE_PRE) != 0;
         const bool has_in = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0, dgelu = (flags & EPI_MUL_DGELU) != 0;
         const f32x2 alpha2 = f2_both(p.alpha);
+        // (GELU's chains are long enough to alternate between two runs of columns; the other forms lose by it: 139264 x 2976 x 384 with GELU 381 / 344 us,
+        // times GELU' 455 / 470)
+        constexpr int RUN = FORM >= 0 && (FORM & EPI_GELU) ? 2 : 1;
         const int in_bufs = p.epi_bufs / 2;
-        Units load = {Walk(p, unit, units), part}, ahead = load;
-        auto fetch_in = [&](int buf) {       // this warp's next input unit into `buf`; the unit after it into L2
-          int col, row;
-          if (next_unit(load, col, row) && lane == 0) {
-            mbar_expect_tx(my_in + buf, 2 * Cfg::EPI_BUF);
-            if (p.epi_tma == 2) {
-              const PixelUnit u = pixel_unit(p, row >> 7, q, col, 0);
-              tma_load_5d(my_out + buf * 2 * Cfg::EPI_BUF, &p.map_in, smem_u32(my_in + buf), u.c, u.par, u.w, u.h, u.b);
-            } else {
-              tma_load_2d(my_out + buf * 2 * Cfg::EPI_BUF, &p.map_in, my_in + buf, col, row);
-            }
+        auto bias_pair = [&](int col) -> float2 {     // columns col, col + 1 (col even)
+          float2 b = make_float2(0.f, 0.f);
+          if (p.epi & EPI_BIAS_F32) {
+            if (col < p.N) b.x = __ldg(static_cast<const float*>(p.bias) + col);
+            if (col + 1 < p.N) b.y = __ldg(static_cast<const float*>(p.bias) + col + 1);
+          } else {
+            if (col < p.N) b.x = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
+            if (col + 1 < p.N) b.y = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col + 1]);
           }
-          if (next_unit(ahead, col, row) && lane == 0) {
-            if (p.epi_tma == 2) {
-              const PixelUnit u = pixel_unit(p, row >> 7, q, col, 0);
-              tma_prefetch_l2_5d(&p.map_in, u.c, u.par, u.w, u.h, u.b);
-            } else {
-              tma_prefetch_l2_2d(&p.map_in, col, row);
-            }
+          return b;
+        };
+        // the input unit at column `col` of row block `m_blk` on its way into buffer `buf`, or (buf < 0) into L2; one lane
+        auto fetch_in = [&](int col, int m_blk, int buf) {
+          if (lane != 0) return;
+          uint8_t* const to = my_out + max(buf, 0) * 2 * Cfg::EPI_BUF;
+          if (buf >= 0) mbar_expect_tx(my_in + buf, 2 * Cfg::EPI_BUF);
+          if (p.epi_tma == 2) {
+            const PixelUnit u = pixel_unit(p, m_blk, q, col, 0);
+            if (buf >= 0) tma_load_5d(to, &p.map_in, smem_u32(my_in + buf), u.c, u.par, u.w, u.h, u.b);
+            else tma_prefetch_l2_5d(&p.map_in, u.c, u.par, u.w, u.h, u.b);
+          } else {
+            if (buf >= 0) tma_load_2d(to, &p.map_in, my_in + buf, col, m_blk * GEMM_BM + q * 32);
+            else tma_prefetch_l2_2d(&p.map_in, col, m_blk * GEMM_BM + q * 32);
           }
         };
-        if (has_in) {
-          int col, row;
-          next_unit(ahead, col, row);        // `ahead` runs one unit in front of `load`
-          fetch_in(0);
+        Walk walk(p, unit, units);
+        float2 bias_here = make_float2(0.f, 0.f);      // of the unit to come
+        {
+          const int col = first_col(walk);
+          if (with_bias && col >= 0) bias_here = bias_pair(col + 2 * lane);
+          if (has_in && col >= 0) fetch_in(col, walk.m_blk(rank), 0);
         }
         uint32_t count = 0;                  // units of this warp so far
         bool failed = false;
-        for (Walk walk(p, unit, units); walk.tile < total_tiles && !failed; walk.next(p), ++tcount) {
+        for (; walk.tile < total_tiles && !failed; ++tcount) {
           const TileCoord tc = walk.coord(p, rank, per_split);
+          Walk after = walk;
+          after.next(p);
           const int acc = tcount % Cfg::ACCS;
           const uint32_t aph = (tcount / Cfg::ACCS) & 1u;
           const int n0 = tc.n_blk * BN;
-          auto bias_pair = [&](int col) -> float2 {     // columns col, col + 1 (col even)
-            float2 b = make_float2(0.f, 0.f);
-            if (p.epi & EPI_BIAS_F32) {
-              if (col < p.N) b.x = __ldg(static_cast<const float*>(p.bias) + col);
-              if (col + 1 < p.N) b.y = __ldg(static_cast<const float*>(p.bias) + col + 1);
-            } else {
-              if (col < p.N) b.x = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
-              if (col + 1 < p.N) b.y = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col + 1]);
-            }
-            return b;
-          };
-          float2 bias_here = make_float2(0.f, 0.f);
-          if (with_bias && part < UNITS) bias_here = bias_pair(n0 + part * 64 + 2 * lane);
           const long long ew0 = clock64();
           const bool tile_ready = mbar_wait<PAIR>(&tfull[acc], aph, abort_flag, p.status, 0x400u + acc, mbar_budget);
           if (!__all_sync(0xffffffffu, tile_ready)) break;
@@ -733,10 +718,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             const uint32_t tcol = tmem_base + acc * BN + u * 64 + (static_cast<uint32_t>(q * 32) << 16);
             tmem_ld_32x32(tcol, v[0]);
             tmem_ld_32x32(tcol + 32, v[1]);
+            // the next unit's bias and input are asked for now: where the epilogue is what bounds the launch, nothing else hides their latency
+            const int next_col = last ? first_col(after) : nb0 + 64 * WARPS_PER_Q;
+            const int next_blk = last ? after.m_blk(rank) : tc.m_blk;
             if (with_bias) {
               __syncwarp();
               asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(bias_base + lane * 8), "f"(bias_here.x), "f"(bias_here.y) : "memory");
-              if (!last) bias_here = bias_pair(nb0 + 64 * WARPS_PER_Q + 2 * lane);
+              if (next_col >= 0) bias_here = bias_pair(next_col + 2 * lane);
             }
             if (has_in) {
               const bool in_ready = mbar_wait<false>(my_in + buf, (in_bufs == 2 ? count >> 1 : count) & 1u, abort_flag, p.status, 0x600u,
@@ -752,57 +740,70 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             if (last) release();
             if (lane == 0) bulk_wait_group_read<0>();     // the unit before has left its buffer
             __syncwarp();
-            if (has_in && in_bufs == 2) fetch_in(buf ^ 1);
+            if (has_in && next_col >= 0) fetch_in(next_col, next_blk, in_bufs == 2 ? buf ^ 1 : -1);
             const uint32_t row_out = out_base + buf * 2 * Cfg::EPI_BUF;
             const int row0 = tc.m_blk * GEMM_BM + q * 32;
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {      // 8 columns: 16 bytes of the output row
-              const uint32_t at = (static_cast<uint32_t>(g) << 4) ^ swz;
-              f32x2 f[4];
+            for (int g2 = 0; g2 < 8; g2 += RUN) {      // 8 columns (16 bytes of the output row) at a time, or twice 8
+              f32x2 f[RUN][4];
+              float bias[RUN][8];
+              uint32_t in[RUN][4];
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                f[k] = f2_pack(__uint_as_float(v[g >> 2][(g & 3) * 8 + 2 * k]), __uint_as_float(v[g >> 2][(g & 3) * 8 + 2 * k + 1]));
-              if (with_bias) {
+              for (int e = 0; e < RUN; ++e) {
+                const int g = g2 + e;
+                if (with_bias) {
 #pragma unroll
-                for (int k = 0; k < 4; k += 2) {
-                  float b0, b1, b2, b3;
-                  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                               : "=f"(b0), "=f"(b1), "=f"(b2), "=f"(b3)
-                               : "r"(bias_base + g * 32 + k * 8));
-                  f[k] = FORM >= 0 ? f2_add(f[k], f2_pack(b0, b1)) : f2_fma(f[k], alpha2, f2_pack(b0, b1));
-                  f[k + 1] = FORM >= 0 ? f2_add(f[k + 1], f2_pack(b2, b3)) : f2_fma(f[k + 1], alpha2, f2_pack(b2, b3));
+                  for (int k = 0; k < 8; k += 4)
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(bias[e][k]), "=f"(bias[e][k + 1]), "=f"(bias[e][k + 2]), "=f"(bias[e][k + 3])
+                                 : "r"(bias_base + g * 32 + k * 4));
                 }
-              } else if (FORM < 0) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) f[k] = f2_mul(f[k], alpha2);
+                if (has_in)
+                  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                               : "=r"(in[e][0]), "=r"(in[e][1]), "=r"(in[e][2]), "=r"(in[e][3])
+                               : "r"(row_out + ((static_cast<uint32_t>(g) << 4) ^ swz))
+                               : "memory");
               }
-              if (save_pre)
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_out + 2 * Cfg::EPI_BUF + at), "r"(f2_to_bf16x2(f[0])),
-                             "r"(f2_to_bf16x2(f[1])), "r"(f2_to_bf16x2(f[2])), "r"(f2_to_bf16x2(f[3]))
-                             : "memory");
-              if (gelu) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) f[k] = gelu_erf2(f[k]);
-              }
-              if (has_in) {
-                uint32_t in[4];
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(in[0]), "=r"(in[1]), "=r"(in[2]), "=r"(in[3])
-                             : "r"(row_out + at)
-                             : "memory");
+              for (int e = 0; e < RUN; ++e)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                  if (dgelu) {
-                    f[k] = f2_mul(f[k], gelu_erf_grad2_bf16(in[k]));
-                  } else {
-                    const float2 x = unpack_bf16x2(in[k]);
-                    f[k] = f2_add(f[k], f2_pack(x.x, x.y));
+                  const int at = ((g2 + e) & 3) * 8 + 2 * k;
+                  f32x2 x = f2_pack(__uint_as_float(v[g2 >> 2][at]), __uint_as_float(v[g2 >> 2][at + 1]));
+                  if (with_bias) {
+                    const f32x2 add = f2_pack(bias[e][2 * k], bias[e][2 * k + 1]);
+                    x = FORM >= 0 ? f2_add(x, add) : f2_fma(x, alpha2, add);
+                  } else if (FORM < 0) {
+                    x = f2_mul(x, alpha2);
+                  }
+                  f[e][k] = x;
+                }
+              if (save_pre) {
+#pragma unroll
+                for (int e = 0; e < RUN; ++e)
+                  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_out + 2 * Cfg::EPI_BUF + ((static_cast<uint32_t>(g2 + e) << 4) ^ swz)),
+                               "r"(f2_to_bf16x2(f[e][0])), "r"(f2_to_bf16x2(f[e][1])), "r"(f2_to_bf16x2(f[e][2])), "r"(f2_to_bf16x2(f[e][3]))
+                               : "memory");
+              }
+#pragma unroll
+              for (int e = 0; e < RUN; ++e)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  if (gelu) f[e][k] = gelu_erf2(f[e][k]);
+                  if (has_in) {
+                    if (dgelu) {
+                      f[e][k] = f2_mul(f[e][k], gelu_erf_grad2_bf16(in[e][k]));
+                    } else {
+                      const float2 r = unpack_bf16x2(in[e][k]);
+                      f[e][k] = f2_add(f[e][k], f2_pack(r.x, r.y));
+                    }
                   }
                 }
-              }
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_out + at), "r"(f2_to_bf16x2(f[0])), "r"(f2_to_bf16x2(f[1])),
-                           "r"(f2_to_bf16x2(f[2])), "r"(f2_to_bf16x2(f[3]))
-                           : "memory");
+#pragma unroll
+              for (int e = 0; e < RUN; ++e)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_out + ((static_cast<uint32_t>(g2 + e) << 4) ^ swz)),
+                             "r"(f2_to_bf16x2(f[e][0])), "r"(f2_to_bf16x2(f[e][1])), "r"(f2_to_bf16x2(f[e][2])), "r"(f2_to_bf16x2(f[e][3]))
+                             : "memory");
             }
             fence_proxy_async_smem();
             __syncwarp();
@@ -820,13 +821,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
               }
               bulk_commit_group();
             }
-            if (has_in && in_bufs == 1) {
+            if (has_in && in_bufs == 1 && next_col >= 0) {
               if (lane == 0) bulk_wait_group_read<0>();
               __syncwarp();
-              fetch_in(0);
+              fetch_in(next_col, next_blk, 0);
             }
           }
-          if (!released && !failed) release();   // a warp without a unit in this tile
+          if (!released && !failed) {   // a warp without a unit in this tile
+            release();
+            const int col = first_col(after);
+            if (with_bias && col >= 0) bias_here = bias_pair(col + 2 * lane);
+            if (has_in && col >= 0) {
+              if (lane == 0) bulk_wait_group_read<0>();
+              fetch_in(col, after.m_blk(rank), in_bufs == 2 ? static_cast<int>(count & 1u) : 0);
+            }
+          }
+          walk = after;
         }
         if (lane == 0) bulk_wait_group_read<0>();
       };

@@ -348,7 +348,7 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
 // 3x3 convolution, padding 1, stride 1 or 2, NHWC bf16, as implicit GEMM.
 //   x: [B, H, W, Cin]   w: [Cout, 9 * Cin_pad] (tap-major, Cin padded to a multiple of 64 with zeros)
 //   y: [B, Ho, Wo, Cout]
-static int image_map(CUtensorMap* out, const void* base, int Cin, int par, int W, int rows, int B, int box_w) {
+static int image_map(CUtensorMap* out, const void* base, int Cin, int par, int W, int rows, int B, int box_w, int box_h = 1) {
   unsigned long long dims[5] = {static_cast<unsigned long long>(Cin), static_cast<unsigned long long>(par),
                                 static_cast<unsigned long long>(W / par), static_cast<unsigned long long>(rows),
                                 static_cast<unsigned long long>(B)};
@@ -356,7 +356,7 @@ static int image_map(CUtensorMap* out, const void* base, int Cin, int par, int W
                                static_cast<unsigned long long>(Cin) * 2ull * par,
                                static_cast<unsigned long long>(Cin) * 2ull * W,
                                static_cast<unsigned long long>(Cin) * 2ull * W * rows};
-  unsigned int box[5] = {64, 1, static_cast<unsigned int>(box_w), 1, 1};
+  unsigned int box[5] = {64, 1, static_cast<unsigned int>(box_w), static_cast<unsigned int>(box_h), 1};
   return make_tensor_map_bf16(out, base, 5, dims, str, box);
 }
 
@@ -409,10 +409,10 @@ struct GatherConv {
 struct ImageLayout {
   unsigned long long dims[5], strides[4];
 };
-static int layout_map(CUtensorMap* out, const void* base, const ImageLayout& l, int box_w) {
+static int layout_map(CUtensorMap* out, const void* base, const ImageLayout& l, int box_w, int box_h) {
   unsigned long long str[4];
   for (int i = 0; i < 4; ++i) str[i] = 2 * l.strides[i];
-  unsigned int box[5] = {64, 1, static_cast<unsigned int>(box_w), 1, 1};
+  unsigned int box[5] = {64, 1, static_cast<unsigned int>(box_w), static_cast<unsigned int>(box_h), 1};
   return make_tensor_map_bf16(out, base, 5, l.dims, str, box);
 }
 
@@ -423,14 +423,33 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   if (c.ntaps * cchunks > GEMM_MAX_KTABLE) return -14;
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
-  const long long m_blocks = static_cast<long long>((c.tiles_w + GEMM_BM - 1) / GEMM_BM) * c.tiles_h * c.B;
+  // (outputs that go to every second pixel, or into another layout, have no per-lane form)
+  const bool strided = c.out_mul != 1 || c.phase_cols != 0;
+  const bool tma_out = c.out_layout != nullptr || (!(epi.flags & ~(EPI_BIAS | EPI_BIAS_F32)) && (strided || gemm_tma_epilogue()));
+  // Pixels of a tile: 128 of a row, or 64 of two rows or 32 of four where fewer tiles cover the image so (96 x 180: 144 instead of 192) and rounds of
+  // CTAs can be saved by it. Not where rows come from a neighbour or every second row is read. Us, 128 x 1 / this: 3x3 convolutions of 96 x 180
+  // pixels, 192 channels 21.8 / 14.5, of 2 x 76 x 131, 128 20.1 / 15.7, of 180 x 129, 192 30.6 / 23.2, of 200 x 400, 192 54.8 / 46.9; in one round anyway 50 x 100
+  // pixels of 384 to every second 12.9 / 14.1.
+  int tile_w = GEMM_BM;
+  long long m_blocks = 0;
+  for (int w = GEMM_BM; w >= 32; w /= 2) {
+    if (w < GEMM_BM && (!tma_out || c.hmul != 1 || halo_lo != nullptr || halo_hi != nullptr)) break;
+    const int high = GEMM_BM / w;
+    const long long count = static_cast<long long>((c.tiles_w + w - 1) / w) * ((c.tiles_h + high - 1) / high) * c.B;
+    if (m_blocks == 0 || (count < m_blocks && m_blocks > num_sms)) {
+      m_blocks = count;
+      tile_w = w;
+    }
+  }
+  const int tile_h = GEMM_BM / tile_w;
   int bn = 0, ctas = 1;
   pick_tile(m_blocks * c.groups, c.N, c.ntaps * cchunks / c.groups, false, epi.flags, true, num_sms, &bn, &ctas);
   p.M = c.B * c.tiles_h * c.tiles_w;
   p.N = c.N;
   p.K = c.ntaps * cchunks * 64;
-  p.tile_n0 = (c.tiles_w + GEMM_BM - 1) / GEMM_BM;
-  p.tile_n1 = c.tiles_h;
+  p.tile_shift = tile_w == 128 ? 7 : (tile_w == 64 ? 6 : 5);
+  p.tile_n0 = (c.tiles_w + tile_w - 1) / tile_w;
+  p.tile_n1 = (c.tiles_h + tile_h - 1) / tile_h;
   p.m_blocks = static_cast<int>(m_blocks);
   p.num_m_tiles = (p.m_blocks + ctas - 1) / ctas;
   p.num_n_tiles = (c.N + bn - 1) / bn;
@@ -443,15 +462,16 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   }
   p.a_mode = OP_TABLE_5D;
   p.b_mode = OP_KMAJOR_2D;
-  int rc = c.in_layout != nullptr ? layout_map(&p.map_a, c.x, *c.in_layout, GEMM_BM) : image_map(&p.map_a, c.x, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
+  int rc = c.in_layout != nullptr ? layout_map(&p.map_a, c.x, *c.in_layout, tile_w, tile_h)
+                                  : image_map(&p.map_a, c.x, c.Cin, c.par, c.W, c.H, c.B, tile_w, tile_h);
   if (rc != 0) return rc;
   rc = map_2d(&p.map_b, c.w, p.K, c.N, p.K, GEMM_BK, bn == 384 ? 64 : bn / ctas);
   if (rc != 0) return rc - 1000;
   rc = attach_halos(p, halo_lo, halo_hi, c.Cin, c.par, c.W, c.H, c.B, GEMM_BM);
   if (rc != 0) return rc;
   // tile (t0, t1, t2) = (w chunk, row, b): base coordinates
-  p.a_mul0[2] = GEMM_BM;
-  p.a_mul1[3] = c.hmul;
+  p.a_mul0[2] = tile_w;
+  p.a_mul1[3] = c.hmul * tile_h;
   p.a_mul2[4] = 1;
   for (int t = 0; t < c.ntaps; ++t)
     for (int k = 0; k < cchunks; ++k) {
@@ -470,14 +490,12 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   p.phase_cols = c.phase_cols;
   std::memcpy(p.out_off, c.out_off, sizeof(p.out_off));
   p.ldc = c.out_c;
-  // (outputs that go to every second pixel have no per-lane form)
-  const bool strided = c.out_mul != 1 || c.phase_cols != 0;
   if (c.out_layout != nullptr) {
-    rc = layout_map(&p.map_c, c.y, *c.out_layout, 32);
-    if (rc == 0 && (p.epi & EPI_RESIDUAL)) rc = layout_map(&p.map_in, p.residual, *c.out_layout, 32);
+    rc = layout_map(&p.map_c, c.y, *c.out_layout, 32, 1);
+    if (rc == 0 && (p.epi & EPI_RESIDUAL)) rc = layout_map(&p.map_in, p.residual, *c.out_layout, 32, 1);
     if (rc != 0) return rc - 5000;
     p.epi_tma = 2;
-  } else if (!(p.epi & ~(EPI_ROW_CONV | EPI_BIAS | EPI_BIAS_F32)) && (strided || gemm_tma_epilogue())) {
+  } else if (tma_out) {
     // 32 pixels x 64 channels per store; rows and channels outside the image are clipped
     const unsigned long long C = static_cast<unsigned long long>(c.out_c), mul = static_cast<unsigned long long>(c.out_mul);
     const unsigned long long row = C * 2ull * mul * c.out_w;

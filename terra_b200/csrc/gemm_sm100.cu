@@ -217,8 +217,9 @@ struct PixelUnit {
 };
 __device__ __forceinline__ PixelUnit pixel_unit(const GemmParams& p, int m_blk, int q, int col, int grp) {
   const int phase = p.phase_cols > 0 ? col / p.phase_cols : grp;
-  return {p.phase_cols > 0 ? col - phase * p.phase_cols : col, p.out_off[phase][1], (m_blk % p.tile_n0) * GEMM_BM + q * 32,
-          (m_blk / p.tile_n0) % p.tile_n1 * p.out_mul + p.out_off[phase][0], m_blk / (p.tile_n0 * p.tile_n1)};
+  const int line = m_blk / p.tile_n0, b = line / p.tile_n1, row = q * 32 >> p.tile_shift;
+  return {p.phase_cols > 0 ? col - phase * p.phase_cols : col, p.out_off[phase][1], ((m_blk - line * p.tile_n0 - row) << p.tile_shift) + q * 32,
+          (((line - b * p.tile_n1) << 7 >> p.tile_shift) + row) * p.out_mul + p.out_off[phase][0], b};
 }
 
 // mbar_wait that adds the time spent to `waited`; a barrier that is complete costs one test and reads no clock.

@@ -15,7 +15,11 @@
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "check.h"
+#include "host_api.h"
+#include "launch_count.h"
 #include "torch_ops.h"
 
 namespace {
@@ -265,21 +269,41 @@ struct NormLayer : torch::CustomClassHolder {
   bool has_res;
 };
 
+// (The launches on the tensors' own pointers: views of them as [B, pixels, C] were a third of the node's host time.)
 struct GroupNormSilu : Function<GroupNormSilu> {
-  static double inverse_count(const Tensor& x, int64_t groups) {
-    return 1.0 / (static_cast<double>(x.size(1)) * x.size(2) * (x.size(3) / groups));
-  }
+  struct Image {
+    int B, C;
+    long long HW;
+    float inv_count;
+    Image(const Tensor& x, int64_t groups) {
+      need(x.is_cuda() && x.dim() == 4 && x.is_contiguous() && x.scalar_type() == torch::kBFloat16, "groupnorm_silu: contiguous NHWC bf16");
+      B = static_cast<int>(x.size(0)), C = static_cast<int>(x.size(3)), HW = x.size(1) * x.size(2);
+      inv_count = static_cast<float>(1.0 / (static_cast<double>(HW) * (C / std::max<int64_t>(groups, 1))));
+    }
+  };
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& gamma, const Tensor& beta, const OptTensor& residual,
                         const Held<NormLayer>& l) {
     const c10::cuda::CUDAGuard guard(x.device());
-    const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
-    const Tensor x3 = x.view(flat);
-    Tensor stats = torch::empty({x.size(0), l->groups, 2}, x.options().dtype(torch::kFloat32));
-    Tensor sums = terra_ops::scratch_take(x, {x.size(0) * l->groups * 2 + 1});      // (and the ticket behind them)
-    terra_ops::groupnorm_mean_rstd(x3, sums, stats, l->groups, inverse_count(x, l->groups), l->eps);
+    const Image im(x, l->groups);
+    need(l->g.numel() == im.C && l->b.numel() == im.C && l->g.is_contiguous() && l->b.is_contiguous() && l->g.scalar_type() == torch::kBFloat16 &&
+             l->b.scalar_type() == torch::kBFloat16,
+         "groupnorm_silu: affine parameters bf16, one per channel");
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    Tensor stats = torch::empty({im.B, l->groups, 2}, x.options().dtype(torch::kFloat32));
+    Tensor sums = terra_ops::scratch_take(x, {im.B * l->groups * 2 + 1});      // (and the ticket behind them)
+    tb::note_launch(2);
+    rc_check(tb::groupnorm_mean_rstd(x.data_ptr(), sums.data_ptr<float>(), stats.data_ptr<float>(), im.B, im.HW, im.C, static_cast<int>(l->groups),
+                                     im.inv_count, static_cast<float>(l->eps), stream),
+             "groupnorm_mean_rstd");
     terra_ops::scratch_give(sums);
-    Tensor y = torch::empty_like(x), y3 = y.view(flat);
-    terra_ops::groupnorm_silu_apply(x3, stats, l->g, l->b, residual.has_value() ? OptTensor(residual->view(flat)) : residual, y3, l->groups);
+    Tensor y = torch::empty_like(x), res;
+    if (residual.has_value()) {
+      need(residual->numel() == x.numel() && residual->is_cuda() && residual->scalar_type() == torch::kBFloat16, "groupnorm_silu: shortcut like the input");
+      res = residual->contiguous();
+    }
+    rc_check(tb::groupnorm_silu_apply(x.data_ptr(), stats.data_ptr<float>(), l->g.data_ptr(), l->b.data_ptr(), res.defined() ? res.data_ptr() : nullptr,
+                                      y.data_ptr(), im.B, im.HW, im.C, static_cast<int>(l->groups), stream),
+             "groupnorm_silu_apply");
     ctx->save_for_backward({x, stats, l->g, l->b});
     hold(ctx, l);
     return y;
@@ -287,16 +311,28 @@ struct GroupNormSilu : Function<GroupNormSilu> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     const auto l = held<NormLayer>(ctx);
-    const Tensor& x = s[0];
+    const Tensor &x = s[0], &stats = s[1], &g = s[2], &b = s[3];
     const Tensor dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
-    const std::vector<int64_t> flat{x.size(0), x.size(1) * x.size(2), x.size(3)};
-    const Tensor x3 = x.view(flat), dy3 = dy.view(flat);
+    // (the saved tensors come back through whatever hooks the caller has set, so their form is checked like any input's)
+    const Image im(x, l->groups);
+    need(dy.sizes() == x.sizes() && dy.scalar_type() == torch::kBFloat16 && stats.is_cuda() && stats.is_contiguous() &&
+             stats.scalar_type() == torch::kFloat32 && stats.numel() == 2 * im.B * l->groups && g.is_cuda() && g.is_contiguous() && b.is_cuda() &&
+             b.is_contiguous() && g.numel() == im.C && b.numel() == im.C && g.scalar_type() == torch::kBFloat16 &&
+             b.scalar_type() == torch::kBFloat16,
+         "groupnorm_silu: saved tensors and the gradient like the forward pass's");
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     ParamGrad gg(l->gamma, "groupnorm: clearing the gradient"), gb(l->beta, "groupnorm: clearing the gradient");
-    Tensor red = zeroed(x, {x.size(0), x.size(3), 2}, "groupnorm: clearing the gradient's sums");
-    terra_ops::groupnorm_silu_bwd_reduce(dy3, x3, s[1], s[2], s[3], red, l->groups, gg.into, gb.into);
-    Tensor dx = torch::empty_like(x), dx3 = dx.view(flat);
-    terra_ops::groupnorm_silu_bwd_apply(dy3, x3, s[1], red, s[2], s[3], dx3, l->groups, inverse_count(x, l->groups));
+    need(gg.into.numel() == im.C && gb.into.numel() == im.C, "groupnorm_silu: gradients of the affine parameters, one per channel");
+    Tensor red = zeroed(x, {im.B, im.C, 2}, "groupnorm: clearing the gradient's sums"), dx = torch::empty_like(x);
+    tb::note_launch(2);
+    rc_check(tb::groupnorm_silu_bwd_reduce(dy.data_ptr(), x.data_ptr(), stats.data_ptr<float>(), g.data_ptr(), b.data_ptr(), red.data_ptr<float>(),
+                                           gg.into.data_ptr<float>(), gb.into.data_ptr<float>(), im.B, im.HW, im.C, static_cast<int>(l->groups),
+                                           stream),
+             "groupnorm_silu_bwd_reduce");
+    rc_check(tb::groupnorm_silu_bwd_apply(dy.data_ptr(), x.data_ptr(), stats.data_ptr<float>(), red.data_ptr<float>(), g.data_ptr(), b.data_ptr(),
+                                          dx.data_ptr(), im.B, im.HW, im.C, static_cast<int>(l->groups), im.inv_count, stream),
+             "groupnorm_silu_bwd_apply");
     return {dx, gg.returned, gb.returned, l->has_res ? dy : Tensor(), Tensor()};
   }
 };

@@ -249,6 +249,16 @@ void pack_taps(const torch::Tensor& w, torch::Tensor& out, int64_t n1, int64_t s
            "pack_taps");
 }
 
+// the same into a matrix of its own: [n1 * n2, taps * channels padded to 64]
+torch::Tensor packed_taps(const torch::Tensor& w, int64_t n1, int64_t s1, int64_t n2, int64_t s2, int64_t channels, int64_t sc,
+                          const std::vector<int64_t>& offsets, int64_t valid2) {
+  need(w.is_cuda() && n1 >= 1 && n2 >= 1 && channels >= 1 && !offsets.empty(), "packed_taps: sizes");
+  const c10::cuda::CUDAGuard guard(w.device());
+  torch::Tensor out = torch::empty({n1 * n2, static_cast<int64_t>(offsets.size()) * ((channels + 63) / 64 * 64)}, w.options());
+  pack_taps(w.contiguous(), out, n1, s1, n2, s2, channels, sc, offsets, valid2);
+  return out;
+}
+
 void grad_inspect(const torch::Tensor& grad, torch::Tensor& out2) {
   need(grad.is_cuda() && grad.is_contiguous() && grad.scalar_type() == torch::kFloat32, "grad_inspect: fp32 contiguous");
   need(out2.scalar_type() == torch::kFloat32 && out2.numel() >= 2, "grad_inspect: out2 fp32 [2]");
@@ -434,6 +444,7 @@ void bind_elementwise(pybind11::module_& m) {
   m.def("adamw_step", &adamw_step);
   m.def("pad_patchify", &pad_patchify);
   m.def("unpatchify_crop", &unpatchify_crop);
+  m.def("packed_taps", &packed_taps);
   m.def("pack_taps", &pack_taps);
   m.def("grad_inspect", &grad_inspect);
   m.def("attn_rowdot", &attn_rowdot);

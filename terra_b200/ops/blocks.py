@@ -96,8 +96,10 @@ def native_node(grads=()) -> bool:
     """Whether a layer may be a node in C++: not while a trace is recorded or a function transform is active (the Python nodes
     are recorded by the first and refuse the second), when single launches are to be observed, or without gradient
     accumulators (which only a backward pass asks for)."""
-    return (not _LAUNCHES_OBSERVED and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
-            and all(g is not None for g in grads))
+    for g in grads:
+        if g is None:
+            return False
+    return not _LAUNCHES_OBSERVED and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
 
 
 def _native_half(comm, geo: WindowGeometry, impl: str) -> bool:

@@ -40,9 +40,7 @@ def _pack_taps(w, n1, s1, n2, s2, channels, sc, offsets, pad2=None):
     valid2, n2 = n2, pad2 or n2
     cpad, taps = (channels + 63) // 64 * 64, len(offsets)
     if w.is_cuda and w.dtype == torch.bfloat16:
-        out = torch.empty(n1 * n2, taps * cpad, device=w.device, dtype=torch.bfloat16)
-        _ext.load().pack_taps(w.contiguous(), out, n1, s1, n2, s2, channels, sc, list(offsets), valid2)
-        return out
+        return _ext.load().packed_taps(w, n1, s1, n2, s2, channels, sc, offsets, valid2)
     steps = [(n1, s1), (valid2, s2), (1, 0), (channels, sc)]
     at = sum(torch.arange(n, device=w.device).view([-1 if d == e else 1 for e in range(4)]) * s for d, (n, s) in enumerate(steps))
     at = at + torch.tensor(list(offsets), device=w.device).view(1, 1, -1, 1)

@@ -171,8 +171,10 @@ class ParamArena:
 
     def zero_grad(self) -> None:
         self.grad.zero_()
+        base = self.grad.data_ptr()
         for p, off in zip(self.params, self.offsets):
-            if p.grad is None or p.grad.data_ptr() != self.grad.data_ptr() + off * 4:
+            g = p.grad
+            if g is None or g.data_ptr() != base + off * 4:
                 p.grad = self.grad[off:off + p.numel()].view(p.shape)
 
     def segment(self, label: str) -> Optional[Segment]:

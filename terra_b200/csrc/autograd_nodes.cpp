@@ -344,6 +344,38 @@ Tensor groupnorm_silu(const Tensor& x, const Tensor& gamma, const Tensor& beta, 
   return GroupNormSilu::apply(x, gamma, beta, residual, l);
 }
 
+// ------------------------------------------------------------------------------------------------ windows of an image and back
+// x, seen as [outer, a, b, inner], with a and b exchanged, in the shape `sizes`
+struct SwapMiddle : Function<SwapMiddle> {
+  static Tensor copy(const Tensor& x, int64_t outer, int64_t a, int64_t b, at::IntArrayRef sizes) {
+    const int64_t bytes = outer * a * b > 0 ? static_cast<int64_t>(x.nbytes()) / (outer * a * b) : 0;
+    need(x.is_cuda() && x.is_contiguous() && bytes > 0 && bytes % 16 == 0 && bytes * outer * a * b == static_cast<int64_t>(x.nbytes()) &&
+             reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0,
+         "swap_middle: contiguous [outer, a, b, inner], inner whole 16-byte vectors");
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor y = torch::empty(sizes, x.options());
+    need(y.numel() == x.numel(), "swap_middle: sizes");
+    tb::note_launch();
+    rc_check(tb::swap_middle_vectors(x.data_ptr(), y.data_ptr(), outer, a, b, bytes / 16, c10::cuda::getCurrentCUDAStream().stream()), "swap_middle");
+    return y;
+  }
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t outer, int64_t a, int64_t b, std::vector<int64_t> sizes) {
+    ctx->saved_data["dims"] = std::vector<int64_t>{outer, a, b};
+    ctx->saved_data["sizes"] = x.sizes().vec();
+    return copy(x, outer, a, b, sizes);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto d = ctx->saved_data["dims"].toIntVector(), sizes = ctx->saved_data["sizes"].toIntVector();
+    Tensor dy = grads[0].contiguous();
+    if (reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 != 0) dy = dy.clone();
+    return {SwapMiddle::apply(dy, d[0], d[2], d[1], sizes), Tensor(), Tensor(), Tensor(), Tensor()};   // itself differentiable, as the operators' is
+  }
+};
+
+Tensor swap_middle(const Tensor& x, int64_t outer, int64_t a, int64_t b, std::vector<int64_t> sizes) {
+  return SwapMiddle::apply(x, outer, a, b, std::move(sizes));
+}
+
 }  // namespace
 
 void bind_nodes(pybind11::module_& m) {
@@ -354,4 +386,5 @@ void bind_nodes(pybind11::module_& m) {
   n.def("conv3x3", &conv3x3);
   n.def("conv_transpose2x2", &conv_transpose2x2);
   n.def("groupnorm_silu", &groupnorm_silu);
+  n.def("swap_middle", &swap_middle, "x as [outer, a, b, inner] with a and b exchanged, in the shape given");
 }

@@ -755,6 +755,27 @@ __global__ void __launch_bounds__(256) fold_taps_kernel(float* __restrict__ src,
         dst[(static_cast<long long>(c0 + warp + 8 * k) * rows + r0) * taps + lane + 32 * i] = old[k][i] + tile[warp + 8 * k][lane + 32 * i];
 }
 
+// out[p][b][a][r] = in[p][a][b][r] (16-byte vectors): image rows of windows to windows of rows and back. Bound by HBM: four vectors a thread, all asked
+// for before the first is stored. Against the tensor operators' copy, which moves two bytes per lane, cold: 23040 x 192 18.4 -> 10.2 us, 139264 x 384
+// 141.2 -> 38.9 us (5.5 TB/s).
+__global__ void __launch_bounds__(256) swap_middle_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, unsigned int A, unsigned int B,
+                                                          unsigned int run, unsigned int total) {
+  chain_begin();
+  constexpr int EACH = 4;
+  uint4 v[EACH];
+  const unsigned int first = blockIdx.x * (256u * EACH) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < EACH; ++k) {
+    const unsigned int i = first + 256u * k;
+    if (i >= total) break;
+    const unsigned int t = i / run, q = t / A, a = t - q * A, p = q / B, b = q - p * B;
+    v[k] = in[static_cast<size_t>((p * A + a) * B + b) * run + (i - t * run)];
+  }
+#pragma unroll
+  for (int k = 0; k < EACH; ++k)
+    if (first + 256u * k < total) out[first + 256u * k] = v[k];
+}
+
 // pass 2: dx = rstd * (dz*gamma - s1/n - xhat * s2/n), s1 = sum_c gamma_c red[b][c][0], s2 likewise with [1]
 __global__ void __launch_bounds__(256, 2) groupnorm_silu_bwd_apply_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
@@ -1352,6 +1373,15 @@ int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa
   const long long total = static_cast<long long>(na) * nb * nc;
   if (total <= 0) return 0;
   launch_chained(strided_add_kernel, grid_for(total, 256), 256, 0, stream, src, dst, na, nb, nc, sa, sb, sc);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+int swap_middle_vectors(const void* in, void* out, long long P, long long A, long long B, long long run, cudaStream_t stream) {
+  const long long total = P * A * B * run;
+  if (P < 0 || A < 0 || B < 0 || run < 0 || total > 0x70000000LL) return -1;
+  if (total == 0) return 0;
+  launch_chained(swap_middle_kernel, static_cast<unsigned>((total + 1023) / 1024), 256, 0, stream, static_cast<const uint4*>(in),
+                 static_cast<uint4*>(out), static_cast<unsigned>(A), static_cast<unsigned>(B), static_cast<unsigned>(run), static_cast<unsigned>(total));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -145,6 +145,8 @@ int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, 
 int groupnorm_finalize(float* sums, float* stats, int cells, float inv_count, float eps, cudaStream_t stream);
 // dst[a*sa + b*sb + c*sc] += src[a][b][c] (fp32, src contiguous [na][nb][nc]); src is zeroed behind the read.
 int strided_add_f32(float* src, float* dst, int na, int nb, int nc, long long sa, long long sb, long long sc, cudaStream_t stream);
+// out[p][b][a][r] = in[p][a][b][r], r over `run` 16-byte vectors
+int swap_middle_vectors(const void* in, void* out, long long P, long long A, long long B, long long run, cudaStream_t stream);
 // dst[c][r][t] += src[t][r][c] (fp32, both contiguous, taps <= 9); src is zeroed behind the read.
 int fold_taps_f32(float* src, float* dst, int taps, int rows, int cols, cudaStream_t stream);
 // Masked loss: loss_sum += sum(f(pred * mask - label)), f = |.| (kind 0) or square (kind 1);

@@ -33,6 +33,16 @@ from . import collectives as C
 from .window_assignment import window_owner_map
 
 
+def _swap_middle(t, outer, a, b, shape):
+    """``t`` as ``[outer, a, b, inner]`` with ``a`` and ``b`` exchanged, in ``shape``, by one copy kernel; None where it does not apply (the tensor
+    operators do it: CPU, other types and layouts, inner parts of no whole 16-byte vectors, traces and function transforms; sizes that do not fit, which
+    they refuse; one of the two of size 1, which they answer without a copy)."""
+    if not (outer > 0 and a > 1 and b > 1 and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and 0 < t.numel() < 1 << 33 and t.data_ptr() % 16 == 0
+            and t.numel() % (8 * outer * a * b) == 0 and torch.autograd.forward_ad._current_level < 0 and B.native_node()):
+        return None
+    return B._ext.load().nodes.swap_middle(t, outer, a, b, shape)
+
+
 class DomainComm:
     """Row-stripe helpers for the sampling blocks (halo rows, GroupNorm statistics)."""
 
@@ -316,6 +326,10 @@ class ParallelContext:
     def stripe_to_windows(self, x):
         """NHWC row stripe ``[B, Ht/wp, Wt, C]`` -> this rank's window-major rows."""
         Bn, h, W, Cn = x.shape
+        if self.local_relayout and h % self.wh == 0 and h * self.world == self.Ht and W == self.Wt:
+            swapped = _swap_middle(x, Bn * h // self.wh, self.wh, self.nWw, (Bn * h * W, Cn))
+            if swapped is not None:
+                return swapped
         if self.local_relayout and self.world > 1:
             win = x.reshape(Bn, h // self.wh, self.wh, self.nWw, self.ww, Cn).permute(0, 1, 3, 2, 4, 5)
             return win.reshape(-1, Cn).contiguous()
@@ -346,6 +360,9 @@ class ParallelContext:
         Cn = rows.shape[-1]
         if self.local_relayout:
             nh = self.nWh // self.world
+            swapped = _swap_middle(rows, batch * nh, self.nWw, self.wh, (batch, nh * self.wh, self.Wt, Cn))
+            if swapped is not None:
+                return swapped
             win = rows.reshape(batch, nh, self.nWw, self.wh, self.ww, Cn).permute(0, 1, 3, 2, 4, 5)
             return win.reshape(batch, nh * self.wh, self.Wt, Cn).contiguous()
         m = self.manager

@@ -149,9 +149,8 @@ def case_conv(a):
         dy = _rand(B, Ho, Wo, C, scale=0.1)
         dw = torch.zeros(9, C, C, device="cuda")
         from .conv import _wgrad_split
-        split, stack = _wgrad_split(B, H, W, a.stride, C, C)      # the model's choice
-        split = a.split or split
-        fn = lambda: ext.conv3x3_wgrad(x, dy, dw, a.stride, split, status_word("cuda"), None, None, stack=stack)
+        split = a.split or _wgrad_split(B, H, W, a.stride, C, C)[0]      # (the model's lower bound)
+        fn = lambda: ext.conv3x3_wgrad_taps(x, dy, dw, a.stride, status_word("cuda"), None, True, split)
         nbytes = (x.numel() + dy.numel()) * 2
     else:
         wp = pack_conv3x3_weight(w)

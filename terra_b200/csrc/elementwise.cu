@@ -1180,9 +1180,13 @@ int grid_for(long long work_items, int block, int max_blocks = 148 * 16) {
 
 }  // namespace
 
-// CALL sees LPR, VPL and EXACT (see the LayerNorm kernels) for rows of NVEC 16-byte vectors. MANY: rows
-// enough that groups of 32 / LPR of them still make warps for every SM; below that a row per warp finishes sooner (shorter chains,
-// more warps).
+// CALL sees LPR, VPL and EXACT (see the LayerNorm kernels) for rows of NVEC 16-byte vectors. MANY: rows enough for groups of 32 / LPR
+// of them; below that a row per warp finishes sooner (shorter chains, more warps). The lines are LN_FWD_GROUPS and LN_BWD_GROUPS rows: beyond them a row per
+// warp means several rows one after the other in every warp, each waiting for its loads and its shuffles, and backward as many
+// more blocks that end in atomics on the same sums. Inputs in L2, us, a row per warp / groups. Forward: C = 192, 1024 rows 1.70 / 1.97,
+// 2048 1.88 / 1.98, 4096 2.59 / 2.06, 17280 5.23 / 3.17; 384, 2048 2.33 / 2.13, 17280 7.29 / 5.39; 96, 2048 1.88 / 1.98, 17280 5.17 / 2.41. Backward: 96,
+// 512 2.06 / 2.59, 2048 3.59 / 2.66; 192, 512 2.79 / 2.67, 1024 3.84 / 2.83, 2048 6.21 / 3.41, 8192 7.76 / 6.88; 384, 2048 6.31 / 4.68, 8192 9.09 / 7.95.
+constexpr long long LN_FWD_GROUPS = 2048, LN_BWD_GROUPS = 1024;
 #define TB_LN_CASE(L, V, E, ...) { constexpr int LPR = L; constexpr int VPL = V; constexpr bool EXACT = E; __VA_ARGS__; }
 #define TB_LN_DISPATCH(NVEC, MANY, ...)                         \
   switch ((MANY) ? (NVEC) : 0) {                                               \
@@ -1220,7 +1224,7 @@ inline int ln_bwd_blocks(int vpl, long long rows) {
 int layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                   long long rows, int C, float eps, cudaStream_t stream) {
   if (C % 8 != 0 || C > 2048) return -1;
-  TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 16,
+  TB_LN_DISPATCH(C / 8, rows >= LN_FWD_GROUPS,
                  launch_chained(layernorm_fwd_kernel<LPR, VPL, EXACT>, grid_for(rows, 8 * (32 / LPR), ln_fwd_blocks(VPL)), 256, 0, stream,
                                 static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
                                 static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(y), mean, rstd, rows, C, eps));
@@ -1256,9 +1260,9 @@ int layernorm_bwd(const void* dy, const void* x, const void* gamma, const float*
     return C <= 768 ? go(ln_bwd_launch<32, 3, false, true, true>) : go(ln_bwd_launch<32, 4, false, true, true>);
   }
   if (dres != nullptr) {
-    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, return go(ln_bwd_launch<LPR, VPL, EXACT, true, false>));
+    TB_LN_DISPATCH(C / 8, rows >= LN_BWD_GROUPS, return go(ln_bwd_launch<LPR, VPL, EXACT, true, false>));
   } else {
-    TB_LN_DISPATCH(C / 8, rows >= 148 * 8 * 8, return go(ln_bwd_launch<LPR, VPL, EXACT, false, false>));
+    TB_LN_DISPATCH(C / 8, rows >= LN_BWD_GROUPS, return go(ln_bwd_launch<LPR, VPL, EXACT, false, false>));
   }
   return -1;
 }

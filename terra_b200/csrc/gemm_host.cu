@@ -14,7 +14,7 @@ namespace tb {
 
 cudaError_t launch_gemm(const GemmParams& p, int bn, int ctas, int num_sms, cudaStream_t stream);
 cudaError_t gemm_read_stalls(unsigned long long* out8, bool reset);
-cudaError_t gemm_ones_tile(void** ptr);
+cudaError_t gemm_ones_rows(void** ptr);
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -335,8 +335,8 @@ int gemm_bf16_peers(const GemmOperand& A, const GemmOperand& B, long long M, lon
   if (epi.row_sums != nullptr) {
     if (!gemm_row_sums_fit(M, ctas * (p.stack == 2 ? 2 : 1)) || p.epi_tma != 3 || !A.mn_major) return -21;
     void* ones = nullptr;
-    if (gemm_ones_tile(&ones) != cudaSuccess) return -20;
-    rc = map_2d(&p.map_in, ones, 64, 64, 64, 64, 64);
+    if (gemm_ones_rows(&ones) != cudaSuccess) return -20;
+    rc = map_2d(&p.map_in, ones, 128, 256, 128, 64, 64);
     if (rc != 0) return rc - 2000;
     p.row_sums = epi.row_sums;
     p.ones_row = static_cast<int>((M + 63) / 64 * 64);
@@ -711,7 +711,7 @@ int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, 
 // All taps' weight gradients as one product (one rank): the channels of the displaced image, box after box of 64 and tap after tap, are the
 // rows, and the other image's channels the columns, so that tiles of 256 rows need no whole number of them in a tap (9 x 384 rows are 13.5 of
 // a pair's, 9 x 192 seven stacked ones where two per tap made nine). With the undisplaced image as operand B its column sums, the bias gradient of
-// a convolution, are one more row, that of a box of ones.
+// a convolution, are one more box of rows, whose rows of ones share them out (g_ones_rows).
 //
 // The plan is the one with the least time by a model, in us: rounds of tiles over the CTAs (pairs), each its k-blocks and a hand-over with the
 // epilogue. Fitted to 900 passes in CUDA graphs: the two layers at 512 to 557056 pixels, 96 to 384 channels, all tiles, half a round to three
@@ -798,8 +798,8 @@ static int tap_wgrad(const void* a, const void* b, float* dw, int B, int Ho, int
   rc = image_map(&p.map_b, b, N, 1, Wo, Ho, B, GEMM_BK);
   if (rc != 0) return rc - 1000;
   void* ones = nullptr;      // (boxes behind the last tap are read in any case)
-  if (gemm_ones_tile(&ones) != cudaSuccess) return -20;
-  rc = map_2d(&p.map_in, ones, 64, 64, 64, 64, 64);
+  if (gemm_ones_rows(&ones) != cudaSuccess) return -20;
+  rc = map_2d(&p.map_in, ones, 128, 256, 128, 64, 64);
   if (rc != 0) return rc - 2000;
   for (int t = 0; t < ntaps; ++t) {
     p.grp_off[t][0] = taps[t].parity;

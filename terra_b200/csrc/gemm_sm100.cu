@@ -99,13 +99,27 @@ struct GemmCfg {
 // [3] TMA thread span, [4] of it waiting for free stages, [5] first epilogue warp span, [6] of it waiting for tiles.
 __device__ unsigned long long g_gemm_stalls[8];
 
-// 64 x 64 bf16 ones: operand rows whose product with B is B's column sums (GemmParams::tap_boxes)
-#define TB_ONES_8(v) v, v, v, v, v, v, v, v
-#define TB_ONES_64(v) TB_ONES_8(TB_ONES_8(v))
-__device__ __align__(1024) uint32_t g_ones_tile[2048] = {TB_ONES_8(TB_ONES_64(0x3F803F80u)), TB_ONES_8(TB_ONES_64(0x3F803F80u)),
-                                                         TB_ONES_8(TB_ONES_64(0x3F803F80u)), TB_ONES_8(TB_ONES_64(0x3F803F80u))};
-#undef TB_ONES_8
-#undef TB_ONES_64
+// Operand rows whose product with B is B's column sums (GemmParams::row_sums): 4 x 64 rows of 128 bf16, of which rows 64 j to 64 j + 63 have a one in
+// column 56 + j. A box of 64 x 64 of them from column 56 - 8 i and row 64 j on is a box of A whose row 8 i + j is ones. The others
+// are 2^-126, not zeros, which would turn an infinity of B into a NaN.
+#define TB_8(...) __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__
+#define TB_LOW 0x00800080u
+#define TB_LOW_4 TB_LOW, TB_LOW, TB_LOW, TB_LOW
+#define TB_ROW(a, b) TB_8(TB_LOW), TB_8(TB_LOW), TB_8(TB_LOW), TB_LOW_4, a, b, TB_LOW, TB_LOW, TB_8(TB_LOW_4)
+#define TB_64_ROWS(a, b) TB_8(TB_8(TB_ROW(a, b)))
+__device__ __align__(1024) uint32_t g_ones_rows[4 * 64 * 64] = {TB_64_ROWS(0x00803F80u, TB_LOW), TB_64_ROWS(0x3F800080u, TB_LOW),
+                                                                TB_64_ROWS(TB_LOW, 0x00803F80u), TB_64_ROWS(TB_LOW, 0x3F800080u)};
+#undef TB_8
+#undef TB_LOW
+#undef TB_LOW_4
+#undef TB_ROW
+#undef TB_64_ROWS
+
+// A k-block's box of g_ones_rows: each of 32 rows of A takes every 32nd k-block, since the tensor core's fp32 sums lose with their length.
+// Error of the bias gradient of 557056 pixels (parts of 871 k-blocks), a row for all k-blocks 2.6e-6, 32 rows 1.1e-7; of 139264 (231)
+// 4.2e-7 and 1.0e-7; of a patch embedding of 557056 patches (484) 1.1e-6 and 1.3e-7. The time is the same.
+__device__ __forceinline__ int ones_col(int kb) { return 56 - (kb & 7) * 8; }
+__device__ __forceinline__ int ones_line(int kb) { return (kb >> 3 & 3) * 64; }
 
 struct TileCoord {
   int grp, m_blk, n_blk, split;
@@ -349,7 +363,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 #pragma unroll
           for (int d = 0; d < 5; ++d) abase[d] = t0 * p.a_mul0[d] + t1 * p.a_mul1[d] + t2 * p.a_mul2[d];
         }
-        // rows over all taps: channel and displacement of this tile's boxes of 64 rows (channel < 0: ones)
+        // rows over all taps: channel and displacement of this tile's boxes of 64 rows (channel < 0: ones or nothing)
         constexpr int BOXES = PEERS ? 1 : STACK * GEMM_BM / 64;
         short box_c[BOXES], box_p[BOXES], box_w[BOXES], box_h[BOXES];
         if (!PEERS && p.tap_boxes > 0) {
@@ -403,7 +417,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 #pragma unroll
             for (int j = 0; j < STACK * GEMM_BM / 64; ++j)
               if (STACK == 1 || j < blocks * (GEMM_BM / 64)) {
-                if (!PEERS && p.row_sums != nullptr && m0 + j * 64 == p.ones_row) tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_in, bar, 0, 0);
+                if (!PEERS && p.row_sums != nullptr && m0 + j * 64 == p.ones_row)
+                  tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_in, bar, ones_col(kb), ones_line(kb));
                 else tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, m0 + j * 64, kb * GEMM_BK);
               }
           } else if (p.a_mode == OP_TABLE_5D) {
@@ -426,7 +441,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
                 tma_load_5d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_a, bar, box_c[j], box_p[j], pix.w * GEMM_BK + box_w[j],
                                   pix.h * p.pix_hmul + box_h[j], pix.b);
               else
-                tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_in, bar, 0, 0);
+                tma_load_2d<PAIR>(sA + j * (GEMM_BK * 128), &p.map_in, bar, ones_col(kb), ones_line(kb));
             }
             pix.next(p);
           } else {  // OP_PIXELS_5D: {channels, parity, w, h, b}
@@ -872,7 +887,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
           if (STACK > 1 && tc.m_blk >= p.m_blocks) break;
           const int dcol = STACK > 1 ? mb : acc;
           int row = tc.m_blk * GEMM_BM + q * 32, group = tc.grp, rows = p.M;      // this warp's rows of the group (tap)
-          const bool ones = p.row_sums != nullptr && row == p.ones_row;
+          const bool ones = p.row_sums != nullptr && (row & ~63) == p.ones_row;
           if (p.tap_boxes > 0) {
             group = (row >> 6) / p.tap_boxes;
             row -= group * p.tap_boxes * 64;
@@ -903,10 +918,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
                                "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
                                : "memory");
               }
-              if (ones) {      // row 0: the column sums of B
+              if (ones) {      // the rows of a column add up to its share of the column sums of B; a lane per column
                 __syncwarp();
-                const int at = (p.epi & EPI_TRANSPOSE) ? lane * 128 + ((lane & 7) << 4) : lane * 4;
-                if (cb + lane < p.N) atomicAdd(p.row_sums + cb + lane, *reinterpret_cast<const float*>(my_out + at));
+                float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int r = 0; r < 32; ++r) {
+                  const int at = (p.epi & EPI_TRANSPOSE) ? lane * 128 + (((r >> 2) ^ (lane & 7)) << 4) + ((r & 3) << 2)
+                                                         : r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + ((lane & 3) << 2);
+                  sum[r & 3] += *reinterpret_cast<const float*>(my_out + at);
+                }
+                if (cb + lane < p.N) atomicAdd(p.row_sums + cb + lane, (sum[0] + sum[1]) + (sum[2] + sum[3]));
                 continue;
               }
               fence_proxy_async_smem();
@@ -956,7 +977,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             return (lr < p.a_rows) ? static_cast<long long>(peer) * p.a_rows + lr : -1;
           } else if (!PEERS && p.tap_boxes > 0) {
             const int g = tc.m_blk * GEMM_BM + r, tap = (g >> 6) / p.tap_boxes, c = g - tap * p.tap_boxes * 64;
-            if (tap >= p.taps) return g == p.ones_row ? -2 : -1;      // -2: the column sums of B
+            if (tap >= p.taps) return (g & ~63) == p.ones_row ? -2 : -1;      // -2: a share of the column sums of B
             return c < p.tap_channels ? static_cast<long long>(tap) * p.tap_channels + c : -1;
           } else {
             const long long g = static_cast<long long>(tc.m_blk) * GEMM_BM + r;
@@ -1261,14 +1282,14 @@ static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t s
   return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, p);
 }
 
-cudaError_t gemm_ones_tile(void** ptr) {
+cudaError_t gemm_ones_rows(void** ptr) {
   static std::atomic<void*> known[64];      // per device: the look-up takes a microsecond
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   *ptr = dev < 64 ? known[dev].load(std::memory_order_relaxed) : nullptr;
   if (*ptr != nullptr) return cudaSuccess;
-  e = cudaGetSymbolAddress(ptr, g_ones_tile);
+  e = cudaGetSymbolAddress(ptr, g_ones_rows);
   if (e == cudaSuccess && dev < 64) known[dev].store(*ptr, std::memory_order_relaxed);
   return e;
 }

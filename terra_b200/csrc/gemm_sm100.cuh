@@ -47,10 +47,10 @@ struct GemmParams {
   short grp_off[16][4];        // per group (tap): {parity, dw, dh, unused} applied to operand B, or A
   // Weight gradients of all taps as one product (tap_boxes > 0, groups = 1): the rows of A are tap_boxes boxes of 64 channels per tap, one
   // tap after the other, so that tiles of 128, 256 or a pair's 2 x 128 rows run on across taps; row (tap, channel) of the output is
-  // row tap * tap_channels + channel. Boxes behind the last tap are ones (map_in: a 64 x 64 tile of them).
+  // row tap * tap_channels + channel. Boxes behind the last tap come from map_in.
   int taps, tap_boxes, tap_channels;
-  // Weight gradients: with row_sums, the box of A from row ones_row on (behind its own) is ones, and the first of these rows, the column sums of
-  // B, is accumulated into row_sums.
+  // Weight gradients: with row_sums, the box of A from row ones_row on (behind its own) is one of map_in's, whose 64 rows (some of ones for every
+  // k-block) add up to the column sums of B and are accumulated into row_sums.
   float* row_sums;
   int ones_row;
   int disp_a;                  // the displaced image is operand A (and the column sums add up over the groups)

@@ -27,10 +27,10 @@
 //     chains to issue from, and half the reads of K and V through the shared-memory port;
 //   * accumulator tiles go to shared memory four 8 x 8 tiles an instruction;
 //   * windows of at most 32 tokens have blocks of their own size, and padding columns cost a comparison, not the masked form.
-// Us, before these three / now (shifted, with bias): 2176 windows of 8 x 8, 12 heads of 32 channels, forward 105 / 88 (66 of HBM
-// traffic), backward 236 / 226 (115); 2448 of 8 x 8, 8 heads of 128 channels 237 / 235 and 626 / 612; 180 of 8 x 12, 12 heads of 16
-// channels 26 / 17 and 50 / 43; 1020 of 7 x 7, 12 heads of 32 channels 93 / 53 and 140 / 120; 1800 of 4 x 8, 8 heads of 32 channels
-// 89 / 22 and 120 / 54. What is left is issue and latency: the shared-memory port is busy 50 (forward) and 70 % (backward) of the time.
+// Us, before these three / now (shifted, with bias): 2176 windows of 8 x 8, 12 heads of 32 channels, forward 105 / 87 (66 of HBM
+// traffic), backward 236 / 227 (115); 2448 of 8 x 8, 8 heads of 128 channels 237 / 236 and 626 / 599; 180 of 8 x 12, 12 heads of 16
+// channels 26 / 16 and 50 / 44; 1020 of 7 x 7, 12 heads of 32 channels 93 / 52 and 140 / 122; 1800 of 4 x 8, 8 heads of 32 channels
+// 89 / 23 and 120 / 57. What is left is issue and latency: the shared-memory port is busy 50 (forward) and 70 % (backward) of the time.
 #include <atomic>
 #include "chained_launch.cuh"
 #include "common.cuh"
@@ -199,9 +199,26 @@ __device__ __forceinline__ void wa_set(float (&v)[4], int i, f32x2 x) { f2_unpac
 // repeat every 1 (3) blocks of 8, so an index is one of 1 (3) per-thread bases plus a compile-time constant; other
 // widths read cofs from shared memory.
 // A warp's block is MT tiles of 16 rows (rows r0 + 16 t and r0 + 16 t + 8 of this thread).
-template <int NPAD, int WW, int MT>
-__device__ __forceinline__ void wa_scores(float (&s)[MT][NPAD / 8][4], float scale2, const float* tb, int rel0, const int* cofs,
+//
+// MASK: of a window that the shifted frame's last row or column cuts; the mask is added where query and key lie in different regions (`tab`).
+// Without the pairs and the constant offsets that took three times as long per element, and the blocks that met such a window finished last.
+// Us, forward and backward, so / this: 180 windows of 8 x 12, 12 heads of 16 channels 24.4 / 15.7 and 51 / 44; 2176 of 8 x 8, 12 heads
+// of 32 93.5 / 87 and 235 / 228. (The mask over the scale as what the products are added to, 16.3 and 44.5, 88.8 and 227, sums a
+// masked product at the mask's magnitude, which rounds HD / 16 times where this rounds once: gradient of the bias table where such
+// products decide 5.2e-6 off instead of 2.0e-6. 32 channels in windows of 8 x 12 spill more here: forward 11.5 / 12.1.)
+template <int NPAD, int WW, int MT, bool MASK>
+__device__ __forceinline__ void wa_scores(float (&s)[MT][NPAD / 8][4], float scale2, const float* tb, int rel0, const int* cofs, const int2* tab,
                                           int r0, int tq, int N, float (&mx)[MT][2]) {
+  auto mask = [&](float (&v)[4], int t, int nb) {
+    if constexpr (MASK) {
+      const int e0 = tab[nb * 8 + tq * 2].y, e1 = tab[nb * 8 + tq * 2 + 1].y;      // regions in bits 8 and up
+      const int f0 = tab[r0 + 16 * t].y, f1 = tab[r0 + 16 * t + 8].y;
+      if ((e0 ^ f0) >> 8) v[0] += -100.f * WA_LOG2E;
+      if ((e1 ^ f0) >> 8) v[1] += -100.f * WA_LOG2E;
+      if ((e0 ^ f1) >> 8) v[2] += -100.f * WA_LOG2E;
+      if ((e1 ^ f1) >> 8) v[3] += -100.f * WA_LOG2E;
+    }
+  };
   if constexpr (WW == 8) {
     // row r0 + 8 is the next window row, same column: its bias at key block nb is row r0's at block nb - 1, and so on for the rows below
     const float* p = tb + ((r0 >> 3) * 15 + (r0 & 7) - 2 * tq + rel0);
@@ -215,10 +232,14 @@ __device__ __forceinline__ void wa_scores(float (&s)[MT][NPAD / 8][4], float sca
 #pragma unroll
       for (int t = 0; t < MT; ++t)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < 2; ++h)
           wa_set(s[t][nb], 2 * h, f2_fma(wa_pair(s[t][nb], 2 * h), f2_both(scale2), f2_pack(b[2 * t + h][0], b[2 * t + h][1])));
-          mx[t][h] = fmaxf(mx[t][h], fmaxf(s[t][nb][2 * h], s[t][nb][2 * h + 1]));
-        }
+#pragma unroll
+      for (int t = 0; t < MT; ++t) {
+        mask(s[t][nb], t, nb);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) mx[t][h] = fmaxf(mx[t][h], fmaxf(s[t][nb][2 * h], s[t][nb][2 * h + 1]));
+      }
 #pragma unroll
       for (int i = 2 * MT - 1; i > 0; --i) b[i][0] = b[i - 1][0], b[i][1] = b[i - 1][1];
     }
@@ -237,6 +258,7 @@ __device__ __forceinline__ void wa_scores(float (&s)[MT][NPAD / 8][4], float sca
         const float* c = p[nb % 3] - (nb / 3) * 46;
         wa_set(s[t][nb], 0, f2_fma(wa_pair(s[t][nb], 0), f2_both(scale2), f2_pack(c[0], c[-1])));
         wa_set(s[t][nb], 2, f2_fma(wa_pair(s[t][nb], 2), f2_both(scale2), f2_pack(c[dr], c[dr - 1])));
+        mask(s[t][nb], t, nb);
         mx[t][0] = fmaxf(mx[t][0], fmaxf(s[t][nb][0], s[t][nb][1]));
         mx[t][1] = fmaxf(mx[t][1], fmaxf(s[t][nb][2], s[t][nb][3]));
       }
@@ -252,6 +274,7 @@ __device__ __forceinline__ void wa_scores(float (&s)[MT][NPAD / 8][4], float sca
         s[t][nb][1] = fmaf(s[t][nb][1], scale2, t0[-co.y]);
         s[t][nb][2] = fmaf(s[t][nb][2], scale2, t1[-co.x]);
         s[t][nb][3] = fmaf(s[t][nb][3], scale2, t1[-co.y]);
+        mask(s[t][nb], t, nb);
         if (nb * 8 + 8 > N) {      // padding columns: their scores are lowest, their probabilities zero
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -272,31 +295,6 @@ __device__ __forceinline__ void wa_zero(float (&d)[MT][NPAD / 8][4]) {
     for (int nb = 0; nb < NPAD / 8; ++nb)
 #pragma unroll
       for (int k = 0; k < 4; ++k) d[t][nb][k] = 0.f;
-}
-
-// What the products of q and k are added to: zero, or in a window that the mask cuts (few: the last row and column of the shifted frame) the
-// mask over the scale where query and key lie in different regions. There it costs a comparison an element and no register beyond the
-// sums' own; a score path of its own took three times as long, and the blocks that met it finished last. Us, such a path / this: 180
-// shifted windows of 8 x 12, 12 heads of 16 channels forward 24.5 / 16.5,
-// backward 49.1 / 42.9; 2176 of 8 x 8, 12 heads of 32 92.4 / 87.8 and 232.8 / 225.9. (Rounding: a masked
-// product loses its low bits to the mask's, which its probability of e^-100 hides.)
-template <int NPAD, int MT>
-__device__ __forceinline__ void wa_start_scores(float (&s)[MT][NPAD / 8][4], bool masked, float scale2, const int2* tab, int r0, int tq) {
-  wa_zero<NPAD, MT>(s);
-  if (!masked) return;
-  const float off = __fdividef(-100.f * WA_LOG2E, scale2);
-#pragma unroll
-  for (int t = 0; t < MT; ++t) {
-    const int reg0 = tab[r0 + 16 * t].y, reg1 = tab[r0 + 16 * t + 8].y;
-#pragma unroll
-    for (int nb = 0; nb < NPAD / 8; ++nb) {
-      const int e0 = tab[nb * 8 + tq * 2].y, e1 = tab[nb * 8 + tq * 2 + 1].y;      // regions in bits 8 and up
-      if ((e0 ^ reg0) >> 8) s[t][nb][0] = off;
-      if ((e1 ^ reg0) >> 8) s[t][nb][1] = off;
-      if ((e0 ^ reg1) >> 8) s[t][nb][2] = off;
-      if ((e1 ^ reg1) >> 8) s[t][nb][3] = off;
-    }
-  }
 }
 
 // d[t] += A(16 rows at `arow` + 16 t, HD channels) * B(NPAD rows at `bmat`)^T, both row-major bf16 in shared memory
@@ -438,8 +436,7 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
   const int items = a.B * my_nw;
   const int q0 = a.my_sp * a.shardN;
   const int q1 = min(N, q0 + a.shardN);
-  // (no scale at all: one that leaves nothing of the products, so that the mask can be divided by it)
-  const float scale2 = a.scale == 0.f ? 1e-30f : a.scale * WA_LOG2E;
+  const float scale2 = a.scale * WA_LOG2E;
   const int ti = tid / a.ww, tj = tid % a.ww;                    // token `tid` of a window
 
   if (tid < NPAD) {
@@ -507,12 +504,13 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
 #pragma unroll 1
         for (int hh = MT == 1 ? 0 : my_head; hh < (MT == 1 ? HPC : my_head + 1); ++hh) {
           float s[MT][NB][4];
-          wa_start_scores<NPAD, MT>(s, masked, scale2, tab, r0, tq);
+          wa_zero<NPAD, MT>(s);
           wa_mma_nt<HD, NPAD, PITCH, MT>(s, Qs + row0 * PITCH + hh * HD, Ks + hh * HD, lane);
           float mx[MT][2], inv[MT][2];
 #pragma unroll
           for (int t = 0; t < MT; ++t) mx[t][0] = mx[t][1] = -1e30f;
-          wa_scores<NPAD, WW, MT>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, r0, tq, N, mx);
+          if (masked) wa_scores<NPAD, WW, MT, true>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, tab, r0, tq, N, mx);
+          else wa_scores<NPAD, WW, MT, false>(s, scale2, bias_s + hh * geo.nrel, rel0, cofs, tab, r0, tq, N, mx);
 #pragma unroll
           for (int t = 0; t < MT; ++t) wa_softmax<NPAD>(s[t], mx[t][0], mx[t][1], inv[t][0], inv[t][1]);
           // O = P V with the numerators as P, the row normalisation applied to the (smaller) output; staged over this
@@ -538,9 +536,11 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
       if (row0 < N) {
         float s1[1][NB][4], dp1[1][NB][4], mx[1][2] = {{-1e30f, -1e30f}}, inv0, inv1;
         float(&s)[NB][4] = s1[0], (&dp)[NB][4] = dp1[0];
-        wa_start_scores<NPAD, 1>(s1, masked, scale2, tab, r0, tq);
+        wa_zero<NPAD, 1>(s1);
         wa_mma_nt<HD, NPAD, PITCH, 1>(s1, Qs + row0 * PITCH, Ks, lane);
-        wa_scores<NPAD, WW, 1>(s1, scale2, bias_s, rel0, cofs, r0, tq, N, mx);
+        // (128 channels: with both forms of constant offsets the compiler spills, 655 / 710 us; WW = 0 reads them, and spares registers)
+        if (masked) wa_scores<NPAD, HD < 128 ? WW : 0, 1, true>(s1, scale2, bias_s, rel0, cofs, tab, r0, tq, N, mx);
+        else wa_scores<NPAD, WW, 1, false>(s1, scale2, bias_s, rel0, cofs, tab, r0, tq, N, mx);
         wa_softmax<NPAD>(s, mx[0][0], mx[0][1], inv0, inv1);
         wa_zero<NPAD, 1>(dp1);
         wa_mma_nt<HD, NPAD, PITCH, 1>(dp1, dOs + row0 * PITCH, Vs, lane);        // dP = dO V^T

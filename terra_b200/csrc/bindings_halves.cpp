@@ -110,12 +110,27 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 // epilogues through the lanes, were 3.7 % slower than the best on average. Us, those plans / this: 17280 rows of 1024 x 1024 44 / 32, 40000 of 3072 x 1024
 // with sums 220 / 186, 139264 of 1536 x 384 134 / 120, of 768 x 768 with sums 169 / 125, 156672 of 3072 x 1024 with sums 820 / 730.
 //
-// Among plans within 3 % the one with most parts is taken, and a part is longer than 32 k-blocks only where 128 x 256 tiles in one round would have it
-// so: the error of the tensor core's fp32 sums grows with their length (128 k-blocks 8.6e-6 of the norm, 192 13e-6).
+// The error of the tensor core's fp32 sums grows with their length (1.0e-6 of the norm at 15 k-blocks, 8.6e-6 at 128, 13e-6 at 192). So among
+// plans within 3 % the one with most parts is taken; a part is longer than 32 k-blocks only where 128 x 256 tiles in one round would have it
+// so; and it is no longer than 15 k-blocks or what the tiles that cover the outputs with least padding have in one round, where that costs
+// no more than 15 %. Without the last of these one size in fifty had parts twice as long as with the 256-row tiles it took before. Error
+// and us, without / with: 557056 rows of 192 x 192 8.4e-6 / 4.0e-6 and 67.5 / 67.7, 156672 of 768 x 192 7.2e-6 / 3.4e-6 and 52.7 / 53.3,
+// 17280 of 1024 x 1024 4.7e-6 / 2.0e-6 and 30.3 / 30.3; at worst 36228 of 256 x 256 1.1e-6 / 0.6e-6 and 10.8 / 12.5. Shorter parts
+// for all that would take them within 15 % cost 139264 rows of 1152 x 384 7 % for what no size had before.
 struct WgradPlan {
   int bn, stack, split;
   bool swapped;      // the transpose: rows are x's columns
 };
+// How many of the tiles of 128 or 256 rows and 128, 192 or 256 columns it takes that cover N x K outputs with least padding (the fewest of such).
+int64_t covering_tiles(int64_t N, int64_t K) {
+  int64_t least = 0, tiles = 0;
+  for (int64_t h : {256, 128})
+    for (int64_t w : {256, 192, 128}) {
+      const int64_t count = (N + h - 1) / h * ((K + w - 1) / w), area = count * h * w;
+      if (tiles == 0 || area < least || (area == least && count < tiles)) least = area, tiles = count;
+    }
+  return tiles;
+}
 WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   struct Tile {
     int request, stack;
@@ -131,6 +146,7 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   const bool pairs = tb::gemm_pairs() && sms >= 2;
   struct Choice {
     WgradPlan plan;
+    int64_t length;
     double time;
   };
   std::vector<Choice> choices;
@@ -153,7 +169,7 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
         const double full = std::min(1.0, static_cast<double>(count * split) / units);
         const double time = rounds * (per * (t.kblock * (0.77 + 0.23 * full) + sum_cost) + t.tile) + (pair ? 1.3 : 0.0) +
                             0.008 * 4e-6 * count * split * high * 128 * std::min<int64_t>(width, cols) + 3.4 + (fused || (swapped && ones_row) ? 0.0 : separate);
-        choices.push_back({{t.request, t.stack, static_cast<int>(split), swapped}, time});
+        choices.push_back({{t.request, t.stack, static_cast<int>(split), swapped}, per, time});
       }
     }
   }
@@ -163,6 +179,14 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   for (const Choice& c : choices)
     if (c.time <= 1.03 * least && (best == nullptr || c.plan.split > best->plan.split || (c.plan.split == best->plan.split && c.time < best->time)))
       best = &c;
+  const int64_t parts = std::max<int64_t>(1, sms / covering_tiles(N, K)), longest = std::max<int64_t>(15, (k_blocks + parts - 1) / parts);
+  if (best->length > longest) {      // the cheapest of those that keep to it, else the shortest parts
+    for (const Choice& c : choices) {
+      if (c.time > 1.15 * least) continue;
+      const int64_t a = std::max(c.length, longest), b = std::max(best->length, longest);
+      if (a < b || (a == b && c.time < best->time)) best = &c;
+    }
+  }
   return best->plan;
 }
 WgradPlan plan_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {

@@ -720,7 +720,8 @@ int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, 
 // 256 104 / 85, 17280 of 192 25 / 21; transposed, 139264 of 384 186 / 161, of 192 69 / 57, of 96 45 / 35. (Of 96 and 128 channels the row of ones
 // costs a tile in ten: 17280 pixels 12.6 / 13.5 and 16.4 / 17.2; folding the gradients takes 2 to 10 us less than it did.)
 // `least_split`: the contraction is cut into so many parts at least (the error of the tensor core's fp32 sums grows with their length: 139264
-// pixels of 384 channels, 18 parts 8.6e-6, 12 parts 13.0e-6), unless they are down to 24 k-blocks (1.6e-6).
+// pixels of 384 channels, 18 parts 8.6e-6, 12 parts 13.0e-6), unless they are down to 15 k-blocks (1.0e-6; down to 24, 1.6e-6, is no
+// faster: 2656 pixels of 384 channels 15.9 / 15.1 us, 600 to every second 14.5 / 14.2).
 static TapPlan model_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool row_sums, bool column_sums, int least_split, int num_sms) {
   struct Tile {
     int width, ctas, stack;
@@ -728,7 +729,7 @@ static TapPlan model_tap_wgrad(int taps, int channels, int N, long long k_blocks
   };
   static const Tile tiles[] = {{128, 1, 1, 0.269, 1.56}, {192, 1, 1, 0.321, 1.92}, {128, 1, 2, 0.495, 3.34}, {192, 1, 2, 0.502, 4.65},
                                {256, 2, 1, 0.334, 2.84}, {384, 2, 1, 0.461, 5.38}};
-  least_split = static_cast<int>(std::min<long long>(least_split, (k_blocks + 23) / 24));
+  least_split = static_cast<int>(std::min<long long>(least_split, (k_blocks + 14) / 15));
   const long long boxes = static_cast<long long>(taps) * ((channels + 63) / 64) + (row_sums ? 1 : 0);
   TapPlan best = {128, 1, 1, 1};
   double least = -1.0;

@@ -16,6 +16,16 @@ def test_linear_layers(M, N, K, sums, longest):
     assert -(-k_blocks // _ext.load().wgrad_plan(N, K, M, sums)[2]) <= longest
 
 
+@pytest.mark.parametrize("B,H,W,stride,C", [(2, 40, 30, 2, 384), (1, 31, 248, 2, 384), (1, 16, 166, 1, 384), (2, 12, 21, 1, 1024), (1, 512, 1088, 1, 384)])
+def test_convolutions_keep_the_least_number_of_parts_down_to_15_k_blocks(B, H, W, stride, C):
+    from terra_b200 import _ext
+    from terra_b200.ops.conv import _wgrad_split
+
+    k_blocks, parts = B * -(-H // stride) * -(-(W // stride) // 64), _wgrad_split(B, H, W, stride, C, C)[0]
+    split = _ext.load().tap_wgrad_plan(9, C, C, k_blocks, True, False, parts)[3]
+    assert -(-k_blocks // split) <= max(15, -(-k_blocks // parts))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,sums,longest", LINEAR[:4])
 def test_error(M, N, K, sums, longest):

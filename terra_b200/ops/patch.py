@@ -71,9 +71,10 @@ def unpatchify_add(patches, x, p, top, left):
 # ------------------------------------------------------------------------------------------------ without the copies (inference)
 def direct_patches_apply(x: torch.Tensor, p, top, left, dim) -> bool:
     """Whether the patch layers may read and write the field ``x`` itself, in a call that keeps nothing for a backward pass: whole patches
-    inside the image and outside it, runs of whole 16-byte vectors, the product's tables and phases."""
+    inside the image and outside it, runs of whole 16-byte vectors from an address of such (tensor maps need one; the copies take any), the
+    product's tables and phases."""
     _, H, W, C = x.shape
-    return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0 and blocks.native_node()
+    return (x.data_ptr() % 16 == 0 and not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0 and blocks.native_node()
             and 1 <= p <= 4 and H % p == W % p == top % p == left % p == 0 and p * C % 8 == 0 and dim % 8 == 0
             and p * ((p * C + 63) // 64) <= 128 and (dim + 63) // 64 <= 128 and _ext.load().gemm_tma_epilogue())
 

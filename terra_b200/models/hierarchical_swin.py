@@ -21,7 +21,7 @@ from ..global_env_config import ON_H200
 from ..memory.activation import activation_checkpoint, activation_config_for_sampling
 from ..ops import blocks as B
 from ..ops.conv import conv3x3, conv_transpose2x2, groupnorm_silu
-from ..ops.patch import direct_patches_apply, embed_image, pad_patchify, patch_kernels_apply, recover_image, unpatchify_add
+from ..ops.patch import ImageField, direct_patches_apply, pad_patchify, patch_kernels_apply, unpatchify_add
 from ..parallel.context import ParallelContext
 from ..profiler.memory_timeline import mark_memory_timeline
 from ..utils.padding import get_padded_shape
@@ -116,6 +116,8 @@ class _SwinBase(nn.Module):
 
     def _patch_embed(self, patches):
         def run(patches):
+            if isinstance(patches, ImageField):
+                return patches.embed(self._embed_linear())
             Bn, h, w, F = patches.shape
             y = B.linear(patches.reshape(-1, F), self._embed_linear(), need_dx=patches.requires_grad)
             return y.reshape(Bn, h, w, -1)
@@ -149,6 +151,8 @@ class _SwinBase(nn.Module):
 
     def _patch_recovery(self, x, residual=None):
         def run(x, residual):
+            if isinstance(residual, ImageField):
+                return residual.recover(x, self._recovery_linear())
             Bn, h, w, D = x.shape
             res = None if residual is None else residual.reshape(Bn * h * w, -1)
             y = B.linear(x.reshape(-1, D), self._recovery_linear(), residual=res)
@@ -205,13 +209,19 @@ class _SwinBase(nn.Module):
         return out
 
     def _core(self, patches, residual):
-        """patches / residual: [B, h_loc, w, p*p*C] (residual may be None) -> same shape."""
+        """patches / residual: [B, h_loc, w, p*p*C] (residual may be None) -> same shape; an ``ImageField`` for both -> the image and the
+        patches in it added up."""
         Bn = patches.shape[0]
         x = self._run_patch_embed_down(patches)
         rows = self.pctx.stripe_to_windows(x)
         rows = self.layers(rows)
         x = self.pctx.windows_to_stripe(rows, Bn)
         return self._run_up_patch_recovery(x, residual)
+
+    def _own_pieces(self) -> bool:
+        """Whether the pieces that patches go through are those above (one put in their place expects tensors)."""
+        return all(getattr(type(self), n) is getattr(_SwinBase, n) and n not in self.__dict__
+                   for n in ("_core", "_run_patch_embed_down", "_run_up_patch_recovery", "_patch_embed", "_patch_recovery"))
 
     def _compute_dtype(self, x):
         return torch.bfloat16 if x.is_cuda else torch.float32
@@ -253,10 +263,11 @@ class SequentialHierarchicalSwin(_SwinBase):
         fits = (raw_h + top + bottom, raw_w + left + right) == tuple(self.padded_shape)
         if fits and patch_kernels_apply(xin, self.padded_shape):
             p = self.patch_size
-            if direct_patches_apply(xin, p, top, left, self.embedding_dim):
-                y = self._forward_image(xin, top, left)
-                return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y
-            y = unpatchify_add(self._core(pad_patchify(xin, p, self.padded_shape, top, left), None), xin, p, top, left)
+            if direct_patches_apply(xin, p, top, left, self.embedding_dim) and self._own_pieces():
+                field = ImageField(xin, p, self.padded_shape, top, left)
+                y = self._core(field, field)
+            else:
+                y = unpatchify_add(self._core(pad_patchify(xin, p, self.padded_shape, top, left), None), xin, p, top, left)
             return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y
         if self.need_padding:
             xin = torch.nn.functional.pad(xin, (0, 0, left, right, top, bottom))
@@ -266,23 +277,6 @@ class SequentialHierarchicalSwin(_SwinBase):
             y = y[:, top:top + raw_h, left:left + raw_w, :]
         y = y + x.to(y.dtype)
         return y.permute(0, 3, 1, 2).contiguous() if self.input_nchw else y
-
-
-    def _forward_image(self, xin, top, left):
-        """``_core`` where nothing is kept for a backward pass (recomputation has no part in it): patch layers on the image itself."""
-        p = self.patch_size
-        mark_memory_timeline("sampling_down_enter", "none")
-        x = self._in_unit(self.patch_embed, lambda t: embed_image(t, self._embed_linear(), p, self.padded_shape, top, left), xin)
-        if self.has_sampling:
-            x = self._down_block(x)
-        mark_memory_timeline("sampling_down_exit", "none")
-        x = self.pctx.windows_to_stripe(self.layers(self.pctx.stripe_to_windows(x)), xin.shape[0])
-        mark_memory_timeline("sampling_up_enter", "none")
-        if self.has_sampling:
-            x = self._up_block(x)
-        y = self._in_unit(self.patch_recovery, lambda t, r: recover_image(t, self._recovery_linear(), r, p, top, left), x, xin)
-        mark_memory_timeline("sampling_up_exit", "none")
-        return y
 
 
 class SequentialSwinReference(SequentialHierarchicalSwin):

@@ -94,6 +94,23 @@ def _pack_recover_bias(b, p):
     return torch.nn.functional.pad(b.view(p, run), (0, -run % 64)).reshape(-1)
 
 
+class ImageField:
+    """A field whose patches and their layers are taken from the image itself, in the place of its patches (``direct_patches_apply``)."""
+
+    def __init__(self, image, p, padded_shape, top, left):
+        self.image, self.p, self.padded_shape, self.top, self.left = image, p, padded_shape, top, left
+
+    @property
+    def shape(self):
+        return (self.image.shape[0], self.padded_shape[0] // self.p, self.padded_shape[1] // self.p, self.p * self.p * self.image.shape[3])
+
+    def embed(self, lin):
+        return embed_image(self.image, lin, self.p, self.padded_shape, self.top, self.left)
+
+    def recover(self, t, lin):
+        return recover_image(t, lin, self.image, self.p, self.top, self.left)
+
+
 def embed_image(x, lin, p, padded_shape, top, left):
     """``linear(pad_patchify(x))`` for ``direct_patches_apply`` fields: ``[B, rows, cols, N]``."""
     w16, y = lin.weight.bf16, torch.empty(x.shape[0], padded_shape[0] // p, padded_shape[1] // p, lin.weight.shape[0], device=x.device, dtype=x.dtype)

@@ -38,3 +38,50 @@ def test_a_field_at_any_address(offset):
         free = m(x)
     check_status("cuda")
     assert _close(free, kept)
+
+
+def _marks(monkeypatch, m, x, grad):
+    from terra_b200.models import hierarchical_swin
+
+    seen = []
+    monkeypatch.setattr(hierarchical_swin, "mark_memory_timeline", lambda phase, label="", **more: seen.append((phase, label)))
+    with torch.set_grad_enabled(grad):
+        y = m(x)
+    return y, seen
+
+
+@pytest.mark.parametrize("modes", [{}, dict(checkpoint_down_mode="D0", checkpoint_up_mode="U1"), dict(checkpoint_down_mode="D1", checkpoint_up_mode="U0")])
+@pytest.mark.parametrize("mode", ["none", "torch", "boundary_offload"])
+def test_checkpoint_modes_and_their_marks(monkeypatch, modes, mode):
+    m = _model(recompute_config=dict(enabled=True, mode=mode, **modes))
+    kept, marks = _marks(monkeypatch, m, _field(), True)
+    free, same = _marks(monkeypatch, m, _field(), False)
+    assert same == marks and len(marks) >= 4 and _close(free, kept)
+
+
+@pytest.mark.parametrize("key", ["checkpoint_down_mode", "checkpoint_up_mode"])
+def test_an_unknown_checkpoint_mode_is_refused(key):
+    m = _model(recompute_config=dict(enabled=True, **{key: "X9"}))
+    with torch.no_grad(), pytest.raises(ValueError):
+        m(_field())
+
+
+@pytest.mark.parametrize("name", ["_core", "_run_patch_embed_down", "_run_up_patch_recovery", "_patch_embed", "_patch_recovery"])
+@pytest.mark.parametrize("bound", [False, True])
+def test_pieces_put_in_place_of_the_model_s_own(name, bound):
+    from terra_b200.models.hierarchical_swin import SequentialHierarchicalSwin
+
+    called = []
+
+    def piece(self, *args):
+        called.append([type(a) for a in args if a is not None])
+        return getattr(super(Mine, self), name)(*args)
+
+    Mine = type("Mine", (SequentialHierarchicalSwin,), {} if bound else {name: piece})
+    m = _model(Mine)
+    if bound:
+        setattr(m, name, lambda *args: piece(m, *args))
+    with torch.no_grad():
+        y = m(_field())
+    assert called and all(t is torch.Tensor for types in called for t in types)
+    assert _close(y, _model()(_field()))

@@ -10,7 +10,7 @@ import torch
 
 # Packed operands are functions of the bf16 working copy of a weight, which changes once per optimizer step. They are
 # cached per parameter and rebuilt when the parameter's version counter (bumped by the in-place optimizer update of the
-# master, or by a checkpoint load) or the working copy's address (arena rebinding) has moved.
+# master, or by a checkpoint load), the working copy's own or its address (arena rebinding) has moved.
 _PACK_CACHE = {}
 
 
@@ -18,7 +18,7 @@ def _packed(weight, w16, kind, builder):
     import weakref
 
     key = (id(weight), kind)
-    stamp = (weight._version, w16.data_ptr(), PACK_EPOCH[0])
+    stamp = (weight._version, w16.data_ptr(), w16._version, PACK_EPOCH[0])
     hit = _PACK_CACHE.get(key)
     if hit is not None and hit[0] == stamp and hit[2]() is weight:
         return hit[1]

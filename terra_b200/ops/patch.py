@@ -111,10 +111,17 @@ class ImageField:
         return recover_image(t, lin, self.image, self.p, self.top, self.left)
 
 
+def _operand(param, kind, build):
+    """The packed form of a parameter; of a graph's capture, packed by the graph, whose replays read the parameters of their time."""
+    if torch.cuda.is_current_stream_capturing():
+        return build(param.bf16)
+    return _packed(param, param.bf16, kind, build)
+
+
 def embed_image(x, lin, p, padded_shape, top, left):
     """``linear(pad_patchify(x))`` for ``direct_patches_apply`` fields: ``[B, rows, cols, N]``."""
-    w16, y = lin.weight.bf16, torch.empty(x.shape[0], padded_shape[0] // p, padded_shape[1] // p, lin.weight.shape[0], device=x.device, dtype=x.dtype)
-    _ext.load().embed_image(x, _packed(lin.weight, w16, f"embed{p}", lambda w: _pack_embed(w, p)), lin.bias.bf16, y, p, top // p, left // p,
+    y = torch.empty(x.shape[0], padded_shape[0] // p, padded_shape[1] // p, lin.weight.shape[0], device=x.device, dtype=x.dtype)
+    _ext.load().embed_image(x, _operand(lin.weight, f"embed{p}", lambda w: _pack_embed(w, p)), lin.bias.bf16, y, p, top // p, left // p,
                             status_word(x.device))
     return y
 
@@ -122,7 +129,7 @@ def embed_image(x, lin, p, padded_shape, top, left):
 def recover_image(t, lin, x, p, top, left):
     """``unpatchify_add(linear(t), x)`` for ``direct_patches_apply`` fields; the sum is rounded once."""
     out = torch.empty_like(x)
-    w = _packed(lin.weight, lin.weight.bf16, f"recover{p}", lambda v: _pack_recover(v, p))
-    b = _packed(lin.bias, lin.bias.bf16, f"recover{p}", lambda v: _pack_recover_bias(v, p))
+    w = _operand(lin.weight, f"recover{p}", lambda v: _pack_recover(v, p))
+    b = _operand(lin.bias, f"recover{p}", lambda v: _pack_recover_bias(v, p))
     _ext.load().recover_image(t.contiguous(), w, b, x, out, p, top // p, left // p, status_word(x.device))
     return out

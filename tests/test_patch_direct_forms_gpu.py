@@ -21,6 +21,12 @@ def _field(offset=0):
     return flat[offset:offset + 64 * 96 * 10].view(1, 64, 96, 10)
 
 
+def _unaligned(x):
+    """``x`` at an address that the copies take"""
+    flat = torch.empty(x.numel() + 8, device="cuda", dtype=x.dtype)
+    return flat[1:1 + x.numel()].view(x.shape).copy_(x)
+
+
 def _close(a, b):
     return ((a.double() - b.double()).norm() <= 2e-2 * b.double().norm()).item()
 
@@ -85,3 +91,38 @@ def test_pieces_put_in_place_of_the_model_s_own(name, bound):
         y = m(_field())
     assert called and all(t is torch.Tensor for types in called for t in types)
     assert _close(y, _model()(_field()))
+
+
+def _linears(model):
+    return model._embed_linear(), model._recovery_linear()
+
+
+def test_weights_changed_in_the_working_copy():
+    from terra_b200.models.hierarchical_swin import SequentialSwinReference
+
+    m, x = _model(SequentialSwinReference), _field()
+    with torch.no_grad():
+        m(x)
+        for lin in _linears(m):
+            for p in lin.parameters():
+                p.bf16.mul_(-0.5)
+        assert _close(m(x), m(_unaligned(x)))
+
+
+def test_a_captured_call_reads_the_weights_of_its_replay():
+    from terra_b200.models.hierarchical_swin import SequentialSwinReference
+
+    m, x = _model(SequentialSwinReference), _field()
+    with torch.no_grad():
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            m(x)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = m(x)
+        for lin in _linears(m):
+            for p in lin.parameters():
+                p.bf16.mul_(-0.5)
+        graph.replay()
+        assert _close(y, m(_unaligned(x)))

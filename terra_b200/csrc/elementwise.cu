@@ -6,6 +6,7 @@
 #include "chained_launch.cuh"
 #include "common.cuh"
 #include "host_api.h"
+#include "shared_limit.h"
 
 namespace tb {
 
@@ -1237,11 +1238,8 @@ static int ln_bwd_launch(const __nv_bfloat16* dy, const __nv_bfloat16* x, const 
                          cudaStream_t stream) {
   const size_t bytes = std::max<size_t>(4 * (SUMS ? 3 : 2) * C * sizeof(float), static_cast<size_t>(RES ? 3 : 2) * VPL * ln_bwd_ahead(VPL) * 128 * 16);
   auto kernel = layernorm_bwd_kernel<LPR, VPL, EXACT, RES, SUMS>;
-  static std::atomic<bool> configured{false};      // (more than the 48 KB that every launch may have)
-  if (bytes > 48 * 1024 && !configured.load(std::memory_order_relaxed)) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess) return -3;
-    configured.store(true, std::memory_order_relaxed);
-  }
+  static SharedLimit limit;
+  if (bytes > 48 * 1024 && limit.raise(reinterpret_cast<const void*>(kernel), 112 * 1024) != cudaSuccess) return -3;
   launch_chained(kernel, grid_for(rows, 4 * (32 / LPR), ln_bwd_blocks(VPL, rows)), 128, bytes, stream, dy, x, gamma, mean, rstd, dx, dgamma,
                  dbeta, dres, rows, C, dsum);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

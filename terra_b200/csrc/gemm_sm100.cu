@@ -32,6 +32,7 @@
 #include <type_traits>
 #include "chained_launch.cuh"
 #include "gemm_sm100.cuh"
+#include "shared_limit.h"
 
 namespace tb {
 
@@ -1236,13 +1237,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 template <int BN, int CTAS, bool PEERS = false, int STACK = 1>
 static cudaError_t launch_bn(const GemmParams& p_in, int num_sms, cudaStream_t stream) {
   using Cfg = GemmCfg<BN, CTAS, STACK>;
-  static std::atomic<bool> configured{false};      // (the backward pass launches without the interpreter's lock)
-  if (!configured.load(std::memory_order_relaxed)) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg::MAX_SMEM);
-    if (e != cudaSuccess) return e;
-    configured.store(true, std::memory_order_relaxed);
-  }
+  static SharedLimit limit;      // (the backward pass launches without the interpreter's lock)
+  const cudaError_t raised = limit.raise(reinterpret_cast<const void*>(gemm_tcgen05_kernel<BN, CTAS, PEERS, STACK>), Cfg::MAX_SMEM);
+  if (raised != cudaSuccess) return raised;
   GemmParams p = p_in;
   if (PEERS || (STACK > 1 && p.epi_tma != 3) || (p.epi_tma == 3 && Cfg::stages_for(2) < 3)) p.epi_tma = 0;
   // (a long contraction hides the epilogue behind its main loop and wants the deeper ring: one buffer for input and output)

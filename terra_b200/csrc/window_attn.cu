@@ -35,6 +35,7 @@
 #include "chained_launch.cuh"
 #include "common.cuh"
 #include "host_api.h"
+#include "shared_limit.h"
 #include "window_geo.cuh"
 
 namespace tb {
@@ -686,11 +687,12 @@ int launch(WindowAttnArgs a, cudaStream_t stream) {
   const size_t sb = Cfg::bytes(nrel);
   if (sb > 227 * 1024) return -20;
   auto kernel = window_attn_kernel<HD, NPAD, HPC, WW, BWD>;
+  static SharedLimit limit;
+  if (limit.raise(reinterpret_cast<const void*>(kernel), 227 * 1024) != cudaSuccess) return -21;
   // resident CTAs per SM for the last shared-memory size seen (one word, so that threads read a matching pair)
   static std::atomic<unsigned long long> known{0};
   unsigned long long k = known.load(std::memory_order_relaxed);
   if ((k >> 8) != sb) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return -21;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, Cfg::THREADS, sb) != cudaSuccess || occ < 1) occ = 1;
     k = (static_cast<unsigned long long>(sb) << 8) | static_cast<unsigned long long>(occ);

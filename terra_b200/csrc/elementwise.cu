@@ -1314,12 +1314,14 @@ static bool gn_small(int B, long long HW, int C) { return static_cast<long long>
 
 // [2][C] sums of the block, and 16 per thread where the threads' rings were. Beyond the 48 KB that every launch may have the kernel is asked for more.
 constexpr int GN_MAX_CHANNELS = 6144;
-template <class Ring, class Kernel>
-static size_t gn_smem(Kernel kernel, const GnShape& s, int C) {
+template <class Ring>
+static size_t gn_smem(const GnShape& s, int C) {
   const int threads = s.block.x * s.block.y;
-  const size_t bytes = 2 * static_cast<size_t>(C) * sizeof(float) + std::max<size_t>(16 * sizeof(float) * threads, Ring::bytes(threads));
-  if (bytes > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-  return bytes;
+  return 2 * static_cast<size_t>(C) * sizeof(float) + std::max<size_t>(16 * sizeof(float) * threads, Ring::bytes(threads));
+}
+template <class Kernel>
+static bool gn_limit(SharedLimit& limit, Kernel kernel, size_t bytes) {
+  return bytes <= 47 * 1024 || limit.raise(reinterpret_cast<const void*>(kernel), 160 * 1024) == cudaSuccess;
 }
 
 static int groupnorm_stats_launch(const void* x, float* sums, int B, long long HW, int C, int groups, float* stats, unsigned int* ticket,
@@ -1329,8 +1331,10 @@ static int groupnorm_stats_launch(const void* x, float* sums, int B, long long H
   // is L2-sized the passes over it are shorter than that, and one block per SM is enough (us, 1 / 3 blocks per SM: 64800 x 192 13 / 21,
   // 139264 x 128 15 / 22, 139264 x 256 20 / 23, 139264 x 384 52 / 29).
   const GnShape s(B, HW, C, 512, gn_small(B, HW, C) ? 1 : 3, 2);
-  launch_chained(groupnorm_stats_kernel, s.grid, s.block, gn_smem<GnStatsRing>(groupnorm_stats_kernel, s, C), stream, static_cast<const __nv_bfloat16*>(x),
-                 sums, HW, C, groups, s.pix, stats, ticket, inv_count, eps);
+  const size_t bytes = gn_smem<GnStatsRing>(s, C);
+  static SharedLimit limit;
+  if (!gn_limit(limit, groupnorm_stats_kernel, bytes)) return -3;
+  launch_chained(groupnorm_stats_kernel, s.grid, s.block, bytes, stream, static_cast<const __nv_bfloat16*>(x), sums, HW, C, groups, s.pix, stats, ticket, inv_count, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {
@@ -1359,7 +1363,10 @@ int groupnorm_silu_bwd_reduce(const void* dy, const void* x, const float* stats,
   if (!gn_sizes_ok(B, HW, C, groups) || C > GN_MAX_CHANNELS) return -1;
   const bool tiny = static_cast<long long>(B) * HW * C <= 1500000LL;      // (not enough pixels for larger blocks)
   const GnShape s(B, HW, C, tiny ? 256 : 512, tiny ? 2 : 1, 2);
-  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, gn_smem<GnPairRing>(groupnorm_silu_bwd_reduce_kernel, s, C), stream,
+  const size_t bytes = gn_smem<GnPairRing>(s, C);
+  static SharedLimit limit;
+  if (!gn_limit(limit, groupnorm_silu_bwd_reduce_kernel, bytes)) return -3;
+  launch_chained(groupnorm_silu_bwd_reduce_kernel, s.grid, s.block, bytes, stream,
                  static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
                  static_cast<const __nv_bfloat16*>(beta), red, HW, C, groups, s.pix, dgamma, dbeta);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -41,3 +41,11 @@ def test_once_per_device(tmp_path):
     src.write_text(PROGRAM)
     subprocess.run(["g++", "-std=c++17", "-I", _ext.CSRC, "-I", os.path.join(CUDA_HOME, "include"), "-o", exe, src], check=True)
     assert subprocess.run([exe], capture_output=True, text=True, check=True).stdout.strip() == "ok"
+
+
+def test_every_limit_of_a_common_launch_goes_through_it():
+    from terra_b200 import _ext
+
+    for name in ("elementwise.cu", "gemm_sm100.cu", "window_attn.cu"):
+        with open(os.path.join(_ext.CSRC, name)) as f:
+            assert "cudaFuncSetAttribute" not in f.read(), name

@@ -1407,8 +1407,10 @@ int groupnorm_silu_bwd_apply(const void* dy, const void* x, const float* stats, 
                              cudaStream_t stream) {
   if (!gn_sizes_ok(B, HW, C, groups)) return -1;
   const GnShape s(B, HW, C, 256, gn_small(B, HW, C) ? 2 : 4, 2);
-  launch_chained(groupnorm_silu_bwd_apply_kernel, s.grid, s.block,
-                 (groups * 2 + 3) / 4 * 4 * sizeof(float) + GnPairRing::bytes(s.block.x * s.block.y), stream,
+  const size_t bytes = (groups * 2 + 3) / 4 * 4 * sizeof(float) + GnPairRing::bytes(s.block.x * s.block.y);
+  static SharedLimit limit;
+  if (!gn_limit(limit, groupnorm_silu_bwd_apply_kernel, bytes)) return -3;
+  launch_chained(groupnorm_silu_bwd_apply_kernel, s.grid, s.block, bytes, stream,
                  static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, red, static_cast<const __nv_bfloat16*>(gamma),
                  static_cast<const __nv_bfloat16*>(beta), static_cast<__nv_bfloat16*>(dx), HW, C, groups, inv_count, s.pix);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -298,7 +298,8 @@ struct GroupNormSilu : Function<GroupNormSilu> {
     terra_ops::scratch_give(sums);
     Tensor y = torch::empty_like(x), res;
     if (residual.has_value()) {
-      need(residual->numel() == x.numel() && residual->is_cuda() && residual->scalar_type() == torch::kBFloat16, "groupnorm_silu: shortcut like the input");
+      need(residual->numel() == x.numel() && residual->is_cuda() && residual->scalar_type() == torch::kBFloat16,
+           "groupnorm_silu: shortcut like the input");
       res = residual->contiguous();
     }
     rc_check(tb::groupnorm_silu_apply(x.data_ptr(), stats.data_ptr<float>(), l->g.data_ptr(), l->b.data_ptr(), res.defined() ? res.data_ptr() : nullptr,

@@ -102,13 +102,14 @@ void column_sums(const Tensor& dy, const Tensor& out) {
 // tiles over the CTAs (or pairs: request 1000 + width), each its k-blocks and a hand-over with the epilogue. A k-block costs less where fewer
 // CTAs than there are SMs share L2's bandwidth; the column sums (the bias gradient) are more MMAs, shared out over the column tiles. Widths of
 // 256 and transposed plans have no room for the sums' accumulators, or the wrong operand: there the sums are two launches that read dy once
-// more, or a row of ones behind x's columns where the last pair has room for it (557056 rows of 384 x 2976 1003 / 890 us).
+// more, or rows of ones behind x's columns where the last pair has room for it (557056 rows of 384 x 2976 1003 / 890 us).
 // Transposed: few outputs of a wide layer (patch embedding: 384 x 2976), 384 rows filling one and a half pairs, 384 columns one tile.
 //
-// Fitted to 9000 passes in CUDA graphs: 200 to 557056 rows, 22 pairs of N and K between 96 and 4096, with and without sums, all tiles, half a
-// round to three; the choice is 0.9 % slower than the best plan on average, 9 % at most. The plans of the fit before, which was made with
-// epilogues through the lanes, were 3.7 % slower than the best on average. Us, those plans / this: 17280 rows of 1024 x 1024 44 / 32, 40000 of 3072 x 1024
-// with sums 220 / 186, 139264 of 1536 x 384 134 / 120, of 768 x 768 with sums 169 / 125, 156672 of 3072 x 1024 with sums 820 / 730.
+// Fitted to 9000 passes in CUDA graphs: 200 to 557056 rows, 22 pairs of N and K between 96 and 4096, with and without sums, all tiles, half
+// a round to three; the choice is 0.9 % slower than the best plan on average, 9 % at most. The plans of the fit before, which was made with
+// epilogues through the lanes, were 3.7 % slower than the best on average. Us, those plans / this: 17280 rows of 1024 x 1024 44 / 32, 40000
+// of 3072 x 1024 with sums 220 / 186, 139264 of 1536 x 384 134 / 120, of 768 x 768 with sums 169 / 125, 156672 of 3072 x 1024 with sums 820
+// / 730.
 //
 // The error of the tensor core's fp32 sums grows with their length (1.0e-6 of the norm at 15 k-blocks, 8.6e-6 at 128, 13e-6 at 192). So among
 // plans within 3 % the one with most parts is taken; a part is longer than 32 k-blocks only where 128 x 256 tiles in one round would have it
@@ -142,7 +143,7 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   const int64_t blocks_256 = ((N + 127) / 128) * ((K + 255) / 256);
   const int64_t least_split = std::max<int64_t>(1, std::min((k_blocks + 31) / 32, sms / blocks_256));
   const double separate = sums ? 8.5 + 2e-6 * M * N / 4.71 : 0.0;
-  const bool ones_row = tb::gemm_row_sums_fit(K, 2);      // (of a transposed plan: the sums are a row of ones behind x's columns)
+  const bool ones_row = tb::gemm_row_sums_fit(K, 2);      // (of a transposed plan: the sums are rows of ones behind x's columns)
   const bool pairs = tb::gemm_pairs() && sms >= 2;
   struct Choice {
     WgradPlan plan;
@@ -168,7 +169,8 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
         const int64_t split = (k_blocks + per - 1) / per, rounds = (count * split + units - 1) / units;
         const double full = std::min(1.0, static_cast<double>(count * split) / units);
         const double time = rounds * (per * (t.kblock * (0.77 + 0.23 * full) + sum_cost) + t.tile) + (pair ? 1.3 : 0.0) +
-                            0.008 * 4e-6 * count * split * high * 128 * std::min<int64_t>(width, cols) + 3.4 + (fused || (swapped && ones_row) ? 0.0 : separate);
+                            0.008 * 4e-6 * count * split * high * 128 * std::min<int64_t>(width, cols) + 3.4 +
+                            (fused || (swapped && ones_row) ? 0.0 : separate);
         choices.push_back({{t.request, t.stack, static_cast<int>(split), swapped}, per, time});
       }
     }

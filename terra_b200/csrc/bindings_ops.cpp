@@ -62,18 +62,6 @@ void groupnorm_stats(const torch::Tensor& x, torch::Tensor& sums, int64_t groups
            "groupnorm_stats");
 }
 
-void groupnorm_mean_rstd(const torch::Tensor& x, torch::Tensor& scratch, torch::Tensor& stats, int64_t groups, double inv_count, double eps) {
-  need(x.is_contiguous() && x.dim() == 3 && x.scalar_type() == torch::kBFloat16, "groupnorm_mean_rstd: [B,HW,C] bf16");
-  need(scratch.is_cuda() && scratch.is_contiguous() && stats.is_contiguous() && scratch.scalar_type() == torch::kFloat32 &&
-           stats.scalar_type() == torch::kFloat32 && stats.numel() == 2 * x.size(0) * groups && scratch.numel() == stats.numel() + 1,
-       "groupnorm_mean_rstd: fp32 stats [B, groups, 2] and as many sums and a ticket");
-  const c10::cuda::CUDAGuard guard(x.device());
-  tb::note_launch();
-  rc_check(tb::groupnorm_mean_rstd(x.data_ptr(), scratch.data_ptr<float>(), stats.data_ptr<float>(), x.size(0), x.size(1), x.size(2), groups,
-                                   static_cast<float>(inv_count), static_cast<float>(eps), cur_stream()),
-           "groupnorm_mean_rstd");
-}
-
 void groupnorm_silu_apply(const torch::Tensor& x, const torch::Tensor& stats, const torch::Tensor& g,
                           const torch::Tensor& b, const c10::optional<torch::Tensor>& res, torch::Tensor& y, int64_t groups) {
   need(x.is_contiguous() && x.dim() == 3, "groupnorm_silu_apply: [B,HW,C]");

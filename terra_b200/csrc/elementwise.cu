@@ -48,10 +48,10 @@ __device__ __forceinline__ f32x2 f2_of_bf16x2(uint32_t v) {
   return f2_pack(f.x, f.y);
 }
 
-// A thread's own 16-byte vectors on their way through shared memory: K tensors, S steps ahead, read two steps at a time (instructions of one issue
-// between those of the other). What kernels over HBM lack beside bandwidth is loads in flight: held in registers, a round's loads are issued,
-// waited for and used in turn, while cp.async fetches the next rounds meanwhile and costs no register. Every thread reads only what it fetched,
-// so there is no barrier.
+// A thread's own 16-byte vectors on their way through shared memory: K tensors, S steps ahead, read two steps at a time (instructions of
+// one issue between those of the other). What kernels over HBM lack beside bandwidth is loads in flight: held in registers, a round's loads
+// are issued, waited for and used in turn, while cp.async fetches the next rounds meanwhile and costs no register. Every thread reads only
+// what it fetched, so there is no barrier.
 template <int K, int S>
 struct LaneRing {
   static_assert(S % 2 == 0 && S >= 4, "rounds of two steps");
@@ -92,15 +92,15 @@ struct LaneRing {
 };
 
 // ------------------------------------------------------------------------------------------ LayerNorm
-// Both kernels are bound by HBM. A row is held in registers by LPR lanes of VPL 16-byte vectors each, so that a warp
-// carries 32 / LPR rows: a row of 48 vectors (C = 384) takes 16 lanes x 3 vectors, with no idle lane, where a whole warp
-// would leave half of its lanes idle in the second vector. LPR is the largest power of two that divides the row's
-// vectors; rows of more than 3 odd vectors per lane fall back to 32 lanes with a bounds test. The backward kernel has the next rows on their way
-// through shared memory, reads a row there twice (three blocks of four warps then share an SM), works on two columns per instruction and ends
-// in vector reductions without shared-memory atomics, which are compare-and-swap loops for floats.
+// Both kernels are bound by HBM. A row is held in registers by LPR lanes of VPL 16-byte vectors each, so that a warp carries 32 / LPR rows:
+// a row of 48 vectors (C = 384) takes 16 lanes x 3 vectors, with no idle lane, where a whole warp would leave half of its lanes idle in the
+// second vector. LPR is the largest power of two that divides the row's vectors; rows of more than 3 odd vectors per lane fall back to 32
+// lanes with a bounds test. The backward kernel has the next rows on their way through shared memory, reads a row there twice (three blocks
+// of four warps then share an SM), works on two columns per instruction and ends in vector reductions without shared-memory atomics, which
+// are compare-and-swap loops for floats.
 // 139264 x 384, one row per warp -> this: forward 49 -> 37 us (33 us at 6.5 TB/s). Backward with shortcut, us, rows in registers and scalar
-// atomics / the rest of this / those ends too: 139264 x 384 79 / 69 / 65 (65 at 6.5 TB/s), 156672 x 1024 262 / 204 / 202 (196), 17280 x 192 11.4 / 11.2 / 8.4, 2048 x 384
-// 10.8 / 10.8 / 6.4, 20000 x 512 23.6 / 21.5 / 15.5; with the shortcut's sums 156672 x 1024 380 / 262 / -.
+// atomics / the rest of this / those ends too: 139264 x 384 79 / 69 / 65 (65 at 6.5 TB/s), 156672 x 1024 262 / 204 / 202 (196), 17280 x 192
+// 11.4 / 11.2 / 8.4, 2048 x 384 10.8 / 10.8 / 6.4, 20000 x 512 23.6 / 21.5 / 15.5; with the shortcut's sums 156672 x 1024 380 / 262 / -.
 template <int LPR>
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -419,15 +419,14 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 }
 
 // ------------------------------------------------------------------------------------------ GroupNorm
-// x: [B, HW, C] bf16. Every kernel is one pass over the image, bound by HBM: a block is (column vectors) x (pixels in
-// flight), so a thread's column constants (statistics, affine parameters) are loaded once for all of its pixels, and it
-// keeps several independent 16-byte loads in flight (LaneRing). blockIdx.y is the sample; the pixel range of a sample is split over
-// blockIdx.x so that the grid is about one resident wave. (Before, the apply kernels divided to find every vector's channel
-// and loaded its constants again, and one load per thread was in flight. 557056 pixels x 384, before -> now: statistics
-// 98 -> 90 us, apply with shortcut 355 -> 225, backward sums 366 -> 258, backward apply 406 -> 264; one copy of the image
-// each way at 6.65 TB/s is 129 us. Then, loads in registers -> in shared memory: apply 228 -> 212 with the shortcut and 190 -> 143 without, backward sums 192 -> 160,
-// backward apply 264 -> 199; 17280 x 192, with one wave of blocks for images that stay in L2: 6.4 -> 4.9, 6.0 -> 4.7, 8.6 -> 8.3, 7.3 -> 6.3, statistics
-// 5.0 -> 4.2.)
+// x: [B, HW, C] bf16. Every kernel is one pass over the image, bound by HBM: a block is (column vectors) x (pixels in flight), so a
+// thread's column constants (statistics, affine parameters) are loaded once for all of its pixels, and it keeps several independent 16-byte
+// loads in flight (LaneRing). blockIdx.y is the sample; the pixel range of a sample is split over blockIdx.x so that the grid is about one
+// resident wave. (Before, the apply kernels divided to find every vector's channel and loaded its constants again, and one load per thread
+// was in flight. 557056 pixels x 384, before -> now: statistics 98 -> 90 us, apply with shortcut 355 -> 225, backward sums 366 -> 258,
+// backward apply 406 -> 264; one copy of the image each way at 6.65 TB/s is 129 us. Then, loads in registers -> in shared memory: apply 228
+// -> 212 with the shortcut and 190 -> 143 without, backward sums 192 -> 160, backward apply 264 -> 199; 17280 x 192, with one wave of
+// blocks for images that stay in L2: 6.4 -> 4.9, 6.0 -> 4.7, 8.6 -> 8.3, 7.3 -> 6.3, statistics 5.0 -> 4.2.)
 //
 // Adds a thread's 16 sums (s, q of its eight channels) over the block's threadIdx.y and leaves them in sh[c] and sh[C + c]. Every thread of
 // the block takes part. Through a buffer of the block's own rather than by shared-memory atomics, which
@@ -756,9 +755,9 @@ __global__ void __launch_bounds__(256) fold_taps_kernel(float* __restrict__ src,
         dst[(static_cast<long long>(c0 + warp + 8 * k) * rows + r0) * taps + lane + 32 * i] = old[k][i] + tile[warp + 8 * k][lane + 32 * i];
 }
 
-// out[p][b][a][r] = in[p][a][b][r] (16-byte vectors): image rows of windows to windows of rows and back. Bound by HBM: four vectors a thread, all asked
-// for before the first is stored. Against the tensor operators' copy, which moves two bytes per lane, cold: 23040 x 192 18.4 -> 10.2 us, 139264 x 384
-// 141.2 -> 38.9 us (5.5 TB/s).
+// out[p][b][a][r] = in[p][a][b][r] (16-byte vectors): image rows of windows to windows of rows and back. Bound by HBM: four vectors a
+// thread, all asked for before the first is stored. Against the tensor operators' copy, which moves two bytes per lane, cold: 23040 x 192
+// 18.4 -> 10.2 us, 139264 x 384 141.2 -> 38.9 us (5.5 TB/s).
 __global__ void __launch_bounds__(256) swap_middle_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, unsigned int A, unsigned int B,
                                                           unsigned int run, unsigned int total) {
   chain_begin();
@@ -995,8 +994,8 @@ __global__ void add_bf16_kernel(const uint4* __restrict__ a, const uint4* __rest
   }
 }
 
-// Packed operands of the implicit GEMMs: out[(n1 * N2 + n2)][t][c] = w[n1 * s1 + n2 * s2 + c * sc + off[t]], zero for
-// c >= C and for n2 >= V2 (rows that only pad). One launch per operand and optimizer step (zero fill, permutation, flip and copy were three to five); the reads
+// Packed operands of the implicit GEMMs: out[(n1 * N2 + n2)][t][c] = w[n1 * s1 + n2 * s2 + c * sc + off[t]], zero for c >= C and for n2 >=
+// V2 (rows that only pad). One launch per operand and optimizer step (zero fill, permutation, flip and copy were three to five); the reads
 // are strided by the taps, which the caches absorb (a weight is at most a few MB).
 struct PackTaps {
   int N2, V2, T, C, Cpad;
@@ -1181,12 +1180,13 @@ int grid_for(long long work_items, int block, int max_blocks = 148 * 16) {
 
 }  // namespace
 
-// CALL sees LPR, VPL and EXACT (see the LayerNorm kernels) for rows of NVEC 16-byte vectors. MANY: rows enough for groups of 32 / LPR
-// of them; below that a row per warp finishes sooner (shorter chains, more warps). The lines are LN_FWD_GROUPS and LN_BWD_GROUPS rows: beyond them a row per
-// warp means several rows one after the other in every warp, each waiting for its loads and its shuffles, and backward as many
-// more blocks that end in atomics on the same sums. Inputs in L2, us, a row per warp / groups. Forward: C = 192, 1024 rows 1.70 / 1.97,
-// 2048 1.88 / 1.98, 4096 2.59 / 2.06, 17280 5.23 / 3.17; 384, 2048 2.33 / 2.13, 17280 7.29 / 5.39; 96, 2048 1.88 / 1.98, 17280 5.17 / 2.41. Backward: 96,
-// 512 2.06 / 2.59, 2048 3.59 / 2.66; 192, 512 2.79 / 2.67, 1024 3.84 / 2.83, 2048 6.21 / 3.41, 8192 7.76 / 6.88; 384, 2048 6.31 / 4.68, 8192 9.09 / 7.95.
+// CALL sees LPR, VPL and EXACT (see the LayerNorm kernels) for rows of NVEC 16-byte vectors. MANY: rows enough for groups of 32 / LPR of
+// them; below that a row per warp finishes sooner (shorter chains, more warps). The lines are LN_FWD_GROUPS and LN_BWD_GROUPS rows: beyond
+// them a row per warp means several rows one after the other in every warp, each waiting for its loads and its shuffles, and backward as
+// many more blocks that end in atomics on the same sums. Inputs in L2, us, a row per warp / groups. Forward: C = 192, 1024 rows 1.70 /
+// 1.97, 2048 1.88 / 1.98, 4096 2.59 / 2.06, 17280 5.23 / 3.17; 384, 2048 2.33 / 2.13, 17280 7.29 / 5.39; 96, 2048 1.88 / 1.98, 17280 5.17 /
+// 2.41. Backward: 96, 512 2.06 / 2.59, 2048 3.59 / 2.66; 192, 512 2.79 / 2.67, 1024 3.84 / 2.83, 2048 6.21 / 3.41, 8192 7.76 / 6.88; 384,
+// 2048 6.31 / 4.68, 8192 9.09 / 7.95.
 constexpr long long LN_FWD_GROUPS = 2048, LN_BWD_GROUPS = 1024;
 #define TB_LN_CASE(L, V, E, ...) { constexpr int LPR = L; constexpr int VPL = V; constexpr bool EXACT = E; __VA_ARGS__; }
 #define TB_LN_DISPATCH(NVEC, MANY, ...)                         \
@@ -1312,7 +1312,8 @@ static bool gn_sizes_ok(int B, long long HW, int C, int groups) {
 // Images that stay in L2 are through before a second wave's blocks have paid for their set-up.
 static bool gn_small(int B, long long HW, int C) { return static_cast<long long>(B) * HW * C * 2 <= 72000000LL; }
 
-// [2][C] sums of the block, and 16 per thread where the threads' rings were. Beyond the 48 KB that every launch may have the kernel is asked for more.
+// [2][C] sums of the block, and 16 per thread where the threads' rings were. Beyond the 48 KB that every launch may have the kernel is
+// asked for more.
 constexpr int GN_MAX_CHANNELS = 6144;
 template <class Ring>
 static size_t gn_smem(const GnShape& s, int C) {
@@ -1334,7 +1335,8 @@ static int groupnorm_stats_launch(const void* x, float* sums, int B, long long H
   const size_t bytes = gn_smem<GnStatsRing>(s, C);
   static SharedLimit limit;
   if (!gn_limit(limit, groupnorm_stats_kernel, bytes)) return -3;
-  launch_chained(groupnorm_stats_kernel, s.grid, s.block, bytes, stream, static_cast<const __nv_bfloat16*>(x), sums, HW, C, groups, s.pix, stats, ticket, inv_count, eps);
+  launch_chained(groupnorm_stats_kernel, s.grid, s.block, bytes, stream, static_cast<const __nv_bfloat16*>(x), sums, HW, C, groups, s.pix, stats,
+                 ticket, inv_count, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 int groupnorm_stats(const void* x, float* sums, int B, long long HW, int C, int groups, cudaStream_t stream) {

@@ -144,17 +144,19 @@ bool gemm_pairs() {
   return on;
 }
 
-// Tile of a plain product or gathered convolution (no peers, no split, no column sums): the width and CTA count with the
-// least time by a model, in us. Persistent CTAs (pairs) take rounds of tiles; a tile takes the longer of its main loop and its
-// epilogue (rounds of 64-column units over the three warps of a lane quadrant, or of 32-column chunks where the lanes store
-// themselves) and a fixed hand-over, and the shorter of the two shows once, before the first or after the last tile. Tiles of 384
-// columns (pairs) have one accumulator: main loop and most of the epilogue follow one another, for 40 KB of operands per k-block where
-// two tiles of 192 read 56 (128 wide, the only even width of a pair with an MN-major B and N = 384: 72).
+// Tile of a plain product or gathered convolution (no peers, no split, no column sums): the width and CTA count with the least time by a
+// model, in us. Persistent CTAs (pairs) take rounds of tiles; a tile takes the longer of its main loop and its epilogue (rounds of
+// 64-column units over the three warps of a lane quadrant, or of 32-column chunks where the lanes store themselves or fp32 sums are
+// accumulated) and a fixed hand-over, and the shorter of the two shows once, before the first or after the last tile. Tiles of 384 columns
+// (pairs) have one accumulator: main loop and most of the epilogue follow one another, for 40 KB of operands per k-block where two tiles of
+// 192 read 56 (128 wide, the only even width of a pair with an MN-major B and N = 384: 72).
 //
 // The constants were fitted to measurements, passes in a CUDA graph at 1.9 GHz, falling to about 1.4 GHz under the
 // power cap in the largest. Products: 512 to 139264 rows, 25 pairs of N and K between 96 and 3072, five epilogues, all seven
-// tiles (3100 times). Convolutions: the five forms, 96 to 384 channels, 16 x 32 to 512 x 1088 pixels (1300 times). The choice is
-// 0.5 % (0.4 %) slower than the best tile on average, more than 10 % in one case of 200. Before the fit and the 384-wide tiles (us, before /
+// tiles (3100 times). Convolutions: the five forms, 96 to 384 channels, 16 x 32 to 512 x 1088 pixels (1300 times). The choice was
+// 0.5 % (0.4 %) slower than the best tile on average, more than 10 % in one case of 200. Since then epilogues with an input or GELU ask for the
+// next unit's operands ahead and take up to a quarter less, which their terms do not know: 34816 x 384 x 384 with residual takes 20.1 us
+// where pairs of 192 columns take 17.1, 34816 x 1536 x 384 with GELU 49.0 / 46.1. Before the fit and the 384-wide tiles (us, before /
 // this, on one GPU): input gradients 139264 x 384 x 1152 118 / 104, 139264 x 384 x 1536 153 / 132, 557056 x 384 x 2976 1113 / 1054;
 // patch embedding 557056 x 384 x 2976 1041 / 931, recovery 557056 x 2976 x 384 1662 / 1576.
 struct TileCosts {
@@ -172,7 +174,7 @@ static void model_tile(long long m_blocks, long long N, int k_blocks, bool b_mn,
   const bool input = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0;
   const double unit = (flags & EPI_MUL_DGELU) ? 2.14 : (flags & EPI_RESIDUAL) ? 1.77 : (flags & (EPI_GELU | EPI_SAVE_PRE)) ? 2.19
                       : (flags & EPI_BIAS) ? cost.bias_unit : cost.plain_unit;
-  const bool by_lane = !gemm_tma_epilogue() || (flags & (EPI_OUT_F32 | EPI_ATOMIC));
+  const bool chunks = !gemm_tma_epilogue() || (flags & (EPI_OUT_F32 | EPI_ATOMIC));
   double least = 0.0;
   for (int ctas : {1, 2}) {
     if (ctas == 2 && (!gemm_pairs() || num_sms < 2)) continue;
@@ -183,9 +185,9 @@ static void model_tile(long long m_blocks, long long N, int k_blocks, bool b_mn,
       const long long tiles = (m_blocks + ctas - 1) / ctas * ((N + bn - 1) / bn), units = num_sms / ctas;
       const long long cols = std::min<long long>(bn, N), rounds = (tiles + units - 1) / units;
       // (single tiles of 256 columns leave no room for the pre-activation's staging buffer beside the operand ring)
-      const bool lanes = by_lane || ((flags & EPI_SAVE_PRE) && !input && bn == 256 && ctas == 1);
+      const bool by_chunk = chunks || ((flags & EPI_SAVE_PRE) && !input && bn == 256 && ctas == 1);
       const double loop = k_blocks * cost.kblock[ctas - 1][w];
-      const double epilogue = unit * (lanes ? ((cols + 31) / 32 + 2) / 3 : ((cols + 63) / 64 + 2) / 3);
+      const double epilogue = unit * (by_chunk ? ((cols + 31) / 32 + 2) / 3 : ((cols + 63) / 64 + 2) / 3);
       double time = cost.start[ctas - 1];
       if (bn == 384) time += rounds * (std::max(loop + epilogue * cost.drain, epilogue) + cost.tile) + (1.0 - cost.drain) * epilogue;
       else time += rounds * (std::max(loop, epilogue) + cost.tile) + cost.tail * std::min(loop, epilogue);
@@ -426,10 +428,10 @@ static int gather_conv(const GatherConv& c, const GemmEpilogue& epi, int num_sms
   // (outputs that go to every second pixel, or into another layout, have no per-lane form)
   const bool strided = c.out_mul != 1 || c.phase_cols != 0;
   const bool tma_out = c.out_layout != nullptr || (!(epi.flags & ~(EPI_BIAS | EPI_BIAS_F32)) && (strided || gemm_tma_epilogue()));
-  // Pixels of a tile: 128 of a row, or 64 of two rows or 32 of four where fewer tiles cover the image so (96 x 180: 144 instead of 192) and rounds of
-  // CTAs can be saved by it. Not where rows come from a neighbour or every second row is read. Us, 128 x 1 / this: 3x3 convolutions of 96 x 180
-  // pixels, 192 channels 21.8 / 14.5, of 2 x 76 x 131, 128 20.1 / 15.7, of 180 x 129, 192 30.6 / 23.2, of 200 x 400, 192 54.8 / 46.9; in one round anyway 50 x 100
-  // pixels of 384 to every second 12.9 / 14.1.
+  // Pixels of a tile: 128 of a row, or 64 of two rows or 32 of four where fewer tiles cover the image so (96 x 180: 144 instead of 192) and
+  // rounds of CTAs can be saved by it. Not where rows come from a neighbour or every second row is read. Us, 128 x 1 / this: 3x3
+  // convolutions of 96 x 180 pixels, 192 channels 21.8 / 14.5, of 2 x 76 x 131, 128 20.1 / 15.7, of 180 x 129, 192 30.6 / 23.2, of 200 x
+  // 400, 192 54.8 / 46.9; in one round anyway 50 x 100 pixels of 384 to every second 12.9 / 14.1.
   int tile_w = GEMM_BM;
   long long m_blocks = 0;
   for (int w = GEMM_BM; w >= 32; w /= 2) {
@@ -555,7 +557,8 @@ int conv3x3_s2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H,
 }
 
 // 2x2 / stride-2 transposed convolution: x [B, H, W, Cin] -> y [B, 2H, 2W, Cout]; w: [4 * Cout_pad, Cin_pad], rows (dy, dx, co);
-// bias: [4 * Cout_pad] (padded to multiples of 64; the padding columns are clipped by the store). One tap, the four output phases side by side in N.
+// bias: [4 * Cout_pad] (padded to multiples of 64; the padding columns are clipped by the store). One tap, the four output phases side by
+// side in N.
 int convt2x2_fwd_bf16(const void* x, const void* w, const void* bias4, void* y, int B, int H, int W, int Cin, int Cout,
                       void* status, int num_sms, cudaStream_t stream) {
   const int pad = (Cout + 63) / 64 * 64;      // a 64-column unit of the epilogue lies inside one phase
@@ -582,9 +585,9 @@ int convt2x2_dgrad_bf16(const void* dy, const void* w, void* dx, int B, int H, i
 }
 
 // Patches of an image [B, H, W, C] (top and left patches of zeros before it, rows x cols of them in all) times w: y [B, rows, cols, N]. A patch's
-// features are p runs of p * C neighbouring elements, one per image row, so that the products read the image itself: 32 bytes of k-block
-// padding per run instead of a copy of the field in patch order. w: [N, p * (p * C padded to 64)].
-// Us, 64800 patches of 16 x 138 features to 192 channels: copy and product 104 + 69, this 68.
+// features are p runs of p * C neighbouring elements, one per image row, so that the products read the image itself: k-block
+// padding (48 bytes a run of 138 or 186 channels) instead of a copy of the field in patch order. w: [N, p * (p * C padded to 64)].
+// Us, 64800 patches of 16 x 138 features to 192 channels: copy and product 104 + 69, this 66.
 int embed_image_bf16(const void* x, const void* w, const void* bias, void* y, int B, int H, int W, int C, int p, int top, int left, int rows,
                      int cols, int N, void* status, int num_sms, cudaStream_t stream) {
   if (p < 1 || p > 4 || H % p != 0 || W % p != 0 || (p * C) % 8 != 0 || N % 8 != 0) return -13;
@@ -605,8 +608,7 @@ int embed_image_bf16(const void* x, const void* w, const void* bias, void* y, in
 
 // The way back: t [B, rows, cols, D] times w, the patches inside the image [B, H, W, C] (top and left of them outside) plus the image x: out. The
 // p runs of a patch are phases side by side in N. w: [p * (p * C padded to 64), D padded to 64], bias alike.
-// Us, 64800 patches of 192 channels: product and copy with the sum 72 + 166, this 170 (floor of the fields 88; the epilogue with a residual takes
-// 3400 cycles a unit).
+// Us, 64800 patches of 192 channels: product and copy with the sum 72 + 166, this 136 (floor of the fields 88).
 int recover_image_bf16(const void* t, const void* w, const void* bias, const void* x, void* out, int B, int H, int W, int C, int p, int top,
                        int left, int rows, int cols, int D, void* status, int num_sms, cudaStream_t stream) {
   if (p < 1 || p > 4 || H % p != 0 || W % p != 0 || (p * C) % 8 != 0 || D % 8 != 0) return -13;
@@ -709,18 +711,18 @@ int convt2x2_wgrad_bf16(const void* x, const void* dy, float* dw, int B, int H, 
 }
 
 // All taps' weight gradients as one product (one rank): the channels of the displaced image, box after box of 64 and tap after tap, are the
-// rows, and the other image's channels the columns, so that tiles of 256 rows need no whole number of them in a tap (9 x 384 rows are 13.5 of
-// a pair's, 9 x 192 seven stacked ones where two per tap made nine). With the undisplaced image as operand B its column sums, the bias gradient of
-// a convolution, are one more box of rows, whose rows of ones share them out (g_ones_rows).
+// rows, and the other image's channels the columns, so that tiles of 256 rows need no whole number of them in a tap (9 x 384 rows are 13.5
+// of a pair's, 9 x 192 seven stacked ones where two per tap made nine). With the undisplaced image as operand B its column sums, the bias
+// gradient of a convolution, are one more box of rows, whose rows of ones share them out (g_ones_rows).
 //
-// The plan is the one with the least time by a model, in us: rounds of tiles over the CTAs (pairs), each its k-blocks and a hand-over with the
-// epilogue. Fitted to 900 passes in CUDA graphs: the two layers at 512 to 557056 pixels, 96 to 384 channels, all tiles, half a round to three
-// and more; the choice is 0.1 % slower than the best plan on average, at most 3 %.
-// Us, a product per tap (two row blocks stacked where that was ahead) / this: 557056 pixels of 384 channels 1251 / 951, of 192 383 / 275, 80000 of
-// 256 104 / 85, 17280 of 192 25 / 21; transposed, 139264 of 384 186 / 161, of 192 69 / 57, of 96 45 / 35. (Of 96 and 128 channels the row of ones
-// costs a tile in ten: 17280 pixels 12.6 / 13.5 and 16.4 / 17.2; folding the gradients takes 2 to 10 us less than it did.)
-// `least_split`: the contraction is cut into so many parts at least (the error of the tensor core's fp32 sums grows with their length: 139264
-// pixels of 384 channels, 18 parts 8.6e-6, 12 parts 13.0e-6), unless they are down to 15 k-blocks (1.0e-6; down to 24, 1.6e-6, is no
+// The plan is the one with the least time by a model, in us: rounds of tiles over the CTAs (pairs), each its k-blocks and a hand-over with
+// the epilogue. Fitted to 900 passes in CUDA graphs: the two layers at 512 to 557056 pixels, 96 to 384 channels, all tiles, half a round to
+// three and more; the choice is 0.1 % slower than the best plan on average, at most 3 %.
+// Us, a product per tap (two row blocks stacked where that was ahead) / this: 557056 pixels of 384 channels 1251 / 951, of 192 383 / 275,
+// 80000 of 256 104 / 85, 17280 of 192 25 / 21; transposed, 139264 of 384 186 / 161, of 192 69 / 57, of 96 45 / 35. (Of 96 and 128 channels
+// the row of ones costs a tile in ten: 17280 pixels 12.6 / 13.5 and 16.4 / 17.2; folding the gradients takes 2 to 10 us less than it did.)
+// `least_split`: the contraction is cut into so many parts at least (the error of the tensor core's fp32 sums grows with their length:
+// 139264 pixels of 384 channels, 18 parts 8.6e-6, 12 parts 13.0e-6), unless they are down to 15 k-blocks (1.0e-6; down to 24, 1.6e-6, is no
 // faster: 2656 pixels of 384 channels 15.9 / 15.1 us, 600 to every second 14.5 / 14.2).
 static TapPlan model_tap_wgrad(int taps, int channels, int N, long long k_blocks, bool row_sums, bool column_sums, int least_split, int num_sms) {
   struct Tile {

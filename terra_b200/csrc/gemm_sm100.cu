@@ -21,7 +21,7 @@
 //     zero fill outside the image, k-blocks enumerate (tap, channel chunk),
 //   * 2x2 / stride-2 transposed convolutions, their input gradient, and the input gradient of the stride-2 3x3
 //     convolution: the same gather with other tap tables, outputs stored to every second pixel through 5-D TMA boxes,
-//   * convolution weight gradients (contraction over pixels, one tile group per tap).
+//   * convolution weight gradients (contraction over pixels; the rows of all taps one after the other, or a tile group per tap).
 // Two further instantiations: CTA pairs (a cluster of two drives one cta_group::2 MMA over a 256-row tile, see GemmCfg)
 // and the tensor-parallel forms (A gathered from the peers' buffers, output scattered to the owners' buffers, see
 // gemm_sm100.cuh).
@@ -100,9 +100,9 @@ struct GemmCfg {
 // [3] TMA thread span, [4] of it waiting for free stages, [5] first epilogue warp span, [6] of it waiting for tiles.
 __device__ unsigned long long g_gemm_stalls[8];
 
-// Operand rows whose product with B is B's column sums (GemmParams::row_sums): 4 x 64 rows of 128 bf16, of which rows 64 j to 64 j + 63 have a one in
-// column 56 + j. A box of 64 x 64 of them from column 56 - 8 i and row 64 j on is a box of A whose row 8 i + j is ones. The others
-// are 2^-126, not zeros, which would turn an infinity of B into a NaN.
+// Operand rows whose product with B is B's column sums (GemmParams::row_sums): 4 x 64 rows of 128 bf16, of which rows 64 j to 64 j + 63
+// have a one in column 56 + j. A box of 64 x 64 of them from column 56 - 8 i and row 64 j on is a box of A whose row 8 i + j is ones. The
+// others are 2^-126, not zeros, which would turn an infinity of B into a NaN.
 #define TB_8(...) __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__, __VA_ARGS__
 #define TB_LOW 0x00800080u
 #define TB_LOW_4 TB_LOW, TB_LOW, TB_LOW, TB_LOW
@@ -127,10 +127,10 @@ struct TileCoord {
   int kb_begin, kb_end;
 };
 
-// Column sums of A (weight-gradient form): every tile of a row block streams the same A tiles, so the sums are shared out by
-// k-block, kb % ways == the tile's place among its row block's `ways` tiles (with a displaced A those of its group). (A 16-column MMA costs as much of the
-// tensor pipe and of the shared-memory port as 40 KB of operand stream: left to the first column tile it made that tile
-// half as slow again, and the launch waits for the slowest.) Returns this tile's first such k-block.
+// Column sums of A (weight-gradient form): every tile of a row block streams the same A tiles, so the sums are shared out by k-block, kb %
+// ways == the tile's place among its row block's `ways` tiles (with a displaced A those of its group). (A 16-column MMA costs as much of
+// the tensor pipe and of the shared-memory port as 40 KB of operand stream: left to the first column tile it made that tile half as slow
+// again, and the launch waits for the slowest.) Returns this tile's first such k-block.
 __device__ __forceinline__ int first_sum_kb(const GemmParams& p, const TileCoord& t, int ways) {
   const int place = p.disp_a ? t.n_blk : t.grp * p.num_n_tiles + t.n_blk;
   return t.kb_begin + (place + ways - t.kb_begin % ways) % ways;
@@ -596,8 +596,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..13)
     // tcgen05.ld hands lane l the 32 columns of accumulator row l. Global memory wants the opposite: neighbouring
-    // lanes on neighbouring addresses. The TMA form (first branch below) stages units for bulk stores. In the other form
-    // (fp32 output, peers, stacked tiles, matrices or operand mixes without a tensor map, TERRA_GEMM_TMA_EPILOGUE=0) every
+    // lanes on neighbouring addresses. The TMA forms (first two branches below) stage units for bulk stores and reductions. In the other form
+    // (fp32 output that is not accumulated, peers, matrices or operand mixes without a tensor map, TERRA_GEMM_TMA_EPILOGUE=0) every
     // transfer of a 32 x 32 chunk goes through the warp's 2 KB exchange buffer: row-per-lane on one side, four lanes per
     // row (eight rows, 64 contiguous bytes each, per instruction) on the global side. 16-byte vectors are XOR
     // swizzled by (row >> 1); the profiler still counts about two wavefronts per ideal one on the row-gathering
@@ -616,7 +616,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       return reinterpret_cast<uint4*>(my_x + rr * 64 + (((vec ^ (rr >> 1)) & 3) << 4));
     };
     constexpr int CPW = (CHUNKS + GEMM_EPI_WARPS / 4 - 1) / (GEMM_EPI_WARPS / 4);   // chunks per warp
-    // the bias gradient that rides on a weight gradient: column 0 of the sums accumulator, lane l holding the sum of A's column (row of D) q * 32 + l
+    // the bias gradient that rides on a weight gradient: column 0 of the sums accumulator, lane l holding the sum of A's column (row of D)
+    // q * 32 + l
     auto add_column_sums = [&](const TileCoord& tc, int dcol) {
       if (!Cfg::CAN_COLSUM || p.colsum == nullptr || part != 0 ||
           first_sum_kb(p, tc, p.disp_a ? p.num_n_tiles : p.groups * p.num_n_tiles) >= tc.kb_end)
@@ -637,17 +638,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       // columns are one unit per warp and tile.
       //
       // What bounds a unit is latency, three warps per scheduler being all there is to hide it. So the form of the epilogue is a
-      // compile-time constant (with the flags tested inside, every pair of elements became a basic block of its own), a unit's
-      // two tensor-memory loads are issued together, the bias of a unit is spread through shared memory once, and the input unit arrives in the buffer its output is staged in: a lane reads and writes
-      // the same 16 bytes. With two such buffers the next unit's load has this unit's processing time to arrive; with one (long contractions,
-      // which want the ring and hide the epilogue) it is on its way from HBM to L2 meanwhile and issued when the store has read the buffer.
-      // The first buffer (4 KB) stages the output; the second takes the saved pre-activation, or alternates with the first.
-      // Cycles per unit with the flags tested inside: bias 2400 (now under 1300), bias and residual 3400 + 800 waiting for the input, GELU
-      // with the pre-activation 4500, times GELU' 6100 + 800. Launches, before / now: 139264 x 1536 x 384 times GELU' 334 -> 261 us, the same with GELU 260
-      // -> 243, 139264 x 384 x 384 63 -> 54, 156672 x 1024 x 1024 with residual 316 -> 279, 17280 x 576 x 192 12.4 -> 10.0.
-      // Where the epilogue bounds the launch no wait for a tile hides a latency, so the next unit's bias is loaded and its input asked for before this one is
-      // worked on, at coordinates that the walk over the tiles has anyway (two walks of units of their own took about 500 cycles a unit, a bias
-      // loaded with its tile 600): times GELU' 254 -> 217 us and 139264 x 2976 x 384 503 -> 440, with residual 388 -> 375 and x 2208 x 192 366 -> 277.
+      // compile-time constant (with the flags tested inside, every pair of elements became a basic block of its own), a unit's two
+      // tensor-memory loads are issued together, the bias of a unit is spread through shared memory once, and the input unit arrives in the
+      // buffer its output is staged in: a lane reads and writes the same 16 bytes. With two such buffers the next unit's load has this
+      // unit's processing time to arrive; with one (long contractions, which want the ring and hide the epilogue) it is on its way from HBM
+      // to L2 meanwhile and issued when the store has read the buffer. The first buffer (4 KB) stages the output; the second takes the
+      // saved pre-activation, or alternates with the first. Cycles per unit with the flags tested inside: bias 2400 (now under 1300), bias
+      // and residual 3400 + 800 waiting for the input, GELU with the pre-activation 4500, times GELU' 6100 + 800. Launches, before / now:
+      // 139264 x 1536 x 384 times GELU' 334 -> 261 us, the same with GELU 260 -> 243, 139264 x 384 x 384 63 -> 54, 156672 x 1024 x 1024
+      // with residual 316 -> 279, 17280 x 576 x 192 12.4 -> 10.0. Where the epilogue bounds the launch no wait for a tile hides a latency,
+      // so the next unit's bias is loaded and its input asked for before this one is worked on, at coordinates that the walk over the tiles
+      // has anyway (two walks of units of their own took about 500 cycles a unit, a bias loaded with its tile 600): times GELU' 254 -> 217
+      // us and 139264 x 2976 x 384 503 -> 440, with residual 388 -> 375 and x 2208 x 192 366 -> 277.
       constexpr int UNITS = BN / 64, WARPS_PER_Q = GEMM_EPI_WARPS / 4;
       uint8_t* my_out = xchg + (warp - 2) * p.epi_bufs * Cfg::EPI_BUF;
       uint64_t* my_in = in_bar + 2 * (warp - 2);
@@ -666,8 +668,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         const bool with_bias = (flags & EPI_BIAS) != 0, gelu = (flags & EPI_GELU) != 0, save_pre = (flags & EPI_SAVE_PRE) != 0;
         const bool has_in = (flags & (EPI_RESIDUAL | EPI_MUL_DGELU)) != 0, dgelu = (flags & EPI_MUL_DGELU) != 0;
         const f32x2 alpha2 = f2_both(p.alpha);
-        // (GELU's chains are long enough to alternate between two runs of columns; the other forms lose by it: 139264 x 2976 x 384 with GELU 381 / 344 us,
-        // times GELU' 455 / 470)
+        // (GELU's chains are long enough to alternate between two runs of columns; the other forms lose by it: 139264 x 2976 x 384 with
+        // GELU 381 / 344 us, times GELU' 455 / 470)
         constexpr int RUN = FORM >= 0 && (FORM & EPI_GELU) ? 2 : 1;
         const int in_bufs = p.epi_bufs / 2;
         auto bias_pair = [&](int col) -> float2 {     // columns col, col + 1 (col even)

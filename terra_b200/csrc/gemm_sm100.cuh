@@ -63,10 +63,10 @@ struct GemmParams {
   const __nv_bfloat16* residual;
   const __nv_bfloat16* aux;
   long long ldc, ldc2, ldr, ldaux;
-  // EPI_ROW_CONV: a tile's rows are 1 << tile_shift consecutive pixels (128, 64 or 32) of as many rows of the tile grid as make 128. Outputs of row h go to row
-  // h * out_mul + out_off[phase][0] and column parity out_off[phase][1] of an image of out_h rows whose columns are
-  // split by parity when out_mul = 2 (out_w columns of each parity); phase = the tile's group, or with phase_cols > 0 the
-  // output column divided by it (N = phases * phase_cols).
+  // EPI_ROW_CONV: a tile's rows are 1 << tile_shift consecutive pixels (128, 64 or 32) of as many rows of the tile grid as make 128.
+  // Outputs of row h go to row h * out_mul + out_off[phase][0] and column parity out_off[phase][1] of an image of out_h rows whose columns
+  // are split by parity when out_mul = 2 (out_w columns of each parity); phase = the tile's group, or with phase_cols > 0 the output column
+  // divided by it (N = phases * phase_cols).
   int out_w, out_h, out_mul, phase_cols, tile_shift;
   short out_off[4][2];
   // k-block ranges per group (groups that contract over different taps), instead of the whole range split by split_k

@@ -40,7 +40,8 @@ struct GemmEpilogue {
   // contraction (sum over tokens of dy[token][n], the bias gradient) into colsum[n] (fp32), from an extra
   // 16-column MMA against a tile of ones. Null: off. Tile widths up to 192.
   float* colsum;
-  float* row_sums;    // weight-gradient form, output stored by TMA reductions: += the column sums of B, as a row of ones in A (gemm_row_sums_fit)
+  float* row_sums;    // weight-gradient form, output stored by TMA reductions: += the column sums of B, as rows of ones
+                      // in A (gemm_row_sums_fit)
   int stack;          // weight-gradient form: 2 = tiles of two 128-row blocks that share a tile of B (widths 128, 192; 256 without colsum)
 };
 

@@ -10,14 +10,11 @@ using OptTensor = c10::optional<torch::Tensor>;
 
 void conv3x3_fwd(const Tensor& x, const Tensor& w, Tensor& y, int64_t stride, int64_t flags, const OptTensor& bias, const OptTensor& residual,
                  const OptTensor& status, const OptTensor& halo_lo, const OptTensor& halo_hi);
-void conv3x3_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t stride, int64_t split_k, const OptTensor& status,
-                   const OptTensor& halo_lo, const OptTensor& halo_hi, const OptTensor& bias_grad, int64_t stack);
 void conv3x3_s2_dgrad(const Tensor& dy, const Tensor& w, Tensor& dx, const OptTensor& status);
 void convt2x2(int64_t op, const Tensor& in, const Tensor& w, const OptTensor& bias4, Tensor& out, const OptTensor& status);
-void convt2x2_wgrad(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t split_k, const OptTensor& status, int64_t stack,
-                    const OptTensor& bias_grad);
-// The weight gradients of one rank, all taps in one product: dw [9, Cin, Cout] or [4, Cout, Cin], accumulated, for fold_taps; bias_grad [Cout]
-// accumulated, by launches of its own unless `fuse_bias`. The contraction is cut into `least_split` parts at least. `plan` ({columns, CTAs, row blocks, split}): instead of the rule's
+// The weight gradients of one rank, all taps in one product: dw [9, Cin, Cout] or [4, Cout, Cin], accumulated, for fold_taps; bias_grad
+// [Cout] accumulated, by launches of its own unless `fuse_bias`. The contraction is cut into `least_split` parts at least. `plan`
+// ({columns, CTAs, row blocks, split}) takes the place of the rule's.
 using TapPlanRequest = c10::optional<std::vector<int64_t>>;
 void conv3x3_wgrad_taps(const Tensor& x, const Tensor& dy, Tensor& dw, int64_t stride, const OptTensor& status, const OptTensor& bias_grad,
                         bool fuse_bias, int64_t least_split, const TapPlanRequest& plan = c10::nullopt);
@@ -30,14 +27,6 @@ Tensor scratch_take(const Tensor& like, at::IntArrayRef sizes);
 void scratch_give(const Tensor& scratch);
 
 void colsum(const Tensor& x, Tensor& out);
-void groupnorm_mean_rstd(const Tensor& x, Tensor& scratch, Tensor& stats, int64_t groups, double inv_count, double eps);
-void groupnorm_silu_apply(const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, const OptTensor& res, Tensor& y,
-                          int64_t groups);
-void groupnorm_silu_bwd_reduce(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& g, const Tensor& b, Tensor& red,
-                               int64_t groups, const OptTensor& dgamma, const OptTensor& dbeta);
-void strided_add(Tensor& src, Tensor& dst, int64_t sa, int64_t sb, int64_t sc);
-void groupnorm_silu_bwd_apply(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& red, const Tensor& g, const Tensor& b,
-                              Tensor& dx, int64_t groups, double inv_count);
 
 void wgrad(const Tensor& dy, const Tensor& x, const Tensor& grad_w, const OptTensor& grad_b, bool fuse_bias, const Tensor& status);
 Tensor linear_product(const Tensor& x, const Tensor& w, bool transposed, const OptTensor& bias, const OptTensor& residual, const Tensor& status);

@@ -602,8 +602,8 @@ __global__ void __launch_bounds__(WaCfg<HD, NPAD, HPC, BWD>::THREADS, (WaCfg<HD,
       }
       __syncthreads();
       // ---- phase 2, a warp per 16 keys: dV = P^T dO, dK = scale dS^T Q. (Half of the warps for dV and half for dK, 32 keys each, read
-      // less of dO and Q but measured up to 6 % slower at 64 tokens.) K and V are dead: their rows stage the results. With sequence parallelism every
-      // rank of the window recomputes the whole window (cheap) and keeps only the gradients of its own token shard, so no
+      // less of dO and Q but measured up to 6 % slower at 64 tokens.) K and V are dead: their rows stage the results. With sequence
+      // parallelism every rank of the window recomputes the whole window (cheap) and keeps only the gradients of its own token shard, so no
       // cross-rank reduction of dK / dV is needed.
       const int qblocks = (N + 15) >> 4;
       if (row0 < N) {

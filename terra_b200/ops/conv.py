@@ -165,7 +165,9 @@ def _stream_cost(heavy, light, bn, split, sms=148):
 def _wgrad_plan(taps, M, N, kblocks):
     """(split-K factor, row blocks per tile) of a convolution's weight gradient: ``taps`` products of ``M`` x ``N`` outputs.
     Two row blocks share a tile of the other operand (15 % less traffic per output) where that also comes out ahead with the
-    single block an odd count leaves over and with whole rounds of CTAs; every split adds 0.2 % for its pass of atomics."""
+    single block an odd count leaves over and with whole rounds of CTAs; every split adds 0.2 % for its pass of atomics. The
+    native nodes of one rank run all taps as one product, with a plan of their own (``gemm_host.cu::model_tap_wgrad``), and take
+    this split as the least number of parts: the sums of a part are as long as here at most, and so is their error."""
     bn = 192 if N % 192 == 0 else 128            # the tile width the kernel picks
     blocks, n = (M + 127) // 128, taps * ((N + bn - 1) // bn)
     best = balanced_split(blocks * n, kblocks)

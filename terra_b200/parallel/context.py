@@ -34,11 +34,11 @@ from .window_assignment import window_owner_map
 
 
 def _swap_middle(t, outer, a, b, shape):
-    """``t`` as ``[outer, a, b, inner]`` with ``a`` and ``b`` exchanged, in ``shape``, by one copy kernel; None where it does not apply (the tensor
-    operators do it: CPU, other types and layouts, inner parts of no whole 16-byte vectors, traces and function transforms; sizes that do not fit, which
-    they refuse; one of the two of size 1, which they answer without a copy)."""
-    if not (outer > 0 and a > 1 and b > 1 and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and 0 < t.numel() < 1 << 33 and t.data_ptr() % 16 == 0
-            and t.numel() % (8 * outer * a * b) == 0 and torch.autograd.forward_ad._current_level < 0 and B.native_node()):
+    """``t`` as ``[outer, a, b, inner]`` with ``a`` and ``b`` exchanged, in ``shape``, by one copy kernel; None where it does not apply
+    (the tensor operators do it: CPU, other types and layouts, inner parts of no whole 16-byte vectors, traces and function transforms;
+    sizes that do not fit, which they refuse; one of the two of size 1, which they answer without a copy)."""
+    if not (outer > 0 and a > 1 and b > 1 and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and 0 < t.numel() < 1 << 33
+            and t.data_ptr() % 16 == 0 and t.numel() % (8 * outer * a * b) == 0 and torch.autograd.forward_ad._current_level < 0 and B.native_node()):
         return None
     return B._ext.load().nodes.swap_middle(t, outer, a, b, shape)
 

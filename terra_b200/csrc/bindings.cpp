@@ -224,9 +224,10 @@ void convt2x2_wgrad(const torch::Tensor& x, const torch::Tensor& dy, torch::Tens
   rc_check(rc, "convt2x2_wgrad");
 }
 
-static void check_patches(const Tensor& image, const Tensor& grid, int64_t p, int64_t top, int64_t left) {
+static void check_patches(const Tensor& image, const Tensor& grid, const Tensor& w, const Tensor& bias, int64_t p, int64_t top, int64_t left) {
   check_image(image, "image");
   check_image(grid, "patches");
+  TORCH_CHECK(grid.device() == image.device() && w.device() == image.device() && bias.device() == image.device(), "patches: operands on one GPU");
   TORCH_CHECK(image.numel() > 0 && image.size(0) == grid.size(0) && p >= 1 && p <= 4 && image.size(1) % p == 0 && image.size(2) % p == 0 && top >= 0 &&
                   left >= 0 && top + image.size(1) / p <= grid.size(1) && left + image.size(2) / p <= grid.size(2) && p * image.size(3) % 8 == 0 &&
                   grid.size(3) % 8 == 0 && p * ((p * image.size(3) + 63) / 64) <= 128 && (grid.size(3) + 63) / 64 <= 128,
@@ -235,7 +236,7 @@ static void check_patches(const Tensor& image, const Tensor& grid, int64_t p, in
 
 // image [B, H, W, C] -> y [B, rows, cols, N]; w [N, p * (p * C padded to 64)], bias [N]; top and left in patches
 void embed_image(const Tensor& image, const Tensor& w, const Tensor& bias, Tensor& y, int64_t p, int64_t top, int64_t left, const OptTensor& status) {
-  check_patches(image, y, p, top, left);
+  check_patches(image, y, w, bias, p, top, left);
   check_packed(w, y.size(3), p, p * image.size(3));
   TORCH_CHECK(bias.scalar_type() == torch::kBFloat16 && bias.is_contiguous() && bias.numel() == y.size(3), "embed_image: bias bf16 [N]");
   const c10::cuda::CUDAGuard guard(image.device());
@@ -248,8 +249,9 @@ void embed_image(const Tensor& image, const Tensor& w, const Tensor& bias, Tenso
 // out = image + the patches of t [B, rows, cols, D] inside it; w [p * (p * C padded to 64), D padded to 64], bias alike
 void recover_image(const Tensor& t, const Tensor& w, const Tensor& bias, const Tensor& image, Tensor& out, int64_t p, int64_t top, int64_t left,
                    const OptTensor& status) {
-  check_patches(image, t, p, top, left);
+  check_patches(image, t, w, bias, p, top, left);
   check_image(out, "out");
+  TORCH_CHECK(out.device() == image.device(), "recover_image: out on the image's GPU");
   const int64_t run = (p * image.size(3) + 63) / 64 * 64;
   check_packed(w, p * run, 1, t.size(3));
   TORCH_CHECK(out.sizes() == image.sizes() && bias.scalar_type() == torch::kBFloat16 && bias.is_contiguous() && bias.numel() == p * run,

@@ -126,3 +126,18 @@ def test_a_captured_call_reads_the_weights_of_its_replay():
                 p.bf16.mul_(-0.5)
         graph.replay()
         assert _close(y, m(_unaligned(x)))
+
+
+@pytest.mark.parametrize("where", ["w", "bias"])
+def test_operands_on_another_device_are_refused(where):
+    from terra_b200 import _ext
+    from terra_b200.ops.gemm import status_word
+
+    x, tokens = _field(), torch.zeros(1, 16, 24, 64, device="cuda", dtype=torch.bfloat16)
+    ops = dict(w=torch.zeros(64, 4 * 64, device="cuda", dtype=torch.bfloat16), bias=torch.zeros(64, device="cuda", dtype=torch.bfloat16))
+    back = dict(w=torch.zeros(4 * 64, 64, device="cuda", dtype=torch.bfloat16), bias=torch.zeros(4 * 64, device="cuda", dtype=torch.bfloat16))
+    ops[where], back[where] = ops[where].cpu(), back[where].cpu()
+    with pytest.raises(RuntimeError):
+        _ext.load().embed_image(x, ops["w"], ops["bias"], tokens, 4, 0, 0, status_word("cuda"))
+    with pytest.raises(RuntimeError):
+        _ext.load().recover_image(tokens, back["w"], back["bias"], x, torch.empty_like(x), 4, 0, 0, status_word("cuda"))

@@ -78,7 +78,7 @@ int gemm_bf16(const GemmOperand& A, const GemmOperand& B, long long M, long long
 // tile of 128 rows each (2: a CTA pair). `gathered`: of a convolution with M / 128 row tiles and K / 64 taps x channel chunks.
 bool gemm_pairs();   // CTA pairs are allowed (TERRA_GEMM_2CTA)
 void gemm_tile(long long M, long long N, long long K, bool b_mn, int flags, bool gathered, int num_sms, int* bn, int* ctas);
-// whether tiles of `blocks` 128-row blocks leave room for a row of ones behind `rows` rows (GemmEpilogue::row_sums)
+// whether tiles of `blocks` 128-row blocks leave room for a box of rows of ones behind `rows` rows (GemmEpilogue::row_sums)
 bool gemm_row_sums_fit(long long rows, int blocks);
 bool gemm_tma_epilogue();   // whether the epilogue may go through TMA (environment switch)
 int gemm_stall_counters(unsigned long long* out8, int reset);

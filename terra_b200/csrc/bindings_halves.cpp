@@ -2,6 +2,7 @@
 // (which the multi-rank layouts use), without the interpreter between them. A small layer is bound by its launches: on 512
 // rows of width 96 the Python form spent about 20 us per launch on the host against 1 to 10 us of kernel time.
 #include <algorithm>
+#include <cstdint>
 #include <tuple>
 #include <vector>
 #include <torch/extension.h>
@@ -122,15 +123,16 @@ struct WgradPlan {
   int bn, stack, split;
   bool swapped;      // the transpose: rows are x's columns
 };
-// How many of the tiles of 128 or 256 rows and 128, 192 or 256 columns it takes that cover N x K outputs with least padding (the fewest of such).
-int64_t covering_tiles(int64_t N, int64_t K) {
-  int64_t least = 0, tiles = 0;
-  for (int64_t h : {256, 128})
-    for (int64_t w : {256, 192, 128}) {
-      const int64_t count = (N + h - 1) / h * ((K + w - 1) / w), area = count * h * w;
-      if (tiles == 0 || area < least || (area == least && count < tiles)) least = area, tiles = count;
+// How many of the tiles of 128 or 256 rows and 128, 192 or 256 columns it takes that cover N x K outputs with least padding: of several, the
+// largest, but with sums 192 columns before 256, which have no room for them.
+int64_t covering_tiles(int64_t N, int64_t K, bool sums) {
+  std::tuple<int64_t, int, int64_t> least{INT64_MAX, 0, 0};
+  for (int64_t h : {128, 256})
+    for (int64_t w : {128, 192, 256}) {
+      const int64_t count = (N + h - 1) / h * ((K + w - 1) / w);
+      least = std::min(least, {count * h * w, !sums ? 0 : w == 192 ? 0 : w == 256 ? 1 : 2, count});
     }
-  return tiles;
+  return std::get<2>(least);
 }
 WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   struct Tile {
@@ -181,7 +183,7 @@ WgradPlan model_wgrad(int64_t N, int64_t K, int64_t M, bool sums) {
   for (const Choice& c : choices)
     if (c.time <= 1.03 * least && (best == nullptr || c.plan.split > best->plan.split || (c.plan.split == best->plan.split && c.time < best->time)))
       best = &c;
-  const int64_t parts = std::max<int64_t>(1, sms / covering_tiles(N, K)), longest = std::max<int64_t>(15, (k_blocks + parts - 1) / parts);
+  const int64_t parts = std::max<int64_t>(1, sms / covering_tiles(N, K, sums)), longest = std::max<int64_t>(15, (k_blocks + parts - 1) / parts);
   if (best->length > longest) {      // the cheapest of those that keep to it, else the shortest parts
     for (const Choice& c : choices) {
       if (c.time > 1.15 * least) continue;

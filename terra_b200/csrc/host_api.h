@@ -38,7 +38,7 @@ struct GemmEpilogue {
   void* status;       // KernelStatus* (device), may be null
   // Weight-gradient form (A read MN-major, fp32 atomic output): also accumulate the sums of A's columns over the
   // contraction (sum over tokens of dy[token][n], the bias gradient) into colsum[n] (fp32), from an extra
-  // 16-column MMA against a tile of ones. Null: off. Tile widths up to 192.
+  // 16-column MMA against tiles with rows of ones. Null: off. Tile widths up to 192.
   float* colsum;
   float* row_sums;    // weight-gradient form, output stored by TMA reductions: += the column sums of B, as rows of ones
                       // in A (gemm_row_sums_fit)

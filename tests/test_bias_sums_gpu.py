@@ -66,3 +66,22 @@ def test_transposed_weight_gradient(M, N, K, pad):
     wgrad_accumulate(dy, x, gw, gb)
     check_status("cuda")
     assert _rel(gb, dy.double().sum(0)) < REL and not gw.any()
+
+
+@pytest.mark.parametrize("M,N,K", [(557056, 2976, 384), (156672, 3072, 1024), (60000, 384, 384), (60001, 288, 96)])
+def test_weight_gradient_with_its_column_sums(M, N, K):
+    """The sums that are an MMA against a tile of ones: each of a k-block's four MMAs has a column of its own."""
+    from terra_b200.ops.blocks import wgrad_accumulate
+    from terra_b200.ops.gemm import check_status
+
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    dy, x = _field(gen, M, N), torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    gw, gb = torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda")
+    wgrad_accumulate(dy, x, gw, gb)
+    check_status("cuda")
+    want = torch.stack([dy[:, c:c + 384].double().sum(0) for c in range(0, N, 384)]).reshape(-1) if N % 384 == 0 else dy.double().sum(0)
+    assert _rel(gb, want) < REL and not gw.any()
+    dy[5, 3], dy[M - 1, 7], dy[M // 2, 9] = float("inf"), float("-inf"), float("nan")
+    gb.zero_()
+    wgrad_accumulate(dy, x[:, :K], gw, gb)
+    assert gb[3] == float("inf") and gb[7] == float("-inf") and gb[9].isnan() and torch.isfinite(gb).sum() == N - 3
